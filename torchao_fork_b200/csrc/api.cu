@@ -17,6 +17,7 @@ int64_t int4_gemv_tc_workspace_bytes(int64_t Np);
 int int4_gemm_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np, int64_t Kp,
                  int G, void* y, int64_t N_out, int64_t ldy, void* workspace, int64_t workspace_bytes, cudaStream_t s);
 int64_t int4_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
+int64_t int8_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
 int int8_gemv(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Kp,
               void* y, int64_t N_out, int64_t ldy, cudaStream_t s);
 int int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Np,
@@ -173,7 +174,7 @@ extern "C" int ao_b200_int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int
 extern "C" int64_t ao_b200_int8_mm_workspace_bytes(int64_t M, int64_t Np, int64_t Kp) {
   // the GEMM's permuted copy of the activations (+ split-K partial sums).  (Routing 2 < M <= 16 batches that do not fit the
   // GEMV staging through the GEMM was measured SLOWER than the plain strip GEMV: 40 vs 18-28 us on 4096 x 14336.)
-  return M > 16 ? ao::int4_gemm_tc_workspace_bytes(M, Np, Kp) : 0;
+  return M > 16 ? ao::int8_gemm_tc_workspace_bytes(M, Np, Kp) : 0;
 }
 
 static int int8_args_ok(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Np,

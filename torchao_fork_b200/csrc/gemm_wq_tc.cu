@@ -1,0 +1,873 @@
+// Weight-only quantized linear for more than a few rows, int4 and int8: fused dequant + GEMM on tcgen05 / tensor memory.
+//
+//   y[m][n] = sum_k x[m][k] * W'[n][k]
+//   int4   W' = bf16_rn((q - 8) * scale + zero): the arithmetic of the reference's tinygemm op (aten._weight_int4pack_mm, behind
+//          torchao/dtypes/uintx/tensor_core_tiled_layout.py:_linear_bf16_act_uint4_weight_impl), one rounding per weight;
+//   int4, few rows (DEFER)   W' unrounded: the affine is applied in fp32 to the sums over 128 k (or a group, if that is
+//          smaller): y += s D + (z - 136 s) X with D = sum x (128 + q), X = sum x;
+//   int8   W' = q, the row scale applied to the bf16-rounded sum (torchao/dtypes/uintx/plain_layout.py:250-266).
+//
+// The tensor-core mapping is transposed so that the dequantized weights never touch shared memory:
+//   MMA M (128 TMEM lanes)  = 128 weight rows (8 strips of the strip-major packed layout)
+//   MMA N (16 .. 256)       = NT activation rows
+//   A operand               = W' in TENSOR MEMORY, written by the dequant warps with tcgen05.st.16x128b: the 16-byte lane chunk
+//                             of the packed layout holds rows g / g + 8 of a strip, which is that store's (lane, column) pattern
+//   B operand               = activations in shared memory (no-swizzle K-major core matrices), one bulk copy per 128 k out of
+//                             a copy of x that stage_x_kernel has put into that order (the k order inside a 32-k block is the
+//                             store's: column 4 i + c holds k = 8 c + 2 i, 2 i + 1, so neither side shuffles)
+//   D                       = fp32 in tensor memory
+//
+// PAIR: two CTAs of a cluster work on 256 weight rows x NT activation rows with cta_group::2 MMAs: each dequantizes its own
+// 128 rows and holds half of the activation tile, so the shared-memory and L2 traffic of the activations is halved.  (One CTA
+// at NT = 256 would need 64 B/clk of shared-memory writes and as much in reads for B alone, of 128 B/clk.)
+//
+// Work split: units of (row block, row tile of x, 128 k), tile-major, dealt out contiguously and evenly to as many CTAs (or
+// pairs) as there are SMs.  A tile whose K is shared between neighbours is summed by the one that arrives last, in CTA order
+// (fp32 partial sums and tickets in the workspace; nobody waits for another CTA), so there is no last wave that is nearly
+// empty and few row blocks still fill the chip.
+//
+// Roles (768 threads): warps 0-3 epilogue (warp = TMEM lane quadrant), 4-19 dequant (one strip each; two sets take
+// alternate units), 20 weight producer (two TMA tensor copies per unit: 8 strips of weights, 8 strips of parameters),
+// 21 activation producer, 22 and 23 MMA issue: the waits, the issue and the commit of a unit take one warp 600 clocks, so up to
+// NT = 64 two warps take alternate units, each with accumulators of its own that the epilogue adds.  At the end all warps
+// add up the tiles that this CTA was the last to reach.  Every wait is bounded: a CTA that gives up sets `status` and returns.
+//
+// Bound by the tensor cores from about 512 rows (8 MMAs of N = 256 take 1024 clocks per unit and pair, the dequant of a unit
+// about 900 clocks per set of warps, two sets in flight), below that by the dequant -> MMA chain of a unit.  Measured, 14336 x 4096,
+// int4 with groups of 128, M = 64 / 256 / 512 / 1000 / 2048: 23.6 / 37.0 / 52.6 / 90 / 168 us, the last 0.85 of 1671 TFLOP/s (one CTA
+// per 128 x 256 tile with the whole K, activations multicast over 4 CTAs, run-time divisions and parameters read from global memory in
+// the dequant loop: 29.9 / 36.5 / 67.0 / 128 / 225 us); int8 8192 x 8192, M = 32 / 512 / 2048: 24 / 63 / 225 us (44 / 66 / 244 us).
+#include <cuda.h>
+#include <cuda_bf16.h>
+
+#include "common.cuh"
+
+namespace ao {
+
+constexpr int kWqEpiWarps = 4, kWqDqWarps = 16;
+constexpr int kWqWProd = kWqEpiWarps + kWqDqWarps, kWqXProd = kWqWProd + 1, kWqMma = kWqXProd + 1;
+constexpr int kWqThreads = (kWqMma + 2) * 32;  // 768
+constexpr int kWqSlots = 4;                    // ring of A in tensor memory: 64 columns (128 k) each
+constexpr int kWqMaxW = 16, kWqMaxX = 8;       // rings of weights and of tiles of x
+constexpr int kWqPitch = 128 * 2 + 16;         // bytes of a row of the output tile in shared memory (rows land on distinct banks)
+constexpr int kWqHeader = 1024;                // mbarriers, TMEM base, give-up flag
+constexpr int kWqMaxSplitTiles = 16;           // tiles per worker from which whole tiles are dealt out (imbalance <= 1/16)
+
+struct WqParams {
+  CUtensorMap wmap;          // weights: rows = strips, row = the strip's bytes; box = 8 strips x 128 k
+  CUtensorMap smap;          // int4 scale / zero: rows = strips, row = 16 words per group; box = 8 strips x the unit's groups
+  const uint8_t* xt;         // staged activations [MT * ranks][KU][x_bytes]
+  const __nv_bfloat16* scale8;
+  __nv_bfloat16* y;
+  float* part;               // shares of split tiles [workers][2][ranks][NT * 128]
+  uint32_t* tickets;         // [tiles][ranks], zeroed by the staging kernel
+  uint32_t* status;
+  int64_t N_out, ldy;
+  int M, NT, BR, KU, MT, w_slots, x_slots, a_slots, n_mma, vec_store;
+  uint32_t off_w;            // weight ring
+  uint32_t x_bytes;          // one unit of staged activations (and, DEFER, its sums)
+  int quantum, base, rem;    // worker c owns units [first(c), first(c + 1)), first(c) = (c base + min(c, rem)) quantum
+};
+
+__host__ __device__ __forceinline__ int wq_first(int c, int base, int rem, int quantum) { return (c * base + (c < rem ? c : rem)) * quantum; }
+__device__ __forceinline__ int wq_owner(int u, int base, int rem, int quantum) {
+  const int v = u / quantum, big = rem * (base + 1);
+  return v < big ? v / (base + 1) : rem + (v - big) / base;
+}
+
+// ---- staging: x -> bf16 units in the B operand's order ---------------------------------------------------------------
+// unit (block b of BR rows, 128-k unit ku): [16 chunks of 8 k][BR rows][8] and, SEG > 0, behind it fp32 sums [128 / SEG][16].
+// Chunk 4 q + i holds of the 32-k quarter q the k = 8 c + 2 i + e at place 2 c + e.  A thread moves 32 k of one row: 64 bytes in,
+// four 16-byte pieces out; a warp covers 8 rows x 128 k, so that every piece of 8 rows is one full 128-byte line.
+// Rows >= M and columns >= Kx are zero.  Bound by HBM / L2: bytes of x in and out once.
+template <int SEG>
+__global__ void __launch_bounds__(256) stage_x_kernel(const __nv_bfloat16* __restrict__ x, int64_t M, int64_t Kx, int64_t ldx, int n_blocks, int BR, int KU,
+                                                      uint32_t x_bytes, uint8_t* __restrict__ xt, uint32_t* __restrict__ tickets, int n_tickets) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int64_t gid = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (gid < n_tickets) tickets[gid] = 0u;
+  const int lane = threadIdx.x & 31, row8 = lane >> 2, quarter = lane & 3;  // quarter: 32-k piece of the unit
+  const int groups = BR / 8;
+  for (int64_t w = gid >> 5; w < (int64_t)n_blocks * groups * KU; w += ((int64_t)gridDim.x * 256) >> 5) {
+    const int ku = (int)(w % KU);
+    const int64_t rg = w / KU;
+    const int b = (int)(rg / groups), r = (int)(rg - (int64_t)b * groups) * 8 + row8;
+    const int64_t m = (int64_t)b * BR + r, k0 = (int64_t)ku * 128 + quarter * 32;
+    uint4 v[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      v[c] = make_uint4(0u, 0u, 0u, 0u);
+      if (m < M && k0 + 8 * c < Kx) v[c] = *reinterpret_cast<const uint4*>(x + m * ldx + k0 + 8 * c);  // Kx % 8 == 0: all or nothing
+    }
+    uint8_t* unit = xt + ((int64_t)b * KU + ku) * x_bytes;
+    uint8_t* dst = unit + ((int64_t)(quarter * 4) * BR + r) * 16;
+    *reinterpret_cast<uint4*>(dst) = make_uint4(v[0].x, v[1].x, v[2].x, v[3].x);
+    *reinterpret_cast<uint4*>(dst + (int64_t)BR * 16) = make_uint4(v[0].y, v[1].y, v[2].y, v[3].y);
+    *reinterpret_cast<uint4*>(dst + (int64_t)BR * 32) = make_uint4(v[0].z, v[1].z, v[2].z, v[3].z);
+    *reinterpret_cast<uint4*>(dst + (int64_t)BR * 48) = make_uint4(v[0].w, v[1].w, v[2].w, v[3].w);
+    if constexpr (SEG > 0) {
+      float s = 0.f;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        float f[8];
+        unpack8(v[c], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s += f[e];
+      }
+      if (SEG >= 64) s += __shfl_xor_sync(0xffffffffu, s, 1);
+      if (SEG >= 128) s += __shfl_xor_sync(0xffffffffu, s, 2);
+      if ((quarter * 32) % SEG == 0) reinterpret_cast<float*>(unit + (int64_t)BR * 256)[(quarter * 32 / SEG) * 16 + r] = s;
+    }
+  }
+}
+
+// ---- PTX wrappers ------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void wq_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void wq_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ bool wq_elect_one() {
+  uint32_t pred;
+  asm volatile("{\n\t.reg .b32 rx;\n\t.reg .pred px;\n\telect.sync rx|px, 0xffffffff;\n\tselp.u32 %0, 1, 0, px;\n\t}" : "=r"(pred));
+  return pred != 0;
+}
+// PAIR: both CTAs' barriers at this offset
+template <bool PAIR>
+__device__ __forceinline__ void wq_commit(uint64_t* bar) {
+  if constexpr (PAIR)
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3)
+                 : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// D(tmem, f32 [128 or 256][N]) (+)= A(tmem, bf16 [..][16]) * B(smem, bf16 [N][16])
+template <bool PAIR>
+__device__ __forceinline__ void wq_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  if constexpr (PAIR)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem),
+                 "l"(b_desc), "r"(idesc), "r"(accumulate)
+                 : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem),
+                 "l"(b_desc), "r"(idesc), "r"(accumulate)
+                 : "memory");
+}
+__device__ __forceinline__ void wq_st_16x128b_x8(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
+               "r"(r[14]), "r"(r[15])
+               : "memory");
+}
+// 16 lanes x 16 columns: thread l holds row l / 4 (d[0], d[1]; second 8 columns d[4], d[5]) and row l / 4 + 8 (d[2], d[3], d[6], d[7]),
+// columns 2 (l % 4), + 1 of each 8
+__device__ __forceinline__ void wq_ld_16x256b_x2(uint32_t taddr, uint32_t* d) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void wq_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// four 8 x 8 blocks of that shape, transposed: lanes 8 i .. 8 i + 7 give the row addresses of block i
+__device__ __forceinline__ void wq_stmatrix_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void wq_tma_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)), "l"(map),
+               "r"(x), "r"(y), "r"(smem_u32(bar))
+               : "memory");
+}
+// arrival on the leader CTA's barrier at this offset (PAIR), else on the own one.  (What it announces is in tensor memory or was
+// written by the async proxy and is complete; .release.cluster here made every arrival wait about 1900 clocks.)
+template <bool PAIR>
+__device__ __forceinline__ void wq_arrive_leader(uint64_t* bar) {
+  if constexpr (PAIR)
+    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\tmbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+  else
+    mbar_arrive(bar);
+}
+// bounded wait: false (and *dead set) after about two seconds, or as soon as another warp of the CTA has given up
+__device__ __forceinline__ bool wq_wait(uint64_t* bar, uint32_t parity, volatile int* dead) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 32; ++i)
+      if (mbar_try_wait(bar, parity)) return true;
+    if (*dead != 0 || clock64() - t0 > 4000000000ll) {
+      *dead = 1;
+      return false;
+    }
+  }
+}
+// barrier of the epilogue warps; true if any of them brings a failure
+__device__ __forceinline__ bool wq_epi_sync(bool failed) {
+  uint32_t any;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+               : "=r"(any)
+               : "r"((uint32_t)failed), "n"(kWqEpiWarps * 32)
+               : "memory");
+  return any != 0;
+}
+// ring position: slot and the parity of its current use
+struct WqRing {
+  int slot = 0;
+  uint32_t use = 0;
+  __device__ __forceinline__ void step(int by, int n) {
+    slot += by;
+    if (slot >= n) {
+      slot -= n;
+      use ^= 1u;
+    }
+  }
+};
+
+// ---- the GEMM ----------------------------------------------------------------------------------------------------------
+// G == 0: int8.  Shared memory: header, output tile, activation ring (x_slots x x_bytes), weight ring (w_slots x [8 strips x 128 k]
+// [8 strips x parameters]).
+template <int G, bool DEFER, bool PAIR>
+__global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_constant__ WqParams p) {
+  extern __shared__ __align__(1024) uint8_t wq_smem[];
+  constexpr bool kI8 = (G == 0);
+  constexpr int kTileB = kI8 ? 1024 : 512;                                // bytes of one (strip, 64-k) tile
+  constexpr int kSegs = DEFER ? (G < 128 ? 128 / (G ? G : 128) : 1) : 1;  // accumulation segments per unit
+  constexpr int kSzWords = kI8 ? 0 : (G < 128 ? 128 / (G ? G : 128) : 1) * 16;
+  constexpr uint32_t kWBytes = 8 * 2 * kTileB, kSBytes = 8 * kSzWords * 4, kWSlot = kWBytes + kSBytes;
+  constexpr int kRanks = PAIR ? 2 : 1;
+  uint64_t* wfull = reinterpret_cast<uint64_t*>(wq_smem);
+  uint64_t* wempty = wfull + kWqMaxW;
+  uint64_t* xfull = wempty + kWqMaxW;     // per slot of x: the tile has landed here
+  uint64_t* xpeer = xfull + kWqMaxX;      // PAIR, leader: ... and in the second CTA
+  uint64_t* xdone = xpeer + kWqMaxX;      // the MMAs on it have retired (DEFER: D is final)
+  uint64_t* dread = xdone + kWqMaxX;      // DEFER: the epilogue has read D and the sums
+  uint64_t* afull = dread + kWqMaxX;      // per slot of A: it is in tensor memory
+  uint64_t* adone = afull + kWqSlots;     // the MMAs on it have retired
+  uint64_t* dfull = adone + kWqSlots;     // accumulator buffers of a tile
+  uint64_t* dempty = dfull + 2;
+  uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(dempty + 2);
+  volatile int* dead = reinterpret_cast<volatile int*>(tmem_base_s + 1);
+  volatile int* s_last = dead + 1;        // [2]: this CTA was the last to reach its first / last tile
+  uint8_t* stage = wq_smem + kWqHeader;   // output tile [NT][kWqPitch]
+  uint8_t* xring = stage + p.NT * kWqPitch;
+  uint8_t* wring = wq_smem + p.off_w;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int worker = blockIdx.x / kRanks, rank = blockIdx.x % kRanks;
+  const int u0 = wq_first(worker, p.base, p.rem, p.quantum), u1 = wq_first(worker + 1, p.base, p.rem, p.quantum);
+  const int KU = p.KU, NT = p.NT, x_slots = p.x_slots, a_slots = p.a_slots, n_mma = p.n_mma;
+  const int d_bufs = NT <= 128 ? 2 : 1;
+  grid_launch_dependents();
+
+  // the weights wait for nobody: their producer fills the ring while the others set up
+  auto load_weights = [&](int u, int slot) {
+    const int t = u / KU, ku = u - t * KU, strip = ((t / p.MT) * kRanks + rank) * 8;
+    uint8_t* dst = wring + slot * kWSlot;
+    mbar_arrive_expect_tx(&wfull[slot], kWSlot);
+    wq_tma_2d(dst, &p.wmap, ku * 256, strip, &wfull[slot]);
+    if constexpr (!kI8) wq_tma_2d(dst + kWBytes, &p.smap, G == 256 ? (ku >> 1) * 16 : ku * kSzWords, strip, &wfull[slot]);
+  };
+  if (warp == kWqWProd) {
+    if (lane < p.w_slots) {
+      mbar_init(&wfull[lane], 1);
+      mbar_init(&wempty[lane], DEFER ? 8 + kWqEpiWarps : 8);  // DEFER: the epilogue reads the parameters
+    }
+    fence_barrier_init();
+    __syncwarp();
+    if (wq_elect_one())
+      for (int i = 0; i < p.w_slots && u0 + i < u1; ++i) load_weights(u0 + i, i);
+    __syncwarp();
+  } else if (warp == kWqMma) {
+    if (lane < x_slots) {
+      mbar_init(&xfull[lane], 1);
+      mbar_init(&xpeer[lane], 1);
+      mbar_init(&xdone[lane], 1);
+      mbar_init(&dread[lane], kWqEpiWarps);
+    } else if (lane >= 8 && lane < 8 + kWqSlots) {
+      mbar_init(&afull[lane - 8], 8 * kRanks);
+      mbar_init(&adone[lane - 8], 1);
+    } else if (lane >= 16 && lane < 18) {
+      mbar_init(&dfull[lane - 16], n_mma);
+      mbar_init(&dempty[lane - 16], kWqEpiWarps * kRanks);
+      s_last[lane - 16] = 0;
+    } else if (lane == 18) {
+      *dead = 0;
+    }
+    fence_barrier_init();
+    __syncwarp();
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_s)), "r"(512));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_s)), "r"(512));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    wq_fence_before();
+  }
+  __syncthreads();
+  if constexpr (PAIR) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  wq_fence_after();
+  const uint32_t tb = *reinterpret_cast<volatile uint32_t*>(tmem_base_s);
+  // columns [0, 256): accumulators (DEFER: one per slot of x and segment, else [buffer][MMA warp]); [256, 512): A ring
+  const uint32_t a_col0 = tb + 256;
+
+  // fp32 sums of 32 rows x 16 columns (fragment order of wq_ld_16x256b_x2, lanes 0-15 in f[0..7], 16-31 in f[8..15]) -> output tile
+  auto to_stage = [&](int q, int c, const float (&f)[16], const float (&sc)[4]) {
+    const uint32_t at = smem_u32(stage) + (uint32_t)(c + 8 * (lane >> 4) + (lane & 7)) * kWqPitch + (32 * q + 8 * ((lane >> 3) & 1)) * 2;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t o[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {  // block i: column group i >> 1, row group i & 1
+        float a = f[8 * h + 4 * (i >> 1) + 2 * (i & 1)], b = f[8 * h + 4 * (i >> 1) + 2 * (i & 1) + 1];
+        // int8: mm result rounded to bf16, THEN multiplied by the row scale and rounded again
+        if constexpr (kI8) a = bf16r(a) * sc[2 * h + (i & 1)], b = bf16r(b) * sc[2 * h + (i & 1)];
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[i]) : "f"(b), "f"(a));
+      }
+      wq_stmatrix_trans(at + 32 * h, o[0], o[1], o[2], o[3]);
+    }
+  };
+  // the row scales (int8) of a thread's four rows 32 q + lane / 4 + 8 i
+  auto row_scales = [&](int nb, int q, float (&sc)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int64_t n = ((int64_t)nb * kRanks + rank) * 128 + 32 * q + (lane >> 2) + 8 * i;
+      sc[i] = kI8 && n < p.N_out ? __bfloat162float(p.scale8[n]) : 0.f;
+    }
+  };
+  // output tile -> y: 16-byte pieces of 256-byte rows; `threads` threads, this one is number `th`
+  auto copy_out = [&](int nb, int mt, int th, int threads) {
+    const int64_t nbase = ((int64_t)nb * kRanks + rank) * 128;
+    const int m0 = mt * NT, rows = min(NT, p.M - m0);
+    const int col = th & 15;
+    const int64_t n0 = nbase + col * 8;
+    if (n0 >= p.N_out) return;
+    __nv_bfloat16* dst = p.y + (int64_t)m0 * p.ldy + n0;
+    const uint32_t src = smem_u32(stage) + col * 16;
+    if (p.vec_store && n0 + 8 <= p.N_out) {
+#pragma unroll 4
+      for (int m = th >> 4; m < rows; m += threads >> 4) *reinterpret_cast<uint4*>(dst + m * p.ldy) = lds128(src + m * kWqPitch);
+    } else {
+      for (int m = th >> 4; m < rows; m += threads >> 4) {
+        const uint4 v = lds128(src + m * kWqPitch);
+        const uint32_t vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (n0 + e < p.N_out) dst[m * p.ldy + e] = __ushort_as_bfloat16((unsigned short)(vv[e >> 1] >> (16 * (e & 1))));
+      }
+    }
+  };
+  // share of worker c in tile t: [NT / 16 column blocks][2 halves x 2 column groups][4 quadrants][32 lanes] float4
+  auto share = [&](int c, int t) {
+    const int slot = wq_first(c, p.base, p.rem, p.quantum) / KU == t ? 0 : 1;
+    return reinterpret_cast<float4*>(p.part) + (((int64_t)c * 2 + slot) * kRanks + rank) * NT * 32;
+  };
+
+  if (warp == kWqWProd) {
+    // ---- weight producer ----
+    if (wq_elect_one()) {
+      WqRing w;
+      w.use = 1;
+      for (int u = u0 + p.w_slots; u < u1; ++u) {
+        if (!wq_wait(&wempty[w.slot], w.use ^ 1u, dead)) break;
+        load_weights(u, w.slot);
+        w.step(1, p.w_slots);
+      }
+    }
+    __syncwarp();
+  } else if (warp == kWqXProd) {
+    // ---- activation producer ----
+    grid_dependency_wait();
+    if (wq_elect_one()) {
+      WqRing x;
+      int t = u0 / KU, ku = u0 - t * KU;
+      for (int u = u0; u < u1; ++u) {
+        if (!wq_wait(DEFER ? &dread[x.slot] : &xdone[x.slot], x.use ^ 1u, dead)) break;
+        mbar_arrive_expect_tx(&xfull[x.slot], p.x_bytes);
+        bulk_g2s(xring + (size_t)x.slot * p.x_bytes, p.xt + ((int64_t)((t % p.MT) * kRanks + rank) * KU + ku) * p.x_bytes, p.x_bytes, &xfull[x.slot]);
+        x.step(1, x_slots);
+        if (++ku == KU) ku = 0, ++t;
+      }
+    }
+    __syncwarp();
+  } else if (warp >= kWqMma) {
+    const int mw = warp - kWqMma;
+    WqRing x, a, d;
+    if (PAIR && rank != 0) {
+      // ---- the pair's second CTA: tells the first one that its half of the activations has landed ----
+      for (int u = u0; u < (mw == 0 ? u1 : u0); ++u) {
+        if (!wq_wait(&xfull[x.slot], x.use, dead)) break;
+        if (wq_elect_one()) wq_arrive_leader<PAIR>(&xpeer[x.slot]);
+        __syncwarp();
+        x.step(1, x_slots);
+      }
+    } else {
+      // ---- MMA issue: 8 x (M 128 / 256, N = NT, K 16) per unit, whole warp in uniform control flow ----
+      x.step(mw, x_slots);
+      a.step(mw, a_slots);
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)NT >> 3) << 17) | (((128u * kRanks) >> 4) << 24);
+      const uint32_t chunk = (uint32_t)p.BR * 16;  // bytes between consecutive 8-k chunks of the B tile
+      const uint32_t desc_hi = (128u >> 4) | (1u << 14), kstep = (2 * chunk) >> 4;
+      const uint32_t desc_lo = ((chunk >> 4) << 16) | (smem_u32(xring) >> 4), xstep = p.x_bytes >> 4;
+      int u = u0;
+      while (u < (mw < n_mma ? u1 : u0)) {
+        const int ue = min(u1, (u / KU + 1) * KU);  // the units of this tile
+        if (!DEFER && !wq_wait(&dempty[d.slot], d.use ^ 1u, dead)) break;
+        const uint32_t dcol = tb + d.slot * 128 + mw * 64;
+        uint32_t acc = 0;
+        bool ok = true;
+        // this warp's units: those whose number in the CTA's sequence is mw (mod n_mma)
+        if (n_mma == 2 && ((u - u0) & 1) != mw) ++u;
+        for (; u < ue; u += n_mma) {
+          const bool ra = mbar_try_wait(&afull[a.slot], a.use), rx = mbar_try_wait(&xfull[x.slot], x.use);
+          ok = (ra || wq_wait(&afull[a.slot], a.use, dead)) && (rx || wq_wait(&xfull[x.slot], x.use, dead));
+          if (PAIR) ok = ok && wq_wait(&xpeer[x.slot], x.use, dead);
+          if (!ok) break;
+          wq_fence_after();
+          if (wq_elect_one()) {
+            const uint32_t b0 = desc_lo + (uint32_t)x.slot * xstep, a0 = a_col0 + a.slot * 64;
+            const uint32_t d0 = DEFER ? tb + x.slot * (kSegs * 16) : dcol;
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks) {
+              const uint64_t bdesc = ((uint64_t)desc_hi << 32) | (b0 + ks * kstep);
+              wq_mma<PAIR>(d0 + (DEFER ? ks / (8 / kSegs) * 16 : 0), a0 + 8 * ks, bdesc, idesc, DEFER ? (ks % (8 / kSegs) != 0) : (ks != 0 ? 1u : acc));
+            }
+            wq_commit<PAIR>(&adone[a.slot]);
+            wq_commit<PAIR>(&xdone[x.slot]);
+          }
+          __syncwarp();
+          acc = 1;
+          x.step(n_mma, x_slots);
+          a.step(n_mma, a_slots);
+        }
+        if (!ok) break;
+        u = ue;
+        if (!DEFER) {
+          if (wq_elect_one()) wq_commit<PAIR>(&dfull[d.slot]);
+          __syncwarp();
+          d.step(1, d_bufs);
+        }
+      }
+    }
+  } else if (warp >= kWqEpiWarps) {
+    // ---- dequant: packed words -> bf16 -> tensor memory; 8 words (int4) of one strip per warp and unit ----
+    const int dq = (warp - kWqEpiWarps) & 7, set = (warp - kWqEpiWarps) >> 3, qd = warp & 3, strip = 2 * qd + (dq >> 2);
+    const uint32_t taddr0 = a_col0 + ((uint32_t)(32 * qd + 16 * (dq >> 2)) << 16);
+    const uint32_t w0_u = smem_u32(wring) + strip * (2 * kTileB) + lane * 16;
+    const uint32_t s0_u = smem_u32(wring) + kWBytes + strip * (kSzWords * 4) + (lane >> 2) * 4;
+    WqRing w, a;
+    w.step(set, p.w_slots);
+    a.step(set, a_slots);
+    // A weight slot of an odd ring is used by the two sets in turn, and a set must not look for its phase of `wfull` before the
+    // other set's phase in between (unit u - w_slots) is over.  That unit has retired when the A slot is free, as long as w_slots >= a_slots:
+    // so with a short odd ring the A slot is waited for first.  (A longer ring cannot be overtaken while one MMA warp keeps the
+    // sets at most a_slots + 1 units apart; with two the ring is even.)
+    const bool a_first = (p.w_slots & 1) && p.w_slots < a_slots + 2;
+    for (int u = u0 + set; u < u1; u += 2) {
+      if (a_first && !wq_wait(&adone[a.slot], a.use ^ 1u, dead)) break;
+      if (!wq_wait(&wfull[w.slot], w.use, dead)) break;
+      const uint32_t wt = w0_u + w.slot * kWSlot;
+      uint32_t r[32];
+      if constexpr (kI8) {
+#pragma unroll
+        for (int q4 = 0; q4 < 4; ++q4) {  // 32-k quarters of the unit; lane chunk: words (row g, k 0-3), (g+8, k 0-3), (g, k 4-7), (g+8, k 4-7)
+          const uint4 w4 = lds128(wt + q4 * 512);
+          const uint32_t wd[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int hrow = j & 1, i0 = 2 * (j >> 1);
+            u8x4_to_bf16x2x2(wd[j], r[2 * (4 * q4 + i0) + hrow], r[2 * (4 * q4 + i0 + 1) + hrow]);
+          }
+        }
+      } else {
+        const uint4 wa = lds128(wt), wb = lds128(wt + 512);
+        const uint32_t wd[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+        uint32_t sz[DEFER ? 1 : kSzWords / 16][2];
+        if constexpr (!DEFER) {
+          const uint32_t st = s0_u + w.slot * kWSlot;
+#pragma unroll
+          for (int h = 0; h < kSzWords / 16; ++h) {
+            sz[h][0] = lds32(st + h * 64);
+            sz[h][1] = lds32(st + h * 64 + 32);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {  // word j: row g + 8 (j & 1), 32-k quarter j >> 1 of the unit
+          const int q4 = j >> 1, hrow = j & 1;
+          uint32_t o[4];
+          if constexpr (DEFER) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) asm("lop3.b32 %0, %1, 0x000f000f, 0x43004300, 0xea;" : "=r"(o[i]) : "r"(wd[j] >> (4 * i)));  // 128 + q
+          } else {
+            const uint32_t szw = sz[q4 * (kSzWords / 16) / 4][hrow];
+            dequant_word(wd[j], __byte_perm(szw, 0, 0x1010), __byte_perm(szw, 0, 0x3232), o);
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) r[2 * (4 * q4 + i) + hrow] = o[i];
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&wempty[w.slot]);  // everything that this warp reads of the slot is in registers
+      if (!wq_wait(&adone[a.slot], a.use ^ 1u, dead)) break;  // the MMAs that read this A slot have retired
+      wq_fence_after();
+      wq_st_16x128b_x8(taddr0 + a.slot * 64, r);
+      wq_st_16x128b_x8(taddr0 + a.slot * 64 + 32, r + 16);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      wq_fence_before();
+      __syncwarp();
+      if (lane == 0) wq_arrive_leader<PAIR>(&afull[a.slot]);
+      w.step(2, p.w_slots);
+      a.step(2, a_slots);
+    }
+  } else {
+    // ---- epilogue ----
+    grid_dependency_wait();
+    const uint32_t lane_col = tb + ((uint32_t)(32 * warp) << 16);
+    WqRing d, x, w;
+    bool ok = true;
+    for (int u = u0, t = u0 / KU; u < u1; ++t) {
+      const int ue = min(u1, (t + 1) * KU), nb = t / p.MT, mt = t - nb * p.MT;
+      const bool whole = u == t * KU && ue == (t + 1) * KU;
+      float4* mine = share(worker, t) + warp * 32 + lane;
+      float sc[4];
+      row_scales(nb, warp, sc);
+      if (whole) wq_epi_sync(false);  // the previous output tile has been copied out
+      if constexpr (DEFER) {
+        float acc[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+        for (; u < ue; ++u) {
+          ok = wq_wait(&wfull[w.slot], w.use, dead) && wq_wait(&xfull[x.slot], x.use, dead) && wq_wait(&xdone[x.slot], x.use, dead);
+          if (!ok) break;
+          wq_fence_after();
+          // parameters of rows 32 warp + lane / 4 + 8 i, sums of columns 2 (lane % 4) + {0, 1, 8, 9}
+          const uint32_t st = smem_u32(wring) + w.slot * kWSlot + kWBytes + 2 * warp * (kSzWords * 4) + (lane >> 2) * 4;
+          const uint32_t xs = smem_u32(xring) + (uint32_t)x.slot * p.x_bytes + 16 * 256 + (lane & 3) * 8;
+#pragma unroll
+          for (int sg = 0; sg < kSegs; ++sg) {
+            uint32_t v[16];
+            wq_ld_16x256b_x2(lane_col + (x.slot * kSegs + sg) * 16, v);
+            wq_ld_16x256b_x2(lane_col + (16u << 16) + (x.slot * kSegs + sg) * 16, v + 8);
+            float s[4], zt[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t szw = lds32(st + (i >> 1) * (kSzWords * 4) + sg * 64 + (i & 1) * 32);
+              s[i] = __uint_as_float(szw << 16);
+              zt[i] = fmaf(-136.f, s[i], __uint_as_float(szw & 0xFFFF0000u));
+            }
+            const float2 xa = lds64f(xs + sg * 64), xb = lds64f(xs + sg * 64 + 32);
+            const float X[4] = {xa.x, xa.y, xb.x, xb.y};
+            wq_ld_wait();
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {  // e: column group e >> 2, row group (e >> 1) & 1, column e & 1
+                const int r = 2 * h + ((e >> 1) & 1), c = 2 * (e >> 2) + (e & 1);
+                acc[8 * h + e] = fmaf(s[r], __uint_as_float(v[8 * h + e]), fmaf(zt[r], X[c], acc[8 * h + e]));
+              }
+          }
+          wq_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(&dread[x.slot]);
+            mbar_arrive(&wempty[w.slot]);
+          }
+          x.step(1, x_slots);
+          w.step(1, p.w_slots);
+        }
+        if (whole) {
+          to_stage(warp, 0, acc, sc);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) __stcg(mine + i * 128, make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]));
+        }
+      } else {
+        ok = wq_wait(&dfull[d.slot], d.use, dead);
+        wq_fence_after();
+        // which accumulators hold something: both MMA warps', unless the tile has one unit here
+        const bool two = n_mma == 2 && ue - u > 1;
+        const uint32_t dcol = lane_col + d.slot * 128 + (n_mma == 2 && ue - u == 1 ? ((u - u0) & 1) * 64 : 0);
+#pragma unroll 1
+        for (int c = 0; c < NT; c += 16) {
+          uint32_t v[16];
+          float f[16];
+          wq_ld_16x256b_x2(dcol + c, v);
+          wq_ld_16x256b_x2(dcol + (16u << 16) + c, v + 8);
+          if (two) {
+            uint32_t v2[16];
+            wq_ld_16x256b_x2(dcol + 64 + c, v2);
+            wq_ld_16x256b_x2(dcol + (16u << 16) + 64 + c, v2 + 8);
+            wq_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]) + __uint_as_float(v2[i]);
+          } else {
+            wq_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
+          }
+          if (c + 16 >= NT) {
+            wq_fence_before();
+            __syncwarp();
+            if (lane == 0) wq_arrive_leader<PAIR>(&dempty[d.slot]);
+          }
+          if (whole) {
+            to_stage(warp, c, f, sc);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) __stcg(mine + (c / 4 + i) * 128, make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]));
+          }
+        }
+        d.step(1, d_bufs);
+        u = ue;
+      }
+      if (!whole) __threadfence();
+      if (wq_epi_sync(!ok)) break;
+      if (whole) {
+        copy_out(nb, mt, threadIdx.x, kWqEpiWarps * 32);
+      } else if (threadIdx.x == 0) {
+        // a tile shared with neighbours: whoever arrives last adds all shares (below)
+        const int c0 = wq_owner(t * KU, p.base, p.rem, p.quantum), c1 = wq_owner(t * KU + KU - 1, p.base, p.rem, p.quantum);
+        if (atomicAdd(&p.tickets[t * kRanks + rank], 1u) == (uint32_t)(c1 - c0)) s_last[t == u0 / KU ? 0 : 1] = 1;
+      }
+    }
+  }
+
+  // ---- shared tiles that this CTA was the last to reach: all warps add the shares in CTA order and finish the rows ----
+  __syncthreads();
+#pragma unroll 1
+  for (int k = 0; k < 2; ++k) {
+    if (s_last[k] == 0) continue;
+    __threadfence();
+    const int t = k == 0 ? u0 / KU : (u1 - 1) / KU, nb = t / p.MT, mt = t - nb * p.MT;
+    const int c0 = wq_owner(t * KU, p.base, p.rem, p.quantum), c1 = wq_owner(t * KU + KU - 1, p.base, p.rem, p.quantum);
+    for (int it = warp; it < NT / 4; it += kWqThreads / 32) {  // (column block, quadrant)
+      const int q = it & 3, c = (it >> 2) * 16;
+      float f[16], sc[4];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) f[i] = 0.f;
+      row_scales(nb, q, sc);
+#pragma unroll 2
+      for (int cc = c0; cc <= c1; ++cc) {
+        const float4* src = share(cc, t) + (c / 4) * 128 + q * 32 + lane;
+        float4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = __ldcg(src + i * 128);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) f[4 * i] += v[i].x, f[4 * i + 1] += v[i].y, f[4 * i + 2] += v[i].z, f[4 * i + 3] += v[i].w;
+      }
+      to_stage(q, c, f, sc);
+    }
+    __syncthreads();
+    copy_out(nb, mt, threadIdx.x, kWqThreads);
+    __syncthreads();
+  }
+
+  // ---- teardown: nobody touches tensor memory any more ----
+  if (*dead != 0) {
+    if (threadIdx.x == 0) atomicExch(p.status, 1u);
+    for (int i = 0; i < 64; ++i) __nanosleep(100000);  // copies and MMAs of this CTA that are still in flight
+  }
+  wq_fence_before();
+  __syncthreads();
+  if constexpr (PAIR) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (warp == kWqMma) {
+    wq_fence_after();
+    if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tb), "r"(512));
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tb), "r"(512));
+  }
+}
+
+// ---- host ---------------------------------------------------------------------------------------------------------------
+static int wq_sm_count() {
+  static int n = 0;
+  if (n == 0) {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    n = v > 0 ? v : kNumSMs;
+  }
+  return n;
+}
+
+// how one call is cut up; a pure function of the shape, so the workspace size is too
+struct WqPlan {
+  bool defer, pair;
+  int NT, BR, MT, NB, KU, ranks, workers, quantum, base, rem;
+  int64_t tiles, n_tickets;
+  uint32_t x_bytes;
+  int64_t off_part, off_xt, bytes;  // [status, tickets][shares][staged activations]
+};
+
+static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
+  if (M <= 0 || Np % 128 != 0 || Kp % 64 != 0 || M > ((int64_t)1 << 22)) return false;
+  w.defer = int4 && M <= 16;
+  w.pair = M > 32;
+  w.ranks = w.pair ? 2 : 1;
+  w.MT = (int)((M + 255) / 256);
+  w.NT = (int)(((M + w.MT - 1) / w.MT + 15) / 16 * 16);
+  w.BR = w.NT / w.ranks;
+  w.KU = (int)((Kp + 127) / 128);
+  w.NB = (int)((Np + 128 * w.ranks - 1) / (128 * w.ranks));
+  w.tiles = (int64_t)w.NB * w.MT;
+  if (w.tiles * w.KU > 2000000000) return false;
+  const int sms = wq_sm_count() / w.ranks;
+  w.quantum = w.tiles >= (int64_t)kWqMaxSplitTiles * sms ? w.KU : 1;
+  const int64_t parts = w.tiles * w.KU / w.quantum;
+  w.workers = (int)(w.quantum > 1 ? sms : (parts / 2 < sms ? (parts + 1) / 2 : sms));
+  w.base = (int)(parts / w.workers);
+  w.rem = (int)(parts % w.workers);
+  w.n_tickets = w.quantum > 1 ? 0 : w.tiles * w.ranks;
+  w.x_bytes = (uint32_t)w.BR * 256 + (w.defer ? 4 * 64 : 0);  // (the sums' space is that of the smallest group)
+  auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
+  w.off_part = up(256 + w.n_tickets * 4);
+  w.off_xt = w.off_part + (w.quantum > 1 ? 0 : up((int64_t)w.workers * 2 * w.ranks * w.NT * 512));
+  w.bytes = w.off_xt + up((int64_t)w.MT * w.ranks * w.KU * w.x_bytes);
+  return true;
+}
+
+using WqEncode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                              CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static WqEncode wq_encode_fn() {
+  static WqEncode fn = []() -> WqEncode {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) return nullptr;
+    return reinterpret_cast<WqEncode>(p);
+  }();
+  return fn;
+}
+// rows of `row_bytes`, read in boxes of 8 rows x box elements
+static bool wq_map(CUtensorMap* map, CUtensorMapDataType type, int elem, const void* base, int64_t row_bytes, int64_t rows, int box) {
+  const cuuint64_t dims[2] = {(cuuint64_t)(row_bytes / elem), (cuuint64_t)rows}, strides[1] = {(cuuint64_t)row_bytes};
+  const cuuint32_t boxes[2] = {(cuuint32_t)box, 8}, steps[2] = {1, 1};
+  return wq_encode_fn()(map, type, 2, const_cast<void*>(base), dims, strides, boxes, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int G, bool DEFER, bool PAIR>
+static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
+  constexpr uint32_t kWSlot = 8 * 2 * (G == 0 ? 1024 : 512) + (G == 0 ? 0 : 8 * (G < 128 ? 128 / (G ? G : 128) : 1) * 64);
+  constexpr size_t kBudget = 226 * 1024;
+  p.n_mma = w.NT <= 64 ? 2 : 1;
+  // tiles of x in flight (an L2 round trip is about 850 clocks; DEFER: as many as there are accumulators); what they and the
+  // output tile leave of shared memory holds weights in flight
+  p.x_slots = w.x_bytes > 24 * 1024 ? 3 : (w.x_bytes > 12 * 1024 ? 5 : (DEFER && G == 32 ? 4 : 8));  // even where two MMA warps alternate
+  const size_t off_w = (kWqHeader + (size_t)w.NT * kWqPitch + (size_t)p.x_slots * w.x_bytes + 127) / 128 * 128;
+  p.off_w = (uint32_t)off_w;
+  p.w_slots = (int)((kBudget - off_w) / kWSlot);
+  if (p.w_slots > kWqMaxW) p.w_slots = kWqMaxW;
+  if (p.n_mma == 2) p.w_slots &= ~1;           // two MMA warps let the two dequant sets drift apart: each set keeps slots of its own
+  p.a_slots = p.w_slots == 3 ? 3 : kWqSlots;   // (see a_first in the kernel)
+  const size_t smem = off_w + (size_t)p.w_slots * kWSlot;
+  auto kern = wq_gemm_kernel<G, DEFER, PAIR>;
+  static bool attr_done = false;
+  if (!attr_done) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBudget) != cudaSuccess) return AO_B200_ERR_CUDA;
+    attr_done = true;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(w.workers * w.ranks));
+  cfg.blockDim = dim3(kWqThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 2;
+  at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = PAIR ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, p) == cudaSuccess ? AO_B200_OK : AO_B200_ERR_CUDA;
+}
+
+template <int SEG>
+static int wq_stage(const void* x, int64_t M, int64_t Kx, int64_t ldx, const WqPlan& w, uint8_t* xt, uint32_t* tickets, cudaStream_t s) {
+  const int n_blocks = w.MT * w.ranks;
+  const int64_t warps = (int64_t)n_blocks * (w.BR / 8) * w.KU;
+  int64_t grid = (warps + 7) / 8;
+  if (grid > 148 * 16) grid = 148 * 16;
+  if (grid * 256 < w.n_tickets) grid = (w.n_tickets + 255) / 256;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, stage_x_kernel<SEG>, static_cast<const __nv_bfloat16*>(x), M, Kx, ldx, n_blocks, w.BR, w.KU, w.x_bytes, xt, tickets,
+                            (int)w.n_tickets) == cudaSuccess
+             ? AO_B200_OK
+             : AO_B200_ERR_CUDA;
+}
+
+// x [M][ldx] bf16 (first Kx columns valid), y [M][ldy] bf16.  G == 0: int8 weights (`sz` is then the bf16 per-row scale)
+static int wq_gemm(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np, int64_t Kp, int G, void* y,
+                   int64_t N_out, int64_t ldy, void* workspace, int64_t workspace_bytes, cudaStream_t s) {
+  WqPlan w;
+  if (!wq_plan(M, Np, Kp, G != 0, w) || wq_encode_fn() == nullptr) return AO_B200_ERR_UNSUPPORTED;
+  if (workspace == nullptr || workspace_bytes < w.bytes || !ao_aligned(workspace, 16)) return AO_B200_ERR_WORKSPACE;
+  auto* ws = static_cast<uint8_t*>(workspace);
+  WqParams p;
+  const bool ok = G ? wq_map(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, packed, Kp * 8, Np / 16, 256) &&
+                          wq_map(&p.smap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, sz, Kp / G * 64, Np / 16, (G < 128 ? 128 / G : 1) * 16)
+                    : wq_map(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_INT64, 8, packed, Kp * 16, Np / 16, 256);
+  if (!ok) return AO_B200_ERR_UNSUPPORTED;
+  p.status = reinterpret_cast<uint32_t*>(ws);
+  p.tickets = reinterpret_cast<uint32_t*>(ws + 256);
+  p.part = reinterpret_cast<float*>(ws + w.off_part);
+  p.xt = ws + w.off_xt;
+  p.scale8 = G ? nullptr : static_cast<const __nv_bfloat16*>(sz);
+  p.y = static_cast<__nv_bfloat16*>(y);
+  p.N_out = N_out;
+  p.ldy = ldy;
+  p.vec_store = (ldy % 8 == 0 && ao_aligned(y, 16)) ? 1 : 0;
+  p.M = (int)M;
+  p.NT = w.NT;
+  p.BR = w.BR;
+  p.KU = w.KU;
+  p.MT = w.MT;
+  p.x_bytes = w.x_bytes;
+  p.quantum = w.quantum;
+  p.base = w.base;
+  p.rem = w.rem;
+  int rc;
+  if (!w.defer) rc = wq_stage<0>(x, M, Kx, ldx, w, ws + w.off_xt, p.tickets, s);
+  else if (G == 32) rc = wq_stage<32>(x, M, Kx, ldx, w, ws + w.off_xt, p.tickets, s);
+  else if (G == 64) rc = wq_stage<64>(x, M, Kx, ldx, w, ws + w.off_xt, p.tickets, s);
+  else rc = wq_stage<128>(x, M, Kx, ldx, w, ws + w.off_xt, p.tickets, s);
+  if (rc != AO_B200_OK) return rc;
+  switch (G) {
+    case 0: return w.pair ? wq_launch<0, false, true>(p, w, s) : wq_launch<0, false, false>(p, w, s);
+#define AO_WQ(GG) \
+  case GG: return w.defer ? wq_launch<GG, true, false>(p, w, s) : (w.pair ? wq_launch<GG, false, true>(p, w, s) : wq_launch<GG, false, false>(p, w, s));
+    AO_WQ(32)
+    AO_WQ(64)
+    AO_WQ(128)
+    AO_WQ(256)
+#undef AO_WQ
+  }
+  return AO_B200_ERR_UNSUPPORTED;
+}
+
+// bytes of the workspace for M rows (0: shape not handled by this kernel).  Its contents need not survive between calls.
+int64_t int4_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp) {
+  WqPlan w;
+  return wq_plan(M, Np, Kp, true, w) ? w.bytes : 0;
+}
+int64_t int8_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp) {
+  WqPlan w;
+  return wq_plan(M, Np, Kp, false, w) ? w.bytes : 0;
+}
+
+int int4_gemm_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np, int64_t Kp, int G, void* y,
+                 int64_t N_out, int64_t ldy, void* workspace, int64_t workspace_bytes, cudaStream_t s) {
+  if (!(G == 32 || G == 64 || G == 128 || G == 256)) return AO_B200_ERR_UNSUPPORTED;
+  return wq_gemm(x, M, Kx, ldx, packed, sz, Np, Kp, G, y, N_out, ldy, workspace, workspace_bytes, s);
+}
+
+// int8 weights: packed = strip-major biased int8 (Np % 128 == 0), scale bf16 [N_out]
+int int8_gemm_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Np, int64_t Kp, void* y, int64_t N_out,
+                 int64_t ldy, void* workspace, int64_t workspace_bytes, cudaStream_t s) {
+  return wq_gemm(x, M, Kx, ldx, packed, scale, Np, Kp, 0, y, N_out, ldy, workspace, workspace_bytes, s);
+}
+
+}  // namespace ao
