@@ -180,6 +180,13 @@ AO_B200_API int ao_b200_hqq_solve(const void* w, int64_t n_groups, int group_siz
                                   void* stream);
 AO_B200_API int ao_b200_hqq_finalize(const void* w, int64_t n_groups, int group_size, const float* scale, const float* zero,
                                      int32_t* q, void* scale_out, void* zero_out, void* stream);
+/* Everything above in one call with the same results, w bf16 [N][K] contiguous, 16-byte aligned: the search (iters <= 64), then q / scale_out / zero_out as ao_b200_hqq_finalize writes them, or, with
+ * q = NULL, the strip-major storage packed [Np/16][Kp/64][32][4] and scale_and_zero [Np/16][Kp/G][16][2], padding zero.
+ * workspace: ao_b200_hqq_search_workspace_bytes, 8-byte aligned. */
+AO_B200_API int64_t ao_b200_hqq_search_workspace_bytes(int64_t n_groups, int group_size);
+AO_B200_API int ao_b200_hqq_search(const void* w, int64_t N, int64_t K, int group_size, double beta, double kappa, double lp_norm,
+                                   int iters, void* workspace, int64_t workspace_bytes, int32_t* q, void* scale_out, void* zero_out,
+                                   int64_t Np, int64_t Kp, void* packed, void* scale_and_zero, void* stream);
 
 /* strip-major int8 layout (this library's format): uint8 [Np/16][Kp/64][2][32][16], BIASED bytes u = q + 128.
  *   strip s (16 rows) x k-tile kt (64 k) = 1024 contiguous bytes = two 32-k halves of 512 bytes; inside a half lane

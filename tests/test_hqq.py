@@ -127,3 +127,38 @@ def test_hqq_device_side_early_stop_equals_the_host_driven_loop(shape, gs):
     assert int(flags[0]) == (1 if ran < HQQ_ITERS else int(flags[0]))
     assert torch.equal(zero_d, zero_h) and torch.equal(scale_d, scale_h)
     assert abs(float(state[0]) - best) <= 1e-12 * max(best, 1.0)
+
+
+@pytest.mark.parametrize("shape,gs", [((4096, 512), 64), ((33, 256), 32), ((130, 448), 64), ((40, 768), 256), ((1, 128), 128)])
+@pytest.mark.parametrize("spread", [0.02, 1.0, 30.0])
+def test_hqq_search_equals_the_iterations_one_by_one(shape, gs, spread):
+    """ao_b200_hqq_search (a group's iterations in registers, the shrinkage evaluated only where it can be positive, Markstein's
+    division) against init / solve / finalize, bit for bit: it adds in the same order.  Spreads from where the shrinkage is always
+    zero to where it seldom is.  The packed form is the plain one packed, padding zero."""
+    from torchao_fork_b200 import _lib
+    from torchao_fork_b200 import ops as aops
+    torch.manual_seed(7)
+    n, k = shape
+    w = (spread * torch.randn(*shape, device="cuda") * torch.exp(0.3 * torch.randn(n, 1, device="cuda"))).to(torch.bfloat16)
+    w[0, :gs] = 0.25
+    L, st, n_groups = _lib.lib(), torch.cuda.current_stream().cuda_stream, n * k // gs
+    scale = torch.empty(n_groups, dtype=torch.float32, device="cuda")
+    zero, err = torch.empty_like(scale), torch.empty(int(L.ao_b200_hqq_blocks(n_groups)), dtype=torch.float32, device="cuda")
+    state = torch.empty(2, dtype=torch.float64, device="cuda")
+    q0 = torch.empty(n, k, dtype=torch.int32, device="cuda")
+    s0 = torch.empty(n, k // gs, dtype=torch.bfloat16, device="cuda")
+    z0 = torch.empty_like(s0)
+    _lib.check(L.ao_b200_hqq_init(w.data_ptr(), n_groups, gs, scale.data_ptr(), zero.data_ptr(), st), "init")
+    _lib.check(L.ao_b200_hqq_solve(w.data_ptr(), n_groups, gs, scale.data_ptr(), zero.data_ptr(), aops.HQQ_BETA, aops.HQQ_KAPPA, aops.HQQ_LP_NORM,
+                                   aops.HQQ_ITERS, err.data_ptr(), state.data_ptr(), st), "solve")
+    _lib.check(L.ao_b200_hqq_finalize(w.data_ptr(), n_groups, gs, scale.data_ptr(), zero.data_ptr(), q0.data_ptr(), s0.data_ptr(), z0.data_ptr(), st),
+               "finalize")
+    q, s, z = T.b200_int4_hqq_quantize(w, gs)
+    assert torch.equal(s, s0) and torch.equal(z, z0) and torch.equal(q, q0)
+    packed, sz = T.b200_int4_hqq_quantize_pack(w, gs)
+    pad = torch.zeros(packed.shape[0] * 16, packed.shape[1] * 64, dtype=torch.int32, device="cuda")
+    pad[:n, :k] = q
+    assert torch.equal(T.b200_int4_unpack(packed), pad)
+    ps, pz = aops.unpack_scales_and_zeros_b200(sz)
+    assert torch.equal(ps[:n, : k // gs], s) and torch.equal(pz[:n, : k // gs], z)
+    assert not ps[n:].any() and not pz[n:].any() and not ps[:, k // gs :].any()

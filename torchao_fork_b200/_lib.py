@@ -56,6 +56,9 @@ SIGNATURES = {
     "ao_b200_hqq_init": [_vp, _i64, _i32, _vp, _vp, _vp],
     "ao_b200_hqq_step": [_vp, _i64, _i32, _vp, _vp, ctypes.c_double, ctypes.c_double, _vp, _vp],
     "ao_b200_hqq_solve": [_vp, _i64, _i32, _vp, _vp, ctypes.c_double, ctypes.c_double, ctypes.c_double, _i32, _vp, _vp, _vp],
+    "ao_b200_hqq_search_workspace_bytes": [_i64, _i32],
+    "ao_b200_hqq_search": [_vp, _i64, _i64, _i32, ctypes.c_double, ctypes.c_double, ctypes.c_double, _i32, _vp, _i64, _vp, _vp, _vp,
+                           _i64, _i64, _vp, _vp, _vp],
     "ao_b200_hqq_finalize": [_vp, _i64, _i32, _vp, _vp, _vp, _vp, _vp, _vp],
     "ao_b200_int8_mm": [_vp, _i64, _i64, _i64, _vp, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _i64, _vp],
     "ao_b200_int8_gemv_fused": [_vp, _i64, _i64, _i64, _vp, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _f32, _vp, _i64, _i32,
@@ -87,7 +90,7 @@ SIGNATURES = {
     "ao_b200_decode_mega_step": [_mp, _vp, _vp],
 }
 _RESTYPES = {"ao_b200_error_string": ctypes.c_char_p, "ao_b200_int4_mm_workspace_bytes": _i64,
-             "ao_b200_int8_mm_workspace_bytes": _i64, "ao_b200_hqq_blocks": _i64,
+             "ao_b200_int8_mm_workspace_bytes": _i64, "ao_b200_hqq_blocks": _i64, "ao_b200_hqq_search_workspace_bytes": _i64,
              "ao_b200_decode_attention_workspace_bytes": _i64,
              "ao_b200_decode_attention_fused_workspace_bytes": _i64, "ao_b200_tp_buffer_bytes": _i64,
              "ao_b200_decode_mega_plan_bytes": _i64, "ao_b200_decode_mega_xchg_bytes": _i64,

@@ -122,7 +122,229 @@ __global__ void __launch_bounds__(kHqqWarps * 32) hqq_finalize_kernel(const __nv
   }
 }
 
+// ---- the whole search: chunks of iterations with the group in registers --------------------------------------------------
+// The iterations of a group depend on no other group; only the early stop looks at all of them.  So a thread keeps 16
+// weights of a group in registers through kHqqChunk iterations and leaves behind the zero point after each of them (`hist`)
+// and the block's error of each (`err`); hqq_mean_kernel adds the errors up, and whoever comes next works out
+// from the means which iteration was the last (hqq_last), so that iterations past the stop cost work but change nothing.
+//
+// Bound by instruction issue: 14 instructions per weight and iteration.  Two things keep it there.  The shrinkage
+// |d| - c |d|^(p - 1) is not positive for |d| <= c^(1 / (2 - p)) (p < 1), 0.17 at the reference's constants, which is above most
+// weights' error: powf runs only above that threshold (less a margin of 1e-3, thousands of times powf's error).  And (q - z) / s
+// is x = n r, r = rn(1 / s), corrected once, x + r (n - x s): the correctly rounded quotient by Markstein's theorem (IBM J. Res.
+// Dev. 34, 1990), as neither r nor the remainder leaves the normal range (s in [2e-38, 2e4], |n| >= 2^-24 or 0).
+// Same numbers as hqq_step_kernel, bit for bit: there lane l of 32 adds elements l + 32 j and the lanes meet in steps of 16, 8, 4, 2, 1;
+// here thread r of L = G / 16 holds the elements of the lanes r, r + L, .. of it, so the first steps of that tree are its own.
+// quantize_ of 4096 x 4096, groups of 64, 20 iterations: 375 us against 1901 us of 20 steps and judges with a separate packing.
+constexpr int kHqqChunk = 10;   // iterations per launch: bounds hist to 10 numbers per group
+constexpr int kHqqMaxIters = 64;
+constexpr int kHqqPer = 16;     // weights per thread
+
+struct HqqChunk {
+  float inv_beta[kHqqChunk], threshold[kHqqChunk];
+  float lp_m1;
+  int first, count;             // iterations [first, first + count)
+};
+
+// number of the last iteration among the first n whose means are known: the first one that does not improve, else n - 1
+__device__ __forceinline__ int hqq_last(const double* __restrict__ mean, int n, bool& stopped) {
+  double best = 1e4;            // (:1956)
+  for (int i = 0; i < n; ++i) {
+    if (!(mean[i] < best)) {
+      stopped = true;
+      return i;
+    }
+    best = mean[i];
+  }
+  stopped = false;
+  return n - 1;
+}
+
+// sign(d) relu(|d| - c |d|^(p - 1)); out of line: sixteen inlined powf would not fit the instruction caches
+__device__ __noinline__ float hqq_shrink(float d, float c, float lp_m1) {
+  const float ad = fabsf(d);
+  return copysignf(fmaxf(__fsub_rn(ad, __fmul_rn(c, powf(ad, lp_m1))), 0.f), d);
+}
+
+template <int G>
+__global__ void __launch_bounds__(256) hqq_iterate_kernel(const __nv_bfloat16* __restrict__ w, int64_t n_groups, HqqChunk ch, float* __restrict__ scale,
+                                                          float* __restrict__ hist, double* __restrict__ err, const double* __restrict__ mean) {
+  constexpr int L = G / kHqqPer, I = 32 / L, J = G / 32;   // threads per group; its lanes per thread; elements per lane
+  constexpr int kGroups = 256 / L;                         // groups per block
+  constexpr float kMagic = 12582912.f;                     // 1.5 * 2^23: adding and subtracting it is rint up to 2^22, and beyond that the clamp decides
+  __shared__ float s_err[kHqqChunk][kGroups];
+  bool stopped = false;
+  if (ch.first > 0) hqq_last(mean, ch.first, stopped);
+  if (stopped) return;
+  const int64_t group = ((int64_t)blockIdx.x * 256 + threadIdx.x) / L;
+  const bool in = group < n_groups, first = threadIdx.x % L == 0;
+  const __nv_bfloat16* wp = w + group * G + threadIdx.x % L;
+  float v[kHqqPer], t[kHqqPer];    // element j I + i: weight i L + 32 j of the thread's
+#pragma unroll
+  for (int j = 0; j < J; ++j)
+#pragma unroll
+    for (int i = 0; i < I; ++i) v[j * I + i] = in ? __bfloat162float(wp[32 * j + L * i]) : 0.f;
+  // sum over the group in the order of 32 lanes with J elements each
+  auto group_sum = [&](float (&x)[kHqqPer]) {
+#pragma unroll
+    for (int j = 1; j < J; ++j)
+#pragma unroll
+      for (int i = 0; i < I; ++i) x[i] += x[j * I + i];
+#pragma unroll
+    for (int o = I / 2; o; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < o; ++i) x[i] += x[i + o];
+    float r = x[0];
+#pragma unroll
+    for (int o = L / 2; o; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    return r;
+  };
+  float s, z;
+  if (ch.first == 0) {             // (:2052-2060), as in hqq_init_kernel
+    float mn = v[0], mx = v[0];
+#pragma unroll
+    for (int j = 1; j < kHqqPer; ++j) mn = fminf(mn, v[j]), mx = fmaxf(mx, v[j]);
+#pragma unroll
+    for (int o = L / 2; o; o >>= 1) {
+      mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    s = fminf(__fdiv_rn(15.f, __fsub_rn(mx, mn)), 2e4f);
+    z = rintf(__fmul_rn(-mn, s));
+    if (in && first) scale[group] = s;
+  } else {
+    s = in ? scale[group] : 1.f;
+    z = in ? hist[(int64_t)(kHqqChunk - 1) * n_groups + group] : 0.f;
+  }
+  const float r = __frcp_rn(s);
+#pragma unroll
+  for (int j = 0; j < kHqqPer; ++j) t[j] = __fmul_rn(v[j], s);
+#pragma unroll 1
+  for (int it = 0; it < ch.count; ++it) {
+    const float c = ch.inv_beta[it], thr = ch.threshold[it];
+    float acc[kHqqPer], e[kHqqPer];
+#pragma unroll
+    for (int j = 0; j < kHqqPer; ++j) {
+      const float wq = fminf(fmaxf(__fsub_rn(__fadd_rn(__fadd_rn(t[j], z), kMagic), kMagic), 0.f), 15.f);
+      const float n = __fsub_rn(wq, z), x = __fmul_rn(n, r);
+      const float wr = __fmaf_rn(__fmaf_rn(-x, s, n), r, x);
+      const float d = __fsub_rn(v[j], wr), ad = fabsf(d);
+      float u = t[j];              // (W - W_e) * scale
+      if (ad > thr) u = __fmul_rn(__fsub_rn(v[j], hqq_shrink(d, c, ch.lp_m1)), s);
+      acc[j] = __fsub_rn(wq, u);
+      e[j] = ad;
+    }
+    z = __fdiv_rn(group_sum(acc), (float)G);
+    const float es = group_sum(e);
+    if (first) {
+      if (in) hist[(int64_t)it * n_groups + group] = z;
+      s_err[it][threadIdx.x / L] = in ? es : 0.f;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < ch.count) {    // eight groups at a time in fp32, as the blocks of hqq_step_kernel; fixed order: the stop is reproducible
+    double sum = 0.0;
+    for (int b = 0; b < kGroups; b += 8) {
+      float f = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f += s_err[threadIdx.x][b + i];
+      sum += (double)f;
+    }
+    err[(int64_t)threadIdx.x * gridDim.x + blockIdx.x] = sum;
+  }
+}
+
+// block i: mean[first + i] = sum of err[i][..] / numel, in double, fixed order
+__global__ void __launch_bounds__(1024) hqq_mean_kernel(const double* __restrict__ err, int64_t n_blocks, double inv_numel, int first, double* __restrict__ mean) {
+  __shared__ double s_sum[1024];
+  bool stopped = false;
+  if (first > 0) hqq_last(mean, first, stopped);
+  if (stopped) return;
+  const double* e = err + blockIdx.x * n_blocks;
+  double t = 0.0;
+  for (int64_t i = threadIdx.x; i < n_blocks; i += 1024) t += e[i];
+  s_sum[threadIdx.x] = t;
+  __syncthreads();
+  for (int o = 512; o; o >>= 1) {
+    if ((int)threadIdx.x < o) s_sum[threadIdx.x] += s_sum[threadIdx.x + o];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) mean[first + blockIdx.x] = s_sum[0] * inv_numel;
+}
+
+// the zero points of the last iteration that ran
+__device__ __forceinline__ const float* hqq_zero(const float* hist, int64_t n_groups, const double* mean, int iters) {
+  bool stopped;
+  return hist + (int64_t)(hqq_last(mean, iters, stopped) % kHqqChunk) * n_groups;
+}
+
+template <int G>
+__global__ void __launch_bounds__(kHqqWarps * 32) hqq_plain_kernel(const __nv_bfloat16* __restrict__ w, int64_t n_groups, const float* __restrict__ scale,
+                                                                   const float* __restrict__ hist, const double* __restrict__ mean, int iters,
+                                                                   int32_t* __restrict__ q, __nv_bfloat16* __restrict__ scale_out,
+                                                                   __nv_bfloat16* __restrict__ zero_out) {
+  const float* zero = hqq_zero(hist, n_groups, mean, iters);
+  const int lane = threadIdx.x & 31;
+  const int64_t group = (int64_t)blockIdx.x * kHqqWarps + (threadIdx.x >> 5);
+  if (group >= n_groups) return;
+  float v[G / 32];
+  load_group<G>(w, group, lane, v);
+  const float s = scale[group], z = zero[group];
+  int32_t* qp = q + group * G + lane;
+#pragma unroll
+  for (int j = 0; j < G / 32; ++j) qp[32 * j] = (int32_t)fminf(fmaxf(rintf(__fadd_rn(__fmul_rn(v[j], s), z)), 0.f), 15.f);
+  if (lane == 0) {
+    const float si = __fdiv_rn(1.f, s);
+    scale_out[group] = __float2bfloat16_rn(si);
+    zero_out[group] = __float2bfloat16_rn(__fmul_rn(__fsub_rn(8.f, z), si));
+  }
+}
+
+// the same straight into the strip-major storage (include/ao_b200.h): thread = 16-byte lane chunk of a (16-row strip, 64-k tile), then
+// one thread per (row, group) of the parameters; padding rows and columns are zero in both.  Bound by HBM: weights in, words out.
+__global__ void __launch_bounds__(256) hqq_packed_kernel(const __nv_bfloat16* __restrict__ w, int64_t N, int64_t K, int64_t Np, int64_t Kp, int G,
+                                                         const float* __restrict__ scale, const float* __restrict__ hist, const double* __restrict__ mean,
+                                                         int iters, uint4* __restrict__ packed, uint32_t* __restrict__ sz) {
+  const int64_t groups = K / G, groups_p = Kp / G;
+  const float* zero = hqq_zero(hist, N * groups, mean, iters);
+  const int64_t chunks = (Np / 16) * (Kp / 64) * 32, total = chunks + Np * groups_p;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    if (i >= chunks) {
+      const int64_t o = i - chunks, row = (o / (groups_p * 16)) * 16 + (o & 15), grp = (o >> 4) % groups_p;
+      uint32_t word = 0;
+      if (row < N && grp < groups) {
+        const float s = scale[row * groups + grp], si = __fdiv_rn(1.f, s);
+        word = float_to_bf16_bits(si) | (float_to_bf16_bits(__fmul_rn(__fsub_rn(8.f, zero[row * groups + grp]), si)) << 16);
+      }
+      sz[o] = word;
+      continue;
+    }
+    const int lane = i & 31, g = lane >> 2, c = lane & 3;
+    int64_t strip, kt;
+    tile_of_slot(i >> 5, Kp / 64, strip, kt);
+    uint32_t words[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int64_t row = strip * 16 + g + 8 * (j & 1), k0 = kt * 64 + 32 * (j >> 1) + 8 * c;
+      uint32_t word = 0;
+      if (row < N && k0 < K) {
+        const int64_t grp = row * groups + k0 / G;
+        const float s = scale[grp], z = zero[grp];
+        float f[8];
+        unpack8(ldg128(w + row * K + k0), f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          word |= (uint32_t)fminf(fmaxf(rintf(__fadd_rn(__fmul_rn(f[e], s), z)), 0.f), 15.f) << (4 * nib_slot(e));
+      }
+      words[j] = word;
+    }
+    packed[i] = make_uint4(words[0], words[1], words[2], words[3]);
+  }
+}
+
 }  // namespace ao
+
+#include <cmath>
 
 using namespace ao;
 
@@ -213,5 +435,63 @@ extern "C" int ao_b200_hqq_finalize(const void* w, int64_t n_groups, int group_s
   const unsigned grid = (unsigned)ao_b200_hqq_blocks(n_groups);
   AO_HQQ_DISPATCH(hqq_finalize_kernel, static_cast<const __nv_bfloat16*>(w), n_groups, scale, zero, q,
                   static_cast<__nv_bfloat16*>(scale_out), static_cast<__nv_bfloat16*>(zero_out));
+  return ao_launch_status();
+}
+
+static int64_t hqq_search_blocks(int64_t n_groups, int group_size) { return (n_groups * group_size + 256 * kHqqPer - 1) / (256 * kHqqPer); }
+
+// [mean double x kHqqMaxIters][err double kHqqChunk x blocks][scale][hist kHqqChunk x n_groups]
+extern "C" int64_t ao_b200_hqq_search_workspace_bytes(int64_t n_groups, int group_size) {
+  if (n_groups <= 0 || group_size < kHqqPer) return 0;
+  return (kHqqMaxIters + kHqqChunk * hqq_search_blocks(n_groups, group_size)) * 8 + (1 + kHqqChunk) * n_groups * 4;
+}
+
+extern "C" int ao_b200_hqq_search(const void* w, int64_t N, int64_t K, int group_size, double beta, double kappa, double lp_norm, int iters,
+                                  void* workspace, int64_t workspace_bytes, int32_t* q, void* scale_out, void* zero_out, int64_t Np, int64_t Kp,
+                                  void* packed, void* scale_and_zero, void* stream) {
+  AO_CHECK_ARG(w && workspace && N > 0 && K > 0 && beta > 0.0 && kappa > 0.0 && iters >= 1 && iters <= kHqqMaxIters);
+  if (!(group_size == 32 || group_size == 64 || group_size == 128 || group_size == 256)) return AO_B200_ERR_UNSUPPORTED;
+  AO_CHECK_ARG(K % group_size == 0 && ao_aligned(w, 16) && ao_aligned(workspace, 8));
+  AO_CHECK_ARG((q && scale_out && zero_out) || (packed && scale_and_zero));
+  AO_CHECK_ARG(!packed || (scale_and_zero && Np % 16 == 0 && Np >= N && Kp % 64 == 0 && Kp % group_size == 0 && Kp >= K && ao_aligned(packed, 16) &&
+                           ao_aligned(scale_and_zero, 4)));
+  const int64_t n_groups = N * (K / group_size), blocks = hqq_search_blocks(n_groups, group_size);
+  AO_CHECK_ARG(blocks <= 2147483647);
+  if (workspace_bytes < ao_b200_hqq_search_workspace_bytes(n_groups, group_size)) return AO_B200_ERR_WORKSPACE;
+  auto s = static_cast<cudaStream_t>(stream);
+  auto wb = static_cast<const __nv_bfloat16*>(w);
+  double* mean = static_cast<double*>(workspace);
+  double* err = mean + kHqqMaxIters;
+  float* scale = reinterpret_cast<float*>(err + kHqqChunk * blocks);
+  float* hist = scale + n_groups;
+  for (int first = 0; first < iters; first += kHqqChunk) {
+    HqqChunk ch;
+    ch.first = first;
+    ch.count = iters - first < kHqqChunk ? iters - first : kHqqChunk;
+    ch.lp_m1 = (float)(lp_norm - 1.0);
+    for (int i = 0; i < ch.count; ++i) {
+      ch.inv_beta[i] = (float)(1.0 / beta);
+      ch.threshold[i] = lp_norm < 1.0 ? (float)(0.999 * std::pow(1.0 / beta, 1.0 / (2.0 - lp_norm))) : 0.f;
+      beta *= kappa;
+    }
+    const unsigned grid = (unsigned)blocks;
+    switch (group_size) {
+      case 32: hqq_iterate_kernel<32><<<grid, 256, 0, s>>>(wb, n_groups, ch, scale, hist, err, mean); break;
+      case 64: hqq_iterate_kernel<64><<<grid, 256, 0, s>>>(wb, n_groups, ch, scale, hist, err, mean); break;
+      case 128: hqq_iterate_kernel<128><<<grid, 256, 0, s>>>(wb, n_groups, ch, scale, hist, err, mean); break;
+      default: hqq_iterate_kernel<256><<<grid, 256, 0, s>>>(wb, n_groups, ch, scale, hist, err, mean); break;
+    }
+    hqq_mean_kernel<<<ch.count, 1024, 0, s>>>(err, blocks, 1.0 / ((double)n_groups * (double)group_size), first, mean);
+  }
+  if (packed) {
+    const int64_t items = (Np / 16) * (Kp / 64) * 32 + Np * (Kp / group_size), want = (items + 255) / 256;
+    hqq_packed_kernel<<<(unsigned)(want < 148 * 16 ? want : 148 * 16), 256, 0, s>>>(wb, N, K, Np, Kp, group_size, scale, hist, mean, iters,
+                                                                                   static_cast<uint4*>(packed), static_cast<uint32_t*>(scale_and_zero));
+  }
+  if (q) {
+    const unsigned grid = (unsigned)ao_b200_hqq_blocks(n_groups);
+    AO_HQQ_DISPATCH(hqq_plain_kernel, wb, n_groups, scale, hist, mean, iters, q, static_cast<__nv_bfloat16*>(scale_out),
+                    static_cast<__nv_bfloat16*>(zero_out));
+  }
   return ao_launch_status();
 }

@@ -147,9 +147,9 @@ class AffineQuantizedTensor(torch.Tensor):
             if use_hqq:
                 # reference: affine_quantized_tensor.py:252-288 -> _choose_qparams_and_quantize_affine_hqq with
                 # nbits = log2(quant_max + 1), axis = 1, group_size = max(block_size), raw_output = False
-                q, scale, zero = torch.ops.torchao.b200_int4_hqq_quantize(
+                packed, sz = torch.ops.torchao.b200_int4_hqq_quantize_pack(
                     input_float if input_float.dtype is torch.bfloat16 else input_float.to(torch.bfloat16), int(block_size[1]))
-                tensor_impl = TensorCoreTiledAQTTensorImpl.from_plain(q, scale, zero, _layout)
+                tensor_impl = TensorCoreTiledAQTTensorImpl(packed, sz, False, _layout)
                 return cls(tensor_impl, block_size, original_shape, quant_min, quant_max, zero_point_domain,
                            dtype=input_float.dtype)
             tensor_impl = TensorCoreTiledAQTTensorImpl.from_hp(

@@ -25,6 +25,7 @@ _SCHEMAS = {
     "b200_int4_quantize": "(Tensor w, Tensor scale, Tensor zero, int group_size) -> Tensor",
     "b200_int4_pack": "(Tensor int_data) -> Tensor",
     "b200_int4_hqq_quantize": "(Tensor w, int group_size) -> (Tensor, Tensor, Tensor)",
+    "b200_int4_hqq_quantize_pack": "(Tensor w, int group_size) -> (Tensor, Tensor)",
     "b200_int4_unpack": "(Tensor packed_w) -> Tensor",
     "b200_int4_dequantize": "(Tensor packed_w, Tensor scales_and_zeros, int group_size) -> Tensor",
     "b200_tinygemm_pack": "(Tensor int_data, int inner_k_tiles) -> Tensor",
@@ -261,29 +262,45 @@ def _(w: Tensor, group_size: int):
 def _int4_hqq_quantize_cuda(w: Tensor, group_size: int):
     """`_choose_qparams_and_quantize_affine_hqq(w, nbits=4, group_size, axis=1, compute_dtype=bf16, raw_output=False)`
     (quant_primitives.py:1998-2111): q int32 (N, K) in 0..15, scale / zero bf16 (N, K/G) in the tinygemm convention.
-    One kernel per solver iteration plus a one-block kernel that applies the reference's global early stop (a mean over
-    the whole tensor) on the device: the launches after the stop return at once, the host never waits."""
+    The early stop (a mean over the whole tensor) is decided on the device; the host never waits."""
     _w_checks(w, group_size)
-    w = w.contiguous()
     n, k = w.shape
-    n_groups = n * (k // group_size)
-    L = _lib.lib()
-    scale = torch.empty(n_groups, dtype=torch.float32, device=w.device)
-    zero = torch.empty_like(scale)
-    err = torch.empty(int(L.ao_b200_hqq_blocks(n_groups)), dtype=torch.float32, device=w.device)
     q = torch.empty((n, k), dtype=torch.int32, device=w.device)
     scale_out = torch.empty((n, k // group_size), dtype=torch.bfloat16, device=w.device)
     zero_out = torch.empty_like(scale_out)
-    with torch.cuda.device(w.device):
-        st = _stream(w)
-        _lib.check(L.ao_b200_hqq_init(w.data_ptr(), n_groups, group_size, scale.data_ptr(), zero.data_ptr(), st), "hqq_init")
-        # early_stop=True (:1968-1972) is decided on the device: no host round trip per iteration
-        state = torch.empty(2, dtype=torch.float64, device=w.device)
-        _lib.check(L.ao_b200_hqq_solve(w.data_ptr(), n_groups, group_size, scale.data_ptr(), zero.data_ptr(), HQQ_BETA,
-                                       HQQ_KAPPA, HQQ_LP_NORM, HQQ_ITERS, err.data_ptr(), state.data_ptr(), st), "hqq_solve")
-        _lib.check(L.ao_b200_hqq_finalize(w.data_ptr(), n_groups, group_size, scale.data_ptr(), zero.data_ptr(),
-                                          q.data_ptr(), scale_out.data_ptr(), zero_out.data_ptr(), st), "hqq_finalize")
+    _hqq_search(w, group_size, (q.data_ptr(), scale_out.data_ptr(), zero_out.data_ptr(), 0, 0, None, None))
     return q, scale_out, zero_out
+
+
+def _hqq_search(w, group_size, outputs):
+    w = w.contiguous()
+    if w.data_ptr() % 16 != 0:
+        w = w.clone()
+    n, k = w.shape
+    L = _lib.lib()
+    ws = torch.empty(int(L.ao_b200_hqq_search_workspace_bytes(n * (k // group_size), group_size)), dtype=torch.uint8, device=w.device)
+    with torch.cuda.device(w.device):
+        _lib.check(L.ao_b200_hqq_search(w.data_ptr(), n, k, group_size, HQQ_BETA, HQQ_KAPPA, HQQ_LP_NORM, HQQ_ITERS, ws.data_ptr(), ws.numel(),
+                                        *outputs, _stream(w)), "hqq_search")
+
+
+@register_custom_op("torchao::b200_int4_hqq_quantize_pack")
+def _(w: Tensor, group_size: int):
+    np_, kp = padded_int4_shape(w.size(0), w.size(1), group_size)
+    return (torch.empty((np_ // 16, kp // 64, 32, 4), dtype=torch.int32, device=w.device),
+            torch.empty((np_ // 16, kp // group_size, 16, 2), dtype=torch.bfloat16, device=w.device))
+
+
+@_impl_cuda("b200_int4_hqq_quantize_pack")
+def _int4_hqq_quantize_pack_cuda(w: Tensor, group_size: int):
+    """The same search, its result written straight into the strip-major storage (what b200_int4_pack and
+    pack_scales_and_zeros_b200 make of the plain result)."""
+    _w_checks(w, group_size)
+    np_, kp = padded_int4_shape(w.size(0), w.size(1), group_size)
+    packed = torch.empty((np_ // 16, kp // 64, 32, 4), dtype=torch.int32, device=w.device)
+    sz = torch.empty((np_ // 16, kp // group_size, 16, 2), dtype=torch.bfloat16, device=w.device)
+    _hqq_search(w, group_size, (None, None, None, np_, kp, packed.data_ptr(), sz.data_ptr()))
+    return packed, sz
 
 
 @register_custom_op("torchao::b200_int4_pack")
