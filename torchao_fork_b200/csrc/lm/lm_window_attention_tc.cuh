@@ -9,15 +9,18 @@
 // m is the largest score so far when it grew by more than 2^8: O is rescaled only then (the weights stay below 256, their
 // bf16 parts lose nothing), and sum and product carry the same factor.
 //
-// Shared-memory tiles are no-swizzle core matrices [16-byte chunk of a row][128 rows][16 bytes]: K-major for queries and keys,
-// the same order read MN-major for the values, so that 16-byte asynchronous copies (8 rows x 64 bytes per instruction: whole
-// sectors, no bank conflicts) lay both down as they come from the ring, the first-token store or the step's rows.
+// Key and value tiles lie in shared memory as [64 columns][128 rows][128 bytes, swizzled]: K-major for the keys, the same
+// order read MN-major for the values, so both come as they are stored: a tile whose keys are neighbours in the step's rows or in
+// the ring by one TMA copy per 64 columns, others (a boundary between the stores, the last tile of a run) by 16-byte
+// asynchronous copies.  (16-byte copies for every tile took 5000 clocks a tile.)
 //
 // Bound by the tensor cores: 128 x 128 x (d + 3 dv) per tile, 2048 clocks at d = dv = 128, beside 1650 issue slots of the weights
 // (two threads per row).  One CTA per SM; late tiles, which see the most keys, start first.
 // Roles (416 threads): warps 0-7 weights and epilogue (lane quadrant = warp % 4, half of the columns = warp / 4), 8-11 loads,
 // 12 MMA issue.  Every wait is bounded; a CTA that gives up writes NaN.
 #pragma once
+#include <cuda.h>
+
 #include "lm_mma.cuh"
 
 namespace lm {
@@ -37,6 +40,9 @@ struct WinPromptArgs {
   int unit_rms;
   __nv_bfloat16* out;
   int64_t ld_out;
+};
+struct WinTcMaps {   // rows of the step's keys and values and of the rings, in boxes of 64 columns x 128 rows
+  CUtensorMap step_k, step_v, ring_k, ring_v;
 };
 
 __device__ __forceinline__ uint32_t tc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -113,7 +119,7 @@ __device__ __forceinline__ float tc_exp2(float x) {
 }
 
 template <int NM>
-__global__ void __launch_bounds__(kTcThreads, 1) window_attention_tc_kernel(WinPromptArgs a, int dv) {
+__global__ void __launch_bounds__(kTcThreads, 1) window_attention_tc_kernel(WinPromptArgs a, int dv, const __grid_constant__ WinTcMaps maps) {
   using T = __nv_bfloat16;
   extern __shared__ __align__(1024) unsigned char smem_tc[];
   uint64_t* kfull = reinterpret_cast<uint64_t*>(smem_tc);   // [2] keys of a tile are there
@@ -122,14 +128,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) window_attention_tc_kernel(WinP
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_s + 1);
   float* xmax = reinterpret_cast<float*>(smem_tc + 1024);   // [2 steps][2 halves][128 rows]
   float* xsum = xmax + 512;                                 // [2 halves][128 rows]
-  const int d = a.d, G = a.G, KD = NM * d, kc = d / 8, vc = dv / 8;
-  unsigned char* Qs = smem_tc + kTcHeader;                  // [NM][kc][128][16 bytes]
-  unsigned char* Ks = Qs + (size_t)NM * kc * 2048;          // [2][kc][128][16]
-  unsigned char* Vs = Ks + (size_t)2 * kc * 2048;           // [2][vc][128][16]
-  float* Os = reinterpret_cast<float*>(Vs + (size_t)2 * vc * 2048);  // [dv][128], two maps only
+  const int d = a.d, G = a.G, KD = NM * d, kc = d / 8, kb = (d + 63) / 64, vb = (dv + 63) / 64;
+  unsigned char* Ks = smem_tc + kTcHeader;                  // [2][kb][128][128 bytes]
+  unsigned char* Vs = Ks + (size_t)2 * kb * 16384;          // [2][vb][128][128]
+  unsigned char* Qs = Vs + (size_t)2 * vb * 16384;          // [NM][kc][128][16 bytes], no swizzle
+  float* Os = reinterpret_cast<float*>(Qs + (size_t)NM * kc * 2048);  // [dv][128], two maps only
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y, g = h / (a.H / G);
-  const int tile = gridDim.x - 1 - blockIdx.x;              // late tiles have the most keys: they start first
+  // late tiles have the most keys: those of all heads start first
+  const int turn = blockIdx.x / a.H, h = blockIdx.x - turn * a.H, g = h / (a.H / G);
+  const int tile = gridDim.x / a.H - 1 - turn;
   const int first = a.tile_first[tile], count = min(a.tile_count[tile], kTcRows);
   const int pa = a.pos[first], back0 = a.back[first];
   const int p0 = pa - back0;                                // the first position the step brings of this sequence
@@ -169,7 +176,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) window_attention_tc_kernel(WinP
     const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
     const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (((uint32_t)dv >> 3) << 17) | ((128u >> 4) << 24);  // B (values) MN-major
     const uint64_t kmaj = ((uint64_t)(2048u >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46);   // chunks 2048 bytes apart, 8-row groups 128
-    const uint64_t mnmaj = ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(2048u >> 4) << 32) | (1ull << 46);  // 8-key groups 128 bytes apart, chunks of dv 2048
+    // swizzled rows of 128 bytes, 8-row groups 1024 bytes apart; MN-major: the next 64 columns 16384 bytes on
+    const uint64_t swk = (1ull << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
+    const uint64_t swmn = ((uint64_t)(16384u >> 4) << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
     const uint32_t q0 = tc_smem(Qs) >> 4, k0 = tc_smem(Ks) >> 4, v0 = tc_smem(Vs) >> 4;
     auto scores = [&](int s) {
       const int b = s & 1, m = s / n_tiles;
@@ -178,7 +187,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) window_attention_tc_kernel(WinP
       if (tc_elect()) {
         if (ok) {
           for (int ks = 0; ks < d / 16; ++ks)
-            tc_mma_ss(tb + b * 128, kmaj | (q0 + (uint32_t)(m * kc + 2 * ks) * 128), kmaj | (k0 + (uint32_t)(b * kc + 2 * ks) * 128), idesc_s, ks != 0);
+            tc_mma_ss(tb + b * 128, kmaj | (q0 + (uint32_t)(m * kc + 2 * ks) * 128), swk | (k0 + (uint32_t)(b * kb + (ks >> 2)) * 1024 + (ks & 3) * 2), idesc_s, ks != 0);
         }
         tc_commit(&sfull[b]);
         tc_commit(&kdone[b]);
@@ -201,7 +210,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) window_attention_tc_kernel(WinP
           for (int part = 0; part < 3; ++part) {
             const uint32_t pa_ = part < 2 ? tb + b * 128 + part * 64 : tb + 256 + b * 64;
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks) tc_mma_ts(col_o, pa_ + 8 * ks, mnmaj | (v0 + (uint32_t)(b * vc) * 128 + ks * 16), idesc_o, part || ks ? 1u : fresh);
+            for (int ks = 0; ks < 8; ++ks) tc_mma_ts(col_o, pa_ + 8 * ks, swmn | (v0 + (uint32_t)(b * vb) * 1024 + ks * 128), idesc_o, part || ks ? 1u : fresh);
           }
         }
         tc_commit(odone);
@@ -210,7 +219,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) window_attention_tc_kernel(WinP
       __syncwarp();
     }
   } else if (warp >= 8) {
-    // ---- loads: this lane's key of every 8-key group, 16-byte chunk lane / 8 of every four ----
+    // ---- loads ----
     const int64_t sl = a.slot[first];
     const T* ring_k = a.ring_k + (sl * a.ring * G + g) * KD;
     const T* ring_v = a.ring_v + (sl * a.ring * G + g) * dv;
@@ -218,44 +227,54 @@ __global__ void __launch_bounds__(kTcThreads, 1) window_attention_tc_kernel(WinP
     const T* first_v = a.first_v + (sl * a.first_rows * G + g) * dv;
     const T* step_k = a.kn + (seg_row0 * G + g) * KD;
     const T* step_v = a.vn + (seg_row0 * G + g) * dv;
-    const int key0 = (warp - 8) * 32 + (lane & 7), ch0 = lane >> 3;
-    auto load = [&](unsigned char* dst, int t, int chunks, int64_t row, const T* step, const T* firsts, const T* ring) {
+    // copies of this lane: its row of every four, 16-byte chunk lane % 8 of every eight
+    const int key0 = (warp - 8) * 32 + (lane >> 3), ch = lane & 7;
+    auto load = [&](unsigned char* dst, uint64_t* full, int t, int cols, int64_t row, const T* step, const T* firsts, const T* ring, const CUtensorMap* step_map,
+                    const CUtensorMap* ring_map, int col) {
+      const int j0 = lo + (t * kTcKeys - nf), boxes = (cols + 63) / 64;   // first position of a tile without kept keys
+      const bool in = t * kTcKeys >= nf && (t + 1) * kTcKeys <= nk;
+      const bool by_step = in && j0 >= p0, by_ring = in && j0 >= a.first_rows && j0 + kTcKeys <= p0 && j0 % a.ring + kTcKeys <= a.ring;
+      if (by_step || by_ring) {
+        const CUtensorMap* map = by_step ? step_map : ring_map;
+        const int y = by_step ? (int)(seg_row0 + (j0 - p0)) : (int)(sl * a.ring + j0 % a.ring);
+        if (warp == 8 && tc_elect()) {
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem(full)), "r"(boxes * 16384) : "memory");
+          for (int k = 0; k < boxes; ++k)
+            asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(tc_smem(dst + k * 16384)),
+                         "l"(map), "r"(col + 64 * k), "r"(y), "r"(tc_smem(full))
+                         : "memory");
+        } else if (warp != 8 && lane == 0) {
+          tc_arrive(full);
+        }
+        __syncwarp();
+        return;
+      }
 #pragma unroll 1
-      for (int kg = 0; kg < 4; ++kg) {
-        const int key = key0 + 8 * kg, kk = t * kTcKeys + key;
-        unsigned char* to = dst + ((size_t)ch0 * 128 + key) * 16;
+      for (int kg = 0; kg < 8; ++kg) {
+        const int key = key0 + 4 * kg, kk = t * kTcKeys + key;
+        unsigned char* to = dst + key * 128 + ((ch ^ (key & 7)) * 16);
         if (kk < nk) {
           const int j = kk < nf ? kk : lo + (kk - nf);
-          const T* src = (j >= p0 ? step + (int64_t)(j - p0) * row : (j < a.first_rows ? firsts + (int64_t)j * row : ring + (int64_t)(j % a.ring) * row)) + ch0 * 8;
-#pragma unroll 4
-          for (int c = ch0; c < chunks; c += 4, to += 4 * 2048, src += 32) cp_async16(to, src);
+          const T* src = (j >= p0 ? step + (int64_t)(j - p0) * row : (j < a.first_rows ? firsts + (int64_t)j * row : ring + (int64_t)(j % a.ring) * row)) + ch * 8;
+          for (int c = ch * 8; c < cols; c += 64, to += 16384, src += 64) cp_async16(to, src);
         } else {   // weights of no key are zero, and so must be what they meet
-          for (int c = ch0; c < chunks; c += 4, to += 4 * 2048) *reinterpret_cast<uint4*>(to) = make_uint4(0, 0, 0, 0);
+          for (int c = ch * 8; c < cols; c += 64, to += 16384) *reinterpret_cast<uint4*>(to) = make_uint4(0, 0, 0, 0);
         }
       }
       cp_async_commit();
-    };
-    // a load has landed: visible to the tensor core (async proxy), then announced
-    auto landed = [&](uint64_t* bar) {
+      cp_async_wait<0>();
+      // visible to the tensor core (async proxy), then announced
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
-      if (lane == 0) tc_arrive(bar);
+      if (lane == 0) tc_arrive(full);
     };
     for (int s = 0; s < steps; ++s) {
       const int b = s & 1, m = s / n_tiles, t = s - m * n_tiles;
       if (s >= 2) tc_wait(&kdone[b], ((s >> 1) - 1) & 1, dead);
-      load(Ks + (size_t)b * kc * 2048, t, kc, (int64_t)G * KD, step_k + m * d, first_k + m * d, ring_k + m * d);
-      if (s > 0) {
-        cp_async_wait<1>();
-        landed(&vfull[b ^ 1]);   // the values of the step before
-      }
+      load(Ks + (size_t)b * kb * 16384, &kfull[b], t, d, (int64_t)G * KD, step_k + m * d, first_k + m * d, ring_k + m * d, &maps.step_k, &maps.ring_k, g * KD + m * d);
       if (s >= 2) tc_wait(&vdone[b], ((s >> 1) - 1) & 1, dead);
-      load(Vs + (size_t)b * vc * 2048, t, vc, (int64_t)G * dv, step_v, first_v, ring_v);
-      cp_async_wait<1>();
-      landed(&kfull[b]);
+      load(Vs + (size_t)b * vb * 16384, &vfull[b], t, dv, (int64_t)G * dv, step_v, first_v, ring_v, &maps.step_v, &maps.ring_v, g * dv);
     }
-    cp_async_wait<0>();
-    landed(&vfull[(steps - 1) & 1]);
   } else {
     // ---- weights and epilogue: thread = (row, half of the columns) ----
     const int q = warp & 3, half = warp >> 2, row = q * 32 + lane;
@@ -263,6 +282,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) window_attention_tc_kernel(WinP
     {
       // queries as bf16 operands (rows past the run are zero); a negative factor goes into their sign
       const float sign = a.scale < 0.f ? -1.f : 1.f;
+#pragma unroll 4
       for (int c = half; c < NM * kc; c += 2) {
         uint4 o = make_uint4(0, 0, 0, 0);
         if (row < count) {
@@ -276,7 +296,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) window_attention_tc_kernel(WinP
       __syncwarp();
       if (lane == 0) tc_arrive(qfull);
     }
-    const float sl2 = fabsf(a.scale) * 1.44269504088896341f;
+    const float sl2 = fmaxf(fabsf(a.scale) * 1.44269504088896341f, 1e-30f);   // (never zero: -inf stays -inf)
     const int i = row < count ? pa + row : -1;   // the row's own position (-1: no row)
     const int w_lo = pa + 32 * q, w_hi = pa + min(count, 32 * q + 32) - 1;   // positions of this warp's rows
     const int blocks = dv / 16;
@@ -328,29 +348,30 @@ __global__ void __launch_bounds__(kTcThreads, 1) window_attention_tc_kernel(WinP
         }
       }
       const float m = m_used == -INFINITY ? 0.f : m_used;
-      float sum = 0.f;
+      // p = p1 + p2 + p3 exactly: the leading 8 bits, cut off twice.  In pieces of 32, so that the exponentials of one piece (8 clocks
+      // a warp) run beside the splitting of another.
+      const uint32_t to = lane_col + tb + b * 128 + half * 32, to3 = lane_col + tb + 256 + b * 64 + half * 32;
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int e = 0; e < 64; ++e) {
-        v[e] = all || v[e] != -INFINITY ? tc_exp2(fmaf(v[e], sl2, -m)) : 0.f;
-        sum += v[e];
-      }
-      l += sum;
-      // p = p1 + p2 + p3 exactly: the leading 8 bits, cut off twice
+      for (int e0 = 0; e0 < 64; e0 += 32) {
 #pragma unroll
-      for (int part = 0; part < 3; ++part) {
-        const uint32_t to = lane_col + (part < 2 ? tb + b * 128 + part * 64 : tb + 256 + b * 64) + half * 32;
+        for (int e = e0; e < e0 + 32; ++e) {
+          v[e] = tc_exp2(fmaf(v[e], sl2, -m));
+          sum[e & 3] += v[e];
+        }
 #pragma unroll
-        for (int e = 0; e < 64; e += 32) {
+        for (int part = 0; part < 3; ++part) {
           uint32_t o[16];
 #pragma unroll
           for (int k = 0; k < 16; ++k) {
-            const uint32_t x = __float_as_uint(v[e + 2 * k]), y = __float_as_uint(v[e + 2 * k + 1]);
+            const uint32_t x = __float_as_uint(v[e0 + 2 * k]), y = __float_as_uint(v[e0 + 2 * k + 1]);
             o[k] = __byte_perm(x, y, 0x7632);
-            if (part < 2) v[e + 2 * k] -= __uint_as_float(x & 0xFFFF0000u), v[e + 2 * k + 1] -= __uint_as_float(y & 0xFFFF0000u);
+            if (part < 2) v[e0 + 2 * k] -= __uint_as_float(x & 0xFFFF0000u), v[e0 + 2 * k + 1] -= __uint_as_float(y & 0xFFFF0000u);
           }
-          tc_st16(to + e / 2, o);
+          tc_st16((part < 2 ? to + part * 64 : to3) + e0 / 2, o);
         }
       }
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_before();
       __syncwarp();
@@ -432,9 +453,30 @@ __global__ void __launch_bounds__(kTcThreads, 1) window_attention_tc_kernel(WinP
   }
 }
 
-inline size_t win_tc_smem(int nm, int d, int dv) { return kTcHeader + ((size_t)(nm + 2) * (d / 8) + 2 * (dv / 8)) * 2048 + (nm == 2 ? (size_t)dv * 512 : 0); }
-// shapes of this kernel (bf16 storage)
+inline size_t win_tc_smem(int nm, int d, int dv) {
+  return kTcHeader + (size_t)2 * ((d + 63) / 64 + (dv + 63) / 64) * 16384 + (size_t)nm * (d / 8) * 2048 + (nm == 2 ? (size_t)dv * 512 : 0);
+}
+// shapes of this kernel (bf16 storage): both tiles twice, the queries and, for two maps, a result have to fit shared memory
 inline bool win_tc_ok(int nm, int d, int dv) { return d % 16 == 0 && dv % 16 == 0 && dv >= 16 && dv <= 128 && win_tc_smem(nm, d, dv) <= 226 * 1024; }
+
+using TcEncode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                              CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+inline TcEncode tc_encode() {
+  static TcEncode fn = []() -> TcEncode {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) return nullptr;
+    return reinterpret_cast<TcEncode>(p);
+  }();
+  return fn;
+}
+// rows of `cols` bf16; how many there are is the caller's to know (the kernel only names rows that the arguments name)
+inline bool tc_rows_map(CUtensorMap* map, const void* base, int64_t cols) {
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)1 << 31}, strides[1] = {(cuuint64_t)cols * 2};
+  const cuuint32_t box[2] = {64, (cuuint32_t)kTcKeys}, steps[2] = {1, 1};
+  return tc_encode()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 template <int NM>
 int launch_win_tc(const WinPromptArgs& a, int dv, int n_tiles, cudaStream_t st) {
@@ -444,7 +486,13 @@ int launch_win_tc(const WinPromptArgs& a, int dv, int n_tiles, cudaStream_t st) 
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) return AO_B200_ERR_CUDA;
     set = true;
   }
-  kern<<<dim3((unsigned)n_tiles, (unsigned)a.H), kTcThreads, win_tc_smem(NM, a.d, dv), st>>>(a, dv);
+  WinTcMaps maps;
+  const int64_t kd = (int64_t)a.G * NM * a.d, vd = (int64_t)a.G * dv;
+  if (tc_encode() == nullptr || !tc_rows_map(&maps.step_k, a.kn, kd) || !tc_rows_map(&maps.step_v, a.vn, vd) || !tc_rows_map(&maps.ring_k, a.ring_k, kd) ||
+      !tc_rows_map(&maps.ring_v, a.ring_v, vd))
+    return AO_B200_ERR_CUDA;
+  if ((int64_t)n_tiles * a.H > 2147483647) return AO_B200_ERR_UNSUPPORTED;
+  kern<<<(unsigned)n_tiles * (unsigned)a.H, kTcThreads, win_tc_smem(NM, a.d, dv), st>>>(a, dv, maps);
   return lm_launch_status();
 }
 
