@@ -255,8 +255,15 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
   grid_launch_dependents();
 
   // the weights wait for nobody: their producer fills the ring while the others set up
-  auto load_weights = [&](int u, int slot) {
-    const int t = u / KU, ku = u - t * KU, strip = ((t / p.MT) * kRanks + rank) * 8;
+  // (running positions: a division per unit is what paced the producers)
+  const int t_first = u0 / KU, ku_first = u0 - t_first * KU;
+  int w_ku = ku_first, w_mt = t_first % p.MT, w_strip = ((t_first / p.MT) * kRanks + rank) * 8;
+  auto load_weights = [&](int slot) {
+    const int ku = w_ku, strip = w_strip;
+    if (++w_ku == KU) {
+      w_ku = 0;
+      if (++w_mt == p.MT) w_mt = 0, w_strip += kRanks * 8;
+    }
     uint8_t* dst = wring + slot * kWSlot;
     mbar_arrive_expect_tx(&wfull[slot], kWSlot);
     wq_tma_2d(dst, &p.wmap, ku * 256, strip, &wfull[slot]);
@@ -270,7 +277,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     fence_barrier_init();
     __syncwarp();
     if (wq_elect_one())
-      for (int i = 0; i < p.w_slots && u0 + i < u1; ++i) load_weights(u0 + i, i);
+      for (int i = 0; i < p.w_slots && u0 + i < u1; ++i) load_weights(i);
     __syncwarp();
   } else if (warp == kWqMma) {
     if (lane < x_slots) {
@@ -306,21 +313,21 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
   // columns [0, 256): accumulators (DEFER: one per slot of x and segment, else [buffer][MMA warp]); [256, 512): A ring
   const uint32_t a_col0 = tb + 256;
 
-  // fp32 sums of 32 rows x 16 columns (fragment order of wq_ld_16x256b_x2, lanes 0-15 in f[0..7], 16-31 in f[8..15]) -> output tile
-  auto to_stage = [&](int q, int c, const float (&f)[16], const float (&sc)[4]) {
-    const uint32_t at = smem_u32(stage) + (uint32_t)(c + 8 * (lane >> 4) + (lane & 7)) * kWqPitch + (32 * q + 8 * ((lane >> 3) & 1)) * 2;
+  // fp32 sums of rows 32 q + 16 h .. + 15, columns c .. c + 15 (fragment order of wq_ld_16x256b_x2) -> output tile
+  auto to_stage = [&](int q, int c, int h, const float* f, const float (&sc)[4]) {
+    const uint32_t at = smem_u32(stage) + (uint32_t)(c + 8 * (lane >> 4) + (lane & 7)) * kWqPitch + (32 * q + 16 * h + 8 * ((lane >> 3) & 1)) * 2;
+    uint32_t o[4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      uint32_t o[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {  // block i: column group i >> 1, row group i & 1
-        float a = f[8 * h + 4 * (i >> 1) + 2 * (i & 1)], b = f[8 * h + 4 * (i >> 1) + 2 * (i & 1) + 1];
-        // int8: mm result rounded to bf16, THEN multiplied by the row scale and rounded again
-        if constexpr (kI8) a = bf16r(a) * sc[2 * h + (i & 1)], b = bf16r(b) * sc[2 * h + (i & 1)];
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[i]) : "f"(b), "f"(a));
+    for (int i = 0; i < 4; ++i) {  // block i: column group i >> 1, row group i & 1
+      float a = f[4 * (i >> 1) + 2 * (i & 1)], b = f[4 * (i >> 1) + 2 * (i & 1) + 1];
+      // int8: mm result rounded to bf16, THEN multiplied by the row scale and rounded again
+      if constexpr (kI8) {
+        const float k = h ? sc[2 + (i & 1)] : sc[i & 1];
+        a = bf16r(a) * k, b = bf16r(b) * k;
       }
-      wq_stmatrix_trans(at + 32 * h, o[0], o[1], o[2], o[3]);
+      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[i]) : "f"(b), "f"(a));
     }
+    wq_stmatrix_trans(at, o[0], o[1], o[2], o[3]);
   };
   // the row scales (int8) of a thread's four rows 32 q + lane / 4 + 8 i
   auto row_scales = [&](int nb, int q, float (&sc)[4]) {
@@ -354,7 +361,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
   };
   // share of worker c in tile t: [NT / 16 column blocks][2 halves x 2 column groups][4 quadrants][32 lanes] float4
   auto share = [&](int c, int t) {
-    const int slot = wq_first(c, p.base, p.rem, p.quantum) / KU == t ? 0 : 1;
+    const int slot = wq_first(c, p.base, p.rem, p.quantum) >= t * KU ? 0 : 1;  // its first tile, or its last
     return reinterpret_cast<float4*>(p.part) + (((int64_t)c * 2 + slot) * kRanks + rank) * NT * 32;
   };
 
@@ -365,7 +372,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
       w.use = 1;
       for (int u = u0 + p.w_slots; u < u1; ++u) {
         if (!wq_wait(&wempty[w.slot], w.use ^ 1u, dead)) break;
-        load_weights(u, w.slot);
+        load_weights(w.slot);
         w.step(1, p.w_slots);
       }
     }
@@ -375,13 +382,21 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     grid_dependency_wait();
     if (wq_elect_one()) {
       WqRing x;
-      int t = u0 / KU, ku = u0 - t * KU;
+      const int64_t tile_bytes = (int64_t)KU * p.x_bytes;
+      const uint8_t* base = p.xt + rank * tile_bytes;
+      int mt = t_first % p.MT, ku = ku_first;
+      const uint8_t* src = base + mt * (kRanks * tile_bytes) + (int64_t)ku * p.x_bytes;
       for (int u = u0; u < u1; ++u) {
         if (!wq_wait(DEFER ? &dread[x.slot] : &xdone[x.slot], x.use ^ 1u, dead)) break;
         mbar_arrive_expect_tx(&xfull[x.slot], p.x_bytes);
-        bulk_g2s(xring + (size_t)x.slot * p.x_bytes, p.xt + ((int64_t)((t % p.MT) * kRanks + rank) * KU + ku) * p.x_bytes, p.x_bytes, &xfull[x.slot]);
+        bulk_g2s(xring + (uint32_t)x.slot * p.x_bytes, src, p.x_bytes, &xfull[x.slot]);
         x.step(1, x_slots);
-        if (++ku == KU) ku = 0, ++t;
+        src += p.x_bytes;
+        if (++ku == KU) {
+          ku = 0;
+          if (++mt == p.MT) mt = 0;
+          src = base + mt * (kRanks * tile_bytes);
+        }
       }
     }
     __syncwarp();
@@ -571,7 +586,8 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
           w.step(1, p.w_slots);
         }
         if (whole) {
-          to_stage(warp, 0, acc, sc);
+          to_stage(warp, 0, 0, acc, sc);
+          to_stage(warp, 0, 1, acc + 8, sc);
         } else {
 #pragma unroll
           for (int i = 0; i < 4; ++i) __stcg(mine + i * 128, make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]));
@@ -606,7 +622,8 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
             if (lane == 0) wq_arrive_leader<PAIR>(&dempty[d.slot]);
           }
           if (whole) {
-            to_stage(warp, c, f, sc);
+            to_stage(warp, c, 0, f, sc);
+            to_stage(warp, c, 1, f + 8, sc);
           } else {
 #pragma unroll
             for (int i = 0; i < 4; ++i) __stcg(mine + (c / 4 + i) * 128, make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]));
@@ -635,22 +652,19 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     __threadfence();
     const int t = k == 0 ? u0 / KU : (u1 - 1) / KU, nb = t / p.MT, mt = t - nb * p.MT;
     const int c0 = wq_owner(t * KU, p.base, p.rem, p.quantum), c1 = wq_owner(t * KU + KU - 1, p.base, p.rem, p.quantum);
-    for (int it = warp; it < NT / 4; it += kWqThreads / 32) {  // (column block, quadrant)
-      const int q = it & 3, c = (it >> 2) * 16;
-      float f[16], sc[4];
+    for (int it = warp; it < NT / 2; it += kWqThreads / 32) {  // (column block, quadrant, half)
+      const int h = it & 1, q = (it >> 1) & 3, c = (it >> 3) * 16;
+      float f[8], sc[4];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) f[i] = 0.f;
+      for (int i = 0; i < 8; ++i) f[i] = 0.f;
       row_scales(nb, q, sc);
-#pragma unroll 2
+#pragma unroll 4
       for (int cc = c0; cc <= c1; ++cc) {
-        const float4* src = share(cc, t) + (c / 4) * 128 + q * 32 + lane;
-        float4 v[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = __ldcg(src + i * 128);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) f[4 * i] += v[i].x, f[4 * i + 1] += v[i].y, f[4 * i + 2] += v[i].z, f[4 * i + 3] += v[i].w;
+        const float4* src = share(cc, t) + (c / 4 + 2 * h) * 128 + q * 32 + lane;
+        const float4 v0 = __ldcg(src), v1 = __ldcg(src + 128);
+        f[0] += v0.x, f[1] += v0.y, f[2] += v0.z, f[3] += v0.w, f[4] += v1.x, f[5] += v1.y, f[6] += v1.z, f[7] += v1.w;
       }
-      to_stage(q, c, f, sc);
+      to_stage(q, c, h, f, sc);
     }
     __syncthreads();
     copy_out(nb, mt, threadIdx.x, kWqThreads);
