@@ -272,6 +272,17 @@ def _linear(func, args, kwargs):
     """reference: affine_quantized_tensor_ops.py:267-296"""
     input_tensor, weight_tensor = args[0], args[1]
     bias = args[2] if len(args) > 2 else kwargs.get("bias")
+    if type(input_tensor) in _PLAIN and (bias is None or type(bias) in _PLAIN):
+        # nobody else has a say in this call: every attribute of the weight that is read below would come back here otherwise
+        with torch._C.DisableTorchFunctionSubclass():
+            return _linear_any(func, input_tensor, weight_tensor, bias)
+    return _linear_any(func, input_tensor, weight_tensor, bias)
+
+
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def _linear_any(func, input_tensor, weight_tensor, bias):
     if not input_tensor.is_floating_point():
         raise NotImplementedError(f"{func} is not implemented for non floating point input")
     try:

@@ -236,12 +236,13 @@ def _linear_bf16_act_uint4_weight_impl(input_tensor, weight_tensor, bias):
         f"need input_tensor shape: {input_tensor.shape} final dim to match weight_tensor shape: "
         f"{weight_tensor.shape} second dim")
     impl = weight_tensor.tensor_impl
-    orig_act_size = input_tensor.size()
-    act_mat = input_tensor.reshape(-1, input_tensor.shape[-1])
+    orig_act_size = input_tensor.shape
+    flat = len(orig_act_size) == 2
+    act_mat = input_tensor if flat else input_tensor.reshape(-1, orig_act_size[-1])
     out_features = weight_tensor.shape[-2]
-    y = torch.ops.torchao.b200_int4_weight_only_mm(act_mat, impl.packed_weight, weight_tensor.block_size[-1],
-                                                   impl.scale_and_zero, out_features)
-    y = y.reshape(*orig_act_size[:-1], out_features)
+    y = _ops.int4_weight_only_mm(act_mat, impl.packed_weight, weight_tensor.block_size[-1], impl.scale_and_zero, out_features)
+    if not flat:
+        y = y.reshape(*orig_act_size[:-1], out_features)
     if bias is not None:
         y += bias
     return y
@@ -380,9 +381,11 @@ def _linear_fp_act_int8_weight_impl(input_tensor, weight_tensor, bias):
     if input_tensor.dtype != torch.bfloat16:
         raise NotImplementedError("B200 int8 weight-only linear takes bfloat16 activations")
     impl = weight_tensor.tensor_impl
-    x2d = input_tensor.reshape(-1, input_tensor.shape[-1])
-    y = torch.ops.torchao.b200_int8_weight_only_mm(x2d, impl.packed, impl.scale)
-    y = y.reshape(*input_tensor.shape[:-1], y.shape[-1])
+    flat = input_tensor.dim() == 2
+    x2d = input_tensor if flat else input_tensor.reshape(-1, input_tensor.shape[-1])
+    y = _ops.int8_weight_only_mm(x2d, impl.packed, impl.scale)
+    if not flat:
+        y = y.reshape(*input_tensor.shape[:-1], y.shape[-1])
     if bias is not None:
         y += bias.to(y.dtype)
     return y

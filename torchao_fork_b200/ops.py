@@ -8,8 +8,11 @@ current CUDA stream to the C ABI of libao_b200.so (include/ao_b200.h).  There is
 """
 from typing import Tuple
 
+from functools import lru_cache
+
 import torch
 from torch import Tensor
+from torch.autograd import forward_ad as _forward_ad
 
 from . import _lib
 
@@ -74,6 +77,35 @@ def _stream(t: Tensor):
 
 def _round_up(a, b):
     return (a + b - 1) // b * b
+
+
+def runs_eagerly(x: Tensor, *others: Tensor) -> bool:
+    """True if calling the CUDA implementation of an op on these tensors does all that going through the dispatcher would: plain
+    tensors (no fake ones, no wrappers), nothing to differentiate in either direction, and no mode, transform or tracer that wants to
+    see the op.  The dispatcher and the schema's boxing are half of the host time of a small linear."""
+    if type(x) is not Tensor or (x.requires_grad and torch.is_grad_enabled()):
+        return False
+    for t in others:
+        if type(t) is not Tensor:
+            return False
+    return (torch._C._len_torch_dispatch_stack() == 0 and torch._C._functorch.peek_interpreter_stack() is None
+            and torch._C._get_tracing_state() is None and _forward_ad._current_level < 0)
+
+
+class _NoGuard:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_NO_GUARD = _NoGuard()
+
+
+def _on(index: int):
+    """Context in which the device `index` is current (nothing to do where it is already)."""
+    return _NO_GUARD if torch._C._cuda_getDevice() == index else torch.cuda.device(index)
 
 
 def padded_int4_shape(n: int, k: int, group_size: int) -> Tuple[int, int]:
@@ -439,12 +471,12 @@ def _(x: Tensor, packed_w: Tensor, group_size: int, scales_and_zeros: Tensor, ou
 _WORKSPACES = {}
 
 
-def _workspace(device, nbytes, tag="int4"):
+def _workspace(device, nbytes, tag="int4", stream=None):
     """Per (device, stream, tag) scratch.  The int4 buffer carries the tensor-memory GEMV's tickets (must stay zero), so
     the int8 GEMM's staging copy lives in its own buffer."""
     if nbytes == 0:
         return None
-    key = (device, torch.cuda.current_stream(device).cuda_stream, tag)
+    key = (device, torch.cuda.current_stream(device).cuda_stream if stream is None else stream, tag)
     ws = _WORKSPACES.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.zeros(nbytes, dtype=torch.uint8, device=device)
@@ -452,30 +484,67 @@ def _workspace(device, nbytes, tag="int4"):
     return ws
 
 
-@_impl_cuda("b200_int4_weight_only_mm")
-def _int4_mm_cuda(x: Tensor, packed_w: Tensor, group_size: int, scales_and_zeros: Tensor, out_features: int):
-    """Same contract as aten._weight_int4pack_mm(x, packed, G, scale_and_zero)
-    (call site torchao/dtypes/uintx/tensor_core_tiled_layout.py:104) on the super-tile layout."""
+@lru_cache(maxsize=4096)
+def _mm_workspace_bytes(bits, m, np_, kp):
+    """A pure function of the shape."""
+    L = _lib.lib()
+    return int((L.ao_b200_int4_mm_workspace_bytes if bits == 4 else L.ao_b200_int8_mm_workspace_bytes)(m, np_, kp))
+
+
+def _mm_rows(x):
+    """The activations as the kernels read them: rows of a multiple of 8 columns, 16-byte aligned -> (tensor, leading dimension)"""
+    if x.size(1) % 8 != 0:
+        x = torch.nn.functional.pad(x, (0, (-x.size(1)) % 8))
+    return _rows(x)
+
+
+def int4_weight_only_mm(x: Tensor, packed_w: Tensor, group_size: int, scales_and_zeros: Tensor, out_features: int) -> Tensor:
+    """torch.ops.torchao.b200_int4_weight_only_mm, without the dispatcher where that adds nothing"""
+    if runs_eagerly(x, packed_w, scales_and_zeros):
+        return _int4_mm_cuda(x, packed_w, group_size, scales_and_zeros, out_features)
+    return torch.ops.torchao.b200_int4_weight_only_mm(x, packed_w, group_size, scales_and_zeros, out_features)
+
+
+def int8_weight_only_mm(x: Tensor, packed_w: Tensor, scale: Tensor) -> Tensor:
+    """torch.ops.torchao.b200_int8_weight_only_mm, without the dispatcher where that adds nothing"""
+    if runs_eagerly(x, packed_w, scale):
+        return _int8_mm_cuda(x, packed_w, scale)
+    return torch.ops.torchao.b200_int8_weight_only_mm(x, packed_w, scale)
+
+
+def _int4_mm_checks(x, packed_w, group_size, scales_and_zeros, out_features):
     np_, kp = _strip_shape_checks(packed_w)
     _sz_checks_b200(scales_and_zeros, np_, kp, group_size)
     _check_cuda_bf16(x, "activation")
     torch._check(x.dim() == 2 and x.size(1) <= kp, lambda: f"x must be (M, K<= {kp}), got {tuple(x.shape)}")
     torch._check(0 < out_features <= np_, lambda: "out_features out of range")
     torch._check(packed_w.is_contiguous() and scales_and_zeros.is_contiguous(), lambda: "weights must be contiguous")
-    m = x.size(0)
-    y = torch.empty((m, out_features), dtype=torch.bfloat16, device=x.device)
+
+
+@_impl_cuda("b200_int4_weight_only_mm")
+def _int4_mm_cuda(x: Tensor, packed_w: Tensor, group_size: int, scales_and_zeros: Tensor, out_features: int):
+    """Same contract as aten._weight_int4pack_mm(x, packed, G, scale_and_zero)
+    (call site torchao/dtypes/uintx/tensor_core_tiled_layout.py:104) on the super-tile layout."""
+    ps, xs = packed_w.shape, x.shape
+    if not (len(ps) == 4 and len(xs) == 2 and x.is_cuda and x.dtype is torch.bfloat16 and packed_w.dtype is torch.int32
+            and scales_and_zeros.dtype is torch.bfloat16 and group_size in (32, 64, 128, 256) and ps[2] == 32 and ps[3] == 4
+            and scales_and_zeros.shape == (ps[0], ps[1] * 64 // group_size, 16, 2) and xs[1] <= ps[1] * 64
+            and 0 < out_features <= ps[0] * 16 and packed_w.is_contiguous() and scales_and_zeros.is_contiguous()):
+        _int4_mm_checks(x, packed_w, group_size, scales_and_zeros, out_features)
+    np_, kp, m = ps[0] * 16, ps[1] * 64, xs[0]
+    device = x.device
+    y = torch.empty((m, out_features), dtype=torch.bfloat16, device=device)
     if m == 0:
         return y
-    if x.size(1) % 8 != 0:
-        x = torch.nn.functional.pad(x, (0, (-x.size(1)) % 8))
-    x, ldx = _rows(x)
-    L = _lib.lib()
-    ws_bytes = L.ao_b200_int4_mm_workspace_bytes(m, np_, kp)
-    ws = _workspace(x.device, ws_bytes)
-    with torch.cuda.device(x.device):
-        _lib.check(L.ao_b200_int4_mm(x.data_ptr(), m, x.size(1), ldx, packed_w.data_ptr(), scales_and_zeros.data_ptr(),
-                                     np_, kp, group_size, y.data_ptr(), out_features, out_features,
-                                     ws.data_ptr() if ws is not None else None, ws_bytes, _stream(x)), "int4_mm")
+    x, ldx = _mm_rows(x)
+    ws_bytes = _mm_workspace_bytes(4, m, np_, kp)
+    stream = torch._C._cuda_getCurrentRawStream(device.index)
+    ws = _workspace(device, ws_bytes, stream=stream)
+    with _on(device.index):
+        rc = _lib.lib().ao_b200_int4_mm(x.data_ptr(), m, x.size(1), ldx, packed_w.data_ptr(), scales_and_zeros.data_ptr(), np_, kp, group_size,
+                                        y.data_ptr(), out_features, out_features, ws.data_ptr() if ws is not None else None, ws_bytes, stream)
+    if rc:
+        _lib.check(rc, "int4_mm")
     return y
 
 
@@ -554,31 +623,39 @@ def _(x: Tensor, packed_w: Tensor, scale: Tensor):
     return torch.empty((x.size(0), scale.numel()), dtype=torch.bfloat16, device=x.device)
 
 
-@_impl_cuda("b200_int8_weight_only_mm")
-def _int8_mm_cuda(x: Tensor, packed_w: Tensor, scale: Tensor):
-    """y = (x @ int_data.T.to(bf16)) * scale with the reference's two bf16 roundings
-    (torchao/dtypes/uintx/plain_layout.py:250-266); out_features = scale.numel()."""
+def _int8_mm_checks(x, packed_w, scale):
     _check_cuda_bf16(x, "activation")
     _check_cuda_bf16(scale, "scale")
     np_, kp = _int8_packed_checks(packed_w)
     n = scale.numel()
     torch._check(x.dim() == 2 and x.size(1) <= kp, lambda: "x / weight K mismatch")
     torch._check(0 < n <= np_, lambda: "scale must have one entry per output row")
+
+
+@_impl_cuda("b200_int8_weight_only_mm")
+def _int8_mm_cuda(x: Tensor, packed_w: Tensor, scale: Tensor):
+    """y = (x @ int_data.T.to(bf16)) * scale with the reference's two bf16 roundings
+    (torchao/dtypes/uintx/plain_layout.py:250-266); out_features = scale.numel()."""
+    ps, xs, n = packed_w.shape, x.shape, scale.numel()
+    if not (len(ps) == 3 and len(xs) == 2 and x.is_cuda and scale.is_cuda and packed_w.is_cuda and x.dtype is torch.bfloat16
+            and scale.dtype is torch.bfloat16 and packed_w.dtype is torch.uint8 and ps[2] == 1024 and packed_w.is_contiguous()
+            and xs[1] <= ps[1] * 64 and 0 < n <= ps[0] * 16):
+        _int8_mm_checks(x, packed_w, scale)
+    np_, kp, m = ps[0] * 16, ps[1] * 64, xs[0]
+    device = x.device
     scale = scale.contiguous()
-    m = x.size(0)
-    y = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
+    y = torch.empty((m, n), dtype=torch.bfloat16, device=device)
     if m == 0:
         return y
-    if x.size(1) % 8 != 0:
-        x = torch.nn.functional.pad(x, (0, (-x.size(1)) % 8))
-    x, ldx = _rows(x)
-    L = _lib.lib()
-    ws_bytes = L.ao_b200_int8_mm_workspace_bytes(m, np_, kp)
-    ws = _workspace(x.device, ws_bytes, "int8")
-    with torch.cuda.device(x.device):
-        _lib.check(L.ao_b200_int8_mm(x.data_ptr(), m, x.size(1), ldx, packed_w.data_ptr(), scale.data_ptr(), np_, kp,
-                                     y.data_ptr(), n, n, ws.data_ptr() if ws is not None else None, ws_bytes, _stream(x)),
-                   "int8_mm")
+    x, ldx = _mm_rows(x)
+    ws_bytes = _mm_workspace_bytes(8, m, np_, kp)
+    stream = torch._C._cuda_getCurrentRawStream(device.index)
+    ws = _workspace(device, ws_bytes, "int8", stream)
+    with _on(device.index):
+        rc = _lib.lib().ao_b200_int8_mm(x.data_ptr(), m, x.size(1), ldx, packed_w.data_ptr(), scale.data_ptr(), np_, kp, y.data_ptr(), n, n,
+                                        ws.data_ptr() if ws is not None else None, ws_bytes, stream)
+    if rc:
+        _lib.check(rc, "int8_mm")
     return y
 
 
