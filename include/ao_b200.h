@@ -118,7 +118,7 @@ AO_B200_API int ao_b200_tinygemm_pack(const int32_t* q, int64_t N, int64_t K, in
  *   y[m][n] = bf16( sum_k fp32( x[m][k] * W'[n][k] ) ),  n < N_out.
  * x: bf16 [M][Kx] row stride ldx (Kx <= Kp, Kx % 8 == 0; k >= Kx reads as zero — no
  * host-side F.pad of the activation); y: bf16 [M][N_out] row stride ldy.
- * M <= 16 -> HBM-bound split-K tensor-core GEMV; larger M -> tcgen05 GEMM.
+ * few rows -> HBM-bound split-K tensor-core GEMV; more rows (from 3 to 17 on, by the weight's size) -> tcgen05 GEMM.
  * workspace: ao_b200_int4_mm_workspace_bytes(...) bytes, zero-initialised once by the
  * caller (the kernels leave it zeroed on exit); may be NULL when that returns 0. */
 AO_B200_API int64_t ao_b200_int4_mm_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
@@ -199,9 +199,16 @@ AO_B200_API int ao_b200_int8_unpack(const void* packed, int64_t Np, int64_t Kp, 
 
 /* Replacement for _linear_fp_act_int8_weight_impl (plain_layout.py:250-266):
  *   y = bf16( bf16( x @ q^T ) * scale ).   x bf16 [M][Kx] (ldx; k >= Kx reads as zero), packed strip-major int8 (Np x Kp),
- *   scale bf16 [N_out], y bf16 [M][N_out] (ldy).  M <= 16: TMA-ring GEMV (gemv_int8_fused.cu); larger M: tcgen05 GEMM
+ *   scale bf16 [N_out], y bf16 [M][N_out] (ldy).  few rows: TMA-ring GEMV (gemv_int8_fused.cu); more: tcgen05 GEMM
  *   (needs Np % 128 == 0 and a workspace of ao_b200_int8_mm_workspace_bytes; otherwise the GEMV is looped). */
 AO_B200_API int64_t ao_b200_int8_mm_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
+/* y = bf16(residual + bf16(x W'^T)), any M: a linear with its residual add where the activations do not fit the fused GEMV.
+ * group_size 0: int8 (`scales` = bf16 row scales), else int4 (`scales` = scale_and_zero).  residual may be y itself.
+ * Np % 128 == 0; workspace: ao_b200_mm_residual_workspace_bytes, its contents need not survive between calls. */
+AO_B200_API int64_t ao_b200_mm_residual_workspace_bytes(int64_t M, int64_t Np, int64_t Kp, int group_size);
+AO_B200_API int ao_b200_mm_residual(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scales, int64_t Np,
+                                    int64_t Kp, int group_size, void* y, int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res,
+                                    void* workspace, int64_t workspace_bytes, void* stream);
 AO_B200_API int ao_b200_int8_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx,
                     const void* packed, const void* scale, int64_t Np, int64_t Kp,
                     void* y, int64_t N_out, int64_t ldy, void* workspace, int64_t workspace_bytes, void* stream);

@@ -58,3 +58,47 @@ def test_splits(bits, m, n, k, group):
 def test_output_rows_off_16_bytes(bits):
     # N not a multiple of 8: rows of y start at odd places, stored element by element
     _check(bits, 50, 323, 256, 64)
+
+
+@pytest.mark.parametrize("m", [2, 3, 8, 9, 12, 16, 17])
+@pytest.mark.parametrize("bits,n,k,group", [(4, 16384, 8192, 128), (4, 8192, 16384, 64), (4, 14336, 4096, 32), (8, 16384, 8192, 0), (8, 640, 14336, 0)])
+def test_few_rows(bits, n, k, group, m):
+    # both sides of the rule that sends calls of up to 16 rows to the GEMM
+    _check(bits, m, n, k, group)
+
+
+@pytest.mark.parametrize("bits,group", [(4, 32), (4, 128), (8, 0)])
+@pytest.mark.parametrize("m,n,k", [(1, 128, 64), (8, 640, 1088), (16, 321, 4096), (17, 640, 1088), (40, 1000, 512), (200, 640, 2048)])
+def test_residual(bits, group, m, n, k):
+    # y = bf16(residual + bf16(x W^T)): the residual's sum of the plain call's result, also in place and with wider rows
+    from torchao_fork_b200 import _lib
+    k = -(-k // max(group, 1)) * max(group, 1)
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    w = torch.randn(n, k, generator=gen, device="cuda").to(torch.bfloat16)
+    x = torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16)
+    if bits == 4:
+        packed, scales = T.b200_int4_quantize_pack(w, group, 1e-6, True)
+        plain = T.b200_int4_weight_only_mm(x, packed, group, scales, n)
+    else:
+        q, scales = T.b200_int8_quantize(w, 1e-6, True)
+        packed = T.b200_int8_pack(q)
+        plain = T.b200_int8_weight_only_mm(x, packed, scales)
+    np_, kp = packed.shape[0] * 16, packed.shape[1] * 64
+    xp = torch.nn.functional.pad(x, (0, kp - k))
+    L = _lib.lib()
+    ws = torch.empty(L.ao_b200_mm_residual_workspace_bytes(m, np_, kp, group), dtype=torch.uint8, device="cuda").random_(0, 255)
+    h = torch.randn(m, n + 3, generator=gen, device="cuda").to(torch.bfloat16)
+    run = lambda res, y: _lib.check(L.ao_b200_mm_residual(  # noqa: E731
+        xp.data_ptr(), m, kp, kp, packed.data_ptr(), scales.data_ptr(), np_, kp, group, y.data_ptr(), n, y.stride(0), res.data_ptr(), res.stride(0),
+        ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream), "mm_residual")
+    y = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+    run(h, y)
+    inside = h.clone()
+    run(inside[:, :n], inside)
+    assert torch.equal(inside[:, :n], y) and torch.equal(inside[:, n:], h[:, n:])
+    if m > 16:   # the plain call is this GEMM too: the same bits
+        assert torch.equal(y, h[:, :n] + plain)
+    # below, the plain call may be a kernel that sums in another order: one rounding of the product apart
+    assert ((y.double() - h[:, :n].double() - plain.double()).norm() / y.double().norm()).item() < 2.0 ** -7
+    assert L.ao_b200_mm_residual(xp.data_ptr(), m, kp, kp, packed.data_ptr(), scales.data_ptr(), np_, kp, group, y.data_ptr(), n, n, h.data_ptr(), n + 3,
+                                 ws.data_ptr(), 16, 0) != 0

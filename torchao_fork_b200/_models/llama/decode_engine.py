@@ -84,11 +84,26 @@ class _Linear:
             self.weight_bytes = self.w.numel() * 2
 
     def workspace_bytes(self, m):
+        L = _lib.lib()
         if self.kind == "int4":
-            return int(_lib.lib().ao_b200_int4_mm_workspace_bytes(m, self.np_, self.kp))
+            return int(L.ao_b200_int4_mm_workspace_bytes(m, self.np_, self.kp))
         if self.kind == "int8":
-            return int(_lib.lib().ao_b200_int8_mm_workspace_bytes(m, self.np_, self.kp))
+            return int(L.ao_b200_int8_mm_workspace_bytes(m, self.np_, self.kp))
         return 0
+
+    def residual_workspace_bytes(self, m):
+        """0: not a shape (or a kind) of the GEMM that adds the residual"""
+        if self.kind == "bf16":
+            return 0
+        return int(_lib.lib().ao_b200_mm_residual_workspace_bytes(m, self.np_, self.kp, self.group_size if self.kind == "int4" else 0))
+
+    def launch_residual(self, x, y, ws, stream):
+        """y = bf16(y + bf16(x W^T)) for any number of rows"""
+        int4 = self.kind == "int4"
+        _lib.check(_lib.lib().ao_b200_mm_residual(
+            x.data_ptr(), x.shape[0], self.k, x.stride(0), self.packed.data_ptr(), (self.sz if int4 else self.scale).data_ptr(), self.np_,
+            self.kp, self.group_size if int4 else 0, y.data_ptr(), self.n, y.stride(0), y.data_ptr(), y.stride(0), ws.data_ptr(), ws.numel(), stream),
+            "mm_residual")
 
     def launch_fused(self, x, y, stream, norm_w=None, eps=0.0, residual=None, epilogue=0, ws=None):
         """ao_b200_int4_gemv_fused / ao_b200_int8_gemv_fused: RMSNorm prologue (norm_w), epilogue 0 plain / 1 residual
@@ -153,13 +168,16 @@ class DecodeEngine:
         self.fused = (fused and all(l.fused_fits(batch_size) for l in probe)
                       and int(model.layers[0].feed_forward.w1.weight.shape[0]) % 128 == 0
                       and type(model.layers[0].feed_forward.w1.weight) is type(model.layers[0].feed_forward.w3.weight))
+        # where only some projections (the longer ones) fit the fused GEMV, those still take it
+        self.parts = fused and not self.fused and tp is None
         for blk in model.layers:
             ff = blk.feed_forward
             fuse = int(ff.w1.weight.shape[0]) % 128 == 0 and type(ff.w1.weight) is type(ff.w3.weight)
             self.layers.append(dict(
                 attn_norm=blk.attention_norm.weight.detach(), ffn_norm=blk.ffn_norm.weight.detach(),
                 wqkv=_Linear([blk.attention.wqkv.weight]), wo=_Linear([blk.attention.wo.weight]),
-                w13=_Linear([ff.w1.weight, ff.w3.weight], interleave_gate_up=self.fused) if fuse else None,
+                w13=_Linear([ff.w1.weight, ff.w3.weight],
+                            interleave_gate_up=self.fused or (self.parts and _Linear([ff.w1.weight]).fused_fits(batch_size))) if fuse else None,
                 w1=None if fuse else _Linear([ff.w1.weight]), w3=None if fuse else _Linear([ff.w3.weight]),
                 w2=_Linear([ff.w2.weight]),
                 k_cache=blk.attention.kv_cache.k_cache, v_cache=blk.attention.kv_cache.v_cache,
@@ -194,6 +212,9 @@ class DecodeEngine:
         lins = [self.output] + [l[k] for l in self.layers for k in ("wqkv", "wo", "w13", "w1", "w3", "w2") if l[k]]
         ws_bytes = max(l.workspace_bytes(B) for l in lins)
         self.ws = torch.zeros(max(ws_bytes, 16), dtype=torch.uint8, device=dev)
+        # the GEMM that adds the residual keeps nothing between launches; the tickets in self.ws have to stay zero, so it has its own
+        self.res_ws = torch.empty(max([16] + [l[k].residual_workspace_bytes(B) for l in self.layers for k in ("wo", "w2")]) if self.parts else 16,
+                                  dtype=torch.uint8, device=dev)
         # sequence splits of the decode attention: one 32-position block per split up to S = 1024 (a block is one DRAM
         # round trip; fewer splits = fewer CTAs and a cheaper merge), <= 32 (the merge keeps one split per lane)
         self.n_split = max(1, min(32, -(-self.S // 32)))
@@ -424,6 +445,8 @@ class DecodeEngine:
             return self._launch_step_fused()
         if self.kv_int8:
             raise NotImplementedError("int8 KV cache: only with the fused decode step (M * K must fit the GEMV staging)")
+        if self.parts:
+            return self._launch_step_parts()
         L = _lib.lib()
         st = torch.cuda.current_stream(self.device).cuda_stream
         B, D = self.B, self.cfg.dim
@@ -466,6 +489,60 @@ class DecodeEngine:
         if self.tp is not None:
             logits = self.tp.gather_logits(self.logits)
         self._sample(logits)
+        self.tok.copy_(self.next_tok)
+        self.pos.add_(1)
+
+    def _launch_step_parts(self):
+        """Batches whose activations do not fit the staging of every fused GEMV: a projection that fits keeps its RMSNorm prologue and
+        residual / SiLU*mul epilogue, another one is a norm (or SiLU*mul) launch and the GEMM, which adds the residual itself."""
+        L = _lib.lib()
+        st = torch.cuda.current_stream(self.device).cuda_stream
+        B, D = self.B, self.cfg.dim
+        n = 1
+        torch.index_select(self.emb, 0, self.tok, out=self.h)
+
+        def normed(lin, weight, y):
+            if lin.fused_fits(B):
+                lin.launch_fused(self.h, y, st, norm_w=weight, eps=self.eps, ws=self.ws)
+                return 1
+            _lib.check(L.ao_b200_rmsnorm(self.h.data_ptr(), None, weight.data_ptr(), None, self.a.data_ptr(), B, D, self.eps, st), "rmsnorm")
+            lin.launch(self.a, y, self.ws, st)
+            return 2
+
+        def residual(lin, x):
+            if lin.fused_fits(B):
+                lin.launch_fused(x, self.h, st, residual=self.h, epilogue=1, ws=self.ws)
+            elif lin.residual_workspace_bytes(B):
+                lin.launch_residual(x, self.h, self.res_ws, st)
+            else:
+                lin.launch(x, self.delta, self.ws, st)
+                self.h.add_(self.delta)
+                return 2
+            return 1
+
+        for l in self.layers:
+            n += normed(l["wqkv"], l["attn_norm"], self.qkv)
+            _lib.check(L.ao_b200_decode_attention_fused(
+                self.qkv.data_ptr(), self.freqs.data_ptr(), self.pos.data_ptr(), l["k_cache"].data_ptr(), l["v_cache"].data_ptr(), self.o.data_ptr(), B,
+                self.H, self.Hkv, self.hd, self.S, 1.0 / math.sqrt(self.hd), self.n_split, self.attn_fused_ws.data_ptr(), self.attn_fused_ws.numel(), st),
+                "decode_attention_fused")
+            n += 1 + residual(l["wo"], self.o)
+            if l["w13"] is not None and l["w13"].interleaved:
+                l["w13"].launch_fused(self.h, self.s, st, norm_w=l["ffn_norm"], eps=self.eps, epilogue=2, ws=self.ws)
+                n += 1
+            else:
+                _lib.check(L.ao_b200_rmsnorm(self.h.data_ptr(), None, l["ffn_norm"].data_ptr(), None, self.a.data_ptr(), B, D, self.eps, st), "rmsnorm")
+                if l["w13"] is not None:
+                    l["w13"].launch(self.a, self.gu, self.ws, st)
+                else:
+                    l["w1"].launch(self.a, self.gu[:, : self.I], self.ws, st)
+                    l["w3"].launch(self.a, self.gu[:, self.I:], self.ws, st)
+                _lib.check(L.ao_b200_silu_mul(self.gu.data_ptr(), self.s.data_ptr(), B, self.I, st), "silu_mul")
+                n += 3
+            n += residual(l["w2"], self.s)
+        n += normed(self.output, self.out_norm, self.logits)
+        self.launches_per_step = n
+        self._sample(self.logits)
         self.tok.copy_(self.next_tok)
         self.pos.add_(1)
 

@@ -15,7 +15,10 @@ int int4_gemv_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* 
                  int64_t ld_res, int epilogue, void* workspace, int64_t workspace_bytes, bool pdl, cudaStream_t s);
 int64_t int4_gemv_tc_workspace_bytes(int64_t Np);
 int int4_gemm_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np, int64_t Kp,
-                 int G, void* y, int64_t N_out, int64_t ldy, void* workspace, int64_t workspace_bytes, cudaStream_t s);
+                 int G, void* y, int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res, void* workspace, int64_t workspace_bytes,
+                 cudaStream_t s);
+bool int4_gemv_fused_fits(int64_t M, int64_t Kp, int G, int max_stages);
+bool int8_gemv_fused_fits(int64_t M, int64_t Kp, int max_stages);
 int64_t int4_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
 int64_t int8_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
 int int8_gemv(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Kp,
@@ -24,7 +27,8 @@ int int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
                     int64_t Kp, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps, const void* residual,
                     int64_t ld_res, int epilogue, int max_stages, bool pdl, cudaStream_t s);
 int int8_gemm_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Np,
-                 int64_t Kp, void* y, int64_t N_out, int64_t ldy, void* workspace, int64_t workspace_bytes, cudaStream_t s);
+                 int64_t Kp, void* y, int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res, void* workspace,
+                 int64_t workspace_bytes, cudaStream_t s);
 }  // namespace ao
 
 extern "C" const char* ao_b200_error_string(int code) {
@@ -74,12 +78,33 @@ const Tunables& tunables() {
 }
 }  // namespace
 
+// Which calls of up to 16 rows take the GEMM (gemm_wq_tc.cu) rather than the GEMV that keeps the activations in shared memory.  The GEMM
+// costs about 10 us of staging, launch and tail whatever the size, then streams 16 rows as fast as 3; the GEMV has no such costs but
+// its time grows with the rows.  Measured (GEMV / GEMM, us): int4 28672 x 8192, 8 rows 39 / 44, 12 rows 63 / 44; 14336 x 4096, 8 rows 15 / 19,
+// 12 rows 20 / 19, 16 rows 23 / 19; 4096 x 4096, 16 rows 14 / 14; int8 28672 x 8192, 12 rows 66 / 47, 14336 x 4096, 16 rows 26 / 22,
+// 4096 x 4096, 16 rows 15 / 15.  Where the activations do not fit, the strip kernels are the other choice: int4 8192 x 28672 64 / 44 from
+// 3 to 16 rows, 4096 x 14336 18 / 20; int8 8192 x 28672, 3 to 16 rows 56 .. 79 / 47, 4096 x 14336, 8 rows 18 / 23, 12 rows 27 / 23.
+static bool few_rows_by_gemm(int64_t M, int64_t Np, int64_t Kp, bool fits, bool int4) {
+  if (M < 3 || Np % 128 != 0) return false;
+  if (M > 16) return true;
+  if (fits) return (M - 8) * Np * Kp >= (int64_t)224 << 20;
+  return Np * Kp >= (int64_t)128 << 20 || (!int4 && M > 8);
+}
+static bool int4_by_gemm(int64_t M, int64_t Np, int64_t Kp, int G) {
+  return tunables().gemm_tc && few_rows_by_gemm(M, Np, Kp, M > 16 || ao::int4_gemv_fused_fits(M, Kp, G, tunables().stages), true);
+}
+static bool int8_by_gemm(int64_t M, int64_t Np, int64_t Kp) {
+  return tunables().gemm_tc && few_rows_by_gemm(M, Np, Kp, M > 16 || ao::int8_gemv_fused_fits(M, Kp, tunables().stages), false);
+}
+
 extern "C" int64_t ao_b200_int4_mm_workspace_bytes(int64_t M, int64_t Np, int64_t Kp) {
   // [0, gemv): tickets + partial sums of the tensor-memory GEMV's split-K (row blocks shared by neighbouring CTAs; the
   // tickets must stay zero between launches, so nothing else may ever be written there); [gemv, ...): the prefill
   // GEMM's permuted copy of the activations (M > 16).  The mma.sync kernels reduce inside the CTA and need none.
   const int64_t gemv = ao::int4_gemv_tc_workspace_bytes(Np);
-  return gemv + (M > 16 ? ao::int4_gemm_tc_workspace_bytes(M, Np, Kp) : 0);
+  // (up to 16 rows whether the GEMM is taken depends on the group size too: room for it wherever it may be)
+  return gemv + (M >= 3 && (M > 16 || few_rows_by_gemm(M, Np, Kp, true, true) || few_rows_by_gemm(M, Np, Kp, false, true))
+                     ? ao::int4_gemm_tc_workspace_bytes(M, Np, Kp) : 0);
 }
 
 extern "C" int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed,
@@ -94,10 +119,10 @@ extern "C" int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
   auto s = static_cast<cudaStream_t>(stream);
   auto xb = static_cast<const __nv_bfloat16*>(x);
   auto yb = static_cast<__nv_bfloat16*>(y);
-  if (M > 16 && tunables().gemm_tc) {
-    // prefill: tensor-memory dequant-GEMM; its staging buffer sits after the GEMV region of the workspace
+  if (int4_by_gemm(M, Np, Kp, group_size)) {
+    // tensor-memory dequant-GEMM; its part of the workspace sits after the GEMV region
     const int64_t off = ao::int4_gemv_tc_workspace_bytes(Np);
-    const int e = ao::int4_gemm_tc(x, M, Kx, ldx, packed, scale_and_zero, Np, Kp, group_size, y, N_out, ldy,
+    const int e = ao::int4_gemm_tc(x, M, Kx, ldx, packed, scale_and_zero, Np, Kp, group_size, y, N_out, ldy, nullptr, 0,
                                    workspace ? static_cast<char*>(workspace) + off : nullptr, workspace_bytes - off, s);
     if (e != AO_B200_ERR_WORKSPACE && e != AO_B200_ERR_UNSUPPORTED) return e;
   }
@@ -172,9 +197,7 @@ extern "C" int ao_b200_int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int
 }
 
 extern "C" int64_t ao_b200_int8_mm_workspace_bytes(int64_t M, int64_t Np, int64_t Kp) {
-  // the GEMM's permuted copy of the activations (+ split-K partial sums).  (Routing 2 < M <= 16 batches that do not fit the
-  // GEMV staging through the GEMM was measured SLOWER than the plain strip GEMV: 40 vs 18-28 us on 4096 x 14336.)
-  return M > 16 ? ao::int8_gemm_tc_workspace_bytes(M, Np, Kp) : 0;
+  return int8_by_gemm(M, Np, Kp) ? ao::int8_gemm_tc_workspace_bytes(M, Np, Kp) : 0;
 }
 
 static int int8_args_ok(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Np,
@@ -194,8 +217,8 @@ extern "C" int ao_b200_int8_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
   auto s = static_cast<cudaStream_t>(stream);
   auto xb = static_cast<const __nv_bfloat16*>(x);
   auto yb = static_cast<__nv_bfloat16*>(y);
-  if (M > 16 && tunables().gemm_tc) {
-    const int e = ao::int8_gemm_tc(x, M, Kx, ldx, packed, scale, Np, Kp, y, N_out, ldy, workspace, workspace_bytes, s);
+  if (int8_by_gemm(M, Np, Kp)) {
+    const int e = ao::int8_gemm_tc(x, M, Kx, ldx, packed, scale, Np, Kp, y, N_out, ldy, nullptr, 0, workspace, workspace_bytes, s);
     if (e != AO_B200_ERR_WORKSPACE && e != AO_B200_ERR_UNSUPPORTED) return e;
   }
   for (int64_t m0 = 0; m0 < M; m0 += 16) {
@@ -222,6 +245,22 @@ extern "C" int ao_b200_int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int
                              epilogue, tunables().stages, tunables().pdl != 0, static_cast<cudaStream_t>(stream));
 }
 
+// ---- y = bf16(residual + bf16(x W'^T)) for any number of rows, always by the GEMM ----------------------------------------
+extern "C" int64_t ao_b200_mm_residual_workspace_bytes(int64_t M, int64_t Np, int64_t Kp, int group_size) {
+  return group_size ? ao::int4_gemm_tc_workspace_bytes(M, Np, Kp) : ao::int8_gemm_tc_workspace_bytes(M, Np, Kp);
+}
+extern "C" int ao_b200_mm_residual(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scales, int64_t Np,
+                                   int64_t Kp, int group_size, void* y, int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res,
+                                   void* workspace, int64_t workspace_bytes, void* stream) {
+  AO_CHECK_ARG(x && packed && scales && y && residual && M > 0);
+  AO_CHECK_ARG(Np > 0 && Kp > 0 && Np % 16 == 0 && Kp % 64 == 0 && N_out > 0 && N_out <= Np && ldy >= N_out && ld_res >= N_out);
+  AO_CHECK_ARG(Kx > 0 && Kx <= Kp && Kx % 8 == 0 && ldx % 8 == 0 && ldx >= Kx);
+  AO_CHECK_ARG(ao_aligned(x, 16) && ao_aligned(packed, 16) && ao_aligned(scales, group_size ? 64 : 2) && ao_aligned(y, 2) && ao_aligned(residual, 2));
+  AO_CHECK_ARG(group_size == 0 || Kp % group_size == 0);
+  auto s = static_cast<cudaStream_t>(stream);
+  return group_size ? ao::int4_gemm_tc(x, M, Kx, ldx, packed, scales, Np, Kp, group_size, y, N_out, ldy, residual, ld_res, workspace, workspace_bytes, s)
+                    : ao::int8_gemm_tc(x, M, Kx, ldx, packed, scales, Np, Kp, y, N_out, ldy, residual, ld_res, workspace, workspace_bytes, s);
+}
 
 // ---- serving-loop plumbing (no reference counterpart) ----------------------------------------------------------------
 // Stream-ordered wait on a 32-bit word in pinned host memory: everything enqueued on `stream` after this call starts only

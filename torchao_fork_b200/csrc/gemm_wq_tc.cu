@@ -59,10 +59,11 @@ struct WqParams {
   const uint8_t* xt;         // staged activations [MT * ranks][KU][x_bytes]
   const __nv_bfloat16* scale8;
   __nv_bfloat16* y;
+  const __nv_bfloat16* residual;  // y = bf16(residual + bf16(sum)); may be y itself
   float* part;               // shares of split tiles [workers][2][ranks][NT * 128]
   uint32_t* tickets;         // [tiles][ranks], zeroed by the staging kernel
   uint32_t* status;
-  int64_t N_out, ldy;
+  int64_t N_out, ldy, ld_res;
   int M, NT, BR, KU, MT, w_slots, x_slots, a_slots, n_mma, vec_store;
   uint32_t off_w;            // weight ring
   uint32_t x_bytes;          // one unit of staged activations (and, DEFER, its sums)
@@ -168,6 +169,11 @@ __device__ __forceinline__ void wq_ld_wait() { asm volatile("tcgen05.wait::ld.sy
 // four 8 x 8 blocks of that shape, transposed: lanes 8 i .. 8 i + 7 give the row addresses of block i
 __device__ __forceinline__ void wq_stmatrix_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {  // one rounding per sum
+  uint32_t d;
+  asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
 }
 __device__ __forceinline__ void wq_tma_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)), "l"(map),
@@ -345,17 +351,29 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     const int64_t n0 = nbase + col * 8;
     if (n0 >= p.N_out) return;
     __nv_bfloat16* dst = p.y + (int64_t)m0 * p.ldy + n0;
+    const __nv_bfloat16* res = p.residual == nullptr ? nullptr : p.residual + (int64_t)m0 * p.ld_res + n0;
     const uint32_t src = smem_u32(stage) + col * 16;
     if (p.vec_store && n0 + 8 <= p.N_out) {
 #pragma unroll 4
-      for (int m = th >> 4; m < rows; m += threads >> 4) *reinterpret_cast<uint4*>(dst + m * p.ldy) = lds128(src + m * kWqPitch);
+      for (int m = th >> 4; m < rows; m += threads >> 4) {
+        uint4 v = lds128(src + m * kWqPitch);
+        if (res != nullptr) {
+          const uint4 r = *reinterpret_cast<const uint4*>(res + m * p.ld_res);
+          v = make_uint4(add_bf16x2(r.x, v.x), add_bf16x2(r.y, v.y), add_bf16x2(r.z, v.z), add_bf16x2(r.w, v.w));
+        }
+        *reinterpret_cast<uint4*>(dst + m * p.ldy) = v;
+      }
     } else {
       for (int m = th >> 4; m < rows; m += threads >> 4) {
         const uint4 v = lds128(src + m * kWqPitch);
         const uint32_t vv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          if (n0 + e < p.N_out) dst[m * p.ldy + e] = __ushort_as_bfloat16((unsigned short)(vv[e >> 1] >> (16 * (e & 1))));
+        for (int e = 0; e < 8; ++e) {
+          if (n0 + e >= p.N_out) continue;
+          __nv_bfloat16 o = __ushort_as_bfloat16((unsigned short)(vv[e >> 1] >> (16 * (e & 1))));
+          if (res != nullptr) o = __float2bfloat16_rn(__bfloat162float(res[m * p.ld_res + e]) + __bfloat162float(o));
+          dst[m * p.ldy + e] = o;
+        }
       }
     }
   };
@@ -473,34 +491,39 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     // so with a short odd ring the A slot is waited for first.  (A longer ring cannot be overtaken while one MMA warp keeps the
     // sets at most a_slots + 1 units apart; with two the ring is even.)
     const bool a_first = (p.w_slots & 1) && p.w_slots < a_slots + 2;
-    for (int u = u0 + set; u < u1; u += 2) {
-      if (a_first && !wq_wait(&adone[a.slot], a.use ^ 1u, dead)) break;
-      if (!wq_wait(&wfull[w.slot], w.use, dead)) break;
-      const uint32_t wt = w0_u + w.slot * kWSlot;
+    // DEFER: the words of the next unit are fetched while this unit's store to tensor memory is on its way (28672 x 8192, 16 rows: 46.4 -> 44.1
+    // us).  The others are bound by the conversions or the MMAs and do best announcing first (int8 8192 x 8192, 2048 rows: 217 against 223 us).
+    constexpr int kWords = kI8 ? 16 : 8, kSzn = (kI8 || DEFER) ? 1 : kSzWords / 16;
+    uint32_t wd[kWords], sz[kSzn][2];
+    auto fetch = [&](int u) {
+      if (u >= u1) return true;
+      if (a_first && !wq_wait(&adone[a.slot], a.use ^ 1u, dead)) return false;
+      if (!wq_wait(&wfull[w.slot], w.use, dead)) return false;
+      const uint32_t wt = w0_u + w.slot * kWSlot, st = s0_u + w.slot * kWSlot;
+#pragma unroll
+      for (int i = 0; i < kWords / 4; ++i) {
+        const uint4 v = lds128(wt + i * 512);
+        wd[4 * i] = v.x, wd[4 * i + 1] = v.y, wd[4 * i + 2] = v.z, wd[4 * i + 3] = v.w;
+      }
+      if constexpr (!kI8 && !DEFER) {
+#pragma unroll
+        for (int h = 0; h < kSzn; ++h) {
+          sz[h][0] = lds32(st + h * 64);
+          sz[h][1] = lds32(st + h * 64 + 32);
+        }
+      }
+      return true;
+    };
+    bool ok = fetch(u0 + set);
+    for (int u = u0 + set; u < u1 && ok; u += 2) {
       uint32_t r[32];
       if constexpr (kI8) {
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {  // 32-k quarters of the unit; lane chunk: words (row g, k 0-3), (g+8, k 0-3), (g, k 4-7), (g+8, k 4-7)
-          const uint4 w4 = lds128(wt + q4 * 512);
-          const uint32_t wd[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int hrow = j & 1, i0 = 2 * (j >> 1);
-            u8x4_to_bf16x2x2(wd[j], r[2 * (4 * q4 + i0) + hrow], r[2 * (4 * q4 + i0 + 1) + hrow]);
-          }
+        for (int j = 0; j < 16; ++j) {  // 32-k quarters of the unit; lane chunk: words (row g, k 0-3), (g+8, k 0-3), (g, k 4-7), (g+8, k 4-7)
+          const int q4 = j >> 2, hrow = j & 1, i0 = 2 * ((j >> 1) & 1);
+          u8x4_to_bf16x2x2(wd[j], r[2 * (4 * q4 + i0) + hrow], r[2 * (4 * q4 + i0 + 1) + hrow]);
         }
       } else {
-        const uint4 wa = lds128(wt), wb = lds128(wt + 512);
-        const uint32_t wd[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-        uint32_t sz[DEFER ? 1 : kSzWords / 16][2];
-        if constexpr (!DEFER) {
-          const uint32_t st = s0_u + w.slot * kWSlot;
-#pragma unroll
-          for (int h = 0; h < kSzWords / 16; ++h) {
-            sz[h][0] = lds32(st + h * 64);
-            sz[h][1] = lds32(st + h * 64 + 32);
-          }
-        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {  // word j: row g + 8 (j & 1), 32-k quarter j >> 1 of the unit
           const int q4 = j >> 1, hrow = j & 1;
@@ -509,7 +532,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
 #pragma unroll
             for (int i = 0; i < 4; ++i) asm("lop3.b32 %0, %1, 0x000f000f, 0x43004300, 0xea;" : "=r"(o[i]) : "r"(wd[j] >> (4 * i)));  // 128 + q
           } else {
-            const uint32_t szw = sz[q4 * (kSzWords / 16) / 4][hrow];
+            const uint32_t szw = sz[q4 * kSzn / 4][hrow];
             dequant_word(wd[j], __byte_perm(szw, 0, 0x1010), __byte_perm(szw, 0, 0x3232), o);
           }
 #pragma unroll
@@ -518,16 +541,20 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&wempty[w.slot]);  // everything that this warp reads of the slot is in registers
-      if (!wq_wait(&adone[a.slot], a.use ^ 1u, dead)) break;  // the MMAs that read this A slot have retired
+      ok = wq_wait(&adone[a.slot], a.use ^ 1u, dead);  // the MMAs that read this A slot have retired
+      if (!ok) break;
       wq_fence_after();
       wq_st_16x128b_x8(taddr0 + a.slot * 64, r);
       wq_st_16x128b_x8(taddr0 + a.slot * 64 + 32, r + 16);
+      uint64_t* full = &afull[a.slot];
+      w.step(2, p.w_slots);
+      a.step(2, a_slots);
+      if (DEFER && !a_first) ok = fetch(u + 2);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       wq_fence_before();
       __syncwarp();
-      if (lane == 0) wq_arrive_leader<PAIR>(&afull[a.slot]);
-      w.step(2, p.w_slots);
-      a.step(2, a_slots);
+      if (lane == 0) wq_arrive_leader<PAIR>(full);
+      if (!DEFER || a_first) ok = fetch(u + 2);  // (a_first waits for MMAs: not before this unit is announced)
     }
   } else {
     // ---- epilogue ----
@@ -547,7 +574,8 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
 #pragma unroll
         for (int i = 0; i < 16; ++i) acc[i] = 0.f;
         for (; u < ue; ++u) {
-          ok = wq_wait(&wfull[w.slot], w.use, dead) && wq_wait(&xfull[x.slot], x.use, dead) && wq_wait(&xdone[x.slot], x.use, dead);
+          const bool rw = mbar_try_wait(&wfull[w.slot], w.use), rx = mbar_try_wait(&xfull[x.slot], x.use), rd = mbar_try_wait(&xdone[x.slot], x.use);
+          ok = (rw || wq_wait(&wfull[w.slot], w.use, dead)) && (rx || wq_wait(&xfull[x.slot], x.use, dead)) && (rd || wq_wait(&xdone[x.slot], x.use, dead));
           if (!ok) break;
           wq_fence_after();
           // parameters of rows 32 warp + lane / 4 + 8 i, sums of columns 2 (lane % 4) + {0, 1, 8, 9}
@@ -815,7 +843,7 @@ static int wq_stage(const void* x, int64_t M, int64_t Kx, int64_t ldx, const WqP
 
 // x [M][ldx] bf16 (first Kx columns valid), y [M][ldy] bf16.  G == 0: int8 weights (`sz` is then the bf16 per-row scale)
 static int wq_gemm(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np, int64_t Kp, int G, void* y,
-                   int64_t N_out, int64_t ldy, void* workspace, int64_t workspace_bytes, cudaStream_t s) {
+                   int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res, void* workspace, int64_t workspace_bytes, cudaStream_t s) {
   WqPlan w;
   if (!wq_plan(M, Np, Kp, G != 0, w) || wq_encode_fn() == nullptr) return AO_B200_ERR_UNSUPPORTED;
   if (workspace == nullptr || workspace_bytes < w.bytes || !ao_aligned(workspace, 16)) return AO_B200_ERR_WORKSPACE;
@@ -833,7 +861,9 @@ static int wq_gemm(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void
   p.y = static_cast<__nv_bfloat16*>(y);
   p.N_out = N_out;
   p.ldy = ldy;
-  p.vec_store = (ldy % 8 == 0 && ao_aligned(y, 16)) ? 1 : 0;
+  p.residual = static_cast<const __nv_bfloat16*>(residual);
+  p.ld_res = ld_res;
+  p.vec_store = (ldy % 8 == 0 && ao_aligned(y, 16) && ld_res % 8 == 0 && ao_aligned(residual, 16)) ? 1 : 0;
   p.M = (int)M;
   p.NT = w.NT;
   p.BR = w.BR;
@@ -873,15 +903,15 @@ int64_t int8_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp) {
 }
 
 int int4_gemm_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np, int64_t Kp, int G, void* y,
-                 int64_t N_out, int64_t ldy, void* workspace, int64_t workspace_bytes, cudaStream_t s) {
+                 int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res, void* workspace, int64_t workspace_bytes, cudaStream_t s) {
   if (!(G == 32 || G == 64 || G == 128 || G == 256)) return AO_B200_ERR_UNSUPPORTED;
-  return wq_gemm(x, M, Kx, ldx, packed, sz, Np, Kp, G, y, N_out, ldy, workspace, workspace_bytes, s);
+  return wq_gemm(x, M, Kx, ldx, packed, sz, Np, Kp, G, y, N_out, ldy, residual, ld_res, workspace, workspace_bytes, s);
 }
 
 // int8 weights: packed = strip-major biased int8 (Np % 128 == 0), scale bf16 [N_out]
 int int8_gemm_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Np, int64_t Kp, void* y, int64_t N_out,
-                 int64_t ldy, void* workspace, int64_t workspace_bytes, cudaStream_t s) {
-  return wq_gemm(x, M, Kx, ldx, packed, scale, Np, Kp, 0, y, N_out, ldy, workspace, workspace_bytes, s);
+                 int64_t ldy, const void* residual, int64_t ld_res, void* workspace, int64_t workspace_bytes, cudaStream_t s) {
+  return wq_gemm(x, M, Kx, ldx, packed, scale, Np, Kp, 0, y, N_out, ldy, residual, ld_res, workspace, workspace_bytes, s);
 }
 
 }  // namespace ao

@@ -640,6 +640,19 @@ static int launch_fused(GemvFusedParams& p, const FusedPlan& pl, bool pdl, cudaS
   return ao_launch_status();
 }
 
+// whether the activations of a call fit this kernel's staging
+bool int4_gemv_fused_fits(int64_t M, int64_t Kp, int G, int max_stages) {
+  FusedPlan pl;
+  const int MT = M <= 8 ? 1 : 2;
+  switch (G) {
+    case 32: return plan_fused<32>((int)M, MT, Kp, max_stages, pl);
+    case 64: return plan_fused<64>((int)M, MT, Kp, max_stages, pl);
+    case 128: return plan_fused<128>((int)M, MT, Kp, max_stages, pl);
+    case 256: return plan_fused<256>((int)M, MT, Kp, max_stages, pl);
+  }
+  return false;
+}
+
 // returns AO_B200_ERR_WORKSPACE when the shape does not fit this kernel (caller may fall back)
 int int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np,
                     int64_t Kp, int G, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps,

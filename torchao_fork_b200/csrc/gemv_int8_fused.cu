@@ -538,6 +538,12 @@ static int launch8(Gemv8Params& p, const Plan8& pl, bool pdl, cudaStream_t s) {
   return ao_launch_status();
 }
 
+// whether the activations of a call fit this kernel's staging
+bool int8_gemv_fused_fits(int64_t M, int64_t Kp, int max_stages) {
+  Plan8 pl;
+  return plan8((int)M, M <= 8 ? 1 : 2, Kp, max_stages, pl);
+}
+
 // returns AO_B200_ERR_WORKSPACE when the activations do not fit the staging (caller falls back)
 int int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Np,
                     int64_t Kp, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps, const void* residual,
