@@ -217,6 +217,17 @@ __global__ void __launch_bounds__(kGroup * 32) decode_attn_fused_kernel(
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = kvh * kGroup + warp;
   const int heads = H + 2 * Hkv;
+  {
+    // the cached rows of this CTA's share on their way to L2 while the projection in front finishes (a prefetch of rows that are
+    // still being written, or of another position's share, costs time and nothing else)
+    const int p = __ldcg(input_pos), ch = (p + n_split) / n_split, f0 = split * ch, f1 = min(p, f0 + ch);
+    const int64_t base = (((int64_t)b * Hkv + kvh) * S + f0) * (hd * 2);
+    if (p >= 0 && p < S)
+      for (int i = threadIdx.x; i < (f1 - f0) * 4; i += kGroup * 32) {   // 128-byte lines: two of a key row, two of a value row
+        const char* at = reinterpret_cast<const char*>(i & 1 ? v_cache : k_cache) + base + (int64_t)(i >> 1) * 128;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
+      }
+  }
   grid_dependency_wait();
   const int pos = *input_pos;
   const int len = pos + 1;
@@ -254,39 +265,53 @@ __global__ void __launch_bounds__(kGroup * 32) decode_attn_fused_kernel(
     qv[2] = __uint_as_float(r.y << 16) * scale;
     qv[3] = __uint_as_float(r.y & 0xFFFF0000u) * scale;
   }
-  // The walk is latency-bound (a few KB per CTA), so it is organised for memory-level parallelism: a block of 32 cache
-  // positions per trip, lane j owns position jb + j for q.K (its whole 256-byte K row: 16 independent 16-byte loads, no
-  // shuffles), the V rows of the block (one coalesced 8-byte load per lane per position) are requested BEFORE the scores
-  // are reduced, and P.V broadcasts the probabilities lane by lane.  One DRAM round trip per 32 positions instead of
-  // one per 4.
+  // The walk is a few KB per CTA, organised for loads in flight and few L1 wavefronts: a block of 32 cache positions per trip,
+  // sixteen lanes to a K row (a 16-byte load per lane: two whole rows, 4 wavefronts, per warp instruction; a whole row per lane
+  // was 32 wavefronts per instruction, which paced batches: a token of 64 sequences through two layers of 32 / 8 heads at 300
+  // positions 475 -> 370 us in all, of 8 sequences 213 -> 197), the V rows of the block (one coalesced 8-byte load per lane per position) requested BEFORE the scores are reduced.
+  // The sixteen partial sums of a lane are added across the half-warp by halving: lane l ends with row 2 (l & 15) + (l >> 4).
+  const int l16 = lane & 15, half_id = lane >> 4, own = 2 * l16 + half_id;
   __shared__ __align__(16) float q_s[kGroup][hd];
   *reinterpret_cast<float4*>(&q_s[warp][lane * 4]) = make_float4(qv[0], qv[1], qv[2], qv[3]);
   __syncwarp();
+  float qk[8];   // this lane's 8 columns of q
+  {
+    const float4 qa = *reinterpret_cast<const float4*>(&q_s[warp][8 * l16]);
+    const float4 qb = *reinterpret_cast<const float4*>(&q_s[warp][8 * l16 + 4]);
+    qk[0] = qa.x, qk[1] = qa.y, qk[2] = qa.z, qk[3] = qa.w, qk[4] = qb.x, qk[5] = qb.y, qk[6] = qb.z, qk[7] = qb.w;
+  }
   float m = -INFINITY, l = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
   for (int jb = j0; jb < j1; jb += 32) {
     const int cnt = min(32, j1 - jb);
-    const bool valid = lane < cnt;
+    const bool valid = own < cnt;
     uint4 kk[16];
     {
-      const uint4* krow = reinterpret_cast<const uint4*>(kb - lane * 4 + (int64_t)(jb + (valid ? lane : 0)) * hd);
+      const __nv_bfloat16* kr = kb - lane * 4 + l16 * 8 + (int64_t)jb * hd;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) kk[i] = krow[i];
+      for (int i = 0; i < 16; ++i) kk[i] = *reinterpret_cast<const uint4*>(kr + (int64_t)min(2 * i + half_id, cnt - 1) * hd);
     }
     uint2 vr[32];
 #pragma unroll
     for (int jj = 0; jj < 32; ++jj)
       vr[jj] = jj < cnt ? *reinterpret_cast<const uint2*>(vb + (int64_t)(jb + jj) * hd) : make_uint2(0u, 0u);
-    float sc = 0.f;
+    float part[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const float4 qa = *reinterpret_cast<const float4*>(&q_s[warp][8 * i]);
-      const float4 qb = *reinterpret_cast<const float4*>(&q_s[warp][8 * i + 4]);
-      sc += qa.x * __uint_as_float(kk[i].x << 16) + qa.y * __uint_as_float(kk[i].x & 0xFFFF0000u) +
-            qa.z * __uint_as_float(kk[i].y << 16) + qa.w * __uint_as_float(kk[i].y & 0xFFFF0000u) +
-            qb.x * __uint_as_float(kk[i].z << 16) + qb.y * __uint_as_float(kk[i].z & 0xFFFF0000u) +
-            qb.z * __uint_as_float(kk[i].w << 16) + qb.w * __uint_as_float(kk[i].w & 0xFFFF0000u);
+    for (int i = 0; i < 16; ++i)
+      part[i] = (qk[0] * __uint_as_float(kk[i].x << 16) + qk[1] * __uint_as_float(kk[i].x & 0xFFFF0000u)) +
+                (qk[2] * __uint_as_float(kk[i].y << 16) + qk[3] * __uint_as_float(kk[i].y & 0xFFFF0000u)) +
+                (qk[4] * __uint_as_float(kk[i].z << 16) + qk[5] * __uint_as_float(kk[i].z & 0xFFFF0000u)) +
+                (qk[6] * __uint_as_float(kk[i].w << 16) + qk[7] * __uint_as_float(kk[i].w & 0xFFFF0000u));
+#pragma unroll
+    for (int o = 8; o; o >>= 1) {
+      const bool up = (l16 & o) != 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < o) {
+          const float send = up ? part[i] : part[i + o], keep = up ? part[i + o] : part[i];
+          part[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
     }
-    if (!valid) sc = -INFINITY;
+    const float sc = valid ? part[0] : -INFINITY;
     float mb = sc;
 #pragma unroll
     for (int o = 16; o; o >>= 1) mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, o));
@@ -301,7 +326,7 @@ __global__ void __launch_bounds__(kGroup * 32) decode_attn_fused_kernel(
     for (int e = 0; e < 4; ++e) acc[e] *= corr;
 #pragma unroll
     for (int jj = 0; jj < 32; ++jj) {
-      const float pw = __shfl_sync(0xffffffffu, pj, jj);  // 0 beyond cnt
+      const float pw = __shfl_sync(0xffffffffu, pj, (jj >> 1) + 16 * (jj & 1));  // 0 beyond cnt
       acc[0] += pw * __uint_as_float(vr[jj].x << 16);
       acc[1] += pw * __uint_as_float(vr[jj].x & 0xFFFF0000u);
       acc[2] += pw * __uint_as_float(vr[jj].y << 16);

@@ -218,6 +218,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) window_attention_tc_kernel(WinP
       }
       __syncwarp();
     }
+    // the last arrival of the tensor core: nothing of this CTA may come after its shared memory has been given back
+    tc_wait(&vdone[(steps - 1) & 1], ((steps - 1) >> 1) & 1, dead);
   } else if (warp >= 8) {
     // ---- loads ----
     const int64_t sl = a.slot[first];
