@@ -288,6 +288,13 @@ AO_B200_API int ao_b200_decode_attention_fused_q8(const void* qkv, const void* f
 /* FeedForward gate (model.py:486): out = bf16( bf16(silu(gate)) * up ), gate_up bf16 [B][2*I] = [w1 x | w3 x]. */
 AO_B200_API int ao_b200_silu_mul(const void* gate_up, void* out, int64_t B, int64_t I, void* stream);
 
+/* The same two for rows of a prompt.
+ * apply_rotary_emb: x bf16 [B][T][H][head_dim] (strides in elements, multiples of 8), freqs_cis bf16 [T][head_dim / 2][2],
+ * y packed; head_dim % 8 == 0.   y[i] = bf16( bf16(silu(gate[i])) * up[i] ), count % 8 == 0.   All 16-byte aligned. */
+AO_B200_API int ao_b200_rotary(const void* x, int64_t stride_b, int64_t stride_t, int64_t stride_h, const void* freqs_cis, void* y, int64_t B,
+                               int64_t T, int64_t H, int64_t head_dim, void* stream);
+AO_B200_API int ao_b200_silu_mul_rows(const void* gate, const void* up, void* y, int64_t count, void* stream);
+
 /* sample (generate.py:79-100: logits_to_probs + multinomial_sample_one_no_sync) in one launch:
  *   lg = float(logits) / max(temperature, 1e-5); entries below the top_k-th largest -> -inf (ties kept, top_k <= 0 or
  *   >= V: keep all); probs = softmax(lg); next_tok[b] = argmax_i probs[i] / noise[b][i]  (first index on ties).

@@ -13,6 +13,8 @@ import torch.nn as nn
 import torch.nn.functional as F
 from torch import Tensor
 
+from ... import _lib
+from ...ops import _on, runs_eagerly
 from ...utils import find_multiple
 
 
@@ -84,6 +86,30 @@ transformer_configs = {
 from ..cache import AffineQuantizedKVCache, KVCache  # noqa: E402,F401  (the cache classes of every model family live together)
 
 
+def _rows_by_kernel(x: Tensor, *others: Tensor) -> bool:
+    """Whether an element-wise step of the block may be one kernel launch: bf16 on one CUDA device, in whole aligned pieces, and nobody
+    who would see the single operations (autograd, tracers, modes)."""
+    if not (x.is_cuda and x.dtype is torch.bfloat16 and x.numel() > 0 and runs_eagerly(x, *others)) or torch.compiler.is_compiling():
+        return False
+    if torch._C._len_torch_function_stack() != 0:
+        return False
+    return all(t.device == x.device and t.dtype is torch.bfloat16 and t.data_ptr() % 16 == 0 and not (t.requires_grad and torch.is_grad_enabled())
+               for t in (x, *others))
+
+
+def _stream(x: Tensor) -> int:
+    return torch._C._cuda_getCurrentRawStream(x.device.index)
+
+
+def silu_mul(gate: Tensor, up: Tensor) -> Tensor:
+    if _rows_by_kernel(gate, up) and gate.shape == up.shape and gate.is_contiguous() and up.is_contiguous() and gate.numel() % 8 == 0:
+        out = torch.empty_like(gate)
+        with _on(gate.device.index):
+            _lib.check(_lib.lib().ao_b200_silu_mul_rows(gate.data_ptr(), up.data_ptr(), out.data_ptr(), gate.numel(), _stream(gate)), "silu_mul_rows")
+        return out
+    return F.silu(gate) * up
+
+
 class RMSNorm(nn.Module):
     """reference: model.py:489-503 — normalise in fp32, cast back, multiply by the weight."""
 
@@ -93,6 +119,15 @@ class RMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(dim))
 
     def forward(self, x: Tensor) -> Tensor:
+        w = self.weight
+        dim = x.shape[-1] if x.dim() else 0
+        if (type(w) is nn.Parameter and _rows_by_kernel(x, w.data) and not (w.requires_grad and torch.is_grad_enabled()) and x.is_contiguous()
+                and w.shape == (dim,) and w.is_contiguous() and dim % 8 == 0 and dim <= 12272):   # a row in 48 KB of shared memory
+            out = torch.empty_like(x)
+            with _on(x.device.index):
+                _lib.check(_lib.lib().ao_b200_rmsnorm(x.data_ptr(), None, w.data_ptr(), None, out.data_ptr(), x.numel() // dim, dim, self.eps,
+                                                      _stream(x)), "rmsnorm")
+            return out
         xf = x.float()
         return (xf * torch.rsqrt(xf.square().mean(-1, keepdim=True) + self.eps)).type_as(x) * self.weight
 
@@ -124,6 +159,13 @@ def precompute_freqs_cis(seq_len, n_elem, base=10000, dtype=torch.bfloat16, use_
 
 def apply_rotary_emb(x: Tensor, freqs_cis: Tensor) -> Tensor:
     """x [B][T][H][hd], rotation of consecutive pairs in fp32 (reference: model.py:547-559)."""
+    if (x.dim() == 4 and _rows_by_kernel(x, freqs_cis) and x.stride(3) == 1 and all(s % 8 == 0 for s in x.stride()[:3]) and x.shape[3] % 8 == 0
+            and freqs_cis.is_contiguous() and freqs_cis.numel() == x.shape[1] * x.shape[3]):
+        b, t, h, d = x.shape
+        out = torch.empty(b, t, h, d, dtype=x.dtype, device=x.device)
+        with _on(x.device.index):
+            _lib.check(_lib.lib().ao_b200_rotary(x.data_ptr(), *x.stride()[:3], freqs_cis.data_ptr(), out.data_ptr(), b, t, h, d, _stream(x)), "rotary")
+        return out
     xs = x.float().reshape(*x.shape[:-1], -1, 2)
     fc = freqs_cis.view(1, xs.size(1), 1, xs.size(3), 2)
     out = torch.stack([xs[..., 0] * fc[..., 0] - xs[..., 1] * fc[..., 1],
@@ -179,7 +221,7 @@ class FeedForward(nn.Module):
         self.w2 = nn.Linear(config.intermediate_size, config.dim, bias=False)
 
     def forward(self, x):
-        return self.w2(F.silu(self.w1(x)) * self.w3(x))
+        return self.w2(silu_mul(self.w1(x), self.w3(x)))
 
 
 class TransformerBlock(nn.Module):

@@ -1,0 +1,67 @@
+// What the Llama block does between its products for rows of a prompt, one pass each: rotation of queries and keys, SiLU * up (the
+// norm is rmsnorm_kernel of decode_ops.cu).  As tensor operations these were ten passes and more over fp32 copies: 700 tokens through two
+// Mistral-7B layers and the output product took 1956 us of which about 850 were such passes, now 1036 in all.  Bound by memory;
+// 16 bytes per thread.  The roundings are those of the single operations: fp32 products rounded before they are added (no fused
+// multiply-add), silu rounded to bf16 before its product.
+#include <cuda_bf16.h>
+
+#include "../../include/ao_b200.h"
+#include "common.cuh"
+
+namespace ao {
+namespace {
+
+__device__ __forceinline__ float lo_f(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
+__device__ __forceinline__ uint32_t pack_rn(float a, float b) { return float_to_bf16_bits(a) | (float_to_bf16_bits(b) << 16); }
+
+__device__ __forceinline__ uint32_t rotate_pair(uint32_t x, uint32_t cs) {
+  const float a = lo_f(x), b = hi_f(x), c = lo_f(cs), s = hi_f(cs);
+  return pack_rn(__fsub_rn(__fmul_rn(a, c), __fmul_rn(b, s)), __fadd_rn(__fmul_rn(b, c), __fmul_rn(a, s)));
+}
+// x [B][T][H][8 n8] (any strides that are whole 16-byte pieces) -> y, packed; freqs [T][8 n8]: cos, sin of every pair
+__global__ void __launch_bounds__(256) rotary_kernel(const uint4* __restrict__ x, int64_t sb, int64_t st, int64_t sh, const uint4* __restrict__ freqs,
+                                                     uint4* __restrict__ y, int T, int H, int n8, int64_t total) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= total) return;
+  const int c = (int)(i % n8);
+  const int64_t r = i / n8;
+  const int h = (int)(r % H);
+  const int64_t bt = r / H;
+  const int t = (int)(bt % T);
+  const uint4 v = x[bt / T * sb + t * st + h * sh + c], f = freqs[(int64_t)t * n8 + c];
+  y[i] = make_uint4(rotate_pair(v.x, f.x), rotate_pair(v.y, f.y), rotate_pair(v.z, f.z), rotate_pair(v.w, f.w));
+}
+
+__device__ __forceinline__ float silu_f(float g) { return __uint_as_float(float_to_bf16_bits(g / (1.f + expf(-g))) << 16); }
+__device__ __forceinline__ uint32_t silu_mul_pair(uint32_t g, uint32_t u) { return pack_rn(silu_f(lo_f(g)) * lo_f(u), silu_f(hi_f(g)) * hi_f(u)); }
+__global__ void __launch_bounds__(256) silu_mul_rows_kernel(const uint4* __restrict__ gate, const uint4* __restrict__ up, uint4* __restrict__ y, int64_t n8) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n8) return;
+  const uint4 g = gate[i], u = up[i];
+  y[i] = make_uint4(silu_mul_pair(g.x, u.x), silu_mul_pair(g.y, u.y), silu_mul_pair(g.z, u.z), silu_mul_pair(g.w, u.w));
+}
+
+}  // namespace
+}  // namespace ao
+
+extern "C" int ao_b200_rotary(const void* x, int64_t stride_b, int64_t stride_t, int64_t stride_h, const void* freqs_cis, void* y, int64_t B, int64_t T,
+                              int64_t H, int64_t head_dim, void* stream) {
+  AO_CHECK_ARG(x && freqs_cis && y && B > 0 && T > 0 && H > 0 && head_dim > 0 && head_dim % 8 == 0);
+  AO_CHECK_ARG(stride_b % 8 == 0 && stride_t % 8 == 0 && stride_h % 8 == 0 && ao_aligned(x, 16) && ao_aligned(freqs_cis, 16) && ao_aligned(y, 16));
+  const int64_t total = B * T * H * (head_dim / 8), blocks = (total + 255) / 256;
+  if (T > 2147483647 || H > 2147483647 || blocks > 2147483647) return AO_B200_ERR_UNSUPPORTED;
+  ao::rotary_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const uint4*>(x), stride_b / 8, stride_t / 8, stride_h / 8, static_cast<const uint4*>(freqs_cis), static_cast<uint4*>(y), (int)T, (int)H,
+      (int)(head_dim / 8), total);
+  return ao_launch_status();
+}
+
+extern "C" int ao_b200_silu_mul_rows(const void* gate, const void* up, void* y, int64_t count, void* stream) {
+  AO_CHECK_ARG(gate && up && y && count > 0 && count % 8 == 0 && ao_aligned(gate, 16) && ao_aligned(up, 16) && ao_aligned(y, 16));
+  const int64_t n8 = count / 8, blocks = (n8 + 255) / 256;
+  if (blocks > 2147483647) return AO_B200_ERR_UNSUPPORTED;
+  ao::silu_mul_rows_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint4*>(gate), static_cast<const uint4*>(up),
+                                                                                        static_cast<uint4*>(y), n8);
+  return ao_launch_status();
+}
