@@ -213,8 +213,8 @@ class DecodeEngine:
         ws_bytes = max(l.workspace_bytes(B) for l in lins)
         self.ws = torch.zeros(max(ws_bytes, 16), dtype=torch.uint8, device=dev)
         # the GEMM that adds the residual keeps nothing between launches; the tickets in self.ws have to stay zero, so it has its own
-        self.res_ws = torch.empty(max([16] + [l[k].residual_workspace_bytes(B) for l in self.layers for k in ("wo", "w2")]) if self.parts else 16,
-                                  dtype=torch.uint8, device=dev)
+        self.res_ws = torch.empty(max([16] + [l[k].residual_workspace_bytes(B) for l in self.layers for k in ("wo", "w2")]),
+                                  dtype=torch.uint8, device=dev) if self.parts else None
         # sequence splits of the decode attention: one 32-position block per split up to S = 1024 (a block is one DRAM
         # round trip; fewer splits = fewer CTAs and a cheaper merge), <= 32 (the merge keeps one split per lane)
         self.n_split = max(1, min(32, -(-self.S // 32)))
