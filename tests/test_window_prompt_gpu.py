@@ -1,0 +1,86 @@
+"""Attention of prompt portions (ao_lm_window_attention_prompt) at the sizes of real layers, through the plan's own tiles: many tiles of
+keys per tile of rows, windows shorter and longer than the run, earlier positions in the ring, last tiles of every kind, one and two
+maps, and a head too large for anything but the plainest tiling.  Against float64.
+
+Bound: queries are rounded to bf16 in front of the product (relative 2^-9 each, near uniform: 2^-9 / sqrt(3) of the scores' norm, which
+moves a weight by |s| times that: below 0.4 % at scores of a few units) and the result is rounded once (2^-9 / sqrt(3)): 1 % holds both.
+Equal calls give equal bits: nothing is summed in an order that depends on time."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+from torchao_fork_b200 import _lib  # noqa: E402
+
+BF16 = 0
+
+
+def _reference(q, k, v, past, window, keep, lam):
+    n, H, maps, d = q.shape
+    G = k.shape[1]
+    i, j = torch.arange(past, past + n, device="cuda")[:, None], torch.arange(past + n, device="cuda")[None, :]
+    hidden = (j > i) | ((i - j >= window) & (j >= keep))
+    out = []
+    for h in range(H):
+        g = h // (H // G)
+        parts = [(q[:, h, m].double() @ k[:, g, m].double().t() * d ** -0.5).masked_fill(hidden, -torch.inf).softmax(-1) @ v[:, g].double()
+                 for m in range(maps)]
+        y = parts[0]
+        if maps == 2:
+            y = y - lam * parts[1]
+            y = y * torch.rsqrt(y.square().mean(-1, keepdim=True) + 1e-6)
+        out.append(y)
+    return torch.cat(out, 1)
+
+
+def _run(q, k, v, past, window, keep, lam):
+    n, H, maps, d = q.shape
+    G, dv = k.shape[1], v.shape[-1]
+    L, p = _lib.lm(), lambda t: t.data_ptr()
+    tile = ctypes.c_int()
+    _lib.lm_check(L.ao_lm_window_attention_prompt_plan(BF16, maps, H, G, d, dv, ctypes.byref(tile)), "plan")
+    assert tile.value > 0
+    ring = max(window, 1) + 37
+    i32 = lambda t: t.to(torch.int32).cuda()  # noqa: E731
+    # the positions before the run as the append leaves them: the last `ring` in the ring, the kept ones beside it, rubbish elsewhere
+    rk, rv = (torch.full((2, ring, t[0].numel()), 50.0, dtype=torch.bfloat16, device="cuda") for t in (k, v))
+    fk, fv = (torch.full((2, keep + 1, t[0].numel()), 50.0, dtype=torch.bfloat16, device="cuda") for t in (k, v))
+    old = torch.arange(max(0, past - ring), past, device="cuda")
+    kept = torch.arange(min(past, keep + 1), device="cuda")
+    for store, first, t in ((rk, fk, k), (rv, fv, v)):
+        store[1, old % ring] = t[old].flatten(1)
+        first[1, kept] = t[kept].flatten(1)
+    kn, vn = k[past:].contiguous(), v[past:].contiguous()
+    first = torch.arange(0, n, tile.value)
+    back = torch.arange(n)
+    slot, pos, bk = i32(back * 0 + 1), i32(back + past), i32(back)
+    tf, tc = i32(first), i32((n - first).clamp(max=tile.value))
+    out = torch.full((n, H * dv), 9.0, dtype=torch.bfloat16, device="cuda")
+    _lib.lm_check(L.ao_lm_window_attention_prompt(
+        p(q), p(kn), p(vn), p(rk), p(rv), p(fk), p(fv), ring, keep + 1, BF16, p(slot), p(pos), p(bk), p(tf), p(tc), tf.numel(), maps, H, G, d, dv, window,
+        keep, d ** -0.5, lam, int(maps == 2), 1e-6, 1.0, p(out), H * dv, torch.cuda.current_stream().cuda_stream), "prompt")
+    torch.cuda.synchronize()
+    return out
+
+
+@pytest.mark.parametrize("maps,d,dv,H,G", [(1, 128, 128, 4, 2), (2, 64, 128, 2, 2), (2, 64, 128, 4, 1), (1, 256, 128, 2, 1), (2, 48, 96, 2, 1)])
+@pytest.mark.parametrize("n,past,window,keep", [
+    (520, 0, 4096, 0), (520, 0, 512, 0), (129, 0, 60, 3), (255, 0, 4096, 0), (127, 1, 512, 0), (128, 300, 512, 0), (161, 127, 4096, 5),
+    (1, 700, 512, 4), (2, 129, 100, 0), (383, 640, 512, 0), (130, 1000, 512, 2), (640, 63, 129, 1)])
+def test_prompt_portions_of_real_sizes(maps, d, dv, H, G, n, past, window, keep):
+    gen = torch.Generator(device="cuda").manual_seed(n + past + d)
+    q = torch.randn(n, H, maps, d, generator=gen, device="cuda") * 1.5
+    k, v = (torch.randn(past + n, G, *w, generator=gen, device="cuda").to(torch.bfloat16) for w in ((maps, d), (dv,)))
+    # from one stretch of keys to the next the scores rise, for some rows only: sums that were started have to be rescaled
+    k[(past + n) // 2 :, :, :, 0] += 6
+    q[::3, :, :, 0] = 12
+    ref, got = _reference(q, k, v, past, window, keep, 0.4), _run(q, k, v, past, window, keep, 0.4)
+    rows = ((got.double() - ref).square().sum(1) / ref.square().sum(1)).sqrt()
+    assert rows.max().item() < 0.02 and ((got.double() - ref).norm() / ref.norm()).item() < 0.01, rows.topk(min(5, n))
+    for _ in range(2):
+        assert torch.equal(_run(q, k, v, past, window, keep, 0.4), got)
