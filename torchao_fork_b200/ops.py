@@ -79,14 +79,25 @@ def _round_up(a, b):
     return (a + b - 1) // b * b
 
 
+def _plain_keys(device="CUDA"):
+    """Dispatch keys of a tensor that is nothing but memory of the device, made inside and outside inference mode"""
+    key = lambda name: torch._C.DispatchKeySet(getattr(torch._C.DispatchKey, name))  # noqa: E731
+    inference = key(device) | key("Autocast" + device)
+    return inference.raw_repr(), (inference | key("ADInplaceOrView") | key("Autograd" + device)).raw_repr()
+
+
+_PLAIN_KEYS = _plain_keys()
+
+
 def runs_eagerly(x: Tensor, *others: Tensor) -> bool:
-    """True if calling the CUDA implementation of an op on these tensors does all that going through the dispatcher would: plain
-    tensors (no fake ones, no wrappers), nothing to differentiate in either direction, and no mode, transform or tracer that wants to
-    see the op.  The dispatcher and the schema's boxing are half of the host time of a small linear."""
-    if type(x) is not Tensor or (x.requires_grad and torch.is_grad_enabled()):
+    """True if calling the CUDA implementation of an op on these tensors does all that going through the dispatcher would: plain CUDA
+    tensors (no fake ones, no wrappers, no other device, no negative view or zero tensor, which have no memory of their own to read),
+    nothing to differentiate in either direction, and no mode, transform or tracer that wants to see the op.  The dispatcher and the
+    schema's boxing are half of the host time of a small linear."""
+    if x.requires_grad and torch.is_grad_enabled():
         return False
-    for t in others:
-        if type(t) is not Tensor:
+    for t in (x, *others):
+        if type(t) is not Tensor or torch._C._dispatch_keys(t).raw_repr() not in _PLAIN_KEYS:
             return False
     return (torch._C._len_torch_dispatch_stack() == 0 and torch._C._functorch.peek_interpreter_stack() is None
             and torch._C._get_tracing_state() is None and _forward_ad._current_level < 0)
