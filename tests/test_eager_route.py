@@ -36,6 +36,32 @@ def test_only_plain_cuda_memory_is_eager():
         assert not ops.runs_eagerly(t)
 
 
+def test_a_tracer_stops_at_the_first_question():
+    f = lambda x: x + 1 if ops.runs_eagerly(x) else x * 2  # noqa: E731
+    x = torch.randn(3)
+    assert torch.equal(torch.compile(f, fullgraph=True, backend="eager")(x), x * 2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 5])
+def test_the_blocks_of_the_llama_model_trace_in_one_graph(rows):
+    import torchao_fork_b200 as ao
+    from torchao_fork_b200._models.llama import ModelArgs
+    from torchao_fork_b200._models.llama.model import FeedForward, RMSNorm, apply_rotary_emb
+    cfg = ModelArgs.from_name("tiny-llama3")
+    torch.manual_seed(0)
+    norm, ff = (m.to("cuda", torch.bfloat16).requires_grad_(False) for m in (RMSNorm(cfg.dim), FeedForward(cfg)))
+    ao.quantize_(ff, ao.Int4WeightOnlyConfig(group_size=64))
+    x = torch.randn(1, rows, cfg.dim, device="cuda").bfloat16()
+    q, freqs = torch.randn(1, rows, 4, 128, device="cuda").bfloat16(), torch.randn(rows, 64, 2, device="cuda").bfloat16()
+    both = lambda x, q, freqs: (ff(norm(x)), apply_rotary_emb(q, freqs))  # noqa: E731
+    torch._dynamo.reset()
+    traced, rotated = torch.compile(both, fullgraph=True, backend="aot_eager")(x, q, freqs)
+    plain, turned = both(x, q, freqs)
+    # the norm adds up in another order: one rounding of its result, 2^-8, and of what follows
+    assert torch.equal(rotated, turned) and (traced - plain).float().norm() < 2.0 ** -7 * plain.float().norm()
+
+
 @pytest.mark.gpu
 def test_plain_cuda_tensors_are_eager_and_wrapped_ones_are_not():
     x = torch.ones(2, device="cuda")

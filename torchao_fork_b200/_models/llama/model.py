@@ -89,7 +89,7 @@ from ..cache import AffineQuantizedKVCache, KVCache  # noqa: E402,F401  (the cac
 def _rows_by_kernel(x: Tensor, *others: Tensor) -> bool:
     """Whether an element-wise step of the block may be one kernel launch: bf16 on one CUDA device, in whole aligned pieces, and nobody
     who would see the single operations (autograd, tracers, modes)."""
-    if not (x.is_cuda and x.dtype is torch.bfloat16 and x.numel() > 0 and runs_eagerly(x, *others)) or torch.compiler.is_compiling():
+    if torch.compiler.is_compiling() or not (x.is_cuda and x.dtype is torch.bfloat16 and x.numel() > 0 and runs_eagerly(x, *others)):
         return False
     if torch._C._len_torch_function_stack() != 0:
         return False

@@ -94,6 +94,8 @@ def runs_eagerly(x: Tensor, *others: Tensor) -> bool:
     tensors (no fake ones, no wrappers, no other device, no negative view or zero tensor, which have no memory of their own to read),
     nothing to differentiate in either direction, and no mode, transform or tracer that wants to see the op.  The dispatcher and the
     schema's boxing are half of the host time of a small linear."""
+    if torch.compiler.is_compiling():   # first: a tracer that follows Python gets no further than this
+        return False
     if x.requires_grad and torch.is_grad_enabled():
         return False
     for t in (x, *others):
