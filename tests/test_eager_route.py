@@ -2,6 +2,7 @@
 the shape of every answer, or the error, is that of the registered op."""
 import pytest
 import torch
+from torch.overrides import BaseTorchFunctionMode
 
 from torchao_fork_b200 import ops
 
@@ -40,6 +41,27 @@ def test_a_tracer_stops_at_the_first_question():
     f = lambda x: x + 1 if ops.runs_eagerly(x) else x * 2  # noqa: E731
     x = torch.randn(3)
     assert torch.equal(torch.compile(f, fullgraph=True, backend="eager")(x), x * 2)
+
+
+def test_a_function_mode_keeps_its_say(monkeypatch):
+    monkeypatch.setattr(ops, "_PLAIN_KEYS", ops._plain_keys("CPU"))
+    x = torch.ones(2)
+    assert ops.runs_eagerly(x)
+    with BaseTorchFunctionMode():
+        assert not ops.runs_eagerly(x)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits,name", [(4, "torchao::b200_int4_weight_only_mm"), (8, "torchao::b200_int8_weight_only_mm")])
+def test_a_profile_names_the_op(bits, name):
+    import torchao_fork_b200 as ao
+    lin = torch.nn.Linear(128, 128, bias=False, device="cuda", dtype=torch.bfloat16).requires_grad_(False)
+    ao.quantize_(lin, ao.Int4WeightOnlyConfig(group_size=64) if bits == 4 else ao.Int8WeightOnlyConfig())
+    x = torch.randn(2, 128, device="cuda").bfloat16()
+    y = lin(x)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        assert torch.equal(lin(x), y)
+    assert name in {e.name for e in prof.events()}
 
 
 @pytest.mark.gpu

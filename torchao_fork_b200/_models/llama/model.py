@@ -91,8 +91,6 @@ def _rows_by_kernel(x: Tensor, *others: Tensor) -> bool:
     who would see the single operations (autograd, tracers, modes)."""
     if torch.compiler.is_compiling() or not (x.is_cuda and x.dtype is torch.bfloat16 and x.numel() > 0 and runs_eagerly(x, *others)):
         return False
-    if torch._C._len_torch_function_stack() != 0:
-        return False
     return all(t.device == x.device and t.dtype is torch.bfloat16 and t.data_ptr() % 16 == 0 and not (t.requires_grad and torch.is_grad_enabled())
                for t in (x, *others))
 

@@ -101,8 +101,9 @@ def runs_eagerly(x: Tensor, *others: Tensor) -> bool:
     for t in (x, *others):
         if type(t) is not Tensor or torch._C._dispatch_keys(t).raw_repr() not in _PLAIN_KEYS:
             return False
-    return (torch._C._len_torch_dispatch_stack() == 0 and torch._C._functorch.peek_interpreter_stack() is None
-            and torch._C._get_tracing_state() is None and _forward_ad._current_level < 0)
+    return (torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+            and torch._C._functorch.peek_interpreter_stack() is None and torch._C._get_tracing_state() is None
+            and _forward_ad._current_level < 0)
 
 
 class _NoGuard:
@@ -512,15 +513,15 @@ def _mm_rows(x):
 
 
 def int4_weight_only_mm(x: Tensor, packed_w: Tensor, group_size: int, scales_and_zeros: Tensor, out_features: int) -> Tensor:
-    """torch.ops.torchao.b200_int4_weight_only_mm, without the dispatcher where that adds nothing"""
-    if runs_eagerly(x, packed_w, scales_and_zeros):
+    """torch.ops.torchao.b200_int4_weight_only_mm, without the dispatcher where that adds nothing (a profile gets its op's name there)"""
+    if runs_eagerly(x, packed_w, scales_and_zeros) and not torch.autograd._profiler_enabled():
         return _int4_mm_cuda(x, packed_w, group_size, scales_and_zeros, out_features)
     return torch.ops.torchao.b200_int4_weight_only_mm(x, packed_w, group_size, scales_and_zeros, out_features)
 
 
 def int8_weight_only_mm(x: Tensor, packed_w: Tensor, scale: Tensor) -> Tensor:
-    """torch.ops.torchao.b200_int8_weight_only_mm, without the dispatcher where that adds nothing"""
-    if runs_eagerly(x, packed_w, scale):
+    """torch.ops.torchao.b200_int8_weight_only_mm, without the dispatcher where that adds nothing (a profile gets its op's name there)"""
+    if runs_eagerly(x, packed_w, scale) and not torch.autograd._profiler_enabled():
         return _int8_mm_cuda(x, packed_w, scale)
     return torch.ops.torchao.b200_int8_weight_only_mm(x, packed_w, scale)
 
