@@ -92,3 +92,16 @@ def test_plain_cuda_tensors_are_eager_and_wrapped_ones_are_not():
     assert ops.runs_eagerly(x) and ops.runs_eagerly(x, inside, x.view(2)) and ops.runs_eagerly(inside)
     for t in (torch._neg_view(x), torch._efficientzerotensor(2, device="cuda"), torch._to_functional_tensor(x), x.cpu()):
         assert not ops.runs_eagerly(t) and not ops.runs_eagerly(x, t)
+
+
+@pytest.mark.gpu
+def test_weights_that_are_not_on_the_device_are_refused():
+    # the op is registered for CUDA, which the activations alone decide: a host address must not get as far as a launch
+    x, packed, group, sz, n = _args(4, "cuda")
+    for p, s in ((packed.cpu(), sz), (packed, sz.cpu())):
+        with pytest.raises(RuntimeError, match="CUDA"):
+            T.b200_int4_weight_only_mm(x, p, group, s, n)
+    x, packed, scale = _args(8, "cuda")
+    for p, s in ((packed.cpu(), scale), (packed, scale.cpu())):
+        with pytest.raises(RuntimeError, match="CUDA"):
+            T.b200_int8_weight_only_mm(x, p, s)

@@ -533,6 +533,7 @@ def _int4_mm_checks(x, packed_w, group_size, scales_and_zeros, out_features):
     torch._check(x.dim() == 2 and x.size(1) <= kp, lambda: f"x must be (M, K<= {kp}), got {tuple(x.shape)}")
     torch._check(0 < out_features <= np_, lambda: "out_features out of range")
     torch._check(packed_w.is_contiguous() and scales_and_zeros.is_contiguous(), lambda: "weights must be contiguous")
+    torch._check(packed_w.is_cuda and scales_and_zeros.is_cuda, lambda: "weights must be CUDA tensors")
 
 
 @_impl_cuda("b200_int4_weight_only_mm")
@@ -540,8 +541,8 @@ def _int4_mm_cuda(x: Tensor, packed_w: Tensor, group_size: int, scales_and_zeros
     """Same contract as aten._weight_int4pack_mm(x, packed, G, scale_and_zero)
     (call site torchao/dtypes/uintx/tensor_core_tiled_layout.py:104) on the super-tile layout."""
     ps, xs = packed_w.shape, x.shape
-    if not (len(ps) == 4 and len(xs) == 2 and x.is_cuda and x.dtype is torch.bfloat16 and packed_w.dtype is torch.int32
-            and scales_and_zeros.dtype is torch.bfloat16 and group_size in (32, 64, 128, 256) and ps[2] == 32 and ps[3] == 4
+    if not (len(ps) == 4 and len(xs) == 2 and x.is_cuda and packed_w.is_cuda and scales_and_zeros.is_cuda
+            and x.dtype is torch.bfloat16 and packed_w.dtype is torch.int32 and scales_and_zeros.dtype is torch.bfloat16 and group_size in (32, 64, 128, 256) and ps[2] == 32 and ps[3] == 4
             and scales_and_zeros.shape == (ps[0], ps[1] * 64 // group_size, 16, 2) and xs[1] <= ps[1] * 64
             and 0 < out_features <= ps[0] * 16 and packed_w.is_contiguous() and scales_and_zeros.is_contiguous()):
         _int4_mm_checks(x, packed_w, group_size, scales_and_zeros, out_features)
