@@ -88,21 +88,27 @@ def _plain_keys(device="CUDA"):
 
 _PLAIN_KEYS = _plain_keys()
 
+# one look-up each: this is asked at every linear
+_is_compiling = torch.compiler.is_compiling
+_dispatch_keys = torch._C._dispatch_keys
+_dispatch_modes, _function_modes = torch._C._len_torch_dispatch_stack, torch._C._len_torch_function_stack
+_interpreter, _tracing_state = torch._C._functorch.peek_interpreter_stack, torch._C._get_tracing_state
+_profiling = torch.autograd._profiler_enabled
+
 
 def runs_eagerly(x: Tensor, *others: Tensor) -> bool:
     """True if calling the CUDA implementation of an op on these tensors does all that going through the dispatcher would: plain CUDA
     tensors (no fake ones, no wrappers, no other device, no negative view or zero tensor, which have no memory of their own to read),
     nothing to differentiate in either direction, and no mode, transform or tracer that wants to see the op.  The dispatcher and the
     schema's boxing are half of the host time of a small linear."""
-    if torch.compiler.is_compiling():   # first: a tracer that follows Python gets no further than this
+    if _is_compiling():   # first: a tracer that follows Python gets no further than this
         return False
     if x.requires_grad and torch.is_grad_enabled():
         return False
     for t in (x, *others):
-        if type(t) is not Tensor or torch._C._dispatch_keys(t).raw_repr() not in _PLAIN_KEYS:
+        if type(t) is not Tensor or _dispatch_keys(t).raw_repr() not in _PLAIN_KEYS:
             return False
-    return (torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
-            and torch._C._functorch.peek_interpreter_stack() is None and torch._C._get_tracing_state() is None
+    return (_dispatch_modes() == 0 and _function_modes() == 0 and _interpreter() is None and _tracing_state() is None
             and _forward_ad._current_level < 0)
 
 
@@ -513,15 +519,16 @@ def _mm_rows(x):
 
 
 def int4_weight_only_mm(x: Tensor, packed_w: Tensor, group_size: int, scales_and_zeros: Tensor, out_features: int) -> Tensor:
-    """torch.ops.torchao.b200_int4_weight_only_mm, without the dispatcher where that adds nothing (a profile gets its op's name there)"""
-    if runs_eagerly(x, packed_w, scales_and_zeros) and not torch.autograd._profiler_enabled():
+    """torch.ops.torchao.b200_int4_weight_only_mm, without the dispatcher where that adds nothing (a profile gets its op's name there;
+    weights that are no plain CUDA tensors are refused by the implementation either way)"""
+    if type(packed_w) is Tensor and type(scales_and_zeros) is Tensor and runs_eagerly(x) and not _profiling():
         return _int4_mm_cuda(x, packed_w, group_size, scales_and_zeros, out_features)
     return torch.ops.torchao.b200_int4_weight_only_mm(x, packed_w, group_size, scales_and_zeros, out_features)
 
 
 def int8_weight_only_mm(x: Tensor, packed_w: Tensor, scale: Tensor) -> Tensor:
-    """torch.ops.torchao.b200_int8_weight_only_mm, without the dispatcher where that adds nothing (a profile gets its op's name there)"""
-    if runs_eagerly(x, packed_w, scale) and not torch.autograd._profiler_enabled():
+    """torch.ops.torchao.b200_int8_weight_only_mm, without the dispatcher where that adds nothing (as above)"""
+    if type(packed_w) is Tensor and type(scale) is Tensor and runs_eagerly(x) and not _profiling():
         return _int8_mm_cuda(x, packed_w, scale)
     return torch.ops.torchao.b200_int8_weight_only_mm(x, packed_w, scale)
 
