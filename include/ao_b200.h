@@ -119,8 +119,10 @@ AO_B200_API int ao_b200_tinygemm_pack(const int32_t* q, int64_t N, int64_t K, in
  * x: bf16 [M][Kx] row stride ldx (Kx <= Kp, Kx % 8 == 0; k >= Kx reads as zero — no
  * host-side F.pad of the activation); y: bf16 [M][N_out] row stride ldy.
  * few rows -> HBM-bound split-K tensor-core GEMV; more rows (from 3 to 17 on, by the weight's size) -> tcgen05 GEMM.
+ * A wait of the GEMM that runs out (about two seconds) leaves NaN in the rows concerned.
  * workspace: ao_b200_int4_mm_workspace_bytes(...) bytes, zero-initialised once by the
- * caller (the kernels leave it zeroed on exit); may be NULL when that returns 0. */
+ * caller (the GEMV's part in front is zero again on exit, the GEMM's behind it is not
+ * and need not be); may be NULL when that returns 0. */
 AO_B200_API int64_t ao_b200_int4_mm_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
 AO_B200_API int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx,
                     const void* packed, const void* scale_and_zero, int64_t Np, int64_t Kp,

@@ -30,7 +30,8 @@
 // alternate units), 20 weight producer (two TMA tensor copies per unit: 8 strips of weights, 8 strips of parameters),
 // 21 activation producer, 22 and 23 MMA issue: the waits, the issue and the commit of a unit take one warp 600 clocks, so up to
 // NT = 64 two warps take alternate units, each with accumulators of its own that the epilogue adds.  At the end all warps
-// add up the tiles that this CTA was the last to reach.  Every wait is bounded: a CTA that gives up sets `status` and returns.
+// add up the tiles that this CTA was the last to reach.  Every wait is bounded: a CTA that gives up fills the rows of all its tiles with NaN
+// (a shared tile then misses a ticket, so nobody else writes it) and returns once its copies and products in flight are over.
 //
 // Bound by the tensor cores from about 512 rows (8 MMAs of N = 256 take 1024 clocks per unit and pair, the dequant of a unit
 // about 900 clocks per set of warps, two sets in flight), below that by the dequant -> MMA chain of a unit.  Measured, 14336 x 4096,
@@ -39,6 +40,8 @@
 // the dequant loop: 29.9 / 36.5 / 67.0 / 128 / 225 us); int8 8192 x 8192, M = 32 / 512 / 2048: 24 / 63 / 225 us (44 / 66 / 244 us).
 #include <cuda.h>
 #include <cuda_bf16.h>
+
+#include <cstdlib>
 
 #include "common.cuh"
 
@@ -62,10 +65,10 @@ struct WqParams {
   const __nv_bfloat16* residual;  // y = bf16(residual + bf16(sum)); may be y itself
   float* part;               // shares of split tiles [workers][2][ranks][NT * 128]
   uint32_t* tickets;         // [tiles][ranks], zeroed by the staging kernel
-  uint32_t* status;
   int64_t N_out, ldy, ld_res;
   int M, NT, BR, KU, MT, w_slots, x_slots, a_slots, n_mma, vec_store;
   uint32_t off_w;            // weight ring
+  long long wait_limit;      // clocks after which a wait gives up
   uint32_t x_bytes;          // one unit of staged activations (and, DEFER, its sums)
   int quantum, base, rem;    // worker c owns units [first(c), first(c + 1)), first(c) = (c base + min(c, rem)) quantum
 };
@@ -189,18 +192,20 @@ __device__ __forceinline__ void wq_arrive_leader(uint64_t* bar) {
   else
     mbar_arrive(bar);
 }
-// bounded wait: false (and *dead set) after about two seconds, or as soon as another warp of the CTA has given up
-__device__ __forceinline__ bool wq_wait(uint64_t* bar, uint32_t parity, volatile int* dead) {
+// bounded wait: false (and *dead set) after `limit` clocks, or as soon as another warp of the CTA has given up.  The lanes of a warp may
+// answer differently then.  So roles of whole warps keep their answer and their place in the loops (their instructions are the
+// warp's); what they must not do any more is announce: neither products nor arrivals that the other CTA of a pair would believe.
+__device__ __forceinline__ bool wq_wait(uint64_t* bar, uint32_t parity, volatile int* dead, long long limit) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   for (;;) {
-#pragma unroll 1
-    for (int i = 0; i < 32; ++i)
-      if (mbar_try_wait(bar, parity)) return true;
-    if (*dead != 0 || clock64() - t0 > 4000000000ll) {
+    if (*dead != 0 || clock64() - t0 > limit) {
       *dead = 1;
       return false;
     }
+#pragma unroll 1
+    for (int i = 0; i < 32; ++i)
+      if (mbar_try_wait(bar, parity)) return true;
   }
 }
 // barrier of the epilogue warps; true if any of them brings a failure
@@ -258,6 +263,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
   const int u0 = wq_first(worker, p.base, p.rem, p.quantum), u1 = wq_first(worker + 1, p.base, p.rem, p.quantum);
   const int KU = p.KU, NT = p.NT, x_slots = p.x_slots, a_slots = p.a_slots, n_mma = p.n_mma;
   const int d_bufs = NT <= 128 ? 2 : 1;
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return wq_wait(bar, parity, dead, p.wait_limit); };
   grid_launch_dependents();
 
   // the weights wait for nobody: their producer fills the ring while the others set up
@@ -389,7 +395,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
       WqRing w;
       w.use = 1;
       for (int u = u0 + p.w_slots; u < u1; ++u) {
-        if (!wq_wait(&wempty[w.slot], w.use ^ 1u, dead)) break;
+        if (!wait(&wempty[w.slot], w.use ^ 1u)) break;
         load_weights(w.slot);
         w.step(1, p.w_slots);
       }
@@ -405,7 +411,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
       int mt = t_first % p.MT, ku = ku_first;
       const uint8_t* src = base + mt * (kRanks * tile_bytes) + (int64_t)ku * p.x_bytes;
       for (int u = u0; u < u1; ++u) {
-        if (!wq_wait(DEFER ? &dread[x.slot] : &xdone[x.slot], x.use ^ 1u, dead)) break;
+        if (!wait(DEFER ? &dread[x.slot] : &xdone[x.slot], x.use ^ 1u)) break;
         mbar_arrive_expect_tx(&xfull[x.slot], p.x_bytes);
         bulk_g2s(xring + (uint32_t)x.slot * p.x_bytes, src, p.x_bytes, &xfull[x.slot]);
         x.step(1, x_slots);
@@ -423,9 +429,10 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     WqRing x, a, d;
     if (PAIR && rank != 0) {
       // ---- the pair's second CTA: tells the first one that its half of the activations has landed ----
+      bool ok = true;
       for (int u = u0; u < (mw == 0 ? u1 : u0); ++u) {
-        if (!wq_wait(&xfull[x.slot], x.use, dead)) break;
-        if (wq_elect_one()) wq_arrive_leader<PAIR>(&xpeer[x.slot]);
+        ok = ok && wait(&xfull[x.slot], x.use);
+        if (wq_elect_one() && ok) wq_arrive_leader<PAIR>(&xpeer[x.slot]);
         __syncwarp();
         x.step(1, x_slots);
       }
@@ -438,21 +445,20 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
       const uint32_t desc_hi = (128u >> 4) | (1u << 14), kstep = (2 * chunk) >> 4;
       const uint32_t desc_lo = ((chunk >> 4) << 16) | (smem_u32(xring) >> 4), xstep = p.x_bytes >> 4;
       int u = u0;
+      bool ok = true;
       while (u < (mw < n_mma ? u1 : u0)) {
         const int ue = min(u1, (u / KU + 1) * KU);  // the units of this tile
-        if (!DEFER && !wq_wait(&dempty[d.slot], d.use ^ 1u, dead)) break;
+        if (!DEFER) ok = ok && wait(&dempty[d.slot], d.use ^ 1u);
         const uint32_t dcol = tb + d.slot * 128 + mw * 64;
         uint32_t acc = 0;
-        bool ok = true;
         // this warp's units: those whose number in the CTA's sequence is mw (mod n_mma)
         if (n_mma == 2 && ((u - u0) & 1) != mw) ++u;
         for (; u < ue; u += n_mma) {
           const bool ra = mbar_try_wait(&afull[a.slot], a.use), rx = mbar_try_wait(&xfull[x.slot], x.use);
-          ok = (ra || wq_wait(&afull[a.slot], a.use, dead)) && (rx || wq_wait(&xfull[x.slot], x.use, dead));
-          if (PAIR) ok = ok && wq_wait(&xpeer[x.slot], x.use, dead);
-          if (!ok) break;
+          ok = ok && (ra || wait(&afull[a.slot], a.use)) && (rx || wait(&xfull[x.slot], x.use));
+          if (PAIR) ok = ok && wait(&xpeer[x.slot], x.use);
           wq_fence_after();
-          if (wq_elect_one()) {
+          if (wq_elect_one() && ok) {
             const uint32_t b0 = desc_lo + (uint32_t)x.slot * xstep, a0 = a_col0 + a.slot * 64;
             const uint32_t d0 = DEFER ? tb + x.slot * (kSegs * 16) : dcol;
 #pragma unroll
@@ -468,10 +474,9 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
           x.step(n_mma, x_slots);
           a.step(n_mma, a_slots);
         }
-        if (!ok) break;
         u = ue;
         if (!DEFER) {
-          if (wq_elect_one()) wq_commit<PAIR>(&dfull[d.slot]);
+          if (wq_elect_one() && ok) wq_commit<PAIR>(&dfull[d.slot]);
           __syncwarp();
           d.step(1, d_bufs);
         }
@@ -495,10 +500,11 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     // us).  The others are bound by the conversions or the MMAs and do best announcing first (int8 8192 x 8192, 2048 rows: 217 against 223 us).
     constexpr int kWords = kI8 ? 16 : 8, kSzn = (kI8 || DEFER) ? 1 : kSzWords / 16;
     uint32_t wd[kWords], sz[kSzn][2];
+    bool ok = true;
     auto fetch = [&](int u) {
-      if (u >= u1) return true;
-      if (a_first && !wq_wait(&adone[a.slot], a.use ^ 1u, dead)) return false;
-      if (!wq_wait(&wfull[w.slot], w.use, dead)) return false;
+      if (u >= u1) return;
+      if (a_first) ok = ok && wait(&adone[a.slot], a.use ^ 1u);
+      ok = ok && wait(&wfull[w.slot], w.use);
       const uint32_t wt = w0_u + w.slot * kWSlot, st = s0_u + w.slot * kWSlot;
 #pragma unroll
       for (int i = 0; i < kWords / 4; ++i) {
@@ -512,10 +518,9 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
           sz[h][1] = lds32(st + h * 64 + 32);
         }
       }
-      return true;
     };
-    bool ok = fetch(u0 + set);
-    for (int u = u0 + set; u < u1 && ok; u += 2) {
+    fetch(u0 + set);
+    for (int u = u0 + set; u < u1; u += 2) {
       uint32_t r[32];
       if constexpr (kI8) {
 #pragma unroll
@@ -541,20 +546,20 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&wempty[w.slot]);  // everything that this warp reads of the slot is in registers
-      ok = wq_wait(&adone[a.slot], a.use ^ 1u, dead);  // the MMAs that read this A slot have retired
-      if (!ok) break;
+      ok = ok && wait(&adone[a.slot], a.use ^ 1u);  // the MMAs that read this A slot have retired
       wq_fence_after();
       wq_st_16x128b_x8(taddr0 + a.slot * 64, r);
       wq_st_16x128b_x8(taddr0 + a.slot * 64 + 32, r + 16);
       uint64_t* full = &afull[a.slot];
+      const bool announce = ok;
       w.step(2, p.w_slots);
       a.step(2, a_slots);
-      if (DEFER && !a_first) ok = fetch(u + 2);
+      if (DEFER && !a_first) fetch(u + 2);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       wq_fence_before();
       __syncwarp();
-      if (lane == 0) wq_arrive_leader<PAIR>(full);
-      if (!DEFER || a_first) ok = fetch(u + 2);  // (a_first waits for MMAs: not before this unit is announced)
+      if (lane == 0 && announce) wq_arrive_leader<PAIR>(full);
+      if (!DEFER || a_first) fetch(u + 2);  // (a_first waits for MMAs: not before this unit is announced)
     }
   } else {
     // ---- epilogue ----
@@ -575,8 +580,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
         for (int i = 0; i < 16; ++i) acc[i] = 0.f;
         for (; u < ue; ++u) {
           const bool rw = mbar_try_wait(&wfull[w.slot], w.use), rx = mbar_try_wait(&xfull[x.slot], x.use), rd = mbar_try_wait(&xdone[x.slot], x.use);
-          ok = (rw || wq_wait(&wfull[w.slot], w.use, dead)) && (rx || wq_wait(&xfull[x.slot], x.use, dead)) && (rd || wq_wait(&xdone[x.slot], x.use, dead));
-          if (!ok) break;
+          ok = ok && (rw || wait(&wfull[w.slot], w.use)) && (rx || wait(&xfull[x.slot], x.use)) && (rd || wait(&xdone[x.slot], x.use));
           wq_fence_after();
           // parameters of rows 32 warp + lane / 4 + 8 i, sums of columns 2 (lane % 4) + {0, 1, 8, 9}
           const uint32_t st = smem_u32(wring) + w.slot * kWSlot + kWBytes + 2 * warp * (kSzWords * 4) + (lane >> 2) * 4;
@@ -621,7 +625,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
           for (int i = 0; i < 4; ++i) __stcg(mine + i * 128, make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]));
         }
       } else {
-        ok = wq_wait(&dfull[d.slot], d.use, dead);
+        ok = ok && wait(&dfull[d.slot], d.use);
         wq_fence_after();
         // which accumulators hold something: both MMA warps', unless the tile has one unit here
         const bool two = n_mma == 2 && ue - u > 1;
@@ -701,7 +705,15 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
 
   // ---- teardown: nobody touches tensor memory any more ----
   if (*dead != 0) {
-    if (threadIdx.x == 0) atomicExch(p.status, 1u);
+    grid_dependency_wait();  // (whoever had y before)
+    for (int t = u0 / KU; t <= (u1 - 1) / KU; ++t) {
+      const int nb = t / p.MT, m0 = (t - nb * p.MT) * NT, rows = min(NT, p.M - m0);
+      const int64_t nbase = ((int64_t)nb * kRanks + rank) * 128;
+      for (int i = threadIdx.x; i < rows * 128; i += kWqThreads) {
+        const int64_t n = nbase + (i & 127);
+        if (n < p.N_out) p.y[(int64_t)(m0 + (i >> 7)) * p.ldy + n] = __ushort_as_bfloat16((unsigned short)0x7FFF);
+      }
+    }
     for (int i = 0; i < 64; ++i) __nanosleep(100000);  // copies and MMAs of this CTA that are still in flight
   }
   wq_fence_before();
@@ -732,7 +744,7 @@ struct WqPlan {
   int NT, BR, MT, NB, KU, ranks, workers, quantum, base, rem;
   int64_t tiles, n_tickets;
   uint32_t x_bytes;
-  int64_t off_part, off_xt, bytes;  // [status, tickets][shares][staged activations]
+  int64_t off_part, off_xt, bytes;  // [tickets][shares][staged activations]
 };
 
 static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
@@ -756,7 +768,7 @@ static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
   w.n_tickets = w.quantum > 1 ? 0 : w.tiles * w.ranks;
   w.x_bytes = (uint32_t)w.BR * 256 + (w.defer ? 4 * 64 : 0);  // (the sums' space is that of the smallest group)
   auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
-  w.off_part = up(256 + w.n_tickets * 4);
+  w.off_part = up(w.n_tickets * 4);
   w.off_xt = w.off_part + (w.quantum > 1 ? 0 : up((int64_t)w.workers * 2 * w.ranks * w.NT * 512));
   w.bytes = w.off_xt + up((int64_t)w.MT * w.ranks * w.KU * w.x_bytes);
   return true;
@@ -853,10 +865,12 @@ static int wq_gemm(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void
                           wq_map(&p.smap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, sz, Kp / G * 64, Np / 16, (G < 128 ? 128 / G : 1) * 16)
                     : wq_map(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_INT64, 8, packed, Kp * 16, Np / 16, 256);
   if (!ok) return AO_B200_ERR_UNSUPPORTED;
-  p.status = reinterpret_cast<uint32_t*>(ws);
-  p.tickets = reinterpret_cast<uint32_t*>(ws + 256);
+  p.tickets = reinterpret_cast<uint32_t*>(ws);
   p.part = reinterpret_cast<float*>(ws + w.off_part);
   p.xt = ws + w.off_xt;
+  // about two seconds; the variable is there for the test of what a wait that runs out leaves behind
+  static const long long limit = []() { const char* e = std::getenv("AO_B200_GEMM_WAIT_CLOCKS"); return e ? std::atoll(e) : 4000000000ll; }();
+  p.wait_limit = limit;
   p.scale8 = G ? nullptr : static_cast<const __nv_bfloat16*>(sz);
   p.y = static_cast<__nv_bfloat16*>(y);
   p.N_out = N_out;
