@@ -102,3 +102,31 @@ def test_residual(bits, group, m, n, k):
     assert ((y.double() - h[:, :n].double() - plain.double()).norm() / y.double().norm()).item() < 2.0 ** -7
     assert L.ao_b200_mm_residual(xp.data_ptr(), m, kp, kp, packed.data_ptr(), scales.data_ptr(), np_, kp, group, y.data_ptr(), n, n, h.data_ptr(), n + 3,
                                  ws.data_ptr(), 16, 0) != 0
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("m", [12, 40, 300])
+def test_weights_written_by_the_kernel_in_front(bits, m):
+    # the weights of a call may be what the launch before it wrote: its result is that of weights long there, time after time
+    n, k = 16384, 8192
+    x, packed, scales, want = None, [], [], []
+    for seed in range(2):
+        gen = torch.Generator(device="cuda").manual_seed(seed)
+        w = torch.randn(n, k, generator=gen, device="cuda").to(torch.bfloat16)
+        x = torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16) if x is None else x
+        if bits == 4:
+            p, sc = T.b200_int4_quantize_pack(w, 128, 1e-6, True)
+        else:
+            q, sc = T.b200_int8_quantize(w, 1e-6, True)
+            p = T.b200_int8_pack(q)
+        packed.append(p), scales.append(sc)
+        torch.cuda.synchronize()
+        want.append(T.b200_int4_weight_only_mm(x, p, 128, sc, n) if bits == 4 else T.b200_int8_weight_only_mm(x, p, sc))
+    pw, sw, got = torch.empty_like(packed[0]), torch.empty_like(scales[0]), []
+    torch.cuda.synchronize()
+    for i in range(24):
+        pw.copy_(packed[i % 2])
+        sw.copy_(scales[i % 2])
+        got.append(T.b200_int4_weight_only_mm(x, pw, 128, sw, n) if bits == 4 else T.b200_int8_weight_only_mm(x, pw, sw))
+    for i, y in enumerate(got):
+        assert torch.equal(y, want[i % 2]), i

@@ -87,8 +87,10 @@ __device__ __forceinline__ int wq_owner(int u, int base, int rem, int quantum) {
 template <int SEG>
 __global__ void __launch_bounds__(256) stage_x_kernel(const __nv_bfloat16* __restrict__ x, int64_t M, int64_t Kx, int64_t ldx, int n_blocks, int BR, int KU,
                                                       uint32_t x_bytes, uint8_t* __restrict__ xt, uint32_t* __restrict__ tickets, int n_tickets) {
-  grid_launch_dependents();
+  // The GEMM behind reads weights and parameters without a wait of its own.  They may be the work of the kernel in front of this
+  // one (quantize_, then a call), so it is let go only when that one is over and its writes are visible.
   grid_dependency_wait();
+  grid_launch_dependents();
   const int64_t gid = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (gid < n_tickets) tickets[gid] = 0u;
   const int lane = threadIdx.x & 31, row8 = lane >> 2, quarter = lane & 3;  // quarter: 32-k piece of the unit
@@ -266,7 +268,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
   auto wait = [&](uint64_t* bar, uint32_t parity) { return wq_wait(bar, parity, dead, p.wait_limit); };
   grid_launch_dependents();
 
-  // the weights wait for nobody: their producer fills the ring while the others set up
+  // the weights do not wait for the staging kernel (see there): their producer fills the ring while the others set up
   // (running positions: a division per unit is what paced the producers)
   const int t_first = u0 / KU, ku_first = u0 - t_first * KU;
   int w_ku = ku_first, w_mt = t_first % p.MT, w_strip = ((t_first / p.MT) * kRanks + rank) * 8;
