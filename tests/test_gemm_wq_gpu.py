@@ -130,3 +130,30 @@ def test_weights_written_by_the_kernel_in_front(bits, m):
         got.append(T.b200_int4_weight_only_mm(x, pw, 128, sw, n) if bits == 4 else T.b200_int8_weight_only_mm(x, pw, sw))
     for i, y in enumerate(got):
         assert torch.equal(y, want[i % 2]), i
+
+
+def test_threads_that_share_a_stream():
+    # a call is a staging launch and the GEMM behind it, over one workspace per stream: nobody's launch may come between them
+    import threading
+    calls, want = [], []
+    for i, (bits, m, n, k) in enumerate(((4, 40, 640, 4096), (4, 130, 1024, 2048), (4, 300, 384, 1024), (4, 24, 640, 8192))):
+        gen = torch.Generator(device="cuda").manual_seed(i)
+        w, x = (torch.randn(r, k, generator=gen, device="cuda").to(torch.bfloat16) for r in (n, m))
+        packed, sz = T.b200_int4_quantize_pack(w, 128, 1e-6, True)
+        calls.append((x, packed, 128, sz, n))
+        want.append(T.b200_int4_weight_only_mm(*calls[-1]))
+    bad, start = [], threading.Barrier(len(calls))
+
+    def work(i):
+        start.wait()
+        for _ in range(100):
+            ys = [T.b200_int4_weight_only_mm(*calls[i]) for _ in range(5)]
+            if not all(torch.equal(y, want[i]) for y in ys):
+                bad.append(i)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(calls))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad

@@ -42,6 +42,7 @@
 #include <cuda_bf16.h>
 
 #include <cstdlib>
+#include <mutex>
 
 #include "common.cuh"
 
@@ -889,6 +890,10 @@ static int wq_gemm(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void
   p.quantum = w.quantum;
   p.base = w.base;
   p.rem = w.rem;
+  // Staging and GEMM go into the stream as neighbours: another thread's call on the same stream may use the same workspace, and
+  // the host is free to run it between the two launches.
+  static std::mutex together;
+  std::lock_guard<std::mutex> lock(together);
   int rc;
   if (!w.defer) rc = wq_stage<0>(x, M, Kx, ldx, w, ws + w.off_xt, p.tickets, s);
   else if (G == 32) rc = wq_stage<32>(x, M, Kx, ldx, w, ws + w.off_xt, p.tickets, s);
