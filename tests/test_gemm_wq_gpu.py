@@ -157,3 +157,37 @@ def test_threads_that_share_a_stream():
     for t in threads:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("group", [32, 64, 128, 256])
+@pytest.mark.parametrize("m", [12, 16])
+def test_few_rows_with_infinities_and_huge_values(group, m):
+    # sums that overflow with 128 + q in the place of q - 8, and do not with the weights themselves; infinities keep their sign
+    n, k = 16384, 8192
+    gen = torch.Generator(device="cuda").manual_seed(group + m)
+    w = (0.02 * torch.randn(n, k, generator=gen, device="cuda")).to(torch.bfloat16)
+    x = torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16)
+    x[0, 77] = torch.inf
+    x[1, 4000], x[1, 8191] = -torch.inf, torch.inf
+    x[2, 5] = torch.nan
+    x[3, ::97] = 3e38
+    x[4, 1024:1152] = -2e37
+    x[5, 0] = 3.3e38
+    x[m - 1, 130], x[m - 1, 131] = torch.inf, torch.inf
+    packed, sz = T.b200_int4_quantize_pack(w, group, 1e-6, True)
+    q = T.b200_int4_unpack(packed)[:n, :k].double().reshape(n, -1, group)
+    p = sz.permute(0, 2, 1, 3).reshape(packed.shape[0] * 16, -1, 2)[:n, : k // group].double()
+    wd = ((q - 8) * p[..., 0:1] + p[..., 1:2]).reshape(n, k)
+    y = T.b200_int4_weight_only_mm(x, packed, group, sz, n)
+    plain = torch.tensor([r for r in range(m) if r not in (0, 1, 2, m - 1)], device="cuda")
+    ref = x[plain].double() @ wd.t()
+    got = y[plain].double()
+    assert got.isfinite().all() and (((got - ref).norm(dim=1) / ref.norm(dim=1)) < 2.0 ** -8).all()
+    # one infinity: the sign of its weight as it is in bf16 (zero: NaN); two: NaN where the signs differ
+    sign = lambda j: wd[:, j].to(torch.bfloat16).sign()  # noqa: E731
+    for row, terms in ((0, [(77, 1)]), (1, [(4000, -1), (8191, 1)]), (m - 1, [(130, 1), (131, 1)])):
+        s = [sg * sign(j) for j, sg in terms]
+        want = torch.where((s[0] != 0) & (s[-1] == s[0]), s[0].float() * torch.inf, torch.full_like(s[0].float(), torch.nan))
+        assert torch.equal(y[row].float().isnan(), want.isnan())
+        assert torch.equal(y[row].float().nan_to_num(nan=0.0), want.nan_to_num(nan=0.0)), row
+    assert y[2].isnan().all()

@@ -4,7 +4,8 @@
 //   int4   W' = bf16_rn((q - 8) * scale + zero): the arithmetic of the reference's tinygemm op (aten._weight_int4pack_mm, behind
 //          torchao/dtypes/uintx/tensor_core_tiled_layout.py:_linear_bf16_act_uint4_weight_impl), one rounding per weight;
 //   int4, few rows (DEFER)   W' unrounded: the affine is applied in fp32 to the sums over 128 k (or a group, if that is
-//          smaller): y += s D + (z - 136 s) X with D = sum x (128 + q), X = sum x;
+//          smaller): y += s D + (z - 136 s) X with D = sum x (128 + q), X = sum x; a segment with infinities, NaN or values above
+//          2^100, where D and X are infinite and their difference is not the sum, is added up weight by weight as above;
 //   int8   W' = q, the row scale applied to the bf16-rounded sum (torchao/dtypes/uintx/plain_layout.py:250-266).
 //
 // The tensor-core mapping is transposed so that the dequantized weights never touch shared memory:
@@ -56,6 +57,8 @@ constexpr int kWqMaxW = 16, kWqMaxX = 8;       // rings of weights and of tiles 
 constexpr int kWqPitch = 128 * 2 + 16;         // bytes of a row of the output tile in shared memory (rows land on distinct banks)
 constexpr int kWqHeader = 1024;                // mbarriers, TMEM base, give-up flag
 constexpr int kWqMaxSplitTiles = 16;           // tiles per worker from which whole tiles are dealt out (imbalance <= 1/16)
+
+constexpr float kWqTop = 1.2676506e30f;        // 2^100: sums of products with 143 stay finite up to here (DEFER)
 
 struct WqParams {
   CUtensorMap wmap;          // weights: rows = strips, row = the strip's bytes; box = 8 strips x 128 k
@@ -114,14 +117,15 @@ __global__ void __launch_bounds__(256) stage_x_kernel(const __nv_bfloat16* __res
     *reinterpret_cast<uint4*>(dst + (int64_t)BR * 32) = make_uint4(v[0].z, v[1].z, v[2].z, v[3].z);
     *reinterpret_cast<uint4*>(dst + (int64_t)BR * 48) = make_uint4(v[0].w, v[1].w, v[2].w, v[3].w);
     if constexpr (SEG > 0) {
-      float s = 0.f;
+      float s = 0.f, top = 0.f;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         float f[8];
         unpack8(v[c], f);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) s += f[e];
+        for (int e = 0; e < 8; ++e) s += f[e], top = fmaxf(top, fabsf(f[e]));
       }
+      if (!(top <= kWqTop)) s = NAN;  // (a NaN among the values is in the sum already)
       if (SEG >= 64) s += __shfl_xor_sync(0xffffffffu, s, 1);
       if (SEG >= 128) s += __shfl_xor_sync(0xffffffffu, s, 2);
       if ((quarter * 32) % SEG == 0) reinterpret_cast<float*>(unit + (int64_t)BR * 256)[(quarter * 32 / SEG) * 16 + r] = s;
@@ -219,6 +223,25 @@ __device__ __forceinline__ bool wq_epi_sync(bool failed) {
                : "r"((uint32_t)failed), "n"(kWqEpiWarps * 32)
                : "memory");
   return any != 0;
+}
+// DEFER: sum over k0 <= k < k1 of x W' for one weight row and one row of x, from the unit in shared memory.  w: the strip's words;
+// x: the row's pieces, `chunk` bytes apart
+__device__ __forceinline__ float wq_exact(uint32_t w, uint32_t x, uint32_t chunk, uint32_t szw, int k0, int k1, int g, int hrow) {
+  const uint32_t s2 = __byte_perm(szw, 0, 0x1010), z2 = __byte_perm(szw, 0, 0x3232);
+  float sum = 0.f;
+#pragma unroll 1
+  for (int k = k0; k < k1; k += 8) {
+    const int q4 = k >> 5, c = (k >> 3) & 3;
+    uint32_t o[4];
+    dequant_word(lds32(w + (q4 >> 1) * 512 + (4 * g + c) * 16 + (2 * (q4 & 1) + hrow) * 4), s2, z2, o);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t xv = lds32(x + (4 * q4 + i) * chunk + c * 4);
+      sum = fmaf(__uint_as_float(xv << 16), __uint_as_float(o[i] << 16), sum);
+      sum = fmaf(__uint_as_float(xv & 0xFFFF0000u), __uint_as_float(o[i] & 0xFFFF0000u), sum);
+    }
+  }
+  return sum;
 }
 // ring position: slot and the parity of its current use
 struct WqRing {
@@ -601,8 +624,27 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
               zt[i] = fmaf(-136.f, s[i], __uint_as_float(szw & 0xFFFF0000u));
             }
             const float2 xa = lds64f(xs + sg * 64), xb = lds64f(xs + sg * 64 + 32);
-            const float X[4] = {xa.x, xa.y, xb.x, xb.y};
+            float X[4] = {xa.x, xa.y, xb.x, xb.y};
+            const bool odd = !(X[0] == X[0] && X[1] == X[1] && X[2] == X[2] && X[3] == X[3]);
             wq_ld_wait();
+            if (odd) {  // the columns whose sum is NaN, weight by weight
+              const uint32_t ws = smem_u32(wring) + w.slot * kWSlot + 2 * warp * (2 * kTileB), xr = smem_u32(xring) + (uint32_t)x.slot * p.x_bytes;
+#pragma unroll 1
+              for (int rc = 0; rc < 16; ++rc) {
+                const int r = rc >> 2, c = rc & 3, at = 8 * (r >> 1) + 4 * (c >> 1) + 2 * (r & 1) + (c & 1);
+                const float Xc = c & 2 ? (c & 1 ? X[3] : X[2]) : (c & 1 ? X[1] : X[0]);
+                if (Xc == Xc) continue;
+                const float sum = wq_exact(ws + (r >> 1) * (2 * kTileB), xr + (2 * (lane & 3) + (c & 1) + 8 * (c >> 1)) * 16, (uint32_t)p.BR * 16,
+                                           lds32(st + (r >> 1) * (kSzWords * 4) + sg * 64 + (r & 1) * 32), sg * (128 / kSegs), (sg + 1) * (128 / kSegs),
+                                           lane >> 2, r & 1);
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                  if (i == at) acc[i] += sum, v[i] = 0u;
+              }
+#pragma unroll
+              for (int c = 0; c < 4; ++c) X[c] = X[c] == X[c] ? X[c] : 0.f;
+            }
+            __syncwarp();
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
