@@ -260,14 +260,14 @@ def time_gemv_launch(engine, which, iters):
     side.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(side):
         for lin in lins[:2]:
-            lin.launch(x, y, engine.ws, side.cuda_stream)
+            lin.launch(x, y, engine.workspace(lin), side.cuda_stream)
     torch.cuda.current_stream().wait_stream(side)
     torch.cuda.synchronize()
     g = torch.cuda.CUDAGraph()
     with torch.cuda.graph(g):
         st = torch.cuda.current_stream().cuda_stream
         for lin in lins:
-            lin.launch(x, y, engine.ws, st)
+            lin.launch(x, y, engine.workspace(lin), st)
     for _ in range(3):
         g.replay()
     torch.cuda.synchronize()

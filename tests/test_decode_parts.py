@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import torchao_fork_b200 as ao
+from torchao_fork_b200 import _lib
 from torchao_fork_b200._models.llama import ModelArgs, Transformer
 from torchao_fork_b200._models.llama.decode_engine import DecodeEngine
 
@@ -55,3 +56,34 @@ def test_parts_match_single_launches(quant, inter, batch):
         out.append(torch.stack(logits))
     ref, got = out
     assert (got - ref).norm().item() < 0.011 * ref.norm().item()
+
+
+@pytest.mark.parametrize("fused", [False, True])
+def test_int8_gemm_and_int4_tickets_keep_apart(fused):
+    """int8 layers whose longest product takes the GEMM beside an int4 output projection large enough for the kernel that counts on zeroed
+    tickets (3 to 5 sequences): repeated steps give repeated logits, and the tickets are zero after each."""
+    torch.manual_seed(5)
+    cfg = ModelArgs(block_size=64, vocab_size=49152, n_layer=1, n_head=40, n_local_heads=10, dim=5120, intermediate_size=28672)
+    old = torch.get_default_dtype()
+    torch.set_default_dtype(torch.bfloat16)
+    try:
+        with torch.device("cuda"):
+            m = Transformer(cfg).eval()
+    finally:
+        torch.set_default_dtype(old)
+    ao.quantize_(m, ao.Int4WeightOnlyConfig(group_size=128), filter_fn=lambda mod, name: name == "output")
+    ao.quantize_(m, ao.Int8WeightOnlyConfig(), filter_fn=lambda mod, name: isinstance(mod, torch.nn.Linear) and name != "output")
+    m.setup_caches(4, 64, device=torch.device("cuda"))
+    eng = DecodeEngine(m, 4, 0.0, None, fused=fused)
+    # both want the front of a workspace
+    assert eng.output.kind == "int4" and eng.layers[0]["w2"].kind == "int8" and eng.layers[0]["w2"].workspace_bytes(4) > 0
+    tok, logits = torch.tensor([1, 2, 3, 4], device="cuda"), []
+    for _ in range(4):
+        eng.set_state(tok, 3)
+        eng.step()
+        logits.append(eng.logits.clone())
+    for other in logits[1:]:
+        assert torch.equal(other, logits[0])
+    # [partial sums][tickets ..]: the last kilobyte in front of the GEMM's part
+    front = int(_lib.lib().ao_b200_int4_mm_workspace_bytes(1, eng.output.np_, eng.output.kp))
+    assert not eng.ws[front - (1 << 20) : front].any()

@@ -210,11 +210,13 @@ class DecodeEngine:
         self.logits = torch.zeros(B, int(model.output.weight.shape[0]), **bf)
         self.next_tok = torch.zeros(B, dtype=torch.int64, device=dev)
         lins = [self.output] + [l[k] for l in self.layers for k in ("wqkv", "wo", "w13", "w1", "w3", "w2") if l[k]]
-        ws_bytes = max(l.workspace_bytes(B) for l in lins)
-        self.ws = torch.zeros(max(ws_bytes, 16), dtype=torch.uint8, device=dev)
-        # the GEMM that adds the residual keeps nothing between launches; the tickets in self.ws have to stay zero, so it has its own
-        self.res_ws = torch.empty(max([16] + [l[k].residual_workspace_bytes(B) for l in self.layers for k in ("wo", "w2")]),
-                                  dtype=torch.uint8, device=dev) if self.parts else None
+        # int4's workspace starts with tickets that have to stay zero between launches.  The int8 GEMM and the one that adds the residual
+        # write theirs from its first byte and keep nothing there: they have their own
+        self.ws = torch.zeros(max([16] + [l.workspace_bytes(B) for l in lins if l.kind == "int4"]), dtype=torch.uint8, device=dev)
+        scratch = [l.workspace_bytes(B) for l in lins if l.kind == "int8"]
+        if self.parts:
+            scratch += [l[k].residual_workspace_bytes(B) for l in self.layers for k in ("wo", "w2")]
+        self.scratch = torch.empty(max([16] + scratch), dtype=torch.uint8, device=dev)
         # sequence splits of the decode attention: one 32-position block per split up to S = 1024 (a block is one DRAM
         # round trip; fewer splits = fewer CTAs and a cheaper merge), <= 32 (the merge keeps one split per lane)
         self.n_split = max(1, min(32, -(-self.S // 32)))
@@ -391,8 +393,14 @@ class DecodeEngine:
         self.launches_per_step = 2 + (1 if self.temperature != 0.0 else 0)
 
     # ------------------------------------------------------------------ one step, eager launches
+    def workspace(self, lin):
+        return self.scratch if lin.kind == "int8" else self.ws
+
+    def _launch(self, lin, x, y, stream):
+        lin.launch(x, y, self.workspace(lin), stream)
+
     def _mm(self, lin, x, y, stream):
-        lin.launch(x, y, self.ws, stream)
+        self._launch(lin, x, y, stream)
         self.launches_per_step += 1
 
     def _launch_step_fused(self):
@@ -506,16 +514,16 @@ class DecodeEngine:
                 lin.launch_fused(self.h, y, st, norm_w=weight, eps=self.eps, ws=self.ws)
                 return 1
             _lib.check(L.ao_b200_rmsnorm(self.h.data_ptr(), None, weight.data_ptr(), None, self.a.data_ptr(), B, D, self.eps, st), "rmsnorm")
-            lin.launch(self.a, y, self.ws, st)
+            self._launch(lin, self.a, y, st)
             return 2
 
         def residual(lin, x):
             if lin.fused_fits(B):
                 lin.launch_fused(x, self.h, st, residual=self.h, epilogue=1, ws=self.ws)
             elif lin.residual_workspace_bytes(B):
-                lin.launch_residual(x, self.h, self.res_ws, st)
+                lin.launch_residual(x, self.h, self.scratch, st)
             else:
-                lin.launch(x, self.delta, self.ws, st)
+                self._launch(lin, x, self.delta, st)
                 self.h.add_(self.delta)
                 return 2
             return 1
@@ -533,10 +541,10 @@ class DecodeEngine:
             else:
                 _lib.check(L.ao_b200_rmsnorm(self.h.data_ptr(), None, l["ffn_norm"].data_ptr(), None, self.a.data_ptr(), B, D, self.eps, st), "rmsnorm")
                 if l["w13"] is not None:
-                    l["w13"].launch(self.a, self.gu, self.ws, st)
+                    self._launch(l["w13"], self.a, self.gu, st)
                 else:
-                    l["w1"].launch(self.a, self.gu[:, : self.I], self.ws, st)
-                    l["w3"].launch(self.a, self.gu[:, self.I:], self.ws, st)
+                    self._launch(l["w1"], self.a, self.gu[:, : self.I], st)
+                    self._launch(l["w3"], self.a, self.gu[:, self.I:], st)
                 _lib.check(L.ao_b200_silu_mul(self.gu.data_ptr(), self.s.data_ptr(), B, self.I, st), "silu_mul")
                 n += 3
             n += residual(l["w2"], self.s)
