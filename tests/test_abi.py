@@ -94,3 +94,14 @@ def test_persistent_kernel_size_queries_without_a_gpu():
     assert L.ao_b200_decode_mega_plan_bytes(ctypes.byref(model(world=3))) == 0      # world must be a power of two
     assert L.ao_b200_decode_mega_plan_bytes(ctypes.byref(model(head_dim=64))) == 0
     assert L.ao_b200_decode_mega_plan_bytes(ctypes.byref(model(group_size=48))) == 0
+
+
+@pytest.mark.parametrize("m", [17, 1000, 1 << 22, (1 << 22) + 1, 1 << 24])
+def test_every_row_count_has_a_gemm_plan(m):
+    """A workspace above the GEMV's own (int8: above nothing) says that the GEMM takes the call; without one it would be a loop of launches of
+    16 rows each.  2^24 rows are what the linears took before they had this GEMM."""
+    from torchao_fork_b200 import _lib
+    L = _lib.lib()
+    for np_, kp in ((128, 64), (256, 1024)):
+        assert L.ao_b200_int8_mm_workspace_bytes(m, np_, kp) >= m * kp * 2
+        assert L.ao_b200_int4_mm_workspace_bytes(m, np_, kp) >= L.ao_b200_int4_mm_workspace_bytes(1, np_, kp) + m * kp * 2

@@ -191,3 +191,16 @@ def test_few_rows_with_infinities_and_huge_values(group, m):
         assert torch.equal(y[row].float().isnan(), want.isnan())
         assert torch.equal(y[row].float().nan_to_num(nan=0.0), want.nan_to_num(nan=0.0)), row
     assert y[2].isnan().all()
+
+
+def test_more_than_four_million_rows():
+    m, n, k = (1 << 22) + 300, 128, 64
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    w = torch.randn(n, k, generator=gen, device="cuda").to(torch.bfloat16)
+    x = torch.randn(m, k, generator=gen, device="cuda", dtype=torch.bfloat16)
+    q, scale = T.b200_int8_quantize(w, 1e-6, True)
+    packed = T.b200_int8_pack(q)
+    y = T.b200_int8_weight_only_mm(x, packed, scale)
+    for rows in (slice(0, 700), slice(1 << 21, (1 << 21) + 300), slice(m - 513, m)):
+        ref = x[rows].double() @ (q.double() * scale.double()[:, None]).t()
+        assert ((y[rows].double() - ref).norm() / ref.norm()).item() < 2.0 ** -8

@@ -793,7 +793,7 @@ struct WqPlan {
 };
 
 static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
-  if (M <= 0 || Np % 128 != 0 || Kp % 64 != 0 || M > ((int64_t)1 << 22)) return false;
+  if (M <= 0 || Np % 128 != 0 || Kp % 64 != 0 || M > ((int64_t)1 << 24)) return false;
   w.defer = int4 && M <= 16;
   w.pair = M > 32;
   w.ranks = w.pair ? 2 : 1;
