@@ -320,7 +320,7 @@ class DecodeEngine:
         pb = int(L.ao_b200_decode_mega_plan_bytes(ctypes.byref(m)))
         assert pb > 0, "ao_b200_decode_mega: unsupported model shape"
         self._mega_trace = None
-        if trace:  # per-CTA, per-phase clock stamps (benchmarks/mega_trace.py)
+        if trace:  # per-CTA, per-phase clock stamps (mega_phase_cycles)
             self._mega_trace = torch.zeros(m.n_cta, 5 * nl + 1, 8, dtype=torch.int64, device=dev)
             m.trace = self._mega_trace.data_ptr()
         self._mega_plan = torch.zeros(pb, dtype=torch.uint8, device=dev)

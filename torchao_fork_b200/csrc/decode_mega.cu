@@ -41,7 +41,7 @@
 
 #include "common.cuh"
 
-// build-time A/B switches (benchmarks/ab_build.sh)
+// build-time A/B switches
 #ifndef AO_MEGA_POLL_SLEEP
 #define AO_MEGA_POLL_SLEEP 0    // ns between two polls of a packet that has not arrived
 #endif
@@ -142,7 +142,7 @@ struct Params {
   int stages;
   uint32_t off_x, off_S, off_red, off_h, off_misc, off_lay;
   unsigned long long timeout_ns;
-  unsigned long long* trace;      // optional: [n_cta][n_phases][8] clock64 stamps (benchmarks/mega_trace.py)
+  unsigned long long* trace;      // optional: [n_cta][n_phases][8] clock64 stamps
   int tp_reduce;                  // world > 1: sum the ranks' partial outputs once per rank (reduce_slice) instead of in every CTA
   int dbg;                        // profiling switches (AO_B200_MEGA_DEBUG): 1 = main loops skip the math (stream only), 2 = count slow polls, 4 = no evict-first hint on the weight stream
 };
