@@ -193,6 +193,19 @@ def test_few_rows_with_infinities_and_huge_values(group, m):
     assert y[2].isnan().all()
 
 
+def test_first_call_of_a_new_thread():
+    # a thread without a current context: the tensor maps have to be made all the same (without them the call is a loop of small products)
+    import threading
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    w, x = (torch.randn(r, 512, generator=gen, device="cuda").to(torch.bfloat16) for r in (640, 200))
+    packed, sz = T.b200_int4_quantize_pack(w, 128, 1e-6, True)
+    want, got = T.b200_int4_weight_only_mm(x, packed, 128, sz, 640), []
+    t = threading.Thread(target=lambda: got.append(T.b200_int4_weight_only_mm(x, packed, 128, sz, 640)))
+    t.start()
+    t.join()
+    assert torch.equal(got[0], want)
+
+
 def test_more_than_four_million_rows():
     m, n, k = (1 << 22) + 300, 128, 64
     gen = torch.Generator(device="cuda").manual_seed(1)

@@ -834,8 +834,14 @@ static WqEncode wq_encode_fn() {
 static bool wq_map(CUtensorMap* map, CUtensorMapDataType type, int elem, const void* base, int64_t row_bytes, int64_t rows, int box) {
   const cuuint64_t dims[2] = {(cuuint64_t)(row_bytes / elem), (cuuint64_t)rows}, strides[1] = {(cuuint64_t)row_bytes};
   const cuuint32_t boxes[2] = {(cuuint32_t)box, 8}, steps[2] = {1, 1};
-  return wq_encode_fn()(map, type, 2, const_cast<void*>(base), dims, strides, boxes, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  auto encode = [&]() {
+    return wq_encode_fn()(map, type, 2, const_cast<void*>(base), dims, strides, boxes, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  if (encode()) return true;
+  // a host thread that has not called the runtime yet has no current context, which the driver's encoder asks for
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess && encode();
 }
 
 template <int G, bool DEFER, bool PAIR>
