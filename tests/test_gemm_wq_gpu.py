@@ -180,7 +180,10 @@ def test_few_rows_with_infinities_and_huge_values(group, m):
     wd = ((q - 8) * p[..., 0:1] + p[..., 1:2]).reshape(n, k)
     y = T.b200_int4_weight_only_mm(x, packed, group, sz, n)
     plain = torch.tensor([r for r in range(m) if r not in (0, 1, 2, m - 1)], device="cuda")
-    ref = x[plain].double() @ wd.t()
+    # marked segments meet the weights as they are in bf16, the others unrounded ones.  (Row 4 has equal activations over a whole group: its
+    # 16 weight values occur eight times each, so their roundings add up in step, to 8 sqrt(16) / sqrt(128) = 2.8 times what they make of
+    # independent terms; against unrounded weights that is 2.8 x 2^-9 sqrt(1 / 3), close to the bound.  So it is not the reference there.)
+    ref = torch.where((x[plain].abs() > 2.0 ** 100).any(1, keepdim=True), x[plain].double() @ wd.to(torch.bfloat16).double().t(), x[plain].double() @ wd.t())
     got = y[plain].double()
     assert got.isfinite().all() and (((got - ref).norm(dim=1) / ref.norm(dim=1)) < 2.0 ** -8).all()
     # one infinity: the sign of its weight as it is in bf16 (zero: NaN); two: NaN where the signs differ
