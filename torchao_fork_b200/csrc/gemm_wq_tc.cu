@@ -4,8 +4,8 @@
 //   int4   W' = bf16_rn((q - 8) * scale + zero): the arithmetic of the reference's tinygemm op (aten._weight_int4pack_mm, behind
 //          torchao/dtypes/uintx/tensor_core_tiled_layout.py:_linear_bf16_act_uint4_weight_impl), one rounding per weight;
 //   int4, few rows (DEFER)   W' unrounded: the affine is applied in fp32 to the sums over 128 k (or a group, if that is
-//          smaller): y += s D + (z - 136 s) X with D = sum x (128 + q), X = sum x; a segment with infinities, NaN or values above
-//          2^100, where D and X are infinite and their difference is not the sum, is added up weight by weight as above;
+//          smaller): y += s D + (z - 136 s) X with D = sum x (128 + q), X = sum x; results that are not finite (x with
+//          infinities, NaN or values above 2^100, where D and X overflow) are added up weight by weight with W' as above;
 //   int8   W' = q, the row scale applied to the bf16-rounded sum (torchao/dtypes/uintx/plain_layout.py:250-266).
 //
 // The tensor-core mapping is transposed so that the dequantized weights never touch shared memory:
@@ -58,19 +58,18 @@ constexpr int kWqPitch = 128 * 2 + 16;         // bytes of a row of the output t
 constexpr int kWqHeader = 1024;                // mbarriers, TMEM base, give-up flag
 constexpr int kWqMaxSplitTiles = 16;           // tiles per worker from which whole tiles are dealt out (imbalance <= 1/16)
 
-constexpr float kWqTop = 1.2676506e30f;        // 2^100: sums of products with 143 stay finite up to here (DEFER)
-
 struct WqParams {
   CUtensorMap wmap;          // weights: rows = strips, row = the strip's bytes; box = 8 strips x 128 k
   CUtensorMap smap;          // int4 scale / zero: rows = strips, row = 16 words per group; box = 8 strips x the unit's groups
   const uint8_t* xt;         // staged activations [MT * ranks][KU][x_bytes]
+  const uint32_t *packed, *sz;  // DEFER: what the maps show, for sums that are done again
   const __nv_bfloat16* scale8;
   __nv_bfloat16* y;
   const __nv_bfloat16* residual;  // y = bf16(residual + bf16(sum)); may be y itself
   float* part;               // shares of split tiles [workers][2][ranks][NT * 128]
   uint32_t* tickets;         // [tiles][ranks], zeroed by the staging kernel
   int64_t N_out, ldy, ld_res;
-  int M, NT, BR, KU, MT, w_slots, x_slots, a_slots, n_mma, vec_store;
+  int M, Kp, NT, BR, KU, MT, w_slots, x_slots, a_slots, n_mma, vec_store;
   uint32_t off_w;            // weight ring
   long long wait_limit;      // clocks after which a wait gives up
   uint32_t x_bytes;          // one unit of staged activations (and, DEFER, its sums)
@@ -117,15 +116,14 @@ __global__ void __launch_bounds__(256) stage_x_kernel(const __nv_bfloat16* __res
     *reinterpret_cast<uint4*>(dst + (int64_t)BR * 32) = make_uint4(v[0].z, v[1].z, v[2].z, v[3].z);
     *reinterpret_cast<uint4*>(dst + (int64_t)BR * 48) = make_uint4(v[0].w, v[1].w, v[2].w, v[3].w);
     if constexpr (SEG > 0) {
-      float s = 0.f, top = 0.f;
+      float s = 0.f;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         float f[8];
         unpack8(v[c], f);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) s += f[e], top = fmaxf(top, fabsf(f[e]));
+        for (int e = 0; e < 8; ++e) s += f[e];
       }
-      if (!(top <= kWqTop)) s = NAN;  // (a NaN among the values is in the sum already)
       if (SEG >= 64) s += __shfl_xor_sync(0xffffffffu, s, 1);
       if (SEG >= 128) s += __shfl_xor_sync(0xffffffffu, s, 2);
       if ((quarter * 32) % SEG == 0) reinterpret_cast<float*>(unit + (int64_t)BR * 256)[(quarter * 32 / SEG) * 16 + r] = s;
@@ -224,24 +222,49 @@ __device__ __forceinline__ bool wq_epi_sync(bool failed) {
                : "memory");
   return any != 0;
 }
-// DEFER: sum over k0 <= k < k1 of x W' for one weight row and one row of x, from the unit in shared memory.  w: the strip's words;
-// x: the row's pieces, `chunk` bytes apart
-__device__ __forceinline__ float wq_exact(uint32_t w, uint32_t x, uint32_t chunk, uint32_t szw, int k0, int k1, int g, int hrow) {
-  const uint32_t s2 = __byte_perm(szw, 0, 0x1010), z2 = __byte_perm(szw, 0, 0x3232);
+// DEFER: the sum of x W' for one weight row and one row of x, all from global memory.  w: the strip's words; sz: the row's
+// parameters, 16 words apart per group; x: the row's pieces in the staged units
+template <int G>
+__device__ __forceinline__ float wq_exact(const uint32_t* w, const uint32_t* sz, const uint8_t* x, uint32_t x_bytes, int K, int g, int hrow) {
   float sum = 0.f;
 #pragma unroll 1
-  for (int k = k0; k < k1; k += 8) {
+  for (int k = 0; k < K; k += 8) {
     const int q4 = k >> 5, c = (k >> 3) & 3;
+    const uint32_t szw = __ldg(sz + (int64_t)(k / G) * 16);
     uint32_t o[4];
-    dequant_word(lds32(w + (q4 >> 1) * 512 + (4 * g + c) * 16 + (2 * (q4 & 1) + hrow) * 4), s2, z2, o);
+    dequant_word(__ldg(w + (int64_t)(k >> 6) * 128 + (4 * g + c) * 4 + 2 * (q4 & 1) + hrow), __byte_perm(szw, 0, 0x1010), __byte_perm(szw, 0, 0x3232), o);
+    const uint8_t* piece = x + (int64_t)(k >> 7) * x_bytes + (q4 & 3) * 4 * 256 + c * 4;  // chunks of 16 rows x 16 bytes
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const uint32_t xv = lds32(x + (4 * q4 + i) * chunk + c * 4);
+      const uint32_t xv = __ldcg(reinterpret_cast<const uint32_t*>(piece + i * 256));
       sum = fmaf(__uint_as_float(xv << 16), __uint_as_float(o[i] << 16), sum);
       sum = fmaf(__uint_as_float(xv & 0xFFFF0000u), __uint_as_float(o[i] & 0xFFFF0000u), sum);
     }
   }
   return sum;
+}
+// DEFER: eight results of row m of x that are not all finite.  D or X may have overflowed where the sum itself does not, or their difference
+// may have lost an infinity's sign, so they are done again from the weights.  Rare, and slow (a row of 8192: milliseconds); out of line and
+// asked for once per result, so that the roles' loops stay as they are (28672 x 8192, 16 rows: 45.1 us without it, 45.8 with it; staging that
+// marks such rows and an epilogue that looks at every unit: 50)
+template <int G>
+__device__ __noinline__ uint4 wq_again(const WqParams& p, uint4 v, int m, int64_t n0) {
+  uint32_t o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll 1
+  for (int e = 0; e < 8; ++e) {
+    const int n = (int)n0 + e, r = n & 15;
+    const uint32_t bits = float_to_bf16_bits(wq_exact<G>(p.packed + (int64_t)(n >> 4) * p.Kp * 2, p.sz + (int64_t)(n >> 4) * (p.Kp / G) * 16 + r,
+                                                         p.xt + m * 16, p.x_bytes, p.Kp, r & 7, r >> 3));
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i == (e >> 1)) o[i] = e & 1 ? (o[i] & 0xFFFFu) | (bits << 16) : (o[i] & 0xFFFF0000u) | bits;
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+// whether any of eight bf16 is an infinity or NaN
+__device__ __forceinline__ bool any_inf_bf16(uint4 v) {
+  const auto half = [](uint32_t w) { return (w & 0x7F80u) == 0x7F80u || (w & 0x7F800000u) == 0x7F800000u; };
+  return half(v.x) || half(v.y) || half(v.z) || half(v.w);
 }
 // ring position: slot and the parity of its current use
 struct WqRing {
@@ -385,19 +408,19 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     __nv_bfloat16* dst = p.y + (int64_t)m0 * p.ldy + n0;
     const __nv_bfloat16* res = p.residual == nullptr ? nullptr : p.residual + (int64_t)m0 * p.ld_res + n0;
     const uint32_t src = smem_u32(stage) + col * 16;
-    if (p.vec_store && n0 + 8 <= p.N_out) {
+    const bool vec = p.vec_store && n0 + 8 <= p.N_out;
 #pragma unroll 4
-      for (int m = th >> 4; m < rows; m += threads >> 4) {
-        uint4 v = lds128(src + m * kWqPitch);
+    for (int m = th >> 4; m < rows; m += threads >> 4) {
+      uint4 v = lds128(src + m * kWqPitch);
+      if constexpr (DEFER)
+        if (__builtin_expect(any_inf_bf16(v), 0)) v = wq_again<G>(p, v, m0 + m, n0);
+      if (vec) {
         if (res != nullptr) {
           const uint4 r = *reinterpret_cast<const uint4*>(res + m * p.ld_res);
           v = make_uint4(add_bf16x2(r.x, v.x), add_bf16x2(r.y, v.y), add_bf16x2(r.z, v.z), add_bf16x2(r.w, v.w));
         }
         *reinterpret_cast<uint4*>(dst + m * p.ldy) = v;
-      }
-    } else {
-      for (int m = th >> 4; m < rows; m += threads >> 4) {
-        const uint4 v = lds128(src + m * kWqPitch);
+      } else {
         const uint32_t vv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
@@ -624,27 +647,8 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
               zt[i] = fmaf(-136.f, s[i], __uint_as_float(szw & 0xFFFF0000u));
             }
             const float2 xa = lds64f(xs + sg * 64), xb = lds64f(xs + sg * 64 + 32);
-            float X[4] = {xa.x, xa.y, xb.x, xb.y};
-            const bool odd = !(X[0] == X[0] && X[1] == X[1] && X[2] == X[2] && X[3] == X[3]);
+            const float X[4] = {xa.x, xa.y, xb.x, xb.y};
             wq_ld_wait();
-            if (odd) {  // the columns whose sum is NaN, weight by weight
-              const uint32_t ws = smem_u32(wring) + w.slot * kWSlot + 2 * warp * (2 * kTileB), xr = smem_u32(xring) + (uint32_t)x.slot * p.x_bytes;
-#pragma unroll 1
-              for (int rc = 0; rc < 16; ++rc) {
-                const int r = rc >> 2, c = rc & 3, at = 8 * (r >> 1) + 4 * (c >> 1) + 2 * (r & 1) + (c & 1);
-                const float Xc = c & 2 ? (c & 1 ? X[3] : X[2]) : (c & 1 ? X[1] : X[0]);
-                if (Xc == Xc) continue;
-                const float sum = wq_exact(ws + (r >> 1) * (2 * kTileB), xr + (2 * (lane & 3) + (c & 1) + 8 * (c >> 1)) * 16, (uint32_t)p.BR * 16,
-                                           lds32(st + (r >> 1) * (kSzWords * 4) + sg * 64 + (r & 1) * 32), sg * (128 / kSegs), (sg + 1) * (128 / kSegs),
-                                           lane >> 2, r & 1);
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                  if (i == at) acc[i] += sum, v[i] = 0u;
-              }
-#pragma unroll
-              for (int c = 0; c < 4; ++c) X[c] = X[c] == X[c] ? X[c] : 0.f;
-            }
-            __syncwarp();
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -930,6 +934,9 @@ static int wq_gemm(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void
   p.ld_res = ld_res;
   p.vec_store = (ldy % 8 == 0 && ao_aligned(y, 16) && ld_res % 8 == 0 && ao_aligned(residual, 16)) ? 1 : 0;
   p.M = (int)M;
+  p.Kp = (int)Kp;
+  p.packed = static_cast<const uint32_t*>(packed);
+  p.sz = static_cast<const uint32_t*>(sz);
   p.NT = w.NT;
   p.BR = w.BR;
   p.KU = w.KU;
