@@ -182,9 +182,10 @@ AO_B200_API int ao_b200_hqq_solve(const void* w, int64_t n_groups, int group_siz
                                   void* stream);
 AO_B200_API int ao_b200_hqq_finalize(const void* w, int64_t n_groups, int group_size, const float* scale, const float* zero,
                                      int32_t* q, void* scale_out, void* zero_out, void* stream);
-/* Everything above in one call with the same results, w bf16 [N][K] contiguous, 16-byte aligned: the search (iters <= 64), then q / scale_out / zero_out as ao_b200_hqq_finalize writes them, or, with
- * q = NULL, the strip-major storage packed [Np/16][Kp/64][32][4] and scale_and_zero [Np/16][Kp/G][16][2], padding zero.
- * workspace: ao_b200_hqq_search_workspace_bytes, 8-byte aligned. */
+/* Everything above in one call with the same results; this is what quantize_ runs, the calls above are the step-by-step form that it is
+ * compared with, bit for bit.  w bf16 [N][K] contiguous, 16-byte aligned: the search (iters <= 64), then q / scale_out / zero_out as
+ * ao_b200_hqq_finalize writes them, or, with q = NULL, the strip-major storage packed [Np/16][Kp/64][32][4] and scale_and_zero
+ * [Np/16][Kp/G][16][2], padding zero.  workspace: ao_b200_hqq_search_workspace_bytes, 8-byte aligned. */
 AO_B200_API int64_t ao_b200_hqq_search_workspace_bytes(int64_t n_groups, int group_size);
 AO_B200_API int ao_b200_hqq_search(const void* w, int64_t N, int64_t K, int group_size, double beta, double kappa, double lp_norm,
                                    int iters, void* workspace, int64_t workspace_bytes, int32_t* q, void* scale_out, void* zero_out,
@@ -202,7 +203,8 @@ AO_B200_API int ao_b200_int8_unpack(const void* packed, int64_t Np, int64_t Kp, 
 /* Replacement for _linear_fp_act_int8_weight_impl (plain_layout.py:250-266):
  *   y = bf16( bf16( x @ q^T ) * scale ).   x bf16 [M][Kx] (ldx; k >= Kx reads as zero), packed strip-major int8 (Np x Kp),
  *   scale bf16 [N_out], y bf16 [M][N_out] (ldy).  few rows: TMA-ring GEMV (gemv_int8_fused.cu); more: tcgen05 GEMM
- *   (needs Np % 128 == 0 and a workspace of ao_b200_int8_mm_workspace_bytes; otherwise the GEMV is looped). */
+ *   (needs Np % 128 == 0 and a workspace of ao_b200_int8_mm_workspace_bytes, which it writes from the first byte and leaves as it is:
+ *   never the one of an int4 call, whose tickets stay zero; otherwise the GEMV is looped). */
 AO_B200_API int64_t ao_b200_int8_mm_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
 /* y = bf16(residual + bf16(x W'^T)), any M: a linear with its residual add where the activations do not fit the fused GEMV.
  * group_size 0: int8 (`scales` = bf16 row scales), else int4 (`scales` = scale_and_zero).  residual may be y itself.

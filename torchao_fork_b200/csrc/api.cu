@@ -99,8 +99,9 @@ static bool int8_by_gemm(int64_t M, int64_t Np, int64_t Kp) {
 
 extern "C" int64_t ao_b200_int4_mm_workspace_bytes(int64_t M, int64_t Np, int64_t Kp) {
   // [0, gemv): tickets + partial sums of the tensor-memory GEMV's split-K (row blocks shared by neighbouring CTAs; the
-  // tickets must stay zero between launches, so nothing else may ever be written there); [gemv, ...): the prefill
-  // GEMM's permuted copy of the activations (M > 16).  The mma.sync kernels reduce inside the CTA and need none.
+  // tickets must stay zero between launches, so nothing else may ever be written there); [gemv, ...): the GEMM's tickets,
+  // shares of split tiles and staged activations, from 3 rows on wherever it may be taken, none of which outlives a call.
+  // The mma.sync kernels reduce inside the CTA and need none.
   const int64_t gemv = ao::int4_gemv_tc_workspace_bytes(Np);
   // (up to 16 rows whether the GEMM is taken depends on the group size too: room for it wherever it may be)
   return gemv + (M >= 3 && (M > 16 || few_rows_by_gemm(M, Np, Kp, true, true) || few_rows_by_gemm(M, Np, Kp, false, true))
