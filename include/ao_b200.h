@@ -208,7 +208,8 @@ AO_B200_API int ao_b200_int8_unpack(const void* packed, int64_t Np, int64_t Kp, 
 AO_B200_API int64_t ao_b200_int8_mm_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
 /* y = bf16(residual + bf16(x W'^T)), any M: a linear with its residual add where the activations do not fit the fused GEMV.
  * group_size 0: int8 (`scales` = bf16 row scales), else int4 (`scales` = scale_and_zero).  residual may be y itself.
- * Np % 128 == 0; workspace: ao_b200_mm_residual_workspace_bytes, its contents need not survive between calls. */
+ * Np % 128 == 0; workspace: ao_b200_mm_residual_workspace_bytes, its contents need not survive between calls.  The weights must have been
+ * there before the kernel in front of this call was launched (they are read while it ends), as with the fused GEMVs. */
 AO_B200_API int64_t ao_b200_mm_residual_workspace_bytes(int64_t M, int64_t Np, int64_t Kp, int group_size);
 AO_B200_API int ao_b200_mm_residual(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scales, int64_t Np,
                                     int64_t Kp, int group_size, void* y, int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res,
