@@ -80,14 +80,15 @@ const Tunables& tunables() {
 
 // Which calls of up to 16 rows take the GEMM (gemm_wq_tc.cu) rather than the GEMV that keeps the activations in shared memory.  The GEMM
 // costs about 10 us of staging, launch and tail whatever the size, then streams 16 rows as fast as 3; the GEMV has no such costs but
-// its time grows with the rows.  Measured (GEMV / GEMM, us): int4 28672 x 8192, 8 rows 39 / 44, 12 rows 63 / 44; 14336 x 4096, 8 rows 15 / 19,
-// 12 rows 20 / 19, 16 rows 23 / 19; 4096 x 4096, 16 rows 14 / 14; int8 28672 x 8192, 12 rows 66 / 47, 14336 x 4096, 16 rows 26 / 22,
-// 4096 x 4096, 16 rows 15 / 15.  Where the activations do not fit, the strip kernels are the other choice: int4 8192 x 28672 64 / 44 from
-// 3 to 16 rows, 4096 x 14336 18 / 20; int8 8192 x 28672, 3 to 16 rows 56 .. 79 / 47, 4096 x 14336, 8 rows 18 / 23, 12 rows 27 / 23.
+// its time grows with the rows.  Measured (GEMV / GEMM, us): int4 28672 x 8192, 8 rows 39 / 46, 12 rows 62 / 46; 14336 x 4096, 8 rows 14 / 20,
+// 12 rows 19.7 / 20.3, 16 rows 23.0 / 20.4; int8 28672 x 8192, 8 rows 51 / 50, 12 rows 66 / 50, 14336 x 4096, 16 rows 25.9 / 22.7; a tie at
+// 4096 x 4096, 16 rows, where the line puts the GEMV.  Where the activations do not fit, the strip kernels are the other choice: int4
+// 8192 x 28672 62 .. 63 / 45 from 3 to 16 rows, 4096 x 14336, 16 rows 18 / 20; int8 8192 x 28672, 3 / 8 / 16 rows 55 / 59 / 78 against 49 .. 51,
+// 4096 x 14336, 8 rows 18 / 23, 12 rows 27 / 23.
 static bool few_rows_by_gemm(int64_t M, int64_t Np, int64_t Kp, bool fits, bool int4) {
   if (M < 3 || Np % 128 != 0) return false;
   if (M > 16) return true;
-  if (fits) return (M - 8) * Np * Kp >= (int64_t)224 << 20;
+  if (fits) return (M - 8) * Np * Kp > (int64_t)224 << 20;
   return Np * Kp >= (int64_t)128 << 20 || (!int4 && M > 8);
 }
 static bool int4_by_gemm(int64_t M, int64_t Np, int64_t Kp, int G) {

@@ -36,9 +36,9 @@
 //
 // Bound by the tensor cores from about 512 rows (8 MMAs of N = 256 take 1024 clocks per unit and pair, the dequant of a unit
 // about 900 clocks per set of warps, two sets in flight), below that by the dequant -> MMA chain of a unit.  Measured, 14336 x 4096,
-// int4 with groups of 128, M = 64 / 256 / 512 / 1000 / 2048: 23.6 / 37.0 / 52.6 / 90 / 168 us, the last 0.85 of 1671 TFLOP/s (one CTA
+// int4 with groups of 128, M = 64 / 256 / 512 / 1000 / 2048: 24.2 / 37.6 / 54.2 / 94 / 174 us, the last 0.85 of 1634 TFLOP/s (one CTA
 // per 128 x 256 tile with the whole K, activations multicast over 4 CTAs, run-time divisions and parameters read from global memory in
-// the dequant loop: 29.9 / 36.5 / 67.0 / 128 / 225 us); int8 8192 x 8192, M = 32 / 512 / 2048: 24 / 63 / 225 us (44 / 66 / 244 us).
+// the dequant loop: 29.9 / 36.5 / 67.0 / 128 / 225 us); int8 8192 x 8192, M = 32 / 512 / 2048: 24 / 63 / 227 us (44 / 66 / 244 us).
 #include <cuda.h>
 #include <cuda_bf16.h>
 
