@@ -1,5 +1,7 @@
 """Which calls of the linears may go past the dispatcher (ops.runs_eagerly): only those for which it would have done nothing.  On the CPU;
 the shape of every answer, or the error, is that of the registered op."""
+import weakref
+
 import pytest
 import torch
 from torch.overrides import BaseTorchFunctionMode
@@ -82,6 +84,46 @@ def test_the_blocks_of_the_llama_model_trace_in_one_graph(rows):
     plain, turned = both(x, q, freqs)
     # the norm adds up in another order: one rounding of its result, 2^-8, and of what follows
     assert torch.equal(rotated, turned) and (traced - plain).float().norm() < 2.0 ** -7 * plain.float().norm()
+
+
+def test_a_workspace_in_a_graph_is_not_given_back(monkeypatch):
+    monkeypatch.setattr(ops, "_WORKSPACES", {})
+    monkeypatch.setattr(ops, "_CAPTURED", {})
+    cpu, capturing = torch.device("cpu"), [False]
+    monkeypatch.setattr(ops, "_capturing", lambda: capturing[0])
+    refs = []
+    for inside in (False, True):
+        capturing[0] = inside
+        small = ops._workspace(cpu, 64, "int8", stream=int(inside))
+        refs.append(weakref.ref(small))
+        capturing[0] = False
+        large = ops._workspace(cpu, 128, "int8", stream=int(inside))   # takes the small one's place
+        assert large is ops._workspace(cpu, 64, "int8", stream=int(inside)) and large is not small
+        del small, large
+    assert refs[0]() is None and refs[1]() is not None
+
+
+@pytest.mark.gpu
+def test_a_graph_outlives_the_growth_of_its_workspace():
+    # int8, 12 rows by the GEMM, captured on the stream that a larger call uses afterwards
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    w, x = (torch.randn(r, 8192, generator=gen, device="cuda").bfloat16() for r in (16384, 12))
+    q, scale = T.b200_int8_quantize(w, 1e-6, True)
+    packed = T.b200_int8_pack(q)
+    want, s = T.b200_int8_weight_only_mm(x, packed, scale), torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        T.b200_int8_weight_only_mm(x, packed, scale)
+        s.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            y = T.b200_int8_weight_only_mm(x, packed, scale)
+        T.b200_int8_weight_only_mm(x.repeat(100, 1), packed, scale)
+        others = [torch.full((1 << 18,), 3.0, device="cuda") for _ in range(64)]   # what would be allocated in its place
+        s.synchronize()
+        g.replay()
+        s.synchronize()
+    assert torch.equal(y, want) and all((t == 3.0).all() for t in others)
 
 
 @pytest.mark.gpu

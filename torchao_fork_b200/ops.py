@@ -94,6 +94,7 @@ _dispatch_keys = torch._C._dispatch_keys
 _dispatch_modes, _function_modes = torch._C._len_torch_dispatch_stack, torch._C._len_torch_function_stack
 _interpreter, _tracing_state = torch._C._functorch.peek_interpreter_stack, torch._C._get_tracing_state
 _profiling = torch.autograd._profiler_enabled
+_capturing = torch.cuda.is_current_stream_capturing
 
 
 def runs_eagerly(x: Tensor, *others: Tensor) -> bool:
@@ -489,6 +490,7 @@ def _(x: Tensor, packed_w: Tensor, group_size: int, scales_and_zeros: Tensor, ou
 
 
 _WORKSPACES = {}
+_CAPTURED = {}   # address -> workspaces that a CUDA graph knows: a larger one that takes their place must not give them back
 
 
 def _workspace(device, nbytes, tag="int4", stream=None):
@@ -501,6 +503,8 @@ def _workspace(device, nbytes, tag="int4", stream=None):
     if ws is None or ws.numel() < nbytes:
         ws = torch.zeros(nbytes, dtype=torch.uint8, device=device)
         _WORKSPACES[key] = ws
+    if _capturing():
+        _CAPTURED[ws.data_ptr()] = ws
     return ws
 
 
