@@ -94,7 +94,7 @@ _dispatch_keys = torch._C._dispatch_keys
 _dispatch_modes, _function_modes = torch._C._len_torch_dispatch_stack, torch._C._len_torch_function_stack
 _interpreter, _tracing_state = torch._C._functorch.peek_interpreter_stack, torch._C._get_tracing_state
 _profiling = torch.autograd._profiler_enabled
-_capturing = torch.cuda.is_current_stream_capturing
+_capturing = torch._C._cuda_isCurrentStreamCapturing
 
 
 def runs_eagerly(x: Tensor, *others: Tensor) -> bool:
