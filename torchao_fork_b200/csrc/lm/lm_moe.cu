@@ -31,7 +31,7 @@ __device__ __forceinline__ void softmax_topk(float* z, int E, int top, int lane,
       if (ov > best || (ov == best && oi < at)) best = ov, at = oi;
     }
     if (lane == 0) {
-      idx_out[k] = at;
+      idx_out[k] = at < E ? at : 0;   // no number left to choose from (a row of NaN): an expert that exists; its weight is NaN
       weight_out[k] = expf(best - mx) / den;
     }
     __syncwarp();
@@ -301,7 +301,7 @@ __global__ void router_topk_renorm_kernel(const float* __restrict__ logits, int6
     const float p = expf(best - first);
     den += p;
     if (lane == 0) {
-      idx[t * top + k] = at;
+      idx[t * top + k] = at < E ? at : 0;            // no number left to choose from (a row of NaN): an expert that exists
       weight[t * top + k] = p;                       // divided by the sum below
       if (at < E) z[at] = -INFINITY;
     }
