@@ -404,7 +404,7 @@ AO_B200_API int ao_lm_window_attention(const float* qn, const void* kn, const vo
                                        void* stream);
 AO_B200_API int64_t ao_lm_window_attention_workspace_bytes(int n_tiles, int n_maps, int H, int G, int dv, int n_split);
 /* The same attention for prompt portions on the tensor cores (bf16 storage; d and dv multiples of 16, dv <= 128): tiles of
- * ao_lm_window_attention_prompt_plan rows (0 = shape not covered), one CTA per (tile, query head). */
+ * ao_lm_window_attention_prompt_plan rows (0 = shape not covered), one or more CTAs per (tile, query head). */
 AO_B200_API int ao_lm_window_attention_prompt_plan(int dt, int n_maps, int H, int G, int d, int dv, int* tile_rows);
 AO_B200_API int ao_lm_window_attention_prompt(const float* qn, const void* kn, const void* vn, const void* ring_k, const void* ring_v,
                                               const void* first_k, const void* first_v, int ring, int first_rows, int dt,

@@ -84,3 +84,30 @@ def test_prompt_portions_of_real_sizes(maps, d, dv, H, G, n, past, window, keep)
     assert rows.max().item() < 0.02 and ((got.double() - ref).norm() / ref.norm()).item() < 0.01, rows.topk(min(5, n))
     for _ in range(2):
         assert torch.equal(_run(q, k, v, past, window, keep, 0.4), got)
+
+
+@pytest.mark.parametrize("maps,d,dv", [(1, 128, 128), (2, 64, 128), (1, 16, 80)])
+@pytest.mark.parametrize("H,G,n", [(2, 2, 300), (12, 3, 513), (40, 8, 640), (150, 150, 500)])
+@pytest.mark.parametrize("scale", [1.0, -1.0, 0.0])
+def test_keys_of_a_tile_shared_out_over_one_to_eight_ctas(maps, d, dv, H, G, n, scale):
+    """Few tiles to many: eight, four, two shares of a tile's keys and one; some shares hold no key at all.  A negative and a zero factor of the
+    scores; result rows of odd length.  Bound as above."""
+    gen = torch.Generator(device="cuda").manual_seed(H + n + d)
+    q = torch.randn(n, H, maps, d, generator=gen, device="cuda") * 1.5
+    k, v = (torch.randn(n, G, *w, generator=gen, device="cuda").to(torch.bfloat16) for w in ((maps, d), (dv,)))
+    L, p = _lib.lm(), lambda t: t.data_ptr()
+    tile = ctypes.c_int()
+    _lib.lm_check(L.ao_lm_window_attention_prompt_plan(BF16, maps, H, G, d, dv, ctypes.byref(tile)), "plan")
+    i32 = lambda t: t.to(torch.int32).cuda()  # noqa: E731
+    first, back = torch.arange(0, n, tile.value), torch.arange(n)
+    slot, pos, tf, tc = i32(back * 0), i32(back), i32(first), i32((n - first).clamp(max=tile.value))
+    rk, rv = torch.zeros(1, 4096, G * maps * d, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, 4096, G * dv, dtype=torch.bfloat16, device="cuda")
+    for extra in (0, 1):
+        out = torch.full((n, H * dv + extra), 9.0, dtype=torch.bfloat16, device="cuda")
+        _lib.lm_check(L.ao_lm_window_attention_prompt(
+            p(q), p(k), p(v), p(rk), p(rv), None, None, 4096, 0, BF16, p(slot), p(pos), p(pos), p(tf), p(tc), tf.numel(), maps, H, G, d, dv, 4096, 0,
+            scale * d ** -0.5, 0.4, int(maps == 2), 1e-6, 1.0, p(out), H * dv + extra, torch.cuda.current_stream().cuda_stream), "prompt")
+        torch.cuda.synchronize()
+        ref = _reference(q * scale, k, v, 0, 4096, 0, 0.4)
+        assert ((out[:, : H * dv].double() - ref).norm() / ref.norm()).item() < 0.01
+        assert extra == 0 or bool((out[:, -1] == 9.0).all())

@@ -11,9 +11,11 @@
 //   the maps' difference, the norm and the constant in fp32.
 // The maps run one after the other over the same key tiles (the values come from L2 the second time); the first map's
 // normalised result waits in shared memory, each thread's own elements, for the second.
+// It takes the shapes that lm_window_attention_tc.cu does not (keys of more than 128 elements).
 // 4 warps x 16 rows.  K and V tiles arrive by cp.async in separate groups: the next keys load while the weights meet the
 // values, the next values during the score product.
 #include "lm_mma.cuh"
+#include "lm_window_attention.cuh"
 
 using namespace lm;
 
@@ -23,20 +25,6 @@ constexpr int kPM = 64;      // query rows per CTA
 constexpr int kPN = 64;      // keys per tile
 constexpr int kPWarps = 4;
 constexpr int kPad = 8;      // bf16 elements added to every shared-memory row: 16-byte rows land on distinct banks
-
-struct WinPromptArgs {
-  const float* qn;                         // [n][H][NM][d] fp32
-  const __nv_bfloat16 *kn, *vn;            // step rows [n][G][NM][d], [n][G][dv]
-  const __nv_bfloat16 *ring_k, *ring_v;    // [slots][ring][G][NM d], [slots][ring][G][dv]
-  const __nv_bfloat16 *first_k, *first_v;  // [slots][first_rows][...]
-  int ring, first_rows;
-  const int32_t *slot, *pos, *back, *tile_first, *tile_count;
-  int H, G, d, window, keep;
-  float scale, lambda, out_scale, eps;
-  int unit_rms;
-  __nv_bfloat16* out;
-  int64_t ld_out;
-};
 
 template <int NV, int NM>   // value size = 16 NV; maps per head
 __global__ void __launch_bounds__(kPWarps * 32) window_attention_prompt_kernel(WinPromptArgs a) {
@@ -317,7 +305,7 @@ int launch_win_prompt(const WinPromptArgs& a, int n_tiles, cudaStream_t st) {
 
 extern "C" int ao_lm_window_attention_prompt_plan(int dt, int n_maps, int H, int G, int d, int dv, int* tile_rows) {
   LM_CHECK_ARG(tile_rows);
-  *tile_rows = win_prompt_ok(dt, n_maps, H, G, d, dv) ? kPM : 0;
+  *tile_rows = !win_prompt_ok(dt, n_maps, H, G, d, dv) ? 0 : (win_tc_ok(n_maps, d, dv) ? kTcRows : kPM);
   return AO_B200_OK;
 }
 
@@ -342,6 +330,7 @@ extern "C" int ao_lm_window_attention_prompt(const float* qn, const void* kn, co
                   static_cast<const T*>(first_v ? first_v : ring_v), ring, first_rows, slot, pos, back, tile_first, tile_count,
                   H, G, d, window, keep, scale, lambda, out_scale, eps, unit_rms, static_cast<T*>(out), ld_out};
   const cudaStream_t st = lm_stream(stream);
+  if (win_tc_ok(n_maps, d, dv)) return launch_win_tc(a, n_maps, dv, n_tiles, st);
 #define LM_WP(NV)                                                    \
   case NV:                                                           \
     return n_maps == 2 ? launch_win_prompt<NV, 2>(a, n_tiles, st) : launch_win_prompt<NV, 1>(a, n_tiles, st);

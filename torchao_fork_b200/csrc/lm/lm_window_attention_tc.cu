@@ -1,0 +1,545 @@
+// Attention under a sliding window for prompt portions on tcgen05 / tensor memory: the computation of window_attention_prompt_kernel
+// (lm_window_attention_mma.cu: the same bf16 queries and keys, the same masks, the fp32 weights as the same three bf16 parts that add up to
+// them exactly, fp32 sums) for tiles of 128 consecutive rows of one sequence x one query head, 64 keys at a time.
+//
+//   S = Q K^T     128 x 64 fp32 in tensor memory
+//   P             exp2(S - m) in fp32, cut into bf16 parts p1 + p2 + p3 (8 bits each, by truncation: exact) and stored to tensor memory
+//                 as the A operand; p1 and p2 lie over S, which is in registers by then
+//   O += P V      three products over the same values, 128 x dv fp32 in tensor memory
+// m is a row's largest score when it last grew by more than 2^8; only then is O rescaled.  Weights stay below 2^8, and sum and product
+// carry the same factor.
+//
+// The keys of a tile are shared out over the C CTAs of a cluster (their results meet in shared memory at the end, each CTA finishes 128 / C
+// of the rows): late tiles have sixteen times the keys of early ones, and a short run has too few tiles to fill the chip.
+//
+// One step after the other: a product is waited for before anything that it read or wrote is touched again, so no hand-over depends on the
+// order in which the tensor core retires its work, and nothing is in flight at the end.  What overlaps is two CTAs per SM (256 columns of
+// tensor memory each): one makes weights while the other multiplies.  Queries, keys and values lie as [64 columns][rows][128 bytes, 16-byte
+// pieces swizzled], which the tensor core reads K-major (queries, keys) or MN-major (values).  (Without swizzle the score product
+// alone took 1340 clocks a step, twice what its operands need.)  Keys and values come by 16-byte cp.async, whole rows by neighbouring threads:
+// the next keys while the weights meet the values, the next values during the next score product.
+// Warps 0-7: loads, weights and results, two threads per row (lane quadrant = warp % 4, half of the columns = warp / 4); warp 8: products.
+// Every wait is bounded; a CTA whose wait ran out goes on without waiting, so that all meet at the end, and marks its rows with NaN.
+//
+// Bound by the chain of a step (scores -> largest -> weights -> parts -> products): about 3400 clocks of which the tensor core works 1170 (d = dv =
+// 128), two chains per SM beside one another; a CTA's start and end (queries, the peers' shares) cost 9000 more.  2048 rows x 16 heads of 128
+// (four key heads): 59.5 us, against 308 us of window_attention_prompt_kernel; the same with all keys of a tile in one CTA 110 us (the last
+// tiles alone took 95), with unswizzled operands 84 us.
+#include "lm_mma.cuh"
+#include "lm_window_attention.cuh"
+
+namespace lm {
+
+namespace {
+
+constexpr int kTcKeys = 64, kTcThreads = 288, kTcRowThreads = 256;
+constexpr uint32_t kTcHeader = 4096;                  // barriers, row exchange
+constexpr uint32_t kTcColumns = 256, kTcO = 128;      // columns 32 h ..: the scores of half h, then its p1 and p2, 16 each; 64 + 16 h ..: its p3; 128 ..: O
+// Two CTAs per SM and no third one, which would wait for tensor memory, perhaps while its cluster waits for it
+constexpr size_t kTcMinSmem = 80 * 1024;
+
+__device__ __forceinline__ uint32_t tc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// bounded: false (and *dead set) after about two seconds
+__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* dead) {
+  const uint32_t at = tc_smem(bar);
+  const long long t0 = clock64();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 32; ++i) {
+      uint32_t ok;
+      asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(at), "r"(parity) : "memory");
+      if (ok) return true;
+    }
+    if (*dead != 0 || clock64() - t0 > 4000000000ll) {
+      *dead = 1;
+      return false;
+    }
+  }
+}
+__device__ __forceinline__ bool tc_elect() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .b32 rx;\n\t.reg .pred px;\n\telect.sync rx|px, 0xffffffff;\n\tselp.u32 %0, 1, 0, px;\n\t}" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ void tc_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_commit(uint64_t* b) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(b)) : "memory");
+}
+__device__ __forceinline__ void tc_mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
+               "r"(acc)
+               : "memory");
+}
+__device__ __forceinline__ void tc_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc),
+               "r"(acc)
+               : "memory");
+}
+__device__ __forceinline__ void tc_arrive(int bar) { asm volatile("bar.arrive %0, %1;" ::"r"(bar), "n"(kTcThreads) : "memory"); }
+__device__ __forceinline__ void tc_sync(int bar) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(kTcThreads) : "memory"); }
+__device__ __forceinline__ void tc_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t tc_peer(uint32_t addr, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float tc_peer_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ float4 tc_peer_f32x4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void tc_cp16(uint32_t smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
+}
+// 32 lanes x 32 / 8 columns, thread = lane.  The load and its wait are one statement: nothing that uses the values can come between them.
+__device__ __forceinline__ void tc_ld32(uint32_t a, uint32_t (&d)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,"
+      "%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\ttcgen05.wait::ld.sync.aligned;"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]),
+        "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15]), "=r"(d[16]), "=r"(d[17]), "=r"(d[18]), "=r"(d[19]), "=r"(d[20]), "=r"(d[21]), "=r"(d[22]),
+        "=r"(d[23]), "=r"(d[24]), "=r"(d[25]), "=r"(d[26]), "=r"(d[27]), "=r"(d[28]), "=r"(d[29]), "=r"(d[30]), "=r"(d[31])
+      : "r"(a)
+      : "memory");
+}
+__device__ __forceinline__ void tc_ld8(uint32_t a, uint32_t (&d)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\ttcgen05.wait::ld.sync.aligned;"
+               : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7])
+               : "r"(a)
+               : "memory");
+}
+__device__ __forceinline__ void tc_st8(uint32_t a, const uint32_t (&d)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(a), "r"(d[0]), "r"(d[1]), "r"(d[2]), "r"(d[3]), "r"(d[4]), "r"(d[5]),
+               "r"(d[6]), "r"(d[7])
+               : "memory");
+}
+__device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// two fp32 side by side, one instruction for both, each rounded as by itself
+struct F2 {
+  uint64_t v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_get(F2 x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ float tc_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// descriptor of an operand in shared memory in rows of 128 swizzled bytes: 1024 bytes from 8 rows to the next 8; `lead` from 64 columns to the
+// next 64 (MN-major only).  (In a cluster a CTA's own addresses carry its rank above bit 24; the descriptor wants the offset.)
+__device__ __forceinline__ uint64_t tc_desc(uint32_t addr, uint32_t lead) {
+  return ((uint64_t)((1024u >> 4) | (1u << 14) | (2u << 29)) << 32) | ((lead >> 4) << 16) | ((addr & 0x3FFFFu) >> 4);
+}
+// where 16-byte piece c of row r lies in a tile of `rows` rows
+__device__ __forceinline__ uint32_t tc_at(int r, int c, int rows) { return (c >> 3) * (rows * 128) + r * 128 + (((c ^ r) & 7) << 4); }
+
+template <int NM, int C>
+__global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(WinPromptArgs a, int dv) {
+  using T = __nv_bfloat16;
+  extern __shared__ __align__(1024) unsigned char smem_tc[];
+  uint64_t* s_ready = reinterpret_cast<uint64_t*>(smem_tc);      // a step's scores are in tensor memory
+  uint64_t* o_ready = s_ready + 1;                               // its values have been added
+  uint32_t* tmem_s = reinterpret_cast<uint32_t*>(s_ready + 2);
+  volatile int* dead = reinterpret_cast<volatile int*>(tmem_s + 1);
+  float* xch = reinterpret_cast<float*>(smem_tc + 1024);         // [2 halves][128 rows] largest score, at the end sum of weights
+  float* row_m = reinterpret_cast<float*>(smem_tc + 2048);       // [128] what a row's weights are relative to, for the peers
+  float* row_l = row_m + 128;                                    // [128] their sum
+  const int d = a.d, G = a.G, KD = NM * d, kc = d / 8, vc = dv / 8, dvh = dv / 2, kb = (d + 63) / 64, vb = (dv + 63) / 64;
+  unsigned char* Qs = smem_tc + kTcHeader;                       // [kb][128 rows][128 bytes], one map at a time
+  unsigned char* Ks = Qs + kb * 16384;                           // [kb][64 keys][128 bytes]
+  unsigned char* Vs = Ks + kb * 8192;                            // [vb][64 keys][128 bytes]
+  const uint32_t pitch = dv * 4 + 16;
+  unsigned char* Ob = smem_tc + kTcHeader;                       // [128 rows][pitch] O for the peers, where Q, K and V were
+  float* Os = reinterpret_cast<float*>(Ob + max(kb * 24576 + vb * 8192, (int)(128 * pitch)));   // [128 / C rows][dv] first of two maps
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // late tiles have the most keys: those of all heads start first
+  const int64_t turn = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) / C;
+  const int rank = blockIdx.x % C;
+  const int h = (int)(turn % a.H), tile = (int)(gridDim.x / C - 1 - turn / a.H), g = h / (a.H / G);
+  const int first = a.tile_first[tile], count = min(a.tile_count[tile], kTcRows);
+  const int pa = a.pos[first];
+  const int lo = max(0, pa - a.window + 1);        // the oldest key of the first row's window
+  const int nf = min(a.keep, lo);                  // kept first positions that lie in front of it
+  const int nk = nf + (pa + count - lo);           // key index kk: the kept ones, then lo .. the last row's own position
+  const int all = (nk + kTcKeys - 1) / kTcKeys, begin = (int)((int64_t)all * rank / C), steps = (int)((int64_t)all * (rank + 1) / C) - begin;   // this CTA's
+
+  if (warp == 8) {
+    if (lane == 0) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(s_ready)) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(o_ready)) : "memory");
+      *dead = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(tmem_s)), "r"(kTcColumns));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    tc_before();
+  }
+  __syncthreads();
+  tc_after();
+  const uint32_t tb = *reinterpret_cast<volatile uint32_t*>(tmem_s);
+  uint32_t parity = 0;
+  bool ok = true;
+
+#pragma unroll 1
+  for (int m = 0; m < NM; ++m) {
+    if (warp == 8) {
+      // ---- products ----
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);              // fp32 <- bf16 x bf16, 128 rows
+      const uint32_t idesc_s = idesc | ((kTcKeys / 8u) << 17), idesc_o = idesc | (1u << 16) | ((uint32_t)vc << 17);   // values: MN-major
+      const uint64_t q_desc = tc_desc(tc_smem(Qs), 0), k_desc = tc_desc(tc_smem(Ks), 0), v_desc = tc_desc(tc_smem(Vs), 8192);
+#pragma unroll 1
+      for (int t = 0; t < steps; ++t, parity ^= 1u) {
+        tc_sync(1);                                        // keys (and, the first time, queries) are there; the parts before have been read
+        tc_after();
+        if (tc_elect() && ok) {
+          for (int ks = 0; ks < kc / 2; ++ks)              // 16 columns each
+            tc_mma_ss(tb, q_desc + (((ks >> 2) * 16384 + (ks & 3) * 32) >> 4), k_desc + (((ks >> 2) * 8192 + (ks & 3) * 32) >> 4), idesc_s, ks != 0);
+          tc_commit(s_ready);
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int b = 0; b < 2; ++b) {                      // 16 keys of either half at a time: their parts (and the values) are there
+          tc_sync(2 + b);
+          tc_after();
+          if (tc_elect() && ok) {
+#pragma unroll
+            for (int i = 0; i < 6; ++i) {
+              const int part = i >> 1, half = i & 1;
+              tc_mma_ts(tb + kTcO, part < 2 ? tb + half * 32 + part * 16 + b * 8 : tb + 64 + half * 16 + b * 8, v_desc + (2 * half + b) * (2048 >> 4), idesc_o,
+                        t > 0 || b > 0 || i > 0);
+            }
+            if (b == 1) tc_commit(o_ready);
+          }
+          __syncwarp();
+        }
+        ok = ok && tc_wait(o_ready, parity, dead);
+      }
+    } else {
+      // ---- loads, weights ----
+      const int64_t seg_row0 = first - a.back[first], s = a.slot[first];
+      const int p0 = pa - a.back[first];                   // the first position the step brings of this sequence
+      // the threads of a row take its 16-byte pieces: 2, 4, 8 or 16 threads, as many as there are pieces, or the next power of two
+      auto load = [&](unsigned char* tile_at, int t, int pieces, int width, int off, const T* step, const T* kept, const T* ring) {
+        const int wide = 32 - __clz(pieces - 1), c = threadIdx.x & ((1 << wide) - 1), rows = kTcRowThreads >> wide;
+        if (c >= pieces) return;
+        const int k0 = (begin + t) * kTcKeys, j0 = lo + (k0 - nf);
+        const uint32_t dst = tc_smem(tile_at);
+        if (k0 >= nf && j0 >= p0 && k0 + kTcKeys <= nk) {  // all from the step's own rows
+          const T* src = step + ((seg_row0 + (j0 - p0) + (threadIdx.x >> wide)) * G + g) * width + off + c * 8;
+          const int64_t next = (int64_t)rows * G * width;
+#pragma unroll 4
+          for (int row = threadIdx.x >> wide; row < kTcKeys; row += rows, src += next) tc_cp16(dst + tc_at(row, c, kTcKeys), src);
+          return;
+        }
+#pragma unroll 1
+        for (int row = threadIdx.x >> wide; row < kTcKeys; row += rows) {
+          const int kk = k0 + row;
+          const uint32_t at = tc_at(row, c, kTcKeys);
+          if (kk < nk) {
+            const int j = kk < nf ? kk : lo + (kk - nf);
+            const T* src = j >= p0 ? step + ((seg_row0 + (j - p0)) * G + g) * width
+                                   : (j < a.first_rows ? kept + ((s * a.first_rows + j) * G + g) * width : ring + ((s * a.ring + j % a.ring) * G + g) * width);
+            tc_cp16(dst + at, src + off + c * 8);
+          } else {                                         // behind the last key: zero
+            *reinterpret_cast<uint4*>(tile_at + at) = make_uint4(0, 0, 0, 0);
+          }
+        }
+      };
+      auto load_k = [&](int t) { load(Ks, t, kc, KD, m * d, a.kn, a.first_k, a.ring_k); };
+      auto load_v = [&](int t) { load(Vs, t, vc, dv, 0, a.vn, a.first_v, a.ring_v); };
+      // this thread's row of the tile and which keys it sees: kk <= see_hi and (kk >= see_lo or kk < see_keep)
+      const int q = warp & 3, half = warp >> 2, r = q * 32 + lane;
+      const uint32_t lanes = tb + ((uint32_t)(32 * q) << 16), mine = lanes + half * 32, o_mine = lanes + kTcO + half * dvh;
+      float m_ref = -INFINITY, l = 0.f;
+      if (steps > 0) {
+        load_k(0);
+        cp_async_commit();
+        // the map's queries as bf16 (rows past the run are zero)
+#pragma unroll 8
+        for (int i = threadIdx.x; i < kTcRows * kc; i += kTcRowThreads) {
+          const int row = i / kc, c = i - row * kc;
+          float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+          if (row < count) {
+            const float* src = a.qn + (((int64_t)(first + row) * a.H + h) * NM + m) * d + c * 8;
+            x = __ldg(reinterpret_cast<const float4*>(src)), y = __ldg(reinterpret_cast<const float4*>(src + 4));
+          }
+          if (a.scale < 0.f) x = make_float4(-x.x, -x.y, -x.z, -x.w), y = make_float4(-y.x, -y.y, -y.z, -y.w);
+          *reinterpret_cast<uint4*>(Qs + tc_at(row, c, kTcRows)) = make_uint4(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w), pack_bf16(y.x, y.y), pack_bf16(y.z, y.w));
+        }
+        cp_async_wait<0>();
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        tc_before();
+        tc_arrive(1);
+        load_v(0);
+        cp_async_commit();
+      }
+      const float to_log2 = fmaxf(fabsf(a.scale) * 1.4426950408889634f, 1e-37f);   // (the sign is the queries'; a hidden key stays -inf)
+#pragma unroll 1
+      for (int t = 0; t < steps; ++t, parity ^= 1u) {
+        ok = ok && tc_wait(s_ready, parity, dead);
+        tc_after();
+        uint32_t x[32];
+        tc_ld32(mine, x);
+        // the row's largest score, in units of log2
+        float top = -INFINITY;
+        {
+          const int k0 = (begin + t) * kTcKeys, base = k0 + half * 32;
+          const bool plain = k0 + kTcKeys <= nk && (k0 + kTcKeys - 1 < nf || lo + (k0 + kTcKeys - 1 - nf) <= pa) &&
+                             pa + count - 1 - (lo + max(k0 - nf, 0)) < a.window;   // every row sees every key of the step
+          if (!plain) {
+            const int hi = (r < count ? nf + (pa + r - lo) : -1) - base, low = nf + max(pa + r - a.window + 1 - lo, 0) - base;
+            const int kept = nf + max(a.keep - lo, 0) - base;
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (!(i <= hi && (i >= low || i < kept))) x[i] = 0xFF800000u;
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) top = fmaxf(top, __uint_as_float(x[i]));
+          top *= to_log2;
+        }
+        // (the two warps of a lane quadrant; the other's value of the step before has been read: both have passed o_ready since)
+        xch[half * kTcRows + r] = top;
+        asm volatile("bar.sync %0, 64;" ::"r"(4 + q) : "memory");
+        top = fmaxf(top, xch[(half ^ 1) * kTcRows + r]);
+        const bool grows = top > m_ref + 8.f;
+        if (__any_sync(0xffffffffu, grows)) {
+          const float f = grows ? tc_exp2(m_ref - top) : 1.f;
+          m_ref = grows ? top : m_ref;
+          l *= f;
+          if (t > 0) {
+            for (int c = 0; c < dvh; c += 8) {
+              uint32_t o[8];
+              tc_ld8(o_mine + c, o);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
+              tc_st8(o_mine + c, o);
+            }
+          }
+        }
+        const float m_use = m_ref == -INFINITY ? 0.f : m_ref;   // (a row that has seen no key yet)
+        const F2 c2 = f2(to_log2, to_log2), nm2 = f2(-m_use, -m_use), minus = f2(-1.f, -1.f);
+        F2 l2 = f2(0.f, 0.f);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          uint32_t p[3][8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float2 t = f2_get(f2_fma(f2(__uint_as_float(x[16 * b + 2 * i]), __uint_as_float(x[16 * b + 2 * i + 1])), c2, nm2));
+            float2 w = make_float2(tc_exp2(t.x), tc_exp2(t.y));
+            l2 = f2_add(l2, f2(w.x, w.y));
+#pragma unroll
+            for (int part = 0; part < 3; ++part) {
+              const uint32_t u0 = __float_as_uint(w.x), u1 = __float_as_uint(w.y);
+              p[part][i] = __byte_perm(u0, u1, 0x7632);    // the upper halves, side by side
+              w = f2_get(f2_fma(f2(__uint_as_float(u0 & 0xFFFF0000u), __uint_as_float(u1 & 0xFFFF0000u)), minus, f2(w.x, w.y)));   // exact
+            }
+          }
+          tc_st8(mine + b * 8, p[0]);
+          tc_st8(mine + 16 + b * 8, p[1]);
+          tc_st8(lanes + 64 + half * 16 + b * 8, p[2]);
+          tc_st_wait();
+          if (b == 0) {
+            cp_async_wait<0>();                            // the step's values
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          }
+          tc_before();
+          tc_arrive(2 + b);
+        }
+        const float2 ls = f2_get(l2);
+        l += ls.x + ls.y;
+        const bool more = t + 1 < steps;
+        if (more) load_k(t + 1);                           // the product that read this step's keys is over
+        cp_async_commit();
+        ok = ok && tc_wait(o_ready, parity, dead);
+        tc_after();
+        if (more) {
+          cp_async_wait<0>();
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          tc_before();
+          tc_arrive(1);
+          load_v(t + 1);
+          cp_async_commit();
+        }
+      }
+      // ---- this CTA's share to where the cluster reads it ----
+      xch[half * kTcRows + r] = l;
+      asm volatile("bar.sync 8, 256;" ::: "memory");       // (also: every warp is past the last product, which read Q, K and V)
+      if (half == 0) {
+        row_m[r] = m_ref;
+        row_l[r] = l + xch[kTcRows + r];
+      }
+      float* dst = reinterpret_cast<float*>(Ob + r * pitch) + half * dvh;
+      for (int c = 0; c < dvh; c += 8) {
+        uint32_t o[8];
+        tc_ld8(o_mine + c, o);
+        if (steps == 0) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o[i] = 0u;
+        }
+        *reinterpret_cast<uint4*>(dst + c) = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4*>(dst + c + 4) = make_uint4(o[4], o[5], o[6], o[7]);
+      }
+      tc_before();
+    }
+    tc_cluster_sync();
+    // ---- rows rank * 128 / C ..: 2 C threads per row, four columns at a time ----
+    if (warp < 8) {
+      constexpr int per = 2 * C;
+      const int rr = threadIdx.x / per, part = threadIdx.x % per, row = rank * (kTcRows / C) + rr;
+      float top = -INFINITY, sum = 0.f;
+      const uint32_t m_at = tc_smem(row_m + row), l_at = tc_smem(row_l + row), o_at = tc_smem(Ob) + row * pitch;
+      float f[C], ls[C];                                   // what each share counts, and its sum of weights
+#pragma unroll
+      for (int c = 0; c < C; ++c) f[c] = tc_peer_f32(tc_peer(m_at, c)), ls[c] = tc_peer_f32(tc_peer(l_at, c));
+#pragma unroll
+      for (int c = 0; c < C; ++c) top = fmaxf(top, f[c]);
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        f[c] = top == -INFINITY ? 1.f : tc_exp2(f[c] - top);
+        sum += f[c] * ls[c];
+      }
+      const float k = 1.f / sum;
+      // U pieces of four columns at a time, all shares of them in flight: use(piece, the row's four results)
+      constexpr int U = C >= 4 ? 1 : 4 / C;
+      auto results = [&](auto&& use) {
+        for (int c0 = part; c0 < dv / 4; c0 += U * per) {
+          float4 v[U][C];
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+              if (c0 + u * per < dv / 4) v[u][c] = tc_peer_f32x4(tc_peer(o_at + (c0 + u * per) * 16, c));
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int c4 = c0 + u * per;
+            if (c4 >= dv / 4) continue;
+            float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+              y.x = fmaf(f[c], v[u][c].x, y.x), y.y = fmaf(f[c], v[u][c].y, y.y), y.z = fmaf(f[c], v[u][c].z, y.z), y.w = fmaf(f[c], v[u][c].w, y.w);
+            y.x *= k, y.y *= k, y.z *= k, y.w *= k;
+            if (NM == 2 && m == 1) {
+              const float4 one = *reinterpret_cast<const float4*>(Os + (size_t)rr * dv + c4 * 4);
+              y.x = one.x - a.lambda * y.x, y.y = one.y - a.lambda * y.y, y.z = one.z - a.lambda * y.z, y.w = one.w - a.lambda * y.w;
+            }
+            use(c4, y);
+          }
+        }
+      };
+      if (m + 1 < NM) {   // the first map's result waits with the thread that made it
+        results([&](int c4, const float4& y) { *reinterpret_cast<float4*>(Os + (size_t)rr * dv + c4 * 4) = y; });
+      } else {
+        float mul = a.out_scale;
+        if (a.unit_rms) {
+          float ss = 0.f;
+          results([&](int, const float4& y) { ss = fmaf(y.x, y.x, fmaf(y.y, y.y, fmaf(y.z, y.z, fmaf(y.w, y.w, ss)))); });
+#pragma unroll
+          for (int o = per / 2; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+          mul /= sqrtf(ss / (float)dv + a.eps);
+        }
+        T* dst = a.out + (int64_t)(first + row) * a.ld_out + (int64_t)h * dv;
+        const bool wide = a.ld_out % 4 == 0 && reinterpret_cast<uintptr_t>(a.out) % 8 == 0, pairs = a.ld_out % 2 == 0;
+        if (row < count) {
+          results([&](int c4, const float4& y) {
+            const uint2 w = make_uint2(pack_bf16(y.x * mul, y.y * mul), pack_bf16(y.z * mul, y.w * mul));
+            if (wide) {
+              *reinterpret_cast<uint2*>(dst + c4 * 4) = w;
+            } else if (pairs) {
+              *reinterpret_cast<uint32_t*>(dst + c4 * 4) = w.x, *reinterpret_cast<uint32_t*>(dst + c4 * 4 + 2) = w.y;
+            } else {   // rows of odd length: every other row starts on an odd element
+              const uint32_t u[2] = {w.x, w.y};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) dst[c4 * 4 + i] = __ushort_as_bfloat16((unsigned short)(u[i >> 1] >> (16 * (i & 1))));
+            }
+          });
+        }
+      }
+    }
+    tc_cluster_sync();   // the peers have read what lies here
+  }
+  if (*dead != 0) {   // a wait ran out: all rows of the tile are marked, after the peers' results, and what is in flight gets the time to land
+    if (threadIdx.x < count)
+      for (int c = 0; c < dv; ++c) a.out[(int64_t)(first + threadIdx.x) * a.ld_out + (int64_t)h * dv + c] = __ushort_as_bfloat16((unsigned short)0x7FFF);
+    for (int i = 0; i < 64; ++i) __nanosleep(100000);
+  }
+  tc_before();
+  __syncthreads();
+  if (warp == 8) {
+    tc_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tb), "r"(kTcColumns));
+  }
+}
+
+template <int NM, int C>
+int launch(const WinPromptArgs& a, int dv, int n_tiles, cudaStream_t st) {
+  const size_t held = (size_t)((a.d + 63) / 64) * 24576 + (size_t)((dv + 63) / 64) * 8192, shares = (size_t)128 * (dv * 4 + 16);
+  size_t smem = kTcHeader + (held > shares ? held : shares) + (NM == 2 ? (size_t)(kTcRows / C) * dv * 4 : 0);
+  if (smem < kTcMinSmem) smem = kTcMinSmem;
+  auto kern = window_attention_tc_kernel<NM, C>;
+  static bool set = false;   // per instantiation
+  if (!set) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 113 * 1024) != cudaSuccess) return AO_B200_ERR_CUDA;
+    set = true;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(n_tiles * C), (unsigned)a.H);
+  cfg.blockDim = dim3(kTcThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = C;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, a, dv) == cudaSuccess) return AO_B200_OK;
+  return lm_launch_status();
+}
+
+// CTAs per tile.  Two from the 148 SMs' worth of CTAs on up to four times what the chip holds at once (2 x 148): beyond that whole tiles
+// balance by themselves, and a share costs its 9000 clocks.  Fewer tiles: as many shares as fill the chip.  Two maps always share, as the
+// first map's result of a whole tile would leave room for one CTA per SM only.
+template <int NM>
+int launch(const WinPromptArgs& a, int dv, int n_tiles, cudaStream_t st) {
+  const int64_t tiles = (int64_t)n_tiles * a.H;
+  if (tiles <= 37) return launch<NM, 8>(a, dv, n_tiles, st);
+  if (tiles <= 74) return launch<NM, 4>(a, dv, n_tiles, st);
+  if (tiles <= 592 || NM == 2) return launch<NM, 2>(a, dv, n_tiles, st);
+  return launch<1, 1>(a, dv, n_tiles, st);
+}
+
+}  // namespace
+
+int launch_win_tc(const WinPromptArgs& a, int n_maps, int dv, int n_tiles, cudaStream_t st) {
+  return n_maps == 2 ? launch<2>(a, dv, n_tiles, st) : launch<1>(a, dv, n_tiles, st);
+}
+
+}  // namespace lm
