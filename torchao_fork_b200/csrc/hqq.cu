@@ -128,19 +128,24 @@ __global__ void __launch_bounds__(kHqqWarps * 32) hqq_finalize_kernel(const __nv
 // and the block's error of each (`err`); hqq_mean_kernel adds the errors up, and whoever comes next works out
 // from the means which iteration was the last (hqq_last), so that iterations past the stop cost work but change nothing.
 //
-// Bound by instruction issue: 26.6 instructions per weight and iteration (of them 14 of arithmetic; the rest is sums, and a branch of its own
-// per weight around the power), issued in 74 % of the cycles: 172 us of ncu time for ten iterations over 4096 x 4096.  Two things keep the
-// arithmetic there.  The shrinkage
-// |d| - c |d|^(p - 1) is not positive for |d| <= c^(1 / (2 - p)) (p < 1), 0.17 at the reference's constants, which is above most
-// weights' error: powf runs only above that threshold (less a margin of 1e-3, thousands of times powf's error).  And (q - z) / s
-// is x = n r, r = rn(1 / s), corrected once, x + r (n - x s): the correctly rounded quotient by Markstein's theorem (IBM J. Res.
-// Dev. 34, 1990), as neither r nor the remainder leaves the normal range (s in [2e-38, 2e4], |n| >= 2^-24 or 0).
+// Bound by the fp32 pipe and instruction issue: ten iterations over 4096 x 4096 take about 80 us.  What keeps the arithmetic at eleven
+// instructions per pair of weights and iteration:
+//  - pairs of weights in one register pair (add, mul, fma .f32x2: the single operation's rounding in each half);
+//  - the group's smallest and largest weight bound every |d| and say whether anything is clamped, so that, as a rule, neither
+//    the clamp nor the shrinkage is looked at per weight.  |d| - c |d|^(p - 1) is not positive for |d| <= c^(1 / (2 - p)) (p < 1), 0.17 at the
+//    reference's constants, which is above most weights' error: powf runs only above that threshold (less a margin of 1e-3, thousands of
+//    times powf's error);
+//  - (q - z) / s is x = n r, r = rn(1 / s), corrected once, x + r (n - x s): the correctly rounded quotient by Markstein's theorem (IBM J. Res.
+//    Dev. 34, 1990), as neither r nor the remainder leaves the normal range (s in [2e-38, 2e4], |n| >= 2^-24 or 0);
+//  - 32 weights per thread, packed as they come: 16 registers, and half as many exchanges per weight as with 16.
 // Same numbers as hqq_step_kernel, bit for bit: there lane l of 32 adds elements l + 32 j and the lanes meet in steps of 16, 8, 4, 2, 1;
-// here thread r of L = G / 16 holds the elements of the lanes r, r + L, .. of it, so the first steps of that tree are its own.
-// quantize_ of 4096 x 4096, groups of 64, 20 iterations: 375 us against 1901 us of 20 steps and judges with a separate packing.
+// here thread r of L = G / 32 holds the elements of the lanes r, r + L, .. of it, so the first steps of that tree are its own.
+// quantize_ of 4096 x 4096, groups of 64, 20 iterations: 214 us; 375 with one weight per instruction and a branch around each power (26.6
+// instructions per weight and iteration); 1901 us of 20 steps and judges with a separate packing.
 constexpr int kHqqChunk = 10;   // iterations per launch: bounds hist to 10 numbers per group
 constexpr int kHqqMaxIters = 64;
-constexpr int kHqqPer = 16;     // weights per thread
+constexpr int kHqqPer = 32;     // weights per thread
+constexpr int kHqqBlocks = 4;   // blocks per SM: 64 registers (3 blocks of 80: 220 us; 16 weights per thread and 4 blocks: 228)
 
 struct HqqChunk {
   float inv_beta[kHqqChunk], threshold[kHqqChunk];
@@ -168,9 +173,56 @@ __device__ __noinline__ float hqq_shrink(float d, float c, float lp_m1) {
   return copysignf(fmaxf(__fsub_rn(ad, __fmul_rn(c, powf(ad, lp_m1))), 0.f), d);
 }
 
+// two fp32 in one register pair: one instruction for both, each with the single operation's rounding
+struct F2 {
+  uint64_t v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_get(F2 x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
+// sum of leaf(i) over the pairs of lanes i, i + O, i + 2 O, .. < I in the order of a tree whose last step adds neighbours O apart; leaf gives
+// the pair's sums of W_q - (W - W_e) s and of |d|
+template <int I, int O, typename Leaf>
+__device__ __forceinline__ void hqq_tree(int i, Leaf&& leaf, F2& acc, float2& e) {
+  if constexpr (O >= I) {
+    leaf(i, acc, e);
+  } else {
+    F2 acc2;
+    float2 e2;
+    hqq_tree<I, 2 * O>(i, leaf, acc, e);
+    hqq_tree<I, 2 * O>(i + O, leaf, acc2, e2);
+    acc = f2_add(acc, acc2);
+    e = make_float2(e.x + e2.x, e.y + e2.y);
+  }
+}
+
 template <int G>
-__global__ void __launch_bounds__(256) hqq_iterate_kernel(const __nv_bfloat16* __restrict__ w, int64_t n_groups, HqqChunk ch, float* __restrict__ scale,
-                                                          float* __restrict__ hist, double* __restrict__ err, const double* __restrict__ mean) {
+__global__ void __launch_bounds__(256, kHqqBlocks) hqq_iterate_kernel(const __nv_bfloat16* __restrict__ w, int64_t n_groups, HqqChunk ch,
+                                                                      float* __restrict__ scale, float* __restrict__ hist, double* __restrict__ err,
+                                                                      const double* __restrict__ mean) {
   constexpr int L = G / kHqqPer, I = 32 / L, J = G / 32;   // threads per group; its lanes per thread; elements per lane
   constexpr int kGroups = 256 / L;                         // groups per block
   constexpr float kMagic = 12582912.f;                     // 1.5 * 2^23: adding and subtracting it is rint up to 2^22, and beyond that the clamp decides
@@ -180,37 +232,26 @@ __global__ void __launch_bounds__(256) hqq_iterate_kernel(const __nv_bfloat16* _
   if (stopped) return;
   const int64_t group = ((int64_t)blockIdx.x * 256 + threadIdx.x) / L;
   const bool in = group < n_groups, first = threadIdx.x % L == 0;
-  const __nv_bfloat16* wp = w + group * G + threadIdx.x % L;
-  float v[kHqqPer], t[kHqqPer];    // element j I + i: weight i L + 32 j of the thread's
+  const unsigned short* wp = reinterpret_cast<const unsigned short*>(w) + group * G + threadIdx.x % L;
+  uint32_t v[kHqqPer / 2];         // pair (j I + i) / 2: weights i L + 32 j (lower half) and (i + 1) L + 32 j of the thread's, bf16
 #pragma unroll
   for (int j = 0; j < J; ++j)
 #pragma unroll
-    for (int i = 0; i < I; ++i) v[j * I + i] = in ? __bfloat162float(wp[32 * j + L * i]) : 0.f;
-  // sum over the group in the order of 32 lanes with J elements each
-  auto group_sum = [&](float (&x)[kHqqPer]) {
+    for (int i = 0; i < I; i += 2) v[(j * I + i) / 2] = in ? (uint32_t)wp[32 * j + L * i] | ((uint32_t)wp[32 * j + L * (i + 1)] << 16) : 0u;
+  auto weights = [&](int k) { return f2(__uint_as_float(v[k] << 16), __uint_as_float(v[k] & 0xFFFF0000u)); };
+  float mn = f2_get(weights(0)).x, mx = mn;
 #pragma unroll
-    for (int j = 1; j < J; ++j)
+  for (int k = 0; k < kHqqPer / 2; ++k) {
+    const float2 f = f2_get(weights(k));
+    mn = fminf(mn, fminf(f.x, f.y)), mx = fmaxf(mx, fmaxf(f.x, f.y));
+  }
 #pragma unroll
-      for (int i = 0; i < I; ++i) x[i] += x[j * I + i];
-#pragma unroll
-    for (int o = I / 2; o; o >>= 1)
-#pragma unroll
-      for (int i = 0; i < o; ++i) x[i] += x[i + o];
-    float r = x[0];
-#pragma unroll
-    for (int o = L / 2; o; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-    return r;
-  };
+  for (int o = L / 2; o; o >>= 1) {
+    mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  }
   float s, z;
   if (ch.first == 0) {             // (:2052-2060), as in hqq_init_kernel
-    float mn = v[0], mx = v[0];
-#pragma unroll
-    for (int j = 1; j < kHqqPer; ++j) mn = fminf(mn, v[j]), mx = fmaxf(mx, v[j]);
-#pragma unroll
-    for (int o = L / 2; o; o >>= 1) {
-      mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    }
     s = fminf(__fdiv_rn(15.f, __fsub_rn(mx, mn)), 2e4f);
     z = rintf(__fmul_rn(-mn, s));
     if (in && first) scale[group] = s;
@@ -218,26 +259,82 @@ __global__ void __launch_bounds__(256) hqq_iterate_kernel(const __nv_bfloat16* _
     s = in ? scale[group] : 1.f;
     z = in ? hist[(int64_t)(kHqqChunk - 1) * n_groups + group] : 0.f;
   }
-  const float r = __frcp_rn(s);
-#pragma unroll
-  for (int j = 0; j < kHqqPer; ++j) t[j] = __fmul_rn(v[j], s);
+  // (the minus signs ride along: -x = n (-r), its remainder n + (-x) s, and -(x + r rem) = (-r) rem + (-x), all rounded as without them)
+  const float nr = -__frcp_rn(s), t_lo = __fmul_rn(mn, s), t_hi = __fmul_rn(mx, s);
+  const F2 s2 = f2(s, s), ns2 = f2(-s, -s), nr2 = f2(nr, nr), minus = f2(-1.f, -1.f), magic = f2(kMagic, kMagic), no_magic = f2(-kMagic, -kMagic);
 #pragma unroll 1
   for (int it = 0; it < ch.count; ++it) {
-    const float c = ch.inv_beta[it], thr = ch.threshold[it];
-    float acc[kHqqPer], e[kHqqPer];
+    // (the compiler would keep all weights unpacked and multiplied beside the packed ones, and have no registers left)
 #pragma unroll
-    for (int j = 0; j < kHqqPer; ++j) {
-      const float wq = fminf(fmaxf(__fsub_rn(__fadd_rn(__fadd_rn(t[j], z), kMagic), kMagic), 0.f), 15.f);
-      const float n = __fsub_rn(wq, z), x = __fmul_rn(n, r);
-      const float wr = __fmaf_rn(__fmaf_rn(-x, s, n), r, x);
-      const float d = __fsub_rn(v[j], wr), ad = fabsf(d);
-      float u = t[j];              // (W - W_e) * scale
-      if (ad > thr) u = __fmul_rn(__fsub_rn(v[j], hqq_shrink(d, c, ch.lp_m1)), s);
-      acc[j] = __fsub_rn(wq, u);
-      e[j] = ad;
+    for (int k = 0; k < kHqqPer / 2; ++k) asm volatile("" : "+r"(v[k]));
+    const float thr = ch.threshold[it];
+    const F2 z2 = f2(z, z), nz2 = f2(-z, -z);
+    // what the group's smallest and largest weight say about all of it: no weight is clamped, and no |d| is above the threshold
+    // (|d| is half a step, or what the clamp cuts off; the margins are a hundred times the roundings of t + z and of the quotient)
+    const float q_lo = __fadd_rn(t_lo, z), q_hi = __fadd_rn(t_hi, z);
+    const bool inside = __all_sync(0xffffffffu, q_lo >= -0.5f && q_hi < 15.5f);
+    const bool small = __all_sync(0xffffffffu, (fmaxf(0.51f, fmaxf(-q_lo, q_hi - 15.f)) + (fabsf(z) + 16.f) * 1e-6f) * -nr <= 0.999f * thr);
+    auto quotients = [&](F2 f, bool clamp, F2& wq, F2& nt) {   // W_q, -W * scale and d = W - W_r of a pair
+      nt = f2_mul(f, ns2);
+      wq = f2_add(f2_add(f2_fma(nt, minus, z2), magic), no_magic);
+      if (clamp) {
+        const float2 q = f2_get(wq);
+        wq = f2(fminf(fmaxf(q.x, 0.f), 15.f), fminf(fmaxf(q.y, 0.f), 15.f));
+      }
+      const F2 n = f2_add(wq, nz2), nx = f2_mul(n, nr2);
+      return f2_get(f2_add(f, f2_fma(f2_fma(nx, s2, n), nr2, nx)));
+    };
+    auto lane_pair = [&](int i, F2& acc, float2& e, auto&& one) {   // J elements each, one after the other
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        F2 a;
+        const float2 d = one((j * I + i) / 2, a);
+        acc = j == 0 ? a : f2_add(acc, a);
+        e = j == 0 ? make_float2(fabsf(d.x), fabsf(d.y)) : make_float2(e.x + fabsf(d.x), e.y + fabsf(d.y));
+      }
+    };
+    F2 acc;
+    float2 e;
+    if (small && inside) {         // W_e = 0: mean of W_q - W * scale
+      hqq_tree<I, 2>(0, [&](int i, F2& a, float2& b) {
+        lane_pair(i, a, b, [&](int k, F2& x) {
+          F2 wq, nt;
+          const float2 d = quotients(weights(k), false, wq, nt);
+          x = f2_add(wq, nt);
+          return d;
+        });
+      }, acc, e);
+    } else if (small) {
+      hqq_tree<I, 2>(0, [&](int i, F2& a, float2& b) {
+        lane_pair(i, a, b, [&](int k, F2& x) {
+          F2 wq, nt;
+          const float2 d = quotients(weights(k), true, wq, nt);
+          x = f2_add(wq, nt);
+          return d;
+        });
+      }, acc, e);
+    } else {
+      const float c = ch.inv_beta[it];
+      hqq_tree<I, 2>(0, [&](int i, F2& a, float2& b) {
+        lane_pair(i, a, b, [&](int k, F2& x) {
+          F2 wq, nt;
+          const float2 d = quotients(weights(k), true, wq, nt), f = f2_get(weights(k)), t = f2_get(nt), q = f2_get(wq);
+          float2 u = make_float2(-t.x, -t.y);              // (W - W_e) * scale
+          if (fabsf(d.x) > thr) u.x = __fmul_rn(__fsub_rn(f.x, hqq_shrink(d.x, c, ch.lp_m1)), s);
+          if (fabsf(d.y) > thr) u.y = __fmul_rn(__fsub_rn(f.y, hqq_shrink(d.y, c, ch.lp_m1)), s);
+          x = f2(__fsub_rn(q.x, u.x), __fsub_rn(q.y, u.y));
+          return d;
+        });
+      }, acc, e);
     }
-    z = __fdiv_rn(group_sum(acc), (float)G);
-    const float es = group_sum(e);
+    const float2 last = f2_get(acc);
+    float sum = last.x + last.y, es = e.x + e.y;
+#pragma unroll
+    for (int o = L / 2; o; o >>= 1) {
+      sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      es += __shfl_xor_sync(0xffffffffu, es, o);
+    }
+    z = __fmul_rn(sum, 1.f / (float)G);                    // (a power of two: the quotient, rounded once too)
     if (first) {
       if (in) hist[(int64_t)it * n_groups + group] = z;
       s_err[it][threadIdx.x / L] = in ? es : 0.f;
@@ -302,45 +399,68 @@ __global__ void __launch_bounds__(kHqqWarps * 32) hqq_plain_kernel(const __nv_bf
   }
 }
 
-// the same straight into the strip-major storage (include/ao_b200.h): thread = 16-byte lane chunk of a (16-row strip, 64-k tile), then
-// one thread per (row, group) of the parameters; padding rows and columns are zero in both.  Bound by HBM: weights in, words out.
-__global__ void __launch_bounds__(256) hqq_packed_kernel(const __nv_bfloat16* __restrict__ w, int64_t N, int64_t K, int64_t Np, int64_t Kp, int G,
+// the same straight into the strip-major storage (include/ao_b200.h): a warp takes (16-row strip, 64-k tile) after tile, thread = 16-byte
+// lane chunk of it, and then one thread per (row, group) of the parameters; padding rows and columns are zero in both.  Bound by HBM: weights in,
+// words out.  With the group size known to the compiler and one 32-bit division per tile: 19.9 us for 4096 x 4096, against 24.6 with 64-bit
+// divisions by it in every thread.
+template <int G>
+__global__ void __launch_bounds__(256) hqq_packed_kernel(const __nv_bfloat16* __restrict__ w, int64_t N, int64_t K, int64_t Np, int64_t Kp,
                                                          const float* __restrict__ scale, const float* __restrict__ hist, const double* __restrict__ mean,
                                                          int iters, uint4* __restrict__ packed, uint32_t* __restrict__ sz) {
-  const int64_t groups = K / G, groups_p = Kp / G;
-  const float* zero = hqq_zero(hist, N * groups, mean, iters);
-  const int64_t chunks = (Np / 16) * (Kp / 64) * 32, total = chunks + Np * groups_p;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    if (i >= chunks) {
-      const int64_t o = i - chunks, row = (o / (groups_p * 16)) * 16 + (o & 15), grp = (o >> 4) % groups_p;
-      uint32_t word = 0;
-      if (row < N && grp < groups) {
-        const float s = scale[row * groups + grp], si = __fdiv_rn(1.f, s);
-        word = float_to_bf16_bits(si) | (float_to_bf16_bits(__fmul_rn(__fsub_rn(8.f, zero[row * groups + grp]), si)) << 16);
-      }
-      sz[o] = word;
-      continue;
+  constexpr int kHalves = G < 64 ? 2 : 1;   // groups per tile
+  __shared__ const float* s_zero;
+  if (threadIdx.x == 0) s_zero = hqq_zero(hist, N * (K / G), mean, iters);
+  __syncthreads();
+  const float* zero = s_zero;
+  const int64_t groups = K / G;
+  const uint32_t k_tiles = (uint32_t)(Kp / 64), groups_p = (uint32_t)(Kp / G);
+  const uint32_t tiles = (uint32_t)(Np / 16) * k_tiles;                 // < 2^32 by far: a tile is 2 KB of weights
+  const int lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+  for (uint64_t tile = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5); tile < tiles; tile += (uint64_t)gridDim.x * 8) {
+    const uint32_t strip = (uint32_t)tile / k_tiles, kt = (uint32_t)tile - strip * k_tiles;
+    const int64_t row0 = (int64_t)strip * 16 + g, k0 = (int64_t)kt * 64 + 8 * c;
+    uint4 raw[4];
+    float s[2][kHalves], z[2][kHalves];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      raw[j] = make_uint4(0u, 0u, 0u, 0u);
+      const int64_t row = row0 + 8 * (j & 1), k = k0 + 32 * (j >> 1);
+      if (row < N && k < K) raw[j] = ldg128(w + row * K + k);
     }
-    const int lane = i & 31, g = lane >> 2, c = lane & 3;
-    int64_t strip, kt;
-    tile_of_slot(i >> 5, Kp / 64, strip, kt);
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int h = 0; h < kHalves; ++h) {
+        const int64_t row = row0 + 8 * r, grp = (k0 + 32 * h) / G;
+        const bool there = row < N && grp < groups;
+        s[r][h] = there ? scale[row * groups + grp] : 0.f;              // (padding: 0 * 0 + 0)
+        z[r][h] = there ? zero[row * groups + grp] : 0.f;
+      }
     uint32_t words[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int64_t row = strip * 16 + g + 8 * (j & 1), k0 = kt * 64 + 32 * (j >> 1) + 8 * c;
+      float f[8];
+      unpack8(raw[j], f);
       uint32_t word = 0;
-      if (row < N && k0 < K) {
-        const int64_t grp = row * groups + k0 / G;
-        const float s = scale[grp], z = zero[grp];
-        float f[8];
-        unpack8(ldg128(w + row * K + k0), f);
+      const bool there = row0 + 8 * (j & 1) < N && k0 + 32 * (j >> 1) < K;
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          word |= (uint32_t)fminf(fmaxf(rintf(__fadd_rn(__fmul_rn(f[e], s), z)), 0.f), 15.f) << (4 * nib_slot(e));
-      }
-      words[j] = word;
+      for (int e = 0; e < 8; ++e)
+        word |= (uint32_t)fminf(fmaxf(rintf(__fadd_rn(__fmul_rn(f[e], s[j & 1][(j >> 1) * (kHalves - 1)]), z[j & 1][(j >> 1) * (kHalves - 1)])), 0.f), 15.f)
+                << (4 * nib_slot(e));
+      words[j] = there ? word : 0u;
     }
-    packed[i] = make_uint4(words[0], words[1], words[2], words[3]);
+    packed[tile * 32 + lane] = make_uint4(words[0], words[1], words[2], words[3]);
+  }
+  const uint64_t params = (uint64_t)Np * groups_p;
+  for (uint64_t o = (uint64_t)blockIdx.x * 256 + threadIdx.x; o < params; o += (uint64_t)gridDim.x * 256) {
+    const uint32_t pair = (uint32_t)(o >> 4), strip = pair / groups_p, grp = pair - strip * groups_p;   // [strip][group][16 rows]
+    const int64_t row = (int64_t)strip * 16 + (o & 15);
+    uint32_t word = 0;
+    if (row < N && grp < groups) {
+      const float sc = scale[row * groups + grp], si = __fdiv_rn(1.f, sc);
+      word = float_to_bf16_bits(si) | (float_to_bf16_bits(__fmul_rn(__fsub_rn(8.f, zero[row * groups + grp]), si)) << 16);
+    }
+    sz[o] = word;
   }
 }
 
@@ -486,9 +606,16 @@ extern "C" int ao_b200_hqq_search(const void* w, int64_t N, int64_t K, int group
     hqq_mean_kernel<<<ch.count, 1024, 0, s>>>(err, blocks, 1.0 / ((double)n_groups * (double)group_size), first, mean);
   }
   if (packed) {
-    const int64_t items = (Np / 16) * (Kp / 64) * 32 + Np * (Kp / group_size), want = (items + 255) / 256;
-    hqq_packed_kernel<<<(unsigned)(want < 148 * 16 ? want : 148 * 16), 256, 0, s>>>(wb, N, K, Np, Kp, group_size, scale, hist, mean, iters,
-                                                                                   static_cast<uint4*>(packed), static_cast<uint32_t*>(scale_and_zero));
+    const int64_t tiles = (Np / 16) * (Kp / 64), want = (tiles + 7) / 8;
+    const unsigned grid = (unsigned)(want < 148 * 16 ? want : 148 * 16);
+    auto* out = static_cast<uint4*>(packed);
+    auto* sz = static_cast<uint32_t*>(scale_and_zero);
+    switch (group_size) {
+      case 32: hqq_packed_kernel<32><<<grid, 256, 0, s>>>(wb, N, K, Np, Kp, scale, hist, mean, iters, out, sz); break;
+      case 64: hqq_packed_kernel<64><<<grid, 256, 0, s>>>(wb, N, K, Np, Kp, scale, hist, mean, iters, out, sz); break;
+      case 128: hqq_packed_kernel<128><<<grid, 256, 0, s>>>(wb, N, K, Np, Kp, scale, hist, mean, iters, out, sz); break;
+      default: hqq_packed_kernel<256><<<grid, 256, 0, s>>>(wb, N, K, Np, Kp, scale, hist, mean, iters, out, sz); break;
+    }
   }
   if (q) {
     const unsigned grid = (unsigned)ao_b200_hqq_blocks(n_groups);
