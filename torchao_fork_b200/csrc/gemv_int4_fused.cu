@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "gemv_stage.cuh"
 
 #ifndef AO_CHAINS
 #define AO_CHAINS 2
@@ -115,8 +116,9 @@ __device__ __forceinline__ float warp_max_f(float v) {
   return v;
 }
 
-template <int G, int MT>
-__global__ void __launch_bounds__(kFThreads, (MT == 1 ? 2 : 1)) int4_gemv_fused_kernel(const GemvFusedParams p) {
+// HR = 4, 8, 16: up to HR rows of <= NH 8-element chunks per thread staged from registers (gemv_stage.cuh); HR = 0: staging in loops
+template <int G, int MT, int NH, int HR>
+__global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) int4_gemv_fused_kernel(const GemvFusedParams p) {
   constexpr int kStageB = stage_bytes<G>();
   constexpr int SEG = G < 128 ? G : 128;  // the correction sums are kept per min(G, 128) k: a warp owns 128 k of a stage
   constexpr int U32 = SEG / 32;           // 32-k halves per accumulation segment
@@ -272,14 +274,34 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 ? 2 : 1)) int4_gemv_fused_
   const int g = lane >> 2, c = lane & 3;
   const int tid = threadIdx.x;  // 0 .. 511
   constexpr int kCT = kFConsumers * 32;
-  grid_dependency_wait();
+  if constexpr (HR == 0) grid_dependency_wait();
   AO_TRACE(5, 2);
 
   // ---- stage the activations: x (* norm_w) -> per-row power-of-two scaling -> fp16, the entries that meet a
   //      "1024 + 16 q" weight pre-divided by 16; then the per-segment correction sums ----
   const int chunks_per_row = KT * 8;  // 16-byte chunks of 8 elements over Kp
   constexpr int CPS = SEG / 8;  // chunks per segment: 4, 8 or 16
-  {
+  if constexpr (HR > 0) {
+    const auto chunk = [](const float (&f)[8], float dn, float (&sum)[2]) {   // (as in the loops below)
+      const float dn16 = dn * 0.0625f;
+      const __half2 h0 = __floats2half2_rn(f[0] * dn, f[1] * dn), h1 = __floats2half2_rn(f[2] * dn16, f[3] * dn16);
+      const __half2 h2 = __floats2half2_rn(f[4] * dn, f[5] * dn), h3 = __floats2half2_rn(f[6] * dn16, f[7] * dn16);
+      const float2 a0 = __half22float2(h0), a1 = __half22float2(h1), a2 = __half22float2(h2), a3 = __half22float2(h3);
+      const float plain = (a0.x + a0.y) + (a2.x + a2.y), div16 = (a1.x + a1.y) + (a3.x + a3.y);
+      sum[0] = plain + div16;
+      sum[1] = fmaf(16.f, div16, plain);
+      return make_uint4(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1), *reinterpret_cast<const uint32_t*>(&h2),
+                        *reinterpret_cast<const uint32_t*>(&h3));
+    };
+    const auto done = [&](int sg, int m, const float (&sum)[2]) {
+      X_s[(sg * 2 + 0) * 8 * MT + m] = sum[1];
+      X_s[(sg * 2 + 1) * 8 * MT + m] = -fmaf(1024.f, sum[0], 8.f * sum[1]);
+    };
+#pragma unroll
+    for (int row0 = 0; row0 < HR; row0 += 8)
+      stage_rows<(HR < 8 ? HR : 8), NH, kCT, 2, SEG>(p.x, p.ldx, p.Kx, row0, p.M, p.norm_w, p.eps, chunks_per_row, x_s, p.x_row_bytes, part, row_scale, chunk,
+                                                     done);
+  } else {
     // rows in batches of four: the four activation loads of a thread are in flight together (one exposed L2 round trip
     // per batch instead of one per row)
     for (int m0 = 0; m0 < p.M; m0 += 4) {
@@ -384,7 +406,6 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 ? 2 : 1)) int4_gemv_fused_
         }
       }
     }
-    named_bar_sync(1, kCT);
     AO_TRACE(5, 5);
     AO_TRACE(5, 6);
   }
@@ -611,11 +632,11 @@ static bool plan_fused(int M, int MT, int64_t Kp, int max_stages, FusedPlan& pl)
   return true;
 }
 
-template <int G, int MT>
+template <int G, int MT, int NH, int HR>
 static int launch_fused(GemvFusedParams& p, const FusedPlan& pl, bool pdl, cudaStream_t s) {
   static bool attr_done = false;
   if (!attr_done) {
-    if (cudaFuncSetAttribute(int4_gemv_fused_kernel<G, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
+    if (cudaFuncSetAttribute(int4_gemv_fused_kernel<G, MT, NH, HR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
         cudaSuccess)
       return AO_B200_ERR_CUDA;
     attr_done = true;
@@ -636,7 +657,7 @@ static int launch_fused(GemvFusedParams& p, const FusedPlan& pl, bool pdl, cudaS
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
-  if (cudaLaunchKernelEx(&cfg, int4_gemv_fused_kernel<G, MT>, p) != cudaSuccess) return AO_B200_ERR_CUDA;
+  if (cudaLaunchKernelEx(&cfg, int4_gemv_fused_kernel<G, MT, NH, HR>, p) != cudaSuccess) return AO_B200_ERR_CUDA;
   return ao_launch_status();
 }
 
@@ -688,7 +709,19 @@ int int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   }
   p.x_row_bytes = pl.x_row_bytes;
   p.off_x = pl.off_x; p.off_X = pl.off_X; p.off_red = pl.off_red; p.off_misc = pl.off_misc;
-#define AO_LF(GG) return MT == 1 ? launch_fused<GG, 1>(p, pl, pdl, s) : launch_fused<GG, 2>(p, pl, pdl, s)
+  // rows in registers: up to 16 chunks of 8 activations per thread, which leaves registers for one CTA per SM only from 8 on; so where
+  // two fit the shared memory (short rows) at most 4.  (int8_gemv_fused draws the same lines.)
+  const int n_iter = (p.KT * 8 + kFConsumers * 32 - 1) / (kFConsumers * 32);
+  const bool alone = pl.smem > 113 * 1024;
+#define AO_LF(GG)                                                                        \
+  do {                                                                                   \
+    if (MT == 2) return n_iter <= 1 ? launch_fused<GG, 2, 1, 16>(p, pl, pdl, s) : launch_fused<GG, 2, 0, 0>(p, pl, pdl, s); \
+    if (M <= 4 && n_iter <= 1) return launch_fused<GG, 1, 1, 4>(p, pl, pdl, s);          \
+    if (M <= 4 && n_iter <= 2 && alone) return launch_fused<GG, 1, 2, 4>(p, pl, pdl, s); \
+    if (n_iter <= 1 && alone) return launch_fused<GG, 1, 1, 8>(p, pl, pdl, s);           \
+    if (n_iter <= 2 && alone) return launch_fused<GG, 1, 2, 8>(p, pl, pdl, s);           \
+    return launch_fused<GG, 1, 0, 0>(p, pl, pdl, s);                                     \
+  } while (0)
   switch (G) {
     case 32: AO_LF(32);
     case 64: AO_LF(64);

@@ -20,6 +20,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "gemv_stage.cuh"
 
 namespace ao {
 
@@ -68,8 +69,8 @@ __device__ __forceinline__ void mma8_f16_16816(float (&d)[4], uint32_t a0, uint3
 __device__ __forceinline__ uint32_t u8_f16_lo(uint32_t w) { return __byte_perm(w, 0x64646464u, 0x4140); }
 __device__ __forceinline__ uint32_t u8_f16_hi(uint32_t w) { return __byte_perm(w, 0x64646464u, 0x4342); }
 
-// NH > 0: M = 1 and every consumer thread owns <= NH chunks of the activation row (register-held staging); NH = 0: the
-// general staging.  One instantiation per case — the staging code runs once per launch with a cold instruction cache, so
+// HR = 1: M = 1 and every consumer thread owns <= NH chunks of the activation row (register-held staging); HR = 4, 8, 16: up to
+// HR rows of <= NH chunks in registers (gemv_stage.cuh); HR = 0: the general staging.  One instantiation per case — the staging code runs once per launch with a cold instruction cache, so
 // code that a launch does not need is not compiled into its kernel (profiles/r01c_imma_code_size_ab.txt).
 __device__ __forceinline__ uint32_t mul_bf16x2_8(uint32_t a, uint32_t b) {
   uint32_t d;
@@ -77,8 +78,8 @@ __device__ __forceinline__ uint32_t mul_bf16x2_8(uint32_t a, uint32_t b) {
   return d;
 }
 
-template <int MT, int NH>
-__global__ void __launch_bounds__(k8Threads, (MT == 1 ? 2 : 1)) int8_gemv_fused_kernel(const Gemv8Params p) {
+template <int MT, int NH, int HR>
+__global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) int8_gemv_fused_kernel(const Gemv8Params p) {
   extern __shared__ __align__(128) uint8_t smem8[];
   uint8_t* ring = smem8;
   uint8_t* x_s = smem8 + p.off_x;                                // [M][x_row_bytes]: bf16 while staging, then scaled fp16
@@ -204,13 +205,13 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 ? 2 : 1)) int8_gemv_fused_
   const int g = lane >> 2, c = lane & 3;
   const int tid = threadIdx.x;  // 0 .. 511
   constexpr int kCT = k8Consumers * 32;
-  constexpr int kHold = NH > 0 ? NH : 1;  // chunks a thread keeps in registers between the two staging passes
+  constexpr int kHold = HR == 1 ? NH : 1;  // chunks a thread keeps in registers between the two staging passes
   const int chunks_per_row = KT * 8;  // 16-byte chunks of 8 elements over Kp
   const int n_iter = (chunks_per_row + kCT - 1) / kCT;
   // Fast path (M = 1, Kp <= 16384): every thread owns <= 4 chunks, all of their loads are issued at once, the normalised
   // bf16 values stay in registers between the two passes, every warp reduces the row statistics itself, and the norm
   // weights (independent of the previous kernel, a DRAM miss) are fetched BEFORE the dependency wait.
-  constexpr bool hold = NH > 0;  // host: p.M == 1 && n_iter <= NH
+  constexpr bool hold = HR == 1;  // host: p.M == 1 && n_iter <= NH
   uint4 xr[kHold], wn4[kHold];
 #pragma unroll
   for (int i = 0; i < kHold; ++i) xr[i] = wn4[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -221,10 +222,24 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 ? 2 : 1)) int8_gemv_fused_
       if ((int64_t)ci * 8 < p.Kx) wn4[i] = __ldg(reinterpret_cast<const uint4*>(p.norm_w + (int64_t)ci * 8));
     }
   }
-  grid_dependency_wait();
+  if constexpr (HR <= 1) grid_dependency_wait();
 
   // ---- stage the activations: x (* norm_w) -> per-row power-of-two scaling -> fp16; per-64-k correction sums ----
-  if constexpr (hold) {
+  if constexpr (HR > 1) {
+    const auto chunk = [](const float (&f)[8], float dn, float (&sum)[1]) {
+      const __half2 h0 = __floats2half2_rn(f[0] * dn, f[1] * dn), h1 = __floats2half2_rn(f[2] * dn, f[3] * dn);
+      const __half2 h2 = __floats2half2_rn(f[4] * dn, f[5] * dn), h3 = __floats2half2_rn(f[6] * dn, f[7] * dn);
+      const float2 a0 = __half22float2(h0), a1 = __half22float2(h1), a2 = __half22float2(h2), a3 = __half22float2(h3);
+      sum[0] = ((a0.x + a0.y) + (a1.x + a1.y)) + ((a2.x + a2.y) + (a3.x + a3.y));
+      return make_uint4(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1), *reinterpret_cast<const uint32_t*>(&h2),
+                        *reinterpret_cast<const uint32_t*>(&h3));
+    };
+    const auto done = [&](int seg, int m, const float (&sum)[1]) { C_s[seg * 8 * MT + m] = -1152.f * sum[0]; };
+#pragma unroll
+    for (int row0 = 0; row0 < HR; row0 += 8)
+      stage_rows<(HR < 8 ? HR : 8), NH, kCT, 1, 64>(p.x, p.ldx, p.Kx, row0, p.M, p.norm_w, p.eps, chunks_per_row, x_s, p.x_row_bytes, part, row_scale, chunk,
+                                                    done);
+  } else if constexpr (hold) {
     float ss = 0.f, amax = 0.f;
 #pragma unroll
     for (int i = 0; i < kHold; ++i) {
@@ -505,11 +520,11 @@ static int sm_count8() {
   return n;
 }
 
-template <int MT, int NH>
+template <int MT, int NH, int HR>
 static int launch8(Gemv8Params& p, const Plan8& pl, bool pdl, cudaStream_t s) {
   static bool attr_done = false;
   if (!attr_done) {
-    if (cudaFuncSetAttribute(int8_gemv_fused_kernel<MT, NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
+    if (cudaFuncSetAttribute(int8_gemv_fused_kernel<MT, NH, HR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
       return AO_B200_ERR_CUDA;
     attr_done = true;
   }
@@ -534,7 +549,7 @@ static int launch8(Gemv8Params& p, const Plan8& pl, bool pdl, cudaStream_t s) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
-  if (cudaLaunchKernelEx(&cfg, int8_gemv_fused_kernel<MT, NH>, p) != cudaSuccess) return AO_B200_ERR_CUDA;
+  if (cudaLaunchKernelEx(&cfg, int8_gemv_fused_kernel<MT, NH, HR>, p) != cudaSuccess) return AO_B200_ERR_CUDA;
   return ao_launch_status();
 }
 
@@ -568,13 +583,20 @@ int int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   p.stages = pl.stages;
   p.x_row_bytes = pl.x_row_bytes;
   p.off_x = pl.off_x; p.off_C = pl.off_C; p.off_red = pl.off_red; p.off_misc = pl.off_misc;
-  if (MT == 2) return launch8<2, 0>(p, pl, pdl, s);
-  // register-held staging: M = 1 and <= 4 chunks of 8 activations per consumer thread (Kp <= 16384)
+  // Rows in registers: chunks of 8 activations per consumer thread and row.  M = 1: <= 4 (Kp <= 16384).  More rows: up to 16 chunks in all,
+  // which leaves registers for one CTA per SM only from 8 on, so where two fit the shared memory (short rows) at most 4.
   const int n_iter = (p.KT * 8 + k8Consumers * 32 - 1) / (k8Consumers * 32);
-  if (M == 1 && n_iter <= 1) return launch8<1, 1>(p, pl, pdl, s);
-  if (M == 1 && n_iter <= 2) return launch8<1, 2>(p, pl, pdl, s);
-  if (M == 1 && n_iter <= 4) return launch8<1, 4>(p, pl, pdl, s);
-  return launch8<1, 0>(p, pl, pdl, s);
+  if (MT == 2) return n_iter <= 1 ? launch8<2, 1, 16>(p, pl, pdl, s) : launch8<2, 0, 0>(p, pl, pdl, s);
+  if (M == 1 && n_iter <= 1) return launch8<1, 1, 1>(p, pl, pdl, s);
+  if (M == 1 && n_iter <= 2) return launch8<1, 2, 1>(p, pl, pdl, s);
+  if (M == 1 && n_iter <= 4) return launch8<1, 4, 1>(p, pl, pdl, s);
+  const bool alone = pl.smem > 113 * 1024;
+  if (M <= 4 && n_iter <= 1) return launch8<1, 1, 4>(p, pl, pdl, s);
+  if (M <= 4 && n_iter <= 2 && alone) return launch8<1, 2, 4>(p, pl, pdl, s);
+  if (M <= 4 && n_iter <= 4 && alone) return launch8<1, 4, 4>(p, pl, pdl, s);
+  if (n_iter <= 1 && alone) return launch8<1, 1, 8>(p, pl, pdl, s);
+  if (n_iter <= 2 && alone) return launch8<1, 2, 8>(p, pl, pdl, s);
+  return launch8<1, 0, 0>(p, pl, pdl, s);
 }
 
 }  // namespace ao

@@ -1,0 +1,147 @@
+// Staging of the activations of a decode GEMV (gemv_int8_fused.cu, gemv_int4_fused.cu) for 2 .. 16 rows, the rows in registers: x (* norm_w)
+// -> per-row power-of-two scaling -> fp16 in shared memory, row scales, sums over a segment of k.
+//
+// The GEMVs of a batch are bound by this staging, not by their weights (which stream into the ring meanwhile): a CTA turns all
+// activations into fp16 before its first product.  8 rows of 4096, from the end of the kernel in front: 4.4 us with the norm and 3.9 without
+// (7.3 and 5.7 in loops over four rows at a time, with the values on their way through shared memory); one token of 8 sequences
+// through four layers of int8: 341 us instead of 367.
+// Here every load of a thread is in flight at once, the values stay in registers between the two passes, and where R sums are wanted over
+// the lanes of a warp, every exchange halves the number of sums a lane still holds (R = 8: 9 exchanges instead of 40).  The sums
+// are those of a butterfly per row, in the same order: same bits.
+#pragma once
+#include <cuda_fp16.h>
+
+#include "common.cuh"
+
+namespace ao {
+
+// x[j] of the lanes that differ in the bits O, O / 2, .., 1 of their number, combined; what a lane ends with belongs to row
+// (lane % (2 O)) * R / (2 O) + j, j < max(1, R / (2 O))
+template <int R, int O, typename Op>
+__device__ __forceinline__ void fold_rows(float (&x)[R], int lane, Op op) {
+  int n = R / 2;
+#pragma unroll
+  for (int o = O; o; o >>= 1, n >>= 1) {
+    if (n >= 1) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int j = 0; j < R / 2; ++j) {
+        if (j < n) {
+          const float keep = up ? x[j + n] : x[j], send = up ? x[j] : x[j + n];
+          x[j] = op(keep, __shfl_xor_sync(0xffffffffu, send, o));
+        }
+      }
+    } else {
+      x[0] = op(x[0], __shfl_xor_sync(0xffffffffu, x[0], o));
+    }
+  }
+}
+
+// Rows row0 .. row0 + R - 1 (below M), N chunks of 8 elements per row and thread, CT threads.  part: [16][CT / 32][2]; row_scale: [16].
+// chunk(f, dn, sums) -> the fp16 words of a chunk with values f, dn the row's factor; what it leaves in sums[0 .. S) is added up over the
+// SEG / 8 chunks of a segment and handed to done(segment, row, sums) by one lane per row.
+// (Sixteen rows are two calls: their 64 registers of values and the rest do not fit 96.)
+template <int R, int N, int CT, int S, int SEG, typename Chunk, typename Done>
+__device__ __forceinline__ void stage_rows(const __nv_bfloat16* x, int64_t ldx, int64_t Kx, int row0, int M, const __nv_bfloat16* norm_w, float eps,
+                                           int chunks_per_row, uint8_t* x_s, uint32_t x_row_bytes, float* part, float* row_scale, Chunk chunk, Done done) {
+  constexpr int W = CT / 32;
+  static_assert(W == 16 && (R == 4 || R == 8), "");
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const auto add = [](float a, float b) { return a + b; };
+  const auto larger = [](float a, float b) { return fmaxf(a, b); };
+  uint4 wn[N], v[N][R];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int64_t k0 = (int64_t)(i * CT + tid) * 8;
+    wn[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (norm_w != nullptr && k0 < Kx) wn[i] = __ldg(reinterpret_cast<const uint4*>(norm_w + k0));   // not the work of the kernel in front
+  }
+  grid_dependency_wait();
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int64_t k0 = (int64_t)(i * CT + tid) * 8;
+#pragma unroll
+    for (int m = 0; m < R; ++m) {
+      v[i][m] = make_uint4(0u, 0u, 0u, 0u);
+      if (row0 + m < M && k0 < Kx) v[i][m] = *reinterpret_cast<const uint4*>(x + (row0 + m) * ldx + k0);
+    }
+  }
+  float ss[R], am[R];
+#pragma unroll
+  for (int m = 0; m < R; ++m) {
+    ss[m] = am[m] = 0.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      uint4& w = v[i][m];
+      float f[8];
+      if (norm_w != nullptr) {
+        unpack8(w, f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss[m] = fmaf(f[e], f[e], ss[m]);
+        // bf16(x * w): the fp32 product of two bf16 is exact, so one packed multiply is the product rounded once
+        const auto mul = [](uint32_t a, uint32_t b) {
+          uint32_t d;
+          asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+          return d;
+        };
+        w = make_uint4(mul(w.x, wn[i].x), mul(w.y, wn[i].y), mul(w.z, wn[i].z), mul(w.w, wn[i].w));
+      }
+      unpack8(w, f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) am[m] = fmaxf(am[m], fabsf(f[e]));
+    }
+  }
+  constexpr int kOwn = 32 / R;   // lanes that end with the same row's numbers
+  fold_rows<R, 16>(ss, lane, add);
+  fold_rows<R, 16>(am, lane, larger);
+  if (lane % kOwn == 0) *reinterpret_cast<float2*>(part + ((row0 + lane / kOwn) * W + warp) * 2) = make_float2(ss[0], am[0]);
+  named_bar_sync(1, CT);
+  // every warp adds the 16 partials of all rows: half a warp, half of the rows
+  float t[R / 2], a[R / 2];
+#pragma unroll
+  for (int j = 0; j < R / 2; ++j) {
+    const float2 p = *reinterpret_cast<const float2*>(part + ((row0 + (lane >> 4) * (R / 2) + j) * W + (lane & 15)) * 2);
+    t[j] = p.x, a[j] = p.y;
+  }
+  fold_rows<R / 2, 8>(t, lane, add);
+  fold_rows<R / 2, 8>(a, lane, larger);
+  // 2^e brings the row's largest magnitude to [2^13, 2^14)
+  int e = 0;
+  if (a[0] > 0.f) e = (int)((__float_as_uint(a[0]) >> 23) & 0xFF) - 127 - 13;
+  e = max(-100, min(100, e));
+  const float up = __uint_as_float((uint32_t)(e + 127) << 23), own_dn = __uint_as_float((uint32_t)(127 - e) << 23);
+  if (warp == 0 && lane % kOwn == 0)   // for the epilogue warp
+    row_scale[row0 + lane / kOwn] = norm_w != nullptr ? up * rsqrtf(t[0] / (float)Kx + eps) : up;
+  float dn[R];
+#pragma unroll
+  for (int m = 0; m < R; ++m) dn[m] = __shfl_sync(0xffffffffu, own_dn, m * kOwn);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int ci = i * CT + tid;
+    if (ci - lane >= chunks_per_row) continue;   // (the whole warp)
+    float sums[S][R];
+#pragma unroll
+    for (int m = 0; m < R; ++m) {
+      float f[8], own[S];
+      unpack8(v[i][m], f);
+      const uint4 w = chunk(f, dn[m], own);
+      if (row0 + m < M && ci < chunks_per_row) *reinterpret_cast<uint4*>(x_s + (size_t)(row0 + m) * x_row_bytes + (size_t)ci * 16) = w;
+#pragma unroll
+      for (int s = 0; s < S; ++s) sums[s][m] = own[s];
+    }
+    constexpr int C = SEG / 8, kEach = R > C ? R / C : 1, kSame = C > R ? C / R : 1;   // lanes per segment; sums per lane, or lanes per sum
+#pragma unroll
+    for (int s = 0; s < S; ++s) fold_rows<R, C / 2>(sums[s], lane, add);
+    if (ci < chunks_per_row && lane % kSame == 0) {
+#pragma unroll
+      for (int j = 0; j < kEach; ++j) {
+        float own[S];
+#pragma unroll
+        for (int s = 0; s < S; ++s) own[s] = sums[s][j];
+        done(ci / C, row0 + (lane % C) * R / C + j, own);
+      }
+    }
+  }
+}
+
+}  // namespace ao
