@@ -215,6 +215,13 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
       const int rbuf = li % kRedBufs;
       const uint32_t use = (uint32_t)(li / kRedBufs);
       const float* rb = red + (size_t)rbuf * (kFConsumers * MT * 128);
+      __nv_bfloat16 res[MT][2][2];   // the strip's residual, fetched before the wait
+#pragma unroll
+      for (int i = 0; i < 4 * MT; ++i) {
+        const int m = 8 * (i >> 2) + 2 * c + ((i >> 1) & 1);
+        const int64_t n = 16 * (int64_t)strip + g + 8 * (i & 1);
+        res[i >> 2][(i >> 1) & 1][i & 1] = p.epilogue == kEpiResidual && m < p.M && n < p.N_out ? p.residual[m * p.ld_res + n] : __float2bfloat16_rn(0.f);
+      }
       mbar_wait(&red_full[rbuf], use & 1u);
       AO_TRACE(4, li);
       float4 sum[MT];
@@ -254,10 +261,9 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
             const int64_t n0 = 16 * (int64_t)strip + g;
             if (p.epilogue == kEpiResidual) {
               if (n0 < p.N_out)
-                p.y[m * p.ldy + n0] = __float2bfloat16_rn(__bfloat162float(p.residual[m * p.ld_res + n0]) + bf16r(v0));
+                p.y[m * p.ldy + n0] = __float2bfloat16_rn(__bfloat162float(res[mt][j][0]) + bf16r(v0));
               if (n0 + 8 < p.N_out)
-                p.y[m * p.ldy + n0 + 8] =
-                    __float2bfloat16_rn(__bfloat162float(p.residual[m * p.ld_res + n0 + 8]) + bf16r(v1));
+                p.y[m * p.ldy + n0 + 8] = __float2bfloat16_rn(__bfloat162float(res[mt][j][1]) + bf16r(v1));
             } else {
               if (n0 < p.N_out) p.y[m * p.ldy + n0] = __float2bfloat16_rn(v0);
               if (n0 + 8 < p.N_out) p.y[m * p.ldy + n0 + 8] = __float2bfloat16_rn(v1);
