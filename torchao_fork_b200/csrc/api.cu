@@ -23,6 +23,10 @@ int64_t int4_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
 int64_t int8_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
 int int8_gemv(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Kp,
               void* y, int64_t N_out, int64_t ldy, cudaStream_t s);
+int int4_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np, int64_t Kp, int G, void* y,
+                    int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res, int max_stages, bool pdl, cudaStream_t s);
+int int8_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Kp, void* y, int64_t N_out,
+                    int64_t ldy, const void* residual, int64_t ld_res, int max_stages, bool pdl, cudaStream_t s);
 int int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Np,
                     int64_t Kp, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps, const void* residual,
                     int64_t ld_res, int epilogue, int max_stages, bool pdl, cudaStream_t s);
@@ -121,6 +125,11 @@ extern "C" int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
   auto s = static_cast<cudaStream_t>(stream);
   auto xb = static_cast<const __nv_bfloat16*>(x);
   auto yb = static_cast<__nv_bfloat16*>(y);
+  if (M >= 3 && M <= 8 && !ao::int4_gemv_fused_fits(M, Kp, group_size, tunables().stages)) {   // too long for one CTA: k shared out (as in ao_b200_mm_residual)
+    const int e = ao::int4_gemv_split(x, M, Kx, ldx, packed, scale_and_zero, Np, Kp, group_size, y, N_out, ldy, nullptr, 0, tunables().stages,
+                                      tunables().pdl != 0, s);
+    if (e != AO_B200_ERR_WORKSPACE) return e;
+  }
   if (int4_by_gemm(M, Np, Kp, group_size)) {
     // tensor-memory dequant-GEMM; its part of the workspace sits after the GEMV region
     const int64_t off = ao::int4_gemv_tc_workspace_bytes(Np);
@@ -219,6 +228,10 @@ extern "C" int ao_b200_int8_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
   auto s = static_cast<cudaStream_t>(stream);
   auto xb = static_cast<const __nv_bfloat16*>(x);
   auto yb = static_cast<__nv_bfloat16*>(y);
+  if (M >= 3 && M <= 8 && !ao::int8_gemv_fused_fits(M, Kp, tunables().stages)) {   // too long for one CTA: k shared out (as in ao_b200_mm_residual)
+    const int e = ao::int8_gemv_split(x, M, Kx, ldx, packed, scale, Kp, y, N_out, ldy, nullptr, 0, tunables().stages, tunables().pdl != 0, s);
+    if (e != AO_B200_ERR_WORKSPACE) return e;
+  }
   if (int8_by_gemm(M, Np, Kp)) {
     const int e = ao::int8_gemm_tc(x, M, Kx, ldx, packed, scale, Np, Kp, y, N_out, ldy, nullptr, 0, workspace, workspace_bytes, s);
     if (e != AO_B200_ERR_WORKSPACE && e != AO_B200_ERR_UNSUPPORTED) return e;
@@ -260,6 +273,16 @@ extern "C" int ao_b200_mm_residual(const void* x, int64_t M, int64_t Kx, int64_t
   AO_CHECK_ARG(ao_aligned(x, 16) && ao_aligned(packed, 16) && ao_aligned(scales, group_size ? 64 : 2) && ao_aligned(y, 2) && ao_aligned(residual, 2));
   AO_CHECK_ARG(group_size == 0 || Kp % group_size == 0);
   auto s = static_cast<cudaStream_t>(stream);
+  // Few rows of long k: the GEMV with k shared out over a cluster stages the activations itself (8 rows of 4096 x 14336: int8 16.3 us against 22.4,
+  // int4 14.5 against 21.8; 3072 x 8192 8.8 against 17.6).  Shorter k (28672 x 4096, int8: 36 against 30) and more rows are the GEMM's; what the GEMM
+  // refuses stays refused.
+  const int64_t need = ao_b200_mm_residual_workspace_bytes(M, Np, Kp, group_size);
+  if (M <= 8 && Kp >= 8192 && need > 0 && workspace != nullptr && workspace_bytes >= need) {
+    const int e = group_size ? ao::int4_gemv_split(x, M, Kx, ldx, packed, scales, Np, Kp, group_size, y, N_out, ldy, residual, ld_res, tunables().stages,
+                                                   tunables().pdl != 0, s)
+                             : ao::int8_gemv_split(x, M, Kx, ldx, packed, scales, Kp, y, N_out, ldy, residual, ld_res, tunables().stages, tunables().pdl != 0, s);
+    if (e != AO_B200_ERR_WORKSPACE) return e;
+  }
   return group_size ? ao::int4_gemm_tc(x, M, Kx, ldx, packed, scales, Np, Kp, group_size, y, N_out, ldy, residual, ld_res, workspace, workspace_bytes, s)
                     : ao::int8_gemm_tc(x, M, Kx, ldx, packed, scales, Np, Kp, y, N_out, ldy, residual, ld_res, workspace, workspace_bytes, s);
 }

@@ -76,6 +76,8 @@ struct GemvFusedParams {
   float eps;
   uint32_t x_row_bytes;       // 2 * Kp + 16
   uint32_t off_x, off_X, off_red, off_misc;  // shared-memory carve-up (bytes)
+  int ks;                     // SPLIT: CTAs of a cluster that share a strip's k; KT is then one CTA's part of it
+  uint32_t off_inbox;
 };
 
 template <int G>
@@ -117,7 +119,8 @@ __device__ __forceinline__ float warp_max_f(float v) {
 }
 
 // HR = 4, 8, 16: up to HR rows of <= NH 8-element chunks per thread staged from registers (gemv_stage.cuh); HR = 0: staging in loops
-template <int G, int MT, int NH, int HR>
+// SPLIT: k shared out over the CTAs of a cluster (gemv_stage.cuh)
+template <int G, int MT, int NH, int HR, bool SPLIT>
 __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) int4_gemv_fused_kernel(const GemvFusedParams p) {
   constexpr int kStageB = stage_bytes<G>();
   constexpr int SEG = G < 128 ? G : 128;  // the correction sums are kept per min(G, 128) k: a warp owns 128 k of a stage
@@ -138,7 +141,8 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   AO_TRACE(5, 0);
   const int stages = p.stages;
-  const int b = blockIdx.x;
+  const int ks = SPLIT ? p.ks : 1, rank = SPLIT ? blockIdx.x % ks : 0;
+  const int b = SPLIT ? blockIdx.x / ks : blockIdx.x;
   // strips [s0, s1) of this CTA: base = n_strips / grid each, the first `rem` CTAs one more (host-computed: no division)
   const int s0 = b * p.strips_base + min(b, p.strips_rem), s1 = s0 + p.strips_base + (b < p.strips_rem ? 1 : 0);
   const int KT = p.KT;
@@ -149,6 +153,9 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
   // flight while the kernel is still waiting for its predecessor (PDL) and staging x.
   grid_launch_dependents();
   AO_TRACE(5, 1);
+  uint64_t* in_full = reinterpret_cast<uint64_t*>(smem + p.off_inbox);                                   // SPLIT, rank 0: [strips]
+  float4* inbox = reinterpret_cast<float4*>(smem + p.off_inbox + kMaxSplitStrips * 8);                   // [strips][ks - 1][MT][32 lanes]
+  if constexpr (SPLIT) split_begin(warp == kFConsumers + 1 && rank == 0, s1 - s0, in_full, (uint32_t)((ks - 1) * MT * 512), lane);
 
   if (warp == kFConsumers) {
     // ===================== producer: lane 0 owns the barriers; `copy_split` lanes share the weight copy ===============
@@ -171,8 +178,8 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
       const int n_groups = KT * 64 / G;
       const int split = p.copy_split;
       for (int strip = s0; strip < s1; ++strip) {
-        const uint8_t* wrow = p.packed + (int64_t)strip * KT * 512;
-        const uint32_t* srow = p.sz + (int64_t)strip * n_groups * 16;
+        const uint8_t* wrow = p.packed + ((int64_t)strip * ks + rank) * KT * 512;
+        const uint32_t* srow = p.sz + ((int64_t)strip * ks + rank) * n_groups * 16;
         for (int ch = 0; ch < n_chunks; ++ch) {
           const int kt0 = ch * kStageTiles;
           const int cnt = min(kStageTiles, KT - kt0);
@@ -201,6 +208,7 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     }
     __syncwarp();
     grid_dependency_wait();  // every kernel of a PDL chain must wait before it exits (transitive ordering)
+    if constexpr (SPLIT) split_meet();
     return;
   }
 
@@ -210,6 +218,7 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     const int g = lane >> 2, c = lane & 3;
     grid_dependency_wait();
     named_bar_sync(2, kFThreads);  // mbarriers initialised
+    if constexpr (SPLIT) split_meet();
     for (int strip = s0; strip < s1; ++strip) {
       const int li = strip - s0;
       const int rbuf = li % kRedBufs;
@@ -240,6 +249,8 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&red_free[rbuf]);
+      if constexpr (SPLIT)
+        if (!split_sums<MT>(sum, row_scale, in_full, inbox, li, rank, ks, lane)) continue;
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         const float vals[2][2] = {{sum[mt].x, sum[mt].z}, {sum[mt].y, sum[mt].w}};  // [col j][row half]: rows g, g+8
@@ -247,7 +258,7 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
         for (int j = 0; j < 2; ++j) {
           const int m = 8 * mt + 2 * c + j;
           if (m >= p.M) continue;
-          const float rsc = row_scale[m];
+          const float rsc = SPLIT ? 1.f : row_scale[m];
           const float v0 = vals[j][0] * rsc, v1 = vals[j][1] * rsc;
           if (p.epilogue == kEpiSiluMul) {
             // rows g = gate (w1), rows g+8 = up (w3) of output index 8*strip + g  (model.py:486)
@@ -305,7 +316,7 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     };
 #pragma unroll
     for (int row0 = 0; row0 < HR; row0 += 8)
-      stage_rows<(HR < 8 ? HR : 8), NH, kCT, 2, SEG>(p.x, p.ldx, p.Kx, row0, p.M, p.norm_w, p.eps, chunks_per_row, x_s, p.x_row_bytes, part, row_scale, chunk,
+      stage_rows<(HR < 8 ? HR : 8), NH, kCT, 2, SEG>(p.x + (int64_t)rank * KT * 64, p.ldx, SPLIT ? min(p.Kx - (int64_t)rank * KT * 64, (int64_t)KT * 64) : p.Kx, row0, p.M, p.norm_w, p.eps, chunks_per_row, x_s, p.x_row_bytes, part, row_scale, chunk,
                                                      done);
   } else {
     // rows in batches of four: the four activation loads of a thread are in flight together (one exposed L2 round trip
@@ -579,6 +590,7 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     __syncwarp();
     if (lane == 0) mbar_arrive(&red_full[rbuf]);
   }
+  if constexpr (SPLIT) split_meet();
 }
 
 // ------------------------------------------------------------------------------------------------ host side
@@ -596,19 +608,19 @@ static int fused_sm_count() {
 struct FusedPlan {
   int stages;
   size_t smem;
-  uint32_t off_x, off_X, off_red, off_misc, x_row_bytes;
+  uint32_t off_x, off_X, off_red, off_misc, off_inbox, x_row_bytes;
 };
 
 // shared-memory plan; returns false when the activations do not fit (caller falls back to the strip kernel)
 template <int G>
-static bool plan_fused(int M, int MT, int64_t Kp, int max_stages, FusedPlan& pl) {
+static bool plan_fused(int M, int MT, int64_t Kp, int max_stages, FusedPlan& pl, size_t inbox = 0) {   // inbox: bytes behind the rest, one CTA per SM
   const size_t stage_b = stage_bytes<G>();
   pl.x_row_bytes = (uint32_t)(2 * Kp + 16);
   const size_t x_bytes = ((size_t)M * pl.x_row_bytes + 127) / 128 * 128;
   const size_t X_bytes = ((size_t)(Kp / (G < 128 ? G : 128)) * 2 * 8 * MT * 4 + 127) / 128 * 128;
   const size_t red_bytes = (size_t)kRedBufs * kFConsumers * MT * 128 * 4;
   const size_t misc = (16 * kFConsumers * 2 + 32) * 4 + (2 * 16 + 2 * kRedBufs) * 8 + 64;
-  const size_t fixed = x_bytes + X_bytes + red_bytes + misc;
+  const size_t fixed = x_bytes + X_bytes + red_bytes + misc + inbox;
   static const size_t two_per_sm = []() {  // AO_B200_SMEM_KB: shared-memory budget per CTA (default: two CTAs per SM)
     const char* e = std::getenv("AO_B200_SMEM_KB");
     return (size_t)(e ? std::atoi(e) : 113) * 1024;
@@ -619,7 +631,7 @@ static bool plan_fused(int M, int MT, int64_t Kp, int max_stages, FusedPlan& pl)
     const char* e = std::getenv("AO_B200_MIN_STAGES2");
     return (size_t)(e ? std::atoi(e) : 4);  // 3 measured slower on w2 (K = 14336): 394 vs 350 us per 32 layers
   }();
-  if (fixed + min2 * stage_b <= two_per_sm) {
+  if (inbox == 0 && fixed + min2 * stage_b <= two_per_sm) {
     st = (int)((two_per_sm - fixed) / stage_b);
   } else if (fixed + 3 * stage_b <= one_per_sm) {
     st = (int)((one_per_sm - fixed) / stage_b);
@@ -634,6 +646,7 @@ static bool plan_fused(int M, int MT, int64_t Kp, int max_stages, FusedPlan& pl)
   pl.off_X = (uint32_t)off; off += X_bytes;
   pl.off_red = (uint32_t)off; off += red_bytes;
   pl.off_misc = (uint32_t)off; off += misc;
+  pl.off_inbox = (uint32_t)((off + 15) / 16 * 16); off += inbox;
   pl.smem = off;
   return true;
 }
@@ -642,7 +655,7 @@ template <int G, int MT, int NH, int HR>
 static int launch_fused(GemvFusedParams& p, const FusedPlan& pl, bool pdl, cudaStream_t s) {
   static bool attr_done = false;
   if (!attr_done) {
-    if (cudaFuncSetAttribute(int4_gemv_fused_kernel<G, MT, NH, HR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
+    if (cudaFuncSetAttribute(int4_gemv_fused_kernel<G, MT, NH, HR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
         cudaSuccess)
       return AO_B200_ERR_CUDA;
     attr_done = true;
@@ -663,8 +676,87 @@ static int launch_fused(GemvFusedParams& p, const FusedPlan& pl, bool pdl, cudaS
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
-  if (cudaLaunchKernelEx(&cfg, int4_gemv_fused_kernel<G, MT, NH, HR>, p) != cudaSuccess) return AO_B200_ERR_CUDA;
+  if (cudaLaunchKernelEx(&cfg, int4_gemv_fused_kernel<G, MT, NH, HR, false>, p) != cudaSuccess) return AO_B200_ERR_CUDA;
   return ao_launch_status();
+}
+
+template <int G, int MT, int NH, int HR>
+static int launch_split(GemvFusedParams& p, int M, int64_t Kp, int max_stages, bool pdl, cudaStream_t s) {
+  auto kern = int4_gemv_fused_kernel<G, MT, NH, HR, true>;
+  static bool attr_done = false;
+  if (!attr_done) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return AO_B200_ERR_CUDA;
+    attr_done = true;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(kFThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.ks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 2 : 1;
+  static int at_once[5] = {};
+  int clusters = split_clusters(reinterpret_cast<const void*>(kern), cfg, p.ks, fused_sm_count(), at_once);
+  if (clusters <= 0) return AO_B200_ERR_WORKSPACE;
+  if (clusters > p.n_strips) clusters = p.n_strips;
+  const int most = (p.n_strips + clusters - 1) / clusters;
+  if (most > kMaxSplitStrips) return AO_B200_ERR_WORKSPACE;
+  FusedPlan pl;
+  if (!plan_fused<G>(M, MT, Kp / p.ks, max_stages, pl, kMaxSplitStrips * 8 + 16 + (size_t)most * (p.ks - 1) * MT * 512)) return AO_B200_ERR_WORKSPACE;
+  if (pl.smem <= 113 * 1024) pl.smem = 114 * 1024;   // (one CTA per SM)
+  p.stages = pl.stages;
+  p.x_row_bytes = pl.x_row_bytes;
+  p.off_x = pl.off_x; p.off_X = pl.off_X; p.off_red = pl.off_red; p.off_misc = pl.off_misc; p.off_inbox = pl.off_inbox;
+  p.strips_base = p.n_strips / clusters;
+  p.strips_rem = p.n_strips % clusters;
+  cfg.gridDim = dim3((unsigned)(clusters * p.ks));
+  cfg.dynamicSmemBytes = pl.smem;
+  if (cudaLaunchKernelEx(&cfg, kern, p) != cudaSuccess) return AO_B200_ERR_CUDA;
+  return ao_launch_status();
+}
+
+template <int G>
+static int launch_split_any(GemvFusedParams& p, int M, int64_t Kp, int max_stages, bool pdl, cudaStream_t s) {
+  const int n_iter = (p.KT * 8 + kFConsumers * 32 - 1) / (kFConsumers * 32);
+  if (n_iter <= 1) return launch_split<G, 1, 1, 8>(p, M, Kp, max_stages, pdl, s);
+  if (n_iter <= 2) return launch_split<G, 1, 2, 8>(p, M, Kp, max_stages, pdl, s);
+  return AO_B200_ERR_WORKSPACE;
+}
+
+// The GEMV without a norm for activations too long for one CTA: k shared out over the CTAs of a cluster (AO_B200_ERR_WORKSPACE: not for this shape).
+int int4_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np, int64_t Kp, int G, void* y,
+                    int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res, int max_stages, bool pdl, cudaStream_t s) {
+  if (M < 2 || M > 8) return AO_B200_ERR_WORKSPACE;
+  GemvFusedParams p{};
+  p.packed = static_cast<const uint8_t*>(packed);
+  p.sz = static_cast<const uint32_t*>(sz);
+  p.x = static_cast<const __nv_bfloat16*>(x);
+  p.residual = static_cast<const __nv_bfloat16*>(residual);
+  p.y = static_cast<__nv_bfloat16*>(y);
+  p.M = (int)M;
+  p.epilogue = residual != nullptr ? kEpiResidual : 0;
+  p.copy_split = 1;
+  p.Kx = Kx; p.ldx = ldx; p.Np = Np; p.N_out = N_out; p.ldy = ldy; p.ld_res = ld_res;
+  p.n_strips = (int)(Np / 16);
+  for (int ks = 2; ks <= 4; ks *= 2) {
+    if (Kp % (ks * (G < 128 ? 128 : G)) != 0) continue;   // whole groups, and whole pairs of tiles (what a warp takes)
+    p.ks = ks;
+    p.KT = (int)(Kp / 64 / ks);
+    int e = AO_B200_ERR_WORKSPACE;
+    switch (G) {
+      case 32: e = launch_split_any<32>(p, (int)M, Kp, max_stages, pdl, s); break;
+      case 64: e = launch_split_any<64>(p, (int)M, Kp, max_stages, pdl, s); break;
+      case 128: e = launch_split_any<128>(p, (int)M, Kp, max_stages, pdl, s); break;
+      case 256: e = launch_split_any<256>(p, (int)M, Kp, max_stages, pdl, s); break;
+    }
+    if (e != AO_B200_ERR_WORKSPACE) return e;
+  }
+  return AO_B200_ERR_WORKSPACE;
 }
 
 // whether the activations of a call fit this kernel's staging
@@ -698,6 +790,10 @@ int int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   p.n_strips = (int)(Np / 16);
   p.eps = eps;
   const int MT = M <= 8 ? 1 : 2;
+  if (norm_w == nullptr && epilogue != kEpiSiluMul && long_activations(M, Kp) && int4_gemv_fused_fits(M, Kp, G, max_stages)) {
+    const int e = int4_gemv_split(x, M, Kx, ldx, packed, sz, Np, Kp, G, y, N_out, ldy, epilogue == kEpiResidual ? residual : nullptr, ld_res, max_stages, pdl, s);
+    if (e != AO_B200_ERR_WORKSPACE) return e;
+  }
   FusedPlan pl;
   bool ok = false;
   switch (G) {
@@ -715,6 +811,7 @@ int int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   }
   p.x_row_bytes = pl.x_row_bytes;
   p.off_x = pl.off_x; p.off_X = pl.off_X; p.off_red = pl.off_red; p.off_misc = pl.off_misc;
+  p.ks = 1, p.off_inbox = 0;
   // rows in registers: up to 16 chunks of 8 activations per thread, which leaves registers for one CTA per SM only from 8 on; so where
   // two fit the shared memory (short rows) at most 4.  (int8_gemv_fused draws the same lines.)
   const int n_iter = (p.KT * 8 + kFConsumers * 32 - 1) / (kFConsumers * 32);

@@ -46,6 +46,8 @@ struct Gemv8Params {
   float eps;
   uint32_t x_row_bytes;           // 2 * Kp + 16
   uint32_t off_x, off_C, off_red, off_misc;
+  int ks;                         // SPLIT: CTAs of a cluster that share a strip's k; KT is then one CTA's part of it
+  uint32_t off_inbox;
 };
 
 __device__ __forceinline__ float warp_sum8(float v) {
@@ -78,7 +80,10 @@ __device__ __forceinline__ uint32_t mul_bf16x2_8(uint32_t a, uint32_t b) {
   return d;
 }
 
-template <int MT, int NH, int HR>
+// SPLIT: the CTAs of a cluster take a quarter or half of k each, for activations that one CTA cannot hold (and would take long to stage).
+// Each sums its part of a strip; those of the other ranks send theirs into shared memory of rank 0, which has room for all its strips,
+// adds them in rank order and finishes the strip.
+template <int MT, int NH, int HR, bool SPLIT>
 __global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) int8_gemv_fused_kernel(const Gemv8Params p) {
   extern __shared__ __align__(128) uint8_t smem8[];
   uint8_t* ring = smem8;
@@ -95,12 +100,16 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int stages = p.stages;
-  const int b = blockIdx.x;
+  const int ks = SPLIT ? p.ks : 1, rank = SPLIT ? blockIdx.x % ks : 0;
+  const int b = SPLIT ? blockIdx.x / ks : blockIdx.x;
   const int s0 = b * p.strips_base + min(b, p.strips_rem), s1 = s0 + p.strips_base + (b < p.strips_rem ? 1 : 0);
   const int KT = p.KT;
   const int n_chunks = (KT + k8StageTiles - 1) / k8StageTiles;
 
   grid_launch_dependents();
+  uint64_t* in_full = reinterpret_cast<uint64_t*>(smem8 + p.off_inbox);         // SPLIT, rank 0: [strips] the others' parts have arrived
+  float4* inbox = reinterpret_cast<float4*>(smem8 + p.off_inbox + kMaxSplitStrips * 8);   // [strips][ks - 1][MT][32 lanes]
+  if constexpr (SPLIT) split_begin(warp == k8Consumers + 1 && rank == 0, s1 - s0, in_full, (uint32_t)((ks - 1) * MT * 512), lane);
 
   if (warp == k8Consumers) {
     // ===================== producer =====================
@@ -121,7 +130,7 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
       int slot = 0;
       uint32_t par = 1;
       for (int strip = s0; strip < s1; ++strip) {
-        const uint8_t* wrow = p.packed + (int64_t)strip * KT * 1024;
+        const uint8_t* wrow = p.packed + ((int64_t)strip * ks + rank) * KT * 1024;
         for (int ch = 0; ch < n_chunks; ++ch) {
           const int kt0 = ch * k8StageTiles;
           const int cnt = min(k8StageTiles, KT - kt0);
@@ -137,6 +146,7 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     }
     __syncwarp();
     grid_dependency_wait();  // every kernel of a PDL chain must wait before it exits (transitive ordering)
+    if constexpr (SPLIT) split_meet();
     return;
   }
 
@@ -145,6 +155,7 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     const int g = lane >> 2, c = lane & 3;
     grid_dependency_wait();
     named_bar_sync(2, k8Threads);
+    if constexpr (SPLIT) split_meet();
     // The scales of a strip are fetched while the strip before it is finished, its residual before the wait: what this warp does behind the last
     // wait is the launch's tail (4096 x 4096, 8 rows with residual: from the last weight to the end 1.3 -> 0.4 us)
     auto scale_of = [&](int64_t n) { return n < p.N_out ? __bfloat162float(p.scale[n]) : 0.f; };
@@ -181,6 +192,8 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&red_free[rbuf]);
+      if constexpr (SPLIT)
+        if (!split_sums<MT>(sum, row_scale, in_full, inbox, li, rank, ks, lane)) continue;
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         const float vals[2][2] = {{sum[mt].x, sum[mt].z}, {sum[mt].y, sum[mt].w}};  // [col j][row half]
@@ -188,7 +201,7 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
         for (int j = 0; j < 2; ++j) {
           const int m = 8 * mt + 2 * c + j;
           if (m >= p.M) continue;
-          const float rsc = row_scale[m];
+          const float rsc = SPLIT ? 1.f : row_scale[m];
           // mm result rounded to bf16, THEN the scale multiply rounds again (plain_layout.py:256-262)
           const float v0 = bf16r(bf16r(vals[j][0] * rsc) * sc0), v1 = bf16r(bf16r(vals[j][1] * rsc) * sc1);
           if (p.epilogue == k8EpiSiluMul) {
@@ -246,7 +259,7 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     const auto done = [&](int seg, int m, const float (&sum)[1]) { C_s[seg * 8 * MT + m] = -1152.f * sum[0]; };
 #pragma unroll
     for (int row0 = 0; row0 < HR; row0 += 8)
-      stage_rows<(HR < 8 ? HR : 8), NH, kCT, 1, 64>(p.x, p.ldx, p.Kx, row0, p.M, p.norm_w, p.eps, chunks_per_row, x_s, p.x_row_bytes, part, row_scale, chunk,
+      stage_rows<(HR < 8 ? HR : 8), NH, kCT, 1, 64>(p.x + (int64_t)rank * KT * 64, p.ldx, SPLIT ? min(p.Kx - (int64_t)rank * KT * 64, (int64_t)KT * 64) : p.Kx, row0, p.M, p.norm_w, p.eps, chunks_per_row, x_s, p.x_row_bytes, part, row_scale, chunk,
                                                     done);
   } else if constexpr (hold) {
     float ss = 0.f, amax = 0.f;
@@ -481,25 +494,27 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     __syncwarp();
     if (lane == 0) mbar_arrive(&red_full[rbuf]);
   }
+  if constexpr (SPLIT) split_meet();
 }
 
 // ------------------------------------------------------------------------------------------------ host side
 struct Plan8 {
   int stages;
   size_t smem;
-  uint32_t off_x, off_C, off_red, off_misc, x_row_bytes;
+  uint32_t off_x, off_C, off_red, off_misc, off_inbox, x_row_bytes;
 };
 
-static bool plan8(int M, int MT, int64_t Kp, int max_stages, Plan8& pl) {
+// inbox: bytes behind everything else, for one CTA per SM
+static bool plan8(int M, int MT, int64_t Kp, int max_stages, Plan8& pl, size_t inbox = 0) {
   pl.x_row_bytes = (uint32_t)(2 * Kp + 16);
   const size_t x_bytes = ((size_t)M * pl.x_row_bytes + 127) / 128 * 128;
   const size_t C_bytes = ((size_t)(Kp / 64) * 8 * MT * 4 + 127) / 128 * 128;
   const size_t red_bytes = (size_t)k8RedBufs * k8Consumers * MT * 128 * 4;
   const size_t misc = (16 * k8Consumers * 2 + 32) * 4 + (2 * 16 + 2 * k8RedBufs) * 8 + 64;
-  const size_t fixed = x_bytes + C_bytes + red_bytes + misc;
+  const size_t fixed = x_bytes + C_bytes + red_bytes + misc + inbox;
   const size_t two_per_sm = 113 * 1024, one_per_sm = 226 * 1024;
   int st = 0;
-  if (MT == 1 && fixed + 4 * (size_t)k8StageBytes <= two_per_sm) {
+  if (MT == 1 && inbox == 0 && fixed + 4 * (size_t)k8StageBytes <= two_per_sm) {
     st = (int)((two_per_sm - fixed) / k8StageBytes);
   } else if (fixed + 3 * (size_t)k8StageBytes <= one_per_sm) {
     st = (int)((one_per_sm - fixed) / k8StageBytes);
@@ -514,6 +529,7 @@ static bool plan8(int M, int MT, int64_t Kp, int max_stages, Plan8& pl) {
   pl.off_C = (uint32_t)off; off += C_bytes;
   pl.off_red = (uint32_t)off; off += red_bytes;
   pl.off_misc = (uint32_t)off; off += misc;
+  pl.off_inbox = (uint32_t)((off + 15) / 16 * 16); off += inbox;
   pl.smem = off;
   return true;
 }
@@ -533,7 +549,7 @@ template <int MT, int NH, int HR>
 static int launch8(Gemv8Params& p, const Plan8& pl, bool pdl, cudaStream_t s) {
   static bool attr_done = false;
   if (!attr_done) {
-    if (cudaFuncSetAttribute(int8_gemv_fused_kernel<MT, NH, HR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
+    if (cudaFuncSetAttribute(int8_gemv_fused_kernel<MT, NH, HR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
       return AO_B200_ERR_CUDA;
     attr_done = true;
   }
@@ -558,7 +574,47 @@ static int launch8(Gemv8Params& p, const Plan8& pl, bool pdl, cudaStream_t s) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
-  if (cudaLaunchKernelEx(&cfg, int8_gemv_fused_kernel<MT, NH, HR>, p) != cudaSuccess) return AO_B200_ERR_CUDA;
+  if (cudaLaunchKernelEx(&cfg, int8_gemv_fused_kernel<MT, NH, HR, false>, p) != cudaSuccess) return AO_B200_ERR_CUDA;
+  return ao_launch_status();
+}
+
+template <int MT, int NH, int HR>
+static int launch8_split(Gemv8Params& p, int M, int64_t Kp, int max_stages, bool pdl, cudaStream_t s) {
+  auto kern = int8_gemv_fused_kernel<MT, NH, HR, true>;
+  static bool attr_done = false;
+  if (!attr_done) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return AO_B200_ERR_CUDA;
+    attr_done = true;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(k8Threads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.ks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 2 : 1;
+  static int at_once[5] = {};
+  int clusters = split_clusters(reinterpret_cast<const void*>(kern), cfg, p.ks, sm_count8(), at_once);
+  if (clusters <= 0) return AO_B200_ERR_WORKSPACE;
+  if (clusters > p.n_strips) clusters = p.n_strips;
+  const int most = (p.n_strips + clusters - 1) / clusters;
+  if (most > kMaxSplitStrips) return AO_B200_ERR_WORKSPACE;
+  Plan8 pl;
+  if (!plan8(M, MT, Kp / p.ks, max_stages, pl, kMaxSplitStrips * 8 + 16 + (size_t)most * (p.ks - 1) * MT * 512)) return AO_B200_ERR_WORKSPACE;
+  if (pl.smem <= 113 * 1024) pl.smem = 114 * 1024;   // (one CTA per SM)
+  p.stages = pl.stages;
+  p.x_row_bytes = pl.x_row_bytes;
+  p.off_x = pl.off_x; p.off_C = pl.off_C; p.off_red = pl.off_red; p.off_misc = pl.off_misc; p.off_inbox = pl.off_inbox;
+  p.strips_base = p.n_strips / clusters;
+  p.strips_rem = p.n_strips % clusters;
+  cfg.gridDim = dim3((unsigned)(clusters * p.ks));
+  cfg.dynamicSmemBytes = pl.smem;
+  if (cudaLaunchKernelEx(&cfg, kern, p) != cudaSuccess) return AO_B200_ERR_CUDA;
   return ao_launch_status();
 }
 
@@ -567,6 +623,9 @@ bool int8_gemv_fused_fits(int64_t M, int64_t Kp, int max_stages) {
   Plan8 pl;
   return plan8((int)M, M <= 8 ? 1 : 2, Kp, max_stages, pl);
 }
+
+int int8_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Kp, void* y, int64_t N_out,
+                    int64_t ldy, const void* residual, int64_t ld_res, int max_stages, bool pdl, cudaStream_t s);
 
 // returns AO_B200_ERR_WORKSPACE when the activations do not fit the staging (caller falls back)
 int int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Np,
@@ -592,8 +651,13 @@ int int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   p.stages = pl.stages;
   p.x_row_bytes = pl.x_row_bytes;
   p.off_x = pl.off_x; p.off_C = pl.off_C; p.off_red = pl.off_red; p.off_misc = pl.off_misc;
+  p.ks = 1, p.off_inbox = 0;
   // Rows in registers: chunks of 8 activations per consumer thread and row.  M = 1: <= 4 (Kp <= 16384).  More rows: up to 16 chunks in all,
   // which leaves registers for one CTA per SM only from 8 on, so where two fit the shared memory (short rows) at most 4.
+  if (norm_w == nullptr && epilogue != k8EpiSiluMul && long_activations(M, Kp)) {
+    const int e = int8_gemv_split(x, M, Kx, ldx, packed, scale, Kp, y, N_out, ldy, epilogue == k8EpiResidual ? residual : nullptr, ld_res, max_stages, pdl, s);
+    if (e != AO_B200_ERR_WORKSPACE) return e;
+  }
   const int n_iter = (p.KT * 8 + k8Consumers * 32 - 1) / (k8Consumers * 32);
   if (MT == 2) return n_iter <= 1 ? launch8<2, 1, 16>(p, pl, pdl, s) : launch8<2, 0, 0>(p, pl, pdl, s);
   if (M == 1 && n_iter <= 1) return launch8<1, 1, 1>(p, pl, pdl, s);
@@ -606,6 +670,33 @@ int int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   if (n_iter <= 1 && alone) return launch8<1, 1, 8>(p, pl, pdl, s);
   if (n_iter <= 2 && alone) return launch8<1, 2, 8>(p, pl, pdl, s);
   return launch8<1, 0, 0>(p, pl, pdl, s);
+}
+
+// The same without a norm for activations too long for one CTA: k shared out over the CTAs of a cluster (AO_B200_ERR_WORKSPACE: not for this shape).
+int int8_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Kp, void* y, int64_t N_out,
+                    int64_t ldy, const void* residual, int64_t ld_res, int max_stages, bool pdl, cudaStream_t s) {
+  if (M < 2 || M > 8) return AO_B200_ERR_WORKSPACE;
+  const int64_t kt = Kp / 64;
+  Gemv8Params p{};
+  p.packed = static_cast<const uint8_t*>(packed);
+  p.scale = static_cast<const __nv_bfloat16*>(scale);
+  p.x = static_cast<const __nv_bfloat16*>(x);
+  p.residual = static_cast<const __nv_bfloat16*>(residual);
+  p.y = static_cast<__nv_bfloat16*>(y);
+  p.M = (int)M;
+  p.epilogue = residual != nullptr ? k8EpiResidual : k8EpiPlain;
+  p.Kx = Kx; p.ldx = ldx; p.N_out = N_out; p.ldy = ldy; p.ld_res = ld_res;
+  p.n_strips = (int)((N_out + 15) / 16);
+  for (int ks = 2; ks <= 4; ks *= 2) {   // (halves where they fit: quarters leave SMs idle that make no whole cluster, and have twice the strips)
+    if (kt % ks != 0) continue;
+    p.ks = ks;
+    p.KT = (int)(kt / ks);
+    const int n_iter = (p.KT * 8 + k8Consumers * 32 - 1) / (k8Consumers * 32);
+    const int e = n_iter <= 1 ? launch8_split<1, 1, 8>(p, (int)M, Kp, max_stages, pdl, s)
+                              : (n_iter <= 2 ? launch8_split<1, 2, 8>(p, (int)M, Kp, max_stages, pdl, s) : AO_B200_ERR_WORKSPACE);
+    if (e != AO_B200_ERR_WORKSPACE) return e;
+  }
+  return AO_B200_ERR_WORKSPACE;
 }
 
 }  // namespace ao

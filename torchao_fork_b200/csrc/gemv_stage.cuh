@@ -144,4 +144,78 @@ __device__ __forceinline__ void stage_rows(const __nv_bfloat16* x, int64_t ldx, 
   }
 }
 
+// ---- k shared out over the CTAs of a cluster (SPLIT kernels) ----------------------------------------------------------------
+// For activations that one CTA cannot hold, or takes long to stage.  Each CTA sums its part of a strip; those of the other ranks send theirs
+// into shared memory of rank 0 (st.async), which has room for all its strips, adds them in rank order and finishes the strip: nobody waits to send.
+constexpr int kMaxSplitStrips = 32;   // strips of a cluster
+
+// Without a norm, up to 8 rows: from here on halves beat whole rows (int8, 8 rows: 3072 x 8192 8.7 us against 12.1, 8192 x 8192 16.0 against 19.1;
+// 4 rows of 4096 x 14336 14.7 against 15.4; int4 8.3 against 10.3, 13.4 against 15.5, 13.4 against 15.9; below: int8, 8 rows of 5120 x 5120 10.0
+// against 9.9, 4 rows of 8192 x 8192 15.2 against 14.4).  More rows are not split: twice the products per weight in CTAs with half the k
+// (16 rows of 8192 x 8192: 26 us against the GEMM's 23).
+static inline bool long_activations(int64_t M, int64_t Kp) { return M <= 8 && M * Kp >= 57344; }
+
+// at the start, by every thread: rank 0's epilogue warp makes the barriers of its `strips` strips; `bytes` arrive at each
+__device__ __forceinline__ void split_begin(bool owner, int strips, uint64_t* in_full, uint32_t bytes, int lane) {
+  if (owner) {
+    if (lane < strips) {
+      mbar_init(&in_full[lane], 1);
+      fence_barrier_init();
+      mbar_arrive_expect_tx(&in_full[lane], bytes);
+    }
+    __syncwarp();
+  }
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+}
+// before the first send, and before a thread leaves
+__device__ __forceinline__ void split_meet() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+// The epilogue warp's sums of strip li, scaled (each rank has scaled its part of a row by itself): false, and sent on, on the other ranks; all
+// parts added on rank 0.  The wait is bounded: NaN after about two seconds.
+template <int MT>
+__device__ __forceinline__ bool split_sums(float4 (&sum)[MT], const float* row_scale, uint64_t* in_full, float4* inbox, int li, int rank, int ks, int lane) {
+  const int c = lane & 3;
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) {
+    const float r0 = row_scale[8 * mt + 2 * c], r1 = row_scale[8 * mt + 2 * c + 1];
+    sum[mt] = make_float4(sum[mt].x * r0, sum[mt].y * r1, sum[mt].z * r0, sum[mt].w * r1);
+  }
+  if (rank != 0) {
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      uint32_t to, bar;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(to) : "r"(smem_u32(inbox + ((li * (ks - 1) + rank - 1) * MT + mt) * 32 + lane)));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(bar) : "r"(smem_u32(&in_full[li])));
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to), "f"(sum[mt].x), "f"(sum[mt].y),
+                   "f"(sum[mt].z), "f"(sum[mt].w), "r"(bar)
+                   : "memory");
+    }
+    return false;
+  }
+  const long long t0 = clock64();
+  bool here = true;
+  while (here && !mbar_try_wait(&in_full[li], 0)) here = clock64() - t0 < 4000000000ll;
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) {
+    for (int r = 0; r + 1 < ks; ++r) {
+      const float4 v = inbox[((li * (ks - 1) + r) * MT + mt) * 32 + lane];
+      sum[mt] = make_float4(sum[mt].x + v.x, sum[mt].y + v.y, sum[mt].z + v.z, sum[mt].w + v.w);
+    }
+    if (!here) sum[mt] = make_float4(__int_as_float(0x7FFFFFFF), __int_as_float(0x7FFFFFFF), __int_as_float(0x7FFFFFFF), __int_as_float(0x7FFFFFFF));
+  }
+  return true;
+}
+// Clusters of ks CTAs, one per SM, that run at the same time: the SMs of a GPC need not be a multiple of ks.  The same for every shape, so asked
+// for once per kernel and ks.
+static inline int split_clusters(const void* kern, cudaLaunchConfig_t cfg, int ks, int sms, int (&at_once)[5]) {
+  if (at_once[ks] == 0) {
+    cfg.gridDim = dim3((unsigned)(sms / ks * ks));
+    cfg.dynamicSmemBytes = 200 * 1024;
+    cfg.numAttrs = 1;   // the cluster dimension
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) cudaGetLastError(), n = 0;
+    at_once[ks] = n > 0 ? n : -1;
+  }
+  return at_once[ks];
+}
+
 }  // namespace ao
