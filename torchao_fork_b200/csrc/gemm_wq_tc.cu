@@ -677,8 +677,33 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
           for (int i = 0; i < 4; ++i) __stcg(mine + i * 128, make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]));
         }
       } else {
+        if (!whole && ue == u1) {
+          // the others' shares of this CTA's last tile, written long ago as a rule, on their way back to L2
+          const int c0 = wq_owner(t * KU, p.base, p.rem, p.quantum), c1 = wq_owner(t * KU + KU - 1, p.base, p.rem, p.quantum);
+          for (int cc = c0; cc <= c1; ++cc)
+            if (cc != worker)
+              for (int i = threadIdx.x; i < NT * 4; i += kWqEpiWarps * 32)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(share(cc, t)) + (int64_t)i * 128));
+        }
         ok = ok && wait(&dfull[d.slot], d.use);
         wq_fence_after();
+        if (!whole && ue == u1) {
+          // This CTA's last tile, and it is shared.  As a rule the others' shares (their first tiles, done long ago) are there: then this one
+          // stays in tensor memory, and all warps finish the tile below.
+          if (wq_epi_sync(!ok)) break;
+          bool here = false;
+          if (threadIdx.x == 0) {
+            const int others = wq_owner(t * KU + KU - 1, p.base, p.rem, p.quantum) - wq_owner(t * KU, p.base, p.rem, p.quantum);
+            uint32_t arrived;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(arrived) : "l"(p.tickets + t * kRanks + rank) : "memory");
+            here = arrived == (uint32_t)others;
+            if (here) s_last[t == u0 / KU ? 0 : 1] = 2;
+          }
+          if (wq_epi_sync(here)) {
+            wq_fence_before();
+            break;
+          }
+        }
         // which accumulators hold something: both MMA warps', unless the tile has one unit here
         const bool two = n_mma == 2 && ue - u > 1;
         const uint32_t dcol = lane_col + d.slot * 128 + (n_mma == 2 && ue - u == 1 ? ((u - u0) & 1) * 64 : 0);
@@ -730,25 +755,76 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
 
   // ---- shared tiles that this CTA was the last to reach: all warps add the shares in CTA order and finish the rows ----
   __syncthreads();
+  wq_fence_after();
 #pragma unroll 1
   for (int k = 0; k < 2; ++k) {
-    if (s_last[k] == 0) continue;
+    const int last = s_last[k];
+    if (last == 0) continue;
     __threadfence();
     const int t = k == 0 ? u0 / KU : (u1 - 1) / KU, nb = t / p.MT, mt = t - nb * p.MT;
     const int c0 = wq_owner(t * KU, p.base, p.rem, p.quantum), c1 = wq_owner(t * KU + KU - 1, p.base, p.rem, p.quantum);
-    for (int it = warp; it < NT / 2; it += kWqThreads / 32) {  // (column block, quadrant, half)
-      const int h = it & 1, q = (it >> 1) & 3, c = (it >> 3) * 16;
-      float f[8], sc[4];
+    // last == 2: this CTA's share is its accumulators (which of them hold something: as in the epilogue)
+    const int us = max(u0, t * KU), held = u1 - us;
+    const bool two = n_mma == 2 && held > 1;
+    const int q = warp & 3;                            // tensor memory: a warp reaches the lanes of its quadrant
+    const uint32_t dcol = tb + ((uint32_t)(32 * q) << 16) + (d_bufs == 2 ? ((t - u0 / KU) & 1) * 128 : 0) + (n_mma == 2 && held == 1 ? ((us - u0) & 1) * 64 : 0);
+    float sc[4];
+    row_scales(nb, q, sc);
+    constexpr int kStep = kWqThreads / 128, kBatch = 3;  // (column block, half) pairs per round of the quadrant's warps; rounds with their loads in flight
+    const auto add8 = [](float (&f)[8], const float4& a, const float4& b) {
+      f[0] += a.x, f[1] += a.y, f[2] += a.z, f[3] += a.w, f[4] += b.x, f[5] += b.y, f[6] += b.z, f[7] += b.w;
+    };
+    const auto at = [&](int cc, int it) { return share(cc, t) + ((it >> 1) * 4 + 2 * (it & 1)) * 128 + q * 32 + lane; };
+    if (!DEFER && last == 2 && c1 - c0 == 1) {
+      // own accumulators and one other share (a sum of two, in either order)
+      const int other = c0 == worker ? c1 : c0;
+#pragma unroll 1
+      for (int it0 = warp >> 2; it0 < NT / 8; it0 += kStep * kBatch) {
+        float4 w[kBatch][2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] = 0.f;
-      row_scales(nb, q, sc);
-#pragma unroll 4
-      for (int cc = c0; cc <= c1; ++cc) {
-        const float4* src = share(cc, t) + (c / 4 + 2 * h) * 128 + q * 32 + lane;
-        const float4 v0 = __ldcg(src), v1 = __ldcg(src + 128);
-        f[0] += v0.x, f[1] += v0.y, f[2] += v0.z, f[3] += v0.w, f[4] += v1.x, f[5] += v1.y, f[6] += v1.z, f[7] += v1.w;
+        for (int j = 0; j < kBatch; ++j) {
+          const int it = min(it0 + j * kStep, NT / 8 - 1);
+          w[j][0] = __ldcg(at(other, it)), w[j][1] = __ldcg(at(other, it) + 128);
+        }
+#pragma unroll
+        for (int j = 0; j < kBatch; ++j) {
+          const int it = it0 + j * kStep, h = it & 1, c = (it >> 1) * 16;
+          if (it >= NT / 8) break;
+          uint32_t v[8], v2[8];
+          float f[8];
+          wq_ld_16x256b_x2(dcol + ((uint32_t)(16 * h) << 16) + c, v);
+          if (two) wq_ld_16x256b_x2(dcol + ((uint32_t)(16 * h) << 16) + 64 + c, v2);
+          wq_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) f[i] = two ? __uint_as_float(v[i]) + __uint_as_float(v2[i]) : __uint_as_float(v[i]);
+          add8(f, w[j][0], w[j][1]);
+          to_stage(q, c, h, f, sc);
+        }
       }
-      to_stage(q, c, h, f, sc);
+    } else {
+#pragma unroll 1
+      for (int it = warp >> 2; it < NT / 8; it += kStep) {
+        const int h = it & 1, c = (it >> 1) * 16;
+        float f[8];
+        uint32_t v[8], v2[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = 0.f, v[i] = v2[i] = 0u;
+        if (!DEFER && last == 2) {
+          wq_ld_16x256b_x2(dcol + ((uint32_t)(16 * h) << 16) + c, v);
+          if (two) wq_ld_16x256b_x2(dcol + ((uint32_t)(16 * h) << 16) + 64 + c, v2);
+          wq_ld_wait();
+        }
+#pragma unroll 4
+        for (int cc = c0; cc <= c1; ++cc) {
+          if (!DEFER && last == 2 && cc == worker) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] += two ? __uint_as_float(v[i]) + __uint_as_float(v2[i]) : __uint_as_float(v[i]);
+          } else {
+            add8(f, __ldcg(at(cc, it)), __ldcg(at(cc, it) + 128));
+          }
+        }
+        to_stage(q, c, h, f, sc);
+      }
     }
     __syncthreads();
     copy_out(nb, mt, threadIdx.x, kWqThreads);
