@@ -308,6 +308,12 @@ AO_B200_API int ao_b200_silu_mul_rows(const void* gate, const void* up, void* y,
  * logits bf16 [B][ldl], next_tok int64 [B]. */
 AO_B200_API int ao_b200_sample(const void* logits, int64_t ldl, int64_t B, int64_t V, float temperature, int top_k,
                                const void* noise, int64_t ldq, void* next_tok, void* stream);
+/* The same at the end of a decode step: the tokens also go to fed_tok int64 [B] (null: nowhere else), which the next step reads, and
+ * *pos (null: none) moves on by one.  ao_b200_embed_rows is that step's beginning: out bf16 [B][D] = rows tok[b] of table [V][D] (D % 8 == 0,
+ * 16-byte aligned; the tokens have to be in [0, V), as for a gather). */
+AO_B200_API int ao_b200_sample_advance(const void* logits, int64_t ldl, int64_t B, int64_t V, float temperature, int top_k,
+                                       const void* noise, int64_t ldq, void* next_tok, void* fed_tok, int32_t* pos, void* stream);
+AO_B200_API int ao_b200_embed_rows(const int64_t* tok, const void* table, int64_t V, int64_t D, int64_t B, void* out, void* stream);
 
 /* ---- tensor-parallel exchange over NVLink peer memory (new: the reference has no int4 TP path
  * names the collective it replaces: ncclAllReduce(sum, bf16) of [B][dim] after the row-parallel wo and w2) ------------

@@ -93,3 +93,23 @@ def test_argument_errors():
     out = torch.zeros(1, dtype=torch.int64, device=DEV)
     rc = _lib.lib().ao_b200_sample(logits.data_ptr(), 16, 1, 16, 0.8, 4, None, 0, out.data_ptr(), None)
     assert rc != 0  # sampling with temperature needs the noise
+
+
+@pytest.mark.parametrize("B,V,D,temperature,top_k", [(1, 199, 8, 0.0, None), (3, 4099, 1032, 0.8, 50), (16, 1000, 4096, 1.0, None)])
+def test_end_and_beginning_of_a_decode_step(B, V, D, temperature, top_k):
+    """sample_advance = ao_b200_sample, its tokens into the fed buffer and the position moved on by one; embed_rows = the rows of those tokens."""
+    torch.manual_seed(V)
+    logits = torch.randn(B, V, device=DEV, dtype=torch.bfloat16)
+    noise = torch.empty(B, V, device=DEV).exponential_(1) if temperature else None
+    want = run_kernel(logits, temperature, top_k, noise)
+    out, fed = (torch.full((B,), -1, dtype=torch.int64, device=DEV) for _ in range(2))
+    pos = torch.tensor([41, 7], dtype=torch.int32, device=DEV)
+    table = torch.randn(V, D, device=DEV, dtype=torch.bfloat16)
+    h = torch.zeros(B + 1, D, device=DEV, dtype=torch.bfloat16)
+    L, st = _lib.lib(), torch.cuda.current_stream().cuda_stream
+    _lib.check(L.ao_b200_sample_advance(logits.data_ptr(), V, B, V, temperature, top_k or 0, None if noise is None else noise.data_ptr(), V, out.data_ptr(),
+                                        fed.data_ptr(), pos.data_ptr(), st), "sample_advance")
+    _lib.check(L.ao_b200_embed_rows(fed.data_ptr(), table.data_ptr(), V, D, B, h.data_ptr(), st), "embed_rows")
+    assert torch.equal(out, want) and torch.equal(fed, want) and pos.tolist() == [42, 7]
+    assert torch.equal(h[:B], table[want]) and not h[B].any()
+    assert L.ao_b200_embed_rows(fed.data_ptr(), table.data_ptr(), V, D + 4, B, h.data_ptr(), st) != 0  # rows of a whole number of 16 bytes

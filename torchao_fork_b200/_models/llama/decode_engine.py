@@ -410,7 +410,7 @@ class DecodeEngine:
         st = torch.cuda.current_stream(self.device).cuda_stream
         B = self.B
         n = 0
-        torch.index_select(self.emb, 0, self.tok, out=self.h)
+        self._embed(st)
         for l in self.layers:
             l["wqkv"].launch_fused(self.h, self.qkv, st, norm_w=l["attn_norm"], eps=self.eps, ws=self.ws)
             if self.kv_int8:
@@ -442,9 +442,7 @@ class DecodeEngine:
         logits = self.logits
         if self.tp is not None:
             logits = self.tp.gather_logits(self.logits)
-        self._sample(logits)
-        self.tok.copy_(self.next_tok)
-        self.pos.add_(1)
+        self._sample(logits, advance=True)
 
     def _launch_step(self):
         if self.mega:
@@ -459,7 +457,7 @@ class DecodeEngine:
         st = torch.cuda.current_stream(self.device).cuda_stream
         B, D = self.B, self.cfg.dim
         self.launches_per_step = 0
-        torch.index_select(self.emb, 0, self.tok, out=self.h)
+        self._embed(st)
         residual = None
         for l in self.layers:
             _lib.check(L.ao_b200_rmsnorm(self.h.data_ptr(), _ptr(residual), l["attn_norm"].data_ptr(),
@@ -496,9 +494,7 @@ class DecodeEngine:
         logits = self.logits
         if self.tp is not None:
             logits = self.tp.gather_logits(self.logits)
-        self._sample(logits)
-        self.tok.copy_(self.next_tok)
-        self.pos.add_(1)
+        self._sample(logits, advance=True)
 
     def _launch_step_parts(self):
         """Batches whose activations do not fit the staging of every fused GEMV: a projection that fits keeps its RMSNorm prologue and
@@ -507,7 +503,7 @@ class DecodeEngine:
         st = torch.cuda.current_stream(self.device).cuda_stream
         B, D = self.B, self.cfg.dim
         n = 1
-        torch.index_select(self.emb, 0, self.tok, out=self.h)
+        self._embed(st)
 
         def normed(lin, weight, y):
             if lin.fused_fits(B):
@@ -550,11 +546,18 @@ class DecodeEngine:
             n += residual(l["w2"], self.s)
         n += normed(self.output, self.out_norm, self.logits)
         self.launches_per_step = n
-        self._sample(self.logits)
-        self.tok.copy_(self.next_tok)
-        self.pos.add_(1)
+        self._sample(self.logits, advance=True)
 
-    def _sample(self, logits):
+    def _embed(self, stream):
+        """the rows of the fed tokens -> h"""
+        D = self.emb.shape[1]
+        if D % 8 == 0 and self.emb.is_contiguous() and self.emb.data_ptr() % 16 == 0:
+            _lib.check(_lib.lib().ao_b200_embed_rows(self.tok.data_ptr(), self.emb.data_ptr(), self.emb.shape[0], D, self.B, self.h.data_ptr(), stream),
+                       "embed_rows")
+        else:
+            torch.index_select(self.emb, 0, self.tok, out=self.h)
+
+    def _sample(self, logits, advance=False):
         """reference: generate.py:79-100 (temperature, top-k, exponential-noise argmax).  The Exp(1) noise is drawn by
         torch's generator exactly as the reference draws it; everything else is one ao_b200_sample launch."""
         noise = None
@@ -562,10 +565,12 @@ class DecodeEngine:
             if self._noise is None or self._noise.shape != logits.shape:
                 self._noise = torch.empty(logits.shape, dtype=torch.float32, device=logits.device)
             noise = self._noise.exponential_(1)
-        _lib.check(_lib.lib().ao_b200_sample(
+        # advance: the token is fed to the next step and the position moves on, in the same launch
+        _lib.check(_lib.lib().ao_b200_sample_advance(
             logits.data_ptr(), logits.stride(0), logits.shape[0], logits.shape[1], float(self.temperature),
             0 if self.top_k is None else int(self.top_k), _ptr(noise), 0 if noise is None else noise.stride(0),
-            self.next_tok.data_ptr(), torch.cuda.current_stream(self.device).cuda_stream), "sample")
+            self.next_tok.data_ptr(), self.tok.data_ptr() if advance else None, self.pos.data_ptr() if advance else None,
+            torch.cuda.current_stream(self.device).cuda_stream), "sample")
 
     def _sample_torch(self, logits):
         """The reference's own op sequence (tests compare the kernel with it on the same noise)."""

@@ -1,6 +1,7 @@
 // Non-GEMM remainder of one Llama decode step: fused residual-add + RMSNorm,
 // RoPE + KV-cache append, GQA decode attention, SiLU*mul.  All read the token position from DEVICE
 // memory so a captured CUDA graph can be replayed for every token.
+#include <cassert>
 #include <mutex>
 
 #include "common.cuh"
@@ -547,6 +548,30 @@ extern "C" int ao_b200_decode_attention_fused(const void* qkv, const void* freqs
   }
 #undef AO_ATTN
   if (e != cudaSuccess) return AO_B200_ERR_CUDA;
+  return ao_launch_status();
+}
+
+// The rows of a decode step's tokens.  A few KB behind a launch: what it costs is its place in the chain (the library's gather took 8 us of a token,
+// and nothing behind it could start early), so a thread moves 16 bytes and the projection behind it is let go at once.
+namespace ao {
+__global__ void __launch_bounds__(128) embed_rows_kernel(const int64_t* __restrict__ tok, const uint4* __restrict__ table, int64_t V, int64_t d8,
+                                                         uint4* __restrict__ out) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  if (i >= d8) return;
+  const int64_t t = tok[blockIdx.y];
+  assert(t >= 0 && t < V);  // a token that the table does not have ends the program, as the library's gather does
+  if (t >= 0 && t < V) out[blockIdx.y * d8 + i] = __ldg(table + t * d8 + i);
+}
+}  // namespace ao
+
+extern "C" int ao_b200_embed_rows(const int64_t* tok, const void* table, int64_t V, int64_t D, int64_t B, void* out, void* stream) {
+  AO_CHECK_ARG(tok && table && out && V > 0 && D > 0 && D % 8 == 0 && B > 0 && B <= 65535 && ao_aligned(table, 16) && ao_aligned(out, 16));
+  const int64_t blocks = (D / 8 + 127) / 128;
+  AO_CHECK_ARG(blocks <= 2147483647);
+  ao::embed_rows_kernel<<<dim3((unsigned)blocks, (unsigned)B), 128, 0, static_cast<cudaStream_t>(stream)>>>(tok, static_cast<const uint4*>(table), V, D / 8,
+                                                                                                      static_cast<uint4*>(out));
   return ao_launch_status();
 }
 

@@ -84,7 +84,7 @@ constexpr int kSampCluster = 8;
 __global__ void __launch_bounds__(kSampThreads) sample_kernel(const __nv_bfloat16* __restrict__ logits, int64_t ldl,
                                                               int V, int slice, float inv_temp_div, int top_k,
                                                               const float* __restrict__ noise, int64_t ldq,
-                                                              int64_t* __restrict__ next_tok) {
+                                                              int64_t* __restrict__ next_tok, int64_t* __restrict__ fed, int32_t* __restrict__ pos) {
   extern __shared__ __align__(16) unsigned short keys[];  // [slice]
   __shared__ uint32_t hist1[256], hist2[256], merged[256];
   __shared__ uint32_t sel_bin, sel_k;
@@ -94,6 +94,12 @@ __global__ void __launch_bounds__(kSampThreads) sample_kernel(const __nv_bfloat1
   __shared__ float red_f[32];
   __shared__ unsigned long long red_u[32];
   cg::cluster_group cluster = cg::this_cluster();
+  // the row's token, into the buffer that the next step reads too; with the first row's the position moves on (every reader of it is behind us)
+  auto take = [&](int64_t token) {
+    next_tok[blockIdx.y] = token;
+    if (fed != nullptr) fed[blockIdx.y] = token;
+    if (pos != nullptr && blockIdx.y == 0) *pos += 1;
+  };
   const int rank = (int)cluster.block_rank();
   const int row = blockIdx.y;
   const int tid = threadIdx.x;
@@ -135,7 +141,7 @@ __global__ void __launch_bounds__(kSampThreads) sample_kernel(const __nv_bfloat1
     if (rank == 0 && tid == 0) {
       unsigned long long b = part_best;
       for (int r = 1; r < kSampCluster; ++r) b = min(b, *cluster.map_shared_rank(&part_best, r));
-      next_tok[row] = (int64_t)b;
+      take((int64_t)b);
     }
     cluster.sync();
     return;
@@ -208,7 +214,7 @@ __global__ void __launch_bounds__(kSampThreads) sample_kernel(const __nv_bfloat1
   if (rank == 0 && tid == 0) {
     unsigned long long b = part_best;
     for (int r = 1; r < kSampCluster; ++r) b = max(b, *cluster.map_shared_rank(&part_best, r));
-    next_tok[row] = 0x7fffffff - (int)(b & 0xffffffffull);
+    take(0x7fffffff - (int)(b & 0xffffffffull));
   }
   cluster.sync();  // nobody leaves while its shared memory may still be read
 }
@@ -218,6 +224,11 @@ __global__ void __launch_bounds__(kSampThreads) sample_kernel(const __nv_bfloat1
 
 extern "C" int ao_b200_sample(const void* logits, int64_t ldl, int64_t B, int64_t V, float temperature, int top_k,
                               const void* noise, int64_t ldq, void* next_tok, void* stream) {
+  return ao_b200_sample_advance(logits, ldl, B, V, temperature, top_k, noise, ldq, next_tok, nullptr, nullptr, stream);
+}
+
+extern "C" int ao_b200_sample_advance(const void* logits, int64_t ldl, int64_t B, int64_t V, float temperature, int top_k, const void* noise, int64_t ldq,
+                                      void* next_tok, void* fed_tok, int32_t* pos, void* stream) {
   AO_CHECK_ARG(logits != nullptr && next_tok != nullptr && B >= 1 && B <= 65535 && V >= 1 && ldl >= V);
   AO_CHECK_ARG(temperature == 0.f || (noise != nullptr && ldq >= V));
   const int slice = (int)((V + ao::kSampCluster - 1) / ao::kSampCluster);
@@ -243,7 +254,8 @@ extern "C" int ao_b200_sample(const void* logits, int64_t ldl, int64_t B, int64_
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (cudaLaunchKernelEx(&cfg, ao::sample_kernel, static_cast<const __nv_bfloat16*>(logits), ldl, (int)V, slice, div, top_k,
-                         static_cast<const float*>(noise), ldq, static_cast<int64_t*>(next_tok)) != cudaSuccess)
+                         static_cast<const float*>(noise), ldq, static_cast<int64_t*>(next_tok),
+                         static_cast<int64_t*>(fed_tok), pos) != cudaSuccess)
     return AO_B200_ERR_CUDA;
   return ao_launch_status();
 }
