@@ -39,8 +39,10 @@ __device__ __forceinline__ uint32_t tinygemm_quant1(float w, float min_val, floa
 //     significant bits, so the true quotient is either exactly representable in fp32 (then the residual is exact and
 //     the step returns it exactly) or at least 2^-18 (relative) away from any bf16 rounding boundary, while the step's
 //     error is < 2^-22: bf16(quotient) is the reference's value in every case;
-//   * rint is an add of 1.5 * 2^23 (round-to-nearest-even in the FMA pipe), the nibbles are assembled with FMAs
-//     (q * 16^slot, exact below 2^16) and converted to integer once per four weights.
+//     Both weights of a register take it together (mul / fma .f32x2: the single operations' roundings);
+//   * rint of a bf16 in [0, 15] is an add of 128 in bf16 (ulp 1 there, ties to even as 128 is even), which leaves 0x4300 + q in each half: shifted and
+//     added up, four registers are a packed word plus a constant.
+// 13 instructions per two weights.
 struct QFast {
   float s, rs;        // scale and its reciprocal
   uint32_t minv2;     // (min_val, min_val) as bf16x2
@@ -60,32 +62,31 @@ __device__ __forceinline__ uint32_t bf2_sub(uint32_t a, uint32_t b) {
   asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
-__device__ __forceinline__ float fast_quot(float a, const QFast& p) {
-  const float x0 = a * p.rs;
-  const float r = fmaf(-p.s, x0, a);
-  return fmaf(r, p.rs, x0);
+// bf16(a / scale) of both halves of a2
+__device__ __forceinline__ uint32_t fast_quot2(uint32_t a2, const QFast& p) {
+  uint32_t t2;
+  asm("{\n\t.reg .b32 lo, hi;\n\t.reg .f32 q0, q1;\n\t.reg .b64 a, s, ns, x, r;\n\t"
+      "shl.b32 lo, %1, 16;\n\tand.b32 hi, %1, 0xffff0000;\n\tmov.b64 a, {lo, hi};\n\tmov.b64 s, {%2, %2};\n\tmov.b64 ns, {%3, %3};\n\t"
+      "mul.rn.f32x2 x, a, s;\n\tfma.rn.f32x2 r, ns, x, a;\n\tfma.rn.f32x2 x, r, s, x;\n\t"
+      "mov.b64 {q0, q1}, x;\n\tcvt.rn.bf16x2.f32 %0, q1, q0;\n\t}"
+      : "=r"(t2)
+      : "r"(a2), "f"(p.rs), "f"(-p.s));
+  return t2;
 }
 // 8 weights (4 bf16x2 registers: element pairs (0,1) (2,3) (4,5) (6,7)) -> one packed word, nibble slots
 // [k0,k0+2,k0+4,k0+6,k0+1,k0+3,k0+5,k0+7]: even elements fill the low 16 bits, odd elements the high 16 bits
 __device__ __forceinline__ uint32_t quant_word_fast(const uint4& raw, const QFast& p) {
   const uint32_t w2[4] = {raw.x, raw.y, raw.z, raw.w};
-  constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
-  constexpr uint32_t k15 = 0x41704170u;  // (15.0, 15.0) bf16x2
-  float lo = 0.f, hi = 0.f, wgt = 1.f;
+  constexpr uint32_t k15 = 0x41704170u, k128 = 0x43004300u;  // (15, 15), (128, 128) bf16x2
+  uint32_t word = 0u - (k128 + (k128 << 4) + (k128 << 8) + (k128 << 12));
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const uint32_t a2 = bf2_sub(w2[j], p.minv2);                                  // bf16(w - min_val)
-    const float q0 = fast_quot(__uint_as_float(a2 << 16), p), q1 = fast_quot(__uint_as_float(a2 & 0xFFFF0000u), p);
-    uint32_t t2;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(t2) : "f"(q1), "f"(q0));            // bf16(a / scale)
-    t2 = bf2_max(bf2_min(t2, k15), 0u);                                           // clamp commutes with rint at 0 and 15
-    const float r0 = (__uint_as_float(t2 << 16) + kMagic) - kMagic;               // rint, ties to even
-    const float r1 = (__uint_as_float(t2 & 0xFFFF0000u) + kMagic) - kMagic;
-    lo = fmaf(r0, wgt, lo);
-    hi = fmaf(r1, wgt, hi);
-    wgt *= 16.f;
+    uint32_t t2 = fast_quot2(bf2_sub(w2[j], p.minv2), p);    // bf16(bf16(w - min_val) / scale)
+    t2 = bf2_max(bf2_min(t2, k15), 0u);                      // clamp commutes with rint at 0 and 15
+    asm("add.rn.bf16x2 %0, %0, %1;" : "+r"(t2) : "r"(k128)); // 128 + rint
+    word += t2 << (4 * j);
   }
-  return static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
+  return word;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -94,6 +95,25 @@ __device__ __forceinline__ uint32_t quant_word_fast(const uint4& raw, const QFas
 // out of registers already in place), reduces min/max over the 4 lanes that share a row,
 // and writes 512-byte tiles with one coalesced 16-byte store per lane.
 // ---------------------------------------------------------------------------------------
+// Minima (maxima) of four lanes with one row pair, [row of the pair][group] -> that of lane c's slot, c & 1 the row, and with two groups c >> 1 the group
+template <int NG, bool kMax>
+__device__ __forceinline__ uint32_t slot_merge(const uint32_t v[2][NG], int c) {
+  uint32_t k[NG];
+#pragma unroll
+  for (int gi = 0; gi < NG; ++gi) {
+    const uint32_t send = (c & 1) ? v[0][gi] : v[1][gi], keep = (c & 1) ? v[1][gi] : v[0][gi];
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, send, 1);
+    k[gi] = kMax ? bf2_max(keep, got) : bf2_min(keep, got);
+  }
+  uint32_t send = k[0], keep = k[0];
+  if (NG == 2) {
+    send = (c & 2) ? k[0] : k[NG - 1];
+    keep = (c & 2) ? k[NG - 1] : k[0];
+  }
+  const uint32_t got = __shfl_xor_sync(0xffffffffu, send, 2);
+  return kMax ? bf2_max(keep, got) : bf2_min(keep, got);
+}
+
 template <int G>
 __global__ void __launch_bounds__(256) int4_quantize_pack_kernel(
     const __nv_bfloat16* __restrict__ w, int64_t N, int64_t K, int64_t ldw, int64_t Np, int64_t Kp,
@@ -142,25 +162,30 @@ __global__ void __launch_bounds__(256) int4_quantize_pack_kernel(
           mx2[j & 1][gi] = bf2_max(mx2[j & 1][gi], v[i]);
         }
       }
-    QParams qp[2][NG];
+    // Of the four lanes of a row pair each takes one (row, group) slot, r + 2 gi = c mod 2 NG: the reduction hands a lane the halves of its own slot,
+    // the slot's parameters (two divisions) are worked out once, and shuffles give them back.  Every lane for itself was a fifth of the instructions.
+    const uint32_t a2 = slot_merge<NG, false>(mn2, c), b2 = slot_merge<NG, true>(mx2, c);
+    const QParams qp = tinygemm_qparams(fminf(__uint_as_float(a2 << 16), __uint_as_float(a2 & 0xFFFF0000u)),
+                                        fmaxf(__uint_as_float(b2 << 16), __uint_as_float(b2 & 0xFFFF0000u)), eps, div_mode);
+    if (c < 2 * NG) {
+      const int64_t row = strip * 16 + g + 8 * (c & 1);
+      const int64_t grp = uk * NG + (NG == 2 ? c >> 1 : 0);
+      sz[sz_index(grp, row, Kp / G)] = float_to_bf16_bits(qp.scale) | (float_to_bf16_bits(qp.zero) << 16);
+    }
     QFast qf[2][NG];
+    {
+      const float rs = __frcp_rn(qp.scale);
+      const uint32_t mb = float_to_bf16_bits(qp.min_val);
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
+      for (int r = 0; r < 2; ++r)
 #pragma unroll
-      for (int gi = 0; gi < NG; ++gi) {
-        uint32_t a2 = mn2[r][gi], b2 = mx2[r][gi];
-        a2 = bf2_min(a2, __shfl_xor_sync(0xffffffffu, a2, 1));
-        a2 = bf2_min(a2, __shfl_xor_sync(0xffffffffu, a2, 2));
-        b2 = bf2_max(b2, __shfl_xor_sync(0xffffffffu, b2, 1));
-        b2 = bf2_max(b2, __shfl_xor_sync(0xffffffffu, b2, 2));
-        const float a = fminf(__uint_as_float(a2 << 16), __uint_as_float(a2 & 0xFFFF0000u));
-        const float b = fmaxf(__uint_as_float(b2 << 16), __uint_as_float(b2 & 0xFFFF0000u));
-        qp[r][gi] = tinygemm_qparams(a, b, eps, div_mode);
-        qf[r][gi].s = qp[r][gi].scale;
-        qf[r][gi].rs = __frcp_rn(qp[r][gi].scale);
-        const uint32_t mb = float_to_bf16_bits(qp[r][gi].min_val);
-        qf[r][gi].minv2 = mb | (mb << 16);
-      }
+        for (int gi = 0; gi < NG; ++gi) {
+          const int from = (lane & ~3) | (r + 2 * gi);
+          qf[r][gi].s = __shfl_sync(0xffffffffu, qp.scale, from);
+          qf[r][gi].rs = __shfl_sync(0xffffffffu, rs, from);
+          qf[r][gi].minv2 = __shfl_sync(0xffffffffu, mb | (mb << 16), from);
+        }
+    }
     // quantize + pack
 #pragma unroll
     for (int t = 0; t < T; ++t) {
@@ -169,16 +194,6 @@ __global__ void __launch_bounds__(256) int4_quantize_pack_kernel(
       for (int j = 0; j < 4; ++j) words[j] = quant_word_fast(raw[t][j], qf[j & 1][(NG == 2) ? (j >> 1) : 0]);
       const int64_t kt = uk * T + t;
       packed[tile_slot(strip, kt, Kp / 64) * 32 + lane] = make_uint4(words[0], words[1], words[2], words[3]);
-    }
-    if (c == 0) {
-#pragma unroll
-      for (int r = 0; r < 2; ++r)
-#pragma unroll
-        for (int gi = 0; gi < NG; ++gi) {
-          const int64_t row = strip * 16 + g + 8 * r;
-          const int64_t grp = uk * NG + gi;
-          sz[sz_index(grp, row, Kp / G)] = float_to_bf16_bits(qp[r][gi].scale) | (float_to_bf16_bits(qp[r][gi].zero) << 16);
-        }
     }
   }
 }
