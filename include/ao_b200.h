@@ -298,6 +298,13 @@ AO_B200_API int ao_b200_silu_mul(const void* gate_up, void* out, int64_t B, int6
  * y packed; head_dim % 8 == 0.   y[i] = bf16( bf16(silu(gate[i])) * up[i] ), count % 8 == 0.   All 16-byte aligned. */
 AO_B200_API int ao_b200_rotary(const void* x, int64_t stride_b, int64_t stride_t, int64_t stride_h, const void* freqs_cis, void* y, int64_t B,
                                int64_t T, int64_t H, int64_t head_dim, void* stream);
+/* The keys of a prompt rotated in the same way and, with the values, stored in the rows pos[t] (int32 or int64 [T], pos_bytes each; negative: from the end) of the caches
+ * [B][H][S][head_dim]; k, v [B][T][H][head_dim] with strides as above.  ao_b200_repeat_heads: [heads][head_elements] -> [heads][rep][head_elements],
+ * keys and values.  head_dim and head_elements multiples of 8, all pointers but pos 16-byte aligned. */
+AO_B200_API int ao_b200_kv_rows(const void* k, int64_t k_stride_b, int64_t k_stride_t, int64_t k_stride_h, const void* v, int64_t v_stride_b,
+                                int64_t v_stride_t, int64_t v_stride_h, const void* freqs_cis, const void* pos, int pos_bytes, void* k_cache,
+                                void* v_cache, int64_t B, int64_t T, int64_t H, int64_t S, int64_t head_dim, void* stream);
+AO_B200_API int ao_b200_repeat_heads(const void* k, const void* v, void* k_out, void* v_out, int64_t heads, int64_t head_elements, int64_t rep, void* stream);
 AO_B200_API int ao_b200_silu_mul_rows(const void* gate, const void* up, void* y, int64_t count, void* stream);
 
 /* sample (generate.py:79-100: logits_to_probs + multinomial_sample_one_no_sync) in one launch:

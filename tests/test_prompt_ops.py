@@ -53,3 +53,30 @@ def test_norm_against_float64(rows, dim):
     # with gradients the single operations run, which have the same bound
     z = m(x)
     assert z.requires_grad and ((z.double() - ref).abs() <= 2.0 ** -7 * 1.01 * ref.abs() + 1e-38).all()
+
+
+@pytest.mark.parametrize("b,t,h,d,s,extra,by_kernel", [(1, 1, 1, 8, 8, 0, True), (2, 37, 3, 64, 40, 64, True), (1, 700, 8, 128, 704, 4096, True),
+                                                       (2, 5, 3, 64, 16, 1, False), (1, 6, 2, 12, 8, 0, False)])
+@torch.no_grad()
+def test_cache_rows_and_shared_heads_equal_the_single_operations(b, t, h, d, s, extra, by_kernel):
+    mine, ref = (M.KVCache(b, s, h, d).cuda() for _ in range(2))
+    for c in (mine, ref):
+        c.k_cache.fill_(3.0), c.v_cache.fill_(5.0)
+    rows = torch.randn(b, t, 2 * h * d + extra, device="cuda").to(torch.bfloat16)
+    k, v = (rows[..., i * h * d: (i + 1) * h * d].view(b, t, h, d) for i in range(2))
+    f = torch.randn(t, d // 2, 2, device="cuda").to(torch.bfloat16)
+    pos = torch.randperm(s, device="cuda")[:t]
+    pos[0] -= s                                                      # a position from the end
+    assert M.kv_rows(mine, pos.int() if h == 3 else pos, k, v, f) == by_kernel   # (both widths of positions)
+    ref.update(pos, _rotary(k, f).transpose(1, 2), v.transpose(1, 2))
+    if by_kernel:
+        assert torch.equal(mine.k_cache, ref.k_cache) and torch.equal(mine.v_cache, ref.v_cache)
+    # not for the kernel: other positions, a cache for more sequences, gradients
+    assert not M.kv_rows(mine, pos.short(), k, v, f) and not M.kv_rows(M.KVCache(b + 1, s, h, d).cuda(), pos, k, v, f) and not M.kv_rows(None, None, k, v, f)
+    with torch.enable_grad():
+        assert not M.kv_rows(mine, pos, k.detach().requires_grad_(), v, f)
+    for rep in (1, 2, 5):
+        ks, vs = M.repeat_heads(ref.k_cache, ref.v_cache, rep)
+        assert torch.equal(ks, ref.k_cache.repeat_interleave(rep, dim=1)) and torch.equal(vs, ref.v_cache.repeat_interleave(rep, dim=1))
+    kt, vt = ref.k_cache.transpose(1, 2), ref.v_cache.transpose(1, 2)
+    assert all(torch.equal(x, y.repeat_interleave(2, dim=1)) for x, y in zip(M.repeat_heads(kt, vt, 2), (kt, vt)))

@@ -77,6 +77,8 @@ SIGNATURES = {
                                           _vp, _i64, _vp],
     "ao_b200_silu_mul": [_vp, _vp, _i64, _i64, _vp],
     "ao_b200_rotary": [_vp, _i64, _i64, _i64, _vp, _vp, _i64, _i64, _i64, _i64, _vp],
+    "ao_b200_kv_rows": [_vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64, _vp, _vp, _i32, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _vp],
+    "ao_b200_repeat_heads": [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp],
     "ao_b200_silu_mul_rows": [_vp, _vp, _vp, _i64, _vp],
     "ao_b200_stream_wait_value32": [_vp, _vp, ctypes.c_uint32],
     "ao_b200_sample": [_vp, _i64, _i64, _i64, _f32, _i32, _vp, _i64, _vp, _vp],

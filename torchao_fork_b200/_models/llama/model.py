@@ -171,6 +171,35 @@ def apply_rotary_emb(x: Tensor, freqs_cis: Tensor) -> Tensor:
     return out.flatten(3).type_as(x)
 
 
+def kv_rows(cache, input_pos, k: Tensor, v: Tensor, freqs_cis: Tensor) -> bool:
+    """k (to be rotated) and v [B][T][H][hd] into the rows input_pos of a plain cache, in one launch; False if that is not for these tensors."""
+    if type(cache) is not KVCache or k.dim() != 4 or not _rows_by_kernel(k, v, freqs_cis, cache.k_cache, cache.v_cache):
+        return False
+    b, t, h, d = k.shape
+    s = cache.k_cache.shape[2]
+    if not (type(input_pos) is Tensor and runs_eagerly(input_pos) and input_pos.dtype in (torch.int32, torch.int64) and input_pos.device == k.device and input_pos.shape == (t,)
+            and input_pos.is_contiguous() and v.shape == k.shape and d % 8 == 0 and freqs_cis.is_contiguous() and freqs_cis.numel() == t * d
+            and all(x.stride(3) == 1 and all(n % 8 == 0 for n in x.stride()[:3]) for x in (k, v))
+            and all(x.shape == (b, h, s, d) and x.is_contiguous() for x in (cache.k_cache, cache.v_cache))):
+        return False
+    with _on(k.device.index):
+        _lib.check(_lib.lib().ao_b200_kv_rows(k.data_ptr(), *k.stride()[:3], v.data_ptr(), *v.stride()[:3], freqs_cis.data_ptr(), input_pos.data_ptr(),
+                                              input_pos.element_size(), cache.k_cache.data_ptr(), cache.v_cache.data_ptr(), b, t, h, s, d, _stream(k)), "kv_rows")
+    return True
+
+
+def repeat_heads(k: Tensor, v: Tensor, rep: int):
+    """[B][H][S][hd] -> [B][H * rep][S][hd], every head for the rep query heads that share it"""
+    if (rep > 1 and k.dim() == 4 and k.shape == v.shape and _rows_by_kernel(k, v) and k.is_contiguous() and v.is_contiguous()
+            and k.shape[2] * k.shape[3] % 8 == 0):
+        b, h, s, d = k.shape
+        ko, vo = (torch.empty(b, h * rep, s, d, dtype=k.dtype, device=k.device) for _ in range(2))
+        with _on(k.device.index):
+            _lib.check(_lib.lib().ao_b200_repeat_heads(k.data_ptr(), v.data_ptr(), ko.data_ptr(), vo.data_ptr(), b * h, s * d, rep, _stream(k)), "repeat_heads")
+        return ko, vo
+    return k.repeat_interleave(rep, dim=1), v.repeat_interleave(rep, dim=1)
+
+
 class Attention(nn.Module):
     """reference: model.py:411-473"""
 
@@ -196,12 +225,14 @@ class Attention(nn.Module):
         q_size, kv_size = self.n_head * self.head_dim, self.n_local_heads * self.head_dim
         q, k, v = self.wqkv(x).split([q_size, kv_size, kv_size], dim=-1)
         q = apply_rotary_emb(q.view(b, t, self.n_head, self.head_dim), freqs_cis).transpose(1, 2)
-        k = apply_rotary_emb(k.view(b, t, self.n_local_heads, self.head_dim), freqs_cis).transpose(1, 2)
-        v = v.view(b, t, self.n_local_heads, self.head_dim).transpose(1, 2)
-        if self.kv_cache is not None:
-            k, v = self.kv_cache.update(input_pos, k, v)
-        rep = self.n_head // self.n_local_heads
-        k, v = k.repeat_interleave(rep, dim=1), v.repeat_interleave(rep, dim=1)
+        k, v = k.view(b, t, self.n_local_heads, self.head_dim), v.view(b, t, self.n_local_heads, self.head_dim)
+        if kv_rows(self.kv_cache, input_pos, k, v, freqs_cis):
+            k, v = self.kv_cache.k_cache, self.kv_cache.v_cache
+        else:
+            k, v = apply_rotary_emb(k, freqs_cis).transpose(1, 2), v.transpose(1, 2)
+            if self.kv_cache is not None:
+                k, v = self.kv_cache.update(input_pos, k, v)
+        k, v = repeat_heads(k, v, self.n_head // self.n_local_heads)
         if mask is not None:
             y = F.scaled_dot_product_attention(q, k, v, attn_mask=mask, dropout_p=0.0)
         else:
