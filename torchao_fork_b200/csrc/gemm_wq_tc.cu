@@ -50,6 +50,7 @@
 namespace ao {
 
 constexpr int kWqEpiWarps = 4, kWqDqWarps = 16;
+constexpr int kWqBehind = 8;  // units (wq_gemm_kernel, t_early)
 constexpr int kWqWProd = kWqEpiWarps + kWqDqWarps, kWqXProd = kWqWProd + 1, kWqMma = kWqXProd + 1;
 constexpr int kWqThreads = (kWqMma + 2) * 32;  // 768
 constexpr int kWqSlots = 4;                    // ring of A in tensor memory: 64 columns (128 k) each
@@ -285,7 +286,7 @@ struct WqRing {
 // ---- the GEMM ----------------------------------------------------------------------------------------------------------
 // G == 0: int8.  Shared memory: header, output tile, activation ring (x_slots x x_bytes), weight ring (w_slots x [8 strips x 128 k]
 // [8 strips x parameters]).
-template <int G, bool DEFER, bool PAIR>
+template <int G, bool DEFER, bool PAIR, bool EARLY>
 __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_constant__ WqParams p) {
   extern __shared__ __align__(1024) uint8_t wq_smem[];
   constexpr bool kI8 = (G == 0);
@@ -306,7 +307,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
   uint64_t* dempty = dfull + 2;
   uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(dempty + 2);
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_base_s + 1);
-  volatile int* s_last = dead + 1;        // [2]: this CTA was the last to reach its first / last tile
+  volatile int* s_last = dead + 1;        // [3]: this CTA was the last to reach its first / last tile; it finishes its last tile from its accumulators
   uint8_t* stage = wq_smem + kWqHeader;   // output tile [NT][kWqPitch]
   uint8_t* xring = stage + p.NT * kWqPitch;
   uint8_t* wring = wq_smem + p.off_w;
@@ -358,6 +359,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
       s_last[lane - 16] = 0;
     } else if (lane == 18) {
       *dead = 0;
+      s_last[2] = 0;
     }
     fence_barrier_init();
     __syncwarp();
@@ -619,6 +621,13 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     const uint32_t lane_col = tb + ((uint32_t)(32 * warp) << 16);
     WqRing d, x, w;
     bool ok = true;
+    // EARLY: this CTA's last tile, if it is shared with the next one alone and that one has more to do behind it: as a rule that one's share was there
+    // long ago.  Then this one stays in tensor memory and all warps finish the tile, at the end: no store of 64 ... 128 KB and its way back.
+    int t_early = -1;
+    if (EARLY && u1 % KU != 0) {
+      const int t = u1 / KU;
+      if (u0 <= t * KU && wq_first(worker + 2, p.base, p.rem, p.quantum) >= (t + 1) * KU + kWqBehind) t_early = t;
+    }
     for (int u = u0, t = u0 / KU; u < u1; ++t) {
       const int ue = min(u1, (t + 1) * KU), nb = t / p.MT, mt = t - nb * p.MT;
       const bool whole = u == t * KU && ue == (t + 1) * KU;
@@ -677,27 +686,16 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
           for (int i = 0; i < 4; ++i) __stcg(mine + i * 128, make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]));
         }
       } else {
-        if (!whole && ue == u1) {
-          // the others' shares of this CTA's last tile, written long ago as a rule, on their way back to L2
-          const int c0 = wq_owner(t * KU, p.base, p.rem, p.quantum), c1 = wq_owner(t * KU + KU - 1, p.base, p.rem, p.quantum);
-          for (int cc = c0; cc <= c1; ++cc)
-            if (cc != worker)
-              for (int i = threadIdx.x; i < NT * 4; i += kWqEpiWarps * 32)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(share(cc, t)) + (int64_t)i * 128));
-        }
         ok = ok && wait(&dfull[d.slot], d.use);
         wq_fence_after();
-        if (!whole && ue == u1) {
-          // This CTA's last tile, and it is shared.  As a rule the others' shares (their first tiles, done long ago) are there: then this one
-          // stays in tensor memory, and all warps finish the tile below.
+        if (EARLY && t == t_early) {
           if (wq_epi_sync(!ok)) break;
           bool here = false;
           if (threadIdx.x == 0) {
-            const int others = wq_owner(t * KU + KU - 1, p.base, p.rem, p.quantum) - wq_owner(t * KU, p.base, p.rem, p.quantum);
             uint32_t arrived;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(arrived) : "l"(p.tickets + t * kRanks + rank) : "memory");
-            here = arrived == (uint32_t)others;
-            if (here) s_last[t == u0 / KU ? 0 : 1] = 2;
+            here = arrived == 1u;
+            if (here) s_last[2] = 1;
           }
           if (wq_epi_sync(here)) {
             wq_fence_before();
@@ -755,74 +753,63 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
 
   // ---- shared tiles that this CTA was the last to reach: all warps add the shares in CTA order and finish the rows ----
   __syncthreads();
-  wq_fence_after();
 #pragma unroll 1
   for (int k = 0; k < 2; ++k) {
-    const int last = s_last[k];
-    if (last == 0) continue;
+    if (s_last[k] == 0) continue;
     __threadfence();
     const int t = k == 0 ? u0 / KU : (u1 - 1) / KU, nb = t / p.MT, mt = t - nb * p.MT;
     const int c0 = wq_owner(t * KU, p.base, p.rem, p.quantum), c1 = wq_owner(t * KU + KU - 1, p.base, p.rem, p.quantum);
-    // last == 2: this CTA's share is its accumulators (which of them hold something: as in the epilogue)
-    const int us = max(u0, t * KU), held = u1 - us;
+    for (int it = warp; it < NT / 2; it += kWqThreads / 32) {  // (column block, quadrant, half)
+      const int h = it & 1, q = (it >> 1) & 3, c = (it >> 3) * 16;
+      float f[8], sc[4];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = 0.f;
+      row_scales(nb, q, sc);
+#pragma unroll 4
+      for (int cc = c0; cc <= c1; ++cc) {
+        const float4* src = share(cc, t) + (c / 4 + 2 * h) * 128 + q * 32 + lane;
+        const float4 v0 = __ldcg(src), v1 = __ldcg(src + 128);
+        f[0] += v0.x, f[1] += v0.y, f[2] += v0.z, f[3] += v0.w, f[4] += v1.x, f[5] += v1.y, f[6] += v1.z, f[7] += v1.w;
+      }
+      to_stage(q, c, h, f, sc);
+    }
+    __syncthreads();
+    copy_out(nb, mt, threadIdx.x, kWqThreads);
+    __syncthreads();
+  }
+  if (EARLY && s_last[2] != 0) {
+    // the last tile: this CTA's share, the first, is its accumulators (which of them hold something: as in the epilogue), the next CTA's is the other
+    wq_fence_after();
+    __threadfence();
+    const int t = u1 / KU, nb = t / p.MT, mt = t - nb * p.MT, held = u1 - t * KU;
     const bool two = n_mma == 2 && held > 1;
-    const int q = warp & 3;                            // tensor memory: a warp reaches the lanes of its quadrant
-    const uint32_t dcol = tb + ((uint32_t)(32 * q) << 16) + (d_bufs == 2 ? ((t - u0 / KU) & 1) * 128 : 0) + (n_mma == 2 && held == 1 ? ((us - u0) & 1) * 64 : 0);
+    const int q = warp & 3;                                // tensor memory: a warp reaches the lanes of its quadrant
+    const uint32_t dcol = tb + ((uint32_t)(32 * q) << 16) + (d_bufs == 2 ? ((t - u0 / KU) & 1) * 128 : 0) + (n_mma == 2 && held == 1 ? ((t * KU - u0) & 1) * 64 : 0);
+    const float4* other = share(worker + 1, t) + q * 32 + lane;
     float sc[4];
     row_scales(nb, q, sc);
-    constexpr int kStep = kWqThreads / 128, kBatch = 3;  // (column block, half) pairs per round of the quadrant's warps; rounds with their loads in flight
-    const auto add8 = [](float (&f)[8], const float4& a, const float4& b) {
-      f[0] += a.x, f[1] += a.y, f[2] += a.z, f[3] += a.w, f[4] += b.x, f[5] += b.y, f[6] += b.z, f[7] += b.w;
-    };
-    const auto at = [&](int cc, int it) { return share(cc, t) + ((it >> 1) * 4 + 2 * (it & 1)) * 128 + q * 32 + lane; };
-    if (!DEFER && last == 2 && c1 - c0 == 1) {
-      // own accumulators and one other share (a sum of two, in either order)
-      const int other = c0 == worker ? c1 : c0;
+    constexpr int kStep = kWqThreads / 128, kBatch = 3;    // (column block, half) pairs per round of the quadrant's warps; rounds with their loads in flight
 #pragma unroll 1
-      for (int it0 = warp >> 2; it0 < NT / 8; it0 += kStep * kBatch) {
-        float4 w[kBatch][2];
+    for (int it0 = warp >> 2; it0 < NT / 8; it0 += kStep * kBatch) {
+      float4 w[kBatch][2];
 #pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-          const int it = min(it0 + j * kStep, NT / 8 - 1);
-          w[j][0] = __ldcg(at(other, it)), w[j][1] = __ldcg(at(other, it) + 128);
-        }
-#pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-          const int it = it0 + j * kStep, h = it & 1, c = (it >> 1) * 16;
-          if (it >= NT / 8) break;
-          uint32_t v[8], v2[8];
-          float f[8];
-          wq_ld_16x256b_x2(dcol + ((uint32_t)(16 * h) << 16) + c, v);
-          if (two) wq_ld_16x256b_x2(dcol + ((uint32_t)(16 * h) << 16) + 64 + c, v2);
-          wq_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) f[i] = two ? __uint_as_float(v[i]) + __uint_as_float(v2[i]) : __uint_as_float(v[i]);
-          add8(f, w[j][0], w[j][1]);
-          to_stage(q, c, h, f, sc);
-        }
+      for (int j = 0; j < kBatch; ++j) {
+        const float4* src = other + min(it0 + j * kStep, NT / 8 - 1) * 256;
+        w[j][0] = __ldcg(src), w[j][1] = __ldcg(src + 128);
       }
-    } else {
-#pragma unroll 1
-      for (int it = warp >> 2; it < NT / 8; it += kStep) {
-        const int h = it & 1, c = (it >> 1) * 16;
-        float f[8];
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j) {
+        const int it = it0 + j * kStep, h = it & 1, c = (it >> 1) * 16;
+        if (it >= NT / 8) break;
         uint32_t v[8], v2[8];
+        float f[8];
+        wq_ld_16x256b_x2(dcol + ((uint32_t)(16 * h) << 16) + c, v);
+        if (two) wq_ld_16x256b_x2(dcol + ((uint32_t)(16 * h) << 16) + 64 + c, v2);
+        wq_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] = 0.f, v[i] = v2[i] = 0u;
-        if (!DEFER && last == 2) {
-          wq_ld_16x256b_x2(dcol + ((uint32_t)(16 * h) << 16) + c, v);
-          if (two) wq_ld_16x256b_x2(dcol + ((uint32_t)(16 * h) << 16) + 64 + c, v2);
-          wq_ld_wait();
-        }
-#pragma unroll 4
-        for (int cc = c0; cc <= c1; ++cc) {
-          if (!DEFER && last == 2 && cc == worker) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] += two ? __uint_as_float(v[i]) + __uint_as_float(v2[i]) : __uint_as_float(v[i]);
-          } else {
-            add8(f, __ldcg(at(cc, it)), __ldcg(at(cc, it) + 128));
-          }
-        }
+        for (int i = 0; i < 8; ++i) f[i] = two ? __uint_as_float(v[i]) + __uint_as_float(v2[i]) : __uint_as_float(v[i]);
+        f[0] += w[j][0].x, f[1] += w[j][0].y, f[2] += w[j][0].z, f[3] += w[j][0].w;
+        f[4] += w[j][1].x, f[5] += w[j][1].y, f[6] += w[j][1].z, f[7] += w[j][1].w;
         to_stage(q, c, h, f, sc);
       }
     }
@@ -942,11 +929,18 @@ static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
   if (p.n_mma == 2) p.w_slots &= ~1;           // two MMA warps let the two dequant sets drift apart: each set keeps slots of its own
   p.a_slots = p.w_slots == 3 ? 3 : kWqSlots;   // (see a_first in the kernel)
   const size_t smem = off_w + (size_t)p.w_slots * kWSlot;
-  auto kern = wq_gemm_kernel<G, DEFER, PAIR>;
-  static bool attr_done = false;
-  if (!attr_done) {
+  // The last tile from the accumulators where every CTA has a tile's worth of units, so that a tile has two owners as a rule: 4096 x 4096, 2048 rows
+  // 63.9 -> 57.1 us; 14336 x 4096 int4, 300 / 1000 rows 39.8 -> 36.2 / 94.0 -> 89.3; 28672 x 4096 int8, 32 / 77 / 300 rows 32.4 -> 30.9 / 37.7 -> 34.9 /
+  // 74.6 -> 70.9.  With less a CTA its neighbour is not there yet or it has several, and the mere presence of the code costs 0.2 to 0.5 us
+  // (14336 x 4096, 77 rows: 25.6 -> 25.8; 4096 x 4096 int8, 200 rows: 28.5 -> 29.0).
+  constexpr bool kCan = !DEFER;
+  const bool early = kCan && (int64_t)w.base * w.quantum >= w.KU;
+  auto kern = wq_gemm_kernel<G, DEFER, PAIR, false>;
+  static bool attr_done[2] = {};
+  if (early) kern = wq_gemm_kernel<G, DEFER, PAIR, kCan>;
+  if (!attr_done[early]) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBudget) != cudaSuccess) return AO_B200_ERR_CUDA;
-    attr_done = true;
+    attr_done[early] = true;
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(w.workers * w.ranks));
