@@ -153,15 +153,17 @@ struct HqqChunk {
   int first, count;             // iterations [first, first + count)
 };
 
-// number of the last iteration among the first n whose means are known: the first one that does not improve, else n - 1
+// number of the last iteration among the first n whose means are known: the first one that does not improve (:1956; up to it each mean is the best so
+// far), else n - 1.  All lanes of a warp together: one look at a mean after the other was 20 dependent loads at the start of every block.
 __device__ __forceinline__ int hqq_last(const double* __restrict__ mean, int n, bool& stopped) {
-  double best = 1e4;            // (:1956)
-  for (int i = 0; i < n; ++i) {
-    if (!(mean[i] < best)) {
+  for (int first = 0; first < n; first += 32) {
+    const int i = first + (threadIdx.x & 31);
+    const bool worse = i < n && !(mean[i] < (i == 0 ? 1e4 : mean[i - 1]));
+    const uint32_t any = __ballot_sync(0xffffffffu, worse);
+    if (any != 0) {
       stopped = true;
-      return i;
+      return first + __ffs(any) - 1;
     }
-    best = mean[i];
   }
   stopped = false;
   return n - 1;
@@ -401,6 +403,7 @@ __global__ void __launch_bounds__(kHqqWarps * 32) hqq_plain_kernel(const __nv_bf
 
 // clamp(rint(w * s + z), 0, 15) of eight weights as a packed word.  The clamp commutes with rint at 0 and 15 (and takes NaN to 0 either way); rint of
 // what is left is an add of 1.5 * 2^23, whose bits are a constant plus q: shifted and added up, eight of them are the word plus a constant.
+// (Product and sum one weight at a time: as f32x2 they came out as one fused operation, and one word in a million differed.)
 __device__ __forceinline__ uint32_t packed_word(const uint4& raw, float s, float z) {
   constexpr uint32_t kMagic = 0x4B400000u;  // 1.5 * 2^23
   const uint32_t w2[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -408,12 +411,8 @@ __device__ __forceinline__ uint32_t packed_word(const uint4& raw, float s, float
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
     float a = __uint_as_float(w2[p] << 16), b = __uint_as_float(w2[p] & 0xFFFF0000u);
-    asm("{\n\t.reg .b64 v, s, z;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 s, {%2, %2};\n\tmov.b64 z, {%3, %3};\n\t"
-        "mul.rn.f32x2 v, v, s;\n\tadd.rn.f32x2 v, v, z;\n\tmov.b64 {%0, %1}, v;\n\t}"
-        : "+f"(a), "+f"(b)
-        : "f"(s), "f"(z));
-    a = fminf(fmaxf(a, 0.f), 15.f) + __uint_as_float(kMagic);
-    b = fminf(fmaxf(b, 0.f), 15.f) + __uint_as_float(kMagic);
+    a = __fadd_rn(fminf(fmaxf(__fadd_rn(__fmul_rn(a, s), z), 0.f), 15.f), __uint_as_float(kMagic));
+    b = __fadd_rn(fminf(fmaxf(__fadd_rn(__fmul_rn(b, s), z), 0.f), 15.f), __uint_as_float(kMagic));
     word += (__float_as_uint(a) - kMagic) << (4 * nib_slot(2 * p));
     word += (__float_as_uint(b) - kMagic) << (4 * nib_slot(2 * p + 1));
   }
@@ -429,10 +428,7 @@ __global__ void __launch_bounds__(256) hqq_packed_kernel(const __nv_bfloat16* __
                                                          const float* __restrict__ scale, const float* __restrict__ hist, const double* __restrict__ mean,
                                                          int iters, uint4* __restrict__ packed, uint32_t* __restrict__ sz) {
   constexpr int kHalves = G < 64 ? 2 : 1;   // groups per tile
-  __shared__ const float* s_zero;
-  if (threadIdx.x == 0) s_zero = hqq_zero(hist, N * (K / G), mean, iters);
-  __syncthreads();
-  const float* zero = s_zero;
+  const float* zero = nullptr;
   const int64_t groups = K / G;
   const uint32_t k_tiles = (uint32_t)(Kp / 64), groups_p = (uint32_t)(Kp / G);
   const uint32_t tiles = (uint32_t)(Np / 16) * k_tiles;                 // < 2^32 by far: a tile is 2 KB of weights
@@ -448,6 +444,7 @@ __global__ void __launch_bounds__(256) hqq_packed_kernel(const __nv_bfloat16* __
       const int64_t row = row0 + 8 * (j & 1), k = k0 + 32 * (j >> 1);
       if (row < N && k < K) raw[j] = ldg128(w + row * K + k);
     }
+    if (zero == nullptr) zero = hqq_zero(hist, N * (K / G), mean, iters);  // (while the first weights are on their way)
 #pragma unroll
     for (int r = 0; r < 2; ++r)
 #pragma unroll
@@ -465,6 +462,7 @@ __global__ void __launch_bounds__(256) hqq_packed_kernel(const __nv_bfloat16* __
     }
     packed[tile * 32 + lane] = make_uint4(words[0], words[1], words[2], words[3]);
   }
+  if (zero == nullptr) zero = hqq_zero(hist, N * (K / G), mean, iters);
   const uint64_t params = (uint64_t)Np * groups_p;
   for (uint64_t o = (uint64_t)blockIdx.x * 256 + threadIdx.x; o < params; o += (uint64_t)gridDim.x * 256) {
     const uint32_t pair = (uint32_t)(o >> 4), strip = pair / groups_p, grp = pair - strip * groups_p;   // [strip][group][16 rows]
