@@ -162,3 +162,14 @@ def test_hqq_search_equals_the_iterations_one_by_one(shape, gs, spread):
     ps, pz = aops.unpack_scales_and_zeros_b200(sz)
     assert torch.equal(ps[:n, : k // gs], s) and torch.equal(pz[:n, : k // gs], z)
     assert not ps[n:].any() and not pz[n:].any() and not ps[:, k // gs :].any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gs,seed", [(64, 34), (32, 35), (128, 36), (256, 37)])
+def test_packed_words_of_many_weights_equal_the_plain_result(gs, seed):
+    """Enough weights that some land within a rounding error of a half: product and sum have to be rounded one after the other in both."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    w = (torch.randn(4096, 4096, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    packed, _ = T.b200_int4_hqq_quantize_pack(w, gs)
+    q, _, _ = T.b200_int4_hqq_quantize(w, gs)
+    assert torch.equal(T.b200_int4_unpack(packed)[:4096, :4096], q)
