@@ -120,6 +120,7 @@ AO_B200_API int ao_b200_tinygemm_pack(const int32_t* q, int64_t N, int64_t K, in
  * host-side F.pad of the activation); y: bf16 [M][N_out] row stride ldy.
  * few rows -> HBM-bound split-K tensor-core GEMV; more rows (from 3 to 17 on, by the weight's size) -> tcgen05 GEMM.
  * A wait of the GEMM that runs out (about two seconds) leaves NaN in the rows concerned.
+ * The weights may be the work of the kernel in front in the stream: they are read behind its end.  (The same for ao_b200_int8_mm.)
  * workspace: ao_b200_int4_mm_workspace_bytes(...) bytes, zero-initialised once by the
  * caller (the GEMV's part in front is zero again on exit, the GEMM's behind it is not
  * and need not be); may be NULL when that returns 0. */
@@ -141,7 +142,8 @@ AO_B200_API int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ld
  * the reference's _weight_int4pack_mm_for_cpu) — see csrc/gemv_int4_fused.cu, csrc/gemv_int4_tc.cu.
  * workspace: ao_b200_int4_mm_workspace_bytes(M, Np, Kp) bytes, zero-initialised once by the caller (the kernels leave
  * it zeroed); with NULL / too small a workspace the call still works but skips the tensor-memory kernel.  Returns
- * AO_B200_ERR_WORKSPACE when M * K does not fit any decode kernel's shared-memory staging (use ao_b200_int4_mm then). */
+ * AO_B200_ERR_WORKSPACE when M * K does not fit any decode kernel's shared-memory staging (use ao_b200_int4_mm then).
+ * The weights must have been there before the kernel in front of this call was launched: they are read while it ends. */
 AO_B200_API int ao_b200_int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx,
                             const void* packed, const void* scale_and_zero, int64_t Np, int64_t Kp,
                             int group_size, void* y, int64_t N_out, int64_t ldy,

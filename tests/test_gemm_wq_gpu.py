@@ -132,6 +132,31 @@ def test_weights_written_by_the_kernel_in_front(bits, m):
         assert torch.equal(y, want[i % 2]), i
 
 
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("m", [1, 2, 3, 8])
+@pytest.mark.parametrize("n,k", [(4096, 14336), (8192, 28672), (4096, 8192)])
+def test_weights_of_few_rows_written_by_the_kernel_in_front(bits, m, n, k):
+    # the same where the call is a GEMV, which starts while the kernel in front of it ends: k of one CTA, and of a cluster's in halves or quarters
+    x, packed, scales, want = None, [], [], []
+    for seed in range(2):
+        gen = torch.Generator(device="cuda").manual_seed(seed)
+        w = torch.randn(n, k, generator=gen, device="cuda").to(torch.bfloat16)
+        x = torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16) if x is None else x
+        p, sc = T.b200_int4_quantize_pack(w, 128, 1e-6, True) if bits == 4 else T.b200_int8_quantize(w, 1e-6, True)
+        p = p if bits == 4 else T.b200_int8_pack(p)
+        packed.append(p), scales.append(sc)
+        torch.cuda.synchronize()
+        want.append(T.b200_int4_weight_only_mm(x, p, 128, sc, n) if bits == 4 else T.b200_int8_weight_only_mm(x, p, sc))
+    pw, sw, got = torch.empty_like(packed[0]), torch.empty_like(scales[0]), []
+    torch.cuda.synchronize()
+    for i in range(24):
+        sw.copy_(scales[i % 2])
+        pw.copy_(packed[i % 2])
+        got.append(T.b200_int4_weight_only_mm(x, pw, 128, sw, n) if bits == 4 else T.b200_int8_weight_only_mm(x, pw, sw))
+    for i, y in enumerate(got):
+        assert torch.equal(y, want[i % 2]), i
+
+
 def test_threads_that_share_a_stream():
     # a call is a staging launch and the GEMM behind it, over one workspace per stream: nobody's launch may come between them
     import threading

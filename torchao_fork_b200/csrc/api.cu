@@ -6,13 +6,13 @@ int int4_gemv(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* pac
               int64_t Kp, int G, void* y, int64_t N_out, int64_t ldy, cudaStream_t s);
 int int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np,
                     int64_t Kp, int G, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps,
-                    const void* residual, int64_t ld_res, int epilogue, int max_stages, bool pdl, cudaStream_t s);
+                    const void* residual, int64_t ld_res, int epilogue, int max_stages, int follow, cudaStream_t s);
 int int4_gemv_imma(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np,
                    int64_t Kp, int G, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps,
-                   const void* residual, int64_t ld_res, int epilogue, int max_stages, bool pdl, cudaStream_t s);
+                   const void* residual, int64_t ld_res, int epilogue, int max_stages, int follow, cudaStream_t s);
 int int4_gemv_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np,
                  int64_t Kp, int G, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps, const void* residual,
-                 int64_t ld_res, int epilogue, void* workspace, int64_t workspace_bytes, bool pdl, cudaStream_t s);
+                 int64_t ld_res, int epilogue, void* workspace, int64_t workspace_bytes, int follow, cudaStream_t s);
 int64_t int4_gemv_tc_workspace_bytes(int64_t Np);
 int int4_gemm_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np, int64_t Kp,
                  int G, void* y, int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res, void* workspace, int64_t workspace_bytes,
@@ -24,12 +24,12 @@ int64_t int8_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
 int int8_gemv(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Kp,
               void* y, int64_t N_out, int64_t ldy, cudaStream_t s);
 int int4_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np, int64_t Kp, int G, void* y,
-                    int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res, int max_stages, bool pdl, cudaStream_t s);
+                    int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res, int max_stages, int follow, cudaStream_t s);
 int int8_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Kp, void* y, int64_t N_out,
-                    int64_t ldy, const void* residual, int64_t ld_res, int max_stages, bool pdl, cudaStream_t s);
+                    int64_t ldy, const void* residual, int64_t ld_res, int max_stages, int follow, cudaStream_t s);
 int int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Np,
                     int64_t Kp, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps, const void* residual,
-                    int64_t ld_res, int epilogue, int max_stages, bool pdl, cudaStream_t s);
+                    int64_t ld_res, int epilogue, int max_stages, int follow, cudaStream_t s);
 int int8_gemm_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Np,
                  int64_t Kp, void* y, int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res, void* workspace,
                  int64_t workspace_bytes, cudaStream_t s);
@@ -80,6 +80,10 @@ const Tunables& tunables() {
   static Tunables t;
   return t;
 }
+// The plain products (ao_b200_int4_mm, ao_b200_int8_mm) may follow the launch that writes their weights (quantize_, then a call); the fused ones and
+// ao_b200_mm_residual ask for weights that are long there.
+int plain_follow() { return tunables().pdl ? ao::kFollowOrdered : ao::kFollowPlain; }
+int settled_follow() { return tunables().pdl ? ao::kFollowSettled : ao::kFollowPlain; }
 }  // namespace
 
 // Which calls of up to 16 rows take the GEMM (gemm_wq_tc.cu) rather than the GEMV that keeps the activations in shared memory.  The GEMM
@@ -127,7 +131,7 @@ extern "C" int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
   auto yb = static_cast<__nv_bfloat16*>(y);
   if (M >= 3 && M <= 8 && !ao::int4_gemv_fused_fits(M, Kp, group_size, tunables().stages)) {   // too long for one CTA: k shared out (as in ao_b200_mm_residual)
     const int e = ao::int4_gemv_split(x, M, Kx, ldx, packed, scale_and_zero, Np, Kp, group_size, y, N_out, ldy, nullptr, 0, tunables().stages,
-                                      tunables().pdl != 0, s);
+                                      plain_follow(), s);
     if (e != AO_B200_ERR_WORKSPACE) return e;
   }
   if (int4_by_gemm(M, Np, Kp, group_size)) {
@@ -145,13 +149,13 @@ extern "C" int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
       // pass 0: tensor-memory kernel when forced; integer-MMA kernel; pass 1: tensor-memory kernel for large weights
       if (((pass == 0 && tunables().gemv_tc == 1) || (pass == 1 && tc_large)) && mc <= 5) {
         e = ao::int4_gemv_tc(xb + m0 * ldx, mc, Kx, ldx, packed, scale_and_zero, Np, Kp, group_size, yb + m0 * ldy, N_out,
-                             ldy, nullptr, 0.f, nullptr, 0, 0, workspace, workspace_bytes, tunables().pdl != 0, s);
+                             ldy, nullptr, 0.f, nullptr, 0, 0, workspace, workspace_bytes, plain_follow(), s);
         if (e == AO_B200_OK) break;
         if (e != AO_B200_ERR_WORKSPACE && e != AO_B200_ERR_UNSUPPORTED) return e;
       }
       if (pass == 0 && tunables().gemv_imma && mc <= 2) {
         e = ao::int4_gemv_imma(xb + m0 * ldx, mc, Kx, ldx, packed, scale_and_zero, Np, Kp, group_size, yb + m0 * ldy, N_out,
-                               ldy, nullptr, 0.f, nullptr, 0, 0, tunables().stages, tunables().pdl != 0, s);
+                               ldy, nullptr, 0.f, nullptr, 0, 0, tunables().stages, plain_follow(), s);
         if (e == AO_B200_OK) break;
         if (e != AO_B200_ERR_WORKSPACE && e != AO_B200_ERR_UNSUPPORTED) return e;
       }
@@ -159,7 +163,7 @@ extern "C" int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
     if (e == AO_B200_OK) continue;
     if (tunables().gemv_version == 3) {
       e = ao::int4_gemv_fused(xb + m0 * ldx, mc, Kx, ldx, packed, scale_and_zero, Np, Kp, group_size, yb + m0 * ldy,
-                              N_out, ldy, nullptr, 0.f, nullptr, 0, 0, tunables().stages, tunables().pdl != 0, s);
+                              N_out, ldy, nullptr, 0.f, nullptr, 0, 0, tunables().stages, plain_follow(), s);
       if (e == AO_B200_OK) continue;
       if (e != AO_B200_ERR_WORKSPACE) return e;
     }
@@ -191,19 +195,19 @@ extern "C" int ao_b200_int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int
     if ((pass == 0 && tunables().gemv_tc == 1) || (pass == 1 && tc_large)) {
       // tensor-memory kernel (M <= 5, Np % 128 == 0, activations + >= 3 ring stages must fit); else the mma.sync kernels
       const int e = ao::int4_gemv_tc(x, M, Kx, ldx, packed, scale_and_zero, Np, Kp, group_size, y, N_out, ldy, norm_weight,
-                                     norm_eps, residual, ld_res, epilogue, workspace, workspace_bytes, tunables().pdl != 0,
+                                     norm_eps, residual, ld_res, epilogue, workspace, workspace_bytes, settled_follow(),
                                      static_cast<cudaStream_t>(stream));
       if (e != AO_B200_ERR_WORKSPACE && e != AO_B200_ERR_UNSUPPORTED) return e;
     }
     if (pass == 0 && tunables().gemv_imma && M <= 2) {
       const int e = ao::int4_gemv_imma(x, M, Kx, ldx, packed, scale_and_zero, Np, Kp, group_size, y, N_out, ldy, norm_weight,
-                                       norm_eps, residual, ld_res, epilogue, tunables().stages, tunables().pdl != 0,
+                                       norm_eps, residual, ld_res, epilogue, tunables().stages, settled_follow(),
                                        static_cast<cudaStream_t>(stream));
       if (e != AO_B200_ERR_WORKSPACE && e != AO_B200_ERR_UNSUPPORTED) return e;
     }
   }
   return ao::int4_gemv_fused(x, M, Kx, ldx, packed, scale_and_zero, Np, Kp, group_size, y, N_out, ldy, norm_weight,
-                             norm_eps, residual, ld_res, epilogue, tunables().stages, tunables().pdl != 0,
+                             norm_eps, residual, ld_res, epilogue, tunables().stages, settled_follow(),
                              static_cast<cudaStream_t>(stream));
 }
 
@@ -229,7 +233,7 @@ extern "C" int ao_b200_int8_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
   auto xb = static_cast<const __nv_bfloat16*>(x);
   auto yb = static_cast<__nv_bfloat16*>(y);
   if (M >= 3 && M <= 8 && !ao::int8_gemv_fused_fits(M, Kp, tunables().stages)) {   // too long for one CTA: k shared out (as in ao_b200_mm_residual)
-    const int e = ao::int8_gemv_split(x, M, Kx, ldx, packed, scale, Kp, y, N_out, ldy, nullptr, 0, tunables().stages, tunables().pdl != 0, s);
+    const int e = ao::int8_gemv_split(x, M, Kx, ldx, packed, scale, Kp, y, N_out, ldy, nullptr, 0, tunables().stages, plain_follow(), s);
     if (e != AO_B200_ERR_WORKSPACE) return e;
   }
   if (int8_by_gemm(M, Np, Kp)) {
@@ -239,7 +243,7 @@ extern "C" int ao_b200_int8_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
   for (int64_t m0 = 0; m0 < M; m0 += 16) {
     const int64_t mc = (M - m0) < 16 ? (M - m0) : 16;
     int e = ao::int8_gemv_fused(xb + m0 * ldx, mc, Kx, ldx, packed, scale, Np, Kp, yb + m0 * ldy, N_out, ldy, nullptr, 0.f,
-                                nullptr, 0, 0, tunables().stages, tunables().pdl != 0, s);
+                                nullptr, 0, 0, tunables().stages, plain_follow(), s);
     if (e == AO_B200_ERR_WORKSPACE) e = ao::int8_gemv(xb + m0 * ldx, mc, Kx, ldx, packed, scale, Kp, yb + m0 * ldy, N_out, ldy, s);
     if (e) return e;
   }
@@ -257,7 +261,7 @@ extern "C" int ao_b200_int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int
   AO_CHECK_ARG(epilogue == 2 || ldy >= N_out);
   AO_CHECK_ARG(!norm_weight || ao_aligned(norm_weight, 16));
   return ao::int8_gemv_fused(x, M, Kx, ldx, packed, scale, Np, Kp, y, N_out, ldy, norm_weight, norm_eps, residual, ld_res,
-                             epilogue, tunables().stages, tunables().pdl != 0, static_cast<cudaStream_t>(stream));
+                             epilogue, tunables().stages, settled_follow(), static_cast<cudaStream_t>(stream));
 }
 
 // ---- y = bf16(residual + bf16(x W'^T)) for any number of rows, always by the GEMM ----------------------------------------
@@ -279,8 +283,8 @@ extern "C" int ao_b200_mm_residual(const void* x, int64_t M, int64_t Kx, int64_t
   const int64_t need = ao_b200_mm_residual_workspace_bytes(M, Np, Kp, group_size);
   if (M <= 8 && Kp >= 8192 && need > 0 && workspace != nullptr && workspace_bytes >= need) {
     const int e = group_size ? ao::int4_gemv_split(x, M, Kx, ldx, packed, scales, Np, Kp, group_size, y, N_out, ldy, residual, ld_res, tunables().stages,
-                                                   tunables().pdl != 0, s)
-                             : ao::int8_gemv_split(x, M, Kx, ldx, packed, scales, Kp, y, N_out, ldy, residual, ld_res, tunables().stages, tunables().pdl != 0, s);
+                                                   settled_follow(), s)
+                             : ao::int8_gemv_split(x, M, Kx, ldx, packed, scales, Kp, y, N_out, ldy, residual, ld_res, tunables().stages, settled_follow(), s);
     if (e != AO_B200_ERR_WORKSPACE) return e;
   }
   return group_size ? ao::int4_gemm_tc(x, M, Kx, ldx, packed, scales, Np, Kp, group_size, y, N_out, ldy, residual, ld_res, workspace, workspace_bytes, s)

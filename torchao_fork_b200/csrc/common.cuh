@@ -153,6 +153,9 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, u
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // PDL: let the next kernel in the stream start launching (its pre-wait prologue overlaps our tail)
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// How a GEMV follows the kernel in front of it in the stream: started behind its end; or started while it ends, with the weights read behind the wait too
+// (ordered: they may be what that kernel writes) or before it (settled: the caller answers for weights that were there before it).
+enum GemvFollow : int { kFollowPlain = 0, kFollowOrdered = 1, kFollowSettled = 2 };
 __device__ __forceinline__ void named_bar_arrive(int id, int threads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }

@@ -69,6 +69,7 @@ struct GemvFusedParams {
   const __nv_bfloat16* residual;  // [M][ld_res] or null (kEpiResidual)
   __nv_bfloat16* y;
   int M, stages, epilogue, copy_split;
+  int settled;                // weights and parameters may be read before the kernel in front is over
   int KT;                     // Kp / 64
   int64_t Kx, ldx, Np, N_out, ldy, ld_res;
   int n_strips;               // Np / 16
@@ -172,6 +173,7 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     }
     __syncwarp();
     named_bar_arrive(2, kFThreads);
+    if (!p.settled) grid_dependency_wait();
     {
       int slot = 0;
       uint32_t par = 1;
@@ -652,7 +654,7 @@ static bool plan_fused(int M, int MT, int64_t Kp, int max_stages, FusedPlan& pl,
 }
 
 template <int G, int MT, int NH, int HR>
-static int launch_fused(GemvFusedParams& p, const FusedPlan& pl, bool pdl, cudaStream_t s) {
+static int launch_fused(GemvFusedParams& p, const FusedPlan& pl, int follow, cudaStream_t s) {
   static bool attr_done = false;
   if (!attr_done) {
     if (cudaFuncSetAttribute(int4_gemv_fused_kernel<G, MT, NH, HR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
@@ -675,13 +677,13 @@ static int launch_fused(GemvFusedParams& p, const FusedPlan& pl, bool pdl, cudaS
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = follow != kFollowPlain ? 1 : 0;
   if (cudaLaunchKernelEx(&cfg, int4_gemv_fused_kernel<G, MT, NH, HR, false>, p) != cudaSuccess) return AO_B200_ERR_CUDA;
   return ao_launch_status();
 }
 
 template <int G, int MT, int NH, int HR>
-static int launch_split(GemvFusedParams& p, int M, int64_t Kp, int max_stages, bool pdl, cudaStream_t s) {
+static int launch_split(GemvFusedParams& p, int M, int64_t Kp, int max_stages, int follow, cudaStream_t s) {
   auto kern = int4_gemv_fused_kernel<G, MT, NH, HR, true>;
   static bool attr_done = false;
   if (!attr_done) {
@@ -699,7 +701,7 @@ static int launch_split(GemvFusedParams& p, int M, int64_t Kp, int max_stages, b
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 2 : 1;
+  cfg.numAttrs = follow != kFollowPlain ? 2 : 1;
   static int at_once[5] = {};
   int clusters = split_clusters(reinterpret_cast<const void*>(kern), cfg, p.ks, fused_sm_count(), at_once);
   if (clusters <= 0) return AO_B200_ERR_WORKSPACE;
@@ -721,16 +723,16 @@ static int launch_split(GemvFusedParams& p, int M, int64_t Kp, int max_stages, b
 }
 
 template <int G>
-static int launch_split_any(GemvFusedParams& p, int M, int64_t Kp, int max_stages, bool pdl, cudaStream_t s) {
+static int launch_split_any(GemvFusedParams& p, int M, int64_t Kp, int max_stages, int follow, cudaStream_t s) {
   const int n_iter = (p.KT * 8 + kFConsumers * 32 - 1) / (kFConsumers * 32);
-  if (n_iter <= 1) return launch_split<G, 1, 1, 8>(p, M, Kp, max_stages, pdl, s);
-  if (n_iter <= 2) return launch_split<G, 1, 2, 8>(p, M, Kp, max_stages, pdl, s);
+  if (n_iter <= 1) return launch_split<G, 1, 1, 8>(p, M, Kp, max_stages, follow, s);
+  if (n_iter <= 2) return launch_split<G, 1, 2, 8>(p, M, Kp, max_stages, follow, s);
   return AO_B200_ERR_WORKSPACE;
 }
 
 // The GEMV without a norm for activations too long for one CTA: k shared out over the CTAs of a cluster (AO_B200_ERR_WORKSPACE: not for this shape).
 int int4_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np, int64_t Kp, int G, void* y,
-                    int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res, int max_stages, bool pdl, cudaStream_t s) {
+                    int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res, int max_stages, int follow, cudaStream_t s) {
   if (M < 2 || M > 8) return AO_B200_ERR_WORKSPACE;
   GemvFusedParams p{};
   p.packed = static_cast<const uint8_t*>(packed);
@@ -739,6 +741,7 @@ int int4_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.y = static_cast<__nv_bfloat16*>(y);
   p.M = (int)M;
+  p.settled = follow == kFollowSettled;
   p.epilogue = residual != nullptr ? kEpiResidual : 0;
   p.copy_split = 1;
   p.Kx = Kx; p.ldx = ldx; p.Np = Np; p.N_out = N_out; p.ldy = ldy; p.ld_res = ld_res;
@@ -749,10 +752,10 @@ int int4_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
     p.KT = (int)(Kp / 64 / ks);
     int e = AO_B200_ERR_WORKSPACE;
     switch (G) {
-      case 32: e = launch_split_any<32>(p, (int)M, Kp, max_stages, pdl, s); break;
-      case 64: e = launch_split_any<64>(p, (int)M, Kp, max_stages, pdl, s); break;
-      case 128: e = launch_split_any<128>(p, (int)M, Kp, max_stages, pdl, s); break;
-      case 256: e = launch_split_any<256>(p, (int)M, Kp, max_stages, pdl, s); break;
+      case 32: e = launch_split_any<32>(p, (int)M, Kp, max_stages, follow, s); break;
+      case 64: e = launch_split_any<64>(p, (int)M, Kp, max_stages, follow, s); break;
+      case 128: e = launch_split_any<128>(p, (int)M, Kp, max_stages, follow, s); break;
+      case 256: e = launch_split_any<256>(p, (int)M, Kp, max_stages, follow, s); break;
     }
     if (e != AO_B200_ERR_WORKSPACE) return e;
   }
@@ -775,7 +778,7 @@ bool int4_gemv_fused_fits(int64_t M, int64_t Kp, int G, int max_stages) {
 // returns AO_B200_ERR_WORKSPACE when the shape does not fit this kernel (caller may fall back)
 int int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np,
                     int64_t Kp, int G, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps,
-                    const void* residual, int64_t ld_res, int epilogue, int max_stages, bool pdl, cudaStream_t s) {
+                    const void* residual, int64_t ld_res, int epilogue, int max_stages, int follow, cudaStream_t s) {
   GemvFusedParams p;
   p.packed = static_cast<const uint8_t*>(packed);
   p.sz = static_cast<const uint32_t*>(sz);
@@ -784,6 +787,7 @@ int int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.y = static_cast<__nv_bfloat16*>(y);
   p.M = (int)M;
+  p.settled = follow == kFollowSettled;
   p.epilogue = epilogue;
   p.KT = (int)(Kp / 64);
   p.Kx = Kx; p.ldx = ldx; p.Np = Np; p.N_out = N_out; p.ldy = ldy; p.ld_res = ld_res;
@@ -791,7 +795,7 @@ int int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   p.eps = eps;
   const int MT = M <= 8 ? 1 : 2;
   if (norm_w == nullptr && epilogue != kEpiSiluMul && long_activations(M, Kp) && int4_gemv_fused_fits(M, Kp, G, max_stages)) {
-    const int e = int4_gemv_split(x, M, Kx, ldx, packed, sz, Np, Kp, G, y, N_out, ldy, epilogue == kEpiResidual ? residual : nullptr, ld_res, max_stages, pdl, s);
+    const int e = int4_gemv_split(x, M, Kx, ldx, packed, sz, Np, Kp, G, y, N_out, ldy, epilogue == kEpiResidual ? residual : nullptr, ld_res, max_stages, follow, s);
     if (e != AO_B200_ERR_WORKSPACE) return e;
   }
   FusedPlan pl;
@@ -818,12 +822,12 @@ int int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   const bool alone = pl.smem > 113 * 1024;
 #define AO_LF(GG)                                                                        \
   do {                                                                                   \
-    if (MT == 2) return n_iter <= 1 ? launch_fused<GG, 2, 1, 16>(p, pl, pdl, s) : launch_fused<GG, 2, 0, 0>(p, pl, pdl, s); \
-    if (M <= 4 && n_iter <= 1) return launch_fused<GG, 1, 1, 4>(p, pl, pdl, s);          \
-    if (M <= 4 && n_iter <= 2 && alone) return launch_fused<GG, 1, 2, 4>(p, pl, pdl, s); \
-    if (n_iter <= 1 && alone) return launch_fused<GG, 1, 1, 8>(p, pl, pdl, s);           \
-    if (n_iter <= 2 && alone) return launch_fused<GG, 1, 2, 8>(p, pl, pdl, s);           \
-    return launch_fused<GG, 1, 0, 0>(p, pl, pdl, s);                                     \
+    if (MT == 2) return n_iter <= 1 ? launch_fused<GG, 2, 1, 16>(p, pl, follow, s) : launch_fused<GG, 2, 0, 0>(p, pl, follow, s); \
+    if (M <= 4 && n_iter <= 1) return launch_fused<GG, 1, 1, 4>(p, pl, follow, s);          \
+    if (M <= 4 && n_iter <= 2 && alone) return launch_fused<GG, 1, 2, 4>(p, pl, follow, s); \
+    if (n_iter <= 1 && alone) return launch_fused<GG, 1, 1, 8>(p, pl, follow, s);           \
+    if (n_iter <= 2 && alone) return launch_fused<GG, 1, 2, 8>(p, pl, follow, s);           \
+    return launch_fused<GG, 1, 0, 0>(p, pl, follow, s);                                     \
   } while (0)
   switch (G) {
     case 32: AO_LF(32);

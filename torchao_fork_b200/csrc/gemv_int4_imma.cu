@@ -45,6 +45,7 @@ struct GemvIParams {
   const __nv_bfloat16* residual;
   __nv_bfloat16* y;
   int M, stages, epilogue, hold;
+  int settled;                    // weights and parameters may be read before the kernel in front is over
   int KT;                         // Kp / 64 (Kp % max(G, 128) == 0)
   int64_t Kx, ldx, N_out, ldy, ld_res;
   int n_strips, strips_base, strips_rem;  // CTA b owns strips [b base + min(b, rem), ...)
@@ -131,6 +132,7 @@ __global__ void __launch_bounds__(kIThreads, 2) int4_gemv_imma_kernel(const Gemv
     }
     __syncwarp();
     named_bar_arrive(2, kIThreads);
+    if (!p.settled) grid_dependency_wait();
     if (lane == 0) {
       int slot = 0;
       uint32_t par = 1;
@@ -539,7 +541,7 @@ static bool plan_imma(int M, int64_t Kp, int G, int max_stages, PlanI& pl) {
 // M <= 2, G in {32, 64, 128, 256}.  Returns AO_B200_ERR_UNSUPPORTED / AO_B200_ERR_WORKSPACE when the shape is not for this kernel.
 int int4_gemv_imma(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np,
                    int64_t Kp, int G, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps,
-                   const void* residual, int64_t ld_res, int epilogue, int max_stages, bool pdl, cudaStream_t s) {
+                   const void* residual, int64_t ld_res, int epilogue, int max_stages, int follow, cudaStream_t s) {
   if (M > 2 || (G != 32 && G != 64 && G != 128 && G != 256) || Kp % (G > 128 ? G : 128) != 0) return AO_B200_ERR_UNSUPPORTED;
   (void)Np;
   GemvIParams p;
@@ -550,6 +552,7 @@ int int4_gemv_imma(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void
   p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.y = static_cast<__nv_bfloat16*>(y);
   p.M = (int)M;
+  p.settled = follow == kFollowSettled;
   p.epilogue = epilogue;
   {
     static const int hold = []() { const char* e = std::getenv("AO_B200_IMMA_HOLD"); return e ? std::atoi(e) : 1; }();
@@ -613,7 +616,7 @@ int int4_gemv_imma(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = follow != kFollowPlain ? 1 : 0;
   if (cudaLaunchKernelEx(&cfg, kern, p) != cudaSuccess) return AO_B200_ERR_CUDA;
   return ao_launch_status();
 }

@@ -59,6 +59,7 @@ struct GemvTcParams {
   const __nv_bfloat16* residual;
   __nv_bfloat16* y;
   int M, N_mma, stages, epilogue;
+  int settled;                // weights may be read before the kernel in front is over
   int KT;                     // Kp / 64
   int64_t Kx, ldx, N_out, ldy, ld_res;
   int n_blocks;               // Np / 128 (row blocks of 8 strips)
@@ -209,6 +210,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) int4_gemv_tc_kernel(const GemvT
   if (warp == kTcProducerWarp) {
     // ===================== TMA producer: per stage 8 strips x 4 KB, lanes 0..7 issue one strip each =====================
     int rb = rb_first, ch = w0;
+    if (!p.settled) grid_dependency_wait();
     for (int it = 0; it < u1 - u0; ++it) {
       const int slot = it % stages;
       const uint32_t par = ((uint32_t)(it / stages) & 1u) ^ 1u;
@@ -584,7 +586,7 @@ int64_t int4_gemv_tc_workspace_bytes(int64_t Np) {
 }
 
 template <int G, int NM>
-static int launch_tc(GemvTcParams& p, bool pdl, cudaStream_t s) {
+static int launch_tc(GemvTcParams& p, int follow, cudaStream_t s) {
   constexpr int GPS = kTcStageK / G;
   const int units = p.n_blocks * p.n_chunks;
   const int grid = units < tc_sm_count() ? units : tc_sm_count();
@@ -622,7 +624,7 @@ static int launch_tc(GemvTcParams& p, bool pdl, cudaStream_t s) {
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = follow != kFollowPlain ? 1 : 0;
   if (cudaLaunchKernelEx(&cfg, int4_gemv_tc_kernel<G, NM>, p) != cudaSuccess) return AO_B200_ERR_CUDA;
   return ao_launch_status();
 }
@@ -630,7 +632,7 @@ static int launch_tc(GemvTcParams& p, bool pdl, cudaStream_t s) {
 // returns AO_B200_ERR_WORKSPACE / AO_B200_ERR_UNSUPPORTED when the shape does not fit this kernel (caller falls back)
 int int4_gemv_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np,
                  int64_t Kp, int G, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps, const void* residual,
-                 int64_t ld_res, int epilogue, void* workspace, int64_t workspace_bytes, bool pdl, cudaStream_t s) {
+                 int64_t ld_res, int epilogue, void* workspace, int64_t workspace_bytes, int follow, cudaStream_t s) {
   if (M > 5 || Np % 128 != 0) return AO_B200_ERR_UNSUPPORTED;
   if (int4_gemv_tc_workspace_bytes(Np) == 0) return AO_B200_ERR_UNSUPPORTED;
   if (workspace == nullptr || workspace_bytes < int4_gemv_tc_workspace_bytes(Np)) return AO_B200_ERR_WORKSPACE;
@@ -642,6 +644,7 @@ int int4_gemv_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* 
   p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.y = static_cast<__nv_bfloat16*>(y);
   p.M = (int)M;
+  p.settled = follow == kFollowSettled;
   p.epilogue = epilogue;
   p.KT = (int)(Kp / 64);
   p.Kx = Kx; p.ldx = ldx; p.N_out = N_out; p.ldy = ldy; p.ld_res = ld_res;
@@ -653,7 +656,7 @@ int int4_gemv_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* 
   static const bool force16 = std::getenv("AO_B200_TC_N16") != nullptr;
   const bool n8 = M <= 2 && !force16;
   p.N_mma = n8 ? 8 : 16;
-#define AO_LT(GG) return n8 ? launch_tc<GG, 8>(p, pdl, s) : launch_tc<GG, 16>(p, pdl, s)
+#define AO_LT(GG) return n8 ? launch_tc<GG, 8>(p, follow, s) : launch_tc<GG, 16>(p, follow, s)
   switch (G) {
     case 32: AO_LT(32);
     case 64: AO_LT(64);

@@ -40,6 +40,7 @@ struct Gemv8Params {
   const __nv_bfloat16* residual;  // [M][ld_res] or null
   __nv_bfloat16* y;
   int M, stages, epilogue;
+  int settled;                    // weights may be read before the kernel in front is over
   int KT;                         // Kp / 64
   int64_t Kx, ldx, N_out, ldy, ld_res;
   int n_strips, strips_base, strips_rem;
@@ -126,6 +127,7 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     }
     __syncwarp();
     named_bar_arrive(2, k8Threads);
+    if (!p.settled) grid_dependency_wait();
     if (lane == 0) {
       int slot = 0;
       uint32_t par = 1;
@@ -546,7 +548,7 @@ static int sm_count8() {
 }
 
 template <int MT, int NH, int HR>
-static int launch8(Gemv8Params& p, const Plan8& pl, bool pdl, cudaStream_t s) {
+static int launch8(Gemv8Params& p, const Plan8& pl, int follow, cudaStream_t s) {
   static bool attr_done = false;
   if (!attr_done) {
     if (cudaFuncSetAttribute(int8_gemv_fused_kernel<MT, NH, HR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
@@ -573,13 +575,13 @@ static int launch8(Gemv8Params& p, const Plan8& pl, bool pdl, cudaStream_t s) {
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = follow != kFollowPlain ? 1 : 0;
   if (cudaLaunchKernelEx(&cfg, int8_gemv_fused_kernel<MT, NH, HR, false>, p) != cudaSuccess) return AO_B200_ERR_CUDA;
   return ao_launch_status();
 }
 
 template <int MT, int NH, int HR>
-static int launch8_split(Gemv8Params& p, int M, int64_t Kp, int max_stages, bool pdl, cudaStream_t s) {
+static int launch8_split(Gemv8Params& p, int M, int64_t Kp, int max_stages, int follow, cudaStream_t s) {
   auto kern = int8_gemv_fused_kernel<MT, NH, HR, true>;
   static bool attr_done = false;
   if (!attr_done) {
@@ -597,7 +599,7 @@ static int launch8_split(Gemv8Params& p, int M, int64_t Kp, int max_stages, bool
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 2 : 1;
+  cfg.numAttrs = follow != kFollowPlain ? 2 : 1;
   static int at_once[5] = {};
   int clusters = split_clusters(reinterpret_cast<const void*>(kern), cfg, p.ks, sm_count8(), at_once);
   if (clusters <= 0) return AO_B200_ERR_WORKSPACE;
@@ -625,12 +627,12 @@ bool int8_gemv_fused_fits(int64_t M, int64_t Kp, int max_stages) {
 }
 
 int int8_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Kp, void* y, int64_t N_out,
-                    int64_t ldy, const void* residual, int64_t ld_res, int max_stages, bool pdl, cudaStream_t s);
+                    int64_t ldy, const void* residual, int64_t ld_res, int max_stages, int follow, cudaStream_t s);
 
 // returns AO_B200_ERR_WORKSPACE when the activations do not fit the staging (caller falls back)
 int int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Np,
                     int64_t Kp, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps, const void* residual,
-                    int64_t ld_res, int epilogue, int max_stages, bool pdl, cudaStream_t s) {
+                    int64_t ld_res, int epilogue, int max_stages, int follow, cudaStream_t s) {
   Gemv8Params p;
   p.packed = static_cast<const uint8_t*>(packed);
   p.scale = static_cast<const __nv_bfloat16*>(scale);
@@ -639,6 +641,7 @@ int int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.y = static_cast<__nv_bfloat16*>(y);
   p.M = (int)M;
+  p.settled = follow == kFollowSettled;
   p.epilogue = epilogue;
   p.KT = (int)(Kp / 64);
   p.Kx = Kx; p.ldx = ldx; p.N_out = N_out; p.ldy = ldy; p.ld_res = ld_res;
@@ -655,26 +658,26 @@ int int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   // Rows in registers: chunks of 8 activations per consumer thread and row.  M = 1: <= 4 (Kp <= 16384).  More rows: up to 16 chunks in all,
   // which leaves registers for one CTA per SM only from 8 on, so where two fit the shared memory (short rows) at most 4.
   if (norm_w == nullptr && epilogue != k8EpiSiluMul && long_activations(M, Kp)) {
-    const int e = int8_gemv_split(x, M, Kx, ldx, packed, scale, Kp, y, N_out, ldy, epilogue == k8EpiResidual ? residual : nullptr, ld_res, max_stages, pdl, s);
+    const int e = int8_gemv_split(x, M, Kx, ldx, packed, scale, Kp, y, N_out, ldy, epilogue == k8EpiResidual ? residual : nullptr, ld_res, max_stages, follow, s);
     if (e != AO_B200_ERR_WORKSPACE) return e;
   }
   const int n_iter = (p.KT * 8 + k8Consumers * 32 - 1) / (k8Consumers * 32);
-  if (MT == 2) return n_iter <= 1 ? launch8<2, 1, 16>(p, pl, pdl, s) : launch8<2, 0, 0>(p, pl, pdl, s);
-  if (M == 1 && n_iter <= 1) return launch8<1, 1, 1>(p, pl, pdl, s);
-  if (M == 1 && n_iter <= 2) return launch8<1, 2, 1>(p, pl, pdl, s);
-  if (M == 1 && n_iter <= 4) return launch8<1, 4, 1>(p, pl, pdl, s);
+  if (MT == 2) return n_iter <= 1 ? launch8<2, 1, 16>(p, pl, follow, s) : launch8<2, 0, 0>(p, pl, follow, s);
+  if (M == 1 && n_iter <= 1) return launch8<1, 1, 1>(p, pl, follow, s);
+  if (M == 1 && n_iter <= 2) return launch8<1, 2, 1>(p, pl, follow, s);
+  if (M == 1 && n_iter <= 4) return launch8<1, 4, 1>(p, pl, follow, s);
   const bool alone = pl.smem > 113 * 1024;
-  if (M <= 4 && n_iter <= 1) return launch8<1, 1, 4>(p, pl, pdl, s);
-  if (M <= 4 && n_iter <= 2 && alone) return launch8<1, 2, 4>(p, pl, pdl, s);
-  if (M <= 4 && n_iter <= 4 && alone) return launch8<1, 4, 4>(p, pl, pdl, s);
-  if (n_iter <= 1 && alone) return launch8<1, 1, 8>(p, pl, pdl, s);
-  if (n_iter <= 2 && alone) return launch8<1, 2, 8>(p, pl, pdl, s);
-  return launch8<1, 0, 0>(p, pl, pdl, s);
+  if (M <= 4 && n_iter <= 1) return launch8<1, 1, 4>(p, pl, follow, s);
+  if (M <= 4 && n_iter <= 2 && alone) return launch8<1, 2, 4>(p, pl, follow, s);
+  if (M <= 4 && n_iter <= 4 && alone) return launch8<1, 4, 4>(p, pl, follow, s);
+  if (n_iter <= 1 && alone) return launch8<1, 1, 8>(p, pl, follow, s);
+  if (n_iter <= 2 && alone) return launch8<1, 2, 8>(p, pl, follow, s);
+  return launch8<1, 0, 0>(p, pl, follow, s);
 }
 
 // The same without a norm for activations too long for one CTA: k shared out over the CTAs of a cluster (AO_B200_ERR_WORKSPACE: not for this shape).
 int int8_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Kp, void* y, int64_t N_out,
-                    int64_t ldy, const void* residual, int64_t ld_res, int max_stages, bool pdl, cudaStream_t s) {
+                    int64_t ldy, const void* residual, int64_t ld_res, int max_stages, int follow, cudaStream_t s) {
   if (M < 2 || M > 8) return AO_B200_ERR_WORKSPACE;
   const int64_t kt = Kp / 64;
   Gemv8Params p{};
@@ -684,6 +687,7 @@ int int8_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.y = static_cast<__nv_bfloat16*>(y);
   p.M = (int)M;
+  p.settled = follow == kFollowSettled;
   p.epilogue = residual != nullptr ? k8EpiResidual : k8EpiPlain;
   p.Kx = Kx; p.ldx = ldx; p.N_out = N_out; p.ldy = ldy; p.ld_res = ld_res;
   p.n_strips = (int)((N_out + 15) / 16);
@@ -692,8 +696,8 @@ int int8_gemv_split(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
     p.ks = ks;
     p.KT = (int)(kt / ks);
     const int n_iter = (p.KT * 8 + k8Consumers * 32 - 1) / (k8Consumers * 32);
-    const int e = n_iter <= 1 ? launch8_split<1, 1, 8>(p, (int)M, Kp, max_stages, pdl, s)
-                              : (n_iter <= 2 ? launch8_split<1, 2, 8>(p, (int)M, Kp, max_stages, pdl, s) : AO_B200_ERR_WORKSPACE);
+    const int e = n_iter <= 1 ? launch8_split<1, 1, 8>(p, (int)M, Kp, max_stages, follow, s)
+                              : (n_iter <= 2 ? launch8_split<1, 2, 8>(p, (int)M, Kp, max_stages, follow, s) : AO_B200_ERR_WORKSPACE);
     if (e != AO_B200_ERR_WORKSPACE) return e;
   }
   return AO_B200_ERR_WORKSPACE;
