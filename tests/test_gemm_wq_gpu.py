@@ -245,3 +245,65 @@ def test_more_than_four_million_rows():
     for rows in (slice(0, 700), slice(1 << 21, (1 << 21) + 300), slice(m - 513, m)):
         ref = x[rows].double() @ (q.double() * scale.double()[:, None]).t()
         assert ((y[rows].double() - ref).norm() / ref.norm()).item() < 2.0 ** -8
+
+
+@pytest.mark.parametrize("bits,group", [(4, 32), (4, 128), (4, 256), (8, 0)])
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("m,k", [(3, 28672), (8, 28672), (5, 14336), (8, 14336), (8, 8192)])
+def test_long_few_rows_with_infinities_huge_and_tiny_values(bits, group, residual, m, k):
+    # calls whose k the CTAs of a cluster share: finite results wherever bf16 products with 32-bit sums have them, infinities with the sign of
+    # their weight, tiny rows as exact as others
+    from torchao_fork_b200 import _lib
+    # the sums have to stay below 3.4e38: 296 terms of 0.02 big have a norm of 0.34 big, of up to 127 big 740 big
+    n, big = 640, 1e38 if bits == 4 else 1e35
+    gen = torch.Generator(device="cuda").manual_seed(m + k + group)
+    w = (0.02 * torch.randn(n, k, generator=gen, device="cuda")).to(torch.bfloat16)
+    x = torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16)
+    if bits == 4:
+        packed, scales = T.b200_int4_quantize_pack(w, group, 1e-6, True)
+        p = scales.permute(0, 2, 1, 3).reshape(packed.shape[0] * 16, -1, 2)[:n, : k // group].double()
+        wd = ((T.b200_int4_unpack(packed)[:n, :k].double().reshape(n, -1, group) - 8) * p[..., 0:1] + p[..., 1:2]).reshape(n, k)
+        wb = wd.to(torch.bfloat16).double()
+    else:
+        q, scales = T.b200_int8_quantize(w, 1e-6, True)
+        packed, wb, wd = T.b200_int8_pack(q), q.double(), q.double() * scales.double()[:, None]
+    # the rows, up to eight of them: an infinity, huge values, tiny ones, two infinities, a NaN, a block of huge ones, a single one, an infinity and a huge value
+    x[0, 77] = torch.inf
+    x[1, ::97] = big
+    x[2] = (x[2].float() * 1e-36).to(torch.bfloat16)
+    signs = {0: [(77, 1)]}
+    if m > 3:
+        x[3, k // 2 - 1], x[3, k - 1] = -torch.inf, torch.inf
+        x[4, 5] = torch.nan
+        signs[3] = [(k // 2 - 1, -1), (k - 1, 1)]
+    if m > 5:
+        x[5, 1024:1152] = -big / 16
+        x[6, k - 8] = big
+        x[7, 130], x[7, k - 130] = torch.inf, big
+        signs[7] = [(130, 1)]
+    if residual:
+        res, L = torch.zeros(m, n, dtype=torch.bfloat16, device="cuda"), _lib.lib()
+        np_, kp = packed.shape[0] * 16, packed.shape[1] * 64
+        ws = torch.empty(L.ao_b200_mm_residual_workspace_bytes(m, np_, kp, group), dtype=torch.uint8, device="cuda")
+        y = torch.empty_like(res)
+        _lib.check(L.ao_b200_mm_residual(x.data_ptr(), m, k, k, packed.data_ptr(), scales.data_ptr(), np_, kp, group, y.data_ptr(), n, n, res.data_ptr(), n,
+                                         ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream), "mm_residual")
+    elif bits == 4:
+        y = T.b200_int4_weight_only_mm(x, packed, group, scales, n)
+    else:
+        y = T.b200_int8_weight_only_mm(x, packed, scales)
+    for row in range(m):
+        got = y[row].double()
+        if row in signs:
+            s = [sg * wb[:, j].sign() for j, sg in signs[row]]
+            want = torch.where((s[0] != 0) & (s[-1] == s[0]), s[0] * torch.inf, torch.full_like(s[0], torch.nan))
+            assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(nan=0.0), want.nan_to_num(nan=0.0)), row
+        elif row == 4:
+            assert got.isnan().all()
+        else:
+            # the weights of a row of huge values may be met as they are in bf16: 2^-9 sqrt(1 / 3) of each, and the result's rounding(s); equal values
+            # over a block add up roundings in step (2.8 times that, against either reference, half of it against their mean)
+            xd = x[row].double()
+            ref = xd @ wd.t()
+            near = min(((got - r).norm() / ref.norm()).item() for r in (ref, xd @ wb.t() if bits == 4 else ref))
+            assert got.isfinite().all() and near < 2.0 ** -8, (row, near)

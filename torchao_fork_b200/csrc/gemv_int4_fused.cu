@@ -119,6 +119,24 @@ __device__ __forceinline__ float warp_max_f(float v) {
   return v;
 }
 
+// The split kernel's sums that are not finite (split_again), with the weights rounded to bf16 as the GEMM and the strip kernel meet them; w, sz: the strip's
+template <int G>
+__device__ __noinline__ float4 again4(const uint8_t* w, const uint32_t* sz, const __nv_bfloat16* x, int64_t ldx, int64_t Kx, int M, float4 sum, int lane) {
+  return split_again(sum, M, Kx, lane, [&](int row, int m, int64_t k) {
+    float f[8];
+    unpack8(*reinterpret_cast<const uint4*>(x + m * ldx + k), f);
+    // word j of a lane's 16 bytes: row g + 8 (j & 1) of the tile's 32-k half j >> 1
+    const uint32_t par = __ldg(sz + (k / G) * 16 + row);
+    uint32_t o[4];
+    dequant_word(__ldg(reinterpret_cast<const uint32_t*>(w + (k >> 6) * 512 + (4 * (row & 7) + ((k >> 3) & 3)) * 16) + 2 * ((k >> 5) & 1) + (row >> 3)),
+                 __byte_perm(par, 0, 0x1010), __byte_perm(par, 0, 0x3232), o);
+    double t = 0.0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) t += (double)f[e] * (double)__uint_as_float(e & 1 ? o[e >> 1] & 0xFFFF0000u : o[e >> 1] << 16);
+    return t;
+  });
+}
+
 // HR = 4, 8, 16: up to HR rows of <= NH 8-element chunks per thread staged from registers (gemv_stage.cuh); HR = 0: staging in loops
 // SPLIT: k shared out over the CTAs of a cluster (gemv_stage.cuh)
 template <int G, int MT, int NH, int HR, bool SPLIT>
@@ -251,8 +269,11 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&red_free[rbuf]);
-      if constexpr (SPLIT)
+      if constexpr (SPLIT) {
         if (!split_sums<MT>(sum, row_scale, in_full, inbox, li, rank, ks, lane)) continue;
+        if (split_overflowed(sum[0], p.M, lane))
+          sum[0] = again4<G>(p.packed + (int64_t)strip * ks * KT * 512, p.sz + (int64_t)strip * ks * (KT * 64 / G) * 16, p.x, p.ldx, p.Kx, p.M, sum[0], lane);
+      }
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         const float vals[2][2] = {{sum[mt].x, sum[mt].z}, {sum[mt].y, sum[mt].w}};  // [col j][row half]: rows g, g+8

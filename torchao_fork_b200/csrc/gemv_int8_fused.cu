@@ -72,6 +72,21 @@ __device__ __forceinline__ void mma8_f16_16816(float (&d)[4], uint32_t a0, uint3
 __device__ __forceinline__ uint32_t u8_f16_lo(uint32_t w) { return __byte_perm(w, 0x64646464u, 0x4140); }
 __device__ __forceinline__ uint32_t u8_f16_hi(uint32_t w) { return __byte_perm(w, 0x64646464u, 0x4342); }
 
+// The split kernel's sums that are not finite (split_again); w: the strip's weights
+__device__ __noinline__ float4 again8(const uint8_t* w, const __nv_bfloat16* x, int64_t ldx, int64_t Kx, int M, float4 sum, int lane) {
+  return split_again(sum, M, Kx, lane, [&](int row, int m, int64_t k) {
+    float f[8];
+    unpack8(*reinterpret_cast<const uint4*>(x + m * ldx + k), f);
+    // word j of a lane's 16 bytes: row g + 8 (j & 1), four k from 4 (j >> 1) on
+    const uint32_t* at = reinterpret_cast<const uint32_t*>(w + (k >> 5) * 512 + (4 * (row & 7) + ((k >> 3) & 3)) * 16) + (row >> 3);
+    const uint32_t u[2] = {__ldg(at), __ldg(at + 2)};
+    double t = 0.0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) t += (double)f[e] * (double)((int)((u[e >> 2] >> (8 * (e & 3))) & 0xFF) - 128);
+    return t;
+  });
+}
+
 // HR = 1: M = 1 and every consumer thread owns <= NH chunks of the activation row (register-held staging); HR = 4, 8, 16: up to
 // HR rows of <= NH chunks in registers (gemv_stage.cuh); HR = 0: the general staging.  One instantiation per case — the staging code runs once per launch with a cold instruction cache, so
 // code that a launch does not need is not compiled into its kernel (profiles/r01c_imma_code_size_ab.txt).
@@ -194,8 +209,11 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&red_free[rbuf]);
-      if constexpr (SPLIT)
+      if constexpr (SPLIT) {
         if (!split_sums<MT>(sum, row_scale, in_full, inbox, li, rank, ks, lane)) continue;
+        if (split_overflowed(sum[0], p.M, lane))
+          sum[0] = again8(p.packed + (int64_t)strip * ks * KT * 1024, p.x, p.ldx, p.Kx, p.M, sum[0], lane);
+      }
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         const float vals[2][2] = {{sum[mt].x, sum[mt].z}, {sum[mt].y, sum[mt].w}};  // [col j][row half]

@@ -105,10 +105,9 @@ __device__ __forceinline__ void stage_rows(const __nv_bfloat16* x, int64_t ldx, 
   }
   fold_rows<R / 2, 8>(t, lane, add);
   fold_rows<R / 2, 8>(a, lane, larger);
-  // 2^e brings the row's largest magnitude to [2^13, 2^14)
+  // 2^e brings the row's largest magnitude to [2^13, 2^14); below 2^-113 to less, as 2^-e has to be a number, which leaves every bf16 exact all the same
   int e = 0;
-  if (a[0] > 0.f) e = (int)((__float_as_uint(a[0]) >> 23) & 0xFF) - 127 - 13;
-  e = max(-100, min(100, e));
+  if (a[0] > 0.f) e = max(-126, (int)((__float_as_uint(a[0]) >> 23) & 0xFF) - 127 - 13);
   const float up = __uint_as_float((uint32_t)(e + 127) << 23), own_dn = __uint_as_float((uint32_t)(127 - e) << 23);
   if (warp == 0 && lane % kOwn == 0)   // for the epilogue warp
     row_scale[row0 + lane / kOwn] = norm_w != nullptr ? up * rsqrtf(t[0] / (float)Kx + eps) : up;
@@ -203,6 +202,42 @@ __device__ __forceinline__ bool split_sums(float4 (&sum)[MT], const float* row_s
     if (!here) sum[mt] = make_float4(__int_as_float(0x7FFFFFFF), __int_as_float(0x7FFFFFFF), __int_as_float(0x7FFFFFFF), __int_as_float(0x7FFFFFFF));
   }
   return true;
+}
+// The sums of a strip (lane (g, c): rows g and g + 8, x and y, z and w; columns 2 c, 2 c + 1 of the M) that are not finite, done again by the whole warp:
+// an infinity has lost its sign against the weights' offset, or one rank's part has overflowed where the total does not.  dot(row, m, k) adds eight
+// products; sums in 64 bits, rounded to 32 once.  Rare, and slow.
+template <typename Dot>
+__device__ __forceinline__ float4 split_again(float4 sum, int M, int64_t Kx, int lane, Dot&& dot) {
+  float v[4] = {sum.x, sum.y, sum.z, sum.w};
+#pragma unroll 1
+  for (int i = 0; i < 4; ++i) {
+    const float own = i == 0 ? v[0] : i == 1 ? v[1] : i == 2 ? v[2] : v[3];
+    uint32_t bad = __ballot_sync(0xffffffffu, 2 * (lane & 3) + (i & 1) < M && !(fabsf(own) < INFINITY));
+    float redone = own;
+#pragma unroll 1
+    for (; bad != 0; bad &= bad - 1) {
+      const int src = __ffs(bad) - 1, row = (src >> 2) + 8 * (i >> 1), m = 2 * (src & 3) + (i & 1);
+      double t = 0.0;
+#pragma unroll 1
+      for (int64_t k = 8 * lane; k - 8 * lane < Kx; k += 256) {
+        if (k < Kx) t += dot(row, m, k);
+        if (__any_sync(0xffffffffu, t != t)) break;   // NaN stays NaN
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == src) redone = (float)t;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j == i) v[j] = redone;
+  }
+  return make_float4(v[0], v[1], v[2], v[3]);
+}
+// whether any of the sums that count is not finite, on any lane
+__device__ __forceinline__ bool split_overflowed(const float4& s, int M, int lane) {
+  const int m = 2 * (lane & 3);
+  const bool low = fabsf(s.x) < INFINITY && fabsf(s.z) < INFINITY, high = fabsf(s.y) < INFINITY && fabsf(s.w) < INFINITY;
+  return __any_sync(0xffffffffu, (m < M && !low) || (m + 1 < M && !high));
 }
 // Clusters of ks CTAs, one per SM, that run at the same time: the SMs of a GPC need not be a multiple of ks.  The same for every shape, so asked
 // for once per kernel and ks.
