@@ -52,8 +52,8 @@ def build(verbose=False, force=False, target="core"):
 def _build_locked(verbose, force, target):
     src_dir, lib_path = TARGETS[target]
     headers = [os.path.join(src_dir, f) for f in os.listdir(src_dir) if f.endswith((".cuh", ".h"))]
-    inc = os.path.join(HERE, "..", "include")
-    headers += [os.path.join(inc, f) for f in os.listdir(inc) if f.endswith(".h")]
+    for shared in (os.path.join(HERE, "..", "include"), CSRC):   # the C headers, and those that both targets include
+        headers += [os.path.join(shared, f) for f in os.listdir(shared) if f.endswith(".h")]
     jobs = []
     objs = []
     for src in sources(target):

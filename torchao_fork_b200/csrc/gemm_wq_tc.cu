@@ -46,6 +46,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "per_device.h"
 
 namespace ao {
 
@@ -936,12 +937,9 @@ static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
   constexpr bool kCan = !DEFER;
   const bool early = kCan && (int64_t)w.base * w.quantum >= w.KU;
   auto kern = wq_gemm_kernel<G, DEFER, PAIR, false>;
-  static bool attr_done[2] = {};
+  static OncePerDevice once[2];
   if (early) kern = wq_gemm_kernel<G, DEFER, PAIR, kCan>;
-  if (!attr_done[early]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBudget) != cudaSuccess) return AO_B200_ERR_CUDA;
-    attr_done[early] = true;
-  }
+  if (!dynamic_smem(once[early], kern, (int)kBudget)) return AO_B200_ERR_CUDA;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(w.workers * w.ranks));
   cfg.blockDim = dim3(kWqThreads);

@@ -676,13 +676,8 @@ static bool plan_fused(int M, int MT, int64_t Kp, int max_stages, FusedPlan& pl,
 
 template <int G, int MT, int NH, int HR>
 static int launch_fused(GemvFusedParams& p, const FusedPlan& pl, int follow, cudaStream_t s) {
-  static bool attr_done = false;
-  if (!attr_done) {
-    if (cudaFuncSetAttribute(int4_gemv_fused_kernel<G, MT, NH, HR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
-        cudaSuccess)
-      return AO_B200_ERR_CUDA;
-    attr_done = true;
-  }
+  static OncePerDevice once;
+  if (!dynamic_smem(once, int4_gemv_fused_kernel<G, MT, NH, HR, false>, 227 * 1024)) return AO_B200_ERR_CUDA;
   // AO_B200_CTAS: co-resident CTAs per SM of ONE launch (the 113 KB plan leaves room for two)
   static const int ctas_per_sm = []() { const char* e = std::getenv("AO_B200_CTAS"); int v = e ? std::atoi(e) : 2; return v < 1 ? 1 : v; }();
   const int max_grid = fused_sm_count() * (pl.smem <= 113 * 1024 && MT == 1 ? ctas_per_sm : 1);
@@ -706,11 +701,8 @@ static int launch_fused(GemvFusedParams& p, const FusedPlan& pl, int follow, cud
 template <int G, int MT, int NH, int HR>
 static int launch_split(GemvFusedParams& p, int M, int64_t Kp, int max_stages, int follow, cudaStream_t s) {
   auto kern = int4_gemv_fused_kernel<G, MT, NH, HR, true>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return AO_B200_ERR_CUDA;
-    attr_done = true;
-  }
+  static OncePerDevice once;
+  if (!dynamic_smem(once, kern, 227 * 1024)) return AO_B200_ERR_CUDA;
   cudaLaunchConfig_t cfg{};
   cfg.blockDim = dim3(kFThreads);
   cfg.stream = s;
@@ -723,7 +715,7 @@ static int launch_split(GemvFusedParams& p, int M, int64_t Kp, int max_stages, i
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = follow != kFollowPlain ? 2 : 1;
-  static int at_once[5] = {};
+  static NumberPerDevice at_once[5];
   int clusters = split_clusters(reinterpret_cast<const void*>(kern), cfg, p.ks, fused_sm_count(), at_once);
   if (clusters <= 0) return AO_B200_ERR_WORKSPACE;
   if (clusters > p.n_strips) clusters = p.n_strips;

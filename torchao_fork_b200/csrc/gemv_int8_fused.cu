@@ -567,12 +567,8 @@ static int sm_count8() {
 
 template <int MT, int NH, int HR>
 static int launch8(Gemv8Params& p, const Plan8& pl, int follow, cudaStream_t s) {
-  static bool attr_done = false;
-  if (!attr_done) {
-    if (cudaFuncSetAttribute(int8_gemv_fused_kernel<MT, NH, HR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
-      return AO_B200_ERR_CUDA;
-    attr_done = true;
-  }
+  static OncePerDevice once;
+  if (!dynamic_smem(once, int8_gemv_fused_kernel<MT, NH, HR, false>, 227 * 1024)) return AO_B200_ERR_CUDA;
   const int max_grid = sm_count8() * (pl.smem <= 113 * 1024 && MT == 1 ? 2 : 1);
   // balanced waves: every CTA gets the same number of strips (+-1 at most on the last few), e.g. 1792 strips on 296 slots
   // -> 256 CTAs x 7 instead of 16 CTAs with a 7th strip while 280 idle
@@ -601,11 +597,8 @@ static int launch8(Gemv8Params& p, const Plan8& pl, int follow, cudaStream_t s) 
 template <int MT, int NH, int HR>
 static int launch8_split(Gemv8Params& p, int M, int64_t Kp, int max_stages, int follow, cudaStream_t s) {
   auto kern = int8_gemv_fused_kernel<MT, NH, HR, true>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return AO_B200_ERR_CUDA;
-    attr_done = true;
-  }
+  static OncePerDevice once;
+  if (!dynamic_smem(once, kern, 227 * 1024)) return AO_B200_ERR_CUDA;
   cudaLaunchConfig_t cfg{};
   cfg.blockDim = dim3(k8Threads);
   cfg.stream = s;
@@ -618,7 +611,7 @@ static int launch8_split(Gemv8Params& p, int M, int64_t Kp, int max_stages, int 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = follow != kFollowPlain ? 2 : 1;
-  static int at_once[5] = {};
+  static NumberPerDevice at_once[5];
   int clusters = split_clusters(reinterpret_cast<const void*>(kern), cfg, p.ks, sm_count8(), at_once);
   if (clusters <= 0) return AO_B200_ERR_WORKSPACE;
   if (clusters > p.n_strips) clusters = p.n_strips;

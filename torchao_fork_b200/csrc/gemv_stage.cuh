@@ -12,6 +12,7 @@
 #include <cuda_fp16.h>
 
 #include "common.cuh"
+#include "per_device.h"
 
 namespace ao {
 
@@ -240,17 +241,18 @@ __device__ __forceinline__ bool split_overflowed(const float4& s, int M, int lan
   return __any_sync(0xffffffffu, (m < M && !low) || (m + 1 < M && !high));
 }
 // Clusters of ks CTAs, one per SM, that run at the same time: the SMs of a GPC need not be a multiple of ks.  The same for every shape, so asked
-// for once per kernel and ks.
-static inline int split_clusters(const void* kern, cudaLaunchConfig_t cfg, int ks, int sms, int (&at_once)[5]) {
-  if (at_once[ks] == 0) {
+// for once per kernel, ks and device.  (0 or less: none.)
+static inline int split_clusters(const void* kern, cudaLaunchConfig_t cfg, int ks, int sms, NumberPerDevice (&at_once)[5]) {
+  int device = -1;
+  cudaGetDevice(&device);
+  return at_once[ks].get(device, [&] {
     cfg.gridDim = dim3((unsigned)(sms / ks * ks));
     cfg.dynamicSmemBytes = 200 * 1024;
     cfg.numAttrs = 1;   // the cluster dimension
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) cudaGetLastError(), n = 0;
-    at_once[ks] = n > 0 ? n : -1;
-  }
-  return at_once[ks];
+    return n > 0 ? n : -1;
+  });
 }
 
 }  // namespace ao

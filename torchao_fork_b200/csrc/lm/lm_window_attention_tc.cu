@@ -25,6 +25,7 @@
 // 128), two chains per SM beside one another; a CTA's start and end (queries, the peers' shares) cost 9000 more.  2048 rows x 16 heads of 128
 // (four key heads): 59.5 us, against 308 us of window_attention_prompt_kernel; the same with all keys of a tile in one CTA 110 us (the last
 // tiles alone took 95), with unswizzled operands 84 us.
+#include "../per_device.h"
 #include "lm_mma.cuh"
 #include "lm_window_attention.cuh"
 
@@ -503,11 +504,8 @@ int launch(const WinPromptArgs& a, int dv, int n_tiles, cudaStream_t st) {
   size_t smem = kTcHeader + (held > shares ? held : shares) + (NM == 2 ? (size_t)(kTcRows / C) * dv * 4 : 0);
   if (smem < kTcMinSmem) smem = kTcMinSmem;
   auto kern = window_attention_tc_kernel<NM, C>;
-  static bool set = false;   // per instantiation
-  if (!set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 113 * 1024) != cudaSuccess) return AO_B200_ERR_CUDA;
-    set = true;
-  }
+  static ao::OncePerDevice once;   // per instantiation
+  if (!ao::dynamic_smem(once, kern, 113 * 1024)) return AO_B200_ERR_CUDA;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(n_tiles * C), (unsigned)a.H);
   cfg.blockDim = dim3(kTcThreads);
