@@ -111,3 +111,35 @@ def test_keys_of_a_tile_shared_out_over_one_to_eight_ctas(maps, d, dv, H, G, n, 
         ref = _reference(q * scale, k, v, 0, 4096, 0, 0.4)
         assert ((out[:, : H * dv].double() - ref).norm() / ref.norm()).item() < 0.01
         assert extra == 0 or bool((out[:, -1] == 9.0).all())
+
+
+@pytest.mark.parametrize("maps,d,dv,H,G", [(1, 128, 128, 4, 2), (2, 64, 128, 2, 2), (1, 16, 80, 40, 2)])
+@pytest.mark.parametrize("n,past,window,keep", [(300, 0, 4096, 0), (520, 40, 100, 3), (700, 0, 512, 0)])
+def test_values_that_are_not_finite_reach_only_rows_that_see_them(maps, d, dv, H, G, n, past, window, keep):
+    """An infinity or NaN among the values of a key makes the results of the rows that see it, in its column, not finite (with two maps their norm
+    spreads it over the row) and no others: a hidden key has no part in a row, whatever the tile that both are in.  Bound as above."""
+    gen = torch.Generator(device="cuda").manual_seed(n + d)
+    q = torch.randn(n, H, maps, d, generator=gen, device="cuda") * 1.5
+    k, v = (torch.randn(past + n, G, *w, generator=gen, device="cuda").to(torch.bfloat16) for w in ((maps, d), (dv,)))
+    ref = _reference(q, k, v, past, window, keep, 0.4).view(n, H, dv)
+    i, j = torch.arange(past, past + n, device="cuda")[:, None], torch.arange(past + n, device="cuda")[None, :]
+    seen = ~((j > i) | ((i - j >= window) & (j >= keep)))
+    for at, g, c, value in ((past + n - 1, 0, 3, torch.inf), (past + n - 37, G - 1, dv - 1, torch.nan), (past + 130, 0, 17, -torch.inf), (past + 130, 0, 18, torch.inf),
+                            (past + 63, 0, 0, torch.nan), (past + 64, G - 1, 9, -torch.inf), (past + 1, 0, 40, torch.inf), (1, 0, 41, torch.inf)):
+        v[at, g, c] = value
+    bad = torch.einsum("ij,jgc->igc", seen.double(), (~v.isfinite()).double()) > 0     # [n][G][dv]
+    bad = bad.repeat_interleave(H // G, 1)
+    if maps == 2:
+        bad = bad.any(-1, keepdim=True).expand(n, H, dv)
+    assert bad.any() and not bad.all(-1).all()
+    got = _run(q, k, v, past, window, keep, 0.4).double().view(n, H, dv)
+    spread = got.isfinite() & bad      # (a norm over an infinity makes the row's other columns zero, not NaN)
+    assert not spread.any() if maps == 1 else bool((got[spread] == 0).all())
+    assert got[~bad].isfinite().all()
+    if maps == 1:                      # (a value set to something finite would have been part of the others' norm)
+        # columns are independent of one another: those without a bad value are what they were
+        err = torch.where(bad, 0.0, got.nan_to_num() - ref)
+        assert (err.norm() / ref.norm()).item() < 0.01
+    else:
+        rows = ~bad.any(-1)
+        assert ((got[rows] - ref[rows]).norm() / ref[rows].norm()).item() < 0.01

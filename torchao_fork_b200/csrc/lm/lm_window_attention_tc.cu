@@ -97,6 +97,7 @@ __device__ __forceinline__ float4 tc_peer_f32x4(uint32_t addr) {
   asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
   return v;
 }
+__device__ __forceinline__ void tc_peer_set(uint32_t addr) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(1) : "memory"); }
 __device__ __forceinline__ void tc_cp16(uint32_t smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
 }
@@ -160,14 +161,82 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t addr, uint32_t lead) {
 // where 16-byte piece c of row r lies in a tile of `rows` rows
 __device__ __forceinline__ uint32_t tc_at(int r, int c, int rows) { return (c >> 3) * (rows * 128) + r * 128 + (((c ^ r) & 7) << 4); }
 
-template <int NM, int C>
-__global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(WinPromptArgs a, int dv) {
+// the row of key kk: the kept positions, then those from lo on, of which the step brings p0 and later ones (its rows from seg_row0 on)
+__device__ __forceinline__ const __nv_bfloat16* win_row(const WinPromptArgs& a, int kk, int nf, int lo, int p0, int64_t seg_row0, int64_t slot, int g, int width,
+                                                        const __nv_bfloat16* step, const __nv_bfloat16* kept, const __nv_bfloat16* ring) {
+  const int j = kk < nf ? kk : lo + (kk - nf);
+  return j >= p0 ? step + ((seg_row0 + (j - p0)) * a.G + g) * width
+                 : (j < a.first_rows ? kept + ((slot * a.first_rows + j) * a.G + g) * width : ring + ((slot * a.ring + j % a.ring) * a.G + g) * width);
+}
+// two bf16, each zero where it is an infinity or NaN
+__device__ __forceinline__ uint32_t finite_or_zero(uint32_t v) {
+  if ((v & 0x7F80u) == 0x7F80u) v &= 0xFFFF0000u;
+  if ((v & 0x7F800000u) == 0x7F800000u) v &= 0xFFFFu;
+  return v;
+}
+// Values that are not finite, of a step in which some rows do not see all keys: a hidden key's weight is 0, and 0 times them is not.  So they are zero
+// in the product (each thread looks at the pieces that it has loaded, which have landed) and are added afterwards to the rows that see their key.
+// marks: [2][2], the step's keys that have such values; zero at first.  n: the how manieth such step this is.
+__device__ __forceinline__ void hide_odd_values(unsigned char* values, int pieces, uint32_t* marks, int n) {
+  const int wide = 32 - __clz(pieces - 1), c = threadIdx.x & ((1 << wide) - 1), rows = kTcRowThreads >> wide;
+  if (threadIdx.x < 2) marks[2 * ((n + 1) & 1) + threadIdx.x] = 0u;   // (who reads these has done so before this step's scores)
+  if (c >= pieces) return;
+  const auto top = [](uint32_t v) { return (v & 0x7F807F80u) + 0x00800080u; };   // the upper bit of a half: its exponent is all ones
+#pragma unroll 1
+  for (int row = threadIdx.x >> wide; row < kTcKeys; row += rows) {
+    uint4* at = reinterpret_cast<uint4*>(values + tc_at(row, c, kTcKeys));
+    const uint4 v = *at;
+    if (((top(v.x) | top(v.y) | top(v.z) | top(v.w)) & 0x80008000u) == 0u) continue;
+    *at = make_uint4(finite_or_zero(v.x), finite_or_zero(v.y), finite_or_zero(v.z), finite_or_zero(v.w));
+    atomicOr(&marks[2 * (n & 1) + (row >> 5)], 1u << (row & 31));
+  }
+}
+// keys: those that hide_odd_values has marked; a row sees key kk where kk <= see_hi and (kk >= see_lo or kk < see_keep).  Whatever their weight, the sum is the infinity or
+// NaN.  Columns [first_column, first_column + columns) of the row, at o_mine in tensor memory.  Out of line: the steps keep their registers.
+__device__ __noinline__ void add_odd_values(const WinPromptArgs& a, uint64_t keys, int k0, int see_hi, int see_lo, int see_keep, int row, int lo, int nf, int g,
+                                            uint32_t o_mine, int dv, int first_column, int columns) {
+  const int back = a.back[row], p0 = a.pos[row] - back;
+  const int64_t seg_row0 = row - back, slot = a.slot[row];
+#pragma unroll 1
+  for (int c = 0; c < columns; c += 8) {
+    uint32_t o[8];
+    tc_ld8(o_mine + c, o);
+#pragma unroll 1
+    for (uint64_t left = keys; left != 0; left &= left - 1) {
+      const int kk = k0 + __ffsll((long long)left) - 1;
+      if (kk > see_hi || (kk < see_lo && kk >= see_keep)) continue;
+      const uint4 v = *reinterpret_cast<const uint4*>(win_row(a, kk, nf, lo, p0, seg_row0, slot, g, dv, a.vn, a.first_v, a.ring_v) + first_column + c);
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float f = __uint_as_float(i & 1 ? w[i >> 1] & 0xFFFF0000u : w[i >> 1] << 16);
+        if (!(fabsf(f) < INFINITY)) o[i] = __float_as_uint(__uint_as_float(o[i]) + f);
+      }
+    }
+    __syncwarp();
+    tc_st8(o_mine + c, o);
+  }
+  tc_st_wait();
+}
+
+// What a CTA's threads agree on, at the start of shared memory
+struct TcShared {
+  uint64_t s_ready, o_ready;   // a step's scores are in tensor memory; its values have been added
+  uint32_t tmem;
+  int dead;                    // a wait has run out
+  uint32_t odd[4];             // CAREFUL: which of a step's 64 keys have a value that is not finite [2 steps][2]
+  int again;                   // a result of the tile is not finite
+};
+
+// The tile, start to end.  CAREFUL (a second time): a value that is not finite has no part in rows that do not see its key.
+template <int NM, int C, bool CAREFUL>
+__device__ __forceinline__ void attend(const WinPromptArgs& a, int dv) {
   using T = __nv_bfloat16;
   extern __shared__ __align__(1024) unsigned char smem_tc[];
-  uint64_t* s_ready = reinterpret_cast<uint64_t*>(smem_tc);      // a step's scores are in tensor memory
-  uint64_t* o_ready = s_ready + 1;                               // its values have been added
-  uint32_t* tmem_s = reinterpret_cast<uint32_t*>(s_ready + 2);
-  volatile int* dead = reinterpret_cast<volatile int*>(tmem_s + 1);
+  TcShared& sh = *reinterpret_cast<TcShared*>(smem_tc);
+  uint64_t *s_ready = &sh.s_ready, *o_ready = &sh.o_ready;
+  volatile int* dead = &sh.dead;
+  const uint32_t tb = *reinterpret_cast<volatile uint32_t*>(&sh.tmem);
   float* xch = reinterpret_cast<float*>(smem_tc + 1024);         // [2 halves][128 rows] largest score, at the end sum of weights
   float* row_m = reinterpret_cast<float*>(smem_tc + 2048);       // [128] what a row's weights are relative to, for the peers
   float* row_l = row_m + 128;                                    // [128] their sum
@@ -190,23 +259,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(WinP
   const int nk = nf + (pa + count - lo);           // key index kk: the kept ones, then lo .. the last row's own position
   const int all = (nk + kTcKeys - 1) / kTcKeys, begin = (int)((int64_t)all * rank / C), steps = (int)((int64_t)all * (rank + 1) / C) - begin;   // this CTA's
 
-  if (warp == 8) {
-    if (lane == 0) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(s_ready)) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(o_ready)) : "memory");
-      *dead = 0;
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp();
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(tmem_s)), "r"(kTcColumns));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    tc_before();
-  }
-  __syncthreads();
-  tc_after();
-  const uint32_t tb = *reinterpret_cast<volatile uint32_t*>(tmem_s);
-  uint32_t parity = 0;
-  bool ok = true;
+  uint32_t parity = CAREFUL ? (uint32_t)(NM * steps) & 1u : 0u;   // of the step's barriers
+  int hidings = 0;                                               // steps in which some rows did not see all keys
+  bool ok = !CAREFUL || *dead == 0;                              // (a wait ran out before: nothing more is issued)
 
 #pragma unroll 1
   for (int m = 0; m < NM; ++m) {
@@ -264,10 +319,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(WinP
           const int kk = k0 + row;
           const uint32_t at = tc_at(row, c, kTcKeys);
           if (kk < nk) {
-            const int j = kk < nf ? kk : lo + (kk - nf);
-            const T* src = j >= p0 ? step + ((seg_row0 + (j - p0)) * G + g) * width
-                                   : (j < a.first_rows ? kept + ((s * a.first_rows + j) * G + g) * width : ring + ((s * a.ring + j % a.ring) * G + g) * width);
-            tc_cp16(dst + at, src + off + c * 8);
+            tc_cp16(dst + at, win_row(a, kk, nf, lo, p0, seg_row0, s, g, width, step, kept, ring) + off + c * 8);
           } else {                                         // behind the last key: zero
             *reinterpret_cast<uint4*>(tile_at + at) = make_uint4(0, 0, 0, 0);
           }
@@ -304,6 +356,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(WinP
       const float to_log2 = fmaxf(fabsf(a.scale) * 1.4426950408889634f, 1e-37f);   // (the sign is the queries'; a hidden key stays -inf)
 #pragma unroll 1
       for (int t = 0; t < steps; ++t, parity ^= 1u) {
+        const int k0 = (begin + t) * kTcKeys;
+        const bool plain = k0 + kTcKeys <= nk && (k0 + kTcKeys - 1 < nf || lo + (k0 + kTcKeys - 1 - nf) <= pa) &&
+                           pa + count - 1 - (lo + max(k0 - nf, 0)) < a.window;   // every row sees every key of the step
         ok = ok && tc_wait(s_ready, parity, dead);
         tc_after();
         uint32_t x[32];
@@ -311,9 +366,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(WinP
         // the row's largest score, in units of log2
         float top = -INFINITY;
         {
-          const int k0 = (begin + t) * kTcKeys, base = k0 + half * 32;
-          const bool plain = k0 + kTcKeys <= nk && (k0 + kTcKeys - 1 < nf || lo + (k0 + kTcKeys - 1 - nf) <= pa) &&
-                             pa + count - 1 - (lo + max(k0 - nf, 0)) < a.window;   // every row sees every key of the step
+          const int base = k0 + half * 32;
           if (!plain) {
             const int hi = (r < count ? nf + (pa + r - lo) : -1) - base, low = nf + max(pa + r - a.window + 1 - lo, 0) - base;
             const int kept = nf + max(a.keep - lo, 0) - base;
@@ -368,6 +421,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(WinP
           tc_st_wait();
           if (b == 0) {
             cp_async_wait<0>();                            // the step's values
+            if (CAREFUL && !plain) hide_odd_values(Vs, vc, sh.odd, hidings);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           }
           tc_before();
@@ -380,6 +434,15 @@ __global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(WinP
         cp_async_commit();
         ok = ok && tc_wait(o_ready, parity, dead);
         tc_after();
+        if (CAREFUL && !plain) {   // (the marks are older than the products that o_ready stands for)
+          const volatile uint32_t* mark = sh.odd + 2 * (hidings++ & 1);
+          const uint64_t keys = mark[0] | ((uint64_t)mark[1] << 32);
+          if (keys != 0) {
+            add_odd_values(a, keys, k0, r < count ? nf + (pa + r - lo) : -1, nf + max(pa + r - a.window + 1 - lo, 0), nf + max(a.keep - lo, 0), first, lo, nf, g, o_mine,
+                           dv, half * dvh, dvh);
+            tc_before();
+          }
+        }
         if (more) {
           cp_async_wait<0>();
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -428,7 +491,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(WinP
       }
       const float k = 1.f / sum;
       // U pieces of four columns at a time, all shares of them in flight: use(piece, the row's four results)
-      constexpr int U = C >= 4 ? 1 : 4 / C;
+      constexpr int U = C >= 4 || NM == 2 ? 1 : 4 / C;   // (two maps, two pieces: 300 bytes of registers spilled, 2048 rows of 16 heads 133 us and not 111)
       auto results = [&](auto&& use) {
         for (int c0 = part; c0 < dv / 4; c0 += U * per) {
           float4 v[U][C];
@@ -468,7 +531,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(WinP
         T* dst = a.out + (int64_t)(first + row) * a.ld_out + (int64_t)h * dv;
         const bool wide = a.ld_out % 4 == 0 && reinterpret_cast<uintptr_t>(a.out) % 8 == 0, pairs = a.ld_out % 2 == 0;
         if (row < count) {
+          bool finite = true;
           results([&](int c4, const float4& y) {
+            if (!CAREFUL) finite = finite && fabsf(y.x * mul) < INFINITY && fabsf(y.y * mul) < INFINITY && fabsf(y.z * mul) < INFINITY && fabsf(y.w * mul) < INFINITY;
             const uint2 w = make_uint2(pack_bf16(y.x * mul, y.y * mul), pack_bf16(y.z * mul, y.w * mul));
             if (wide) {
               *reinterpret_cast<uint2*>(dst + c4 * 4) = w;
@@ -480,13 +545,50 @@ __global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(WinP
               for (int i = 0; i < 4; ++i) dst[c4 * 4 + i] = __ushort_as_bfloat16((unsigned short)(u[i >> 1] >> (16 * (i & 1))));
             }
           });
+          if (!finite) {
+#pragma unroll
+            for (int c = 0; c < C; ++c) tc_peer_set(tc_peer(tc_smem(&sh.again), c));
+          }
         }
       }
     }
     tc_cluster_sync();   // the peers have read what lies here
   }
-  if (*dead != 0) {   // a wait ran out: all rows of the tile are marked, after the peers' results, and what is in flight gets the time to land
-    if (threadIdx.x < count)
+}
+
+template <int NM, int C>
+__device__ __noinline__ void attend_carefully(const WinPromptArgs& a, int dv) {
+  attend<NM, C, true>(a, dv);
+}
+
+template <int NM, int C>
+__global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(const __grid_constant__ WinPromptArgs a, int dv) {
+  extern __shared__ __align__(1024) unsigned char smem_tc[];
+  TcShared& sh = *reinterpret_cast<TcShared*>(smem_tc);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 8) {
+    if (lane == 0) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&sh.s_ready)) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&sh.o_ready)) : "memory");
+      sh.dead = sh.again = 0;
+      sh.odd[0] = sh.odd[1] = sh.odd[2] = sh.odd[3] = 0u;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&sh.tmem)), "r"(kTcColumns));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    tc_before();
+  }
+  __syncthreads();
+  tc_after();
+  attend<NM, C, false>(a, dv);
+  // A hidden key's weight is 0, and 0 times a value that is not finite is not: where a result is not finite (on any CTA of the cluster, which has
+  // told the others) the tile is done once more with an eye to that.  (Looking at the values of every step that hides keys: 2048 rows 62 us, not 60.)
+  if (*reinterpret_cast<volatile int*>(&sh.again) != 0) attend_carefully<NM, C>(a, dv);
+  const int tile = (int)(gridDim.x / C - 1 - ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) / C / a.H), h = (int)(((int64_t)blockIdx.y * gridDim.x + blockIdx.x) / C % a.H);
+  if (*reinterpret_cast<volatile int*>(&sh.dead) != 0) {   // a wait ran out: all rows of the tile are marked, after the peers' results, and what is in flight gets the time to land
+    const int first = a.tile_first[tile];
+    if (threadIdx.x < min(a.tile_count[tile], kTcRows))
       for (int c = 0; c < dv; ++c) a.out[(int64_t)(first + threadIdx.x) * a.ld_out + (int64_t)h * dv + c] = __ushort_as_bfloat16((unsigned short)0x7FFF);
     for (int i = 0; i < 64; ++i) __nanosleep(100000);
   }
@@ -494,7 +596,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(WinP
   __syncthreads();
   if (warp == 8) {
     tc_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tb), "r"(kTcColumns));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*reinterpret_cast<volatile uint32_t*>(&sh.tmem)), "r"(kTcColumns));
   }
 }
 
