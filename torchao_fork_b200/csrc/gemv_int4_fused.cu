@@ -122,18 +122,14 @@ __device__ __forceinline__ float warp_max_f(float v) {
 // The split kernel's sums that are not finite (split_again), with the weights rounded to bf16 as the GEMM and the strip kernel meet them; w, sz: the strip's
 template <int G>
 __device__ __noinline__ float4 again4(const uint8_t* w, const uint32_t* sz, const __nv_bfloat16* x, int64_t ldx, int64_t Kx, int M, float4 sum, int lane) {
-  return split_again(sum, M, Kx, lane, [&](int row, int m, int64_t k) {
-    float f[8];
-    unpack8(*reinterpret_cast<const uint4*>(x + m * ldx + k), f);
+  return split_again(sum, x, ldx, M, Kx, lane, [&](int row, int64_t k, float (&out)[8]) {
     // word j of a lane's 16 bytes: row g + 8 (j & 1) of the tile's 32-k half j >> 1
     const uint32_t par = __ldg(sz + (k / G) * 16 + row);
     uint32_t o[4];
     dequant_word(__ldg(reinterpret_cast<const uint32_t*>(w + (k >> 6) * 512 + (4 * (row & 7) + ((k >> 3) & 3)) * 16) + 2 * ((k >> 5) & 1) + (row >> 3)),
                  __byte_perm(par, 0, 0x1010), __byte_perm(par, 0, 0x3232), o);
-    double t = 0.0;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) t += (double)f[e] * (double)__uint_as_float(e & 1 ? o[e >> 1] & 0xFFFF0000u : o[e >> 1] << 16);
-    return t;
+    for (int i = 0; i < 4; ++i) out[2 * i] = __uint_as_float(o[i] << 16), out[2 * i + 1] = __uint_as_float(o[i] & 0xFFFF0000u);
   });
 }
 

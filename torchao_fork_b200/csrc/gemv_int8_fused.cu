@@ -74,16 +74,12 @@ __device__ __forceinline__ uint32_t u8_f16_hi(uint32_t w) { return __byte_perm(w
 
 // The split kernel's sums that are not finite (split_again); w: the strip's weights
 __device__ __noinline__ float4 again8(const uint8_t* w, const __nv_bfloat16* x, int64_t ldx, int64_t Kx, int M, float4 sum, int lane) {
-  return split_again(sum, M, Kx, lane, [&](int row, int m, int64_t k) {
-    float f[8];
-    unpack8(*reinterpret_cast<const uint4*>(x + m * ldx + k), f);
+  return split_again(sum, x, ldx, M, Kx, lane, [&](int row, int64_t k, float (&out)[8]) {
     // word j of a lane's 16 bytes: row g + 8 (j & 1), four k from 4 (j >> 1) on
     const uint32_t* at = reinterpret_cast<const uint32_t*>(w + (k >> 5) * 512 + (4 * (row & 7) + ((k >> 3) & 3)) * 16) + (row >> 3);
     const uint32_t u[2] = {__ldg(at), __ldg(at + 2)};
-    double t = 0.0;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) t += (double)f[e] * (double)((int)((u[e >> 2] >> (8 * (e & 3))) & 0xFF) - 128);
-    return t;
+    for (int e = 0; e < 8; ++e) out[e] = (float)((int)((u[e >> 2] >> (8 * (e & 3))) & 0xFF) - 128);
   });
 }
 

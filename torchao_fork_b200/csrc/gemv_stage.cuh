@@ -204,35 +204,76 @@ __device__ __forceinline__ bool split_sums(float4 (&sum)[MT], const float* row_s
   }
   return true;
 }
-// The sums of a strip (lane (g, c): rows g and g + 8, x and y, z and w; columns 2 c, 2 c + 1 of the M) that are not finite, done again by the whole warp:
-// an infinity has lost its sign against the weights' offset, or one rank's part has overflowed where the total does not.  dot(row, m, k) adds eight
-// products; sums in 64 bits, rounded to 32 once.  Rare, and slow.
-template <typename Dot>
-__device__ __forceinline__ float4 split_again(float4 sum, int M, int64_t Kx, int lane, Dot&& dot) {
-  float v[4] = {sum.x, sum.y, sum.z, sum.w};
+// The sums of a strip (lane (g, c): rows g and g + 8, x and y, z and w; columns 2 c, 2 c + 1 of the M) where some are not finite, done again by the whole
+// warp: an infinity has lost its sign against the weights' offset, or one rank's part has overflowed where the total does not.  weights(row, k, w): eight
+// of them from k on, as fp32.  A row of x with infinities or NaN is decided by these alone; one without is added up in 64 bits and rounded to 32 once, a
+// weight row at a time.  (Every row with an infinity: 8 rows of 4096 x 14336 0.23 ms, 7 of 8192 x 28672 about 1.5.)
+template <typename Weights>
+__device__ __forceinline__ float4 split_again(float4 sum, const __nv_bfloat16* x, int64_t ldx, int M, int64_t Kx, int lane, Weights&& weights) {
+  const auto bad = [](float v) { return !(fabsf(v) < INFINITY); };
 #pragma unroll 1
-  for (int i = 0; i < 4; ++i) {
-    const float own = i == 0 ? v[0] : i == 1 ? v[1] : i == 2 ? v[2] : v[3];
-    uint32_t bad = __ballot_sync(0xffffffffu, 2 * (lane & 3) + (i & 1) < M && !(fabsf(own) < INFINITY));
-    float redone = own;
+  for (int m = 0; m < M; ++m) {
+    const bool mine = (lane & 3) == m >> 1;
+    const bool low = mine && bad(m & 1 ? sum.y : sum.x), high = mine && bad(m & 1 ? sum.w : sum.z);
+    if (!__any_sync(0xffffffffu, low || high)) continue;
+    const __nv_bfloat16* row_x = x + m * ldx;
+    double t = 0.0;               // of weight row lane & 15
+    bool odd = false;             // the row of x has something that is not finite
+    const auto top = [](uint32_t u) { return (u & 0x7F807F80u) + 0x00800080u; };   // the upper bit of a half: its exponent is all ones
 #pragma unroll 1
-    for (; bad != 0; bad &= bad - 1) {
-      const int src = __ffs(bad) - 1, row = (src >> 2) + 8 * (i >> 1), m = 2 * (src & 3) + (i & 1);
-      double t = 0.0;
-#pragma unroll 1
-      for (int64_t k = 8 * lane; k - 8 * lane < Kx; k += 256) {
-        if (k < Kx) t += dot(row, m, k);
-        if (__any_sync(0xffffffffu, t != t)) break;   // NaN stays NaN
+    for (int64_t k0 = 0; k0 < Kx; k0 += 8 * 256) {
+      uint4 v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int64_t k = k0 + i * 256 + 8 * lane;
+        v[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (k < Kx) v[i] = *reinterpret_cast<const uint4*>(row_x + k);
       }
+      uint32_t own = 0u;          // which of this lane's eight
 #pragma unroll
-      for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (lane == src) redone = (float)t;
+      for (int i = 0; i < 8; ++i) own |= (((top(v[i].x) | top(v[i].y) | top(v[i].z) | top(v[i].w)) & 0x80008000u) != 0u ? 1u : 0u) << i;
+      uint32_t at = __ballot_sync(0xffffffffu, own != 0u);
+      odd = odd || at != 0u;
+#pragma unroll 1
+      for (; at != 0u; at &= at - 1) {
+        const int src = __ffs(at) - 1;
+#pragma unroll 1
+        for (uint32_t left = __shfl_sync(0xffffffffu, own, src); left != 0u; left &= left - 1) {
+          float f[8], w[8];
+          const int64_t there = k0 + (__ffs(left) - 1) * 256 + 8 * src;
+          unpack8(*reinterpret_cast<const uint4*>(row_x + there), f);
+          weights(lane & 15, there, w);
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (bad(f[e])) t += (double)f[e] * (double)w[e];
+        }
+        if (__all_sync(0xffffffffu, t != t)) break;   // (NaN stays NaN)
+      }
+      if (__all_sync(0xffffffffu, t != t)) break;
     }
+    if (!odd) {
+#pragma unroll 1
+      for (int row = 0; row < 16; ++row) {
+        if (!__any_sync(0xffffffffu, (lane >> 2) == (row & 7) && (row < 8 ? low : high))) continue;
+        double part = 0.0;
+#pragma unroll 2
+        for (int64_t k = 8 * lane; k < Kx; k += 256) {
+          float f[8], w[8];
+          unpack8(*reinterpret_cast<const uint4*>(row_x + k), f);
+          weights(row, k, w);
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (j == i) v[j] = redone;
+          for (int e = 0; e < 8; ++e) part += (double)f[e] * (double)w[e];
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        if ((lane & 15) == row) t = part;
+      }
+    }
+    const float lo = __shfl_sync(0xffffffffu, (float)t, lane >> 2), hi = __shfl_sync(0xffffffffu, (float)t, (lane >> 2) + 8);
+    if (low) (m & 1 ? sum.y : sum.x) = lo;
+    if (high) (m & 1 ? sum.w : sum.z) = hi;
   }
-  return make_float4(v[0], v[1], v[2], v[3]);
+  return sum;
 }
 // whether any of the sums that count is not finite, on any lane
 __device__ __forceinline__ bool split_overflowed(const float4& s, int M, int lane) {
