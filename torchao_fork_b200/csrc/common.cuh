@@ -149,6 +149,10 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, u
                "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
+// global -> L2 (bytes % 16 == 0, 16-byte aligned): fetches ahead of a wait without reading, as what the kernel in front writes meets it in L2
+__device__ __forceinline__ void bulk_prefetch_l2(const void* src_gmem, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src_gmem), "r"(bytes) : "memory");
+}
 // PDL: wait until the grids this launch programmatically depends on have completed (no-op otherwise)
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // PDL: let the next kernel in the stream start launching (its pre-wait prologue overlaps our tail)

@@ -187,7 +187,11 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     }
     __syncwarp();
     named_bar_arrive(2, kFThreads);
-    if (!p.settled) grid_dependency_wait();
+    if (!p.settled) {
+      if (lane == 0 && s1 > s0)
+        bulk_prefetch_l2(p.packed + ((int64_t)s0 * ks + rank) * KT * 512, min((uint32_t)(stages * kStageTiles), (uint32_t)((SPLIT ? 1 : s1 - s0) * KT)) * 512u);
+      grid_dependency_wait();
+    }
     {
       int slot = 0;
       uint32_t par = 1;

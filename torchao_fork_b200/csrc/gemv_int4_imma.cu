@@ -132,7 +132,10 @@ __global__ void __launch_bounds__(kIThreads, 2) int4_gemv_imma_kernel(const Gemv
     }
     __syncwarp();
     named_bar_arrive(2, kIThreads);
-    if (!p.settled) grid_dependency_wait();
+    if (!p.settled) {
+      if (lane == 0 && s1 > s0) bulk_prefetch_l2(p.packed + (int64_t)s0 * KT * 512, min((uint32_t)(stages * kIStageTiles), (uint32_t)((s1 - s0) * KT)) * 512u);
+      grid_dependency_wait();
+    }
     if (lane == 0) {
       int slot = 0;
       uint32_t par = 1;

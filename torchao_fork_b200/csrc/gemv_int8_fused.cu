@@ -138,7 +138,11 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     }
     __syncwarp();
     named_bar_arrive(2, k8Threads);
-    if (!p.settled) grid_dependency_wait();
+    if (!p.settled) {
+      if (lane == 0 && s1 > s0)
+        bulk_prefetch_l2(p.packed + ((int64_t)s0 * ks + rank) * KT * 1024, min((uint32_t)(stages * k8StageTiles), (uint32_t)((SPLIT ? 1 : s1 - s0) * KT)) * 1024u);
+      grid_dependency_wait();
+    }
     if (lane == 0) {
       int slot = 0;
       uint32_t par = 1;
