@@ -656,7 +656,7 @@ static bool plan_fused(int M, int MT, int64_t Kp, int max_stages, FusedPlan& pl,
   }();
   if (inbox == 0 && fixed + min2 * stage_b <= two_per_sm) {
     st = (int)((two_per_sm - fixed) / stage_b);
-  } else if (fixed + 3 * stage_b <= one_per_sm) {
+  } else if (fixed + (inbox != 0 ? kSplitStages : 3) * stage_b <= one_per_sm) {
     st = (int)((one_per_sm - fixed) / stage_b);
   } else {
     return false;

@@ -536,7 +536,7 @@ static bool plan8(int M, int MT, int64_t Kp, int max_stages, Plan8& pl, size_t i
   int st = 0;
   if (MT == 1 && inbox == 0 && fixed + 4 * (size_t)k8StageBytes <= two_per_sm) {
     st = (int)((two_per_sm - fixed) / k8StageBytes);
-  } else if (fixed + 3 * (size_t)k8StageBytes <= one_per_sm) {
+  } else if (fixed + (inbox != 0 ? kSplitStages : 3) * (size_t)k8StageBytes <= one_per_sm) {
     st = (int)((one_per_sm - fixed) / k8StageBytes);
   } else {
     return false;

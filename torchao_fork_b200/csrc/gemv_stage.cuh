@@ -148,6 +148,9 @@ __device__ __forceinline__ void stage_rows(const __nv_bfloat16* x, int64_t ldx, 
 // For activations that one CTA cannot hold, or takes long to stage.  Each CTA sums its part of a strip; those of the other ranks send theirs
 // into shared memory of rank 0 (st.async), which has room for all its strips, adds them in rank order and finishes the strip: nobody waits to send.
 constexpr int kMaxSplitStrips = 32;   // strips of a cluster
+// Stages of the weight ring that have to fit beside the activations and the inbox.  With three the ring no longer covers the way from memory (int4
+// 8192 x 28672, 8 rows 46 us and the GEMM 45 to 46, 16384 x 28672, 7 rows 82 and 78; int8 104 and 86); with four it does (40.5 at 7 rows; 73 at 6).
+constexpr int kSplitStages = 4;
 
 // Without a norm, up to 8 rows: from here on halves beat whole rows (int8, 8 rows: 3072 x 8192 8.7 us against 12.1, 8192 x 8192 16.0 against 19.1;
 // 4 rows of 4096 x 14336 14.7 against 15.4; int4 8.3 against 10.3, 13.4 against 15.5, 13.4 against 15.9; below: int8, 8 rows of 5120 x 5120 10.0
