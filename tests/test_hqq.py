@@ -173,3 +173,33 @@ def test_packed_words_of_many_weights_equal_the_plain_result(gs, seed):
     packed, _ = T.b200_int4_hqq_quantize_pack(w, gs)
     q, _, _ = T.b200_int4_hqq_quantize(w, gs)
     assert torch.equal(T.b200_int4_unpack(packed)[:4096, :4096], q)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,gs,spread", [((4096, 4096), 64, 0.05), ((1024, 4096), 32, 0.05), ((1024, 4096), 128, 1.0), ((1024, 4096), 256, 0.02)])
+def test_zero_points_of_the_search_equal_those_of_the_steps_in_32_bits(shape, gs, spread):
+    """ao_b200_hqq_search against init / solve, the fp32 zero points as they are left in the workspace ([means 64 x 8 bytes][errors 10 x 8 bytes per
+    8192 weights][scale][zero points of the last ten iterations]), bit for bit: a product and a sum rounded as one would show in their last bits."""
+    from torchao_fork_b200 import _lib
+    from torchao_fork_b200 import ops as aops
+    g = torch.Generator(device="cuda").manual_seed(gs)
+    n, k = shape
+    w = (spread * torch.randn(n, k, device="cuda", generator=g)).to(torch.bfloat16)
+    L, st, n_groups = _lib.lib(), torch.cuda.current_stream().cuda_stream, n * k // gs
+    scale = torch.empty(n_groups, dtype=torch.float32, device="cuda")
+    zero, err = torch.empty_like(scale), torch.empty(int(L.ao_b200_hqq_blocks(n_groups)), dtype=torch.float32, device="cuda")
+    state = torch.empty(2, dtype=torch.float64, device="cuda")
+    args = (aops.HQQ_BETA, aops.HQQ_KAPPA, aops.HQQ_LP_NORM, aops.HQQ_ITERS)
+    _lib.check(L.ao_b200_hqq_init(w.data_ptr(), n_groups, gs, scale.data_ptr(), zero.data_ptr(), st), "init")
+    _lib.check(L.ao_b200_hqq_solve(w.data_ptr(), n_groups, gs, scale.data_ptr(), zero.data_ptr(), *args, err.data_ptr(), state.data_ptr(), st), "solve")
+    ws = torch.empty(int(L.ao_b200_hqq_search_workspace_bytes(n_groups, gs)), dtype=torch.uint8, device="cuda")
+    q = torch.empty(n, k, dtype=torch.int32, device="cuda")
+    s, z = (torch.empty(n, k // gs, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    _lib.check(L.ao_b200_hqq_search(w.data_ptr(), n, k, gs, *args, ws.data_ptr(), ws.numel(), q.data_ptr(), s.data_ptr(), z.data_ptr(), 0, 0, None, None, st),
+               "search")
+    ran = int(state[1:].view(torch.int32)[1])
+    at = (64 + 10 * (-(-n * k // 8192))) * 8
+    own = ws[at : at + 4 * n_groups * 11].view(torch.float32)
+    assert torch.equal(own[:n_groups], scale)
+    last = (ran - 1) % 10
+    assert torch.equal(own[n_groups * (1 + last) : n_groups * (2 + last)].view(torch.int32), zero.view(torch.int32))

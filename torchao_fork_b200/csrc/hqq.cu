@@ -123,14 +123,15 @@ __global__ void __launch_bounds__(kHqqWarps * 32) hqq_finalize_kernel(const __nv
 }
 
 // ---- the whole search: chunks of iterations with the group in registers --------------------------------------------------
-// The iterations of a group depend on no other group; only the early stop looks at all of them.  So a thread keeps 16
+// The iterations of a group depend on no other group; only the early stop looks at all of them.  So a thread keeps 32
 // weights of a group in registers through kHqqChunk iterations and leaves behind the zero point after each of them (`hist`)
 // and the block's error of each (`err`); hqq_mean_kernel adds the errors up, and whoever comes next works out
 // from the means which iteration was the last (hqq_last), so that iterations past the stop cost work but change nothing.
 //
 // Bound by the fp32 pipe and instruction issue: ten iterations over 4096 x 4096 take about 80 us.  What keeps the arithmetic at eleven
 // instructions per pair of weights and iteration:
-//  - pairs of weights in one register pair (add, mul, fma .f32x2: the single operation's rounding in each half);
+//  - pairs of weights in one register pair (add, mul, fma .f32x2: the single operation's rounding in each half.  But a product whose one use is a sum
+//    can come out as one fused operation, .rn or not, so such a sum is a fused one already, with a factor of one);
 //  - the group's smallest and largest weight bound every |d| and say whether anything is clamped, so that, as a rule, neither
 //    the clamp nor the shrinkage is looked at per weight.  |d| - c |d|^(p - 1) is not positive for |d| <= c^(1 / (2 - p)) (p < 1), 0.17 at the
 //    reference's constants, which is above most weights' error: powf runs only above that threshold (less a margin of 1e-3, thousands of
@@ -175,7 +176,7 @@ __device__ __noinline__ float hqq_shrink(float d, float c, float lp_m1) {
   return copysignf(fmaxf(__fsub_rn(ad, __fmul_rn(c, powf(ad, lp_m1))), 0.f), d);
 }
 
-// two fp32 in one register pair: one instruction for both, each with the single operation's rounding
+// two fp32 in one register pair: one instruction for both, each with the single operation's rounding (see above for a product that is added)
 struct F2 {
   uint64_t v;
 };
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(256, kHqqBlocks) hqq_iterate_kernel(const __nv
   }
   // (the minus signs ride along: -x = n (-r), its remainder n + (-x) s, and -(x + r rem) = (-r) rem + (-x), all rounded as without them)
   const float nr = -__frcp_rn(s), t_lo = __fmul_rn(mn, s), t_hi = __fmul_rn(mx, s);
-  const F2 s2 = f2(s, s), ns2 = f2(-s, -s), nr2 = f2(nr, nr), minus = f2(-1.f, -1.f), magic = f2(kMagic, kMagic), no_magic = f2(-kMagic, -kMagic);
+  const F2 s2 = f2(s, s), ns2 = f2(-s, -s), nr2 = f2(nr, nr), one = f2(1.f, 1.f), minus = f2(-1.f, -1.f), magic = f2(kMagic, kMagic), no_magic = f2(-kMagic, -kMagic);
 #pragma unroll 1
   for (int it = 0; it < ch.count; ++it) {
     // (the compiler would keep all weights unpacked and multiplied beside the packed ones, and have no registers left)
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(256, kHqqBlocks) hqq_iterate_kernel(const __nv
         lane_pair(i, a, b, [&](int k, F2& x) {
           F2 wq, nt;
           const float2 d = quotients(weights(k), false, wq, nt);
-          x = f2_add(wq, nt);
+          x = f2_fma(nt, one, wq);
           return d;
         });
       }, acc, e);
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(256, kHqqBlocks) hqq_iterate_kernel(const __nv
         lane_pair(i, a, b, [&](int k, F2& x) {
           F2 wq, nt;
           const float2 d = quotients(weights(k), true, wq, nt);
-          x = f2_add(wq, nt);
+          x = f2_fma(nt, one, wq);
           return d;
         });
       }, acc, e);
