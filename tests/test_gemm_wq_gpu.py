@@ -307,3 +307,43 @@ def test_long_few_rows_with_infinities_huge_and_tiny_values(bits, group, residua
             ref = xd @ wd.t()
             near = min(((got - r).norm() / ref.norm()).item() for r in (ref, xd @ wb.t() if bits == 4 else ref))
             assert got.isfinite().all() and near < 2.0 ** -8, (row, near)
+
+
+@pytest.mark.parametrize("bits,group", [(4, 32), (4, 128), (8, 0)])
+@pytest.mark.parametrize("m", [24, 32, 48, 64, 77, 128, 144, 256, 300])
+@pytest.mark.parametrize("residual", [False, True])
+def test_last_tile_from_the_accumulators(bits, group, m, residual):
+    """28672 x 2048: 16 units a tile and 24 for each CTA or pair of 148 or 74, so every other tile is shared by two with at least eight units behind it, and
+    its first owner finishes it from its accumulators if the second one was there before.  By the deal (25 c mod 16) it holds any number of units of it,
+    one among them.  Up to 32 rows one CTA, up to 64 two issuing warps, up to 128 two accumulator buffers, from 257 on two row tiles.  Whether that path is taken
+    depends on time: equal calls give equal bits all the same.  Bound as above; a wrong tile would show in its 128 columns, so they are looked at by themselves."""
+    from torchao_fork_b200 import _lib
+    n, k = 28672, 2048
+    gen = torch.Generator(device="cuda").manual_seed(m + bits)
+    w = torch.randn(n, k, generator=gen, device="cuda").to(torch.bfloat16)
+    x = torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16)
+    if bits == 4:
+        packed, scales = T.b200_int4_quantize_pack(w, group, 1e-6, True)
+        p = scales.permute(0, 2, 1, 3).reshape(packed.shape[0] * 16, -1, 2)[:n, : k // group].double()
+        wd = ((T.b200_int4_unpack(packed)[:n, :k].double().reshape(n, -1, group) - 8) * p[..., 0:1] + p[..., 1:2]).reshape(n, k)
+        run = lambda: T.b200_int4_weight_only_mm(x, packed, group, scales, n)  # noqa: E731
+    else:
+        q, scales = T.b200_int8_quantize(w, 1e-6, True)
+        packed, wd = T.b200_int8_pack(q), q.double() * scales.double()[:, None]
+        run = lambda: T.b200_int8_weight_only_mm(x, packed, scales)  # noqa: E731
+    ref, h = x.double() @ wd.t(), None
+    if residual:
+        L = _lib.lib()
+        h = torch.randn(m, n, generator=gen, device="cuda").to(torch.bfloat16)
+        ws = torch.empty(L.ao_b200_mm_residual_workspace_bytes(m, n, k, group), dtype=torch.uint8, device="cuda")
+
+        def run():
+            y = torch.empty_like(h)
+            _lib.check(L.ao_b200_mm_residual(x.data_ptr(), m, k, k, packed.data_ptr(), scales.data_ptr(), n, k, group, y.data_ptr(), n, n, h.data_ptr(), n,
+                                             ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream), "mm_residual")
+            return y
+        ref = ref + h.double()
+    y = run()
+    tiles = lambda t: t.reshape(m, n // 128, 128).square().sum((0, 2)).sqrt()  # noqa: E731
+    assert (tiles(y.double() - ref) / tiles(ref)).max().item() < 2.0 ** -8
+    assert all(torch.equal(run(), y) for _ in range(12))

@@ -3,8 +3,8 @@ picks who goes on, copies land and matrix products retire when the scheduler say
 the parity of its phase, so a wait that may look for a phase too early takes the one before for it, and the role then meets the wrong unit.
 
 What is modelled: the rings of weights, activations and tensor-memory operands, the two sets of dequant warps (two warps each), one or
-two issuing warps, one CTA or a pair, the accumulators and the epilogue, both forms (DEFER: the epilogue reads every unit).  What each
-slot holds is followed, and every read and overwrite is checked.  The ring sizes are those of wq_launch for every row count and group."""
+two issuing warps, one CTA or a pair, the accumulators and the epilogue, both forms (DEFER: the epilogue reads every unit), and the last tile that
+stays in its accumulators until all warps finish it (EARLY: each CTA of a pair decides for itself).  What each slot holds is followed, and every read and overwrite is checked.  The ring sizes are those of wq_launch for every row count and group."""
 import random
 
 import pytest
@@ -67,7 +67,7 @@ EPI = 2     # epilogue warps (the kernel has 4)
 
 
 class Model:
-    def __init__(self, rng, cfg, units, ku, first=0, a_first=None):
+    def __init__(self, rng, cfg, units, ku, first=0, a_first=None, early=False, early_before_products=False):
         self.rng, self.c, self.u0, self.u1, self.ku = rng, cfg, first, first + units, ku
         ranks = range(2 if cfg["pair"] else 1)
         self.ranks, self.lead = ranks, 0
@@ -91,6 +91,9 @@ class Model:
         # (wq_gemm_kernel: a_first)
         self.a_first = (w % 2 == 1 and w < a + 2) if a_first is None else a_first
         self.done_tiles = [[] for _ in ranks]
+        # EARLY: the last tile is shared with the next CTA, whose share this rank finds there (by time, so at random), or does not
+        self.stays = [early and not cfg["defer"] and self.u1 % ku != 0 and first <= self.u1 // ku * ku and rng.random() < 0.7 for _ in ranks]
+        self.early_before_products, self.kept = early_before_products, [None for _ in ranks]
 
     def check(self, ok, what):
         if not ok:
@@ -239,18 +242,33 @@ class Model:
                     w.step(1)
                     u += 1
             else:
-                yield lambda: self.dfull[r][d.slot].over(d.use)
-                n = c["n_mma"]
-                two = n == 2 and end - u > 1
-                got = set()
-                for mw in ((0, 1) if two else ((u - self.u0) & 1,) if n == 2 else (0,)):
-                    got |= self.dbuf[d.slot][mw]
-                self.check(got == set(range(u, end)), f"tile {t} has units {got}, not {u} .. {end - 1}")
+                last = self.stays[r] and end == self.u1
+                if not (last and self.early_before_products):
+                    yield lambda: self.dfull[r][d.slot].over(d.use)
+                if last:   # the tile is left where it is: buffer and, with one unit, whose accumulator (as the kernel works them out at the end)
+                    slot = (t - self.u0 // self.ku) % c["d"]
+                    self.check(slot == d.slot, "another buffer than the epilogue's")
+                    self.kept[r] = (slot, t * self.ku, end, (t * self.ku - self.u0) & 1)
+                    break
+                self.drained(d.slot, t, u, end, (u - self.u0) & 1)
                 self.dempty[0][d.slot].arrive()
                 d.step(1)
                 u = end
             t += 1
         self.done_tiles[r].append(warp)
+
+    def drained(self, slot, t, u, end, parity):
+        n = self.c["n_mma"]
+        two = n == 2 and end - u > 1
+        got = set()
+        for mw in ((0, 1) if two else (parity,) if n == 2 else (0,)):
+            got |= self.dbuf[slot][mw]
+        self.check(got == set(range(u, end)), f"tile {t} has units {got}, not {u} .. {end - 1}")
+
+    def meet(self, r):
+        # all warps of the CTA, as soon as each is through with its own part
+        slot, u, end, parity = self.kept[r]
+        self.drained(slot, u // self.ku, u, end, parity)
 
     def run(self):
         roles = [self.weights(r) for r in self.ranks] + [self.rows(r) for r in self.ranks] + [self.issue(m) for m in range(self.c["n_mma"])]
@@ -258,6 +276,7 @@ class Model:
         roles += [self.epilogue(r, k) for r in self.ranks for k in range(EPI)]
         if self.c["pair"]:
             roles.append(self.peer())
+        mine = {r: [g for g in roles if g.gi_frame.f_locals.get("r", 0 if g.gi_code.co_name != "peer" else 1) == r] for r in self.ranks}
         # a role's speed: now and then one of them, or a copy, is held back for long
         waits = {}
         for g in roles:
@@ -267,7 +286,12 @@ class Model:
                 pass
         weight = {g: self.rng.choice([1, 1, 5, 40]) for g in roles}
         lazy_copies, lazy_products = self.rng.choice([1, 10, 60]), self.rng.choice([1, 10, 60])
+        met = set()
         while waits or self.flying or any(self.queue):
+            for r in self.ranks:   # the CTA's own roles are over (what its issuing warp has asked for may be under way)
+                if self.kept[r] and r not in met and not any(g in waits for g in mine[r]):
+                    met.add(r)
+                    self.meet(r)
             ready = [g for g in waits if waits[g]()]
             choices = [(g, weight[g]) for g in ready]
             choices += [("copy", 40 / lazy_copies)] if self.flying else []
@@ -286,6 +310,8 @@ class Model:
                     del waits[pick]
         for r in self.ranks:
             self.check(len(self.done_tiles[r]) == EPI, "an epilogue warp did not finish")
+            if self.kept[r]:
+                self.meet(r)   # (nothing has written there since)
 
 
 def _plans():
@@ -315,11 +341,19 @@ def test_every_order_of_the_roles_keeps_units_apart(m, group, cfg):
         Model(rng, cfg, rng.randint(1, 40), ku, first=rng.randint(0, 2 * ku)).run()
 
 
+@pytest.mark.parametrize("m,group,cfg", [p for p in PLANS if not p[2]["defer"]], ids=[f"{m} rows, group {g}" for m, g, c in PLANS if not c["defer"]])
+def test_a_last_tile_may_stay_in_its_accumulators(m, group, cfg):
+    for seed in range(12):
+        rng = random.Random(1000 + seed)
+        ku = rng.choice([2, 3, 5, 8, 64])
+        Model(rng, cfg, rng.choice([rng.randint(1, 40), ku + 1, 2 * ku + 1, ku + 2]), ku, first=rng.choice([0, 0, rng.randint(0, 2 * ku)]), early=True).run()
+
+
 def _found(cfg, **kw):
     for seed in range(300):
         rng = random.Random(seed)
         try:
-            Model(rng, cfg, 40, 64, **kw).run()
+            Model(rng, cfg, 40, 64 if "early" not in kw else 9, **kw).run()
         except Wrong:
             return True
     return False
@@ -330,3 +364,6 @@ def test_the_model_sees_what_the_rules_prevent():
     short = dict(w=3, x=3, a=3, n_mma=1, d=1, defer=False, pair=True)
     assert _found(short, a_first=False) and not _found(short)
     assert _found(dict(w=5, x=8, a=4, n_mma=2, d=2, defer=False, pair=False), a_first=False)
+    # a last tile that is taken without waiting for its products
+    even = plan(64, 128)
+    assert _found(even, early=True, early_before_products=True) and not _found(even, early=True)
