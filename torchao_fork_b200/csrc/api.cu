@@ -1,5 +1,6 @@
 // C-ABI entry points that dispatch between kernels + misc.
 #include "common.cuh"
+#include "gemv_stage.cuh"
 
 namespace ao {
 int int4_gemv(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np,
@@ -90,9 +91,9 @@ int settled_follow() { return tunables().pdl ? ao::kFollowSettled : ao::kFollowP
 // costs about 10 us of staging, launch and tail whatever the size, then streams 16 rows as fast as 3; the GEMV has no such costs but
 // its time grows with the rows.  Measured (GEMV / GEMM, us): int4 28672 x 8192, 8 rows 39 / 46, 12 rows 62 / 46; 14336 x 4096, 8 rows 14 / 20,
 // 12 rows 19.7 / 20.3, 16 rows 23.0 / 20.4; int8 28672 x 8192, 8 rows 51 / 50, 12 rows 66 / 50, 14336 x 4096, 16 rows 25.9 / 22.7; a tie at
-// 4096 x 4096, 16 rows, where the line puts the GEMV.  Where the activations do not fit, the strip kernels are the other choice: int4
-// 8192 x 28672 62 .. 63 / 45 from 3 to 16 rows, 4096 x 14336, 16 rows 18 / 20; int8 8192 x 28672, 3 / 8 / 16 rows 55 / 59 / 78 against 49 .. 51,
-// 4096 x 14336, 8 rows 18 / 23, 12 rows 27 / 23.
+// 4096 x 4096, 16 rows, where the line puts the GEMV.  Where the activations do not fit one CTA, up to 8 rows share k over a cluster if that takes them
+// (share_k, which is asked first); for the others, 9 to 16 rows as a rule, the strip kernels are the other choice: int4 8192 x 28672 62 .. 63 / 45 from 3 to 16
+// rows, 4096 x 14336, 16 rows 18 / 20; int8 8192 x 28672, 16 rows 78 / 51, 4096 x 14336, 12 rows 27 / 23.
 static bool few_rows_by_gemm(int64_t M, int64_t Np, int64_t Kp, bool fits, bool int4) {
   if (M < 3 || Np % 128 != 0) return false;
   if (M > 16) return true;
@@ -129,7 +130,7 @@ extern "C" int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
   auto s = static_cast<cudaStream_t>(stream);
   auto xb = static_cast<const __nv_bfloat16*>(x);
   auto yb = static_cast<__nv_bfloat16*>(y);
-  if (M >= 3 && M <= 8 && !ao::int4_gemv_fused_fits(M, Kp, group_size, tunables().stages)) {   // too long for one CTA: k shared out (as in ao_b200_mm_residual)
+  if (ao::share_k(M, Kp, ao::Instead::kNothingFits) && !ao::int4_gemv_fused_fits(M, Kp, group_size, tunables().stages)) {
     const int e = ao::int4_gemv_split(x, M, Kx, ldx, packed, scale_and_zero, Np, Kp, group_size, y, N_out, ldy, nullptr, 0, tunables().stages,
                                       plain_follow(), s);
     if (e != AO_B200_ERR_WORKSPACE) return e;
@@ -232,7 +233,7 @@ extern "C" int ao_b200_int8_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
   auto s = static_cast<cudaStream_t>(stream);
   auto xb = static_cast<const __nv_bfloat16*>(x);
   auto yb = static_cast<__nv_bfloat16*>(y);
-  if (M >= 3 && M <= 8 && !ao::int8_gemv_fused_fits(M, Kp, tunables().stages)) {   // too long for one CTA: k shared out (as in ao_b200_mm_residual)
+  if (ao::share_k(M, Kp, ao::Instead::kNothingFits) && !ao::int8_gemv_fused_fits(M, Kp, tunables().stages)) {
     const int e = ao::int8_gemv_split(x, M, Kx, ldx, packed, scale, Kp, y, N_out, ldy, nullptr, 0, tunables().stages, plain_follow(), s);
     if (e != AO_B200_ERR_WORKSPACE) return e;
   }
@@ -264,7 +265,7 @@ extern "C" int ao_b200_int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int
                              epilogue, tunables().stages, settled_follow(), static_cast<cudaStream_t>(stream));
 }
 
-// ---- y = bf16(residual + bf16(x W'^T)) for any number of rows, always by the GEMM ----------------------------------------
+// ---- y = bf16(residual + bf16(x W'^T)) for any number of rows: by the GEMM, a few rows of long k by the GEMV over clusters ----------------------------------------
 extern "C" int64_t ao_b200_mm_residual_workspace_bytes(int64_t M, int64_t Np, int64_t Kp, int group_size) {
   return group_size ? ao::int4_gemm_tc_workspace_bytes(M, Np, Kp) : ao::int8_gemm_tc_workspace_bytes(M, Np, Kp);
 }
@@ -277,11 +278,9 @@ extern "C" int ao_b200_mm_residual(const void* x, int64_t M, int64_t Kx, int64_t
   AO_CHECK_ARG(ao_aligned(x, 16) && ao_aligned(packed, 16) && ao_aligned(scales, group_size ? 64 : 2) && ao_aligned(y, 2) && ao_aligned(residual, 2));
   AO_CHECK_ARG(group_size == 0 || Kp % group_size == 0);
   auto s = static_cast<cudaStream_t>(stream);
-  // Few rows of long k: the GEMV with k shared out over a cluster stages the activations itself (8 rows of 4096 x 14336: int8 16.3 us against 22.4,
-  // int4 14.5 against 21.8; 3072 x 8192 8.8 against 17.6).  Shorter k (28672 x 4096, int8: 36 against 30) and more rows are the GEMM's; what the GEMM
-  // refuses stays refused.
+  // what the GEMM refuses stays refused
   const int64_t need = ao_b200_mm_residual_workspace_bytes(M, Np, Kp, group_size);
-  if (M <= 8 && Kp >= 8192 && need > 0 && workspace != nullptr && workspace_bytes >= need) {
+  if (ao::share_k(M, Kp, ao::Instead::kGemm) && need > 0 && workspace != nullptr && workspace_bytes >= need) {
     const int e = group_size ? ao::int4_gemv_split(x, M, Kx, ldx, packed, scales, Np, Kp, group_size, y, N_out, ldy, residual, ld_res, tunables().stages,
                                                    settled_follow(), s)
                              : ao::int8_gemv_split(x, M, Kx, ldx, packed, scales, Kp, y, N_out, ldy, residual, ld_res, tunables().stages, settled_follow(), s);

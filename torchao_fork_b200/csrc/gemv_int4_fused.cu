@@ -337,10 +337,12 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
       X_s[(sg * 2 + 0) * 8 * MT + m] = sum[1];
       X_s[(sg * 2 + 1) * 8 * MT + m] = -fmaf(1024.f, sum[0], 8.f * sum[1]);
     };
+    const __nv_bfloat16* own_x = p.x + (int64_t)rank * KT * 64;     // SPLIT: this CTA's part of k
+    const int64_t own_k = SPLIT ? min(p.Kx - (int64_t)rank * KT * 64, (int64_t)KT * 64) : p.Kx;
 #pragma unroll
     for (int row0 = 0; row0 < HR; row0 += 8)
-      stage_rows<(HR < 8 ? HR : 8), NH, kCT, 2, SEG>(p.x + (int64_t)rank * KT * 64, p.ldx, SPLIT ? min(p.Kx - (int64_t)rank * KT * 64, (int64_t)KT * 64) : p.Kx, row0, p.M, p.norm_w, p.eps, chunks_per_row, x_s, p.x_row_bytes, part, row_scale, chunk,
-                                                     done);
+      stage_rows<(HR < 8 ? HR : 8), NH, kCT, 2, SEG>(own_x, p.ldx, own_k, row0, p.M, p.norm_w, p.eps, chunks_per_row, x_s, p.x_row_bytes, part, row_scale, chunk,
+                                                    done);
   } else {
     // rows in batches of four: the four activation loads of a thread are in flight together (one exposed L2 round trip
     // per batch instead of one per row)
@@ -807,7 +809,7 @@ int int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   p.n_strips = (int)(Np / 16);
   p.eps = eps;
   const int MT = M <= 8 ? 1 : 2;
-  if (norm_w == nullptr && epilogue != kEpiSiluMul && long_activations(M, Kp) && int4_gemv_fused_fits(M, Kp, G, max_stages)) {
+  if (norm_w == nullptr && epilogue != kEpiSiluMul && share_k(M, Kp, Instead::kWholeRows) && int4_gemv_fused_fits(M, Kp, G, max_stages)) {
     const int e = int4_gemv_split(x, M, Kx, ldx, packed, sz, Np, Kp, G, y, N_out, ldy, epilogue == kEpiResidual ? residual : nullptr, ld_res, max_stages, follow, s);
     if (e != AO_B200_ERR_WORKSPACE) return e;
   }

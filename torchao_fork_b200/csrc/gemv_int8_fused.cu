@@ -84,7 +84,8 @@ __device__ __noinline__ float4 again8(const uint8_t* w, const __nv_bfloat16* x, 
 }
 
 // HR = 1: M = 1 and every consumer thread owns <= NH chunks of the activation row (register-held staging); HR = 4, 8, 16: up to
-// HR rows of <= NH chunks in registers (gemv_stage.cuh); HR = 0: the general staging.  One instantiation per case — the staging code runs once per launch with a cold instruction cache, so
+// HR rows of <= NH chunks in registers (gemv_stage.cuh); HR = 0: the general staging.  One instantiation per case — the staging code runs
+// once per launch with a cold instruction cache, so
 // code that a launch does not need is not compiled into its kernel (profiles/r01c_imma_code_size_ab.txt).
 __device__ __forceinline__ uint32_t mul_bf16x2_8(uint32_t a, uint32_t b) {
   uint32_t d;
@@ -277,9 +278,11 @@ __global__ void __launch_bounds__(k8Threads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
                         *reinterpret_cast<const uint32_t*>(&h3));
     };
     const auto done = [&](int seg, int m, const float (&sum)[1]) { C_s[seg * 8 * MT + m] = -1152.f * sum[0]; };
+    const __nv_bfloat16* own_x = p.x + (int64_t)rank * KT * 64;     // SPLIT: this CTA's part of k
+    const int64_t own_k = SPLIT ? min(p.Kx - (int64_t)rank * KT * 64, (int64_t)KT * 64) : p.Kx;
 #pragma unroll
     for (int row0 = 0; row0 < HR; row0 += 8)
-      stage_rows<(HR < 8 ? HR : 8), NH, kCT, 1, 64>(p.x + (int64_t)rank * KT * 64, p.ldx, SPLIT ? min(p.Kx - (int64_t)rank * KT * 64, (int64_t)KT * 64) : p.Kx, row0, p.M, p.norm_w, p.eps, chunks_per_row, x_s, p.x_row_bytes, part, row_scale, chunk,
+      stage_rows<(HR < 8 ? HR : 8), NH, kCT, 1, 64>(own_x, p.ldx, own_k, row0, p.M, p.norm_w, p.eps, chunks_per_row, x_s, p.x_row_bytes, part, row_scale, chunk,
                                                     done);
   } else if constexpr (hold) {
     float ss = 0.f, amax = 0.f;
@@ -666,12 +669,12 @@ int int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const voi
   p.x_row_bytes = pl.x_row_bytes;
   p.off_x = pl.off_x; p.off_C = pl.off_C; p.off_red = pl.off_red; p.off_misc = pl.off_misc;
   p.ks = 1, p.off_inbox = 0;
-  // Rows in registers: chunks of 8 activations per consumer thread and row.  M = 1: <= 4 (Kp <= 16384).  More rows: up to 16 chunks in all,
-  // which leaves registers for one CTA per SM only from 8 on, so where two fit the shared memory (short rows) at most 4.
-  if (norm_w == nullptr && epilogue != k8EpiSiluMul && long_activations(M, Kp)) {
+  if (norm_w == nullptr && epilogue != k8EpiSiluMul && share_k(M, Kp, Instead::kWholeRows)) {
     const int e = int8_gemv_split(x, M, Kx, ldx, packed, scale, Kp, y, N_out, ldy, epilogue == k8EpiResidual ? residual : nullptr, ld_res, max_stages, follow, s);
     if (e != AO_B200_ERR_WORKSPACE) return e;
   }
+  // Rows in registers: chunks of 8 activations per consumer thread and row.  M = 1: <= 4 (Kp <= 16384).  More rows: up to 16 chunks in all,
+  // which leaves registers for one CTA per SM only from 8 on, so where two fit the shared memory (short rows) at most 4.
   const int n_iter = (p.KT * 8 + k8Consumers * 32 - 1) / (k8Consumers * 32);
   if (MT == 2) return n_iter <= 1 ? launch8<2, 1, 16>(p, pl, follow, s) : launch8<2, 0, 0>(p, pl, follow, s);
   if (M == 1 && n_iter <= 1) return launch8<1, 1, 1>(p, pl, follow, s);

@@ -9,6 +9,7 @@
 // reference has op boundaries (W * scale, + zero, ...), i.e. the reference's CPU path; its CUDA path runs the same
 // iteration in fp16, which this does not imitate.  The result feeds the same packed format as the tinygemm recipe.
 #include "common.cuh"
+#include "f32x2.h"
 
 namespace ao {
 
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(kHqqWarps * 32) hqq_finalize_kernel(const __nv
 // Bound by the fp32 pipe and instruction issue: ten iterations over 4096 x 4096 take about 80 us.  What keeps the arithmetic at eleven
 // instructions per pair of weights and iteration:
 //  - pairs of weights in one register pair (add, mul, fma .f32x2: the single operation's rounding in each half.  But a product whose one use is a sum
-//    can come out as one fused operation, .rn or not, so such a sum is a fused one already, with a factor of one);
+//    can come out as one fused operation (f32x2.h), so such a sum is a fused one already, with a factor of one);
 //  - the group's smallest and largest weight bound every |d| and say whether anything is clamped, so that, as a rule, neither
 //    the clamp nor the shrinkage is looked at per weight.  |d| - c |d|^(p - 1) is not positive for |d| <= c^(1 / (2 - p)) (p < 1), 0.17 at the
 //    reference's constants, which is above most weights' error: powf runs only above that threshold (less a margin of 1e-3, thousands of
@@ -174,36 +175,6 @@ __device__ __forceinline__ int hqq_last(const double* __restrict__ mean, int n, 
 __device__ __noinline__ float hqq_shrink(float d, float c, float lp_m1) {
   const float ad = fabsf(d);
   return copysignf(fmaxf(__fsub_rn(ad, __fmul_rn(c, powf(ad, lp_m1))), 0.f), d);
-}
-
-// two fp32 in one register pair: one instruction for both, each with the single operation's rounding (see above for a product that is added)
-struct F2 {
-  uint64_t v;
-};
-__device__ __forceinline__ F2 f2(float a, float b) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 f2_get(F2 x) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
-  F2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
-  F2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-  F2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return r;
 }
 
 // sum of leaf(i) over the pairs of lanes i, i + O, i + 2 O, .. < I in the order of a tree whose last step adds neighbours O apart; leaf gives

@@ -25,6 +25,7 @@
 // 128), two chains per SM beside one another; a CTA's start and end (queries, the peers' shares) cost 9000 more.  2048 rows x 16 heads of 128
 // (four key heads): 59.5 us, against 308 us of window_attention_prompt_kernel; the same with all keys of a tile in one CTA 110 us (the last
 // tiles alone took 95), with unswizzled operands 84 us.
+#include "../f32x2.h"
 #include "../per_device.h"
 #include "lm_mma.cuh"
 #include "lm_window_attention.cuh"
@@ -124,30 +125,11 @@ __device__ __forceinline__ void tc_st8(uint32_t a, const uint32_t (&d)[8]) {
                : "memory");
 }
 __device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// two fp32 side by side, one instruction for both, each rounded as by itself
-struct F2 {
-  uint64_t v;
-};
-__device__ __forceinline__ F2 f2(float a, float b) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 f2_get(F2 x) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
-  F2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-  F2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return r;
-}
+using ao::F2;
+using ao::f2;
+using ao::f2_add;
+using ao::f2_fma;
+using ao::f2_get;
 __device__ __forceinline__ float tc_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
