@@ -489,7 +489,7 @@ def run_b200(args):
         line["standalone_gemv_kernels"] = {"per_shape": standalone, "all_layers": {"gbs": b_all / t_all / 1e9, "frac": b_all / t_all / 1e9 / peak},
                                            "how": "each linear's own kernel launched back to back over the 32 layers' weights in a CUDA graph (PDL chain), CUDA events"}
         if "wo" in standalone and standalone["wo"]["n"] == 4096 and standalone["wo"]["k"] == 4096:
-            line["config1"] = dict(standalone["wo"], workload="single Linear 4096x4096, Int4WeightOnlyConfig(group_size=128), M=1 (BASELINE.json configs[0])")
+            line["config1"] = dict(standalone["wo"], workload="single Linear 4096x4096, Int4WeightOnlyConfig(group_size=128), M=1")
         traffic = None
         tp_path = os.path.join(ROOT, "profiles", "traffic.json")
         tr = json.load(open(tp_path)) if os.path.exists(tp_path) else {}
@@ -571,7 +571,7 @@ def run_b200(args):
                                      timeout=600, env={k: v for k, v in os.environ.items() if k not in ("RANK", "WORLD_SIZE", "LOCAL_RANK")})
                 ref_line = json.loads([l for l in out.stdout.splitlines() if l.startswith("{")][-1])
                 line["cpu_baseline"] = ref_line["cpu_baseline"]
-            except Exception as e:  # the checker is optional at run time; the product path is not
+            except Exception as e:  # the oracle is optional at run time; the product path is not
                 line["cpu_baseline"] = {"value": None, "unit": "tok/s", "cores": 0, "kind": "reference",
                                         "sample": f"unavailable: {type(e).__name__}: {e}"}
         emit(line)

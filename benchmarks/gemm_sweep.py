@@ -1,4 +1,4 @@
-"""BASELINE.json config 5: int4 / int8 weight-only GEMM sweep, M in {1, 16, 128, 1024, 4096} over the ten Llama-3 8B / 70B
+"""int4 / int8 weight-only GEMM sweep, M in {1, 16, 128, 1024, 4096} over the ten Llama-3 8B / 70B
 (N, K) shapes, through the public ops (torchao::b200_int4_weight_only_mm / b200_int8_weight_only_mm — what F.linear on a
 quantized weight dispatches to).  One CSV row per (dtype, M, N, K):
 

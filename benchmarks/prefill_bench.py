@@ -1,4 +1,4 @@
-"""BASELINE.json config 3 (second half): the 2048-token prefill of Llama-3-8B through the model, end to end
+"""The 2048-token prefill of Llama-3-8B through the model, end to end
 (reference: torchao/_models/llama/generate.py:103-108 `prefill` = one eager forward over the prompt + sampling).
 Linears run the tcgen05 dequant-GEMM (csrc/gemm_wq_tc.cu, int4 and int8 instantiations); attention is torch SDPA,
 norms / RoPE torch ops, as in the reference.  Prints one JSON line per workload:

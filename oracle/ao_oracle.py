@@ -1,7 +1,7 @@
 """CPU oracle for the weight-only quantized linear path (TEST INFRASTRUCTURE ONLY).
 
-This file is a numpy restatement of the reference algorithm.  It is the checker
-for the CUDA kernels; it is never the product.  Only ``tests/``,
+This file is a numpy restatement of the reference algorithm.  The CUDA
+kernels are compared with it; it is never the product.  Only ``tests/``,
 ``__graft_entry__.smoke()`` and ``bench.py``'s ``cpu_baseline`` / ``--impl
 reference`` legs may import it.
 
@@ -487,7 +487,7 @@ def kv_cache_update(cache, cache_scale, pos, val, div_mode="ieee"):
 
 # --------------------------------------------------------------------------
 # Int4Tensor (row N3): fbgemm-gpu-genai's int4_row_quantize_zp + pack_int4, restated
-# (third-party, absent from /root/reference: fbgemm_gpu/experimental/gen_ai/quantize.py, >= 1.2.0 as required by
+# (third-party, absent from the reference's tree: fbgemm_gpu/experimental/gen_ai/quantize.py, >= 1.2.0 as required by
 # torchao/quantization/quantize_/workflows/int4/int4_tensor.py:22-26,71-73) -- parity with fbgemm itself is UNPINNED.
 # --------------------------------------------------------------------------
 def int4_row_quantize_zp(w, group_size, div_mode="ieee"):

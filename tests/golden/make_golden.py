@@ -1,7 +1,6 @@
 """Generate tests/golden/*.npz by running the REFERENCE's own Python functions on CPU.
 
-Run in the build container only (needs /root/reference, which does not exist on
-the GPU box):
+Run where the reference's tree is (/root/reference):
 
     PYTHONPATH=/root/reference python tests/golden/make_golden.py
 

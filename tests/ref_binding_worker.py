@@ -2,7 +2,7 @@
 the integration guide describes — ctypes-load libao_b200.so, CUDA backends for the reference's own
 `torchao::unpack_tensor_core_tiled_layout` / `dequantize_tensor_core_tiled_layout` schemas (torchao/ops.py:16-21), the
 int4 layout's `from_plain` and linear impl routed to the strip-major kernels — and then runs the checks of the
-reference's own tests (restated from /root/reference/test/test_ops.py:282-467, which does not travel to the GPU box)
+reference's own tests (restated from test/test_ops.py:282-467, which is not part of its installed package)
 against it.  Test infrastructure, run in a process of its own:
 
     PYTHONPATH=oracle/_ref python tests/ref_binding_worker.py <path to libao_b200.so> <out.json>

@@ -1,4 +1,4 @@
-"""Runs the UNMODIFIED reference (oracle/_ref = pip install --target of /root/reference) on the GPU, in a process of its
+"""Runs the UNMODIFIED reference (oracle/_ref = pip install --target of its tree) on the GPU, in a process of its
 own (the reference and this repo both own the `torchao::` op namespace).  Test infrastructure, not a test:
 
     PYTHONPATH=oracle/_ref python tests/ref_worker.py <mode> <in.pt> <out.pt>

@@ -60,7 +60,7 @@ def _edge(n, k, g):
     return w
 
 
-SHAPES = [(4096, 4096), (6144, 4096), (14336, 4096), (4096, 14336)]   # BASELINE.json: Llama-3-8B (N, K)
+SHAPES = [(4096, 4096), (6144, 4096), (14336, 4096), (4096, 14336)]   # Llama-3-8B (N, K)
 
 
 def _weights():
@@ -138,7 +138,7 @@ def test_int8_quantize_and_linear_match_the_reference_running_on_the_gpu():
 
 @pytest.mark.parametrize("mega", [True, False])
 def test_llama_decode_matches_the_reference_transformer(mega):
-    """Row a16: reference model.py / generate.py semantics as the checker.  Same bf16 weights, both sides quantize with
+    """Row a16: reference model.py / generate.py semantics as the oracle.  Same bf16 weights, both sides quantize with
     their own quantize_ (bit-identical integers, test above), same prompt; every decode step is fed the REFERENCE's
     token.  Logits: SQNR >= 35 dB per step (bf16 logits; the kernels differ in summation order and in where the
     dequantised weight is rounded), argmax identical wherever the reference's top-2 margin exceeds 0.25."""

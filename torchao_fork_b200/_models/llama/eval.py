@@ -1,7 +1,7 @@
 """Perplexity evaluation of the gpt-fast Llama on the B200 weight-only path.
 
 The reference evaluates through lm-evaluation-harness (torchao/_models/llama/eval.py:33-236 `run_evaluation`,
-torchao/_models/_eval.py:29-126 `TransformerEvalWrapper`): third-party, absent from /root/reference and from this image,
+torchao/_models/_eval.py:29-126 `TransformerEvalWrapper`): third-party, absent from the reference's tree and from this image,
 and its task data (wikitext) needs the network.  What the harness does for a perplexity task is restated here so that a
 token file is all it takes:
 

@@ -166,7 +166,7 @@ class Generator:
                 for i in range(n):
                     eng.graph_stream.replay()
                     # an event recorded behind the graph reaches the host sooner than the stream's own completion
-                    # (measured: ~50 us per token less for the one-kernel graph, benchmarks/e2e_probe2.py)
+                    # (measured: ~50 us per token less for the one-kernel graph)
                     done.record(stream)
                     done.synchronize()
                     callback(self.h_out)

@@ -27,39 +27,16 @@
 #include "common.cuh"
 #include "gemv_stage.cuh"
 
-#ifndef AO_CHAINS
-#define AO_CHAINS 2
-#endif
-#ifndef AO_STAGE_TILES
-#define AO_STAGE_TILES 32
-#endif
-#ifndef AO_EXP
-#define AO_EXP 0  // benchmarks/gemv_trace.cu ablations only
-#endif
-
 namespace ao {
 
 constexpr int kFConsumers = 16;
 constexpr int kFThreads = (kFConsumers + 2) * 32;  // + TMA producer warp + epilogue warp
 constexpr int kRedBufs = 2;                       // partial-sum buffers between the consumers and the epilogue warp
-constexpr int kStageTiles = AO_STAGE_TILES;  // k-tiles (of 64 k) per stage: 16 KB of weights per 32
+constexpr int kStageTiles = 32;              // k-tiles (of 64 k) per stage: 16 KB of weights
+constexpr int kMostChains = 2;               // accumulators of a segment
 constexpr int kTilesPerWarp = kStageTiles / kFConsumers;  // 2 k-tiles = 128 k per warp per stage
 
 enum { kEpiPlain = 0, kEpiResidual = 1, kEpiSiluMul = 2 };
-
-// AO_GEMV_TRACE (benchmarks/gemv_trace.cu only): per-warp, per-stage SM clock stamps of one CTA
-#ifdef AO_GEMV_TRACE
-constexpr int kTraceIts = 256, kTraceKinds = 6;
-__device__ long long ao_trace[kTraceKinds][kFConsumers + 2][kTraceIts];
-__device__ int ao_trace_cta = 0;
-#define AO_TRACE(kind, it)                                                                  \
-  do {                                                                                      \
-    if ((int)blockIdx.x == ao_trace_cta && (threadIdx.x & 31) == 0 && (it) < kTraceIts)     \
-      ao_trace[kind][threadIdx.x >> 5][it] = clock64();                                     \
-  } while (0)
-#else
-#define AO_TRACE(kind, it) do { } while (0)
-#endif
 
 struct GemvFusedParams {
   const uint8_t* packed;      // strip-major [Np/16][Kp/64][512 B]
@@ -154,7 +131,6 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
   uint64_t* red_free = red_full + kRedBufs;                            // [2]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  AO_TRACE(5, 0);
   const int stages = p.stages;
   const int ks = SPLIT ? p.ks : 1, rank = SPLIT ? blockIdx.x % ks : 0;
   const int b = SPLIT ? blockIdx.x / ks : blockIdx.x;
@@ -167,7 +143,6 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
   // barrier 2 only when they first need an mbarrier (after the activation staging), so the first stages are in
   // flight while the kernel is still waiting for its predecessor (PDL) and staging x.
   grid_launch_dependents();
-  AO_TRACE(5, 1);
   uint64_t* in_full = reinterpret_cast<uint64_t*>(smem + p.off_inbox);                                   // SPLIT, rank 0: [strips]
   float4* inbox = reinterpret_cast<float4*>(smem + p.off_inbox + kMaxSplitStrips * 8);                   // [strips][ks - 1][MT][32 lanes]
   if constexpr (SPLIT) split_begin(warp == kFConsumers + 1 && rank == 0, s1 - s0, in_full, (uint32_t)((ks - 1) * MT * 512), lane);
@@ -206,9 +181,7 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
           const int n_grp = cnt * 64 / G;
           uint8_t* wdst = ring + (size_t)slot * kStageB;
           if (lane == 0) {
-            AO_TRACE(0, (strip - s0) * n_chunks + ch);
             mbar_wait(&empty[slot], par);
-            AO_TRACE(1, (strip - s0) * n_chunks + ch);
             mbar_arrive_expect_tx(&full[slot], (uint32_t)(cnt * 512 + n_grp * 64));
             bulk_g2s(wdst + kStageTiles * 512, srow + (int64_t)(kt0 * 64 / G) * 16, (uint32_t)(n_grp * 64), &full[slot]);
           }
@@ -252,7 +225,6 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
         res[i >> 2][(i >> 1) & 1][i & 1] = p.epilogue == kEpiResidual && m < p.M && n < p.N_out ? p.residual[m * p.ld_res + n] : __float2bfloat16_rn(0.f);
       }
       mbar_wait(&red_full[rbuf], use & 1u);
-      AO_TRACE(4, li);
       float4 sum[MT];
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
@@ -305,7 +277,6 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
           }
         }
       }
-      AO_TRACE(5, li);
     }
     return;
   }
@@ -315,7 +286,6 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
   const int tid = threadIdx.x;  // 0 .. 511
   constexpr int kCT = kFConsumers * 32;
   if constexpr (HR == 0) grid_dependency_wait();
-  AO_TRACE(5, 2);
 
   // ---- stage the activations: x (* norm_w) -> per-row power-of-two scaling -> fp16, the entries that meet a
   //      "1024 + 16 q" weight pre-divided by 16; then the per-segment correction sums ----
@@ -391,7 +361,6 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
       }
     }
     named_bar_sync(1, kCT);
-    AO_TRACE(5, 3);
     if (warp < p.M) {
       // warp w finishes row w: 16 (sum sq, amax) partials -> 2^e and the epilogue scale
       float t = 0.f, amax = 0.f;
@@ -412,7 +381,6 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
       }
     }
     named_bar_sync(1, kCT);
-    AO_TRACE(5, 4);
     // rescale to fp16 and, in the same pass, the per-segment correction sums: a segment is SEG / 8 consecutive chunks
     // = SEG / 8 consecutive lanes.  X[seg][m] = sum of the scaled activations, C[seg][m] = 1024 * (sum of the STORED
     // values) + 8 * X, stored negated:  sum_k x_k (q_k - 8) = (MMA result) - C  ->  the accumulator starts at -C.
@@ -448,8 +416,6 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
         }
       }
     }
-    AO_TRACE(5, 5);
-    AO_TRACE(5, 6);
   }
   named_bar_sync(2, kFThreads);  // the producer has initialised the mbarriers (long ago)
 
@@ -494,7 +460,7 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     for (int t = 0; t < kTilesPerWarp; ++t) wv[t] = lds128(stage_u + w_off_r + t * 512u);
     // kChains independent accumulators per segment: back-to-back mma.sync on ONE accumulator serialise on the HMMA
     // latency (~50 clk under load: removing the MMAs altogether took the kernel from 82 to 56 us)
-    constexpr int kChains = (2 * U32 < AO_CHAINS) ? 2 * U32 : AO_CHAINS;
+    constexpr int kChains = 2 * U32 < kMostChains ? 2 * U32 : kMostChains;
     float acc[kChains][MT][4];
 #pragma unroll
     for (int t = 0; t < kTilesPerWarp; ++t) {
@@ -507,12 +473,8 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
         const int j0 = (2 * (q32 % U32)) % kChains, j1 = (2 * (q32 % U32) + 1) % kChains;
         const uint32_t wl = words[2 * h], wh = words[2 * h + 1];  // rows g and g + 8
         const uint32_t wl8 = wl >> 8, wh8 = wh >> 8;
-#if AO_EXP == 2
-        const uint32_t a0l = wl, a1l = wl, a2l = wl8, a3l = wl8, a0h = wh, a1h = wh, a2h = wh8, a3h = wh8;
-#else
         const uint32_t a0l = nib_f16_lo(wl), a1l = nib_f16_hi(wl), a2l = nib_f16_lo(wl8), a3l = nib_f16_hi(wl8);
         const uint32_t a0h = nib_f16_lo(wh), a1h = nib_f16_hi(wh), a2h = nib_f16_lo(wh8), a3h = nib_f16_hi(wh8);
-#endif
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) {
           if (x_on[mt]) xx[mt] = lds128(x_u0[mt] + xo + q32 * 64);
@@ -529,13 +491,8 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[j1][mt][e] = 0.f;
           }
-#if AO_EXP == 1
-          asm volatile("" ::"r"(a0l), "r"(a0h), "r"(a1l), "r"(a1h), "r"(a2l), "r"(a2h), "r"(a3l), "r"(a3h), "r"(xx[mt].x),
-                       "r"(xx[mt].y), "r"(xx[mt].z), "r"(xx[mt].w));
-#else
           mma_f16_16816(acc[j0][mt], a0l, a0h, a1l, a1h, xx[mt].x, xx[mt].y);
           mma_f16_16816(acc[j1][mt], a2l, a2h, a3l, a3h, xx[mt].z, xx[mt].w);
-#endif
         }
         if (q32 % U32 == U32 - 1) {
           // segment complete: y += s * acc + z * X   (fp32)
@@ -572,11 +529,7 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
 
     uint32_t xo = 0, X_u = X_u0_r;
     for (int ch = 0; ch < n_chunks; ++ch) {
-      AO_TRACE(0, (strip - s0) * n_chunks + ch);
-#if AO_EXP != 3 && AO_EXP != 5
       mbar_wait(&full[slot], par);
-#endif
-      AO_TRACE(1, (strip - s0) * n_chunks + ch);
       if (ch < n_full) {
         consume(std::true_type{}, kStageTiles, xo, X_u, yacc);
       } else if (tl0 < KT - ch * kStageTiles) {
@@ -584,7 +537,6 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[slot]);
-      AO_TRACE(2, (strip - s0) * n_chunks + ch);
       xo += kStageTiles * 128u;
       X_u += kXChunk;
       stage_u += kStageB;
@@ -598,16 +550,11 @@ __global__ void __launch_bounds__(kFThreads, (MT == 1 && HR * NH < 8 ? 2 : 1)) i
     // ---- strip done: the 16 partials go to shared memory and the warp goes straight on to the next strip; the
     //      epilogue warp sums them.  (A consumer doubling as the reducer falls behind by the reduction, the next
     //      reducer has to wait for it, and the lag chains: strip time became compute + reduce, 2700 clk.) ----
-#if AO_EXP == 4 || AO_EXP == 5
-    if (yacc[0][0] == 123.456f) p.y[strip] = __float2bfloat16_rn(yacc[0][1] + yacc[0][2] + yacc[0][3]);
-    continue;
-#endif
     const int li = strip - s0;
     const int rbuf = li % kRedBufs;
     const uint32_t use = (uint32_t)(li / kRedBufs);  // n-th use of this buffer
     float* rb = red + (size_t)rbuf * (kFConsumers * MT * 128);
     if (use > 0) mbar_wait(&red_free[rbuf], (use - 1) & 1u);  // the epilogue of kRedBufs strips ago has read it
-    AO_TRACE(3, li);
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
       *reinterpret_cast<float4*>(rb + ((warp * MT + mt) * 32 + lane) * 4) =

@@ -10,7 +10,7 @@
 // is EXACT in int32, and  sum_k x (q - 8) = 2^e ( D2 * 65536 + D1 * 256 + D0 - 8 * sum_k xi ).  What is left per packed
 // word (8 weights) on the CUDA cores is one shift and two lop3 (nibbles -> bytes), a quarter of a shared-memory load and
 // a quarter of a tensor-memory store: ~4 issue slots against ~14 for the mma.sync kernel (gemv_int4_fused.cu), whose
-// ALU pipe is what caps it at ~70 % of HBM peak.  (Measured, benchmarks/tc_probe.cu: kind::i8 M128 N<=64 K32 with A in
+// ALU pipe is what caps it at ~70 % of HBM peak.  (Measured: kind::i8 M128 N<=64 K32 with A in
 // TMEM retires one MMA per 45 clocks = 2 KB of int4 per 45 clocks per SM = 13 TB/s; 16x128b tensor-memory stores run at
 // 480 B/clk/SM.)
 //
@@ -38,18 +38,6 @@ constexpr int kTcStageK = kTcStageTiles * 64;
 constexpr int kTcABufs = 3;                        // TMEM A ring: 128 columns (512 k of int8) per buffer
 constexpr int kTcDBufs = 8;                        // TMEM accumulator ring: N columns per buffer
 constexpr int kTcLimbs = 3;
-
-#ifdef AO_TC_TRACE
-constexpr int kTcTraceIts = 128;
-__device__ long long ao_tc_trace[6][kTcMmaWarp + 1][kTcTraceIts];
-#define TC_TRACE(kind, it)                                                              \
-  do {                                                                                  \
-    if (blockIdx.x == 0 && (threadIdx.x & 31) == 0 && (it) < kTcTraceIts)               \
-      ao_tc_trace[kind][threadIdx.x >> 5][it] = clock64();                              \
-  } while (0)
-#else
-#define TC_TRACE(kind, it) do { } while (0)
-#endif
 
 struct GemvTcParams {
   const uint8_t* packed;      // strip-major [Np/16][Kp/64][512 B]
@@ -177,7 +165,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) int4_gemv_tc_kernel(const GemvT
   const int rb_first = u0 / n_chunks, w0 = u0 - rb_first * n_chunks;
   const int win_len = min(n_chunks, u1 - u0);
   grid_launch_dependents();
-  TC_TRACE(5, 0);
 
   if (warp == kTcMmaWarp) {
     // ---- barriers + tensor-memory allocation, then the other warps are let in (named barrier 2) ----
@@ -204,7 +191,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) int4_gemv_tc_kernel(const GemvT
   named_bar_sync(2, kTcThreads);  // barriers initialised, TMEM base published
   tc_fence_after();
   const uint32_t tb = *tmem_base_s;
-  TC_TRACE(5, 1);
   const uint32_t a_col0 = tb, d_col0 = tb + kTcABufs * 128;
 
   if (warp == kTcProducerWarp) {
@@ -216,7 +202,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) int4_gemv_tc_kernel(const GemvT
       const uint32_t par = ((uint32_t)(it / stages) & 1u) ^ 1u;
       const int cnt = min(kTcStageTiles, KT - ch * kTcStageTiles);
       uint8_t* dst = ring + (size_t)slot * kStageB;
-      TC_TRACE(0, it);
       if (lane == 0) {
         mbar_wait(&empty[slot], par);
         mbar_arrive_expect_tx(&full[slot], (uint32_t)(8 * cnt * 512));
@@ -227,7 +212,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) int4_gemv_tc_kernel(const GemvT
         bulk_g2s(dst + lane * (kTcStageTiles * 512), p.packed + (strip * KT + (int64_t)ch * kTcStageTiles) * 512,
                  (uint32_t)(cnt * 512), &full[slot]);
       }
-      TC_TRACE(1, it);
       if (++ch == n_chunks) { ch = 0; ++rb; }
     }
     __syncwarp();
@@ -244,10 +228,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) int4_gemv_tc_kernel(const GemvT
     for (int it = 0; it < u1 - u0; ++it) {
       const int abuf = it % kTcABufs;
       const int cnt = min(kTcStageTiles, KT - ch * kTcStageTiles);
-      TC_TRACE(0, it);
       mbar_wait(&a_full[abuf], (uint32_t)(it / kTcABufs) & 1u);
       tc_fence_after();
-      TC_TRACE(1, it);
       const uint32_t a_base = a_col0 + abuf * 128;
       const uint32_t x_base = xs_u + (uint32_t)lc * kXStage;
       const int n_grp = cnt * 2 / MPG;
@@ -269,7 +251,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) int4_gemv_tc_kernel(const GemvT
       }
       if (tc_elect_one()) tc_commit(&a_empty[abuf]);
       __syncwarp();
-      TC_TRACE(2, it);
       if (++ch == n_chunks) ch = 0;
       if (++lc == n_chunks) lc = 0;
     }
@@ -324,13 +305,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) int4_gemv_tc_kernel(const GemvT
     for (int it = 0; it < u1 - u0; ++it) {
       const int cnt = min(kTcStageTiles, KT - ch * kTcStageTiles);
       const int ngrp = cnt * 64 / G;
-      TC_TRACE(0, it);
       uint32_t szw[GPS];
 #pragma unroll
       for (int gl = 0; gl < GPS; ++gl) szw[gl] = sz_next[gl];
       const bool seg_end = (ch == n_chunks - 1) || (it == u1 - u0 - 1);
       if (it + 1 < u1 - u0) load_sz(ch + 1 < n_chunks ? rb : rb + 1, ch + 1 < n_chunks ? ch + 1 : 0, sz_next);
-      TC_TRACE(1, it);
 #pragma unroll
       for (int gl = 0; gl < GPS; ++gl) {
         if (gl >= ngrp) break;
@@ -355,7 +334,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) int4_gemv_tc_kernel(const GemvT
           yacc[m] = fmaf(s, val, fmaf(t, sxg[m], yacc[m]));
         }
       }
-      TC_TRACE(2, it);
       if (seg_end) {
         if (seg_ch0 == 0 && ch == n_chunks - 1) {
           finalize(rb, yacc);  // the whole K of this row block was ours
@@ -509,7 +487,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) int4_gemv_tc_kernel(const GemvT
           if (wi < n_win_chunks && (wi % CPG) == 0) sx[(size_t)(wi / CPG) * 8 + m] = (float)sum;
         }
       }
-      TC_TRACE(5, 2);
       fence_proxy_async();  // the B operand is read by the tensor core through the async proxy
       named_bar_arrive(3, kCT + 32 + kTcEpiWarps * 32);
     }
@@ -520,12 +497,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) int4_gemv_tc_kernel(const GemvT
     for (int it = 0; it < u1 - u0; ++it) {
       const int slot = it % stages, abuf = it % kTcABufs;
       const int cnt = min(kTcStageTiles, KT - ch * kTcStageTiles);
-      TC_TRACE(0, it);
       mbar_wait(&full[slot], (uint32_t)(it / stages) & 1u);
-      TC_TRACE(3, it);
       mbar_wait(&a_empty[abuf], ((uint32_t)(it / kTcABufs) & 1u) ^ 1u);
       tc_fence_after();
-      TC_TRACE(1, it);
       const uint32_t stage_u = ring_u + slot * kStageB;
 #pragma unroll
       for (int sh = 0; sh < 2; ++sh) {
@@ -550,7 +524,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) int4_gemv_tc_kernel(const GemvT
         mbar_arrive(&empty[slot]);
         mbar_arrive(&a_full[abuf]);
       }
-      TC_TRACE(2, it);
       if (++ch == n_chunks) ch = 0;
     }
   }

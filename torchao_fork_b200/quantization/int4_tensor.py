@@ -5,7 +5,7 @@ Mirror of torchao/quantization/quantize_/workflows/int4/int4_tensor.py:29-490: s
 3-D weights carry a leading batch dimension), same non-tensor attributes (`block_size`, `shape`), same ops
 (linear, bmm, slice with aliasing preserved, view, squeeze, detach / clone / to / copy_).
 
-The reference quantizes and multiplies through a third-party dependency that is NOT in /root/reference:
+The reference quantizes and multiplies through a third-party dependency that is NOT in its own tree:
 fbgemm-gpu-genai >= 1.2.0 (`fbgemm_gpu.experimental.gen_ai.quantize.int4_row_quantize_zp` / `pack_int4`,
 `torch.ops.fbgemm.bf16i4bf16_rowwise[_batched]`).  Their published algorithm is restated here:
 
