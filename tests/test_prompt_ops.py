@@ -80,3 +80,27 @@ def test_cache_rows_and_shared_heads_equal_the_single_operations(b, t, h, d, s, 
         assert torch.equal(ks, ref.k_cache.repeat_interleave(rep, dim=1)) and torch.equal(vs, ref.v_cache.repeat_interleave(rep, dim=1))
     kt, vt = ref.k_cache.transpose(1, 2), ref.v_cache.transpose(1, 2)
     assert all(torch.equal(x, y.repeat_interleave(2, dim=1)) for x, y in zip(M.repeat_heads(kt, vt, 2), (kt, vt)))
+
+
+@pytest.mark.parametrize("where", ["object", "class"])
+@torch.no_grad()
+def test_a_replaced_update_of_the_cache_is_called(where, monkeypatch):
+    """A program that wraps KVCache.update (to record or change what is cached) sees every call, on the object or on the class."""
+    att, seen = M.Attention(M.ModelArgs(dim=256, n_head=4, n_local_heads=2)).to("cuda", torch.bfloat16), []
+    att.kv_cache = M.KVCache(1, 16, 2, 64).cuda()
+    plain = M.KVCache.update
+
+    def update(self, pos, k, v):
+        seen.append(pos.numel())
+        return plain(self, pos, k, 2 * v)
+
+    x, pos, f = torch.randn(1, 5, 256, device="cuda").to(torch.bfloat16), torch.arange(5, device="cuda"), torch.randn(5, 32, 2, device="cuda").to(torch.bfloat16)
+    mask = torch.ones(1, 1, 5, 16, dtype=torch.bool, device="cuda").tril()
+    att(x, f, mask, pos)
+    v = att.kv_cache.v_cache.clone()
+    if where == "object":
+        att.kv_cache.update = update.__get__(att.kv_cache)
+    else:
+        monkeypatch.setattr(M.KVCache, "update", update)
+    att(x, f, mask, pos)
+    assert seen == [5] and torch.equal(att.kv_cache.v_cache, 2 * v) and v.any()

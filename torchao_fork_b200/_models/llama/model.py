@@ -171,9 +171,12 @@ def apply_rotary_emb(x: Tensor, freqs_cis: Tensor) -> Tensor:
     return out.flatten(3).type_as(x)
 
 
+_CACHE_UPDATE = KVCache.update   # (a cache whose update somebody has replaced is asked through it)
+
+
 def kv_rows(cache, input_pos, k: Tensor, v: Tensor, freqs_cis: Tensor) -> bool:
     """k (to be rotated) and v [B][T][H][hd] into the rows input_pos of a plain cache, in one launch; False if that is not for these tensors."""
-    if type(cache) is not KVCache or k.dim() != 4 or not _rows_by_kernel(k, v, freqs_cis, cache.k_cache, cache.v_cache):
+    if type(cache) is not KVCache or getattr(cache.update, "__func__", None) is not _CACHE_UPDATE or k.dim() != 4 or not _rows_by_kernel(k, v, freqs_cis, cache.k_cache, cache.v_cache):
         return False
     b, t, h, d = k.shape
     s = cache.k_cache.shape[2]
