@@ -21,10 +21,10 @@
 // Warps 0-7: loads, weights and results, two threads per row (lane quadrant = warp % 4, half of the columns = warp / 4); warp 8: products.
 // Every wait is bounded; a CTA whose wait ran out goes on without waiting, so that all meet at the end, and marks its rows with NaN.
 //
-// Bound by the chain of a step (scores -> largest -> weights -> parts -> products): about 3400 clocks of which the tensor core works 1170 (d = dv =
-// 128), two chains per SM beside one another; a CTA's start and end (queries, the peers' shares) cost 9000 more.  2048 rows x 16 heads of 128
-// (four key heads): 59.5 us, against 308 us of window_attention_prompt_kernel; the same with all keys of a tile in one CTA 110 us (the last
-// tiles alone took 95), with unswizzled operands 84 us.
+// Bound by the chain of a step (scores -> largest -> weights -> parts -> products): about 3600 clocks with two CTAs on the SM, of which the tensor core
+// works 1170 for each (d = dv = 128); a CTA's start (queries, first keys) takes 6000 clocks more and its end (the peers' shares) 9000.  2048 rows x 16
+// heads of 128 (four key heads): 8.5 steps a CTA, 60 us, tensor pipe active in 31 % of the clocks, against 308 us of window_attention_prompt_kernel; the same with
+// all keys of a tile in one CTA 110 us (the last tiles alone took 95), with unswizzled operands 84 us.
 #include "../f32x2.h"
 #include "../per_device.h"
 #include "lm_mma.cuh"
