@@ -113,3 +113,17 @@ def test_end_and_beginning_of_a_decode_step(B, V, D, temperature, top_k):
     assert torch.equal(out, want) and torch.equal(fed, want) and pos.tolist() == [42, 7]
     assert torch.equal(h[:B], table[want]) and not h[B].any()
     assert L.ao_b200_embed_rows(fed.data_ptr(), table.data_ptr(), V, D + 4, B, h.data_ptr(), st) != 0  # rows of a whole number of 16 bytes
+
+
+@pytest.mark.parametrize("B,V,top_k", [(1, 199, None), (3, 4099, 50), (2, 128256, 200)])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+def test_rows_without_a_probability_name_a_token_that_exists(B, V, top_k, value):
+    """A row of logits that are NaN or infinite has no probabilities: every score is NaN, and argmax names the first token.  (What the kernel named for
+    such rows was no token at all, and the next step read the embedding table there.)  Other rows are not concerned."""
+    logits = torch.randn(B, V, device=DEV).to(torch.bfloat16)
+    noise = torch.empty(B, V, device=DEV).exponential_(1)
+    want = run_kernel(logits, 0.8, top_k, noise)
+    logits[B - 1] = value
+    got = run_kernel(logits, 0.8, top_k, noise)
+    assert got[B - 1].item() == 0 and torch.equal(got[: B - 1], want[: B - 1])
+    assert 0 <= run_kernel(logits, 0.0, None, None)[B - 1].item() < V

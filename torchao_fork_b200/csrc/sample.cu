@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kSampThreads) sample_kernel(const __nv_bfloat1
   if (rank == 0 && tid == 0) {
     unsigned long long b = part_best;
     for (int r = 1; r < kSampCluster; ++r) b = max(b, *cluster.map_shared_rank(&part_best, r));
-    take(0x7fffffff - (int)(b & 0xffffffffull));
+    take(b == 0 ? 0 : 0x7fffffff - (int)(b & 0xffffffffull));   // (no score is a number: the first token, as an argmax over NaN names; it has to be one that exists)
   }
   cluster.sync();  // nobody leaves while its shared memory may still be read
 }
