@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kHqqWarps * 32) hqq_finalize_kernel(const __nv
 //  - 32 weights per thread, packed as they come: 16 registers, and half as many exchanges per weight as with 16.
 // Same numbers as hqq_step_kernel, bit for bit: there lane l of 32 adds elements l + 32 j and the lanes meet in steps of 16, 8, 4, 2, 1;
 // here thread r of L = G / 32 holds the elements of the lanes r, r + L, .. of it, so the first steps of that tree are its own.
-// quantize_ of 4096 x 4096, groups of 64, 20 iterations: 207 us; 375 with one weight per instruction and a branch around each power (26.6
+// The search over 4096 x 4096, groups of 64, 20 iterations, in all its kernels: 207 us (a call by itself waits for the host, 350 and more); 375 with one weight per instruction and a branch around each power (26.6
 // instructions per weight and iteration); 1901 us of 20 steps and judges with a separate packing.
 constexpr int kHqqChunk = 10;   // iterations per launch: bounds hist to 10 numbers per group
 constexpr int kHqqMaxIters = 64;

@@ -42,8 +42,8 @@ __device__ __forceinline__ uint32_t tinygemm_quant1(float w, float min_val, floa
 //     (mul / fma .f32x2: the single operations' roundings);
 //   * rint of a bf16 in [0, 15] is an add of 128 in bf16 (ulp 1 there, ties to even as 128 is even), which leaves 0x4300 + q in
 //     each half: shifted and added up, four registers are a packed word plus a constant.
-// About 13 instructions for two weights; one quotient at a time with rint and the nibbles in fp32 took 20 a weight.  28672 x 8192, groups of 128: 101 us
-// of kernel (0.9 of the copy rate; 130 before), a call 154.6 -> 124.8 us; groups of 32: a call 213.7 -> 154.0 us.
+// About 13 instructions for two weights; one quotient at a time with rint and the nibbles in fp32 took 20 a weight.  28672 x 8192, groups of 128: 97 us
+// of kernel (0.93 of the copy rate; 130 before).  A call by itself is as long as the host takes to enqueue it, 180 to 230 us.
 struct QFast {
   float s, rs;        // scale and its reciprocal
   uint32_t minv2;     // (min_val, min_val) as bf16x2
