@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(kHqqWarps * 32) hqq_finalize_kernel(const __nv
 // and the block's error of each (`err`); hqq_mean_kernel adds the errors up, and whoever comes next works out
 // from the means which iteration was the last (hqq_last), so that iterations past the stop cost work but change nothing.
 //
-// Bound by the fp32 pipe and instruction issue: ten iterations over 4096 x 4096 take about 80 us.  What keeps the arithmetic at eleven
+// Bound by the fp32 pipe and instruction issue: ten iterations over 4096 x 4096 take 95 us.  What keeps the arithmetic at eleven
 // instructions per pair of weights and iteration:
 //  - pairs of weights in one register pair (add, mul, fma .f32x2: the single operation's rounding in each half.  But a product whose one use is a sum
 //    can come out as one fused operation (f32x2.h), so such a sum is a fused one already, with a factor of one);
@@ -142,8 +142,9 @@ __global__ void __launch_bounds__(kHqqWarps * 32) hqq_finalize_kernel(const __nv
 //  - 32 weights per thread, packed as they come: 16 registers, and half as many exchanges per weight as with 16.
 // Same numbers as hqq_step_kernel, bit for bit: there lane l of 32 adds elements l + 32 j and the lanes meet in steps of 16, 8, 4, 2, 1;
 // here thread r of L = G / 32 holds the elements of the lanes r, r + L, .. of it, so the first steps of that tree are its own.
-// The search over 4096 x 4096, groups of 64, 20 iterations, in all its kernels: 207 us (a call by itself waits for the host, 350 and more); 375 with one weight per instruction and a branch around each power (26.6
-// instructions per weight and iteration); 1901 us of 20 steps and judges with a separate packing.
+// The search over 4096 x 4096, groups of 64, 20 iterations, in all its kernels: 207 us (a call by itself waits for the host, 350 and more); 375 with
+// one weight per instruction and a branch around each power (26.6 instructions per weight and iteration); 1901 of 20 steps and judges with
+// a separate packing.
 constexpr int kHqqChunk = 10;   // iterations per launch: bounds hist to 10 numbers per group
 constexpr int kHqqMaxIters = 64;
 constexpr int kHqqPer = 32;     // weights per thread
