@@ -152,13 +152,14 @@ constexpr int kMaxSplitStrips = 32;   // strips of a cluster
 // 8192 x 28672, 8 rows 46 us and the GEMM 45 to 46, 16384 x 28672, 7 rows 82 and 78; int8 104 and 86); with four it does (40.5 at 7 rows; 73 at 6).
 constexpr int kSplitStages = 4;
 
-// Which products of 2 to 8 rows without a norm share k: a line for each kernel that the call would take otherwise (us, that kernel / halves or quarters of k).
+// Which products of 2 to 8 rows without a norm share k: a line for each kernel that the call would take otherwise (us, that kernel / halves or
+// quarters of k).
 //  - the GEMV over whole rows (they fit one CTA): 57344 activations.  int8, 8 rows of 3072 x 8192 12.1 / 8.7, of 8192 x 8192 19.1 / 16.0, 4 of
 //    4096 x 14336 15.4 / 14.7; int4 10.3 / 8.3, 15.5 / 13.4, 15.9 / 13.4.  Below: int8, 8 rows of 5120 x 5120 9.9 / 10.0, 4 of 8192 x 8192 14.4 / 15.2;
 //  - nothing fits, so a strip kernel or the GEMM: 3 rows (the kernels for up to 2 rows ask for less).  Int4 4096 x 14336, 8 rows 17.8 / 14.1, 8192 x 28672,
 //    3 / 7 rows 45.2 / 38.7, 45.5 / 40.5; int8 17.7 / 16.4, 50.7 / 40.9, 50.8 / 45.5, 8 rows 50.8 / 49.4;
-//  - the GEMM, which adds residuals: k of 8192.  Int4 3072 x 8192, 2 / 8 rows 14.9 / 7.6, 16.2 / 8.2, 8192 x 28672, 3 / 7 rows 45.5 / 38.2, 46 / 40.4; int8 15.7 / 8.1,
-//    17.4 / 8.7, 48.4 / 40.1, 49.5 / 45.4, 28672 x 8192, 8 rows 49.7 / 44.7.  Below: int8 28672 x 4096, 8 rows 30 / 36.
+//  - the GEMM, which adds residuals: k of 8192.  Int4 3072 x 8192, 2 / 8 rows 14.9 / 7.6, 16.2 / 8.2, 8192 x 28672, 3 / 7 rows 45.5 / 38.2, 46 / 40.4; int8
+//    15.7 / 8.1, 17.4 / 8.7, 48.4 / 40.1, 49.5 / 45.4, 28672 x 8192, 8 rows 49.7 / 44.7.  Below: int8 28672 x 4096, 8 rows 30 / 36.
 // More rows are not split: twice the products per weight in CTAs with half the k (16 rows of 8192 x 8192: 26 us against the GEMM's 23).
 enum class Instead { kWholeRows, kNothingFits, kGemm };
 static inline bool share_k(int64_t M, int64_t Kp, Instead instead) {
@@ -181,7 +182,7 @@ __device__ __forceinline__ void split_begin(bool owner, int strips, uint64_t* in
 // before the first send, and before a thread leaves
 __device__ __forceinline__ void split_meet() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 // The epilogue warp's sums of strip li, scaled (each rank has scaled its part of a row by itself): false, and sent on, on the other ranks; all
-// parts added on rank 0.  The wait is bounded: NaN after about two seconds.
+// parts added on rank 0.  The wait is bounded: NaN after about two seconds, which the caller takes for sums that are to be done again.
 template <int MT>
 __device__ __forceinline__ bool split_sums(float4 (&sum)[MT], const float* row_scale, uint64_t* in_full, float4* inbox, int li, int rank, int ks, int lane) {
   const int c = lane & 3;

@@ -173,8 +173,8 @@ __device__ __forceinline__ void hide_odd_values(unsigned char* values, int piece
     atomicOr(&marks[2 * (n & 1) + (row >> 5)], 1u << (row & 31));
   }
 }
-// keys: those that hide_odd_values has marked; a row sees key kk where kk <= see_hi and (kk >= see_lo or kk < see_keep).  Whatever their weight, the sum is the infinity or
-// NaN.  Columns [first_column, first_column + columns) of the row, at o_mine in tensor memory.  Out of line: the steps keep their registers.
+// keys: those that hide_odd_values has marked; a row sees key kk where kk <= see_hi and (kk >= see_lo or kk < see_keep).  Whatever their weight, the
+// sum is the infinity or NaN.  Columns [first_column, first_column + columns) of the row, at o_mine in tensor memory.  Out of line: the steps keep their registers.
 __device__ __noinline__ void add_odd_values(const WinPromptArgs& a, uint64_t keys, int k0, int see_hi, int see_lo, int see_keep, int row, int lo, int nf, int g,
                                             uint32_t o_mine, int dv, int first_column, int columns) {
   const int back = a.back[row], p0 = a.pos[row] - back;
@@ -420,8 +420,8 @@ __device__ __forceinline__ void attend(const WinPromptArgs& a, int dv) {
           const volatile uint32_t* mark = sh.odd + 2 * (hidings++ & 1);
           const uint64_t keys = mark[0] | ((uint64_t)mark[1] << 32);
           if (keys != 0) {
-            add_odd_values(a, keys, k0, r < count ? nf + (pa + r - lo) : -1, nf + max(pa + r - a.window + 1 - lo, 0), nf + max(a.keep - lo, 0), first, lo, nf, g, o_mine,
-                           dv, half * dvh, dvh);
+            add_odd_values(a, keys, k0, r < count ? nf + (pa + r - lo) : -1, nf + max(pa + r - a.window + 1 - lo, 0), nf + max(a.keep - lo, 0), first, lo, nf,
+                           g, o_mine, dv, half * dvh, dvh);
             tc_before();
           }
         }
@@ -567,8 +567,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(cons
   // A hidden key's weight is 0, and 0 times a value that is not finite is not: where a result is not finite (on any CTA of the cluster, which has
   // told the others) the tile is done once more with an eye to that.  (Looking at the values of every step that hides keys: 2048 rows 62 us, not 60.)
   if (*reinterpret_cast<volatile int*>(&sh.again) != 0) attend_carefully<NM, C>(a, dv);
-  const int tile = (int)(gridDim.x / C - 1 - ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) / C / a.H), h = (int)(((int64_t)blockIdx.y * gridDim.x + blockIdx.x) / C % a.H);
-  if (*reinterpret_cast<volatile int*>(&sh.dead) != 0) {   // a wait ran out: all rows of the tile are marked, after the peers' results, and what is in flight gets the time to land
+  if (*reinterpret_cast<volatile int*>(&sh.dead) != 0) {   // a wait ran out: all rows of the tile are marked, after the peers' results, and what is in
+    const int64_t turn = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) / C;   // flight gets the time to land
+    const int h = (int)(turn % a.H), tile = (int)(gridDim.x / C - 1 - turn / a.H);
     const int first = a.tile_first[tile];
     if (threadIdx.x < min(a.tile_count[tile], kTcRows))
       for (int c = 0; c < dv; ++c) a.out[(int64_t)(first + threadIdx.x) * a.ld_out + (int64_t)h * dv + c] = __ushort_as_bfloat16((unsigned short)0x7FFF);
