@@ -144,6 +144,7 @@ AO_B200_API int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ld
  * it zeroed); with NULL / too small a workspace the call still works but skips the tensor-memory kernel.  Returns
  * AO_B200_ERR_WORKSPACE when M * K does not fit any decode kernel's shared-memory staging (use ao_b200_int4_mm then).
  * The weights must have been there before the kernel in front of this call was launched: they are read while it ends. */
+AO_B200_API int ao_b200_gemv_fused_fits(int64_t M, int64_t Kp, int group_size);  /* 1: M rows of Kp fit a fused call (group_size 0: int8) */
 AO_B200_API int ao_b200_int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx,
                             const void* packed, const void* scale_and_zero, int64_t Np, int64_t Kp,
                             int group_size, void* y, int64_t N_out, int64_t ldy,

@@ -87,3 +87,31 @@ def test_int8_gemm_and_int4_tickets_keep_apart(fused):
     # [partial sums][tickets ..]: the last kilobyte in front of the GEMM's part
     front = int(_lib.lib().ao_b200_int4_mm_workspace_bytes(1, eng.output.np_, eng.output.kp))
     assert not eng.ws[front - (1 << 20) : front].any()
+
+
+def test_projection_whose_correction_sums_do_not_fit_beside_its_rows():
+    """Five rows of 14336 leave room for the sums over groups of 128 but not for those of 64: the step takes that projection's other form."""
+    test_parts_match_single_launches("int4", 14336, 5)
+
+
+@pytest.mark.parametrize("group", [0, 32, 64, 128, 256])
+def test_calls_that_fit_are_taken_and_the_others_refused(group):
+    L, st = _lib.lib(), torch.cuda.current_stream().cuda_stream
+    seen = set()
+    for K in (4096, 8192, 12288, 14336, 20480, 28672, 36864):
+        N = 128
+        w = torch.randn(N, K, device="cuda").to(torch.bfloat16)
+        if group:
+            packed, scales = torch.ops.torchao.b200_int4_quantize_pack(w, group, 1e-6, True)
+        else:
+            q, scales = torch.ops.torchao.b200_int8_quantize(w, 1e-6, True)
+            packed = torch.ops.torchao.b200_int8_pack(q)
+        for M in (1, 2, 3, 5, 8, 9, 16):
+            x, y = torch.randn(M, K, device="cuda").to(torch.bfloat16), torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+            args = (x.data_ptr(), M, K, K, packed.data_ptr(), scales.data_ptr(), N, K)
+            tail = (y.data_ptr(), N, N, None, 0.0, None, 0, 0)
+            rc = L.ao_b200_int4_gemv_fused(*args, group, *tail, None, 0, st) if group else L.ao_b200_int8_gemv_fused(*args, *tail, st)
+            fits = L.ao_b200_gemv_fused_fits(M, K, group)
+            seen.add(fits)
+            assert rc == (0 if fits else 4), (M, K, group, rc, fits)
+    assert seen == {0, 1} and L.ao_b200_gemv_fused_fits(17, 4096, group) == 0

@@ -75,6 +75,7 @@ SIGNATURES = {
                                        _vp],
     "ao_b200_decode_attention_fused_q8": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _f32, _i32,
                                           _vp, _i64, _vp],
+    "ao_b200_gemv_fused_fits": [_i64, _i64, _i32],
     "ao_b200_silu_mul": [_vp, _vp, _i64, _i64, _vp],
     "ao_b200_rotary": [_vp, _i64, _i64, _i64, _vp, _vp, _i64, _i64, _i64, _i64, _vp],
     "ao_b200_kv_rows": [_vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64, _vp, _vp, _i32, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _vp],

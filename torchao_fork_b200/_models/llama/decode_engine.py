@@ -122,7 +122,8 @@ class _Linear:
             "int4_gemv_fused")
 
     def fused_fits(self, m):
-        return self.kind in ("int4", "int8") and m <= 16 and m * (2 * self.kp + 16) <= 150 * 1024
+        return (self.kind in ("int4", "int8") and m <= 16 and m * (2 * self.kp + 16) <= 150 * 1024
+                and bool(_lib.lib().ao_b200_gemv_fused_fits(m, self.kp, self.group_size if self.kind == "int4" else 0)))
 
     def launch(self, x: torch.Tensor, y: torch.Tensor, ws: Optional[torch.Tensor], stream: int):
         m = x.shape[0]

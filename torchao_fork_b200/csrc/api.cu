@@ -8,6 +8,7 @@ int int4_gemv(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* pac
 int int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np,
                     int64_t Kp, int G, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps,
                     const void* residual, int64_t ld_res, int epilogue, int max_stages, int follow, cudaStream_t s);
+bool int4_gemv_imma_fits(int64_t M, int64_t Kp, int G, int max_stages);
 int int4_gemv_imma(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np,
                    int64_t Kp, int G, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps,
                    const void* residual, int64_t ld_res, int epilogue, int max_stages, int follow, cudaStream_t s);
@@ -173,6 +174,14 @@ extern "C" int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
     if (e) return e;
   }
   return AO_B200_OK;
+}
+
+extern "C" int ao_b200_gemv_fused_fits(int64_t M, int64_t Kp, int group_size) {
+  if (M <= 0 || M > 16 || Kp <= 0 || Kp % 64 != 0) return 0;
+  const int stages = tunables().stages;
+  if (group_size == 0) return ao::int8_gemv_fused_fits(M, Kp, stages);
+  if (Kp % group_size != 0) return 0;
+  return ao::int4_gemv_fused_fits(M, Kp, group_size, stages) || (tunables().gemv_imma && ao::int4_gemv_imma_fits(M, Kp, group_size, stages));
 }
 
 extern "C" int ao_b200_int4_gemv_fused(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed,

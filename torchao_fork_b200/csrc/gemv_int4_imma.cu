@@ -541,6 +541,12 @@ static bool plan_imma(int M, int64_t Kp, int G, int max_stages, PlanI& pl) {
   return true;
 }
 
+// whether the activations of a call fit this kernel's staging
+bool int4_gemv_imma_fits(int64_t M, int64_t Kp, int G, int max_stages) {
+  PlanI pl;
+  return M <= 2 && (G == 32 || G == 64 || G == 128 || G == 256) && Kp % (G > 128 ? G : 128) == 0 && plan_imma((int)M, Kp, G, max_stages, pl);
+}
+
 // M <= 2, G in {32, 64, 128, 256}.  Returns AO_B200_ERR_UNSUPPORTED / AO_B200_ERR_WORKSPACE when the shape is not for this kernel.
 int int4_gemv_imma(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np,
                    int64_t Kp, int G, void* y, int64_t N_out, int64_t ldy, const void* norm_w, float eps,
