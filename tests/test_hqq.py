@@ -203,3 +203,40 @@ def test_zero_points_of_the_search_equal_those_of_the_steps_in_32_bits(shape, gs
     assert torch.equal(own[:n_groups], scale)
     last = (ran - 1) % 10
     assert torch.equal(own[n_groups * (1 + last) : n_groups * (2 + last)].view(torch.int32), zero.view(torch.int32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gs", [32, 64, 128, 256])
+@pytest.mark.parametrize("shape,iters,kappa", [((3, 512), 1, 1.01), ((37, 768), 9, 1.01), ((601, 2048), 11, 0.97), ((5000, 1024), 33, 1.05)])
+def test_groups_at_rest_give_what_their_iterations_would(shape, iters, kappa, gs):
+    """Groups that come to rest early, late and never (a spread of row scales from 0.01 to 10, constant groups, a NaN and an infinity), counts of iterations
+    around those of a launch, thresholds that fall and that rise: the search's zero points are those of the steps, bit for bit (NaN where those are)."""
+    from torchao_fork_b200 import _lib
+    from torchao_fork_b200 import ops as aops
+    g = torch.Generator(device="cuda").manual_seed(gs + iters)
+    n, k = shape
+    w = (10 ** (3 * torch.rand(n, 1, device="cuda", generator=g) - 2) * torch.randn(n, k, device="cuda", generator=g)).to(torch.bfloat16)
+    w[0, :gs], w[1, :gs] = 0.25, 0.0
+    L, st, n_groups = _lib.lib(), torch.cuda.current_stream().cuda_stream, n * k // gs
+    args = (aops.HQQ_BETA, kappa, aops.HQQ_LP_NORM, iters)
+    for odd in (False, True):
+        if odd:
+            w[2, 3], w[-1, -1] = float("nan"), float("inf")
+        scale = torch.empty(n_groups, dtype=torch.float32, device="cuda")
+        zero, err = torch.empty_like(scale), torch.empty(int(L.ao_b200_hqq_blocks(n_groups)), dtype=torch.float32, device="cuda")
+        state = torch.empty(2, dtype=torch.float64, device="cuda")
+        _lib.check(L.ao_b200_hqq_init(w.data_ptr(), n_groups, gs, scale.data_ptr(), zero.data_ptr(), st), "init")
+        _lib.check(L.ao_b200_hqq_solve(w.data_ptr(), n_groups, gs, scale.data_ptr(), zero.data_ptr(), *args, err.data_ptr(), state.data_ptr(), st), "solve")
+        ws = torch.empty(int(L.ao_b200_hqq_search_workspace_bytes(n_groups, gs)), dtype=torch.uint8, device="cuda").fill_(0x7F)
+        q = torch.empty(n, k, dtype=torch.int32, device="cuda")
+        s, z = (torch.empty(n, k // gs, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        _lib.check(L.ao_b200_hqq_search(w.data_ptr(), n, k, gs, *args, ws.data_ptr(), ws.numel(), q.data_ptr(), s.data_ptr(), z.data_ptr(), 0, 0, None, None,
+                                        st), "search")
+        ran = int(state[1:].view(torch.int32)[1])
+        at = (64 + 10 * (-(-n * k // 8192))) * 8
+        own = ws[at : at + 4 * n_groups * 11].view(torch.float32)
+        last = (ran - 1) % 10
+        got = own[n_groups * (1 + last) : n_groups * (2 + last)]
+        same = (got.view(torch.int32) == zero.view(torch.int32)) | (got.isnan() & zero.isnan())
+        assert bool(same.all()), int((~same).sum())
+        assert bool(zero.isnan().any()) == odd

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(kHqqWarps * 32) hqq_finalize_kernel(const __nv
 // and the block's error of each (`err`); hqq_mean_kernel adds the errors up, and whoever comes next works out
 // from the means which iteration was the last (hqq_last), so that iterations past the stop cost work but change nothing.
 //
-// Bound by the fp32 pipe and instruction issue: ten iterations over 4096 x 4096 take 95 us.  What keeps the arithmetic at eleven
+// Bound by the fp32 pipe and instruction issue: ten iterations of all groups of 4096 x 4096 take 95 us.  What keeps the arithmetic at eleven
 // instructions per pair of weights and iteration:
 //  - pairs of weights in one register pair (add, mul, fma .f32x2: the single operation's rounding in each half.  But a product whose one use is a sum
 //    can come out as one fused operation (f32x2.h), so such a sum is a fused one already, with a factor of one);
@@ -142,17 +142,23 @@ __global__ void __launch_bounds__(kHqqWarps * 32) hqq_finalize_kernel(const __nv
 //  - 32 weights per thread, packed as they come: 16 registers, and half as many exchanges per weight as with 16.
 // Same numbers as hqq_step_kernel, bit for bit: there lane l of 32 adds elements l + 32 j and the lanes meet in steps of 16, 8, 4, 2, 1;
 // here thread r of L = G / 32 holds the elements of the lanes r, r + L, .. of it, so the first steps of that tree are its own.
-// The search over 4096 x 4096, groups of 64, 20 iterations, in all its kernels: 207 us (a call by itself waits for the host, 350 and more); 375 with
-// one weight per instruction and a branch around each power (26.6 instructions per weight and iteration); 1901 of 20 steps and judges with
-// a separate packing.
+// What keeps the iterations few: a group whose zero point comes out as it went in, bit for bit, while no |d| of it can pass the smallest threshold still
+// to come, gives the same zero point and error in every iteration that follows, so it is at rest and its lanes take the next group.  A zero point
+// moves by the mean rounding error and settles as soon as no weight crosses a rounding boundary on the way: of normal weights in groups of 32 / 64 / 128 / 256
+// 2.4 / 3.4 / 4.8 / 6.7 iterations of 20 move it, and one more shows it.  (Groups that never rest, as with weights of spread 3, where powf decides: 1361 -> 1549 us.)
+// The search over 4096 x 4096, groups of 64, 20 iterations, in all its kernels: 199 us with all iterations of all groups, 108 without those at rest
+// (groups of 32 / 128 / 256: 212 / 227 / 186 -> 113 / 121 / 130).  Taken back: groups put together anew among a block's warps after each iteration (155),
+// rounds of two and three iterations over a block's list (141).
 constexpr int kHqqChunk = 10;   // iterations per launch: bounds hist to 10 numbers per group
 constexpr int kHqqMaxIters = 64;
 constexpr int kHqqPer = 32;     // weights per thread
-constexpr int kHqqBlocks = 4;   // blocks per SM: 64 registers (3 blocks of 80: 220 us; 16 weights per thread and 4 blocks: 228)
+constexpr int kHqqThreads = 256, kHqqBlocks = 4;   // per block; per SM: 64 registers (with all iterations of all groups 207 us, 3 blocks of 80 220; 16 weights per thread and 4 blocks 228)
+constexpr int kHqqShare = 512;  // groups of a block at a time, at most; a multiple of 8
 
 struct HqqChunk {
   float inv_beta[kHqqChunk], threshold[kHqqChunk];
   float lp_m1;
+  float least;                  // smallest threshold of this launch's iterations and of those that follow
   int first, count;             // iterations [first, first + count)
 };
 
@@ -194,138 +200,232 @@ __device__ __forceinline__ void hqq_tree(int i, Leaf&& leaf, F2& acc, float2& e)
   }
 }
 
+// A block takes contiguous groups, at most kHqqShare at a time; L lanes of a warp take one group, two iterations, and then the next one if theirs is over, each
+// at its own count.  rest: per group, the error of a group that has come to rest, else -1 (written by a launch for the next).
 template <int G>
-__global__ void __launch_bounds__(256, kHqqBlocks) hqq_iterate_kernel(const __nv_bfloat16* __restrict__ w, int64_t n_groups, HqqChunk ch,
-                                                                      float* __restrict__ scale, float* __restrict__ hist, double* __restrict__ err,
-                                                                      const double* __restrict__ mean) {
+__global__ void __launch_bounds__(kHqqThreads, kHqqBlocks) hqq_iterate_kernel(const __nv_bfloat16* __restrict__ w, int64_t n_groups, HqqChunk ch, int share,
+                                                                              float* __restrict__ scale, float* __restrict__ hist, double* __restrict__ err,
+                                                                              const double* __restrict__ mean, float* __restrict__ rest) {
   constexpr int L = G / kHqqPer, I = 32 / L, J = G / 32;   // threads per group; its lanes per thread; elements per lane
-  constexpr int kGroups = 256 / L;                         // groups per block
   constexpr float kMagic = 12582912.f;                     // 1.5 * 2^23: adding and subtracting it is rint up to 2^22, and beyond that the clamp decides
-  __shared__ float s_err[kHqqChunk][kGroups];
+  constexpr int kAtRest = 256;
+  __shared__ float s_err[kHqqChunk][kHqqShare], s_z[kHqqShare], s_es[kHqqShare], s_threshold[kHqqChunk], s_inv_beta[kHqqChunk];
+  __shared__ short s_done[kHqqShare];                      // iterations whose results are there; + kAtRest: the others are as the last one
+  __shared__ short s_todo[kHqqShare];
+  __shared__ int s_n, s_next;                              // how many; the next ones to be fetched
+  __shared__ double s_total[kHqqChunk];
   bool stopped = false;
   if (ch.first > 0) hqq_last(mean, ch.first, stopped);
   if (stopped) return;
-  const int64_t group = ((int64_t)blockIdx.x * 256 + threadIdx.x) / L;
-  const bool in = group < n_groups, first = threadIdx.x % L == 0;
-  const unsigned short* wp = reinterpret_cast<const unsigned short*>(w) + group * G + threadIdx.x % L;
-  uint32_t v[kHqqPer / 2];         // pair (j I + i) / 2: weights i L + 32 j (lower half) and (i + 1) L + 32 j of the thread's, bf16
-#pragma unroll
-  for (int j = 0; j < J; ++j)
-#pragma unroll
-    for (int i = 0; i < I; i += 2) v[(j * I + i) / 2] = in ? (uint32_t)wp[32 * j + L * i] | ((uint32_t)wp[32 * j + L * (i + 1)] << 16) : 0u;
-  auto weights = [&](int k) { return f2(__uint_as_float(v[k] << 16), __uint_as_float(v[k] & 0xFFFF0000u)); };
-  float mn = f2_get(weights(0)).x, mx = mn;
-#pragma unroll
-  for (int k = 0; k < kHqqPer / 2; ++k) {
-    const float2 f = f2_get(weights(k));
-    mn = fminf(mn, fminf(f.x, f.y)), mx = fmaxf(mx, fmaxf(f.x, f.y));
-  }
-#pragma unroll
-  for (int o = L / 2; o; o >>= 1) {
-    mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  }
-  float s, z;
-  if (ch.first == 0) {             // (:2052-2060), as in hqq_init_kernel
-    s = fminf(__fdiv_rn(15.f, __fsub_rn(mx, mn)), 2e4f);
-    z = rintf(__fmul_rn(-mn, s));
-    if (in && first) scale[group] = s;
-  } else {
-    s = in ? scale[group] : 1.f;
-    z = in ? hist[(int64_t)(kHqqChunk - 1) * n_groups + group] : 0.f;
-  }
-  // (the minus signs ride along: -x = n (-r), its remainder n + (-x) s, and -(x + r rem) = (-r) rem + (-x), all rounded as without them)
-  const float nr = -__frcp_rn(s), t_lo = __fmul_rn(mn, s), t_hi = __fmul_rn(mx, s);
-  const F2 s2 = f2(s, s), ns2 = f2(-s, -s), nr2 = f2(nr, nr), one = f2(1.f, 1.f), minus = f2(-1.f, -1.f), magic = f2(kMagic, kMagic), no_magic = f2(-kMagic, -kMagic);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane % L;
+  if (threadIdx.x < kHqqChunk) s_total[threadIdx.x] = 0.0, s_threshold[threadIdx.x] = ch.threshold[threadIdx.x], s_inv_beta[threadIdx.x] = ch.inv_beta[threadIdx.x];
 #pragma unroll 1
-  for (int it = 0; it < ch.count; ++it) {
-    // (the compiler would keep all weights unpacked and multiplied beside the packed ones, and have no registers left)
-#pragma unroll
-    for (int k = 0; k < kHqqPer / 2; ++k) asm volatile("" : "+r"(v[k]));
-    const float thr = ch.threshold[it];
-    const F2 z2 = f2(z, z), nz2 = f2(-z, -z);
-    // what the group's smallest and largest weight say about all of it: no weight is clamped, and no |d| is above the threshold
-    // (|d| is half a step, or what the clamp cuts off; the margins are a hundred times the roundings of t + z and of the quotient)
-    const float q_lo = __fadd_rn(t_lo, z), q_hi = __fadd_rn(t_hi, z);
-    const bool inside = __all_sync(0xffffffffu, q_lo >= -0.5f && q_hi < 15.5f);
-    const bool small = __all_sync(0xffffffffu, (fmaxf(0.51f, fmaxf(-q_lo, q_hi - 15.f)) + (fabsf(z) + 16.f) * 1e-6f) * -nr <= 0.999f * thr);
-    auto quotients = [&](F2 f, bool clamp, F2& wq, F2& nt) {   // W_q, -W * scale and d = W - W_r of a pair
-      nt = f2_mul(f, ns2);
-      wq = f2_add(f2_add(f2_fma(nt, minus, z2), magic), no_magic);
-      if (clamp) {
-        const float2 q = f2_get(wq);
-        wq = f2(fminf(fmaxf(q.x, 0.f), 15.f), fminf(fmaxf(q.y, 0.f), 15.f));
+  for (int64_t base = (int64_t)blockIdx.x * share; base < n_groups; base += (int64_t)gridDim.x * share) {
+    const int here = (int)(n_groups - base < share ? n_groups - base : share);
+    if (threadIdx.x == 0) s_n = s_next = 0;
+    __syncthreads();
+#pragma unroll 1
+    for (int g0 = warp * 32; g0 < here; g0 += kHqqThreads) {
+      const int g = g0 + lane;
+      bool todo = g < here;
+      if (todo && ch.first > 0) {
+        const float e = rest[base + g];
+        s_z[g] = hist[(int64_t)(kHqqChunk - 1) * n_groups + base + g];
+        todo = e < 0.f;
+        if (!todo) s_es[g] = e, s_done[g] = kAtRest;
       }
-      const F2 n = f2_add(wq, nz2), nx = f2_mul(n, nr2);
-      return f2_get(f2_add(f, f2_fma(f2_fma(nx, s2, n), nr2, nx)));
-    };
-    auto lane_pair = [&](int i, F2& acc, float2& e, auto&& one) {   // J elements each, one after the other
+      const uint32_t any = __ballot_sync(0xffffffffu, todo);
+      int at = 0;
+      if (any != 0 && lane == 0) at = atomicAdd(&s_n, __popc(any));
+      at = __shfl_sync(0xffffffffu, at, 0) + __popc(any & ((1u << lane) - 1u));
+      if (todo) s_todo[at] = (short)g;
+    }
+    __syncthreads();
+    const int n = s_n;
+    uint32_t v[kHqqPer / 2];       // pair (j I + i) / 2: weights i L + 32 j (lower half) and (i + 1) L + 32 j of the thread's, bf16
 #pragma unroll
-      for (int j = 0; j < J; ++j) {
-        F2 a;
-        const float2 d = one((j * I + i) / 2, a);
-        acc = j == 0 ? a : f2_add(acc, a);
-        e = j == 0 ? make_float2(fabsf(d.x), fabsf(d.y)) : make_float2(e.x + fabsf(d.x), e.y + fabsf(d.y));
+    for (int k = 0; k < kHqqPer / 2; ++k) v[k] = 0u;
+    float s = 1.f, z = 0.f, t_lo = 0.f, t_hi = 0.f;
+    int g = 0, it = 0;
+    bool moves = false;            // the lane has a group, which is neither at rest nor through
+    auto weights = [&](int k) { return f2(__uint_as_float(v[k] << 16), __uint_as_float(v[k] & 0xFFFF0000u)); };
+#pragma unroll 1
+    for (;;) {
+      const uint32_t idle = __ballot_sync(0xffffffffu, !moves);
+      if (idle != 0 && *reinterpret_cast<volatile int*>(&s_next) < n) {
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&s_next, __popc(idle) / L);
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(idle & ((1u << lane) - 1u)) / L;
+        const bool fresh = !moves && at < n;
+        if (fresh) {
+          g = s_todo[at], it = 0, moves = true;
+          const unsigned short* wp = reinterpret_cast<const unsigned short*>(w) + (base + g) * G;
+          if constexpr (L <= 2) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              uint4 x[L];
+#pragma unroll
+              for (int h = 0; h < L; ++h) x[h] = ldg128(wp + (c * L + h) * 8);
+              if constexpr (L == 1) {
+                v[4 * c] = x[0].x, v[4 * c + 1] = x[0].y, v[4 * c + 2] = x[0].z, v[4 * c + 3] = x[0].w;
+              } else {
+                const uint32_t half = part ? 0x7632u : 0x5410u;
+#pragma unroll
+                for (int h = 0; h < L; ++h) v[4 * c + 2 * h] = __byte_perm(x[h].x, x[h].y, half), v[4 * c + 2 * h + 1] = __byte_perm(x[h].z, x[h].w, half);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < J; ++j)
+#pragma unroll
+              for (int i = 0; i < I; i += 2) v[(j * I + i) / 2] = (uint32_t)wp[32 * j + L * i + part] | ((uint32_t)wp[32 * j + L * (i + 1) + part] << 16);
+          }
+        }
+        uint32_t lo2 = v[0], hi2 = v[0];
+#pragma unroll
+        for (int k = 1; k < kHqqPer / 2; ++k) {
+          asm("min.bf16x2 %0, %0, %1;" : "+r"(lo2) : "r"(v[k]));
+          asm("max.bf16x2 %0, %0, %1;" : "+r"(hi2) : "r"(v[k]));
+        }
+        float mn = fminf(__uint_as_float(lo2 << 16), __uint_as_float(lo2 & 0xFFFF0000u)), mx = fmaxf(__uint_as_float(hi2 << 16), __uint_as_float(hi2 & 0xFFFF0000u));
+#pragma unroll
+        for (int o = L / 2; o; o >>= 1) {
+          mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        }
+        if (fresh) {
+          if (ch.first == 0) {     // (:2052-2060), as in hqq_init_kernel
+            s = fminf(__fdiv_rn(15.f, __fsub_rn(mx, mn)), 2e4f);
+            z = rintf(__fmul_rn(-mn, s));
+            if (part == 0) scale[base + g] = s;
+          } else {
+            s = scale[base + g], z = s_z[g];
+          }
+          t_lo = __fmul_rn(mn, s), t_hi = __fmul_rn(mx, s);
+        }
       }
-    };
-    F2 acc;
-    float2 e;
-    if (small && inside) {         // W_e = 0: mean of W_q - W * scale
-      hqq_tree<I, 2>(0, [&](int i, F2& a, float2& b) {
-        lane_pair(i, a, b, [&](int k, F2& x) {
-          F2 wq, nt;
-          const float2 d = quotients(weights(k), false, wq, nt);
-          x = f2_fma(nt, one, wq);
-          return d;
-        });
-      }, acc, e);
-    } else if (small) {
-      hqq_tree<I, 2>(0, [&](int i, F2& a, float2& b) {
-        lane_pair(i, a, b, [&](int k, F2& x) {
-          F2 wq, nt;
-          const float2 d = quotients(weights(k), true, wq, nt);
-          x = f2_fma(nt, one, wq);
-          return d;
-        });
-      }, acc, e);
-    } else {
-      const float c = ch.inv_beta[it];
-      hqq_tree<I, 2>(0, [&](int i, F2& a, float2& b) {
-        lane_pair(i, a, b, [&](int k, F2& x) {
-          F2 wq, nt;
-          const float2 d = quotients(weights(k), true, wq, nt), f = f2_get(weights(k)), t = f2_get(nt), q = f2_get(wq);
-          float2 u = make_float2(-t.x, -t.y);              // (W - W_e) * scale
-          if (fabsf(d.x) > thr) u.x = __fmul_rn(__fsub_rn(f.x, hqq_shrink(d.x, c, ch.lp_m1)), s);
-          if (fabsf(d.y) > thr) u.y = __fmul_rn(__fsub_rn(f.y, hqq_shrink(d.y, c, ch.lp_m1)), s);
-          x = f2(__fsub_rn(q.x, u.x), __fsub_rn(q.y, u.y));
-          return d;
-        });
-      }, acc, e);
-    }
-    const float2 last = f2_get(acc);
-    float sum = last.x + last.y, es = e.x + e.y;
+      if (!__any_sync(0xffffffffu, moves)) break;
+      // (the minus signs ride along: -x = n (-r), its remainder n + (-x) s, and -(x + r rem) = (-r) rem + (-x), all rounded as without them)
+      const float nr = -__frcp_rn(s);
+      const F2 s2 = f2(s, s), ns2 = f2(-s, -s), nr2 = f2(nr, nr), one = f2(1.f, 1.f), minus = f2(-1.f, -1.f), magic = f2(kMagic, kMagic), no_magic = f2(-kMagic, -kMagic);
+#pragma unroll 1
+      for (int twice = 0; twice < 2; ++twice) {
+        // (the compiler would keep all weights unpacked and multiplied beside the packed ones, and have no registers left)
 #pragma unroll
-    for (int o = L / 2; o; o >>= 1) {
-      sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      es += __shfl_xor_sync(0xffffffffu, es, o);
-    }
-    z = __fmul_rn(sum, 1.f / (float)G);                    // (a power of two: the quotient, rounded once too)
-    if (first) {
-      if (in) hist[(int64_t)it * n_groups + group] = z;
-      s_err[it][threadIdx.x / L] = in ? es : 0.f;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < ch.count) {    // eight groups at a time in fp32, as the blocks of hqq_step_kernel; fixed order: the stop is reproducible
-    double sum = 0.0;
-    for (int b = 0; b < kGroups; b += 8) {
-      float f = 0.f;
+        for (int k = 0; k < kHqqPer / 2; ++k) asm volatile("" : "+r"(v[k]));
+        const float thr = s_threshold[it];
+        const F2 z2 = f2(z, z), nz2 = f2(-z, -z);
+        // what the group's smallest and largest weight say about all of it: no weight is clamped, and no |d| is above the threshold
+        // (|d| is half a step, or what the clamp cuts off; the margins are a hundred times the roundings of t + z and of the quotient)
+        const float q_lo = __fadd_rn(t_lo, z), q_hi = __fadd_rn(t_hi, z);
+        const float bound = (fmaxf(0.51f, fmaxf(-q_lo, q_hi - 15.f)) + (fabsf(z) + 16.f) * 1e-6f) * -nr;
+        const bool inside = __all_sync(0xffffffffu, !moves || (q_lo >= -0.5f && q_hi < 15.5f));
+        const bool small = __all_sync(0xffffffffu, !moves || bound <= 0.999f * thr);
+        auto quotients = [&](F2 f, bool clamp, F2& wq, F2& nt) {   // W_q, -W * scale and d = W - W_r of a pair
+          nt = f2_mul(f, ns2);
+          wq = f2_add(f2_add(f2_fma(nt, minus, z2), magic), no_magic);
+          if (clamp) {
+            const float2 q = f2_get(wq);
+            wq = f2(fminf(fmaxf(q.x, 0.f), 15.f), fminf(fmaxf(q.y, 0.f), 15.f));
+          }
+          const F2 n = f2_add(wq, nz2), nx = f2_mul(n, nr2);
+          return f2_get(f2_add(f, f2_fma(f2_fma(nx, s2, n), nr2, nx)));
+        };
+        auto lane_pair = [&](int i, F2& acc, float2& e, auto&& one) {   // J elements each, one after the other
 #pragma unroll
-      for (int i = 0; i < 8; ++i) f += s_err[threadIdx.x][b + i];
-      sum += (double)f;
+          for (int j = 0; j < J; ++j) {
+            F2 a;
+            const float2 d = one((j * I + i) / 2, a);
+            acc = j == 0 ? a : f2_add(acc, a);
+            e = j == 0 ? make_float2(fabsf(d.x), fabsf(d.y)) : make_float2(e.x + fabsf(d.x), e.y + fabsf(d.y));
+          }
+        };
+        F2 acc;
+        float2 e;
+        if (small && inside) {         // W_e = 0: mean of W_q - W * scale
+          hqq_tree<I, 2>(0, [&](int i, F2& a, float2& b) {
+            lane_pair(i, a, b, [&](int k, F2& x) {
+              F2 wq, nt;
+              const float2 d = quotients(weights(k), false, wq, nt);
+              x = f2_fma(nt, one, wq);
+              return d;
+            });
+          }, acc, e);
+        } else if (small) {
+          hqq_tree<I, 2>(0, [&](int i, F2& a, float2& b) {
+            lane_pair(i, a, b, [&](int k, F2& x) {
+              F2 wq, nt;
+              const float2 d = quotients(weights(k), true, wq, nt);
+              x = f2_fma(nt, one, wq);
+              return d;
+            });
+          }, acc, e);
+        } else {
+          const float c = s_inv_beta[it];
+          hqq_tree<I, 2>(0, [&](int i, F2& a, float2& b) {
+            lane_pair(i, a, b, [&](int k, F2& x) {
+              F2 wq, nt;
+              const float2 d = quotients(weights(k), true, wq, nt), f = f2_get(weights(k)), t = f2_get(nt), q = f2_get(wq);
+              float2 u = make_float2(-t.x, -t.y);              // (W - W_e) * scale
+              if (fabsf(d.x) > thr) u.x = __fmul_rn(__fsub_rn(f.x, hqq_shrink(d.x, c, ch.lp_m1)), s);
+              if (fabsf(d.y) > thr) u.y = __fmul_rn(__fsub_rn(f.y, hqq_shrink(d.y, c, ch.lp_m1)), s);
+              x = f2(__fsub_rn(q.x, u.x), __fsub_rn(q.y, u.y));
+              return d;
+            });
+          }, acc, e);
+        }
+        const float2 last = f2_get(acc);
+        float sum = last.x + last.y, es = e.x + e.y;
+#pragma unroll
+        for (int o = L / 2; o; o >>= 1) {
+          sum += __shfl_xor_sync(0xffffffffu, sum, o);
+          es += __shfl_xor_sync(0xffffffffu, es, o);
+        }
+        if (moves) {
+          const float next = __fmul_rn(sum, 1.f / (float)G);   // (a power of two: the quotient, rounded once too)
+          const bool rests = __float_as_uint(next) == __float_as_uint(z) && bound <= 0.999f * ch.least;
+          z = next;
+          moves = !rests && it + 1 < ch.count;
+          if (part == 0) {
+            hist[(int64_t)it * n_groups + base + g] = z;
+            s_err[it][g] = es;
+            if (!moves) s_z[g] = z, s_es[g] = es, s_done[g] = (short)(it + 1 + (rests ? kAtRest : 0));
+          }
+          it += moves;
+        }
+      }
     }
-    err[(int64_t)threadIdx.x * gridDim.x + blockIdx.x] = sum;
+    __syncthreads();
+    // what a group at rest would have given in the iterations that were left out
+#pragma unroll 1
+    for (int g = threadIdx.x; g < (here + 7) / 8 * 8; g += kHqqThreads) {
+      const bool in = g < here;
+      const int done = in ? s_done[g] : kAtRest;
+      const float e = in ? s_es[g] : 0.f, z = in ? s_z[g] : 0.f;
+      for (int it = done & (kAtRest - 1); it < ch.count; ++it) {
+        s_err[it][g] = e;
+        if (in) hist[(int64_t)it * n_groups + base + g] = z;
+      }
+      if (in) rest[base + g] = done & kAtRest ? e : -1.f;
+    }
+    __syncthreads();
+    // eight groups at a time in fp32, as the blocks of hqq_step_kernel; fixed order: the stop is reproducible
+#pragma unroll 1
+    for (int it = warp; it < ch.count; it += kHqqThreads / 32) {
+      double sum = 0.0;
+      for (int b = lane * 8; b < here; b += 256) {
+        float f = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f += s_err[it][b + i];
+        sum += (double)f;
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (lane == 0) s_total[it] += sum;
+    }
+    __syncthreads();
   }
+  if (threadIdx.x < ch.count) err[(int64_t)threadIdx.x * gridDim.x + blockIdx.x] = s_total[threadIdx.x];
 }
 
 // block i: mean[first + i] = sum of err[i][..] / numel, in double, fixed order
@@ -545,12 +645,12 @@ extern "C" int ao_b200_hqq_finalize(const void* w, int64_t n_groups, int group_s
   return ao_launch_status();
 }
 
-static int64_t hqq_search_blocks(int64_t n_groups, int group_size) { return (n_groups * group_size + 256 * kHqqPer - 1) / (256 * kHqqPer); }
+static int64_t hqq_search_blocks(int64_t n_groups, int group_size) { return (n_groups * group_size + 8191) / 8192; }
 
-// [mean double x kHqqMaxIters][err double kHqqChunk x blocks][scale][hist kHqqChunk x n_groups]
+// [mean double x kHqqMaxIters][err double kHqqChunk x blocks][scale][hist kHqqChunk x n_groups][rest]
 extern "C" int64_t ao_b200_hqq_search_workspace_bytes(int64_t n_groups, int group_size) {
   if (n_groups <= 0 || group_size < kHqqPer) return 0;
-  return (kHqqMaxIters + kHqqChunk * hqq_search_blocks(n_groups, group_size)) * 8 + (1 + kHqqChunk) * n_groups * 4;
+  return (kHqqMaxIters + kHqqChunk * hqq_search_blocks(n_groups, group_size)) * 8 + (2 + kHqqChunk) * n_groups * 4;
 }
 
 extern "C" int ao_b200_hqq_search(const void* w, int64_t N, int64_t K, int group_size, double beta, double kappa, double lp_norm, int iters,
@@ -571,24 +671,33 @@ extern "C" int ao_b200_hqq_search(const void* w, int64_t N, int64_t K, int group
   double* err = mean + kHqqMaxIters;
   float* scale = reinterpret_cast<float*>(err + kHqqChunk * blocks);
   float* hist = scale + n_groups;
+  float* rest = hist + kHqqChunk * n_groups;
+  // as many blocks as the chip holds at once; their groups in equal shares, as many times as it takes
+  const int64_t most = (int64_t)kHqqBlocks * kNumSMs, rounds = (n_groups + most * kHqqShare - 1) / (most * kHqqShare);
+  int share = (int)((n_groups + rounds * most * 8 - 1) / (rounds * most * 8) * 8);
+  if (share < 8192 / group_size) share = 8192 / group_size;   // (a block's worth of threads, and what `blocks` counts)
+  const unsigned grid = (unsigned)((n_groups + share - 1) / share < most ? (n_groups + share - 1) / share : most);
+  float inv_beta[kHqqMaxIters], threshold[kHqqMaxIters];
+  for (int i = 0; i < iters; ++i) {
+    inv_beta[i] = (float)(1.0 / beta);
+    threshold[i] = lp_norm < 1.0 ? (float)(0.999 * std::pow(1.0 / beta, 1.0 / (2.0 - lp_norm))) : 0.f;
+    beta *= kappa;
+  }
   for (int first = 0; first < iters; first += kHqqChunk) {
     HqqChunk ch;
     ch.first = first;
     ch.count = iters - first < kHqqChunk ? iters - first : kHqqChunk;
     ch.lp_m1 = (float)(lp_norm - 1.0);
-    for (int i = 0; i < ch.count; ++i) {
-      ch.inv_beta[i] = (float)(1.0 / beta);
-      ch.threshold[i] = lp_norm < 1.0 ? (float)(0.999 * std::pow(1.0 / beta, 1.0 / (2.0 - lp_norm))) : 0.f;
-      beta *= kappa;
-    }
-    const unsigned grid = (unsigned)blocks;
+    ch.least = threshold[first];
+    for (int i = first; i < iters; ++i) ch.least = threshold[i] < ch.least ? threshold[i] : ch.least;
+    for (int i = 0; i < ch.count; ++i) ch.inv_beta[i] = inv_beta[first + i], ch.threshold[i] = threshold[first + i];
     switch (group_size) {
-      case 32: hqq_iterate_kernel<32><<<grid, 256, 0, s>>>(wb, n_groups, ch, scale, hist, err, mean); break;
-      case 64: hqq_iterate_kernel<64><<<grid, 256, 0, s>>>(wb, n_groups, ch, scale, hist, err, mean); break;
-      case 128: hqq_iterate_kernel<128><<<grid, 256, 0, s>>>(wb, n_groups, ch, scale, hist, err, mean); break;
-      default: hqq_iterate_kernel<256><<<grid, 256, 0, s>>>(wb, n_groups, ch, scale, hist, err, mean); break;
+      case 32: hqq_iterate_kernel<32><<<grid, kHqqThreads, 0, s>>>(wb, n_groups, ch, share, scale, hist, err, mean, rest); break;
+      case 64: hqq_iterate_kernel<64><<<grid, kHqqThreads, 0, s>>>(wb, n_groups, ch, share, scale, hist, err, mean, rest); break;
+      case 128: hqq_iterate_kernel<128><<<grid, kHqqThreads, 0, s>>>(wb, n_groups, ch, share, scale, hist, err, mean, rest); break;
+      default: hqq_iterate_kernel<256><<<grid, kHqqThreads, 0, s>>>(wb, n_groups, ch, share, scale, hist, err, mean, rest); break;
     }
-    hqq_mean_kernel<<<ch.count, 1024, 0, s>>>(err, blocks, 1.0 / ((double)n_groups * (double)group_size), first, mean);
+    hqq_mean_kernel<<<ch.count, 1024, 0, s>>>(err, (int64_t)grid, 1.0 / ((double)n_groups * (double)group_size), first, mean);
   }
   if (packed) {
     const int64_t tiles = (Np / 16) * (Kp / 64), want = (tiles + 7) / 8;
