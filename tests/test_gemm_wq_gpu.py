@@ -347,3 +347,41 @@ def test_last_tile_from_the_accumulators(bits, group, m, residual):
     tiles = lambda t: t.reshape(m, n // 128, 128).square().sum((0, 2)).sqrt()  # noqa: E731
     assert (tiles(y.double() - ref) / tiles(ref)).max().item() < 2.0 ** -8
     assert all(torch.equal(run(), y) for _ in range(12))
+
+
+@pytest.mark.parametrize("m", [511, 512, 513, 640, 769, 1041])
+@pytest.mark.parametrize("bits,n,k,group", [(4, 640, 1088, 32), (4, 321, 1088, 64), (4, 8192, 512, 128), (4, 384, 512, 256), (8, 8320, 192, 0), (8, 8192, 64, 0), (8, 640, 1088, 0)])
+def test_activations_read_in_place(bits, n, k, group, m):
+    # both sides of the line in rows and in outputs; half a unit at the end of k; tiles that end inside and outside of x
+    _check(bits, m, n, k, group)
+
+
+@pytest.mark.parametrize("bits,group", [(4, 64), (8, 0)])
+def test_activations_read_in_place_out_of_wider_rows(bits, group):
+    # rows further apart than they are long, from an odd multiple of 16 bytes on, with NaN and infinities around them; k shorter than the weights'
+    from torchao_fork_b200 import _lib
+    gen = torch.Generator(device="cuda").manual_seed(bits)
+    n, k, kx, m, ld = 640, 1152, 1096, 700, 1320
+    w = torch.randn(n, k, generator=gen, device="cuda").to(torch.bfloat16)
+    x = torch.full((m + 2, ld), float("nan"), device="cuda", dtype=torch.bfloat16)
+    x[1::2] = float("inf")
+    x[1 : m + 1, 24 : 24 + kx] = torch.randn(m, kx, generator=gen, device="cuda").to(torch.bfloat16)
+    if bits == 4:
+        packed, scales = T.b200_int4_quantize_pack(w, group, 1e-6, True)
+        wd = T.b200_int4_dequantize(packed, scales, group).double()[:n]
+    else:
+        q, scales = T.b200_int8_quantize(w, 1e-6, True)
+        packed = T.b200_int8_pack(q)
+        wd = q.double() * scales.double()[:, None]
+    np_, kp = packed.shape[0] * 16, packed.shape[1] * 64
+    L, st = _lib.lib(), torch.cuda.current_stream().cuda_stream
+    y = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+    xp = x.data_ptr() + (ld + 24) * 2
+    if bits == 4:
+        ws = torch.zeros(L.ao_b200_int4_mm_workspace_bytes(m, np_, kp), dtype=torch.uint8, device="cuda")
+        _lib.check(L.ao_b200_int4_mm(xp, m, kx, ld, packed.data_ptr(), scales.data_ptr(), np_, kp, group, y.data_ptr(), n, n, ws.data_ptr(), ws.numel(), st), "int4_mm")
+    else:
+        ws = torch.empty(L.ao_b200_int8_mm_workspace_bytes(m, np_, kp), dtype=torch.uint8, device="cuda").random_(0, 255)
+        _lib.check(L.ao_b200_int8_mm(xp, m, kx, ld, packed.data_ptr(), scales.data_ptr(), np_, kp, y.data_ptr(), n, n, ws.data_ptr(), ws.numel(), st), "int8_mm")
+    ref = x[1 : m + 1, 24 : 24 + kx].double() @ wd[:, :kx].t()
+    assert ((y.double() - ref).norm() / ref.norm()).item() < 2.0 ** -8

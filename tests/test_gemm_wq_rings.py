@@ -367,3 +367,26 @@ def test_the_model_sees_what_the_rules_prevent():
     # a last tile that is taken without waiting for its products
     even = plan(64, 128)
     assert _found(even, early=True, early_before_products=True) and not _found(even, early=True)
+
+
+def direct_plan(m, group):
+    """the same for calls that read the activations where they are: their ring starts on a multiple of 1024 bytes"""
+    c = plan(m, group)
+    mt = -(-m // 256)
+    nt = -(-(-(-m // mt)) // 16) * 16
+    wb = 8 * 2 * (512 if group else 1024) + (8 * (128 // group if group < 128 else 1) * 64 if group else 0)
+    off = -(-(-(-(HEADER + nt * PITCH) // 1024) * 1024 + c["x"] * nt // 2 * 256) // 128) * 128
+    c["w"] = min(MAX_W, (BUDGET - off) // wb)
+    c["a"] = 3 if c["w"] == 3 else A_SLOTS
+    return c
+
+
+@pytest.mark.parametrize("group", [0, 32, 64, 128, 256])
+def test_rings_of_activations_read_in_place(group):
+    plans = {tuple(sorted(direct_plan(m, group).items())): direct_plan(m, group) for m in range(512, 4200, 3)}
+    for cfg in plans.values():
+        assert cfg["w"] >= 2 and cfg["a"] <= cfg["w"] and cfg["n_mma"] == 1
+        for seed in range(6):
+            rng = random.Random(seed)
+            ku = rng.choice([1, 2, 3, 5, 8, 64])
+            Model(rng, cfg, rng.randint(1, 40), ku, first=rng.randint(0, 2 * ku), early=seed % 2 == 1).run()

@@ -15,7 +15,9 @@
 //                             of the packed layout holds rows g / g + 8 of a strip, which is that store's (lane, column) pattern
 //   B operand               = activations in shared memory (no-swizzle K-major core matrices), one bulk copy per 128 k out of
 //                             a copy of x that stage_x_kernel has put into that order (the k order inside a 32-k block is the
-//                             store's: column 4 i + c holds k = 8 c + 2 i, 2 i + 1, so neither side shuffles)
+//                             store's: column 4 i + c holds k = 8 c + 2 i, 2 i + 1, so neither side shuffles); or, DIRECT, straight
+//                             out of x by TMA (rows of 128 swizzled bytes, k in its own order), and the dequant warps turn the
+//                             weights round to match (wq_turn_int4, wq_turn_int8), which takes no staging but 12 instructions a word
 //   D                       = fp32 in tensor memory
 //
 // PAIR: two CTAs of a cluster work on 256 weight rows x NT activation rows with cta_group::2 MMAs: each dequantizes its own
@@ -58,11 +60,13 @@ constexpr int kWqSlots = 4;                    // ring of A in tensor memory: 64
 constexpr int kWqMaxW = 16, kWqMaxX = 8;       // rings of weights and of tiles of x
 constexpr int kWqPitch = 128 * 2 + 16;         // bytes of a row of the output tile in shared memory (rows land on distinct banks)
 constexpr int kWqHeader = 1024;                // mbarriers, TMEM base, give-up flag
+constexpr int kWqDirectRows = 512, kWqDirectN = 8192;  // from and up to which the GEMM reads the activations where they are (wq_plan)
 constexpr int kWqMaxSplitTiles = 16;           // tiles per worker from which whole tiles are dealt out (imbalance <= 1/16)
 
 struct WqParams {
   CUtensorMap wmap;          // weights: rows = strips, row = the strip's bytes; box = 8 strips x 128 k
   CUtensorMap smap;          // int4 scale / zero: rows = strips, row = 16 words per group; box = 8 strips x the unit's groups
+  CUtensorMap xmap;          // DIRECT, activations: box = BR rows x 64 k, 128 bytes per row, 16-byte pieces swizzled; zeros past M and Kx
   const uint8_t* xt;         // staged activations [MT * ranks][KU][x_bytes]
   const uint32_t *packed, *sz;  // DEFER: what the maps show, for sums that are done again
   const __nv_bfloat16* scale8;
@@ -72,7 +76,7 @@ struct WqParams {
   uint32_t* tickets;         // [tiles][ranks], zeroed by the staging kernel
   int64_t N_out, ldy, ld_res;
   int M, Kp, NT, BR, KU, MT, w_slots, x_slots, a_slots, n_mma, vec_store;
-  uint32_t off_w;            // weight ring
+  uint32_t off_x, off_w;     // activation ring, weight ring
   long long wait_limit;      // clocks after which a wait gives up
   uint32_t x_bytes;          // one unit of staged activations (and, DEFER, its sums)
   int quantum, base, rem;    // worker c owns units [first(c), first(c + 1)), first(c) = (c base + min(c, rem)) quantum
@@ -134,6 +138,14 @@ __global__ void __launch_bounds__(256) stage_x_kernel(const __nv_bfloat16* __res
       if ((quarter * 32) % SEG == 0) reinterpret_cast<float*>(unit + (int64_t)BR * 256)[(quarter * 32 / SEG) * 16 + r] = s;
     }
   }
+}
+
+// DIRECT: nothing to stage, but the tickets (n >= 1 words); lets the GEMM go as stage_x_kernel does
+__global__ void __launch_bounds__(256) clear_tickets_kernel(uint32_t* __restrict__ tickets, int n, bool settled) {
+  if (settled) grid_launch_dependents();
+  grid_dependency_wait();
+  if (!settled) grid_launch_dependents();
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) tickets[i] = 0u;
 }
 
 // ---- PTX wrappers ------------------------------------------------------------------------------------------------------
@@ -271,6 +283,30 @@ __device__ __forceinline__ bool any_inf_bf16(uint4 v) {
   const auto half = [](uint32_t w) { return (w & 0x7F80u) == 0x7F80u || (w & 0x7F800000u) == 0x7F800000u; };
   return half(v.x) || half(v.y) || half(v.z) || half(v.w);
 }
+// Between the four lanes c of a row group: lane c has of each of two words the weights k = 8 c + 2 i, + 1 (i = 0 .. 3, pair i at bits 4 i and 16 + 4 i)
+// and gets those of k = 8 c' + 2 c, + 1 (c' = 0 .. 3, at bits 4 c' and 16 + 4 c'): the place of a pair in the word and the lane change roles, first
+// their upper bits (bytes), then their lower ones (half bytes).
+__device__ __forceinline__ void wq_turn_int4(uint32_t& a, uint32_t& b, int lane) {
+  constexpr uint32_t kLow = 0x0F0F0F0Fu;
+  const bool up = lane & 2, odd = lane & 1;
+  uint32_t r = __shfl_xor_sync(0xffffffffu, __byte_perm(a, b, up ? 0x6420u : 0x7531u), 2);
+  a = __byte_perm(a, r, up ? 0x3514u : 0x5240u);
+  b = __byte_perm(b, r, up ? 0x3716u : 0x7260u);
+  const uint32_t keep = odd ? ~kLow : kLow, s0 = odd ? 0u : 4u, s4 = 4u - s0;
+  r = __shfl_xor_sync(0xffffffffu, ((a >> s0) & kLow) | ((b << s4) & ~kLow), 1);
+  a = (a & keep) | ((r << s0) & ~keep);
+  b = (b & keep) | ((r >> s4) & ~keep);
+}
+// the same for bytes: a has the pairs i = 0, 1, b has 2, 3; after it a has those of c' = 0, 1, b of c' = 2, 3
+__device__ __forceinline__ void wq_turn_int8(uint32_t& a, uint32_t& b, int lane) {
+  const bool up = lane & 2, odd = lane & 1;
+  uint32_t r = __shfl_xor_sync(0xffffffffu, up ? a : b, 2);
+  a = up ? r : a;
+  b = up ? b : r;
+  r = __shfl_xor_sync(0xffffffffu, __byte_perm(a, b, odd ? 0x5410u : 0x7632u), 1);
+  a = __byte_perm(a, r, odd ? 0x3254u : 0x5410u);
+  b = __byte_perm(b, r, odd ? 0x3276u : 0x7610u);
+}
 // ring position: slot and the parity of its current use
 struct WqRing {
   int slot = 0;
@@ -287,7 +323,7 @@ struct WqRing {
 // ---- the GEMM ----------------------------------------------------------------------------------------------------------
 // G == 0: int8.  Shared memory: header, output tile, activation ring (x_slots x x_bytes), weight ring (w_slots x [8 strips x 128 k]
 // [8 strips x parameters]).
-template <int G, bool DEFER, bool PAIR, bool EARLY>
+template <int G, bool DEFER, bool PAIR, bool DIRECT, bool EARLY>
 __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_constant__ WqParams p) {
   extern __shared__ __align__(1024) uint8_t wq_smem[];
   constexpr bool kI8 = (G == 0);
@@ -310,7 +346,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_base_s + 1);
   volatile int* s_last = dead + 1;        // [3]: this CTA was the last to reach its first / last tile; it finishes its last tile from its accumulators
   uint8_t* stage = wq_smem + kWqHeader;   // output tile [NT][kWqPitch]
-  uint8_t* xring = stage + p.NT * kWqPitch;
+  uint8_t* xring = wq_smem + p.off_x;
   uint8_t* wring = wq_smem + p.off_w;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int worker = blockIdx.x / kRanks, rank = blockIdx.x % kRanks;
@@ -462,19 +498,26 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     if (wq_elect_one()) {
       WqRing x;
       const int64_t tile_bytes = (int64_t)KU * p.x_bytes;
-      const uint8_t* base = p.xt + rank * tile_bytes;
+      const uint8_t* base = DIRECT ? nullptr : p.xt + rank * tile_bytes;
       int mt = t_first % p.MT, ku = ku_first;
-      const uint8_t* src = base + mt * (kRanks * tile_bytes) + (int64_t)ku * p.x_bytes;
+      const uint8_t* src = DIRECT ? nullptr : base + mt * (kRanks * tile_bytes) + (int64_t)ku * p.x_bytes;
       for (int u = u0; u < u1; ++u) {
         if (!wait(DEFER ? &dread[x.slot] : &xdone[x.slot], x.use ^ 1u)) break;
         mbar_arrive_expect_tx(&xfull[x.slot], p.x_bytes);
-        bulk_g2s(xring + (uint32_t)x.slot * p.x_bytes, src, p.x_bytes, &xfull[x.slot]);
+        uint8_t* dst = xring + (uint32_t)x.slot * p.x_bytes;
+        if constexpr (DIRECT) {
+          const int row = (mt * kRanks + rank) * p.BR;
+          wq_tma_2d(dst, &p.xmap, ku * 128, row, &xfull[x.slot]);
+          wq_tma_2d(dst + p.BR * 128, &p.xmap, ku * 128 + 64, row, &xfull[x.slot]);
+        } else {
+          bulk_g2s(dst, src, p.x_bytes, &xfull[x.slot]);
+          src += p.x_bytes;
+        }
         x.step(1, x_slots);
-        src += p.x_bytes;
         if (++ku == KU) {
           ku = 0;
           if (++mt == p.MT) mt = 0;
-          src = base + mt * (kRanks * tile_bytes);
+          if (!DIRECT) src = base + mt * (kRanks * tile_bytes);
         }
       }
     }
@@ -496,9 +539,11 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
       x.step(mw, x_slots);
       a.step(mw, a_slots);
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)NT >> 3) << 17) | (((128u * kRanks) >> 4) << 24);
-      const uint32_t chunk = (uint32_t)p.BR * 16;  // bytes between consecutive 8-k chunks of the B tile
-      const uint32_t desc_hi = (128u >> 4) | (1u << 14), kstep = (2 * chunk) >> 4;
-      const uint32_t desc_lo = ((chunk >> 4) << 16) | (smem_u32(xring) >> 4), xstep = p.x_bytes >> 4;
+      // B tile: chunks of 8 k, `chunk` bytes from one to the next.  DIRECT: [64 k][BR rows][128 bytes], 1024 bytes from 8 rows to the next
+      const uint32_t chunk = (uint32_t)p.BR * 16;
+      const uint32_t desc_hi = DIRECT ? (1024u >> 4) | (1u << 14) | (2u << 29) : (128u >> 4) | (1u << 14);
+      const uint32_t kstep = DIRECT ? 32u >> 4 : (2 * chunk) >> 4, khalf = DIRECT ? ((uint32_t)p.BR * 128 - 4 * 32) >> 4 : 0u;
+      const uint32_t desc_lo = (DIRECT ? 0u : (chunk >> 4) << 16) | ((smem_u32(xring) & 0x3FFFFu) >> 4), xstep = p.x_bytes >> 4;
       int u = u0;
       bool ok = true;
       while (u < (mw < n_mma ? u1 : u0)) {
@@ -518,7 +563,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
             const uint32_t d0 = DEFER ? tb + x.slot * (kSegs * 16) : dcol;
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks) {
-              const uint64_t bdesc = ((uint64_t)desc_hi << 32) | (b0 + ks * kstep);
+              const uint64_t bdesc = ((uint64_t)desc_hi << 32) | (b0 + ks * kstep + (ks >= 4 ? khalf : 0u));
               wq_mma<PAIR>(d0 + (DEFER ? ks / (8 / kSegs) * 16 : 0), a0 + 8 * ks, bdesc, idesc, DEFER ? (ks % (8 / kSegs) != 0) : (ks != 0 ? 1u : acc));
             }
             wq_commit<PAIR>(&adone[a.slot]);
@@ -577,6 +622,17 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     fetch(u0 + set);
     for (int u = u0 + set; u < u1; u += 2) {
       uint32_t r[32];
+      if constexpr (DIRECT) {  // x is in its own order, so the weights have to be
+#pragma unroll
+        for (int j = 0; j < kWords; j += kI8 ? 4 : 2) {
+          if constexpr (kI8) {
+            wq_turn_int8(wd[j], wd[j + 2], lane);
+            wq_turn_int8(wd[j + 1], wd[j + 3], lane);
+          } else {
+            wq_turn_int4(wd[j], wd[j + 1], lane);
+          }
+        }
+      }
       if constexpr (kI8) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {  // 32-k quarters of the unit; lane chunk: words (row g, k 0-3), (g+8, k 0-3), (g, k 4-7), (g+8, k 4-7)
@@ -856,7 +912,7 @@ static int wq_sm_count() {
 
 // how one call is cut up; a pure function of the shape, so the workspace size is too
 struct WqPlan {
-  bool defer, pair;
+  bool defer, pair, direct;
   int NT, BR, MT, NB, KU, ranks, workers, quantum, base, rem;
   int64_t tiles, n_tickets;
   uint32_t x_bytes;
@@ -867,6 +923,11 @@ static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
   if (M <= 0 || Np % 128 != 0 || Kp % 64 != 0 || M > ((int64_t)1 << 24)) return false;
   w.defer = int4 && M <= 16;
   w.pair = M > 32;
+  // Staging takes time by M x K, reading in place (the weights turned round among the lanes) by the units, M x K x N.  Staged / in place, us: int8
+  // 4096 x 14336, 1000 rows 102.4 / 97.5, 700 rows 74.8 / 72.1; int4 4096 x 14336, 700 / 1000 rows 72.0 / 67.3, 97.8 / 92.4; 6144 x 4096 and 4096 x 4096, 700 rows
+  // 41.5 / 39.2, 34.9 / 33.4; int8 8192 x 8192, 2048 rows 217.5 / 215; but int4 14336 x 4096, 700 and 2048 rows 65.2 / 65.6, 166.4 / 166.3; 300 rows of 4096 x 14336
+  // 40.6 / 42.7, 64 rows of 28672 x 8192 51.4 / 58.8, where the lanes' turn lengthens the way from a unit's weights to its product
+  w.direct = M >= kWqDirectRows && Np <= kWqDirectN;
   w.ranks = w.pair ? 2 : 1;
   w.MT = (int)((M + 255) / 256);
   w.NT = (int)(((M + w.MT - 1) / w.MT + 15) / 16 * 16);
@@ -886,7 +947,7 @@ static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
   auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
   w.off_part = up(w.n_tickets * 4);
   w.off_xt = w.off_part + (w.quantum > 1 ? 0 : up((int64_t)w.workers * 2 * w.ranks * w.NT * 512));
-  w.bytes = w.off_xt + up((int64_t)w.MT * w.ranks * w.KU * w.x_bytes);
+  w.bytes = w.off_xt + up((int64_t)w.MT * w.ranks * w.KU * w.x_bytes);  // (DIRECT too: a workspace for many rows does for fewer)
   return true;
 }
 
@@ -901,12 +962,15 @@ static WqEncode wq_encode_fn() {
   }();
   return fn;
 }
-// rows of `row_bytes`, read in boxes of 8 rows x box elements
-static bool wq_map(CUtensorMap* map, CUtensorMapDataType type, int elem, const void* base, int64_t row_bytes, int64_t rows, int box) {
-  const cuuint64_t dims[2] = {(cuuint64_t)(row_bytes / elem), (cuuint64_t)rows}, strides[1] = {(cuuint64_t)row_bytes};
-  const cuuint32_t boxes[2] = {(cuuint32_t)box, 8}, steps[2] = {1, 1};
+// rows of `row_bytes`, `pitch` apart (0: one behind the other), read in boxes of 8 rows x box elements
+// or of box_rows, then swizzled as rows of 128 bytes
+static bool wq_map(CUtensorMap* map, CUtensorMapDataType type, int elem, const void* base, int64_t row_bytes, int64_t rows, int box, int64_t pitch = 0,
+                   int box_rows = 0) {
+  const cuuint64_t dims[2] = {(cuuint64_t)(row_bytes / elem), (cuuint64_t)rows}, strides[1] = {(cuuint64_t)(pitch ? pitch : row_bytes)};
+  const cuuint32_t boxes[2] = {(cuuint32_t)box, (cuuint32_t)(box_rows ? box_rows : 8)}, steps[2] = {1, 1};
   auto encode = [&]() {
-    return wq_encode_fn()(map, type, 2, const_cast<void*>(base), dims, strides, boxes, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+    return wq_encode_fn()(map, type, 2, const_cast<void*>(base), dims, strides, boxes, steps, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          box_rows ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   };
   if (encode()) return true;
@@ -915,7 +979,7 @@ static bool wq_map(CUtensorMap* map, CUtensorMapDataType type, int elem, const v
   return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess && encode();
 }
 
-template <int G, bool DEFER, bool PAIR>
+template <int G, bool DEFER, bool PAIR, bool DIRECT>
 static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
   constexpr uint32_t kWSlot = 8 * 2 * (G == 0 ? 1024 : 512) + (G == 0 ? 0 : 8 * (G < 128 ? 128 / (G ? G : 128) : 1) * 64);
   constexpr size_t kBudget = 226 * 1024;
@@ -923,7 +987,9 @@ static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
   // tiles of x in flight (an L2 round trip is about 850 clocks; DEFER: as many as there are accumulators); what they and the
   // output tile leave of shared memory holds weights in flight
   p.x_slots = w.x_bytes > 24 * 1024 ? 3 : (w.x_bytes > 12 * 1024 ? 5 : (DEFER && G == 32 ? 4 : 8));  // even where two MMA warps alternate
-  const size_t off_w = (kWqHeader + (size_t)w.NT * kWqPitch + (size_t)p.x_slots * w.x_bytes + 127) / 128 * 128;
+  const size_t unit = DIRECT ? 1024 : 16;      // (rows of 128 swizzled bytes: eight of them have to lie as the hardware counts)
+  p.off_x = (uint32_t)((kWqHeader + (size_t)w.NT * kWqPitch + unit - 1) / unit * unit);
+  const size_t off_w = (p.off_x + (size_t)p.x_slots * w.x_bytes + 127) / 128 * 128;
   p.off_w = (uint32_t)off_w;
   p.w_slots = (int)((kBudget - off_w) / kWSlot);
   if (p.w_slots > kWqMaxW) p.w_slots = kWqMaxW;
@@ -936,9 +1002,9 @@ static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
   // (14336 x 4096, 77 rows: 25.6 -> 25.8; 4096 x 4096 int8, 200 rows: 28.5 -> 29.0).
   constexpr bool kCan = !DEFER;
   const bool early = kCan && (int64_t)w.base * w.quantum >= w.KU;
-  auto kern = wq_gemm_kernel<G, DEFER, PAIR, false>;
+  auto kern = wq_gemm_kernel<G, DEFER, PAIR, DIRECT, false>;
   static OncePerDevice once[2];
-  if (early) kern = wq_gemm_kernel<G, DEFER, PAIR, kCan>;
+  if (early) kern = wq_gemm_kernel<G, DEFER, PAIR, DIRECT, kCan>;
   if (!dynamic_smem(once[early], kern, (int)kBudget)) return AO_B200_ERR_CUDA;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(w.workers * w.ranks));
@@ -979,6 +1045,19 @@ static int wq_stage(const void* x, int64_t M, int64_t Kx, int64_t ldx, const WqP
              : AO_B200_ERR_CUDA;
 }
 
+static int wq_clear(uint32_t* tickets, int64_t n, bool settled, cudaStream_t s) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(n > 148 * 256 ? 148 : (n + 255) / 256 + (n == 0)));
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, clear_tickets_kernel, tickets, (int)n, settled) == cudaSuccess ? AO_B200_OK : AO_B200_ERR_CUDA;
+}
+
 // x [M][ldx] bf16 (first Kx columns valid), y [M][ldy] bf16.  G == 0: int8 weights (`sz` is then the bf16 per-row scale)
 static int wq_gemm(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np, int64_t Kp, int G, void* y,
                    int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res, void* workspace, int64_t workspace_bytes, cudaStream_t s) {
@@ -990,7 +1069,7 @@ static int wq_gemm(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void
   const bool ok = G ? wq_map(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, packed, Kp * 8, Np / 16, 256) &&
                           wq_map(&p.smap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, sz, Kp / G * 64, Np / 16, (G < 128 ? 128 / G : 1) * 16)
                     : wq_map(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_INT64, 8, packed, Kp * 16, Np / 16, 256);
-  if (!ok) return AO_B200_ERR_UNSUPPORTED;
+  if (!ok || (w.direct && !wq_map(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, Kx * 2, M, 64, ldx * 2, w.BR))) return AO_B200_ERR_UNSUPPORTED;
   p.tickets = reinterpret_cast<uint32_t*>(ws);
   p.part = reinterpret_cast<float*>(ws + w.off_part);
   p.xt = ws + w.off_xt;
@@ -1022,15 +1101,21 @@ static int wq_gemm(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void
   std::lock_guard<std::mutex> lock(together);
   const bool settled = residual != nullptr;  // (ao_b200_mm_residual's contract)
   int rc;
-  if (!w.defer) rc = wq_stage<0>(x, M, Kx, ldx, w, ws + w.off_xt, p.tickets, settled, s);
+  if (w.direct) rc = wq_clear(p.tickets, w.n_tickets, settled, s);
+  else if (!w.defer) rc = wq_stage<0>(x, M, Kx, ldx, w, ws + w.off_xt, p.tickets, settled, s);
   else if (G == 32) rc = wq_stage<32>(x, M, Kx, ldx, w, ws + w.off_xt, p.tickets, settled, s);
   else if (G == 64) rc = wq_stage<64>(x, M, Kx, ldx, w, ws + w.off_xt, p.tickets, settled, s);
   else rc = wq_stage<128>(x, M, Kx, ldx, w, ws + w.off_xt, p.tickets, settled, s);
   if (rc != AO_B200_OK) return rc;
   switch (G) {
-    case 0: return w.pair ? wq_launch<0, false, true>(p, w, s) : wq_launch<0, false, false>(p, w, s);
-#define AO_WQ(GG) \
-  case GG: return w.defer ? wq_launch<GG, true, false>(p, w, s) : (w.pair ? wq_launch<GG, false, true>(p, w, s) : wq_launch<GG, false, false>(p, w, s));
+    case 0:
+      return w.direct ? wq_launch<0, false, true, true>(p, w, s)
+                      : (w.pair ? wq_launch<0, false, true, false>(p, w, s) : wq_launch<0, false, false, false>(p, w, s));
+#define AO_WQ(GG)                                                                                        \
+  case GG:                                                                                               \
+    return w.direct ? wq_launch<GG, false, true, true>(p, w, s)                                          \
+                    : (w.defer ? wq_launch<GG, true, false, false>(p, w, s)                              \
+                               : (w.pair ? wq_launch<GG, false, true, false>(p, w, s) : wq_launch<GG, false, false, false>(p, w, s)));
     AO_WQ(32)
     AO_WQ(64)
     AO_WQ(128)
