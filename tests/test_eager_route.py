@@ -147,3 +147,75 @@ def test_weights_that_are_not_on_the_device_are_refused():
     for p, s in ((packed.cpu(), scale), (packed, scale.cpu())):
         with pytest.raises(RuntimeError, match="CUDA"):
             T.b200_int8_weight_only_mm(x, p, s)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 3, 17, 64])
+@pytest.mark.parametrize("bits,call,op", CALLS)
+def test_the_native_host_side_gives_what_the_python_one_gives(bits, call, op, rows, monkeypatch):
+    host = ops._host()
+    assert host is not None, "python -m torchao_fork_b200.build host"
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    w = torch.randn(320, 512, generator=gen, device="cuda").bfloat16()
+    if bits == 4:
+        packed, sz = T.b200_int4_quantize_pack(w, 64, 1e-6, True)
+        rest = (packed, 64, sz, 320)
+    else:
+        q, scale = T.b200_int8_quantize(w, 1e-6, True)
+        rest = (T.b200_int8_pack(q), scale)
+    native, scratch = (host.int4_mm, ops._int4_scratch) if bits == 4 else (host.int8_mm, ops._int8_scratch)
+    big = torch.randn(rows + 1, 1032, generator=gen, device="cuda").bfloat16()
+    stream = torch.cuda.Stream()
+    for x, taken in ((big[:rows, :512], True), (big[1:, 8:520], True), (big[:rows, :504], True), (big[:rows, 1:513], False), (big[:rows, :511], False),
+                     (big[:rows, :1024:2], False), (big[:0, :512], False), (big[:rows, :512].contiguous(), True)):
+        y = native(x, *rest, scratch)
+        assert (type(y) is torch.Tensor) == taken and (taken or y is None)
+        if not taken and x.shape == (1, 512):   # (one row off 16 bytes counts as contiguous and is refused behind Python too)
+            continue
+        want = op(x, *rest)
+        assert torch.equal(call(x, *rest), want) and (not taken or torch.equal(y, want))
+        with torch.cuda.stream(stream), torch.inference_mode():
+            stream.wait_stream(torch.cuda.default_stream())
+            inside = call(x, *rest)
+            assert inside.is_inference() and torch.equal(inside, want)
+        torch.cuda.default_stream().wait_stream(stream)
+    for x in (big[:rows, :512].float(), big[:rows, :512].cpu(), big[0, :512]):
+        assert native(x, *rest, scratch) is None
+    wrong = big[:rows, :520]
+    assert native(wrong, *rest, scratch) is None
+    with pytest.raises(RuntimeError):
+        call(wrong, *rest)
+    monkeypatch.setattr(ops, "_host", lambda: None)
+    assert torch.equal(call(big[:rows, :512], *rest), op(big[:rows, :512], *rest))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("recipe", ["int4", "hqq", "int8"])
+def test_a_quantized_weight_is_a_parameter_like_any_other(recipe):
+    import copy
+
+    import torchao_fork_b200 as ao
+    config = ao.Int8WeightOnlyConfig() if recipe == "int8" else ao.Int4WeightOnlyConfig(group_size=64, use_hqq=recipe == "hqq")
+    lin = torch.nn.Linear(256, 128, bias=False, device="cuda", dtype=torch.bfloat16)
+    x, w = torch.randn(4, 256, device="cuda").bfloat16(), lin.weight.detach().clone()
+    ao.quantize_(lin, config)
+    p = lin.weight
+    assert isinstance(p, torch.nn.Parameter) and not p.requires_grad and p.is_leaf and [n for n, _ in lin.named_parameters()] == ["weight"]
+    y = lin(x)
+    for other in (copy.deepcopy(lin), torch.nn.Linear(256, 128, bias=False, device="meta", dtype=torch.bfloat16)):
+        if other.weight.is_meta:
+            other.load_state_dict(lin.state_dict(), assign=True)
+        assert isinstance(other.weight, torch.nn.Parameter) and type(other.weight) is type(p) and torch.equal(other(x), y)
+    # the dispatcher's way, as under a profile, makes the same
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        again = torch.nn.Linear(256, 128, bias=False, device="cuda", dtype=torch.bfloat16)
+        again.weight = torch.nn.Parameter(w, requires_grad=False)
+        ao.quantize_(again, config)
+    assert any("b200_int" in e.name for e in prof.events())
+    for n in p.tensor_impl.__tensor_flatten__()[0]:
+        assert torch.equal(getattr(p.tensor_impl, n), getattr(again.weight.tensor_impl, n))
+    # a weight that the config does not fit stays what it was, a parameter of its own
+    odd = torch.nn.Linear(250, 128, bias=False, device="cuda", dtype=torch.bfloat16)
+    if recipe == "int4":
+        ao.quantize_(odd, config)
+        assert type(odd.weight) is torch.nn.Parameter

@@ -127,6 +127,24 @@ def lib():
     return _lib
 
 
+def host():
+    """The native host side of the eager linears (csrc/host), bound to the loaded library; None where it has not been built for this torch and
+    this Python (the same steps then run in Python, before the same kernels)."""
+    import importlib.machinery
+    import importlib.util
+
+    from . import build as _build
+    path = _build.host_path()
+    if not os.path.exists(path):
+        return None
+    loader = importlib.machinery.ExtensionFileLoader("ao_b200_host", path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("ao_b200_host", loader, origin=path))
+    loader.exec_module(module)
+    names = ("ao_b200_int4_mm", "ao_b200_int4_mm_workspace_bytes", "ao_b200_int8_mm", "ao_b200_int8_mm_workspace_bytes")
+    module.bind(*(ctypes.cast(getattr(lib(), n), ctypes.c_void_p).value for n in names))
+    return module
+
+
 def check(code, what):
     if code != 0:
         msg = lib().ao_b200_error_string(code).decode()

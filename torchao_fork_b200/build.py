@@ -1,12 +1,16 @@
 """Build the CUDA libraries (sm_100a) in-tree with nvcc.  No torch dependency: each library is a plain C-ABI shared
-object.  Two targets, built independently so that a model only compiles what it runs:
+object.  Two targets, built independently so that a model only compiles what it runs, and the native host side of the eager linears,
+which belongs to one version of torch and of Python (its file name says which; without it the same steps run in Python):
     core  lib/libao_b200.so      csrc/*.cu      weight-only quantized linears, the Llama decode kernels (include/ao_b200.h)
     lm    lib/libao_b200_lm.so   csrc/lm/*.cu   sequence-model mechanisms on an fp32 residual stream (include/ao_b200_lm.h)
-Usage: python -m torchao_fork_b200.build [core|lm|all] [-v] [-f]"""
+    host  lib/ao_b200_host.*.so  csrc/host/*.cpp
+Usage: python -m torchao_fork_b200.build [core|lm|host|all] [-v] [-f]"""
 import fcntl
 import os
+import re
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -37,16 +41,44 @@ def _stale(out, deps):
 
 
 def build(verbose=False, force=False, target="core"):
-    """Compiles what is stale of `target` ("core", "lm" or "all") and links it; returns the library's path (the core
+    """Compiles what is stale of `target` ("core", "lm", "host" or "all") and links it; returns the library's path (the core
     library's for "all").  Safe to call from several processes at once (a lock file serialises them)."""
     if target == "all":
+        build(verbose, force, "host")
         build(verbose, force, "lm")
         return build(verbose, force, "core")
     os.makedirs(LIBDIR, exist_ok=True)
     os.makedirs(OBJDIR, exist_ok=True)
     with open(os.path.join(OBJDIR, f".{target}.lock"), "w") as lock:
         fcntl.flock(lock, fcntl.LOCK_EX)
-        return _build_locked(verbose, force, target)
+        return _build_host(verbose, force) if target == "host" else _build_locked(verbose, force, target)
+
+
+def host_path():
+    """Where the host module for this torch and this Python lies."""
+    import torch
+    return os.path.join(LIBDIR, "ao_b200_host." + re.sub(r"[^0-9A-Za-z]+", "_", f"{sys.implementation.cache_tag}-torch-{torch.__version__}") + ".so")
+
+
+def _build_host(verbose, force):
+    import torch
+    out, src_dir = host_path(), os.path.join(CSRC, "host")
+    srcs = sorted(os.path.join(src_dir, f) for f in os.listdir(src_dir) if f.endswith(".cpp"))
+    if force or _stale(out, srcs):
+        base = os.path.dirname(torch.__file__)
+        include = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
+                   os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")]
+        tmp = out + f".{os.getpid()}.tmp"
+        cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               *(a for i in include for a in ("-isystem", i)), *srcs, "-o", tmp, "-L" + os.path.join(base, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+               "-ltorch_python"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if verbose or r.returncode:
+            sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+        if r.returncode:
+            raise RuntimeError("g++ failed: " + " ".join(cmd))
+        os.replace(tmp, out)
+    return out
 
 
 def _build_locked(verbose, force, target):

@@ -107,6 +107,7 @@ class AffineQuantizedTensor(torch.Tensor):
         """reference: affine_quantized_tensor.py:231-373.  The reference runs pre_process ->
         choose_qparams -> quantize -> post_process -> from_plain as ~15 eager kernels; the two
         supported recipes are each ONE fused B200 kernel here (results bit-identical)."""
+        from .. import ops as _ops
         from .layouts import PlainAQTTensorImpl, TensorCoreTiledAQTTensorImpl, TensorCoreTiledLayout
 
         if zero_point_domain is None:
@@ -147,7 +148,7 @@ class AffineQuantizedTensor(torch.Tensor):
             if use_hqq:
                 # reference: affine_quantized_tensor.py:252-288 -> _choose_qparams_and_quantize_affine_hqq with
                 # nbits = log2(quant_max + 1), axis = 1, group_size = max(block_size), raw_output = False
-                packed, sz = torch.ops.torchao.b200_int4_hqq_quantize_pack(
+                packed, sz = _ops.int4_hqq_quantize_pack(
                     input_float if input_float.dtype is torch.bfloat16 else input_float.to(torch.bfloat16), int(block_size[1]))
                 tensor_impl = TensorCoreTiledAQTTensorImpl(packed, sz, False, _layout)
                 return cls(tensor_impl, block_size, original_shape, quant_min, quant_max, zero_point_domain,

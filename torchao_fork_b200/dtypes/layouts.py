@@ -86,7 +86,7 @@ class TensorCoreTiledAQTTensorImpl(AQTTensorImpl):
     @classmethod
     def from_hp(cls, weight: torch.Tensor, group_size: int, eps: float, _layout: Layout):
         """bf16 (N, K) -> storage in ONE kernel (pad + qparams + quantize + pack)."""
-        packed, sz = torch.ops.torchao.b200_int4_quantize_pack(weight, group_size, eps, _qp.CUDA_DIV_SEMANTICS)
+        packed, sz = _ops.int4_quantize_pack(weight, group_size, eps, _qp.CUDA_DIV_SEMANTICS)
         return cls(packed, sz, False, _layout)
 
     @classmethod
@@ -217,7 +217,7 @@ def _aqt_is_tensor_core_tile_uint4(aqt):
 def _linear_bf16_act_uint4_weight_check(input_tensor, weight_tensor, bias):
     """reference: tensor_core_tiled_layout.py:58-71"""
     return (
-        not is_traceable_wrapper_subclass(input_tensor)
+        (type(input_tensor) is torch.Tensor or not is_traceable_wrapper_subclass(input_tensor))
         and input_tensor.dtype == torch.bfloat16
         and isinstance(weight_tensor, AffineQuantizedTensor)
         and _aqt_is_tensor_core_tile_uint4(weight_tensor)
@@ -285,9 +285,9 @@ class PlainAQTTensorImpl(AQTTensorImpl):
     @classmethod
     def from_hp(cls, weight, eps, zero_point_dtype, _layout):
         """bf16 (N, K) -> int8 data + scale in ONE kernel, then the strip-major pack."""
-        q, scale = torch.ops.torchao.b200_int8_quantize(weight, eps, _qp.CUDA_DIV_SEMANTICS)
+        q, scale = _ops.int8_quantize(weight, eps, _qp.CUDA_DIV_SEMANTICS)
         zp = torch.zeros(scale.shape, dtype=zero_point_dtype, device=weight.device)
-        return cls(torch.ops.torchao.b200_int8_pack(q), scale, zp, _layout, q.shape)
+        return cls(_ops.int8_pack(q), scale, zp, _layout, q.shape)
 
     @classmethod
     def from_plain(cls, int_data, scale, zero_point, _layout):
@@ -363,7 +363,7 @@ def _aqt_is_int8(aqt):
 def _linear_fp_act_int8_weight_check(input_tensor, weight_tensor, bias):
     """reference: plain_layout.py:232-247"""
     return (
-        not is_traceable_wrapper_subclass(input_tensor)
+        (type(input_tensor) is torch.Tensor or not is_traceable_wrapper_subclass(input_tensor))
         and input_tensor.is_floating_point()
         and isinstance(weight_tensor, AffineQuantizedTensor)
         and _aqt_is_int8(weight_tensor)

@@ -216,6 +216,8 @@ def _dequant_tinygemm_cuda(packed_w: Tensor, scales_and_zeros: Tensor, group_siz
 
 # ------------------------------------------------------------------ B200 int4 ops
 def _w_checks(w, group_size):
+    if w.dim() == 2 and w.is_cuda and w.dtype is torch.bfloat16 and group_size in (32, 64, 128, 256) and w.size(1) % group_size == 0:
+        return
     torch._check(w.dim() == 2, lambda: f"weight must be 2-D, got {w.dim()}D")
     _check_cuda_bf16(w, "weight")
     _check_group(group_size)
@@ -246,14 +248,23 @@ def _int4_quantize_pack_cuda(w: Tensor, group_size: int, eps: float, cuda_div_se
     n, k = w.shape
     np_, kp = padded_int4_shape(n, k, group_size)
     w, ldw = _rows(w)
-    packed = torch.empty((np_ // 16, kp // 64, 32, 4), dtype=torch.int32, device=w.device)
-    sz = torch.empty((np_ // 16, kp // group_size, 16, 2), dtype=torch.bfloat16, device=w.device)
-    with torch.cuda.device(w.device):
-        _lib.check(_lib.lib().ao_b200_int4_quantize_pack(
+    device = w.device
+    packed = torch.empty((np_ // 16, kp // 64, 32, 4), dtype=torch.int32, device=device)
+    sz = torch.empty((np_ // 16, kp // group_size, 16, 2), dtype=torch.bfloat16, device=device)
+    with _on(device.index):
+        rc = _lib.lib().ao_b200_int4_quantize_pack(
             w.data_ptr(), n, k, ldw, np_, kp, group_size, eps,
             _lib.DIV_RECIP if cuda_div_semantics else _lib.DIV_IEEE,
-            packed.data_ptr(), sz.data_ptr(), _stream(w)), "int4_quantize_pack")
+            packed.data_ptr(), sz.data_ptr(), torch._C._cuda_getCurrentRawStream(device.index))
+    _lib.check(rc, "int4_quantize_pack")
     return packed, sz
+
+
+def int4_quantize_pack(w: Tensor, group_size: int, eps: float, cuda_div_semantics: bool):
+    """torch.ops.torchao.b200_int4_quantize_pack, without the dispatcher where that adds nothing (as int4_weight_only_mm)"""
+    if runs_eagerly(w) and not _profiling():
+        return _int4_quantize_pack_cuda(w, group_size, eps, cuda_div_semantics)
+    return torch.ops.torchao.b200_int4_quantize_pack(w, group_size, eps, cuda_div_semantics)
 
 
 @register_custom_op("torchao::b200_int4_choose_qparams")
@@ -332,9 +343,10 @@ def _hqq_search(w, group_size, outputs):
     n, k = w.shape
     L = _lib.lib()
     ws = torch.empty(int(L.ao_b200_hqq_search_workspace_bytes(n * (k // group_size), group_size)), dtype=torch.uint8, device=w.device)
-    with torch.cuda.device(w.device):
-        _lib.check(L.ao_b200_hqq_search(w.data_ptr(), n, k, group_size, HQQ_BETA, HQQ_KAPPA, HQQ_LP_NORM, HQQ_ITERS, ws.data_ptr(), ws.numel(),
-                                        *outputs, _stream(w)), "hqq_search")
+    with _on(w.device.index):
+        rc = L.ao_b200_hqq_search(w.data_ptr(), n, k, group_size, HQQ_BETA, HQQ_KAPPA, HQQ_LP_NORM, HQQ_ITERS, ws.data_ptr(), ws.numel(),
+                                  *outputs, torch._C._cuda_getCurrentRawStream(w.device.index))
+    _lib.check(rc, "hqq_search")
 
 
 @register_custom_op("torchao::b200_int4_hqq_quantize_pack")
@@ -354,6 +366,13 @@ def _int4_hqq_quantize_pack_cuda(w: Tensor, group_size: int):
     sz = torch.empty((np_ // 16, kp // group_size, 16, 2), dtype=torch.bfloat16, device=w.device)
     _hqq_search(w, group_size, (None, None, None, np_, kp, packed.data_ptr(), sz.data_ptr()))
     return packed, sz
+
+
+def int4_hqq_quantize_pack(w: Tensor, group_size: int):
+    """torch.ops.torchao.b200_int4_hqq_quantize_pack, without the dispatcher where that adds nothing (as int4_weight_only_mm)"""
+    if runs_eagerly(w) and not _profiling():
+        return _int4_hqq_quantize_pack_cuda(w, group_size)
+    return torch.ops.torchao.b200_int4_hqq_quantize_pack(w, group_size)
 
 
 @register_custom_op("torchao::b200_int4_pack")
@@ -508,6 +527,18 @@ def _workspace(device, nbytes, tag="int4", stream=None):
     return ws
 
 
+_host = lru_cache(maxsize=1)(_lib.host)
+_device = lru_cache(maxsize=64)(lambda index: torch.device("cuda", index))
+
+
+def _int4_scratch(index, stream, nbytes):
+    return _workspace(_device(index), nbytes, stream=stream)
+
+
+def _int8_scratch(index, stream, nbytes):
+    return _workspace(_device(index), nbytes, "int8", stream)
+
+
 @lru_cache(maxsize=4096)
 def _mm_workspace_bytes(bits, m, np_, kp):
     """A pure function of the shape."""
@@ -524,8 +555,16 @@ def _mm_rows(x):
 
 def int4_weight_only_mm(x: Tensor, packed_w: Tensor, group_size: int, scales_and_zeros: Tensor, out_features: int) -> Tensor:
     """torch.ops.torchao.b200_int4_weight_only_mm, without the dispatcher where that adds nothing (a profile gets its op's name there;
-    weights that are no plain CUDA tensors are refused by the implementation either way)"""
+    weights that are no plain CUDA tensors are refused by the implementation either way).  What follows is native code if it has been built; it
+    answers None to anything that wants mending or refusing."""
     if type(packed_w) is Tensor and type(scales_and_zeros) is Tensor and runs_eagerly(x) and not _profiling():
+        host = _host()
+        if host is not None:
+            y = host.int4_mm(x, packed_w, group_size, scales_and_zeros, out_features, _int4_scratch)
+            if type(y) is Tensor:
+                return y
+            if y is not None:
+                _lib.check(y, "int4_mm")
         return _int4_mm_cuda(x, packed_w, group_size, scales_and_zeros, out_features)
     return torch.ops.torchao.b200_int4_weight_only_mm(x, packed_w, group_size, scales_and_zeros, out_features)
 
@@ -533,6 +572,13 @@ def int4_weight_only_mm(x: Tensor, packed_w: Tensor, group_size: int, scales_and
 def int8_weight_only_mm(x: Tensor, packed_w: Tensor, scale: Tensor) -> Tensor:
     """torch.ops.torchao.b200_int8_weight_only_mm, without the dispatcher where that adds nothing (as above)"""
     if type(packed_w) is Tensor and type(scale) is Tensor and runs_eagerly(x) and not _profiling():
+        host = _host()
+        if host is not None:
+            y = host.int8_mm(x, packed_w, scale, _int8_scratch)
+            if type(y) is Tensor:
+                return y
+            if y is not None:
+                _lib.check(y, "int8_mm")
         return _int8_mm_cuda(x, packed_w, scale)
     return torch.ops.torchao.b200_int8_weight_only_mm(x, packed_w, scale)
 
@@ -582,17 +628,26 @@ def _(w: Tensor, eps: float, cuda_div_semantics: bool):
 
 @_impl_cuda("b200_int8_quantize")
 def _int8_quantize_cuda(w: Tensor, eps: float, cuda_div_semantics: bool):
-    torch._check(w.dim() == 2, lambda: "weight must be 2-D")
-    _check_cuda_bf16(w, "weight")
+    if not (w.dim() == 2 and w.is_cuda and w.dtype is torch.bfloat16):
+        torch._check(w.dim() == 2, lambda: "weight must be 2-D")
+        _check_cuda_bf16(w, "weight")
     w = w.contiguous()
     n, k = w.shape
-    q = torch.empty((n, k), dtype=torch.int8, device=w.device)
-    scale = torch.empty((n,), dtype=torch.bfloat16, device=w.device)
-    with torch.cuda.device(w.device):
-        _lib.check(_lib.lib().ao_b200_int8_quantize(w.data_ptr(), n, k, k, eps,
-                                                    _lib.DIV_RECIP if cuda_div_semantics else _lib.DIV_IEEE,
-                                                    q.data_ptr(), scale.data_ptr(), _stream(w)), "int8_quantize")
+    device = w.device
+    q = torch.empty((n, k), dtype=torch.int8, device=device)
+    scale = torch.empty((n,), dtype=torch.bfloat16, device=device)
+    with _on(device.index):
+        rc = _lib.lib().ao_b200_int8_quantize(w.data_ptr(), n, k, k, eps, _lib.DIV_RECIP if cuda_div_semantics else _lib.DIV_IEEE,
+                                              q.data_ptr(), scale.data_ptr(), torch._C._cuda_getCurrentRawStream(device.index))
+    _lib.check(rc, "int8_quantize")
     return q, scale
+
+
+def int8_quantize(w: Tensor, eps: float, cuda_div_semantics: bool):
+    """torch.ops.torchao.b200_int8_quantize, without the dispatcher where that adds nothing (as int4_weight_only_mm)"""
+    if runs_eagerly(w) and not _profiling():
+        return _int8_quantize_cuda(w, eps, cuda_div_semantics)
+    return torch.ops.torchao.b200_int8_quantize(w, eps, cuda_div_semantics)
 
 
 def padded_int8_shape(n: int, k: int) -> Tuple[int, int]:
@@ -621,11 +676,19 @@ def _int8_pack_cuda(int_data: Tensor):
     int_data = int_data.contiguous()
     n, k = int_data.shape
     np_, kp = padded_int8_shape(n, k)
-    packed = torch.empty((np_ // 16, kp // 64, 1024), dtype=torch.uint8, device=int_data.device)
-    with torch.cuda.device(int_data.device):
-        _lib.check(_lib.lib().ao_b200_int8_pack(int_data.data_ptr(), n, k, np_, kp, packed.data_ptr(), _stream(int_data)),
-                   "int8_pack")
+    device = int_data.device
+    packed = torch.empty((np_ // 16, kp // 64, 1024), dtype=torch.uint8, device=device)
+    with _on(device.index):
+        rc = _lib.lib().ao_b200_int8_pack(int_data.data_ptr(), n, k, np_, kp, packed.data_ptr(), torch._C._cuda_getCurrentRawStream(device.index))
+    _lib.check(rc, "int8_pack")
     return packed
+
+
+def int8_pack(int_data: Tensor):
+    """torch.ops.torchao.b200_int8_pack, without the dispatcher where that adds nothing (as int4_weight_only_mm)"""
+    if runs_eagerly(int_data) and not _profiling():
+        return _int8_pack_cuda(int_data)
+    return torch.ops.torchao.b200_int8_pack(int_data)
 
 
 @register_custom_op("torchao::b200_int8_unpack")
