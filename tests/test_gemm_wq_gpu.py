@@ -385,3 +385,18 @@ def test_activations_read_in_place_out_of_wider_rows(bits, group):
         _lib.check(L.ao_b200_int8_mm(xp, m, kx, ld, packed.data_ptr(), scales.data_ptr(), np_, kp, y.data_ptr(), n, n, ws.data_ptr(), ws.numel(), st), "int8_mm")
     ref = x[1 : m + 1, 24 : 24 + kx].double() @ wd[:, :kx].t()
     assert ((y.double() - ref).norm() / ref.norm()).item() < 2.0 ** -8
+
+
+@pytest.mark.parametrize("k", [64, 192, 256, 320, 1088, 4160])
+@pytest.mark.parametrize("bits,group,m", [(4, 32, 16), (4, 64, 9), (4, 64, 60), (4, 32, 100), (8, 0, 16), (8, 0, 33), (8, 0, 128)])
+def test_long_units(bits, group, m, k):
+    # units of 256 k whose second half is there, in part or not at all; tiles of one unit and of several, shared and whole
+    for n in (128, 640, 16384):
+        _check(bits, m, n, k, group)
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("m", [3, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(12288, 4096), (12160, 4096), (24576, 4096), (24448, 4096), (8192, 24576), (8064, 24576)])
+def test_few_rows_on_both_sides_of_their_lines(bits, m, n, k):
+    _check(bits, m, n, k, 128)

@@ -390,3 +390,28 @@ def test_rings_of_activations_read_in_place(group):
             rng = random.Random(seed)
             ku = rng.choice([1, 2, 3, 5, 8, 64])
             Model(rng, cfg, rng.randint(1, 40), ku, first=rng.randint(0, 2 * ku), early=seed % 2 == 1).run()
+
+
+def long_plan(m, group):
+    """the same for calls of up to 128 rows, whose units have 256 k: rings of half as many slots of operands"""
+    c = plan(m, group)
+    nt = -(-m // 16) * 16
+    xb = 2 * (nt // (2 if c["pair"] else 1) * 256 + (256 if c["defer"] else 0))
+    wb = 2 * (8 * 2 * (512 if group else 1024) + (8 * (128 // group if group < 128 else 1) * 64 if group else 0))
+    c["x"] = 3 if xb > 24 * 1024 else 4 if xb > 9 * 1024 or (c["defer"] and group == 64) else 2 if c["defer"] and group == 32 else 6
+    off = -(-(HEADER + nt * PITCH + c["x"] * xb) // 128) * 128
+    c["w"], c["a"] = min(MAX_W, (BUDGET - off) // wb), A_SLOTS // 2
+    if c["n_mma"] == 2:
+        c["w"] &= ~1
+    return c
+
+
+@pytest.mark.parametrize("group", [0, 32, 64, 128, 256])
+def test_rings_of_long_units(group):
+    plans = {tuple(sorted(long_plan(m, group).items())): (m, long_plan(m, group)) for m in range(1, 129)}
+    for m, cfg in plans.values():
+        assert cfg["w"] >= 2 and (cfg["n_mma"] == 1 or (cfg["w"] % 2 == 0 and cfg["x"] % 2 == 0))
+        for seed in range(8):
+            rng = random.Random(seed)
+            ku = rng.choice([1, 2, 3, 5, 8, 64])
+            Model(rng, cfg, rng.randint(1, 40), ku, first=rng.randint(0, 2 * ku), early=seed % 2 == 1 and not cfg["defer"]).run()

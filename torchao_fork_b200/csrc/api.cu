@@ -89,16 +89,17 @@ int settled_follow() { return tunables().pdl ? ao::kFollowSettled : ao::kFollowP
 }  // namespace
 
 // Which calls of up to 16 rows take the GEMM (gemm_wq_tc.cu) rather than the GEMV that keeps the activations in shared memory.  The GEMM
-// costs about 10 us of staging, launch and tail whatever the size, then streams 16 rows as fast as 3; the GEMV has no such costs but
-// its time grows with the rows.  Measured (GEMV / GEMM, us): int4 28672 x 8192, 8 rows 39 / 46, 12 rows 62 / 46; 14336 x 4096, 8 rows 14 / 20,
-// 12 rows 19.7 / 20.3, 16 rows 23.0 / 20.4; int8 28672 x 8192, 8 rows 51 / 50, 12 rows 66 / 50, 14336 x 4096, 16 rows 25.9 / 22.7; a tie at
-// 4096 x 4096, 16 rows, where the line puts the GEMV.  Where the activations do not fit one CTA, up to 8 rows share k over a cluster if that takes them
-// (share_k, which is asked first); for the others, 9 to 16 rows as a rule, the strip kernels are the other choice: int4 8192 x 28672 62 .. 63 / 45 from 3 to 16
-// rows, 4096 x 14336, 16 rows 18 / 20; int8 8192 x 28672, 16 rows 78 / 51, 4096 x 14336, 12 rows 27 / 23.
+// costs about 10 us of staging, launch and tail whatever the size, then streams 16 rows as fast as 3; the GEMV has no such costs but takes twice the
+// products from 9 rows on.  Measured (GEMV / GEMM, us): int4 8 rows of 28672 x 8192 35.9 / 37.5, of 28672 x 4096 21.2 / 23.9; 9 rows of 14336 x 4096 18.4 / 17.5,
+// 8192 x 8192 20.1 / 18.8, 10240 x 8192 27.3 / 20.8, 28672 x 4096 27.8 / 24.0, but 6144 x 4096 12.7 / 14.1; 16 rows of 6144 x 4096 14.0 / 14.3; int8 9 rows of
+// 28672 x 4096 31.3 / 27.9, 10240 x 8192 26.1 / 26.6, 14336 x 4096 20.1 / 20.2, 16 rows of that 25.9 / 20.8, 9 and 16 of 6144 x 4096 13.1 / 14.9, 15.1 / 15.1.  Where
+// the activations do not fit one CTA, up to 8 rows share k over a cluster if that takes them (share_k, which is asked first); for the others, 9 to 16 rows
+// as a rule, the strip kernels are the other choice: int4 8192 x 28672 62 .. 63 / 38 from 3 to 16 rows, 4096 x 14336, 16 rows 18.2 / 18.5; int8 8192 x 28672,
+// 16 rows 78 / 49, 4096 x 14336, 12 rows 27 / 21.
 static bool few_rows_by_gemm(int64_t M, int64_t Np, int64_t Kp, bool fits, bool int4) {
   if (M < 3 || Np % 128 != 0) return false;
   if (M > 16) return true;
-  if (fits) return (M - 8) * Np * Kp > (int64_t)224 << 20;
+  if (fits) return M > 8 && (Np * Kp >= (int64_t)(int4 ? 48 : 96) << 20 || (M - 8) * Np * Kp > (int64_t)224 << 20);
   return Np * Kp >= (int64_t)128 << 20 || (!int4 && M > 8);
 }
 static bool int4_by_gemm(int64_t M, int64_t Np, int64_t Kp, int G) {
@@ -131,7 +132,9 @@ extern "C" int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
   auto s = static_cast<cudaStream_t>(stream);
   auto xb = static_cast<const __nv_bfloat16*>(x);
   auto yb = static_cast<__nv_bfloat16*>(y);
-  if (ao::share_k(M, Kp, ao::Instead::kNothingFits) && !ao::int4_gemv_fused_fits(M, Kp, group_size, tunables().stages)) {
+  // (a large weight: 8192 x 28672, 3 to 7 rows 41 us with k shared, 37.5 by the GEMM; int8 44 to 48 and 48)
+  if (ao::share_k(M, Kp, ao::Instead::kNothingFits) && !(Np * Kp >= (int64_t)192 << 20 && tunables().gemm_tc && Np % 128 == 0) &&
+      !ao::int4_gemv_fused_fits(M, Kp, group_size, tunables().stages)) {
     const int e = ao::int4_gemv_split(x, M, Kx, ldx, packed, scale_and_zero, Np, Kp, group_size, y, N_out, ldy, nullptr, 0, tunables().stages,
                                       plain_follow(), s);
     if (e != AO_B200_ERR_WORKSPACE) return e;

@@ -24,7 +24,7 @@
 // 128 rows and holds half of the activation tile, so the shared-memory and L2 traffic of the activations is halved.  (One CTA
 // at NT = 256 would need 64 B/clk of shared-memory writes and as much in reads for B alone, of 128 B/clk.)
 //
-// Work split: units of (row block, row tile of x, 128 k), tile-major, dealt out contiguously and evenly to as many CTAs (or
+// Work split: units of (row block, row tile of x, 128 k; up to 128 rows 256 k), tile-major, dealt out contiguously and evenly to as many CTAs (or
 // pairs) as there are SMs.  A tile whose K is shared between neighbours is summed by the one that arrives last, in CTA order
 // (fp32 partial sums and tickets in the workspace; nobody waits for another CTA), so there is no last wave that is nearly
 // empty and few row blocks still fill the chip.
@@ -37,8 +37,11 @@
 // (a shared tile then misses a ticket, so nobody else writes it) and returns once its copies and products in flight are over.
 //
 // Bound by the tensor cores from about 512 rows (8 MMAs of N = 256 take 1024 clocks per unit and pair, the dequant of a unit
-// about 900 clocks per set of warps, two sets in flight), below that by the dequant -> MMA chain of a unit.  Measured, 14336 x 4096,
-// int4 with groups of 128, M = 64 / 256 / 512 / 1000 / 2048: 24.2 / 37.6 / 54.2 / 94 / 174 us, the last 0.85 of 1634 TFLOP/s (one CTA
+// about 900 clocks per set of warps, two sets in flight), below that by the dequant -> MMA chain of a unit: conversions (all 16 warps at them at the
+// same time, 440 clocks per 128 k and set) and, once per unit, the way over six barriers, about 700 clocks of each role.  Hence units of 256 k up to
+// 128 rows: int4 28672 x 8192, 16 / 32 / 64 rows 46.9 / 47.7 / 49.5 -> 37.4 / 38.0 / 41.1 us, 14336 x 4096, 77 rows 26.1 -> 23.8, int8 28672 x 8192 and
+// 14336 x 4096, 16 rows 49.5 -> 46.5, 23.3 -> 20.2; from 144 rows on they give nothing (200 rows 75.2 and 75.3; int8 300 rows 40.2 and 42.5).  Measured,
+// 14336 x 4096, int4 with groups of 128, M = 64 / 256 / 512 / 1000 / 2048: 22 / 37.6 / 54.2 / 94 / 174 us, the last 0.85 of 1634 TFLOP/s (one CTA
 // per 128 x 256 tile with the whole K, activations multicast over 4 CTAs, run-time divisions and parameters read from global memory in
 // the dequant loop: 29.9 / 36.5 / 67.0 / 128 / 225 us); int8 8192 x 8192, M = 32 / 512 / 2048: 24 / 63 / 227 us (44 / 66 / 244 us).
 #include <cuda.h>
@@ -48,6 +51,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "f32x2.h"
 #include "per_device.h"
 
 namespace ao {
@@ -56,11 +60,12 @@ constexpr int kWqEpiWarps = 4, kWqDqWarps = 16;
 constexpr int kWqBehind = 8;  // units (wq_gemm_kernel, t_early; 0, 4 and 16 measure the same, without the path 300 rows of 14336 x 4096 take 41.3 us, not 37.4)
 constexpr int kWqWProd = kWqEpiWarps + kWqDqWarps, kWqXProd = kWqWProd + 1, kWqMma = kWqXProd + 1;
 constexpr int kWqThreads = (kWqMma + 2) * 32;  // 768
-constexpr int kWqSlots = 4;                    // ring of A in tensor memory: 64 columns (128 k) each
+constexpr int kWqSlots = 4;                    // ring of A in tensor memory: 64 columns (128 k) each, or half as many of 256 k
 constexpr int kWqMaxW = 16, kWqMaxX = 8;       // rings of weights and of tiles of x
 constexpr int kWqPitch = 128 * 2 + 16;         // bytes of a row of the output tile in shared memory (rows land on distinct banks)
 constexpr int kWqHeader = 1024;                // mbarriers, TMEM base, give-up flag
 constexpr int kWqDirectRows = 512, kWqDirectN = 8192;  // from and up to which the GEMM reads the activations where they are (wq_plan)
+constexpr int kWqLongNT = 128;                 // rows of a tile up to which a unit has 256 k (both sides: above)
 constexpr int kWqMaxSplitTiles = 16;           // tiles per worker from which whole tiles are dealt out (imbalance <= 1/16)
 
 struct WqParams {
@@ -78,7 +83,7 @@ struct WqParams {
   int M, Kp, NT, BR, KU, MT, w_slots, x_slots, a_slots, n_mma, vec_store;
   uint32_t off_x, off_w;     // activation ring, weight ring
   long long wait_limit;      // clocks after which a wait gives up
-  uint32_t x_bytes;          // one unit of staged activations (and, DEFER, its sums)
+  uint32_t x_bytes, x_sub;   // one unit of staged activations (and, DEFER, its sums), 128 k of it
   int quantum, base, rem;    // worker c owns units [first(c), first(c + 1)), first(c) = (c base + min(c, rem)) quantum
 };
 
@@ -89,7 +94,7 @@ __device__ __forceinline__ int wq_owner(int u, int base, int rem, int quantum) {
 }
 
 // ---- staging: x -> bf16 units in the B operand's order ---------------------------------------------------------------
-// unit (block b of BR rows, 128-k unit ku): [16 chunks of 8 k][BR rows][8] and, SEG > 0, behind it fp32 sums [128 / SEG][16].
+// piece (block b of BR rows, 128 k number ku; one or two make a unit): [16 chunks of 8 k][BR rows][8] and, SEG > 0, behind it fp32 sums [128 / SEG][16].
 // Chunk 4 q + i holds of the 32-k quarter q the k = 8 c + 2 i + e at place 2 c + e.  A thread moves 32 k of one row: 64 bytes in,
 // four 16-byte pieces out; a warp covers 8 rows x 128 k, so that every piece of 8 rows is one full 128-byte line.
 // Rows >= M and columns >= Kx are zero.  Bound by HBM / L2: bytes of x in and out once.
@@ -271,7 +276,7 @@ __device__ __noinline__ uint4 wq_again(const WqParams& p, uint4 v, int m, int64_
   for (int e = 0; e < 8; ++e) {
     const int n = (int)n0 + e, r = n & 15;
     const uint32_t bits = float_to_bf16_bits(wq_exact<G>(p.packed + (int64_t)(n >> 4) * p.Kp * 2, p.sz + (int64_t)(n >> 4) * (p.Kp / G) * 16 + r,
-                                                         p.xt + m * 16, p.x_bytes, p.Kp, r & 7, r >> 3));
+                                                         p.xt + m * 16, p.x_sub, p.Kp, r & 7, r >> 3));
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       if (i == (e >> 1)) o[i] = e & 1 ? (o[i] & 0xFFFFu) | (bits << 16) : (o[i] & 0xFFFF0000u) | bits;
@@ -323,14 +328,15 @@ struct WqRing {
 // ---- the GEMM ----------------------------------------------------------------------------------------------------------
 // G == 0: int8.  Shared memory: header, output tile, activation ring (x_slots x x_bytes), weight ring (w_slots x [8 strips x 128 k]
 // [8 strips x parameters]).
-template <int G, bool DEFER, bool PAIR, bool DIRECT, bool EARLY>
+template <int G, bool DEFER, bool PAIR, bool DIRECT, bool EARLY, int KW>
 __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_constant__ WqParams p) {
   extern __shared__ __align__(1024) uint8_t wq_smem[];
   constexpr bool kI8 = (G == 0);
   constexpr int kTileB = kI8 ? 1024 : 512;                                // bytes of one (strip, 64-k) tile
   constexpr int kSegs = DEFER ? (G < 128 ? 128 / (G ? G : 128) : 1) : 1;  // accumulation segments per unit
   constexpr int kSzWords = kI8 ? 0 : (G < 128 ? 128 / (G ? G : 128) : 1) * 16;
-  constexpr uint32_t kWBytes = 8 * 2 * kTileB, kSBytes = 8 * kSzWords * 4, kWSlot = kWBytes + kSBytes;
+  constexpr uint32_t kWBytes = 8 * 2 * kTileB, kSBytes = 8 * kSzWords * 4, kWSub = kWBytes + kSBytes, kWSlot = KW * kWSub;
+  constexpr int kAllSegs = KW * kSegs;  // of a unit, KW times 128 k
   constexpr int kRanks = PAIR ? 2 : 1;
   uint64_t* wfull = reinterpret_cast<uint64_t*>(wq_smem);
   uint64_t* wempty = wfull + kWqMaxW;
@@ -368,8 +374,11 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     }
     uint8_t* dst = wring + slot * kWSlot;
     mbar_arrive_expect_tx(&wfull[slot], kWSlot);
-    wq_tma_2d(dst, &p.wmap, ku * 256, strip, &wfull[slot]);
-    if constexpr (!kI8) wq_tma_2d(dst + kWBytes, &p.smap, G == 256 ? (ku >> 1) * 16 : ku * kSzWords, strip, &wfull[slot]);
+#pragma unroll
+    for (int j = 0; j < KW; ++j) {  // (128 k past the end: zeros)
+      wq_tma_2d(dst + j * kWSub, &p.wmap, (ku * KW + j) * 256, strip, &wfull[slot]);
+      if constexpr (!kI8) wq_tma_2d(dst + j * kWSub + kWBytes, &p.smap, G == 256 ? ((ku * KW + j) >> 1) * 16 : (ku * KW + j) * kSzWords, strip, &wfull[slot]);
+    }
   };
   if (warp == kWqWProd) {
     if (lane < p.w_slots) {
@@ -543,7 +552,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
       const uint32_t chunk = (uint32_t)p.BR * 16;
       const uint32_t desc_hi = DIRECT ? (1024u >> 4) | (1u << 14) | (2u << 29) : (128u >> 4) | (1u << 14);
       const uint32_t kstep = DIRECT ? 32u >> 4 : (2 * chunk) >> 4, khalf = DIRECT ? ((uint32_t)p.BR * 128 - 4 * 32) >> 4 : 0u;
-      const uint32_t desc_lo = (DIRECT ? 0u : (chunk >> 4) << 16) | ((smem_u32(xring) & 0x3FFFFu) >> 4), xstep = p.x_bytes >> 4;
+      const uint32_t desc_lo = (DIRECT ? 0u : (chunk >> 4) << 16) | ((smem_u32(xring) & 0x3FFFFu) >> 4), xstep = p.x_bytes >> 4, xsub = p.x_sub >> 4;
       int u = u0;
       bool ok = true;
       while (u < (mw < n_mma ? u1 : u0)) {
@@ -559,11 +568,11 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
           if (PAIR) ok = ok && wait(&xpeer[x.slot], x.use);
           wq_fence_after();
           if (wq_elect_one() && ok) {
-            const uint32_t b0 = desc_lo + (uint32_t)x.slot * xstep, a0 = a_col0 + a.slot * 64;
-            const uint32_t d0 = DEFER ? tb + x.slot * (kSegs * 16) : dcol;
+            const uint32_t b0 = desc_lo + (uint32_t)x.slot * xstep, a0 = a_col0 + a.slot * (64 * KW);
+            const uint32_t d0 = DEFER ? tb + x.slot * (kAllSegs * 16) : dcol;
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks) {
-              const uint64_t bdesc = ((uint64_t)desc_hi << 32) | (b0 + ks * kstep + (ks >= 4 ? khalf : 0u));
+            for (int ks = 0; ks < 8 * KW; ++ks) {
+              const uint64_t bdesc = ((uint64_t)desc_hi << 32) | (b0 + (ks & 7) * kstep + ((ks & 7) >= 4 ? khalf : 0u) + (ks >= 8 ? xsub : 0u));
               wq_mma<PAIR>(d0 + (DEFER ? ks / (8 / kSegs) * 16 : 0), a0 + 8 * ks, bdesc, idesc, DEFER ? (ks % (8 / kSegs) != 0) : (ks != 0 ? 1u : acc));
             }
             wq_commit<PAIR>(&adone[a.slot]);
@@ -601,11 +610,8 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     constexpr int kWords = kI8 ? 16 : 8, kSzn = (kI8 || DEFER) ? 1 : kSzWords / 16;
     uint32_t wd[kWords], sz[kSzn][2];
     bool ok = true;
-    auto fetch = [&](int u) {
-      if (u >= u1) return;
-      if (a_first) ok = ok && wait(&adone[a.slot], a.use ^ 1u);
-      ok = ok && wait(&wfull[w.slot], w.use);
-      const uint32_t wt = w0_u + w.slot * kWSlot, st = s0_u + w.slot * kWSlot;
+    auto words = [&](int j) {  // of the unit's j-th 128 k
+      const uint32_t wt = w0_u + w.slot * kWSlot + j * kWSub, st = s0_u + w.slot * kWSlot + j * kWSub;
 #pragma unroll
       for (int i = 0; i < kWords / 4; ++i) {
         const uint4 v = lds128(wt + i * 512);
@@ -619,48 +625,64 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
         }
       }
     };
+    auto fetch = [&](int u) {
+      if (u >= u1) return;
+      if (a_first) ok = ok && wait(&adone[a.slot], a.use ^ 1u);
+      ok = ok && wait(&wfull[w.slot], w.use);
+      words(0);
+    };
     fetch(u0 + set);
     for (int u = u0 + set; u < u1; u += 2) {
       uint32_t r[32];
-      if constexpr (DIRECT) {  // x is in its own order, so the weights have to be
+      auto convert = [&]() {
+        if constexpr (DIRECT) {  // x is in its own order, so the weights have to be
 #pragma unroll
-        for (int j = 0; j < kWords; j += kI8 ? 4 : 2) {
-          if constexpr (kI8) {
-            wq_turn_int8(wd[j], wd[j + 2], lane);
-            wq_turn_int8(wd[j + 1], wd[j + 3], lane);
-          } else {
-            wq_turn_int4(wd[j], wd[j + 1], lane);
+          for (int j = 0; j < kWords; j += kI8 ? 4 : 2) {
+            if constexpr (kI8) {
+              wq_turn_int8(wd[j], wd[j + 2], lane);
+              wq_turn_int8(wd[j + 1], wd[j + 3], lane);
+            } else {
+              wq_turn_int4(wd[j], wd[j + 1], lane);
+            }
           }
         }
-      }
-      if constexpr (kI8) {
+        if constexpr (kI8) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {  // 32-k quarters of the unit; lane chunk: words (row g, k 0-3), (g+8, k 0-3), (g, k 4-7), (g+8, k 4-7)
-          const int q4 = j >> 2, hrow = j & 1, i0 = 2 * ((j >> 1) & 1);
-          u8x4_to_bf16x2x2(wd[j], r[2 * (4 * q4 + i0) + hrow], r[2 * (4 * q4 + i0 + 1) + hrow]);
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {  // word j: row g + 8 (j & 1), 32-k quarter j >> 1 of the unit
-          const int q4 = j >> 1, hrow = j & 1;
-          uint32_t o[4];
-          if constexpr (DEFER) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) asm("lop3.b32 %0, %1, 0x000f000f, 0x43004300, 0xea;" : "=r"(o[i]) : "r"(wd[j] >> (4 * i)));  // 128 + q
-          } else {
-            const uint32_t szw = sz[q4 * kSzn / 4][hrow];
-            dequant_word(wd[j], __byte_perm(szw, 0, 0x1010), __byte_perm(szw, 0, 0x3232), o);
+          for (int j = 0; j < 16; ++j) {  // 32-k quarters of the unit; lane chunk: words (row g, k 0-3), (g+8, k 0-3), (g, k 4-7), (g+8, k 4-7)
+            const int q4 = j >> 2, hrow = j & 1, i0 = 2 * ((j >> 1) & 1);
+            u8x4_to_bf16x2x2(wd[j], r[2 * (4 * q4 + i0) + hrow], r[2 * (4 * q4 + i0 + 1) + hrow]);
           }
+        } else {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) r[2 * (4 * q4 + i) + hrow] = o[i];
+          for (int j = 0; j < 8; ++j) {  // word j: row g + 8 (j & 1), 32-k quarter j >> 1 of the unit
+            const int q4 = j >> 1, hrow = j & 1;
+            uint32_t o[4];
+            if constexpr (DEFER) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) asm("lop3.b32 %0, %1, 0x000f000f, 0x43004300, 0xea;" : "=r"(o[i]) : "r"(wd[j] >> (4 * i)));  // 128 + q
+            } else {
+              const uint32_t szw = sz[q4 * kSzn / 4][hrow];
+              dequant_word(wd[j], __byte_perm(szw, 0, 0x1010), __byte_perm(szw, 0, 0x3232), o);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r[2 * (4 * q4 + i) + hrow] = o[i];
+          }
         }
-      }
+      };
+      convert();
+      if constexpr (KW == 2) words(1);
       __syncwarp();
       if (lane == 0) mbar_arrive(&wempty[w.slot]);  // everything that this warp reads of the slot is in registers
       ok = ok && wait(&adone[a.slot], a.use ^ 1u);  // the MMAs that read this A slot have retired
       wq_fence_after();
-      wq_st_16x128b_x8(taddr0 + a.slot * 64, r);
-      wq_st_16x128b_x8(taddr0 + a.slot * 64 + 32, r + 16);
+      const uint32_t ta = taddr0 + a.slot * (64 * KW);
+      wq_st_16x128b_x8(ta, r);
+      wq_st_16x128b_x8(ta + 32, r + 16);
+      if constexpr (KW == 2) {
+        convert();
+        wq_st_16x128b_x8(ta + 64, r);
+        wq_st_16x128b_x8(ta + 96, r + 16);
+      }
       uint64_t* full = &afull[a.slot];
       const bool announce = ok;
       w.step(2, p.w_slots);
@@ -701,13 +723,15 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
           ok = ok && (rw || wait(&wfull[w.slot], w.use)) && (rx || wait(&xfull[x.slot], x.use)) && (rd || wait(&xdone[x.slot], x.use));
           wq_fence_after();
           // parameters of rows 32 warp + lane / 4 + 8 i, sums of columns 2 (lane % 4) + {0, 1, 8, 9}
-          const uint32_t st = smem_u32(wring) + w.slot * kWSlot + kWBytes + 2 * warp * (kSzWords * 4) + (lane >> 2) * 4;
-          const uint32_t xs = smem_u32(xring) + (uint32_t)x.slot * p.x_bytes + 16 * 256 + (lane & 3) * 8;
+          const uint32_t st0 = smem_u32(wring) + w.slot * kWSlot + kWBytes + 2 * warp * (kSzWords * 4) + (lane >> 2) * 4;
+          const uint32_t xs0 = smem_u32(xring) + (uint32_t)x.slot * p.x_bytes + 16 * 256 + (lane & 3) * 8;
 #pragma unroll
-          for (int sg = 0; sg < kSegs; ++sg) {
+          for (int all = 0; all < kAllSegs; ++all) {
+            const int sg = all % kSegs;
+            const uint32_t st = st0 + all / kSegs * kWSub, xs = xs0 + all / kSegs * p.x_sub;
             uint32_t v[16];
-            wq_ld_16x256b_x2(lane_col + (x.slot * kSegs + sg) * 16, v);
-            wq_ld_16x256b_x2(lane_col + (16u << 16) + (x.slot * kSegs + sg) * 16, v + 8);
+            wq_ld_16x256b_x2(lane_col + (x.slot * kAllSegs + all) * 16, v);
+            wq_ld_16x256b_x2(lane_col + (16u << 16) + (x.slot * kAllSegs + all) * 16, v + 8);
             float s[4], zt[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -718,12 +742,15 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
             const float2 xa = lds64f(xs + sg * 64), xb = lds64f(xs + sg * 64 + 32);
             const float X[4] = {xa.x, xa.y, xb.x, xb.y};
             wq_ld_wait();
+            const F2 x2[2] = {f2(X[0], X[1]), f2(X[2], X[3])};
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
-              for (int e = 0; e < 8; ++e) {  // e: column group e >> 2, row group (e >> 1) & 1, column e & 1
-                const int r = 2 * h + ((e >> 1) & 1), c = 2 * (e >> 2) + (e & 1);
-                acc[8 * h + e] = fmaf(s[r], __uint_as_float(v[8 * h + e]), fmaf(zt[r], X[c], acc[8 * h + e]));
+              for (int e = 0; e < 8; e += 2) {  // e: column group e >> 2, row group (e >> 1) & 1, column e & 1
+                const int r = 2 * h + ((e >> 1) & 1);
+                const F2 part = f2_fma(f2(zt[r], zt[r]), x2[e >> 2], f2(acc[8 * h + e], acc[8 * h + e + 1]));
+                const float2 y = f2_get(f2_fma(f2(s[r], s[r]), f2(__uint_as_float(v[8 * h + e]), __uint_as_float(v[8 * h + e + 1])), part));
+                acc[8 * h + e] = y.x, acc[8 * h + e + 1] = y.y;
               }
           }
           wq_fence_before();
@@ -913,11 +940,14 @@ static int wq_sm_count() {
 // how one call is cut up; a pure function of the shape, so the workspace size is too
 struct WqPlan {
   bool defer, pair, direct;
+  int KW;  // 128 k per unit
   int NT, BR, MT, NB, KU, ranks, workers, quantum, base, rem;
   int64_t tiles, n_tickets;
-  uint32_t x_bytes;
+  uint32_t x_bytes, x_sub;
   int64_t off_part, off_xt, bytes;  // [tickets][shares][staged activations]
 };
+
+static int kw_of(const WqPlan& w) { return !w.direct && w.NT <= kWqLongNT ? 2 : 1; }
 
 static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
   if (M <= 0 || Np % 128 != 0 || Kp % 64 != 0 || M > ((int64_t)1 << 24)) return false;
@@ -932,7 +962,8 @@ static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
   w.MT = (int)((M + 255) / 256);
   w.NT = (int)(((M + w.MT - 1) / w.MT + 15) / 16 * 16);
   w.BR = w.NT / w.ranks;
-  w.KU = (int)((Kp + 127) / 128);
+  w.KW = kw_of(w);
+  w.KU = (int)((Kp + 128 * w.KW - 1) / (128 * w.KW));
   w.NB = (int)((Np + 128 * w.ranks - 1) / (128 * w.ranks));
   w.tiles = (int64_t)w.NB * w.MT;
   if (w.tiles * w.KU > 2000000000) return false;
@@ -943,7 +974,8 @@ static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
   w.base = (int)(parts / w.workers);
   w.rem = (int)(parts % w.workers);
   w.n_tickets = w.quantum > 1 ? 0 : w.tiles * w.ranks;
-  w.x_bytes = (uint32_t)w.BR * 256 + (w.defer ? 4 * 64 : 0);  // (the sums' space is that of the smallest group)
+  w.x_sub = (uint32_t)w.BR * 256 + (w.defer ? 4 * 64 : 0);  // (the sums' space is that of the smallest group)
+  w.x_bytes = w.KW * w.x_sub;
   auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
   w.off_part = up(w.n_tickets * 4);
   w.off_xt = w.off_part + (w.quantum > 1 ? 0 : up((int64_t)w.workers * 2 * w.ranks * w.NT * 512));
@@ -979,14 +1011,16 @@ static bool wq_map(CUtensorMap* map, CUtensorMapDataType type, int elem, const v
   return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess && encode();
 }
 
-template <int G, bool DEFER, bool PAIR, bool DIRECT>
+template <int G, bool DEFER, bool PAIR, bool DIRECT, int KW>
 static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
-  constexpr uint32_t kWSlot = 8 * 2 * (G == 0 ? 1024 : 512) + (G == 0 ? 0 : 8 * (G < 128 ? 128 / (G ? G : 128) : 1) * 64);
+  constexpr uint32_t kWSlot = KW * (8 * 2 * (G == 0 ? 1024 : 512) + (G == 0 ? 0 : 8 * (G < 128 ? 128 / (G ? G : 128) : 1) * 64));
   constexpr size_t kBudget = 226 * 1024;
   p.n_mma = w.NT <= 64 ? 2 : 1;
   // tiles of x in flight (an L2 round trip is about 850 clocks; DEFER: as many as there are accumulators); what they and the
   // output tile leave of shared memory holds weights in flight
-  p.x_slots = w.x_bytes > 24 * 1024 ? 3 : (w.x_bytes > 12 * 1024 ? 5 : (DEFER && G == 32 ? 4 : 8));  // even where two MMA warps alternate
+  // (even where two MMA warps alternate)
+  if (KW == 2) p.x_slots = w.x_bytes > 24 * 1024 ? 3 : (w.x_bytes > 9 * 1024 || (DEFER && G == 64) ? 4 : (DEFER && G == 32 ? 2 : 6));
+  else p.x_slots = w.x_bytes > 24 * 1024 ? 3 : (w.x_bytes > 12 * 1024 ? 5 : (DEFER && G == 32 ? 4 : 8));
   const size_t unit = DIRECT ? 1024 : 16;      // (rows of 128 swizzled bytes: eight of them have to lie as the hardware counts)
   p.off_x = (uint32_t)((kWqHeader + (size_t)w.NT * kWqPitch + unit - 1) / unit * unit);
   const size_t off_w = (p.off_x + (size_t)p.x_slots * w.x_bytes + 127) / 128 * 128;
@@ -994,7 +1028,7 @@ static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
   p.w_slots = (int)((kBudget - off_w) / kWSlot);
   if (p.w_slots > kWqMaxW) p.w_slots = kWqMaxW;
   if (p.n_mma == 2) p.w_slots &= ~1;           // two MMA warps let the two dequant sets drift apart: each set keeps slots of its own
-  p.a_slots = p.w_slots == 3 ? 3 : kWqSlots;   // (see a_first in the kernel)
+  p.a_slots = KW == 2 ? kWqSlots / 2 : (p.w_slots == 3 ? 3 : kWqSlots);   // (see a_first in the kernel)
   const size_t smem = off_w + (size_t)p.w_slots * kWSlot;
   // The last tile from the accumulators where every CTA has a tile's worth of units, so that a tile has two owners as a rule: 4096 x 4096, 2048 rows
   // 63.9 -> 57.1 us; 14336 x 4096 int4, 300 / 1000 rows 39.8 -> 36.2 / 94.0 -> 89.3; 28672 x 4096 int8, 32 / 77 / 300 rows 32.4 -> 30.9 / 37.7 -> 34.9 /
@@ -1002,9 +1036,9 @@ static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
   // (14336 x 4096, 77 rows: 25.6 -> 25.8; 4096 x 4096 int8, 200 rows: 28.5 -> 29.0).
   constexpr bool kCan = !DEFER;
   const bool early = kCan && (int64_t)w.base * w.quantum >= w.KU;
-  auto kern = wq_gemm_kernel<G, DEFER, PAIR, DIRECT, false>;
+  auto kern = wq_gemm_kernel<G, DEFER, PAIR, DIRECT, false, KW>;
   static OncePerDevice once[2];
-  if (early) kern = wq_gemm_kernel<G, DEFER, PAIR, DIRECT, kCan>;
+  if (early) kern = wq_gemm_kernel<G, DEFER, PAIR, DIRECT, kCan, KW>;
   if (!dynamic_smem(once[early], kern, (int)kBudget)) return AO_B200_ERR_CUDA;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(w.workers * w.ranks));
@@ -1026,7 +1060,8 @@ static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
 template <int SEG>
 static int wq_stage(const void* x, int64_t M, int64_t Kx, int64_t ldx, const WqPlan& w, uint8_t* xt, uint32_t* tickets, bool settled, cudaStream_t s) {
   const int n_blocks = w.MT * w.ranks;
-  const int64_t warps = (int64_t)n_blocks * (w.BR / 8) * w.KU;
+  const int ku = w.KU * w.KW;  // (whole units)
+  const int64_t warps = (int64_t)n_blocks * (w.BR / 8) * ku;
   int64_t grid = (warps + 7) / 8;
   if (grid > 148 * 16) grid = 148 * 16;
   if (grid * 256 < w.n_tickets) grid = (w.n_tickets + 255) / 256;
@@ -1039,7 +1074,7 @@ static int wq_stage(const void* x, int64_t M, int64_t Kx, int64_t ldx, const WqP
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, stage_x_kernel<SEG>, static_cast<const __nv_bfloat16*>(x), M, Kx, ldx, n_blocks, w.BR, w.KU, w.x_bytes, xt, tickets,
+  return cudaLaunchKernelEx(&cfg, stage_x_kernel<SEG>, static_cast<const __nv_bfloat16*>(x), M, Kx, ldx, n_blocks, w.BR, ku, w.x_sub, xt, tickets,
                             (int)w.n_tickets, settled) == cudaSuccess
              ? AO_B200_OK
              : AO_B200_ERR_CUDA;
@@ -1092,6 +1127,7 @@ static int wq_gemm(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void
   p.KU = w.KU;
   p.MT = w.MT;
   p.x_bytes = w.x_bytes;
+  p.x_sub = w.x_sub;
   p.quantum = w.quantum;
   p.base = w.base;
   p.rem = w.rem;
@@ -1109,13 +1145,15 @@ static int wq_gemm(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void
   if (rc != AO_B200_OK) return rc;
   switch (G) {
     case 0:
-      return w.direct ? wq_launch<0, false, true, true>(p, w, s)
-                      : (w.pair ? wq_launch<0, false, true, false>(p, w, s) : wq_launch<0, false, false, false>(p, w, s));
-#define AO_WQ(GG)                                                                                        \
-  case GG:                                                                                               \
-    return w.direct ? wq_launch<GG, false, true, true>(p, w, s)                                          \
-                    : (w.defer ? wq_launch<GG, true, false, false>(p, w, s)                              \
-                               : (w.pair ? wq_launch<GG, false, true, false>(p, w, s) : wq_launch<GG, false, false, false>(p, w, s)));
+      if (w.direct) return wq_launch<0, false, true, true, 1>(p, w, s);
+      if (w.KW == 2) return w.pair ? wq_launch<0, false, true, false, 2>(p, w, s) : wq_launch<0, false, false, false, 2>(p, w, s);
+      return wq_launch<0, false, true, false, 1>(p, w, s);
+#define AO_WQ(GG)                                                                                                              \
+  case GG:                                                                                                                     \
+    if (w.direct) return wq_launch<GG, false, true, true, 1>(p, w, s);                                                         \
+    if (w.defer) return wq_launch<GG, true, false, false, 2>(p, w, s);                                                         \
+    if (w.KW == 2) return w.pair ? wq_launch<GG, false, true, false, 2>(p, w, s) : wq_launch<GG, false, false, false, 2>(p, w, s); \
+    return wq_launch<GG, false, true, false, 1>(p, w, s);
     AO_WQ(32)
     AO_WQ(64)
     AO_WQ(128)
