@@ -97,32 +97,46 @@ __device__ __forceinline__ int wq_owner(int u, int base, int rem, int quantum) {
 // piece (block b of BR rows, 128 k number ku; one or two make a unit): [16 chunks of 8 k][BR rows][8] and, SEG > 0, behind it fp32 sums [128 / SEG][16].
 // Chunk 4 q + i holds of the 32-k quarter q the k = 8 c + 2 i + e at place 2 c + e.  A thread moves 32 k of one row: 64 bytes in,
 // four 16-byte pieces out; a warp covers 8 rows x 128 k, so that every piece of 8 rows is one full 128-byte line.
-// Rows >= M and columns >= Kx are zero.  Bound by HBM / L2: bytes of x in and out once.
+// Rows >= M and columns >= Kx are zero.  Bound by HBM / L2: bytes of x in and out once; for few rows by the way there and back, which the GEMM's first
+// weights are in if they ask first.  So the first piece is brought to L2 before the wait (which reads nothing: what the kernel in front writes meets it
+// there), and a block takes no more threads and registers than a CTA of the GEMM leaves (768 x 80 of 65536), so that neither waits for the other's SM.
+// In a chain, against blocks of 256 and no prefetch: int4 24 rows of 14336 x 4096 20.9 -> 19.8 us, 20 of 4096 x 4096 14.0 -> 13.4, 128 of 14336 x 4096 26.8 ->
+// 25.7, int8 32 of 8192 x 8192 24.1 -> 23.4.  (The GEMM let go behind the loads instead of at once: 24 -> 26.2 us at 77 rows.)
+constexpr int kStageThreads = 64;
 template <int SEG>
-__global__ void __launch_bounds__(256) stage_x_kernel(const __nv_bfloat16* __restrict__ x, int64_t M, int64_t Kx, int64_t ldx, int n_blocks, int BR, int KU,
-                                                      uint32_t x_bytes, uint8_t* __restrict__ xt, uint32_t* __restrict__ tickets, int n_tickets,
-                                                      bool settled) {
+__global__ void __launch_bounds__(kStageThreads, 16) stage_x_kernel(const __nv_bfloat16* __restrict__ x, int64_t M, int64_t Kx, int64_t ldx, uint32_t pieces, int BR, int KU,
+                                                                    uint32_t x_bytes, uint8_t* __restrict__ xt, uint32_t* __restrict__ tickets, int n_tickets,
+                                                                    bool settled) {
   // The GEMM behind reads weights and parameters without a wait of its own.  They may be the work of the kernel in front of this
   // one (quantize_, then a call), so it is let go only when that one is over and its writes are visible; at once where the caller
   // answers for the weights (settled), as a decode step does: 16 tokens of 8 sequences through four layers 5842 us, behind the wait 5968
   if (settled) grid_launch_dependents();
+  const uint32_t gid = blockIdx.x * kStageThreads + threadIdx.x, step = gridDim.x * (kStageThreads / 32), groups = (uint32_t)BR / 8;
+  const int lane = threadIdx.x & 31, row8 = lane >> 2, quarter = lane & 3;  // quarter: 32-k piece of the unit
+  uint32_t w = gid >> 5;
+  if (w < pieces) {
+    const uint32_t rg = w / (uint32_t)KU, ku = w - rg * (uint32_t)KU;
+    const int64_t m = (int64_t)rg * 8 + row8, k0 = (int64_t)ku * 128 + quarter * 32;
+    if (m < M && k0 < Kx) asm volatile("prefetch.global.L2 [%0];" ::"l"(x + m * ldx + k0));
+  }
   grid_dependency_wait();
   if (!settled) grid_launch_dependents();
-  const int64_t gid = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (gid < n_tickets) tickets[gid] = 0u;
-  const int lane = threadIdx.x & 31, row8 = lane >> 2, quarter = lane & 3;  // quarter: 32-k piece of the unit
-  const int groups = BR / 8;
-  for (int64_t w = gid >> 5; w < (int64_t)n_blocks * groups * KU; w += ((int64_t)gridDim.x * 256) >> 5) {
-    const int ku = (int)(w % KU);
-    const int64_t rg = w / KU;
-    const int b = (int)(rg / groups), r = (int)(rg - (int64_t)b * groups) * 8 + row8;
-    const int64_t m = (int64_t)b * BR + r, k0 = (int64_t)ku * 128 + quarter * 32;
-    uint4 v[4];
+  uint4 v[4];
+  // a warp's piece: 8 rows x 128 k
+  auto load = [&](uint32_t w) {
+    const uint32_t rg = w / (uint32_t)KU, ku = w - rg * (uint32_t)KU;         // row group: 8 rows, block after block
+    const int64_t m = (int64_t)rg * 8 + row8, k0 = (int64_t)ku * 128 + quarter * 32;
+    const __nv_bfloat16* src = x + m * ldx + k0;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       v[c] = make_uint4(0u, 0u, 0u, 0u);
-      if (m < M && k0 + 8 * c < Kx) v[c] = *reinterpret_cast<const uint4*>(x + m * ldx + k0 + 8 * c);  // Kx % 8 == 0: all or nothing
+      if (m < M && k0 + 8 * c < Kx) v[c] = *reinterpret_cast<const uint4*>(src + 8 * c);  // Kx % 8 == 0: all or nothing
     }
+  };
+  if (w < pieces) load(w);
+  for (int i = (int)gid; i < n_tickets; i += gridDim.x * kStageThreads) tickets[i] = 0u;
+  while (w < pieces) {
+    const uint32_t rg = w / (uint32_t)KU, ku = w - rg * (uint32_t)KU, b = rg / groups, r = (rg - b * groups) * 8 + row8;
     uint8_t* unit = xt + ((int64_t)b * KU + ku) * x_bytes;
     uint8_t* dst = unit + ((int64_t)(quarter * 4) * BR + r) * 16;
     *reinterpret_cast<uint4*>(dst) = make_uint4(v[0].x, v[1].x, v[2].x, v[3].x);
@@ -142,15 +156,17 @@ __global__ void __launch_bounds__(256) stage_x_kernel(const __nv_bfloat16* __res
       if (SEG >= 128) s += __shfl_xor_sync(0xffffffffu, s, 2);
       if ((quarter * 32) % SEG == 0) reinterpret_cast<float*>(unit + (int64_t)BR * 256)[(quarter * 32 / SEG) * 16 + r] = s;
     }
+    w += step;
+    if (w < pieces) load(w);
   }
 }
 
 // DIRECT: nothing to stage, but the tickets (n >= 1 words); lets the GEMM go as stage_x_kernel does
-__global__ void __launch_bounds__(256) clear_tickets_kernel(uint32_t* __restrict__ tickets, int n, bool settled) {
+__global__ void __launch_bounds__(kStageThreads, 16) clear_tickets_kernel(uint32_t* __restrict__ tickets, int n, bool settled) {
   if (settled) grid_launch_dependents();
   grid_dependency_wait();
   if (!settled) grid_launch_dependents();
-  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) tickets[i] = 0u;
+  for (int i = blockIdx.x * kStageThreads + threadIdx.x; i < n; i += gridDim.x * kStageThreads) tickets[i] = 0u;
 }
 
 // ---- PTX wrappers ------------------------------------------------------------------------------------------------------
@@ -1059,22 +1075,21 @@ static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
 
 template <int SEG>
 static int wq_stage(const void* x, int64_t M, int64_t Kx, int64_t ldx, const WqPlan& w, uint8_t* xt, uint32_t* tickets, bool settled, cudaStream_t s) {
-  const int n_blocks = w.MT * w.ranks;
   const int ku = w.KU * w.KW;  // (whole units)
-  const int64_t warps = (int64_t)n_blocks * (w.BR / 8) * ku;
-  int64_t grid = (warps + 7) / 8;
-  if (grid > 148 * 16) grid = 148 * 16;
-  if (grid * 256 < w.n_tickets) grid = (w.n_tickets + 255) / 256;
+  const int64_t pieces = (int64_t)w.MT * w.ranks * (w.BR / 8) * ku;
+  if (pieces > 0x7fffffff) return AO_B200_ERR_UNSUPPORTED;   // (2 KB of activations each)
+  int64_t grid = (pieces + kStageThreads / 32 - 1) / (kStageThreads / 32);
+  if (grid > 148 * 32) grid = 148 * 32;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(256);
+  cfg.blockDim = dim3(kStageThreads);
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, stage_x_kernel<SEG>, static_cast<const __nv_bfloat16*>(x), M, Kx, ldx, n_blocks, w.BR, ku, w.x_sub, xt, tickets,
+  return cudaLaunchKernelEx(&cfg, stage_x_kernel<SEG>, static_cast<const __nv_bfloat16*>(x), M, Kx, ldx, (uint32_t)pieces, w.BR, ku, w.x_sub, xt, tickets,
                             (int)w.n_tickets, settled) == cudaSuccess
              ? AO_B200_OK
              : AO_B200_ERR_CUDA;
@@ -1082,8 +1097,8 @@ static int wq_stage(const void* x, int64_t M, int64_t Kx, int64_t ldx, const WqP
 
 static int wq_clear(uint32_t* tickets, int64_t n, bool settled, cudaStream_t s) {
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(n > 148 * 256 ? 148 : (n + 255) / 256 + (n == 0)));
-  cfg.blockDim = dim3(256);
+  cfg.gridDim = dim3((unsigned)(n > 148 * kStageThreads ? 148 : (n + kStageThreads - 1) / kStageThreads + (n == 0)));
+  cfg.blockDim = dim3(kStageThreads);
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
