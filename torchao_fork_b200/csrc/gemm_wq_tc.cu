@@ -216,6 +216,11 @@ __device__ __forceinline__ void wq_ld_wait() { asm volatile("tcgen05.wait::ld.sy
 __device__ __forceinline__ void wq_stmatrix_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {  // one rounding per product
+  uint32_t d;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
 __device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {  // one rounding per sum
   uint32_t d;
   asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -442,27 +447,26 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
   const uint32_t a_col0 = tb + 256;
 
   // fp32 sums of rows 32 q + 16 h .. + 15, columns c .. c + 15 (fragment order of wq_ld_16x256b_x2) -> output tile
-  auto to_stage = [&](int q, int c, int h, const float* f, const float (&sc)[4]) {
+  auto to_stage = [&](int q, int c, int h, const float* f, const uint32_t (&sc)[4]) {
     const uint32_t at = smem_u32(stage) + (uint32_t)(c + 8 * (lane >> 4) + (lane & 7)) * kWqPitch + (32 * q + 16 * h + 8 * ((lane >> 3) & 1)) * 2;
     uint32_t o[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {  // block i: column group i >> 1, row group i & 1
-      float a = f[4 * (i >> 1) + 2 * (i & 1)], b = f[4 * (i >> 1) + 2 * (i & 1) + 1];
-      // int8: mm result rounded to bf16, THEN multiplied by the row scale and rounded again
-      if constexpr (kI8) {
-        const float k = h ? sc[2 + (i & 1)] : sc[i & 1];
-        a = bf16r(a) * k, b = bf16r(b) * k;
-      }
+      const float a = f[4 * (i >> 1) + 2 * (i & 1)], b = f[4 * (i >> 1) + 2 * (i & 1) + 1];
       asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[i]) : "f"(b), "f"(a));
+      // int8: mm result rounded to bf16, THEN multiplied by the row scale and rounded again (the product of two bf16 is exact in fp32, so a packed
+      // multiply rounds it once, as a product in fp32 and a conversion do, with a quarter of the instructions: int8 8192 x 8192, 2048 rows 220.2 -> 217.7 us,
+      // 14336 x 4096, 700 / 300 rows 70.5 -> 68.6, 40.0 -> 38.9)
+      if constexpr (kI8) o[i] = mul_bf16x2(o[i], h ? sc[2 + (i & 1)] : sc[i & 1]);
     }
     wq_stmatrix_trans(at, o[0], o[1], o[2], o[3]);
   };
-  // the row scales (int8) of a thread's four rows 32 q + lane / 4 + 8 i
-  auto row_scales = [&](int nb, int q, float (&sc)[4]) {
+  // the row scales (int8) of a thread's four rows 32 q + lane / 4 + 8 i, each twice
+  auto row_scales = [&](int nb, int q, uint32_t (&sc)[4]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int64_t n = ((int64_t)nb * kRanks + rank) * 128 + 32 * q + (lane >> 2) + 8 * i;
-      sc[i] = kI8 && n < p.N_out ? __bfloat162float(p.scale8[n]) : 0.f;
+      sc[i] = kI8 && n < p.N_out ? __bfloat16_as_ushort(p.scale8[n]) * 0x10001u : 0u;
     }
   };
   // output tile -> y: 16-byte pieces of 256-byte rows; `threads` threads, this one is number `th`
@@ -727,7 +731,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
       const int ue = min(u1, (t + 1) * KU), nb = t / p.MT, mt = t - nb * p.MT;
       const bool whole = u == t * KU && ue == (t + 1) * KU;
       float4* mine = share(worker, t) + warp * 32 + lane;
-      float sc[4];
+      uint32_t sc[4];
       row_scales(nb, warp, sc);
       if (whole) wq_epi_sync(false);  // the previous output tile has been copied out
       if constexpr (DEFER) {
@@ -861,7 +865,8 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     const int c0 = wq_owner(t * KU, p.base, p.rem, p.quantum), c1 = wq_owner(t * KU + KU - 1, p.base, p.rem, p.quantum);
     for (int it = warp; it < NT / 2; it += kWqThreads / 32) {  // (column block, quadrant, half)
       const int h = it & 1, q = (it >> 1) & 3, c = (it >> 3) * 16;
-      float f[8], sc[4];
+      float f[8];
+      uint32_t sc[4];
 #pragma unroll
       for (int i = 0; i < 8; ++i) f[i] = 0.f;
       row_scales(nb, q, sc);
@@ -886,7 +891,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     const int q = warp & 3;                                // tensor memory: a warp reaches the lanes of its quadrant
     const uint32_t dcol = tb + ((uint32_t)(32 * q) << 16) + (d_bufs == 2 ? ((t - u0 / KU) & 1) * 128 : 0) + (n_mma == 2 && held == 1 ? ((t * KU - u0) & 1) * 64 : 0);
     const float4* other = share(worker + 1, t) + q * 32 + lane;
-    float sc[4];
+    uint32_t sc[4];
     row_scales(nb, q, sc);
     constexpr int kStep = kWqThreads / 128, kBatch = 3;    // (column block, half) pairs per round of the quadrant's warps; rounds with their loads in flight
 #pragma unroll 1
