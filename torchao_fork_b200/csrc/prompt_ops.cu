@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(256) repeat_heads_kernel(const uint4* __restri
 __device__ __forceinline__ float silu_f(float g) { return __uint_as_float(float_to_bf16_bits(g / (1.f + expf(-g))) << 16); }
 __device__ __forceinline__ uint32_t silu_mul_pair(uint32_t g, uint32_t u) { return pack_rn(silu_f(lo_f(g)) * lo_f(u), silu_f(hi_f(g)) * hi_f(u)); }
 __global__ void __launch_bounds__(256) silu_mul_rows_kernel(const uint4* __restrict__ gate, const uint4* __restrict__ up, uint4* __restrict__ y, int64_t n8) {
+  grid_launch_dependents();   // (a kernel that follows programmatically waits before it reads)
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= n8) return;
   const uint4 g = gate[i], u = up[i];
