@@ -25,6 +25,10 @@
 // works 1170 for each (d = dv = 128); a CTA's start (queries, first keys) takes 6000 clocks more and its end (the peers' shares) 9000.  2048 rows x 16
 // heads of 128 (four key heads): 8.5 steps a CTA, 60 us, tensor pipe active in 31 % of the clocks, against 308 us of window_attention_prompt_kernel; the same with
 // all keys of a tile in one CTA 110 us (the last tiles alone took 95), with unswizzled operands 84 us.
+// A warp's instructions follow one another at nearly five clocks each, so what counts is their number, about 740 per step at first: addresses once per map
+// instead of once per load, the largest score three at a time, O to shared memory 32 columns at a time: 57.6 -> 55.8 us, 117 rows of two maps 20.5 -> 19.2.
+// Taken back: the next step's scores beside this one's weights (two score buffers, p3 in shared memory: 57.4 -> 56.6, small sizes up to 5 % more); an early
+// and a late tile per cluster, in one wave (60.3).
 #include "../f32x2.h"
 #include "../per_device.h"
 #include "lm_mma.cuh"
@@ -130,6 +134,11 @@ using ao::f2;
 using ao::f2_add;
 using ao::f2_fma;
 using ao::f2_get;
+__device__ __forceinline__ float tc_max3(float a, float b, float c) {
+  float y;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
 __device__ __forceinline__ float tc_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -283,32 +292,45 @@ __device__ __forceinline__ void attend(const WinPromptArgs& a, int dv) {
       // ---- loads, weights ----
       const int64_t seg_row0 = first - a.back[first], s = a.slot[first];
       const int p0 = pa - a.back[first];                   // the first position the step brings of this sequence
-      // the threads of a row take its 16-byte pieces: 2, 4, 8 or 16 threads, as many as there are pieces, or the next power of two
-      auto load = [&](unsigned char* tile_at, int t, int pieces, int width, int off, const T* step, const T* kept, const T* ring) {
-        const int wide = 32 - __clz(pieces - 1), c = threadIdx.x & ((1 << wide) - 1), rows = kTcRowThreads >> wide;
-        if (c >= pieces) return;
+      // the threads of a row take its 16-byte pieces: 2, 4, 8 or 16 threads, as many as there are pieces, or the next power of two.  `src`: this thread's piece of
+      // the first key's row (key index 0), were it among the step's own rows
+      struct Pieces {
+        int c, row0, rows;
+        const T* src;
+      };
+      auto pieces_of = [&](int pieces, int width, int off, const T* step) {
+        const int wide = 32 - __clz(pieces - 1), c = threadIdx.x & ((1 << wide) - 1), row0 = threadIdx.x >> wide;
+        return Pieces{c < pieces ? c : -1, row0, kTcRowThreads >> wide, step + ((seg_row0 + (lo - nf - p0) + row0) * G + g) * width + off + c * 8};
+      };
+      auto load = [&](unsigned char* tile_at, int t, const Pieces& p, int width, int off, const T* step, const T* kept, const T* ring) {
+        if (p.c < 0) return;
         const int k0 = (begin + t) * kTcKeys, j0 = lo + (k0 - nf);
-        const uint32_t dst = tc_smem(tile_at);
+        const uint32_t dst = tc_smem(tile_at) + tc_at(p.row0, p.c, kTcKeys);   // (rows a multiple of 8 apart: the same swizzle)
         if (k0 >= nf && j0 >= p0 && k0 + kTcKeys <= nk) {  // all from the step's own rows
-          const T* src = step + ((seg_row0 + (j0 - p0) + (threadIdx.x >> wide)) * G + g) * width + off + c * 8;
-          const int64_t next = (int64_t)rows * G * width;
-#pragma unroll 4
-          for (int row = threadIdx.x >> wide; row < kTcKeys; row += rows, src += next) tc_cp16(dst + tc_at(row, c, kTcKeys), src);
+          const T* src = p.src + (int64_t)k0 * (G * width);
+          if (p.rows == 16) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) tc_cp16(dst + i * (16 * 128), src + (int64_t)i * 16 * (G * width));
+          } else {
+#pragma unroll 1
+            for (int row = p.row0; row < kTcKeys; row += p.rows) tc_cp16(dst + (row - p.row0) * 128, src + (int64_t)(row - p.row0) * (G * width));
+          }
           return;
         }
 #pragma unroll 1
-        for (int row = threadIdx.x >> wide; row < kTcKeys; row += rows) {
+        for (int row = p.row0; row < kTcKeys; row += p.rows) {
           const int kk = k0 + row;
-          const uint32_t at = tc_at(row, c, kTcKeys);
+          const uint32_t at = tc_at(row, p.c, kTcKeys);
           if (kk < nk) {
-            tc_cp16(dst + at, win_row(a, kk, nf, lo, p0, seg_row0, s, g, width, step, kept, ring) + off + c * 8);
+            tc_cp16(tc_smem(tile_at) + at, win_row(a, kk, nf, lo, p0, seg_row0, s, g, width, step, kept, ring) + off + p.c * 8);
           } else {                                         // behind the last key: zero
             *reinterpret_cast<uint4*>(tile_at + at) = make_uint4(0, 0, 0, 0);
           }
         }
       };
-      auto load_k = [&](int t) { load(Ks, t, kc, KD, m * d, a.kn, a.first_k, a.ring_k); };
-      auto load_v = [&](int t) { load(Vs, t, vc, dv, 0, a.vn, a.first_v, a.ring_v); };
+      const Pieces kp = pieces_of(kc, KD, m * d, a.kn), vp = pieces_of(vc, dv, 0, a.vn);
+      auto load_k = [&](int t) { load(Ks, t, kp, KD, m * d, a.kn, a.first_k, a.ring_k); };
+      auto load_v = [&](int t) { load(Vs, t, vp, dv, 0, a.vn, a.first_v, a.ring_v); };
       // this thread's row of the tile and which keys it sees: kk <= see_hi and (kk >= see_lo or kk < see_keep)
       const int q = warp & 3, half = warp >> 2, r = q * 32 + lane;
       const uint32_t lanes = tb + ((uint32_t)(32 * q) << 16), mine = lanes + half * 32, o_mine = lanes + kTcO + half * dvh;
@@ -317,16 +339,16 @@ __device__ __forceinline__ void attend(const WinPromptArgs& a, int dv) {
         load_k(0);
         cp_async_commit();
         // the map's queries as bf16 (rows past the run are zero)
-#pragma unroll 8
-        for (int i = threadIdx.x; i < kTcRows * kc; i += kTcRowThreads) {
-          const int row = i / kc, c = i - row * kc;
-          float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
-          if (row < count) {
-            const float* src = a.qn + (((int64_t)(first + row) * a.H + h) * NM + m) * d + c * 8;
-            x = __ldg(reinterpret_cast<const float4*>(src)), y = __ldg(reinterpret_cast<const float4*>(src + 4));
+        const float* mine_q = a.qn + (((int64_t)(first + kp.row0) * a.H + h) * NM + m) * d + kp.c * 8;
+        const int64_t next_q = (int64_t)kp.rows * a.H * NM * d;
+        if (kp.c >= 0) {
+#pragma unroll 4
+          for (int row = kp.row0; row < kTcRows; row += kp.rows, mine_q += next_q) {
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+            if (row < count) x = __ldg(reinterpret_cast<const float4*>(mine_q)), y = __ldg(reinterpret_cast<const float4*>(mine_q + 4));
+            if (a.scale < 0.f) x = make_float4(-x.x, -x.y, -x.z, -x.w), y = make_float4(-y.x, -y.y, -y.z, -y.w);
+            *reinterpret_cast<uint4*>(Qs + tc_at(row, kp.c, kTcRows)) = make_uint4(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w), pack_bf16(y.x, y.y), pack_bf16(y.z, y.w));
           }
-          if (a.scale < 0.f) x = make_float4(-x.x, -x.y, -x.z, -x.w), y = make_float4(-y.x, -y.y, -y.z, -y.w);
-          *reinterpret_cast<uint4*>(Qs + tc_at(row, c, kTcRows)) = make_uint4(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w), pack_bf16(y.x, y.y), pack_bf16(y.z, y.w));
         }
         cp_async_wait<0>();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -357,7 +379,7 @@ __device__ __forceinline__ void attend(const WinPromptArgs& a, int dv) {
               if (!(i <= hi && (i >= low || i < kept))) x[i] = 0xFF800000u;
           }
 #pragma unroll
-          for (int i = 0; i < 32; ++i) top = fmaxf(top, __uint_as_float(x[i]));
+          for (int i = 0; i < 32; i += 2) top = tc_max3(top, __uint_as_float(x[i]), __uint_as_float(x[i + 1]));
           top *= to_log2;
         }
         // (the two warps of a lane quadrant; the other's value of the step before has been read: both have passed o_ready since)
@@ -442,15 +464,26 @@ __device__ __forceinline__ void attend(const WinPromptArgs& a, int dv) {
         row_l[r] = l + xch[kTcRows + r];
       }
       float* dst = reinterpret_cast<float*>(Ob + r * pitch) + half * dvh;
-      for (int c = 0; c < dvh; c += 8) {
-        uint32_t o[8];
-        tc_ld8(o_mine + c, o);
-        if (steps == 0) {
+      if (dvh == 64) {
+#pragma unroll 1
+        for (int c = 0; c < 64; c += 32) {
+          uint32_t o[32];
+          tc_ld32(o_mine + c, o);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] = 0u;
+          for (int i = 0; i < 32; i += 4)
+            *reinterpret_cast<uint4*>(dst + c + i) = steps == 0 ? make_uint4(0u, 0u, 0u, 0u) : make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
         }
-        *reinterpret_cast<uint4*>(dst + c) = make_uint4(o[0], o[1], o[2], o[3]);
-        *reinterpret_cast<uint4*>(dst + c + 4) = make_uint4(o[4], o[5], o[6], o[7]);
+      } else {
+        for (int c = 0; c < dvh; c += 8) {
+          uint32_t o[8];
+          tc_ld8(o_mine + c, o);
+          if (steps == 0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = 0u;
+          }
+          *reinterpret_cast<uint4*>(dst + c) = make_uint4(o[0], o[1], o[2], o[3]);
+          *reinterpret_cast<uint4*>(dst + c + 4) = make_uint4(o[4], o[5], o[6], o[7]);
+        }
       }
       tc_before();
     }
