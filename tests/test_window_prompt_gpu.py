@@ -143,3 +143,49 @@ def test_values_that_are_not_finite_reach_only_rows_that_see_them(maps, d, dv, H
     else:
         rows = ~bad.any(-1)
         assert ((got[rows] - ref[rows]).norm() / ref[rows].norm()).item() < 0.01
+
+
+@pytest.mark.parametrize("maps,d,H,G,n", [(1, 128, 16, 4, 600), (1, 128, 4, 2, 130), (2, 64, 8, 4, 300)])
+@pytest.mark.parametrize("captured", [False, True])
+def test_inputs_of_the_kernel_in_front_and_calls_behind_each_other(maps, d, H, G, n, captured):
+    """The launch may begin while the kernel in front ends.  That kernel writes the queries, keys and values here, and takes its time; calls follow
+    one another into buffers that the next copy reads: the same bits as calls with everything at rest between them."""
+    dv, L, p = 128, _lib.lm(), lambda t: t.data_ptr()
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    tile = ctypes.c_int()
+    _lib.lm_check(L.ao_lm_window_attention_prompt_plan(BF16, maps, H, G, d, dv, ctypes.byref(tile)), "plan")
+    i32 = lambda t: t.to(torch.int32).cuda()  # noqa: E731
+    first, back = torch.arange(0, n, tile.value), torch.arange(n)
+    slot, pos, tf, tc = i32(back * 0), i32(back), i32(first), i32((n - first).clamp(max=tile.value))
+    rk, rv = torch.zeros(1, 1024, G * maps * d, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, 1024, G * dv, dtype=torch.bfloat16, device="cuda")
+    sets = [(torch.randn(n, H, maps, d, generator=gen, device="cuda"), *(torch.randn(n, G, *w, generator=gen, device="cuda").to(torch.bfloat16)
+                                                                        for w in ((maps, d), (dv,)))) for _ in range(3)]
+    q, k, v = (torch.empty_like(t) for t in sets[0])
+    out, big = torch.empty(n, H * dv, dtype=torch.bfloat16, device="cuda"), torch.ones(1 << 24, device="cuda")
+
+    def call(one, result):
+        q.copy_(one[0]), k.copy_(one[1])
+        big.mul_(1.0)
+        v.copy_(one[2])
+        _lib.lm_check(L.ao_lm_window_attention_prompt(
+            p(q), p(k), p(v), p(rk), p(rv), None, None, 1024, 0, BF16, p(slot), p(pos), p(pos), p(tf), p(tc), tf.numel(), maps, H, G, d, dv, 1024, 0,
+            d ** -0.5, 0.4, int(maps == 2), 1e-6, 1.0, p(out), H * dv, torch.cuda.current_stream().cuda_stream), "prompt")
+        result.copy_(out)
+
+    want = [torch.empty_like(out) for _ in sets]
+    for one, result in zip(sets, want):
+        call(one, result)
+        torch.cuda.synchronize()
+    got = [torch.zeros_like(out) for _ in range(6)]
+    graph = torch.cuda.CUDAGraph() if captured else None
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=stream) if captured else torch.cuda.stream(stream):
+        for i, result in enumerate(got):
+            call(sets[i % 3], result)
+    with torch.cuda.stream(stream):
+        if captured:
+            graph.replay()
+    stream.synchronize()
+    for i, result in enumerate(got):
+        assert torch.equal(result, want[i % 3]), i

@@ -27,8 +27,10 @@
 // all keys of a tile in one CTA 110 us (the last tiles alone took 95), with unswizzled operands 84 us.
 // A warp's instructions follow one another at nearly five clocks each, so what counts is their number, about 740 per step at first: addresses once per map
 // instead of once per load, the largest score three at a time, O to shared memory 32 columns at a time: 57.6 -> 55.8 us, 117 rows of two maps 20.5 -> 19.2.
-// Taken back: the next step's scores beside this one's weights (two score buffers, p3 in shared memory: 57.4 -> 56.6, small sizes up to 5 % more); an early
-// and a late tile per cluster, in one wave (60.3).
+// Launched while the kernel in front ends (nothing of memory is touched before the wait): in a series of calls 59.4 -> 56.7 us.  Letting the kernel behind
+// start as early: 55.0, but 16 to 23 us calls up to 4 us more, as its CTAs take the places of the last ones of this.
+// Taken back: four threads per row (16 warps for the weights: 70.0 us in place of 55.8); the next step's scores beside this one's weights (two score buffers,
+// p3 in shared memory: 57.4 -> 56.6, small sizes up to 5 % more); an early and a late tile per cluster, in one wave (60.3).
 #include "../f32x2.h"
 #include "../per_device.h"
 #include "lm_mma.cuh"
@@ -594,6 +596,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) window_attention_tc_kernel(cons
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     tc_before();
   }
+  pdl_wait();
   __syncthreads();
   tc_after();
   attend<NM, C, false>(a, dv);
@@ -629,13 +632,15 @@ int launch(const WinPromptArgs& a, int dv, int n_tiles, cudaStream_t st) {
   cfg.blockDim = dim3(kTcThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = C;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   if (cudaLaunchKernelEx(&cfg, kern, a, dv) == cudaSuccess) return AO_B200_OK;
   return lm_launch_status();
 }
