@@ -1041,7 +1041,7 @@ static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
   // output tile leave of shared memory holds weights in flight
   // (even where two MMA warps alternate)
   if (KW == 2) p.x_slots = w.x_bytes > 24 * 1024 ? 3 : (w.x_bytes > 9 * 1024 || (DEFER && G == 64) ? 4 : (DEFER && G == 32 ? 2 : 6));
-  else p.x_slots = w.x_bytes > 24 * 1024 ? 3 : (w.x_bytes > 12 * 1024 ? 5 : (DEFER && G == 32 ? 4 : 8));
+  else p.x_slots = w.x_bytes > 24 * 1024 ? 3 : 5;   // (144 rows and more: 18 KB at least)
   const size_t unit = DIRECT ? 1024 : 16;      // (rows of 128 swizzled bytes: eight of them have to lie as the hardware counts)
   p.off_x = (uint32_t)((kWqHeader + (size_t)w.NT * kWqPitch + unit - 1) / unit * unit);
   const size_t off_w = (p.off_x + (size_t)p.x_slots * w.x_bytes + 127) / 128 * 128;
