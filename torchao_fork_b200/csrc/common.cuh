@@ -157,6 +157,22 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src_gmem, uint32_t 
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // PDL: let the next kernel in the stream start launching (its pre-wait prologue overlaps our tail)
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Launch that may begin while the kernel in front ends.  The kernel calls grid_dependency_wait() in every thread before it touches memory, and before any
+// grid_launch_dependents(): what follows counts on all that is in front of this kernel being over by then.
+template <typename... P, typename... A>
+static inline int launch_early(void (*kernel)(P...), dim3 grid, int threads, void* stream, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return e == cudaSuccess ? ao_launch_status() : (cudaGetLastError(), AO_B200_ERR_CUDA);
+}
 // How a GEMV follows the kernel in front of it in the stream: started behind its end; or started while it ends, with the weights read behind the wait too
 // (ordered: they may be what that kernel writes) or before it (settled: the caller answers for weights that were there before it).
 enum GemvFollow : int { kFollowPlain = 0, kFollowOrdered = 1, kFollowSettled = 2 };

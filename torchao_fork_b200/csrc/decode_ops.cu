@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(kThreads) rmsnorm_pieces_kernel(const __nv_bfl
                                                                   const __nv_bfloat16* __restrict__ weight, __nv_bfloat16* __restrict__ h_out,
                                                                   __nv_bfloat16* __restrict__ y, int dim, float eps) {
   __shared__ float s_part[kThreads / 32];
+  grid_dependency_wait();
   grid_launch_dependents();
   const int64_t at = (int64_t)blockIdx.x * dim;
   uint4 v[N], wv[N];
@@ -503,10 +504,9 @@ extern "C" int ao_b200_rmsnorm(const void* x, const void* residual, const void* 
   AO_CHECK_ARG(ao_aligned(x, 16) && ao_aligned(weight, 16) && ao_aligned(y, 16));
   AO_CHECK_ARG((!residual || ao_aligned(residual, 16)) && (!h_out || ao_aligned(h_out, 16)));
   auto pieces = [&](auto* kernel) {
-    kernel<<<static_cast<unsigned>(rows), 512, 0, static_cast<cudaStream_t>(stream)>>>(
+    return ao::launch_early(kernel, dim3(static_cast<unsigned>(rows)), 512, stream,
         static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(residual), static_cast<const __nv_bfloat16*>(weight),
         static_cast<__nv_bfloat16*>(h_out), static_cast<__nv_bfloat16*>(y), (int)dim, eps);
-    return ao_launch_status();
   };
   if (dim <= 512 * 8) return pieces(rmsnorm_pieces_kernel<512, 1>);
   if (dim <= 512 * 16) return pieces(rmsnorm_pieces_kernel<512, 2>);

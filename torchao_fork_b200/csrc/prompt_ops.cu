@@ -1,7 +1,8 @@
 // What the Llama block does between its products for rows of a prompt, one pass each: rotation of queries and keys, SiLU * up (the
 // norm is rmsnorm_kernel of decode_ops.cu).  As tensor operations these were ten passes and more over fp32 copies: 700 tokens through two
 // Mistral-7B layers and the output product took 1956 us of which about 850 were such passes, now 1036 in all.  Bound by memory;
-// 16 bytes per thread.  The roundings are those of the single operations: fp32 products rounded before they are added (no fused
+// 16 bytes per thread.  Each is launched while the kernel in front ends (launch_early) and waits for it
+// before anything else: that forward 949 -> 918 us.  The roundings are those of the single operations: fp32 products rounded before they are added (no fused
 // multiply-add), silu rounded to bf16 before its product.
 #include <cassert>
 
@@ -24,6 +25,7 @@ __device__ __forceinline__ uint32_t rotate_pair(uint32_t x, uint32_t cs) {
 // x [B][T][H][8 n8] (any strides that are whole 16-byte pieces) -> y, packed; freqs [T][8 n8]: cos, sin of every pair
 __global__ void __launch_bounds__(256) rotary_kernel(const uint4* __restrict__ x, int64_t sb, int64_t st, int64_t sh, const uint4* __restrict__ freqs,
                                                      uint4* __restrict__ y, int T, int H, int n8, int64_t total) {
+  grid_dependency_wait();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= total) return;
   const int c = (int)(i % n8);
@@ -40,6 +42,7 @@ __global__ void __launch_bounds__(256) rotary_kernel(const uint4* __restrict__ x
 __global__ void __launch_bounds__(256) kv_rows_kernel(const uint4* __restrict__ k, int64_t kb, int64_t kt, int64_t kh, const uint4* __restrict__ v, int64_t vb,
                                                       int64_t vt, int64_t vh, const uint4* __restrict__ freqs, const void* __restrict__ pos, bool pos64,
                                                       uint4* __restrict__ k_cache, uint4* __restrict__ v_cache, int T, int H, int S, int n8, int64_t total) {
+  grid_dependency_wait();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= total) return;
   const int c = (int)(i % n8);
@@ -60,6 +63,7 @@ __global__ void __launch_bounds__(256) kv_rows_kernel(const uint4* __restrict__ 
 // that read a head rep times: 19 us a layer for 704 positions of 8 heads, rep 4; 11.5 MB to write).
 __global__ void __launch_bounds__(256) repeat_heads_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v, uint4* __restrict__ k_out,
                                                            uint4* __restrict__ v_out, int64_t head, int64_t total, int rep) {
+  grid_dependency_wait();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= total) return;
   const uint4 x = (blockIdx.y == 0 ? k : v)[i];
@@ -70,6 +74,7 @@ __global__ void __launch_bounds__(256) repeat_heads_kernel(const uint4* __restri
 __device__ __forceinline__ float silu_f(float g) { return __uint_as_float(float_to_bf16_bits(g / (1.f + expf(-g))) << 16); }
 __device__ __forceinline__ uint32_t silu_mul_pair(uint32_t g, uint32_t u) { return pack_rn(silu_f(lo_f(g)) * lo_f(u), silu_f(hi_f(g)) * hi_f(u)); }
 __global__ void __launch_bounds__(256) silu_mul_rows_kernel(const uint4* __restrict__ gate, const uint4* __restrict__ up, uint4* __restrict__ y, int64_t n8) {
+  grid_dependency_wait();
   grid_launch_dependents();   // (a kernel that follows programmatically waits before it reads)
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= n8) return;
@@ -86,10 +91,9 @@ extern "C" int ao_b200_rotary(const void* x, int64_t stride_b, int64_t stride_t,
   AO_CHECK_ARG(stride_b % 8 == 0 && stride_t % 8 == 0 && stride_h % 8 == 0 && ao_aligned(x, 16) && ao_aligned(freqs_cis, 16) && ao_aligned(y, 16));
   const int64_t total = B * T * H * (head_dim / 8), blocks = (total + 255) / 256;
   if (T > 2147483647 || H > 2147483647 || blocks > 2147483647) return AO_B200_ERR_UNSUPPORTED;
-  ao::rotary_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  return ao::launch_early(ao::rotary_kernel, dim3((unsigned)blocks), 256, stream,
       static_cast<const uint4*>(x), stride_b / 8, stride_t / 8, stride_h / 8, static_cast<const uint4*>(freqs_cis), static_cast<uint4*>(y), (int)T, (int)H,
       (int)(head_dim / 8), total);
-  return ao_launch_status();
 }
 
 extern "C" int ao_b200_kv_rows(const void* k, int64_t k_stride_b, int64_t k_stride_t, int64_t k_stride_h, const void* v, int64_t v_stride_b, int64_t v_stride_t,
@@ -101,10 +105,9 @@ extern "C" int ao_b200_kv_rows(const void* k, int64_t k_stride_b, int64_t k_stri
   AO_CHECK_ARG((pos_bytes == 4 || pos_bytes == 8) && ao_aligned(pos, pos_bytes));
   const int64_t total = B * T * H * (head_dim / 8), blocks = (total + 255) / 256;
   if (T > 2147483647 || H > 2147483647 || S > 2147483647 || blocks > 2147483647) return AO_B200_ERR_UNSUPPORTED;
-  ao::kv_rows_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  return ao::launch_early(ao::kv_rows_kernel, dim3((unsigned)blocks), 256, stream,
       static_cast<const uint4*>(k), k_stride_b / 8, k_stride_t / 8, k_stride_h / 8, static_cast<const uint4*>(v), v_stride_b / 8, v_stride_t / 8, v_stride_h / 8,
       static_cast<const uint4*>(freqs_cis), pos, pos_bytes == 8, static_cast<uint4*>(k_cache), static_cast<uint4*>(v_cache), (int)T, (int)H, (int)S, (int)(head_dim / 8), total);
-  return ao_launch_status();
 }
 
 extern "C" int ao_b200_repeat_heads(const void* k, const void* v, void* k_out, void* v_out, int64_t heads, int64_t head_elements, int64_t rep, void* stream) {
@@ -112,16 +115,14 @@ extern "C" int ao_b200_repeat_heads(const void* k, const void* v, void* k_out, v
   AO_CHECK_ARG(ao_aligned(k, 16) && ao_aligned(v, 16) && ao_aligned(k_out, 16) && ao_aligned(v_out, 16));
   const int64_t head = head_elements / 8, total = heads * head, blocks = (total + 255) / 256;
   if (rep > 2147483647 || blocks > 2147483647) return AO_B200_ERR_UNSUPPORTED;
-  ao::repeat_heads_kernel<<<dim3((unsigned)blocks, 2), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  return ao::launch_early(ao::repeat_heads_kernel, dim3((unsigned)blocks, 2), 256, stream,
       static_cast<const uint4*>(k), static_cast<const uint4*>(v), static_cast<uint4*>(k_out), static_cast<uint4*>(v_out), head, total, (int)rep);
-  return ao_launch_status();
 }
 
 extern "C" int ao_b200_silu_mul_rows(const void* gate, const void* up, void* y, int64_t count, void* stream) {
   AO_CHECK_ARG(gate && up && y && count > 0 && count % 8 == 0 && ao_aligned(gate, 16) && ao_aligned(up, 16) && ao_aligned(y, 16));
   const int64_t n8 = count / 8, blocks = (n8 + 255) / 256;
   if (blocks > 2147483647) return AO_B200_ERR_UNSUPPORTED;
-  ao::silu_mul_rows_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint4*>(gate), static_cast<const uint4*>(up),
-                                                                                        static_cast<uint4*>(y), n8);
-  return ao_launch_status();
+  return ao::launch_early(ao::silu_mul_rows_kernel, dim3((unsigned)blocks), 256, stream, static_cast<const uint4*>(gate), static_cast<const uint4*>(up),
+                          static_cast<uint4*>(y), n8);
 }
