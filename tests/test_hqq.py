@@ -240,3 +240,32 @@ def test_groups_at_rest_give_what_their_iterations_would(shape, iters, kappa, gs
         same = (got.view(torch.int32) == zero.view(torch.int32)) | (got.isnan() & zero.isnan())
         assert bool(same.all()), int((~same).sum())
         assert bool(zero.isnan().any()) == odd
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gs", [32, 64, 128, 256])
+@pytest.mark.parametrize("over", [-7, -1, 0, 1, 9])
+def test_lists_that_end_inside_a_warp(gs, over):
+    """A block's warps race for the last groups of its list, and a warp gets none, some or all of what its lanes could take; whether it fetches at all is one
+    answer for all its lanes.  Groups that rest at once beside groups that never do, so that lanes come free one by one; several times over,
+    as the race ends otherwise each time, and the numbers must not."""
+    n_groups = 8192 // gs * 3 + over   # three blocks' worth, a little less, a little more
+    g = torch.Generator(device="cuda").manual_seed(gs + over)
+    w = torch.randn(n_groups, gs, device="cuda", generator=g) * (10 ** (3 * torch.rand(n_groups, 1, device="cuda", generator=g) - 2))
+    w = w.to(torch.bfloat16)
+    from torchao_fork_b200 import _lib
+    from torchao_fork_b200 import ops as aops
+    L, st = _lib.lib(), torch.cuda.current_stream().cuda_stream
+    scale = torch.empty(n_groups, dtype=torch.float32, device="cuda")
+    zero, err = torch.empty_like(scale), torch.empty(int(L.ao_b200_hqq_blocks(n_groups)), dtype=torch.float32, device="cuda")
+    state = torch.empty(2, dtype=torch.float64, device="cuda")
+    q0 = torch.empty(n_groups, gs, dtype=torch.int32, device="cuda")
+    s0, z0 = (torch.empty(n_groups, 1, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    _lib.check(L.ao_b200_hqq_init(w.data_ptr(), n_groups, gs, scale.data_ptr(), zero.data_ptr(), st), "init")
+    _lib.check(L.ao_b200_hqq_solve(w.data_ptr(), n_groups, gs, scale.data_ptr(), zero.data_ptr(), aops.HQQ_BETA, aops.HQQ_KAPPA, aops.HQQ_LP_NORM,
+                                   aops.HQQ_ITERS, err.data_ptr(), state.data_ptr(), st), "solve")
+    _lib.check(L.ao_b200_hqq_finalize(w.data_ptr(), n_groups, gs, scale.data_ptr(), zero.data_ptr(), q0.data_ptr(), s0.data_ptr(), z0.data_ptr(), st),
+               "finalize")
+    for _ in range(5):
+        q, s, z = T.b200_int4_hqq_quantize(w, gs)
+        assert torch.equal(s, s0) and torch.equal(z, z0) and torch.equal(q, q0)

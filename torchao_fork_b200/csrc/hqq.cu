@@ -146,8 +146,8 @@ __global__ void __launch_bounds__(kHqqWarps * 32) hqq_finalize_kernel(const __nv
 // to come, gives the same zero point and error in every iteration that follows, so it is at rest and its lanes take the next group.  A zero point
 // moves by the mean rounding error and settles as soon as no weight crosses a rounding boundary on the way: of normal weights in groups of 32 / 64 / 128 / 256
 // 2.4 / 3.4 / 4.8 / 6.7 iterations of 20 move it, and one more shows it.  (Groups that never rest, as with weights of spread 3, where powf decides: 1361 -> 1549 us.)
-// The search over 4096 x 4096, groups of 64, 20 iterations, in all its kernels: 199 us with all iterations of all groups, 108 without those at rest
-// (groups of 32 / 128 / 256: 212 / 227 / 186 -> 113 / 121 / 130).  Taken back: groups put together anew among a block's warps after each iteration (155),
+// The search over 4096 x 4096, groups of 64, 20 iterations, in all its kernels: 199 us with all iterations of all groups, 105 without those at rest
+// (groups of 32 / 128 / 256: 212 / 227 / 186 -> 113 / 120 / 129).  Taken back: groups put together anew among a block's warps after each iteration (155),
 // rounds of two and three iterations over a block's list (141).
 constexpr int kHqqChunk = 10;   // iterations per launch: bounds hist to 10 numbers per group
 constexpr int kHqqMaxIters = 64;
@@ -252,10 +252,13 @@ __global__ void __launch_bounds__(kHqqThreads, kHqqBlocks) hqq_iterate_kernel(co
 #pragma unroll 1
     for (;;) {
       const uint32_t idle = __ballot_sync(0xffffffffu, !moves);
-      if (idle != 0 && *reinterpret_cast<volatile int*>(&s_next) < n) {
-        int at = 0;
-        if (lane == 0) at = atomicAdd(&s_next, __popc(idle) / L);
-        at = __shfl_sync(0xffffffffu, at, 0) + __popc(idle & ((1u << lane) - 1u)) / L;
+      int next = n;                // lane 0 looks for its warp: other warps move s_next meanwhile, and all lanes have to come to the same answer
+      if (idle != 0) {
+        if (lane == 0 && *reinterpret_cast<volatile int*>(&s_next) < n) next = atomicAdd(&s_next, __popc(idle) / L);
+        next = __shfl_sync(0xffffffffu, next, 0);
+      }
+      if (next < n) {
+        const int at = next + __popc(idle & ((1u << lane) - 1u)) / L;
         const bool fresh = !moves && at < n;
         if (fresh) {
           g = s_todo[at], it = 0, moves = true;
