@@ -217,6 +217,16 @@ AO_B200_API int64_t ao_b200_mm_residual_workspace_bytes(int64_t M, int64_t Np, i
 AO_B200_API int ao_b200_mm_residual(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scales, int64_t Np,
                                     int64_t Kp, int group_size, void* y, int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res,
                                     void* workspace, int64_t workspace_bytes, void* stream);
+/* How the GEMM of these products (csrc/gemm_wq_tc.cu) cuts up a call of M rows of Kp on Np outputs, group_size 0: int8; for tests and tools.
+ * No launch, no GPU: without one 148 SMs are counted on.  AO_B200_ERR_UNSUPPORTED: not a shape of the GEMM. */
+typedef struct {
+  int64_t tiles;                            /* of rows_per_tile rows x 128 outputs (pair: 256) */
+  int32_t rows_per_tile, row_tiles, unit_k, units_per_tile;
+  int32_t pair, defer, in_place, early;     /* 0 / 1 */
+  int32_t workers, quantum, base, rem;      /* worker c starts at unit (c base + min(c, rem)) quantum of tiles x units_per_tile */
+  int32_t weight_slots, activation_slots, operand_slots, issuers;
+} ao_b200_mm_cut;
+AO_B200_API int ao_b200_mm_plan(int64_t M, int64_t Np, int64_t Kp, int group_size, ao_b200_mm_cut* cut);
 AO_B200_API int ao_b200_int8_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx,
                     const void* packed, const void* scale, int64_t Np, int64_t Kp,
                     void* y, int64_t N_out, int64_t ldy, void* workspace, int64_t workspace_bytes, void* stream);

@@ -4,30 +4,34 @@ the parity of its phase, so a wait that may look for a phase too early takes the
 
 What is modelled: the rings of weights, activations and tensor-memory operands, the two sets of dequant warps (two warps each), one or
 two issuing warps, one CTA or a pair, the accumulators and the epilogue, both forms (DEFER: the epilogue reads every unit), and the last tile that
-stays in its accumulators until all warps finish it (EARLY: each CTA of a pair decides for itself).  What each slot holds is followed, and every read and overwrite is checked.  The ring sizes are those of wq_launch for every row count and group."""
+stays in its accumulators until all warps finish it (EARLY: each CTA of a pair decides for itself).  What each slot holds is followed, and every read and overwrite is checked.  The ring sizes are those that the
+library names for every row count and group, with activations staged and read in place."""
+import ctypes
+import os
 import random
 
 import pytest
 
-HEADER, PITCH, BUDGET, MAX_W, A_SLOTS = 1024, 272, 226 * 1024, 16, 4
+from torchao_fork_b200 import _lib
+
+if not os.path.exists(_lib.LIB_PATH):
+    pytest.skip("libao_b200.so not built (python -m torchao_fork_b200.build)", allow_module_level=True)
+
+A_SLOTS = 4   # of 128 k in tensor memory
 
 
-def plan(m, group):
-    """wq_plan and wq_launch: ring sizes of a call of m rows (group 0: int8)"""
-    int4 = group != 0
-    defer, pair = int4 and m <= 16, m > 32
-    mt = -(-m // 256)
-    nt = -(-(-(-m // mt)) // 16) * 16
-    br = nt // (2 if pair else 1)
-    xb = br * 256 + (256 if defer else 0)
-    wb = 8 * 2 * (512 if int4 else 1024) + (8 * (128 // group if group < 128 else 1) * 64 if int4 else 0)
-    n_mma = 2 if nt <= 64 else 1
-    x = 3 if xb > 24 * 1024 else 5 if xb > 12 * 1024 else 4 if defer and group == 32 else 8
-    off = -(-(HEADER + nt * PITCH + x * xb) // 128) * 128
-    w = min(MAX_W, (BUDGET - off) // wb)
-    if n_mma == 2:
-        w &= ~1
-    return dict(w=w, x=x, a=3 if w == 3 else A_SLOTS, n_mma=n_mma, d=2 if nt <= 128 else 1, defer=defer, pair=pair)
+def cut(m, np_, kp, group):
+    """How the library cuts up a call (ao_b200_mm_plan; group 0: int8)"""
+    c = _lib.MmCut()
+    _lib.check(_lib.lib().ao_b200_mm_plan(m, np_, kp, group, ctypes.byref(c)), "mm_plan")
+    return c
+
+
+def plan(m, group, np_=16384):
+    """The rings of a call of m rows"""
+    c = cut(m, np_, 8192, group)
+    return dict(w=c.weight_slots, x=c.activation_slots, a=c.operand_slots, n_mma=c.issuers, d=2 if c.rows_per_tile <= 128 else 1, defer=bool(c.defer),
+                pair=bool(c.pair))
 
 
 class Wrong(Exception):
@@ -317,9 +321,10 @@ class Model:
 def _plans():
     seen = {}
     for group in (0, 32, 64, 128, 256):
-        for m in list(range(1, 530)) + [600, 1000, 2048, 4096]:
-            c = plan(m, group)
-            seen.setdefault(tuple(sorted(c.items())), (m, group, c))
+        for m in list(range(1, 1030)) + [2048, 4096]:
+            for np_ in (16384, 8192):   # above 8192 outputs activations are staged, up to there read in place from 512 rows on
+                c = plan(m, group, np_)
+                seen.setdefault(tuple(sorted(c.items())), (m, group, c))
     return list(seen.values())
 
 
@@ -330,7 +335,7 @@ def test_plans_cover_short_odd_and_even_rings_one_and_two_issuers():
     kinds = {(c["w"] % 2, c["w"] < c["a"] + 2, c["n_mma"], c["defer"], c["pair"]) for _, _, c in PLANS}
     assert any(w and short for w, short, *_ in kinds) and any(not w and n == 2 for w, _, n, *_ in kinds)
     for _, _, c in PLANS:
-        assert c["w"] >= 2 and c["a"] <= max(c["w"], A_SLOTS) and (c["n_mma"] == 1 or (c["w"] % 2 == 0 and c["x"] % 2 == 0 and c["a"] % 2 == 0))
+        assert c["w"] >= 2 and 2 <= c["a"] <= max(c["w"], A_SLOTS) and (c["n_mma"] == 1 or (c["w"] % 2 == 0 and c["x"] % 2 == 0 and c["a"] % 2 == 0))
 
 
 @pytest.mark.parametrize("m,group,cfg", PLANS, ids=[f"{m} rows, group {g}" for m, g, _ in PLANS])
@@ -367,51 +372,3 @@ def test_the_model_sees_what_the_rules_prevent():
     # a last tile that is taken without waiting for its products
     even = plan(64, 128)
     assert _found(even, early=True, early_before_products=True) and not _found(even, early=True)
-
-
-def direct_plan(m, group):
-    """the same for calls that read the activations where they are: their ring starts on a multiple of 1024 bytes"""
-    c = plan(m, group)
-    mt = -(-m // 256)
-    nt = -(-(-(-m // mt)) // 16) * 16
-    wb = 8 * 2 * (512 if group else 1024) + (8 * (128 // group if group < 128 else 1) * 64 if group else 0)
-    off = -(-(-(-(HEADER + nt * PITCH) // 1024) * 1024 + c["x"] * nt // 2 * 256) // 128) * 128
-    c["w"] = min(MAX_W, (BUDGET - off) // wb)
-    c["a"] = 3 if c["w"] == 3 else A_SLOTS
-    return c
-
-
-@pytest.mark.parametrize("group", [0, 32, 64, 128, 256])
-def test_rings_of_activations_read_in_place(group):
-    plans = {tuple(sorted(direct_plan(m, group).items())): direct_plan(m, group) for m in range(512, 4200, 3)}
-    for cfg in plans.values():
-        assert cfg["w"] >= 2 and cfg["a"] <= cfg["w"] and cfg["n_mma"] == 1
-        for seed in range(6):
-            rng = random.Random(seed)
-            ku = rng.choice([1, 2, 3, 5, 8, 64])
-            Model(rng, cfg, rng.randint(1, 40), ku, first=rng.randint(0, 2 * ku), early=seed % 2 == 1).run()
-
-
-def long_plan(m, group):
-    """the same for calls of up to 128 rows, whose units have 256 k: rings of half as many slots of operands"""
-    c = plan(m, group)
-    nt = -(-m // 16) * 16
-    xb = 2 * (nt // (2 if c["pair"] else 1) * 256 + (256 if c["defer"] else 0))
-    wb = 2 * (8 * 2 * (512 if group else 1024) + (8 * (128 // group if group < 128 else 1) * 64 if group else 0))
-    c["x"] = 3 if xb > 24 * 1024 else 4 if xb > 9 * 1024 or (c["defer"] and group == 64) else 2 if c["defer"] and group == 32 else 6
-    off = -(-(HEADER + nt * PITCH + c["x"] * xb) // 128) * 128
-    c["w"], c["a"] = min(MAX_W, (BUDGET - off) // wb), A_SLOTS // 2
-    if c["n_mma"] == 2:
-        c["w"] &= ~1
-    return c
-
-
-@pytest.mark.parametrize("group", [0, 32, 64, 128, 256])
-def test_rings_of_long_units(group):
-    plans = {tuple(sorted(long_plan(m, group).items())): (m, long_plan(m, group)) for m in range(1, 129)}
-    for m, cfg in plans.values():
-        assert cfg["w"] >= 2 and (cfg["n_mma"] == 1 or (cfg["w"] % 2 == 0 and cfg["x"] % 2 == 0))
-        for seed in range(8):
-            rng = random.Random(seed)
-            ku = rng.choice([1, 2, 3, 5, 8, 64])
-            Model(rng, cfg, rng.randint(1, 40), ku, first=rng.randint(0, 2 * ku), early=seed % 2 == 1 and not cfg["defer"]).run()

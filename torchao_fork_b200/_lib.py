@@ -31,6 +31,14 @@ class MegaModel(ctypes.Structure):
 
 _mp = ctypes.POINTER(MegaModel)
 
+
+class MmCut(ctypes.Structure):
+    """ao_b200_mm_cut (include/ao_b200.h)"""
+    _fields_ = [("tiles", _i64)] + [(n, ctypes.c_int32) for n in (
+        "rows_per_tile", "row_tiles", "unit_k", "units_per_tile", "pair", "defer", "in_place", "early", "workers", "quantum", "base", "rem",
+        "weight_slots", "activation_slots", "operand_slots", "issuers")]
+
+
 # name -> argtypes (all return int unless listed in _RESTYPES)
 SIGNATURES = {
     "ao_b200_error_string": [_i32],
@@ -53,6 +61,7 @@ SIGNATURES = {
     "ao_b200_int8_unpack": [_vp, _i64, _i64, _i64, _i64, _vp, _vp],
     "ao_b200_int8_mm_workspace_bytes": [_i64, _i64, _i64],
     "ao_b200_mm_residual_workspace_bytes": [_i64, _i64, _i64, _i32],
+    "ao_b200_mm_plan": [_i64, _i64, _i64, _i32, ctypes.POINTER(MmCut)],
     "ao_b200_mm_residual": [_vp, _i64, _i64, _i64, _vp, _vp, _i64, _i64, _i32, _vp, _i64, _i64, _vp, _i64, _vp, _i64, _vp],
     "ao_b200_hqq_blocks": [_i64],
     "ao_b200_hqq_init": [_vp, _i64, _i32, _vp, _vp, _vp],

@@ -22,6 +22,7 @@ int int4_gemm_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* 
 bool int4_gemv_fused_fits(int64_t M, int64_t Kp, int G, int max_stages);
 bool int8_gemv_fused_fits(int64_t M, int64_t Kp, int max_stages);
 int64_t int4_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
+bool gemm_tc_plan(int64_t M, int64_t Np, int64_t Kp, int G, ao_b200_mm_cut& c);
 int64_t int8_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
 int int8_gemv(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scale, int64_t Kp,
               void* y, int64_t N_out, int64_t ldy, cudaStream_t s);
@@ -280,6 +281,11 @@ extern "C" int ao_b200_int8_gemv_fused(const void* x, int64_t M, int64_t Kx, int
 // ---- y = bf16(residual + bf16(x W'^T)) for any number of rows: by the GEMM, a few rows of long k by the GEMV over clusters ----------------------------------------
 extern "C" int64_t ao_b200_mm_residual_workspace_bytes(int64_t M, int64_t Np, int64_t Kp, int group_size) {
   return group_size ? ao::int4_gemm_tc_workspace_bytes(M, Np, Kp) : ao::int8_gemm_tc_workspace_bytes(M, Np, Kp);
+}
+extern "C" int ao_b200_mm_plan(int64_t M, int64_t Np, int64_t Kp, int group_size, ao_b200_mm_cut* cut) {
+  AO_CHECK_ARG(cut != nullptr && M > 0 && Np > 0 && Kp > 0);
+  AO_CHECK_ARG(group_size == 0 || group_size == 32 || group_size == 64 || group_size == 128 || group_size == 256);
+  return ao::gemm_tc_plan(M, Np, Kp, group_size, *cut) ? AO_B200_OK : AO_B200_ERR_UNSUPPORTED;
 }
 extern "C" int ao_b200_mm_residual(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* scales, int64_t Np,
                                    int64_t Kp, int group_size, void* y, int64_t N_out, int64_t ldy, const void* residual, int64_t ld_res,

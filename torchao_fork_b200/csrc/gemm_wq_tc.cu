@@ -1032,35 +1032,53 @@ static bool wq_map(CUtensorMap* map, CUtensorMapDataType type, int elem, const v
   return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess && encode();
 }
 
-template <int G, bool DEFER, bool PAIR, bool DIRECT, int KW>
-static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
-  constexpr uint32_t kWSlot = KW * (8 * 2 * (G == 0 ? 1024 : 512) + (G == 0 ? 0 : 8 * (G < 128 ? 128 / (G ? G : 128) : 1) * 64));
-  constexpr size_t kBudget = 226 * 1024;
-  p.n_mma = w.NT <= 64 ? 2 : 1;
+// rings in shared and tensor memory of a call with groups of G (0: int8), a function of its plan too
+struct WqRings {
+  int n_mma, x_slots, w_slots, a_slots;
+  uint32_t off_x, off_w, w_slot;  // activation ring, weight ring, bytes of a slot of weights
+  bool early;
+};
+constexpr size_t kWqBudget = 226 * 1024;
+
+static WqRings wq_rings(const WqPlan& w, int G) {
+  WqRings r;
+  r.n_mma = w.NT <= 64 ? 2 : 1;
+  r.w_slot = (uint32_t)(w.KW * (8 * 2 * (G == 0 ? 1024 : 512) + (G == 0 ? 0 : 8 * (G < 128 ? 128 / G : 1) * 64)));
   // tiles of x in flight (an L2 round trip is about 850 clocks; DEFER: as many as there are accumulators); what they and the
   // output tile leave of shared memory holds weights in flight
   // (even where two MMA warps alternate)
-  if (KW == 2) p.x_slots = w.x_bytes > 24 * 1024 ? 3 : (w.x_bytes > 9 * 1024 || (DEFER && G == 64) ? 4 : (DEFER && G == 32 ? 2 : 6));
-  else p.x_slots = w.x_bytes > 24 * 1024 ? 3 : 5;   // (144 rows and more: 18 KB at least)
-  const size_t unit = DIRECT ? 1024 : 16;      // (rows of 128 swizzled bytes: eight of them have to lie as the hardware counts)
-  p.off_x = (uint32_t)((kWqHeader + (size_t)w.NT * kWqPitch + unit - 1) / unit * unit);
-  const size_t off_w = (p.off_x + (size_t)p.x_slots * w.x_bytes + 127) / 128 * 128;
-  p.off_w = (uint32_t)off_w;
-  p.w_slots = (int)((kBudget - off_w) / kWSlot);
-  if (p.w_slots > kWqMaxW) p.w_slots = kWqMaxW;
-  if (p.n_mma == 2) p.w_slots &= ~1;           // two MMA warps let the two dequant sets drift apart: each set keeps slots of its own
-  p.a_slots = KW == 2 ? kWqSlots / 2 : (p.w_slots == 3 ? 3 : kWqSlots);   // (see a_first in the kernel)
-  const size_t smem = off_w + (size_t)p.w_slots * kWSlot;
+  if (w.KW == 2) r.x_slots = w.x_bytes > 24 * 1024 ? 3 : (w.x_bytes > 9 * 1024 || (w.defer && G == 64) ? 4 : (w.defer && G == 32 ? 2 : 6));
+  else r.x_slots = w.x_bytes > 24 * 1024 ? 3 : 5;   // (144 rows and more: 18 KB at least)
+  const size_t unit = w.direct ? 1024 : 16;    // (rows of 128 swizzled bytes: eight of them have to lie as the hardware counts)
+  r.off_x = (uint32_t)((kWqHeader + (size_t)w.NT * kWqPitch + unit - 1) / unit * unit);
+  r.off_w = (uint32_t)((r.off_x + (size_t)r.x_slots * w.x_bytes + 127) / 128 * 128);
+  r.w_slots = (int)((kWqBudget - r.off_w) / r.w_slot);
+  if (r.w_slots > kWqMaxW) r.w_slots = kWqMaxW;
+  if (r.n_mma == 2) r.w_slots &= ~1;           // two MMA warps let the two dequant sets drift apart: each set keeps slots of its own
+  r.a_slots = w.KW == 2 ? kWqSlots / 2 : (r.w_slots == 3 ? 3 : kWqSlots);   // (see a_first in the kernel)
   // The last tile from the accumulators where every CTA has a tile's worth of units, so that a tile has two owners as a rule: 4096 x 4096, 2048 rows
   // 63.9 -> 57.1 us; 14336 x 4096 int4, 300 / 1000 rows 39.8 -> 36.2 / 94.0 -> 89.3; 28672 x 4096 int8, 32 / 77 / 300 rows 32.4 -> 30.9 / 37.7 -> 34.9 /
   // 74.6 -> 70.9.  With less a CTA its neighbour is not there yet or it has several, and the mere presence of the code costs 0.2 to 0.5 us
   // (14336 x 4096, 77 rows: 25.6 -> 25.8; 4096 x 4096 int8, 200 rows: 28.5 -> 29.0).
-  constexpr bool kCan = !DEFER;
-  const bool early = kCan && (int64_t)w.base * w.quantum >= w.KU;
+  r.early = !w.defer && (int64_t)w.base * w.quantum >= w.KU;
+  return r;
+}
+
+template <int G, bool DEFER, bool PAIR, bool DIRECT, int KW>
+static int wq_launch(WqParams& p, const WqPlan& w, cudaStream_t s) {
+  const WqRings r = wq_rings(w, G);
+  p.n_mma = r.n_mma;
+  p.x_slots = r.x_slots;
+  p.w_slots = r.w_slots;
+  p.a_slots = r.a_slots;
+  p.off_x = r.off_x;
+  p.off_w = r.off_w;
+  const size_t smem = r.off_w + (size_t)r.w_slots * r.w_slot;
+  const bool early = r.early;
   auto kern = wq_gemm_kernel<G, DEFER, PAIR, DIRECT, false, KW>;
   static OncePerDevice once[2];
-  if (early) kern = wq_gemm_kernel<G, DEFER, PAIR, DIRECT, kCan, KW>;
-  if (!dynamic_smem(once[early], kern, (int)kBudget)) return AO_B200_ERR_CUDA;
+  if (early) kern = wq_gemm_kernel<G, DEFER, PAIR, DIRECT, !DEFER, KW>;
+  if (!dynamic_smem(once[early], kern, (int)kWqBudget)) return AO_B200_ERR_CUDA;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(w.workers * w.ranks));
   cfg.blockDim = dim3(kWqThreads);
@@ -1191,6 +1209,30 @@ int64_t int4_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp) {
 int64_t int8_gemm_tc_workspace_bytes(int64_t M, int64_t Np, int64_t Kp) {
   WqPlan w;
   return wq_plan(M, Np, Kp, false, w) ? w.bytes : 0;
+}
+// how a call of M rows is cut up (ao_b200_mm_plan)
+bool gemm_tc_plan(int64_t M, int64_t Np, int64_t Kp, int G, ao_b200_mm_cut& c) {
+  WqPlan w;
+  if (!wq_plan(M, Np, Kp, G != 0, w)) return false;
+  const WqRings r = wq_rings(w, G);
+  c.rows_per_tile = w.NT;
+  c.row_tiles = w.MT;
+  c.tiles = w.tiles;
+  c.unit_k = 128 * w.KW;
+  c.units_per_tile = w.KU;
+  c.pair = w.pair;
+  c.defer = w.defer;
+  c.in_place = w.direct;
+  c.workers = w.workers;
+  c.quantum = w.quantum;
+  c.base = w.base;
+  c.rem = w.rem;
+  c.weight_slots = r.w_slots;
+  c.activation_slots = r.x_slots;
+  c.operand_slots = r.a_slots;
+  c.issuers = r.n_mma;
+  c.early = r.early;
+  return true;
 }
 
 int int4_gemm_tc(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void* packed, const void* sz, int64_t Np, int64_t Kp, int G, void* y,
