@@ -372,3 +372,33 @@ def test_the_model_sees_what_the_rules_prevent():
     # a last tile that is taken without waiting for its products
     even = plan(64, 128)
     assert _found(even, early=True, early_before_products=True) and not _found(even, early=True)
+
+
+def _first(c, worker):
+    return (worker * c.base + min(worker, c.rem)) * c.quantum
+
+
+SHAPES = [(m, np_, kp, g) for m in (1, 16, 17, 32, 33, 64, 100, 128, 129, 600, 5000) for np_ in (128, 256, 1024, 1152, 4096, 14336, 28672)
+          for kp in (64, 128, 256, 512, 768, 1024, 1280, 1792, 2304, 2816, 3328, 4096, 4160, 9472, 16384) for g in (0, 128)]
+
+
+def test_every_unit_is_dealt_to_one_worker():
+    for m, np_, kp, g in SHAPES:
+        c = cut(m, np_, kp, g)
+        assert c.units_per_tile * c.unit_k >= kp > (c.units_per_tile - 1) * c.unit_k and c.row_tiles * c.rows_per_tile >= m
+        assert c.tiles == c.row_tiles * -(-np_ // (256 if c.pair else 128))
+        assert 1 <= c.workers <= 148 // (2 if c.pair else 1) and _first(c, 0) == 0 and _first(c, c.workers) == c.tiles * c.units_per_tile
+        assert c.base >= 1   # nobody goes without: the roles of a worker without units would wait for each other
+
+
+def test_small_weights_are_cut_at_the_ends_of_tiles():
+    """Fewer than four units of 256 k for each SM, and up to 16 in a tile: a worker's units are all of one tile"""
+    met = 0
+    for m, np_, kp, g in SHAPES:
+        c = cut(m, np_, kp, g)
+        sms = 148 // (2 if c.pair else 1)
+        if c.unit_k != 256 or c.units_per_tile > 16 or c.tiles > sms or c.tiles * c.units_per_tile >= 4 * sms:
+            continue
+        ku, met = c.units_per_tile, met + 1
+        assert all(_first(c, i) // ku == (_first(c, i + 1) - 1) // ku for i in range(c.workers)), (m, np_, kp, g)
+    assert met > 400

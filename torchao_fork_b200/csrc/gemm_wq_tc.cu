@@ -25,7 +25,7 @@
 // at NT = 256 would need 64 B/clk of shared-memory writes and as much in reads for B alone, of 128 B/clk.)
 //
 // Work split: units of (row block, row tile of x, 128 k; up to 128 rows 256 k), tile-major, dealt out contiguously and evenly to as many CTAs (or
-// pairs) as there are SMs.  A tile whose K is shared between neighbours is summed by the one that arrives last, in CTA order
+// pairs) as there are SMs (small weights: tile by tile, wq_owners).  A tile whose K is shared between neighbours is summed by the one that arrives last, in CTA order
 // (fp32 partial sums and tickets in the workspace; nobody waits for another CTA), so there is no last wave that is nearly
 // empty and few row blocks still fill the chip.
 //
@@ -970,6 +970,25 @@ struct WqPlan {
 
 static int kw_of(const WqPlan& w) { return !w.direct && w.NT <= kWqLongNT ? 2 : 1; }
 
+// Small weights, up to 128 rows: where an even deal leaves a worker fewer than four units of 256 k, tiles are not cut where it happens to fall, but each
+// goes to so many owners, with equally many of its units each.  The number of owners per tile; 0: dealt evenly.  In units, a worker that holds pieces of
+// two tiles pays about 13 beside its own (two drains, two shares out, tickets, and the tile that it finishes); owners of one tile 5, and the adding up of a share
+// of NT rows for each of them; one owner nothing.  (One unit takes an owner as long as two, which go to its two sets of dequant warps.)  us, units of 128 k
+// evenly / of 256 k evenly / as here: int4, 17 rows, 4096 x 256 6.0 / 7.2 / 5.8, x 768 9.4 / 13.1 / 7.0, x 1280 11.4 / 13.8 / 8.0, x 2816 13.4 / 15.0 / 11.2, x 4096
+// 14.7 / 13.5 / 11.6, 14336 x 1024 12.9 / 12.2 / 8.2, 128 rows, 4096 x 256 9.0 / 11.8 / 9.0, 8192 x 768 16.4 / 18.6 / 10.9, x 2304 20.4 / 20.2 / 15.9, 4096 x 4096
+// 23.2 / 21.7 / 18.3; int8, 17 rows, 1024 x 768 9.7 / 14.2 / 7.2, 4096 x 2304 13.7 / 14.9 / 11.8; 8 rows with a residual, int4 4096 x 768 8.9 / 10.2 / 5.7.  Not as
+// good as units of 128 k: 1024 x 2304, 17 rows 10.2 / 11.9 / 10.4, int8 10.4 / 12.9 / 10.8, x 2816 11.0 / 13.7 / 11.3.
+static int wq_owners(const WqPlan& w, int sms) {
+  if (w.KW != 2 || w.tiles > sms || w.tiles * w.KU >= 4 * (int64_t)sms) return 0;
+  int64_t best = 160 * ((w.tiles * w.KU + sms - 1) / sms + 13);   // in 160ths of a unit
+  int owners = 0;
+  for (int s = 1; s <= w.KU && w.tiles * s <= sms; ++s) {
+    const int64_t cost = s == 1 ? 160 * w.KU : 160 * (w.KU / s > 2 ? w.KU / s : 2) + 800 + s * (w.NT > 32 ? w.NT : 32);
+    if (w.KU % s == 0 && cost < best) best = cost, owners = s;
+  }
+  return owners;
+}
+
 static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
   if (M <= 0 || Np % 128 != 0 || Kp % 64 != 0 || M > ((int64_t)1 << 24)) return false;
   w.defer = int4 && M <= 16;
@@ -990,16 +1009,22 @@ static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
   if (w.tiles * w.KU > 2000000000) return false;
   const int sms = wq_sm_count() / w.ranks;
   w.quantum = w.tiles >= (int64_t)kWqMaxSplitTiles * sms ? w.KU : 1;
-  const int64_t parts = w.tiles * w.KU / w.quantum;
+  int64_t parts = w.tiles * w.KU / w.quantum;
   w.workers = (int)(w.quantum > 1 ? sms : (parts / 2 < sms ? (parts + 1) / 2 : sms));
+  const bool shared = w.quantum == 1;
+  if (const int owners = wq_owners(w, sms)) {
+    if (owners == 1) w.quantum = w.KU;
+    parts = w.tiles * w.KU / w.quantum;
+    w.workers = (int)w.tiles * owners;
+  }
   w.base = (int)(parts / w.workers);
   w.rem = (int)(parts % w.workers);
-  w.n_tickets = w.quantum > 1 ? 0 : w.tiles * w.ranks;
+  w.n_tickets = shared ? w.tiles * w.ranks : 0;
   w.x_sub = (uint32_t)w.BR * 256 + (w.defer ? 4 * 64 : 0);  // (the sums' space is that of the smallest group)
   w.x_bytes = w.KW * w.x_sub;
   auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
   w.off_part = up(w.n_tickets * 4);
-  w.off_xt = w.off_part + (w.quantum > 1 ? 0 : up((int64_t)w.workers * 2 * w.ranks * w.NT * 512));
+  w.off_xt = w.off_part + (!shared ? 0 : up((int64_t)w.workers * 2 * w.ranks * w.NT * 512));
   w.bytes = w.off_xt + up((int64_t)w.MT * w.ranks * w.KU * w.x_bytes);  // (DIRECT too: a workspace for many rows does for fewer)
   return true;
 }
