@@ -176,7 +176,8 @@ def test_packed_words_of_many_weights_equal_the_plain_result(gs, seed):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("shape,gs,spread", [((4096, 4096), 64, 0.05), ((1024, 4096), 32, 0.05), ((1024, 4096), 128, 1.0), ((1024, 4096), 256, 0.02)])
+@pytest.mark.parametrize("shape,gs,spread", [((4096, 4096), 64, 0.05), ((1024, 4096), 32, 0.05), ((1024, 4096), 128, 1.0), ((1024, 4096), 256, 0.02),
+                                             ((2900, 4096), 32, 30.0), ((2900, 4096), 256, 1.0)])   # (the last two: dealt in pieces, several to a block)
 def test_zero_points_of_the_search_equal_those_of_the_steps_in_32_bits(shape, gs, spread):
     """ao_b200_hqq_search against init / solve, the fp32 zero points as they are left in the workspace ([means 64 x 8 bytes][errors 10 x 8 bytes per
     8192 weights][scale][zero points of the last ten iterations]), bit for bit: a product and a sum rounded as one would show in their last bits."""

@@ -145,12 +145,12 @@ __global__ void __launch_bounds__(kHqqWarps * 32) hqq_finalize_kernel(const __nv
 // What keeps the iterations few: a group whose zero point comes out as it went in, bit for bit, while no |d| of it can pass the smallest threshold still
 // to come, gives the same zero point and error in every iteration that follows, so it is at rest and its lanes take the next group.  A zero point
 // moves by the mean rounding error and settles as soon as no weight crosses a rounding boundary on the way: of normal weights in groups of 32 / 64 / 128 / 256
-// 2.4 / 3.4 / 4.8 / 6.7 iterations of 20 move it, and one more shows it.  (Groups that never rest, as with weights of spread 3, where powf decides: 1361 -> 1549 us.)
-// The search over 4096 x 4096, groups of 64, 20 iterations, in all its kernels: 199 us with all iterations of all groups, 105 without those at rest
-// (groups of 32 / 128 / 256: 212 / 227 / 186 -> 113 / 120 / 129).  Taken back: groups put together anew among a block's warps after each iteration (155),
+// 2.4 / 3.4 / 4.8 / 6.7 iterations of 20 move it, and one more shows it.  (Groups that never rest, as with weights of spread 3, where powf decides: hqq_deal_kernel.)
+// The search over 4096 x 4096, groups of 64, 20 iterations, in all its kernels: 199 us with all iterations of all groups, 109 without those at rest
+// (groups of 32 / 128 / 256: 213 / 226 / 186 -> 120 / 127 / 135).  Taken back: groups put together anew among a block's warps after each iteration (155),
 // rounds of two and three iterations over a block's list (141).
 constexpr int kHqqChunk = 10;   // iterations per launch: bounds hist to 10 numbers per group
-constexpr int kHqqMaxIters = 64;
+constexpr int kHqqMaxIters = 64, kHqqLaunches = (kHqqMaxIters + kHqqChunk - 1) / kHqqChunk;
 constexpr int kHqqPer = 32;     // weights per thread
 constexpr int kHqqThreads = 256, kHqqBlocks = 4;   // per block; per SM: 64 registers (with all iterations of all groups 207 us, 3 blocks of 80 220; 16 weights per thread and 4 blocks 228)
 constexpr int kHqqShare = 512;  // groups of a block at a time, at most; a multiple of 8
@@ -200,12 +200,50 @@ __device__ __forceinline__ void hqq_tree(int i, Leaf&& leaf, F2& acc, float2& e)
   }
 }
 
+// How the launches deal out the groups: in equal contiguous shares, as long as most groups can come to rest (a block's lanes then go on without a gap), else in
+// pieces of what a block holds at once, to whoever is through with the last one.
+struct HqqDeal {
+  int fine, next[kHqqLaunches];  // pieces; the next one of each launch
+};
+__host__ __device__ __forceinline__ int hqq_piece(int group_size) { return 8192 / group_size; }   // groups of 256 threads (and of what an error is kept of)
+// what the group's smallest and largest weight say about all of it: how far |d| can go (half a step, or what the clamp cuts off; the margins are a hundred times
+// the roundings of t + z and of the quotient).  t_lo, t_hi: both times the scale
+__device__ __forceinline__ float hqq_bound(float t_lo, float t_hi, float z, float recip) {
+  const float q_lo = __fadd_rn(t_lo, z), q_hi = __fadd_rn(t_hi, z);
+  return (fmaxf(0.51f, fmaxf(-q_lo, q_hi - 15.f)) + (fabsf(z) + 16.f) * 1e-6f) * recip;
+}
+
+// Pieces, where more than one in 16 of a sample of groups, as they are at first, has a |d| that may pass the smallest threshold: those never rest, and in shares
+// blocks end with few of their warps at work, and rows cost differently.  4096 x 4096, groups of 64, us, in launches of a block per piece without rest / in shares /
+// in pieces: normal weights (rows of e^(0.3 normal) times) the spread 3 1362 / 1546 / 1340, 1 1035 / 1290 / 1085, 0.8 753 / 919 / 775, 0.6 468 / 524 /
+// 462, 0.4 320 / 279 / 310, 0.02 198 / 109 / 128.
+// One launch of one block; 8 threads per group, 128 groups.
+__global__ void __launch_bounds__(1024) hqq_deal_kernel(const __nv_bfloat16* __restrict__ w, int64_t n_groups, int G, float least, HqqDeal* __restrict__ deal) {
+  const int64_t step = (n_groups + 127) / 128, group = (threadIdx.x >> 3) * step;
+  float mn = INFINITY, mx = -INFINITY;
+  if (group < n_groups) {
+    for (int i = threadIdx.x & 7; i < G / 8; i += 8) {
+      float f[8];
+      unpack8(ldg128(reinterpret_cast<const unsigned short*>(w) + group * G + 8 * i), f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) mn = fminf(mn, f[j]), mx = fmaxf(mx, f[j]);
+    }
+  }
+#pragma unroll
+  for (int o = 4; o; o >>= 1) mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o)), mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  const float s = fminf(__fdiv_rn(15.f, __fsub_rn(mx, mn)), 2e4f), z = rintf(__fmul_rn(-mn, s));
+  const bool never = !(hqq_bound(__fmul_rn(mn, s), __fmul_rn(mx, s), z, __frcp_rn(s)) <= 0.999f * least);
+  const int count = __syncthreads_count(group < n_groups && never), all = __syncthreads_count(group < n_groups);
+  if (threadIdx.x == 0) deal->fine = 16 * count > all;
+  if (threadIdx.x < kHqqLaunches) deal->next[threadIdx.x] = 0;
+}
+
 // A block takes contiguous groups, at most kHqqShare at a time; L lanes of a warp take one group, two iterations, and then the next one if theirs is over, each
 // at its own count.  rest: per group, the error of a group that has come to rest, else -1 (written by a launch for the next).
 template <int G>
-__global__ void __launch_bounds__(kHqqThreads, kHqqBlocks) hqq_iterate_kernel(const __nv_bfloat16* __restrict__ w, int64_t n_groups, HqqChunk ch, int share,
+__global__ void __launch_bounds__(kHqqThreads, kHqqBlocks) hqq_iterate_kernel(const __nv_bfloat16* __restrict__ w, int64_t n_groups, HqqChunk ch, int share, int64_t n_err,
                                                                               float* __restrict__ scale, float* __restrict__ hist, double* __restrict__ err,
-                                                                              const double* __restrict__ mean, float* __restrict__ rest) {
+                                                                              const double* __restrict__ mean, float* __restrict__ rest, HqqDeal* __restrict__ deal) {
   constexpr int L = G / kHqqPer, I = 32 / L, J = G / 32;   // threads per group; its lanes per thread; elements per lane
   constexpr float kMagic = 12582912.f;                     // 1.5 * 2^23: adding and subtracting it is rint up to 2^22, and beyond that the clamp decides
   constexpr int kAtRest = 256;
@@ -213,17 +251,23 @@ __global__ void __launch_bounds__(kHqqThreads, kHqqBlocks) hqq_iterate_kernel(co
   __shared__ short s_done[kHqqShare];                      // iterations whose results are there; + kAtRest: the others are as the last one
   __shared__ short s_todo[kHqqShare];
   __shared__ int s_n, s_next;                              // how many; the next ones to be fetched
-  __shared__ double s_total[kHqqChunk];
+  __shared__ int s_piece;
   bool stopped = false;
   if (ch.first > 0) hqq_last(mean, ch.first, stopped);
   if (stopped) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane % L;
-  if (threadIdx.x < kHqqChunk) s_total[threadIdx.x] = 0.0, s_threshold[threadIdx.x] = ch.threshold[threadIdx.x], s_inv_beta[threadIdx.x] = ch.inv_beta[threadIdx.x];
+  if (threadIdx.x < kHqqChunk) s_threshold[threadIdx.x] = ch.threshold[threadIdx.x], s_inv_beta[threadIdx.x] = ch.inv_beta[threadIdx.x];
 #pragma unroll 1
-  for (int64_t base = (int64_t)blockIdx.x * share; base < n_groups; base += (int64_t)gridDim.x * share) {
-    const int here = (int)(n_groups - base < share ? n_groups - base : share);
-    if (threadIdx.x == 0) s_n = s_next = 0;
+  for (int64_t turn = blockIdx.x;; turn += gridDim.x) {
+    const bool fine = deal->fine != 0;
+    if (threadIdx.x == 0) {
+      s_n = s_next = 0;
+      if (fine) s_piece = atomicAdd(&deal->next[ch.first / kHqqChunk], 1);
+    }
     __syncthreads();
+    const int64_t piece = fine ? s_piece : turn, base = piece * (fine ? hqq_piece(G) : share);
+    if (base >= n_groups) break;
+    const int most = fine ? hqq_piece(G) : share, here = (int)(n_groups - base < most ? n_groups - base : most);
 #pragma unroll 1
     for (int g0 = warp * 32; g0 < here; g0 += kHqqThreads) {
       const int g = g0 + lane;
@@ -318,10 +362,8 @@ __global__ void __launch_bounds__(kHqqThreads, kHqqBlocks) hqq_iterate_kernel(co
         for (int k = 0; k < kHqqPer / 2; ++k) asm volatile("" : "+r"(v[k]));
         const float thr = s_threshold[it];
         const F2 z2 = f2(z, z), nz2 = f2(-z, -z);
-        // what the group's smallest and largest weight say about all of it: no weight is clamped, and no |d| is above the threshold
-        // (|d| is half a step, or what the clamp cuts off; the margins are a hundred times the roundings of t + z and of the quotient)
-        const float q_lo = __fadd_rn(t_lo, z), q_hi = __fadd_rn(t_hi, z);
-        const float bound = (fmaxf(0.51f, fmaxf(-q_lo, q_hi - 15.f)) + (fabsf(z) + 16.f) * 1e-6f) * -nr;
+        // no weight of the group is clamped, and no |d| is above the threshold
+        const float q_lo = __fadd_rn(t_lo, z), q_hi = __fadd_rn(t_hi, z), bound = hqq_bound(t_lo, t_hi, z, -nr);
         const bool inside = __all_sync(0xffffffffu, !moves || (q_lo >= -0.5f && q_hi < 15.5f));
         const bool small = __all_sync(0xffffffffu, !moves || bound <= 0.999f * thr);
         auto quotients = [&](F2 f, bool clamp, F2& wq, F2& nt) {   // W_q, -W * scale and d = W - W_r of a pair
@@ -424,20 +466,22 @@ __global__ void __launch_bounds__(kHqqThreads, kHqqBlocks) hqq_iterate_kernel(co
       }
 #pragma unroll
       for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      if (lane == 0) s_total[it] += sum;
+      if (lane == 0) err[(int64_t)it * n_err + piece] = sum;
     }
     __syncthreads();
   }
-  if (threadIdx.x < ch.count) err[(int64_t)threadIdx.x * gridDim.x + blockIdx.x] = s_total[threadIdx.x];
 }
 
 // block i: mean[first + i] = sum of err[i][..] / numel, in double, fixed order
-__global__ void __launch_bounds__(1024) hqq_mean_kernel(const double* __restrict__ err, int64_t n_blocks, double inv_numel, int first, double* __restrict__ mean) {
+__global__ void __launch_bounds__(1024) hqq_mean_kernel(const double* __restrict__ err, int64_t n_err, int64_t n_groups, int share, int piece, double inv_numel, int first,
+                                                        double* __restrict__ mean, const HqqDeal* __restrict__ deal) {
   __shared__ double s_sum[1024];
   bool stopped = false;
   if (first > 0) hqq_last(mean, first, stopped);
   if (stopped) return;
-  const double* e = err + blockIdx.x * n_blocks;
+  const int most = deal->fine ? piece : share;
+  const int64_t n_blocks = (n_groups + most - 1) / most;
+  const double* e = err + blockIdx.x * n_err;
   double t = 0.0;
   for (int64_t i = threadIdx.x; i < n_blocks; i += 1024) t += e[i];
   s_sum[threadIdx.x] = t;
@@ -650,10 +694,10 @@ extern "C" int ao_b200_hqq_finalize(const void* w, int64_t n_groups, int group_s
 
 static int64_t hqq_search_blocks(int64_t n_groups, int group_size) { return (n_groups * group_size + 8191) / 8192; }
 
-// [mean double x kHqqMaxIters][err double kHqqChunk x blocks][scale][hist kHqqChunk x n_groups][rest]
+// [mean double x kHqqMaxIters][err double kHqqChunk x blocks][scale][hist kHqqChunk x n_groups][rest][deal]
 extern "C" int64_t ao_b200_hqq_search_workspace_bytes(int64_t n_groups, int group_size) {
   if (n_groups <= 0 || group_size < kHqqPer) return 0;
-  return (kHqqMaxIters + kHqqChunk * hqq_search_blocks(n_groups, group_size)) * 8 + (2 + kHqqChunk) * n_groups * 4;
+  return (kHqqMaxIters + kHqqChunk * hqq_search_blocks(n_groups, group_size)) * 8 + (2 + kHqqChunk) * n_groups * 4 + (int64_t)sizeof(HqqDeal);
 }
 
 extern "C" int ao_b200_hqq_search(const void* w, int64_t N, int64_t K, int group_size, double beta, double kappa, double lp_norm, int iters,
@@ -675,10 +719,11 @@ extern "C" int ao_b200_hqq_search(const void* w, int64_t N, int64_t K, int group
   float* scale = reinterpret_cast<float*>(err + kHqqChunk * blocks);
   float* hist = scale + n_groups;
   float* rest = hist + kHqqChunk * n_groups;
-  // as many blocks as the chip holds at once; their groups in equal shares, as many times as it takes
+  HqqDeal* deal = reinterpret_cast<HqqDeal*>(rest + n_groups);
+  // as many blocks as the chip holds at once; their groups in equal shares, as many times as it takes (hqq_iterate_kernel: or in pieces)
   const int64_t most = (int64_t)kHqqBlocks * kNumSMs, rounds = (n_groups + most * kHqqShare - 1) / (most * kHqqShare);
   int share = (int)((n_groups + rounds * most * 8 - 1) / (rounds * most * 8) * 8);
-  if (share < 8192 / group_size) share = 8192 / group_size;   // (a block's worth of threads, and what `blocks` counts)
+  if (share < hqq_piece(group_size)) share = hqq_piece(group_size);   // (a block's worth of threads, and what `blocks` counts)
   const unsigned grid = (unsigned)((n_groups + share - 1) / share < most ? (n_groups + share - 1) / share : most);
   float inv_beta[kHqqMaxIters], threshold[kHqqMaxIters];
   for (int i = 0; i < iters; ++i) {
@@ -693,14 +738,15 @@ extern "C" int ao_b200_hqq_search(const void* w, int64_t N, int64_t K, int group
     ch.lp_m1 = (float)(lp_norm - 1.0);
     ch.least = threshold[first];
     for (int i = first; i < iters; ++i) ch.least = threshold[i] < ch.least ? threshold[i] : ch.least;
+    if (first == 0) hqq_deal_kernel<<<1, 1024, 0, s>>>(wb, n_groups, group_size, ch.least, deal);
     for (int i = 0; i < ch.count; ++i) ch.inv_beta[i] = inv_beta[first + i], ch.threshold[i] = threshold[first + i];
     switch (group_size) {
-      case 32: hqq_iterate_kernel<32><<<grid, kHqqThreads, 0, s>>>(wb, n_groups, ch, share, scale, hist, err, mean, rest); break;
-      case 64: hqq_iterate_kernel<64><<<grid, kHqqThreads, 0, s>>>(wb, n_groups, ch, share, scale, hist, err, mean, rest); break;
-      case 128: hqq_iterate_kernel<128><<<grid, kHqqThreads, 0, s>>>(wb, n_groups, ch, share, scale, hist, err, mean, rest); break;
-      default: hqq_iterate_kernel<256><<<grid, kHqqThreads, 0, s>>>(wb, n_groups, ch, share, scale, hist, err, mean, rest); break;
+      case 32: hqq_iterate_kernel<32><<<grid, kHqqThreads, 0, s>>>(wb, n_groups, ch, share, blocks, scale, hist, err, mean, rest, deal); break;
+      case 64: hqq_iterate_kernel<64><<<grid, kHqqThreads, 0, s>>>(wb, n_groups, ch, share, blocks, scale, hist, err, mean, rest, deal); break;
+      case 128: hqq_iterate_kernel<128><<<grid, kHqqThreads, 0, s>>>(wb, n_groups, ch, share, blocks, scale, hist, err, mean, rest, deal); break;
+      default: hqq_iterate_kernel<256><<<grid, kHqqThreads, 0, s>>>(wb, n_groups, ch, share, blocks, scale, hist, err, mean, rest, deal); break;
     }
-    hqq_mean_kernel<<<ch.count, 1024, 0, s>>>(err, (int64_t)grid, 1.0 / ((double)n_groups * (double)group_size), first, mean);
+    hqq_mean_kernel<<<ch.count, 1024, 0, s>>>(err, blocks, n_groups, share, hqq_piece(group_size), 1.0 / ((double)n_groups * (double)group_size), first, mean, deal);
   }
   if (packed) {
     const int64_t tiles = (Np / 16) * (Kp / 64), want = (tiles + 7) / 8;
