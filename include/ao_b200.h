@@ -63,7 +63,8 @@ enum {
 };
 
 AO_B200_API const char* ao_b200_error_string(int code);
-AO_B200_API int ao_b200_abi_version(void);
+#define AO_B200_ABI_VERSION 5
+AO_B200_API int ao_b200_abi_version(void);   /* AO_B200_ABI_VERSION of the library */
 
 /* ---------------------------------------------------------------- int4: quantize ---- */
 

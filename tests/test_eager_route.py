@@ -219,3 +219,54 @@ def test_a_quantized_weight_is_a_parameter_like_any_other(recipe):
     if recipe == "int4":
         ao.quantize_(odd, config)
         assert type(odd.weight) is torch.nn.Parameter
+
+
+@pytest.mark.parametrize("what", ["missing", "garbage", "of another version", "older than its binding"])
+def test_a_host_module_that_does_not_load_counts_as_not_built(what, monkeypatch, tmp_path):
+    import os
+
+    from torchao_fork_b200 import _lib, build
+    if not os.path.exists(_lib.LIB_PATH) or not os.path.exists(build.host_path()):
+        pytest.skip("python -m torchao_fork_b200.build")
+    path = tmp_path / "ao_b200_host.so"
+    if what == "garbage":
+        path.write_bytes(b"\x7fELF" + b"\0" * 200)
+    elif what != "missing":
+        path = build.host_path()
+        monkeypatch.setattr(_lib, "lib", lambda real=_lib.lib(): _Like(real, 4 if what == "of another version" else "older"))
+    monkeypatch.setattr(build, "host_path", lambda: str(path))
+    with pytest.warns(RuntimeWarning, match="in Python"):
+        assert _lib.host() is None
+
+
+class _Like:
+    """The library, but for its version"""
+    def __init__(self, real, version):
+        self.real, self.ao_b200_abi_version = real, lambda: version
+
+    def __getattr__(self, name):
+        return getattr(self.real, name)
+
+
+def test_the_host_module_of_this_build_is_bound():
+    import os
+
+    from torchao_fork_b200 import _lib, build
+    if not os.path.exists(_lib.LIB_PATH) or not os.path.exists(build.host_path()):
+        pytest.skip("python -m torchao_fork_b200.build")
+    assert callable(_lib.host().int4_mm) and callable(_lib.host().int8_mm)
+
+
+def test_a_build_without_a_cpp_compiler_has_its_libraries(monkeypatch, capsys):
+    from torchao_fork_b200 import build
+    done = []
+
+    def host(verbose, force):
+        done.append("host")
+        raise FileNotFoundError("g++")
+    monkeypatch.setattr(build, "_build_locked", lambda verbose, force, target: done.append(target) or build.TARGETS[target][1])
+    monkeypatch.setattr(build, "_build_host", host)
+    assert build.build(target="all") == build.LIB and set(done) == {"lm", "core", "host"}
+    assert "not built" in capsys.readouterr().err
+    with pytest.raises(FileNotFoundError):     # asked for by name it has to be there
+        build.build(target="host")

@@ -137,20 +137,26 @@ def lib():
 
 
 def host():
-    """The native host side of the eager linears (csrc/host), bound to the loaded library; None where it has not been built for this torch and
-    this Python (the same steps then run in Python, before the same kernels)."""
+    """The native host side of the eager linears (csrc/host), bound to the loaded library; None, with a warning, where it has not been built for this
+    torch and this Python, does not load or is of another version than the library (the same steps then run in Python, before the same kernels)."""
     import importlib.machinery
     import importlib.util
+    import warnings
 
     from . import build as _build
-    path = _build.host_path()
-    if not os.path.exists(path):
+    path, names = _build.host_path(), ("ao_b200_int4_mm", "ao_b200_int4_mm_workspace_bytes", "ao_b200_int8_mm", "ao_b200_int8_mm_workspace_bytes")
+    functions = [ctypes.cast(getattr(lib(), n), ctypes.c_void_p).value for n in names]
+    try:
+        if not os.path.exists(path):
+            raise ImportError("not built")
+        loader = importlib.machinery.ExtensionFileLoader("ao_b200_host", path)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("ao_b200_host", loader, origin=path))
+        loader.exec_module(module)
+        module.bind(lib().ao_b200_abi_version(), *functions)
+    except (ImportError, OSError, AttributeError, TypeError) as e:   # (AttributeError, TypeError: a module that is older than this binding)
+        warnings.warn(f"{path}: {e}; eager linears take their host steps in Python, about 8 us a call more (python -m torchao_fork_b200.build host)",
+                      RuntimeWarning, stacklevel=2)
         return None
-    loader = importlib.machinery.ExtensionFileLoader("ao_b200_host", path)
-    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("ao_b200_host", loader, origin=path))
-    loader.exec_module(module)
-    names = ("ao_b200_int4_mm", "ao_b200_int4_mm_workspace_bytes", "ao_b200_int8_mm", "ao_b200_int8_mm_workspace_bytes")
-    module.bind(*(ctypes.cast(getattr(lib(), n), ctypes.c_void_p).value for n in names))
     return module
 
 

@@ -50,7 +50,7 @@ extern "C" const char* ao_b200_error_string(int code) {
   return "unknown error";
 }
 
-extern "C" int ao_b200_abi_version(void) { return 5; }
+extern "C" int ao_b200_abi_version(void) { return AO_B200_ABI_VERSION; }
 
 #include <cstdlib>
 namespace {

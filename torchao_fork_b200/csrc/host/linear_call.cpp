@@ -2,7 +2,8 @@
 // the call (no mode, tracer, transform, gradient or wrapper: runs_eagerly) and the launch -- checks, output, workspace, stream, device -- as native code.
 // Through Python and ctypes these take about 5 us more, of about 22 that a call of one row takes, while its kernel takes 5.  Everything that is not
 // plainly in order (shapes, types, strides, alignment, no rows) is left to the Python code, which mends or refuses it: the answer is then None.
-// An error code of the library comes back as an int.
+// An error code of the library comes back as an int.  The functions' types are those of the header that this module is built with, and a library of another
+// version is refused (bind).
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -11,14 +12,14 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include "../../../include/ao_b200.h"
+
 namespace {
 
-using Bytes = int64_t (*)(int64_t, int64_t, int64_t);
-using Int4Mm = int (*)(const void*, int64_t, int64_t, int64_t, const void*, const void*, int64_t, int64_t, int, void*, int64_t, int64_t, void*, int64_t, void*);
-using Int8Mm = int (*)(const void*, int64_t, int64_t, int64_t, const void*, const void*, int64_t, int64_t, void*, int64_t, int64_t, void*, int64_t, void*);
-Bytes int4_bytes, int8_bytes;
-Int4Mm int4_mm_fn;
-Int8Mm int8_mm_fn;
+decltype(&ao_b200_int4_mm_workspace_bytes) int4_bytes;
+decltype(&ao_b200_int8_mm_workspace_bytes) int8_bytes;
+decltype(&ao_b200_int4_mm) int4_mm_fn;
+decltype(&ao_b200_int8_mm) int8_mm_fn;
 
 // rows as the kernels read them: bf16 [m][k], whole 16-byte pieces
 bool rows_ok(const at::Tensor& x) {
@@ -101,14 +102,16 @@ PyObject* int8_mm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// the library's functions by their addresses: int4_mm, its workspace_bytes, int8_mm, its workspace_bytes
+// the library's version, and its functions by their addresses: int4_mm, its workspace_bytes, int8_mm, its workspace_bytes
 PyObject* bind(PyObject*, PyObject* args) {
   unsigned long long f[4];
-  if (!PyArg_ParseTuple(args, "KKKK", f, f + 1, f + 2, f + 3)) return nullptr;
-  int4_mm_fn = reinterpret_cast<Int4Mm>(f[0]);
-  int4_bytes = reinterpret_cast<Bytes>(f[1]);
-  int8_mm_fn = reinterpret_cast<Int8Mm>(f[2]);
-  int8_bytes = reinterpret_cast<Bytes>(f[3]);
+  int version;
+  if (!PyArg_ParseTuple(args, "iKKKK", &version, f, f + 1, f + 2, f + 3)) return nullptr;
+  if (version != AO_B200_ABI_VERSION) return PyErr_Format(PyExc_ImportError, "built for version %d of the library, which is %d", AO_B200_ABI_VERSION, version);
+  int4_mm_fn = reinterpret_cast<decltype(int4_mm_fn)>(f[0]);
+  int4_bytes = reinterpret_cast<decltype(int4_bytes)>(f[1]);
+  int8_mm_fn = reinterpret_cast<decltype(int8_mm_fn)>(f[2]);
+  int8_bytes = reinterpret_cast<decltype(int8_bytes)>(f[3]);
   Py_RETURN_NONE;
 }
 
