@@ -83,9 +83,11 @@ __global__ void __launch_bounds__(kThreads) rmsnorm_kernel(const __nv_bfloat16* 
 }
 
 // The same for rows of up to 8 kThreads N columns, which a thread keeps as the N 16-byte pieces that they come in: same sums in the same order, same
-// bits.  700 rows of 4096: the rows' way through shared memory (as fp32, eight ways on a bank) took 5.3 us, without it 4.3.  What is behind
+// bits.  700 rows of 4096: the rows' way through shared memory (as fp32, eight ways on a bank) took 5.3 us, without it 4.3.  With a residual all loads of
+// both rows have to be out before the first sum, and the weights wait in the residual's registers: 4096 rows of 4096 / 8192 / 16384 25.5 / 46.4 / 95.2 us through
+// shared memory, 26.2 / 50.6 / 114.5 with the residual fetched piece by piece, 22.9 / 42.8 / 82.3 so.  What is behind
 // may start when it likes: a kernel that follows programmatically waits before it reads.
-template <int kThreads, int N>
+template <int kThreads, int N, bool RES>
 __global__ void __launch_bounds__(kThreads) rmsnorm_pieces_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
                                                                   const __nv_bfloat16* __restrict__ weight, __nv_bfloat16* __restrict__ h_out,
                                                                   __nv_bfloat16* __restrict__ y, int dim, float eps) {
@@ -93,12 +95,12 @@ __global__ void __launch_bounds__(kThreads) rmsnorm_pieces_kernel(const __nv_bfl
   grid_dependency_wait();
   grid_launch_dependents();
   const int64_t at = (int64_t)blockIdx.x * dim;
-  uint4 v[N], wv[N];
+  uint4 v[N], wv[N];               // (wv: the residual's pieces first, RES)
   float ss = 0.f;
 #pragma unroll
   for (int n = 0; n < N; ++n) {
     const int i = (threadIdx.x + n * kThreads) * 8;
-    if (i < dim) v[n] = *reinterpret_cast<const uint4*>(x + at + i), wv[n] = __ldg(reinterpret_cast<const uint4*>(weight + i));
+    if (i < dim) v[n] = *reinterpret_cast<const uint4*>(x + at + i), wv[n] = *reinterpret_cast<const uint4*>(RES ? residual + at + i : weight + i);
   }
 #pragma unroll
   for (int n = 0; n < N; ++n) {
@@ -106,9 +108,9 @@ __global__ void __launch_bounds__(kThreads) rmsnorm_pieces_kernel(const __nv_bfl
     if (i >= dim) continue;
     float f[8];
     unpack8(v[n], f);
-    if (residual != nullptr) {
+    if constexpr (RES) {
       float r[8];
-      unpack8(*reinterpret_cast<const uint4*>(residual + at + i), r);
+      unpack8(wv[n], r);
 #pragma unroll
       for (int e = 0; e < 8; ++e) f[e] = bf16r(f[e] + r[e]);
       uint32_t o[4];
@@ -116,6 +118,7 @@ __global__ void __launch_bounds__(kThreads) rmsnorm_pieces_kernel(const __nv_bfl
       for (int e = 0; e < 4; ++e) o[e] = float_to_bf16_bits(f[2 * e]) | (float_to_bf16_bits(f[2 * e + 1]) << 16);
       v[n] = make_uint4(o[0], o[1], o[2], o[3]);
       if (h_out) *reinterpret_cast<uint4*>(h_out + at + i) = v[n];
+      wv[n] = *reinterpret_cast<const uint4*>(weight + i);
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
@@ -508,9 +511,9 @@ extern "C" int ao_b200_rmsnorm(const void* x, const void* residual, const void* 
         static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(residual), static_cast<const __nv_bfloat16*>(weight),
         static_cast<__nv_bfloat16*>(h_out), static_cast<__nv_bfloat16*>(y), (int)dim, eps);
   };
-  if (dim <= 512 * 8) return pieces(rmsnorm_pieces_kernel<512, 1>);
-  if (dim <= 512 * 16) return pieces(rmsnorm_pieces_kernel<512, 2>);
-  if (dim <= 512 * 32) return pieces(rmsnorm_pieces_kernel<512, 4>);
+  if (dim <= 512 * 8) return residual ? pieces(rmsnorm_pieces_kernel<512, 1, true>) : pieces(rmsnorm_pieces_kernel<512, 1, false>);
+  if (dim <= 512 * 16) return residual ? pieces(rmsnorm_pieces_kernel<512, 2, true>) : pieces(rmsnorm_pieces_kernel<512, 2, false>);
+  if (dim <= 512 * 32) return residual ? pieces(rmsnorm_pieces_kernel<512, 4, true>) : pieces(rmsnorm_pieces_kernel<512, 4, false>);
   const size_t smem = dim * sizeof(float);
   static bool attr_set = false;
   if (!attr_set && smem > 48 * 1024) {
