@@ -322,7 +322,7 @@ def _plans():
     seen = {}
     for group in (0, 32, 64, 128, 256):
         for m in list(range(1, 1030)) + [2048, 4096]:
-            for np_ in (16384, 8192):   # above 8192 outputs activations are staged, up to there read in place from 512 rows on
+            for np_ in (16384, 8192, 4096, 2048):   # above 8192 outputs activations are staged; from 512 rows on they are read in place up to 2048, 4096 or 8192
                 c = plan(m, group, np_)
                 seen.setdefault(tuple(sorted(c.items())), (m, group, c))
     return list(seen.values())
@@ -402,3 +402,11 @@ def test_small_weights_are_cut_at_the_ends_of_tiles():
         ku, met = c.units_per_tile, met + 1
         assert all(_first(c, i) // ku == (_first(c, i + 1) - 1) // ku for i in range(c.workers)), (m, np_, kp, g)
     assert met > 400
+
+
+@pytest.mark.parametrize("group,np_,tiles", [(0, 2048, (176, 208, 224, 240, 256)), (0, 2176, (224, 240, 256)), (0, 4096, (224, 240, 256)), (0, 4224, (240, 256)),
+                                             (0, 8192, (240, 256)), (128, 4096, (176, 208, 224, 240, 256)), (128, 8192, (208, 224, 240, 256)), (128, 8320, ())])
+def test_activations_are_read_in_place_where_the_products_of_a_tile_cover_the_turn(group, np_, tiles):
+    for m in (511, 513, 528, 600, 640, 700, 768, 800, 1000, 1040, 2048):
+        c = cut(m, np_, 4096, group)
+        assert bool(c.in_place) == (m >= 512 and c.rows_per_tile in tiles), m

@@ -64,7 +64,7 @@ constexpr int kWqSlots = 4;                    // ring of A in tensor memory: 64
 constexpr int kWqMaxW = 16, kWqMaxX = 8;       // rings of weights and of tiles of x
 constexpr int kWqPitch = 128 * 2 + 16;         // bytes of a row of the output tile in shared memory (rows land on distinct banks)
 constexpr int kWqHeader = 1024;                // mbarriers, TMEM base, give-up flag
-constexpr int kWqDirectRows = 512, kWqDirectN = 8192;  // from and up to which the GEMM reads the activations where they are (wq_plan)
+constexpr int kWqDirectRows = 512, kWqDirectN = 8192;  // from and up to which, at most, the GEMM reads the activations where they are (wq_plan)
 constexpr int kWqLongNT = 128;                 // rows of a tile up to which a unit has 256 k (both sides: above)
 constexpr int kWqMaxSplitTiles = 16;           // tiles per worker from which whole tiles are dealt out (imbalance <= 1/16)
 
@@ -993,14 +993,17 @@ static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
   if (M <= 0 || Np % 128 != 0 || Kp % 64 != 0 || M > ((int64_t)1 << 24)) return false;
   w.defer = int4 && M <= 16;
   w.pair = M > 32;
-  // Staging takes time by M x K, reading in place (the weights turned round among the lanes) by the units, M x K x N.  Staged / in place, us: int8
-  // 4096 x 14336, 1000 rows 102.4 / 97.5, 700 rows 74.8 / 72.1; int4 4096 x 14336, 700 / 1000 rows 72.0 / 67.3, 97.8 / 92.4; 6144 x 4096 and 4096 x 4096, 700 rows
-  // 41.5 / 39.2, 34.9 / 33.4; int8 8192 x 8192, 2048 rows 217.5 / 215; but int4 14336 x 4096, 700 and 2048 rows 65.2 / 65.6, 166.4 / 166.3; 300 rows of 4096 x 14336
-  // 40.6 / 42.7, 64 rows of 28672 x 8192 51.4 / 58.8, where the lanes' turn lengthens the way from a unit's weights to its product
-  w.direct = M >= kWqDirectRows && Np <= kWqDirectN;
   w.ranks = w.pair ? 2 : 1;
   w.MT = (int)((M + 255) / 256);
   w.NT = (int)(((M + w.MT - 1) / w.MT + 15) / 16 * 16);
+  // Staging takes time by M x K, reading in place (the weights turned round among the lanes) by the units, M x K x N.  Staged / in place, us: int8
+  // 4096 x 14336, 1000 rows 102.4 / 97.5, 700 rows 74.8 / 72.1; int4 4096 x 14336, 700 / 1000 rows 72.0 / 67.3, 97.8 / 92.4; 6144 x 4096 and 4096 x 4096, 700 rows
+  // 41.5 / 39.2, 34.9 / 33.4; int8 8192 x 8192, 2048 rows 217.5 / 215; but int4 14336 x 4096, 700 and 2048 rows 65.2 / 65.6, 166.4 / 166.3; 300 rows of 4096 x 14336
+  // 40.6 / 42.7, 64 rows of 28672 x 8192 51.4 / 58.8, where the lanes' turn lengthens the way from a unit's weights to its product.  So it is with tiles of
+  // fewer rows, whose products no longer cover the turn: int8 8192 x 8192, 528 / 600 rows (tiles of 176 / 208) 58.2 / 64.3, 66.5 / 70.5, 640 (224) 69.6 / 72.4, 700 (240)
+  // 76.7 / 76.9, 4096 x 4096, 800 (208) 1.02 times, 640 (224) 0.98, 2048 x 8192, 528 0.99; int4 8192 x 8192, 528 1.03, 560 (192) 1.01, 4096 x 14336, 528 0.99
+  const int64_t most = int4 ? (w.NT < 192 ? kWqDirectN / 2 : kWqDirectN) : (w.NT < 224 ? kWqDirectN / 4 : (w.NT < 240 ? kWqDirectN / 2 : kWqDirectN));
+  w.direct = M >= kWqDirectRows && Np <= most;
   w.BR = w.NT / w.ranks;
   w.KW = kw_of(w);
   w.KU = (int)((Kp + 128 * w.KW - 1) / (128 * w.KW));
