@@ -407,3 +407,9 @@ def test_few_rows_on_both_sides_of_their_lines(bits, m, n, k):
 def test_small_weights(bits, group, m, n, k):
     # tiles of one owner, of a few, and of as many as they have units (the number: wq_owners)
     _check(bits, m, n, k, group)
+
+
+@pytest.mark.parametrize("group,m,n,k", [(128, 9, 18432, 4096), (128, 11, 18304, 4096), (64, 9, 24576, 4096), (64, 10, 24448, 4096), (32, 9, 20480, 4096), (32, 10, 20352, 4096),
+                                         (256, 12, 14336, 4096), (256, 12, 14464, 4096), (32, 3, 8192, 24576), (64, 8, 8192, 24576), (64, 3, 8192, 24576), (128, 3, 8192, 24576)])
+def test_few_rows_by_group_on_both_sides_of_their_lines(group, m, n, k):
+    _check(4, m, n, k, group)

@@ -91,23 +91,27 @@ int settled_follow() { return tunables().pdl ? ao::kFollowSettled : ao::kFollowP
 
 // Which calls of up to 16 rows take the GEMM (gemm_wq_tc.cu) rather than the GEMV that keeps the activations in shared memory.  The GEMM
 // costs about 10 us of staging, launch and tail whatever the size, then streams 16 rows as fast as 3; the GEMV has no such costs but takes twice the
-// products from 9 rows on.  Measured (GEMV / GEMM, us): int4 8 rows of 28672 x 8192 35.9 / 37.5, of 28672 x 4096 21.2 / 23.9; 9 rows of 14336 x 4096 18.4 / 17.5,
-// 8192 x 8192 20.1 / 18.8, 10240 x 8192 27.3 / 20.8, 28672 x 4096 27.8 / 24.0, but 6144 x 4096 12.7 / 14.1; 16 rows of 6144 x 4096 14.0 / 14.3; int8 9 rows of
-// 28672 x 4096 31.3 / 27.9, 10240 x 8192 26.1 / 26.6, 14336 x 4096 20.1 / 20.2, 16 rows of that 25.9 / 20.8, 9 and 16 of 6144 x 4096 13.1 / 14.9, 15.1 / 15.1.  Where
+// products from 9 rows on, and more with each.  Measured (GEMV / GEMM, us, in a chain): int4, groups of 128, 8 rows of 28672 x 8192 34.2 / 36, 9 rows of 12288 x 4096 16.0 /
+// 16.9, 16384 x 4096 17.7 / 18.5, 20480 x 4096 20.6 / 19.9, 28672 x 4096 26.5 / 23.5, 12 rows of 12288 x 4096 16.7 / 17.4, 14336 x 4096 18.1 / 18.1, 16384 x 4096 21.0 / 18.6, 16
+// rows of 12288 x 4096 18.8 / 17.3 (groups of 256 the same); smaller groups lengthen the GEMM's epilogue: groups of 64, 9 rows of 14336 x 4096 18.7 / 19.4, 20480 x 4096
+// 22.4 / 22.8, 24576 x 4096 25.7 / 25.8, 28672 x 4096 28.9 / 27.3, 12 rows of 14336 x 4096 19.4 / 19.5, 16384 x 4096 22.0 / 20.7; of 32, 9 rows of 16384 x 4096 22.2 / 23.4, 20480 x
+// 4096 26.4 / 26.2, 12 rows of 16384 x 4096 26.2 / 23.4; int8, 9 rows of 20480 x 4096 23.1 / 23.1, 24576 x 4096 26.4 / 26.1, 28672 x 4096 29.4 / 26.2.  (A rule by size and rows: in
+// between, weights whose row blocks go round the SMs evenly are the GEMM's earlier, 9 rows of 18944 x 3584 18.3 / 14.2.)  Where
 // the activations do not fit one CTA, up to 8 rows share k over a cluster if that takes them (share_k, which is asked first); for the others, 9 to 16 rows
 // as a rule, the strip kernels are the other choice: int4 8192 x 28672 62 .. 63 / 38 from 3 to 16 rows, 4096 x 14336, 16 rows 18.2 / 18.5; int8 8192 x 28672,
 // 16 rows 78 / 49, 4096 x 14336, 12 rows 27 / 21.
-static bool few_rows_by_gemm(int64_t M, int64_t Np, int64_t Kp, bool fits, bool int4) {
+static bool few_rows_by_gemm(int64_t M, int64_t Np, int64_t Kp, bool fits, int G) {  // (G 0: int8)
   if (M < 3 || Np % 128 != 0) return false;
   if (M > 16) return true;
-  if (fits) return M > 8 && (Np * Kp >= (int64_t)(int4 ? 48 : 96) << 20 || (M - 8) * Np * Kp > (int64_t)224 << 20);
-  return Np * Kp >= (int64_t)128 << 20 || (!int4 && M > 8);
+  const int64_t line = G == 0 || G == 64 ? 96 : (G == 32 ? 80 : 72);
+  if (fits) return M > 8 && (Np * Kp >= line << 20 || (M - 8) * Np * Kp > (int64_t)224 << 20);
+  return Np * Kp >= (int64_t)128 << 20 || (G == 0 && M > 8);
 }
 static bool int4_by_gemm(int64_t M, int64_t Np, int64_t Kp, int G) {
-  return tunables().gemm_tc && few_rows_by_gemm(M, Np, Kp, M > 16 || ao::int4_gemv_fused_fits(M, Kp, G, tunables().stages), true);
+  return tunables().gemm_tc && few_rows_by_gemm(M, Np, Kp, M > 16 || ao::int4_gemv_fused_fits(M, Kp, G, tunables().stages), G);
 }
 static bool int8_by_gemm(int64_t M, int64_t Np, int64_t Kp) {
-  return tunables().gemm_tc && few_rows_by_gemm(M, Np, Kp, M > 16 || ao::int8_gemv_fused_fits(M, Kp, tunables().stages), false);
+  return tunables().gemm_tc && few_rows_by_gemm(M, Np, Kp, M > 16 || ao::int8_gemv_fused_fits(M, Kp, tunables().stages), 0);
 }
 
 extern "C" int64_t ao_b200_int4_mm_workspace_bytes(int64_t M, int64_t Np, int64_t Kp) {
@@ -117,7 +121,7 @@ extern "C" int64_t ao_b200_int4_mm_workspace_bytes(int64_t M, int64_t Np, int64_
   // The mma.sync kernels reduce inside the CTA and need none.
   const int64_t gemv = ao::int4_gemv_tc_workspace_bytes(Np);
   // (up to 16 rows whether the GEMM is taken depends on the group size too: room for it wherever it may be)
-  return gemv + (M >= 3 && (M > 16 || few_rows_by_gemm(M, Np, Kp, true, true) || few_rows_by_gemm(M, Np, Kp, false, true))
+  return gemv + (M >= 3 && (M > 16 || few_rows_by_gemm(M, Np, Kp, true, 128) || few_rows_by_gemm(M, Np, Kp, false, 128))
                      ? ao::int4_gemm_tc_workspace_bytes(M, Np, Kp) : 0);
 }
 
@@ -133,8 +137,9 @@ extern "C" int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx
   auto s = static_cast<cudaStream_t>(stream);
   auto xb = static_cast<const __nv_bfloat16*>(x);
   auto yb = static_cast<__nv_bfloat16*>(y);
-  // (a large weight: 8192 x 28672, 3 to 7 rows 41 us with k shared, 37.5 by the GEMM; int8 44 to 48 and 48)
-  if (ao::share_k(M, Kp, ao::Instead::kNothingFits) && !(Np * Kp >= (int64_t)192 << 20 && tunables().gemm_tc && Np % 128 == 0) &&
+  // (a large weight: 8192 x 28672, 3 / 7 rows 39.2 / 40.8 us with k shared, 35.8 / 35.8 by the GEMM; but groups of 64 40.8 / 43.1 and 41.5 / 41.9, 16384 x 14336, 6 rows
+  // 37.4 and 41.7, groups of 32 42.6 and 49.6; int8 44 to 48 and 48)
+  if (ao::share_k(M, Kp, ao::Instead::kNothingFits) && !(Np * Kp >= (int64_t)192 << 20 && group_size > 64 && tunables().gemm_tc && Np % 128 == 0) &&
       !ao::int4_gemv_fused_fits(M, Kp, group_size, tunables().stages)) {
     const int e = ao::int4_gemv_split(x, M, Kx, ldx, packed, scale_and_zero, Np, Kp, group_size, y, N_out, ldy, nullptr, 0, tunables().stages,
                                       plain_follow(), s);

@@ -157,7 +157,7 @@ constexpr int kSplitStages = 4;
 //  - the GEMV over whole rows (they fit one CTA): 57344 activations.  int8, 8 rows of 3072 x 8192 12.1 / 8.7, of 8192 x 8192 19.1 / 16.0, 4 of
 //    4096 x 14336 15.4 / 14.7; int4 10.3 / 8.3, 15.5 / 13.4, 15.9 / 13.4.  Below: int8, 8 rows of 5120 x 5120 9.9 / 10.0, 4 of 8192 x 8192 14.4 / 15.2;
 //  - nothing fits, so a strip kernel or the GEMM: 3 rows (the kernels for up to 2 rows ask for less).  Int4 4096 x 14336, 8 rows 17.8 / 14.1, 8192 x 28672,
-//    3 / 7 rows 45.2 / 38.7, 45.5 / 40.5 (the GEMM since 37.5: ao_b200_int4_mm does not ask there any more); int8 17.7 / 16.4, 50.7 / 40.9, 50.8 / 45.5, 8 rows 50.8 / 49.4;
+//    3 / 7 rows 45.2 / 38.7, 45.5 / 40.5 (the GEMM since 35.8: for groups of 128 and 256 ao_b200_int4_mm does not ask there); int8 17.7 / 16.4, 50.7 / 40.9, 50.8 / 45.5, 8 rows 50.8 / 49.4;
 //  - the GEMM, which adds residuals: k of 8192.  Int4 3072 x 8192, 2 / 8 rows 14.9 / 7.6, 16.2 / 8.2, 8192 x 28672, 3 / 7 rows 45.5 / 38.2, 46 / 40.4; int8
 //    15.7 / 8.1, 17.4 / 8.7, 48.4 / 40.1, 49.5 / 45.4, 28672 x 8192, 8 rows 49.7 / 44.7.  Below: int8 28672 x 4096, 8 rows 30 / 36.
 // More rows are not split: twice the products per weight in CTAs with half the k (16 rows of 8192 x 8192: 26 us against the GEMM's 23).
