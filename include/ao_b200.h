@@ -124,7 +124,8 @@ AO_B200_API int ao_b200_tinygemm_pack(const int32_t* q, int64_t N, int64_t K, in
  * The weights may be the work of the kernel in front in the stream: they are read behind its end.  (The same for ao_b200_int8_mm.)
  * workspace: ao_b200_int4_mm_workspace_bytes(...) bytes, zero-initialised once by the
  * caller (the GEMV's part in front is zero again on exit, the GEMM's behind it is not
- * and need not be); may be NULL when that returns 0. */
+ * and need not be); may be NULL when that returns 0.  The size is for that number of rows: fewer rows may need more (tiles of 256 rows give larger
+ * shares than tiles of 144), so a workspace for several counts takes the largest of their sizes.  (The same for the other two workspace functions.) */
 AO_B200_API int64_t ao_b200_int4_mm_workspace_bytes(int64_t M, int64_t Np, int64_t Kp);
 AO_B200_API int ao_b200_int4_mm(const void* x, int64_t M, int64_t Kx, int64_t ldx,
                     const void* packed, const void* scale_and_zero, int64_t Np, int64_t Kp,
@@ -248,7 +249,9 @@ AO_B200_API int ao_b200_int8_gemv_fused(const void* x, int64_t M, int64_t Kx, in
 
 /* RMSNorm.forward (model.py:489-503) with an optional fused residual add:
  *   h = bf16(x + residual) (written to h_out when non-NULL);  y = bf16( bf16(h * rsqrt(mean(h^2)+eps)) * weight ).
- * x, residual, h_out, y: bf16 [rows][dim]; weight bf16 [dim]; dim % 8 == 0. */
+ * x, residual, h_out, y: bf16 [rows][dim]; weight bf16 [dim]; dim % 8 == 0.
+ * Up to 16384 columns a kernel that is launched programmatically behind it (cudaLaunchAttributeProgrammaticStreamSerialization) may start before y and h_out
+ * are written: it waits (griddepcontrol.wait) before it reads them.  Plain launches, copies and events wait as ever. */
 AO_B200_API int ao_b200_rmsnorm(const void* x, const void* residual, const void* weight, void* h_out, void* y,
                     int64_t rows, int64_t dim, float eps, void* stream);
 
@@ -309,7 +312,8 @@ AO_B200_API int ao_b200_silu_mul(const void* gate_up, void* out, int64_t B, int6
 
 /* The same two for rows of a prompt.
  * apply_rotary_emb: x bf16 [B][T][H][head_dim] (strides in elements, multiples of 8), freqs_cis bf16 [T][head_dim / 2][2],
- * y packed; head_dim % 8 == 0.   y[i] = bf16( bf16(silu(gate[i])) * up[i] ), count % 8 == 0.   All 16-byte aligned. */
+ * y packed; head_dim % 8 == 0.   y[i] = bf16( bf16(silu(gate[i])) * up[i] ), count % 8 == 0 (a kernel launched
+ * programmatically behind it: as behind ao_b200_rmsnorm).   All 16-byte aligned. */
 AO_B200_API int ao_b200_rotary(const void* x, int64_t stride_b, int64_t stride_t, int64_t stride_h, const void* freqs_cis, void* y, int64_t B,
                                int64_t T, int64_t H, int64_t head_dim, void* stream);
 /* The keys of a prompt rotated in the same way and, with the values, stored in the rows pos[t] (int32 or int64 [T], pos_bytes each; negative: from the end) of the caches

@@ -120,7 +120,7 @@ class RMSNorm(nn.Module):
         w = self.weight
         dim = x.shape[-1] if x.dim() else 0
         if (type(w) is nn.Parameter and _rows_by_kernel(x, w.data) and not (w.requires_grad and torch.is_grad_enabled()) and x.is_contiguous()
-                and w.shape == (dim,) and w.is_contiguous() and dim % 8 == 0 and dim <= 12272):   # a row in 48 KB of shared memory
+                and w.shape == (dim,) and w.is_contiguous() and dim % 8 == 0 and dim <= 12272):   # (the kernel takes more; longer rows have always been tensor operations)
             out = torch.empty_like(x)
             with _on(x.device.index):
                 _lib.check(_lib.lib().ao_b200_rmsnorm(x.data_ptr(), None, w.data_ptr(), None, out.data_ptr(), x.numel() // dim, dim, self.eps,

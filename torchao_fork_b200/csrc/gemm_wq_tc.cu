@@ -40,7 +40,7 @@
 // about 900 clocks per set of warps, two sets in flight), below that by the dequant -> MMA chain of a unit: conversions (all 16 warps at them at the
 // same time, 440 clocks per 128 k and set) and, once per unit, the way over six barriers, about 700 clocks of each role.  Hence units of 256 k up to
 // 128 rows: int4 28672 x 8192, 16 / 32 / 64 rows 46.9 / 47.7 / 49.5 -> 37.4 / 38.0 / 41.1 us, 14336 x 4096, 77 rows 26.1 -> 23.8, int8 28672 x 8192 and
-// 14336 x 4096, 16 rows 49.5 -> 46.5, 23.3 -> 20.2; from 144 rows on they give nothing (200 rows 75.2 and 75.3; int8 300 rows 40.2 and 42.5).  Measured,
+// 14336 x 4096, 16 rows 49.5 -> 46.5, 23.3 -> 20.2; from 144 rows on they give nothing (int4 28672 x 8192, 200 rows 75.2 and 75.3; int8 14336 x 4096, 300 rows 40.2 and 42.5).  Measured,
 // 14336 x 4096, int4 with groups of 128, M = 64 / 256 / 512 / 1000 / 2048: 22 / 37.6 / 54.2 / 94 / 174 us, the last 0.85 of 1634 TFLOP/s (one CTA
 // per 128 x 256 tile with the whole K, activations multicast over 4 CTAs, run-time divisions and parameters read from global memory in
 // the dequant loop: 29.9 / 36.5 / 67.0 / 128 / 225 us); int8 8192 x 8192, M = 32 / 512 / 2048: 24 / 63 / 227 us (44 / 66 / 244 us).
@@ -1028,7 +1028,9 @@ static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
   auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
   w.off_part = up(w.n_tickets * 4);
   w.off_xt = w.off_part + (!shared ? 0 : up((int64_t)w.workers * 2 * w.ranks * w.NT * 512));
-  w.bytes = w.off_xt + up((int64_t)w.MT * w.ranks * w.KU * w.x_bytes);  // (DIRECT too: a workspace for many rows does for fewer)
+  w.bytes = w.off_xt + up((int64_t)w.MT * w.ranks * w.KU * w.x_bytes);
+  // (DIRECT too, where nobody writes the copy, 29 MB of 68 at int8 4096 x 14336, 1000 rows: callers count on room for one wherever the GEMM takes a call.  The size
+  // is that of these rows; fewer may need more, as shares go by NT: int4 4096 x 4096, 256 rows 41 MB, 257 rows 24 MB.)
   return true;
 }
 

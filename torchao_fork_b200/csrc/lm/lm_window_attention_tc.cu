@@ -26,7 +26,8 @@
 // heads of 128 (four key heads): 8.5 steps a CTA, 60 us, tensor pipe active in 31 % of the clocks, against 308 us of window_attention_prompt_kernel; the same with
 // all keys of a tile in one CTA 110 us (the last tiles alone took 95), with unswizzled operands 84 us.
 // A warp's instructions follow one another at nearly five clocks each, so what counts is their number, about 740 per step at first: addresses once per map
-// instead of once per load, the largest score three at a time, O to shared memory 32 columns at a time: 57.6 -> 55.8 us, 117 rows of two maps 20.5 -> 19.2.
+// instead of once per load, the largest score three at a time, O to shared memory 32 columns at a time: 57.6 -> 55.8 us, 117 rows of two maps 20.5 -> 19.2,
+// heads of 64 (keys in rows of 8 pieces, values drained 8 columns at a time) 2048 rows 50.7 -> 47.8, 200 rows of 8 heads 11.1 -> 10.3, of 96 55.3 -> 51.3.
 // Launched while the kernel in front ends (nothing of memory is touched before the wait): in a series of calls 59.4 -> 56.7 us.  Letting the kernel behind
 // start as early: 55.0, but 16 to 23 us calls up to 4 us more, as its CTAs take the places of the last ones of this.
 // Taken back: four threads per row (16 warps for the weights: 70.0 us in place of 55.8); the next step's scores beside this one's weights (two score buffers,
