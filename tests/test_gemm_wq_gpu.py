@@ -413,3 +413,35 @@ def test_small_weights(bits, group, m, n, k):
                                          (256, 12, 14336, 4096), (256, 12, 14464, 4096), (32, 3, 8192, 24576), (64, 8, 8192, 24576), (64, 3, 8192, 24576), (128, 3, 8192, 24576)])
 def test_few_rows_by_group_on_both_sides_of_their_lines(group, m, n, k):
     _check(4, m, n, k, group)
+
+
+@pytest.mark.parametrize("bits,group", [(4, 64), (8, 0)])
+@pytest.mark.parametrize("m", [100, 600, 1024])
+def test_results_over_the_activations(bits, group, m):
+    # y in x's own memory, plain and with the rows themselves as residual: from 512 rows on the GEMM would read them while it writes
+    from torchao_fork_b200 import _lib
+    n = k = 1024
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    w = (torch.randn(n, k, generator=gen, device="cuda") / 32).to(torch.bfloat16)
+    x = torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16)
+    L, st = _lib.lib(), torch.cuda.current_stream().cuda_stream
+    if bits == 4:
+        packed, scales = T.b200_int4_quantize_pack(w, group, 1e-6, True)
+        plain = T.b200_int4_weight_only_mm(x, packed, group, scales, n)
+        size, call, rest = L.ao_b200_int4_mm_workspace_bytes, L.ao_b200_int4_mm, (n, k, group)
+    else:
+        q, scales = T.b200_int8_quantize(w, 1e-6, True)
+        packed = T.b200_int8_pack(q)
+        plain = T.b200_int8_weight_only_mm(x, packed, scales)
+        size, call, rest = L.ao_b200_int8_mm_workspace_bytes, L.ao_b200_int8_mm, (n, k)
+    ws = torch.zeros(max(size(m, n, k), L.ao_b200_mm_residual_workspace_bytes(m, n, k, group)), dtype=torch.uint8, device="cuda")
+    p = lambda t: t.data_ptr()  # noqa: E731
+    for _ in range(5):
+        over, both = x.clone(), x.clone()
+        _lib.check(call(p(over), m, k, k, p(packed), p(scales), *rest, p(over), n, n, p(ws), ws.numel(), st), "mm")
+        _lib.check(L.ao_b200_mm_residual(p(both), m, k, k, p(packed), p(scales), n, k, group, p(both), n, n, p(both), n, p(ws), ws.numel(), st), "mm_residual")
+        # (two orders of the same sums, each rounded within 2^-9 of its value: 2^-8 of the whole; a wrong row would be off by its size)
+        assert ((over.double() - plain.double()).norm() / plain.double().norm()).item() < 2.0 ** -8
+        want = (x.float() + plain.float()).to(torch.bfloat16)
+        assert ((both.double() - want.double()).norm() / want.double().norm()).item() < 2.0 ** -7
+        assert (over.float() - plain.float()).abs().amax(1).max() < 0.05 * plain.float().abs().max()

@@ -1029,8 +1029,8 @@ static bool wq_plan(int64_t M, int64_t Np, int64_t Kp, bool int4, WqPlan& w) {
   w.off_part = up(w.n_tickets * 4);
   w.off_xt = w.off_part + (!shared ? 0 : up((int64_t)w.workers * 2 * w.ranks * w.NT * 512));
   w.bytes = w.off_xt + up((int64_t)w.MT * w.ranks * w.KU * w.x_bytes);
-  // (DIRECT too, where nobody writes the copy, 29 MB of 68 at int8 4096 x 14336, 1000 rows: callers count on room for one wherever the GEMM takes a call.  The size
-  // is that of these rows; fewer may need more, as shares go by NT: int4 4096 x 4096, 256 rows 41 MB, 257 rows 24 MB.)
+  // (DIRECT too, where nobody writes the copy as a rule, 29 MB of 68 at int8 4096 x 14336, 1000 rows: wq_gemm may stage all the same.  The size is that of these rows;
+  // fewer may need more, as shares go by NT: int4 4096 x 4096, 256 rows 41 MB, 257 rows 24 MB.)
   return true;
 }
 
@@ -1172,7 +1172,11 @@ static int wq_gemm(const void* x, int64_t M, int64_t Kx, int64_t ldx, const void
   const bool ok = G ? wq_map(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, packed, Kp * 8, Np / 16, 256) &&
                           wq_map(&p.smap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, sz, Kp / G * 64, Np / 16, (G < 128 ? 128 / G : 1) * 16)
                     : wq_map(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_INT64, 8, packed, Kp * 16, Np / 16, 256);
-  if (!ok || (w.direct && !wq_map(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, Kx * 2, M, 64, ldx * 2, w.BR))) return AO_B200_ERR_UNSUPPORTED;
+  if (!ok) return AO_B200_ERR_UNSUPPORTED;
+  // Results may be written over the activations: then they are staged first (there is room: wq_plan), as where they are no tensor that the copy engine takes
+  const auto x0 = reinterpret_cast<uintptr_t>(x), y0 = reinterpret_cast<uintptr_t>(y);
+  const bool apart = x0 + ((M - 1) * ldx + Kx) * 2 <= y0 || y0 + ((M - 1) * ldy + N_out) * 2 <= x0;
+  w.direct = w.direct && apart && wq_map(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, Kx * 2, M, 64, ldx * 2, w.BR);
   p.tickets = reinterpret_cast<uint32_t*>(ws);
   p.part = reinterpret_cast<float*>(ws + w.off_part);
   p.xt = ws + w.off_xt;
