@@ -445,3 +445,10 @@ def test_results_over_the_activations(bits, group, m):
         want = (x.float() + plain.float()).to(torch.bfloat16)
         assert ((both.double() - want.double()).norm() / want.double().norm()).item() < 2.0 ** -7
         assert (over.float() - plain.float()).abs().amax(1).max() < 0.05 * plain.float().abs().max()
+
+
+@pytest.mark.parametrize("bits,group", [(4, 128), (4, 32), (8, 0)])
+@pytest.mark.parametrize("m,n,k", [(17, 28672, 1280), (33, 28672, 768), (64, 28672, 2048), (128, 28672, 1280), (100, 20480, 1536)])
+def test_last_tile_from_the_accumulators_of_long_units(bits, group, m, n, k):
+    # a few units of 256 k a tile and more tiles than SMs: the neighbour has two units and more to do behind its share of the tile
+    _check(bits, m, n, k, group)

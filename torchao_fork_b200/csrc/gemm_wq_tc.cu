@@ -58,6 +58,7 @@ namespace ao {
 
 constexpr int kWqEpiWarps = 4, kWqDqWarps = 16;
 constexpr int kWqBehind = 8;  // units (wq_gemm_kernel, t_early; 0, 4 and 16 measure the same, without the path 300 rows of 14336 x 4096 take 41.3 us, not 37.4)
+constexpr int kWqBehindLong = 2;  // of 256 k: int4 28672 x 1280, 128 rows 22.9 us with 4 and 8, 19.9 with 2 and 1; 28672 x 2048, 64 rows 23.0 with 8, 20.2 with 4 and less
 constexpr int kWqWProd = kWqEpiWarps + kWqDqWarps, kWqXProd = kWqWProd + 1, kWqMma = kWqXProd + 1;
 constexpr int kWqThreads = (kWqMma + 2) * 32;  // 768
 constexpr int kWqSlots = 4;                    // ring of A in tensor memory: 64 columns (128 k) each, or half as many of 256 k
@@ -725,7 +726,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) wq_gemm_kernel(const __grid_con
     int t_early = -1;
     if (EARLY && u1 % KU != 0) {
       const int t = u1 / KU;
-      if (u0 <= t * KU && wq_first(worker + 2, p.base, p.rem, p.quantum) >= (t + 1) * KU + kWqBehind) t_early = t;
+      if (u0 <= t * KU && wq_first(worker + 2, p.base, p.rem, p.quantum) >= (t + 1) * KU + (KW == 2 ? kWqBehindLong : kWqBehind)) t_early = t;
     }
     for (int u = u0, t = u0 / KU; u < u1; ++t) {
       const int ue = min(u1, (t + 1) * KU), nb = t / p.MT, mt = t - nb * p.MT;
