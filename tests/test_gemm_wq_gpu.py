@@ -402,7 +402,7 @@ def test_few_rows_on_both_sides_of_their_lines(bits, m, n, k):
     _check(bits, m, n, k, 128)
 
 
-@pytest.mark.parametrize("k", [256, 512, 768, 1280, 2048, 2304, 2816, 3328, 4096])
+@pytest.mark.parametrize("k", [256, 512, 768, 1280, 2048, 2304, 2816, 3328, 4096, 9472, 11008])   # (9472: 37 units, dealt as 39)
 @pytest.mark.parametrize("bits,group,m,n", [(4, 128, 17, 1024), (4, 32, 32, 321), (4, 256, 33, 4096), (4, 64, 128, 8192), (8, 0, 17, 1000), (8, 0, 16, 14336), (8, 0, 64, 640)])
 def test_small_weights(bits, group, m, n, k):
     # tiles of one owner, of a few, and of as many as they have units (the number: wq_owners)

@@ -971,22 +971,26 @@ struct WqPlan {
 
 static int kw_of(const WqPlan& w) { return !w.direct && w.NT <= kWqLongNT ? 2 : 1; }
 
-// Small weights, up to 128 rows: where an even deal leaves a worker fewer than four units of 256 k, tiles are not cut where it happens to fall, but each
-// goes to so many owners, with equally many of its units each.  The number of owners per tile; 0: dealt evenly.  In units, a worker that holds pieces of
-// two tiles pays about 13 beside its own (two drains, two shares out, tickets, and the tile that it finishes); owners of one tile 5, and the adding up of a share
-// of NT rows for each of them; one owner nothing.  (One unit takes an owner as long as two, which go to its two sets of dequant warps.)  us, units of 128 k
-// evenly / of 256 k evenly / as here: int4, 17 rows, 4096 x 256 6.0 / 7.2 / 5.8, x 768 9.4 / 13.1 / 7.0, x 1280 11.4 / 13.8 / 8.0, x 2816 13.4 / 15.0 / 11.2, x 4096
-// 14.7 / 13.5 / 11.6, 14336 x 1024 12.9 / 12.2 / 8.2, 128 rows, 4096 x 256 9.0 / 11.8 / 9.0, 8192 x 768 16.4 / 18.6 / 10.9, x 2304 20.4 / 20.2 / 15.9, 4096 x 4096
-// 23.2 / 21.7 / 18.3; int8, 17 rows, 1024 x 768 9.7 / 14.2 / 7.2, 4096 x 2304 13.7 / 14.9 / 11.8; 8 rows with a residual, int4 4096 x 768 8.9 / 10.2 / 5.7.  Not as
-// good as units of 128 k: 1024 x 2304, 17 rows 10.2 / 11.9 / 10.4, int8 10.4 / 12.9 / 10.8, x 2816 11.0 / 13.7 / 11.3.
-static int wq_owners(const WqPlan& w, int sms) {
-  if (w.KW != 2 || w.tiles > sms || w.tiles * w.KU >= 4 * (int64_t)sms) return 0;
-  int64_t best = 160 * ((w.tiles * w.KU + sms - 1) / sms + 13);   // in 160ths of a unit
-  int owners = 0;
-  for (int s = 1; s <= w.KU && w.tiles * s <= sms; ++s) {
-    const int64_t cost = s == 1 ? 160 * w.KU : 160 * (w.KU / s > 2 ? w.KU / s : 2) + 800 + s * (w.NT > 32 ? w.NT : 32);
-    if (w.KU % s == 0 && cost < best) best = cost, owners = s;
+// Small weights, up to 128 rows and a tile per SM: where an even deal leaves a worker fewer than ten units of 256 k, tiles are not cut where it happens to fall, if
+// it costs less, but each goes to so many owners, with equally many of its units each (KU may grow by an eighth, of zeros, to divide).  The number of owners per tile; 0:
+// dealt evenly.  In units, a worker that holds pieces of two tiles pays 10 to 13 beside its own (two drains, two shares out, tickets, and the tile that it finishes);
+// owners of one tile 5 (two or three pairs of CTAs 7), and the adding up of a share of NT rows for each of them; one owner nothing.  (One unit takes an owner as long as two, which
+// go to its two sets of dequant warps.)  us, units of 128 k evenly / of 256 k evenly / as here: int4, 17 rows, 4096 x 256 6.0 / 7.2 / 5.8, x 768 9.4 / 13.1 / 7.0, x 1280 11.4 /
+// 13.8 / 8.0, x 2816 13.4 / 15.0 / 11.2, x 4096 14.7 / 13.5 / 11.6, 14336 x 1024 12.9 / 12.2 / 8.2, 128 rows, 4096 x 256 9.0 / 11.8 / 9.0, 8192 x 768 16.4 / 18.6 / 10.9, x 2304
+// 20.4 / 20.2 / 15.9, 4096 x 4096 23.2 / 21.7 / 18.3; int8, 17 rows, 1024 x 768 9.7 / 14.2 / 7.2, 4096 x 2304 13.7 / 14.9 / 11.8, 77 rows 14336 x 3328 25.2 / 27.5 / 22; 8 rows with
+// a residual, int4 4096 x 768 8.9 / 10.2 / 5.7.  Of 2856 sizes 31 are 2 to 6 % slower than with units of 128 k, most of them int8 on 10240 outputs; beyond ten units a
+// worker an even deal was not slower than those (whole tiles are faster up to a tile per worker there too: int4 14336 x 4096, 128 rows 26.5 / 22.0, not taken here).
+static int wq_owners(WqPlan& w, int sms) {
+  if (w.KW != 2 || w.tiles > sms || w.tiles * w.KU >= 10 * (int64_t)sms) return 0;
+  int64_t best = 160 * ((w.tiles * w.KU + sms - 1) / sms + (w.tiles * w.KU < 4 * (int64_t)sms ? 13 : 10));   // in 160ths of a unit
+  int owners = 0, units = w.KU;
+  for (int ku = w.KU; ku <= w.KU + (w.KU + 7) / 8; ++ku) {
+    for (int s = 1; s <= ku && w.tiles * s <= sms; ++s) {
+      const int64_t cost = s == 1 ? 160 * ku : 160 * (ku / s > 2 ? ku / s : 2) + (w.pair && s < 4 ? 1120 : 800) + s * (w.NT > 32 ? w.NT : 32);
+      if (ku % s == 0 && cost < best) best = cost, owners = s, units = ku;
+    }
   }
+  w.KU = units;
   return owners;
 }
 
