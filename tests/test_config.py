@@ -73,7 +73,7 @@ def test_foreign_types_are_rejected(evil):
 
 
 def test_rejecting_does_not_run_anything():
-    # the advisor's proof of concept: this dictionary used to spawn a process
+    # this dictionary used to spawn a process
     code = ("import sys; sys.path.insert(0, %r)\n"
             "from torchao_fork_b200.core.config import config_from_dict\n"
             "try:\n"

@@ -977,8 +977,8 @@ static int kw_of(const WqPlan& w) { return !w.direct && w.NT <= kWqLongNT ? 2 : 
 // owners of one tile 5 (two or three pairs of CTAs 7), and the adding up of a share of NT rows for each of them; one owner nothing.  (One unit takes an owner as long as two, which
 // go to its two sets of dequant warps.)  us, units of 128 k evenly / of 256 k evenly / as here: int4, 17 rows, 4096 x 256 6.0 / 7.2 / 5.8, x 768 9.4 / 13.1 / 7.0, x 1280 11.4 /
 // 13.8 / 8.0, x 2816 13.4 / 15.0 / 11.2, x 4096 14.7 / 13.5 / 11.6, 14336 x 1024 12.9 / 12.2 / 8.2, 128 rows, 4096 x 256 9.0 / 11.8 / 9.0, 8192 x 768 16.4 / 18.6 / 10.9, x 2304
-// 20.4 / 20.2 / 15.9, 4096 x 4096 23.2 / 21.7 / 18.3; int8, 17 rows, 1024 x 768 9.7 / 14.2 / 7.2, 4096 x 2304 13.7 / 14.9 / 11.8, 77 rows 14336 x 3328 25.2 / 27.5 / 22; 8 rows with
-// a residual, int4 4096 x 768 8.9 / 10.2 / 5.7.  Of 2856 sizes 31 are 2 to 6 % slower than with units of 128 k, most of them int8 on 10240 outputs; beyond ten units a
+// 20.4 / 20.2 / 15.9, 4096 x 4096 23.2 / 21.7 / 18.3; int8, 17 rows, 1024 x 768 9.7 / 14.2 / 7.2, 4096 x 2304 13.7 / 14.9 / 11.8, 100 rows 14336 x 2816 25.0 / 25.3 / 19.6; 8 rows with
+// a residual, int4 4096 x 768 8.9 / 10.2 / 5.7.  Of 900 sizes of 17 to 128 rows 6 are 2 to 6 % slower than with units of 128 k, most of them int8 and dealt evenly; beyond ten units a
 // worker an even deal was not slower than those (whole tiles are faster up to a tile per worker there too: int4 14336 x 4096, 128 rows 26.5 / 22.0, not taken here).
 static int wq_owners(WqPlan& w, int sms) {
   if (w.KW != 2 || w.tiles > sms || w.tiles * w.KU >= 10 * (int64_t)sms) return 0;
